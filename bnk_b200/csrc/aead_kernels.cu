@@ -21,7 +21,7 @@
 // FMA pipe.  The MAC input is ciphertext | zero pad to 16 | le64(0) | le64(ct_len),
 // RFC 8439 section 2.8 with empty AAD; nonce = 32 zero bits | le64(counter) and the
 // header is le32(4) | le32(receiver index) | le64(counter) (WireGuard whitepaper 5.4.6).
-#include "bnk_internal.cuh"
+#include "filter_device.cuh"
 
 namespace {
 
@@ -219,8 +219,7 @@ __device__ __forceinline__ uint32_t wg_padded_len(uint32_t len, uint32_t mtu) {
 }
 
 // ---------------------------------------------------------------------------
-// Descriptor of one packet, validated.  `writer` says whether this thread records the
-// outcome of a refused packet (one thread per packet does).
+// Descriptor of one packet, validated; the outcome of a refused packet is recorded here.
 // ---------------------------------------------------------------------------
 struct Desc {
     uint32_t off, body /* bytes under the cipher */, in_len /* bytes to fetch */, n_lo, n_hi, slot;
@@ -228,7 +227,7 @@ struct Desc {
 };
 
 template <bool OPEN>
-__device__ __forceinline__ Desc load_desc(const AeadArgs &a, uint32_t pkt, bool have, bool writer) {
+__device__ __forceinline__ Desc load_desc(const AeadArgs &a, uint32_t pkt, bool have) {
     Desc d{0, 0, 0, 0, 0, 0, false};
     if (!have) return d;
     uint8_t st = BNK_PKT_OK;
@@ -265,10 +264,10 @@ __device__ __forceinline__ Desc load_desc(const AeadArgs &a, uint32_t pkt, bool 
             st = BNK_PKT_MALFORMED;
             d.live = false;
         } else {
-            const uint4 hdr = *reinterpret_cast<const uint4 *>(a.ring + d.off);
+            const uint4 hdr = *reinterpret_cast<const uint4 *>(a.out + d.off);
             d.n_lo = hdr.z;
             d.n_hi = hdr.w;
-            if (writer) a.counter[pkt] = ((uint64_t)hdr.w << 32) | hdr.z;
+            a.res[0].counter[pkt] = ((uint64_t)hdr.w << 32) | hdr.z;
             if (hdr.x != 4u) {
                 st = BNK_PKT_MALFORMED;
                 d.live = false;
@@ -279,10 +278,8 @@ __device__ __forceinline__ Desc load_desc(const AeadArgs &a, uint32_t pkt, bool 
         }
     }
     if (!d.live) {
-        if (writer) {
-            a.status[pkt] = st;
-            a.out_len[pkt] = 0;
-        }
+        a.res[0].status[pkt] = st;
+        a.res[0].out_len[pkt] = 0;
         d.body = 0;
         d.in_len = 0;
     }
@@ -294,17 +291,17 @@ __device__ __forceinline__ Desc load_desc(const AeadArgs &a, uint32_t pkt, bool 
 // The throughput kernel: used when the batch is large enough to fill the GPU with one packet per thread.
 // ---------------------------------------------------------------------------
 template <bool OPEN>
-__global__ void __launch_bounds__(kThreads, BNK_MIN_CTAS) aead_kernel(const AeadArgs a) {
+__global__ void __launch_bounds__(kThreads, BNK_MIN_CTAS) aead_kernel(const __grid_constant__ AeadArgs a) {
     let_next_kernel_start();
     wait_for_kernel_in_front();
     const uint32_t idx = blockIdx.x * kThreads + threadIdx.x;
     const bool have = idx < a.n;
     const uint32_t pkt = have ? (a.order ? a.order[idx] : idx) : 0u;
-    const Desc dsc = load_desc<OPEN>(a, pkt, have, true);
+    const Desc dsc = load_desc<OPEN>(a, pkt, have);
     const uint32_t off = dsc.off, body = dsc.body, in_len = dsc.in_len, n_lo = dsc.n_lo, n_hi = dsc.n_hi, slot = dsc.slot;
     const bool live = dsc.live;
     const uint32_t nblk = (body + 63u) >> 6;
-    uint8_t *const data = a.ring + (size_t)off + BNK_WG_HEADER; // 16-byte aligned
+    uint8_t *const data = a.out + (size_t)off + BNK_WG_HEADER; // 16-byte aligned
 
     uint32_t key[8];
     Poly poly;
@@ -392,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, BNK_MIN_CTAS) aead_kernel(const Aead
     uint8_t *tagp = data + body;
 
     if (!OPEN) {
-        *reinterpret_cast<uint4 *>(a.ring + off) = make_uint4(4u, a.remote_index[slot], n_lo, n_hi);
+        *reinterpret_cast<uint4 *>(a.out + off) = make_uint4(4u, a.remote_index[slot], n_lo, n_hi);
         if ((body & 3u) == 0) {
             uint32_t *t32 = reinterpret_cast<uint32_t *>(tagp);
             t32[0] = tag[0]; t32[1] = tag[1]; t32[2] = tag[2]; t32[3] = tag[3];
@@ -402,8 +399,8 @@ __global__ void __launch_bounds__(kThreads, BNK_MIN_CTAS) aead_kernel(const Aead
 #pragma unroll
                 for (int k = 0; k < 4; k++) tagp[4 * w + k] = (uint8_t)(tag[w] >> (8 * k));
         }
-        a.status[pkt] = BNK_PKT_OK;
-        a.out_len[pkt] = BNK_WG_HEADER + body + BNK_WG_TAG;
+        a.res[0].status[pkt] = BNK_PKT_OK;
+        a.res[0].out_len[pkt] = BNK_WG_HEADER + body + BNK_WG_TAG;
     } else {
         uint32_t diff = 0;
         if ((body & 3u) == 0) {
@@ -416,16 +413,16 @@ __global__ void __launch_bounds__(kThreads, BNK_MIN_CTAS) aead_kernel(const Aead
                 for (int k = 0; k < 4; k++) diff |= (uint32_t)(tagp[4 * w + k] ^ (uint8_t)(tag[w] >> (8 * k)));
         }
         if (diff == 0) {
-            a.status[pkt] = body ? BNK_PKT_OK : BNK_PKT_KEEPALIVE;
-            a.out_len[pkt] = body;
+            a.res[0].status[pkt] = body ? BNK_PKT_OK : BNK_PKT_KEEPALIVE;
+            a.res[0].out_len[pkt] = body;
         } else {
             // forged or damaged: no plaintext may leave, wipe what the fused pass wrote
             uint8_t *dst = data;
             uint32_t k = 0;
             for (; k + 16u <= body; k += 16u) *reinterpret_cast<uint4 *>(dst + k) = make_uint4(0, 0, 0, 0);
             for (; k < body; k++) dst[k] = 0;
-            a.status[pkt] = BNK_PKT_AUTH_FAIL;
-            a.out_len[pkt] = 0;
+            a.res[0].status[pkt] = BNK_PKT_AUTH_FAIL;
+            a.res[0].out_len[pkt] = 0;
         }
     }
 }
@@ -522,200 +519,426 @@ __device__ __forceinline__ void p26_finish(const P26 &x, const uint32_t (&pad)[4
 }
 
 // ---------------------------------------------------------------------------
-// Kernel 2, warp per packet: the latency kernel for batches too small to fill the GPU with one
-// packet per thread (a 128-packet batch takes ~24 sequential cipher blocks per thread there).
-// Lane j of a round takes one 64-byte chunk: its ChaCha20 block and the Poly1305 Horner steps over
-// its four 16-byte blocks starting from zero, Q_j = sum_s b_s r^(5-s).  The chunks of a round, up
-// to 30, sit right-aligned in lanes 31-F..30; lane 30-F carries the running state in; a binary
-// tree over the warp (five shuffle + multiply steps with r^4, r^8, ... r^64) folds them to
-//   state' = state * r^(4F) + sum_j Q_j * r^(4(F-1-j))
-// on lane 30.  Lane 31 then continues sequentially over what is left of the packet (up to three whole
-// blocks and a ragged one) and the length block, and makes the tag.  Block 0 of the keystream (the
-// one-time Poly1305 key) is computed by the carry lane of the first round in the same pass as the data
-// blocks.  Accesses are coalesced by construction: consecutive lanes hold consecutive 64 bytes.
+// Kernel 2, warp per packet: the kernel for batches too small to fill the GPU with one packet per thread, and for
+// batches that stay in the caller's pinned memory (AeadArgs::in / out are then host addresses and the host link is
+// the bound).
+//
+// A round covers up to 31 cipher blocks (1984 payload bytes; a full-size packet is one round).  The warp brings the
+// round's bytes into shared memory in 16-byte pieces with cp.async, in windows that start on 128-byte lines: over
+// the host link an instruction then asks for whole lines (measured on 4096 x 1440 B, read and written in place:
+// 172 us against 177 with windows at the packet's own 16-byte alignment).  Lane 0 computes cipher block 0 (the
+// one-time Poly1305 key), lane j the round's block j, all in the same pass.  For Poly1305 the round's 16-byte blocks
+// are laid out from the right, four to a lane, the length block last in lane 31, so that every lane runs the same
+// Horner steps from zero (the lane of the first block starts from the state carried in) and a binary tree over the
+// lanes with r^4, r^8 ... folds them; no lane works through a ragged end while the others idle.  What leaves the
+// round is put together in shared memory and written in the same pieces, so ragged ends cost one store instruction.
+// A tag is checked before a one-round packet's plaintext is written.
+//
+// A warp takes tiles of a.tile consecutive packets (one in small batches); the descriptors of a tile lie in its
+// lanes, and the next packet's bytes are on their way while one is computed.  Few warps are enough to keep the host
+// link busy, and more of them in flight make it slower (read + write of 4096 x 1440 B: 172 us from 16 CTAs of 8
+// warps, 184 from 148, 225 from 512), so the grid is capped for host-resident rings (wpp_grid).
 // ---------------------------------------------------------------------------
-constexpr uint32_t kWppFull = 30;
+constexpr uint32_t kWppWarps = 8;
+constexpr uint32_t kRoundBlocks = 31;
+constexpr uint32_t kRoundBytes = kRoundBlocks * 64;
+constexpr uint32_t kStagePieces = 136; // <= 7 of the first line + header + 124 body + 1 of the tag, rounded to the swizzle's 8
 
-template <bool OPEN>
-__global__ void __launch_bounds__(128) aead_wpp_kernel(const AeadArgs a) {
-    let_next_kernel_start();    // open side: the grouping + replay launch behind may take its place already
-    wait_for_kernel_in_front(); // seal side: the counters come from the grouping launch in front
-    __shared__ uint4 stage_all[4][128]; // per warp: the 16-byte pieces of one round (up to 30 chunks of 64 bytes)
+// Lane j reads its four pieces 4j .. 4j+3 with 16-byte loads: the plain layout would put eight lanes on two bank
+// groups; flipping the low bits of the piece number by its line number spreads them over all eight.
+__device__ __forceinline__ uint32_t stage_at(uint32_t piece) { return piece ^ ((piece >> 3) & 3u); }
+__device__ __forceinline__ void copy_async16(void *smem, const void *gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+// The pieces of round `rnd` of a packet: where they lie and how many there are.
+struct Round {
+    uint64_t window;  // ring offset of the 128-byte line the first piece lies in
+    uint32_t first;   // piece number (from the window) of the header (round 0) or of the round's first body byte
+    uint32_t body;    // piece number of the round's first body byte
+    __device__ __forceinline__ Round(uint32_t off, uint32_t rnd) {
+        const uint64_t at = rnd == 0 ? (uint64_t)off : (uint64_t)off + BNK_WG_HEADER + (uint64_t)rnd * kRoundBytes;
+        window = at & ~127ull;
+        first = (uint32_t)(at & 127u) >> 4;
+        body = first + (rnd == 0 ? 1u : 0u);
+    }
+};
+
+//
+// Seal batches of up to kRankMax packets in pinned memory hand out their nonces here (a.send_counter): every CTA reads
+// the batch's slots, a warp counts the packets of its slot in front of its own, and of the packets of a slot the one
+// that reads the counter last moves it past them all.  A grouping launch in front costs more than this reading.
+// NOTE: the flows of the packets are recorded from the bytes in the stage, each step of the table's atomics behind a
+// piece of the cipher work.
+// Word `lane` (0..15) of the 64 bytes that start at a piece.
+__device__ __forceinline__ uint32_t stage_word(const uint4 *stage, uint32_t piece) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (idx >= a.n) return; // a whole warp at a time
-    const uint32_t pkt = a.order ? a.order[idx] : idx;
-    const Desc dsc = load_desc<OPEN>(a, pkt, true, lane == 0);
-    if (!dsc.live) return;
-    const uint32_t body = dsc.body, in_len = dsc.in_len;
-    uint8_t *const data = a.ring + (size_t)dsc.off + BNK_WG_HEADER;
+    return reinterpret_cast<const uint32_t *>(&stage[stage_at(piece + ((lane >> 2) & 3u))])[lane & 3u];
+}
 
-    uint32_t key[8];
-    {
-        const uint4 *kp = reinterpret_cast<const uint4 *>(a.keys + (size_t)dsc.slot * 8);
-        const uint4 ka = kp[0], kb = kp[1];
-        key[0] = ka.x; key[1] = ka.y; key[2] = ka.z; key[3] = ka.w;
-        key[4] = kb.x; key[5] = kb.y; key[6] = kb.z; key[7] = kb.w;
-    }
-    const uint32_t full_total = body >> 6, tail_bytes = body & 63u;
-    P26 r = p26_zero(), state = p26_zero();
-    uint32_t pad[4] = {0, 0, 0, 0};
-    uint32_t ct[16]; // the lane's ciphertext words of the current round (lane 31: the ragged tail)
-#pragma unroll
-    for (int i = 0; i < 16; i++) ct[i] = 0;
+template <bool OPEN, bool NOTE>
+__global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __grid_constant__ AeadArgs a) {
+    static_assert(!(OPEN && NOTE), "flows are recorded on the seal side");
+    let_next_kernel_start(); // open side: the grouping + replay launch behind may take its place already
+    // What a ring in device memory holds may come from the kernel in front; a pinned ring and its descriptors are the
+    // host's, and only the counters of a seal come from there.
+    if (!a.over_link) wait_for_kernel_in_front();
+    __shared__ __align__(128) uint4 stage_all[kWppWarps][2][kStagePieces];
+    __shared__ __align__(16) uint4 key_all[kWppWarps][2][2];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t T = a.tile, tiles = (a.n + T - 1) / T, step = gridDim.x * kWppWarps;
 
-    uint32_t done = 0;
-    bool first = true, last_round;
-    do {
-        const uint32_t remaining = full_total - done;
-        last_round = remaining <= kWppFull;
-        const uint32_t F = last_round ? remaining : kWppFull;
-        const bool is_chunk = lane + F >= 31u && lane <= 30u;
-        const bool is_carry = lane + F == 30u;
-        const bool is_tail = last_round && lane == 31u && tail_bytes != 0;
-        const bool works = is_chunk || is_tail;
-        const uint32_t chunk = is_tail ? full_total : done + (lane + F - 31u);
-        const uint32_t base = chunk * 64u;
-
-        // The round's F chunks are 64 F consecutive bytes.  The warp fetches them as 16-byte pieces in piece order
-        // (lane l takes pieces l, 32 + l, ...: every load instruction covers 512 consecutive bytes) and hands each
-        // chunk lane its four pieces through shared memory.  Fetched chunk by chunk instead, a load instruction
-        // touches thirty-two separate 16-byte pieces 64 bytes apart: the same bytes from device memory, but when the
-        // ring is the caller's pinned host memory (small batches run there, no copies) every piece is a PCIe read
-        // of its own, and few of those can be in flight.
-        const uint32_t round_base = done * 64u;
-        uint4 *const stage = stage_all[threadIdx.x >> 5];
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const uint32_t q = 32u * c + lane;
-            if (q < 4u * F) {
-                uint4 v = make_uint4(0, 0, 0, 0);
-                if (round_base + 16u * q < in_len) v = *reinterpret_cast<const uint4 *>(data + round_base + 16u * q);
-                stage[q] = v;
+    struct Tile { // one packet's descriptor in each of the first T lanes
+        uint32_t off, len, slot, valid, remote;
+        uint64_t ctr;
+    };
+    auto load_tile = [&](uint32_t t) {
+        Tile d{0, 0, 0, 0, 0, 0};
+        const uint32_t i = t * T + lane;
+        if (t < tiles && lane < T && i < a.n) {
+            d.off = a.off[i];
+            d.len = a.len[i];
+            if (!OPEN || !a.demux) d.slot = a.slot[i];
+        }
+        return d;
+    };
+    auto load_keypair = [&](Tile &d, uint32_t t) { // what hangs on the slot: asked for once the slot is there
+        const uint32_t i = t * T + lane;
+        if (!OPEN && a.send_counter == nullptr && t < tiles && lane < T && i < a.n) d.ctr = a.counter[i];
+        if (!(OPEN && a.demux) && d.slot < a.max_slots) {
+            d.valid = a.valid[d.slot];
+            if (!OPEN) d.remote = a.remote_index[d.slot];
+        }
+    };
+    // Starts the copies of a packet's first round (and of its keys when the slot is known) into stage `buf`.
+    auto fetch = [&](uint32_t off, uint32_t len, uint32_t slot, uint32_t buf) {
+        uint4 *const stage = stage_all[warp][buf];
+        if (!(off & 15u)) {
+            const Round r(off, 0);
+            uint32_t from, bytes; // pieces from `from` on, to the piece of byte `bytes` of the body
+            bool fits;
+            if (OPEN) {
+                from = r.first;
+                fits = len >= BNK_WG_HEADER + BNK_WG_TAG && (uint64_t)off + len <= a.ring_bytes;
+                const uint32_t body = len - (BNK_WG_HEADER + BNK_WG_TAG);
+                bytes = body <= kRoundBytes ? body + BNK_WG_TAG : kRoundBytes;
+            } else {
+                from = r.body;
+                fits = (uint64_t)off + BNK_WG_HEADER + len <= a.ring_bytes;
+                bytes = min(len, kRoundBytes);
+            }
+            if (fits) {
+                const uint32_t end = r.body + ((bytes + 15u) >> 4);
+                for (uint32_t q = lane; q < end; q += 32)
+                    if (q >= from) copy_async16(&stage[stage_at(q)], a.in + r.window + 16u * q);
             }
         }
-        __syncwarp();
-        uint32_t d[16];
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (is_chunk) v = stage[4u * (chunk - done) + c];
-            else if (is_tail && base + 16u * c < in_len) v = *reinterpret_cast<const uint4 *>(data + base + 16u * c);
-            d[4 * c + 0] = v.x; d[4 * c + 1] = v.y; d[4 * c + 2] = v.z; d[4 * c + 3] = v.w;
+        if ((!OPEN || !a.demux) && slot < a.max_slots && lane < 2)
+            copy_async16(&key_all[warp][buf][lane], a.keys + (size_t)slot * 8 + 4u * lane);
+        copy_async_commit();
+    };
+
+    uint32_t t = blockIdx.x * kWppWarps + warp, buf = 0;
+    Tile cur = load_tile(t);
+    __shared__ uint32_t slots[OPEN ? 1 : kRankMax];
+    if (!OPEN && a.send_counter) { // one tile of one packet per warp
+        for (uint32_t i = threadIdx.x; i < a.n; i += blockDim.x) slots[i] = a.slot[i];
+        __syncthreads();
+    }
+    if (t < tiles) fetch(__shfl_sync(0xffffffffu, cur.off, 0), __shfl_sync(0xffffffffu, cur.len, 0),
+                         __shfl_sync(0xffffffffu, cur.slot, 0), 0);
+    if (a.over_link) wait_for_kernel_in_front();
+    load_keypair(cur, t);
+    if (!OPEN && a.send_counter && t < tiles) {
+        const uint32_t mine = slots[t];
+        uint32_t before = 0, all = 0;
+        for (uint32_t base = 0; base < a.n; base += 32) {
+            const uint32_t same = __ballot_sync(0xffffffffu, base + lane < a.n && slots[base + lane] == mine);
+            all += __popc(same);
+            before += __popc(base + 32 <= t ? same : base > t ? 0u : same & ((1u << (t - base)) - 1u));
         }
-        __syncwarp(); // the pieces are read: the stage may take the output
-        uint32_t x[16];
-        chacha20_block(x, key, works ? chunk + 1u : 0u, dsc.n_lo, dsc.n_hi); // idle lanes and the carry lane: block 0
-        if (first) {
-            const int src = 30 - (int)F; // the carry lane holds block 0
-            const uint32_t k0 = __shfl_sync(0xffffffffu, x[0], src), k1 = __shfl_sync(0xffffffffu, x[1], src);
-            const uint32_t k2 = __shfl_sync(0xffffffffu, x[2], src), k3 = __shfl_sync(0xffffffffu, x[3], src);
-            r = p26_words(k0 & 0x0fffffffu, k1 & 0x0ffffffcu, k2 & 0x0ffffffcu, k3 & 0x0ffffffcu, 0u);
-#pragma unroll
-            for (int i = 0; i < 4; i++) pad[i] = __shfl_sync(0xffffffffu, x[4 + i], src);
-        }
-        if (works) {
-            const int in_left = (int)in_len - (int)base;
-            const int body_left = (int)body - (int)base;
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                uint32_t o[4];
-#pragma unroll
-                for (int w = 0; w < 4; w++) {
-                    const int k = 16 * c + 4 * w;
-                    const uint32_t in_w = keep_bytes(d[4 * c + w], in_left - k);
-                    o[w] = keep_bytes(in_w ^ x[4 * c + w], body_left - k);
-                    ct[4 * c + w] = OPEN ? in_w : o[w];
-                }
-                if (is_chunk) { // a whole chunk lies inside the body: out through the stage, in piece order
-                    stage[4u * (chunk - done) + c] = make_uint4(o[0], o[1], o[2], o[3]);
-                } else if (16 * c + 16 <= body_left) {
-                    *reinterpret_cast<uint4 *>(data + base + 16u * c) = make_uint4(o[0], o[1], o[2], o[3]);
-                } else if (16 * c < body_left) {
-                    uint8_t *dst = data + base + 16u * c;
-                    const int tail = body_left - 16 * c;
-#pragma unroll
-                    for (int k = 0; k < 15; k++)
-                        if (k < tail) dst[k] = (uint8_t)(o[k >> 2] >> (8 * (k & 3)));
-                }
+        if (lane == 0 && mine < a.max_slots) {
+            const uint64_t base = *(volatile uint64_t *)&a.send_counter[mine];
+            cur.ctr = saturating_counter(base, before);
+            __threadfence();
+            if (atomicAdd(&a.arrived[mine], 1u) + 1u == all) { // every packet of the slot has read it
+                a.send_counter[mine] = saturating_counter(base, all);
+                a.arrived[mine] = 0u;
             }
         }
-        __syncwarp();
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const uint32_t q = 32u * c + lane;
-            if (q < 4u * F) *reinterpret_cast<uint4 *>(data + round_base + 16u * q) = stage[q];
-        }
-        __syncwarp(); // before the next round writes the stage
-        // Horner over the lane's own four blocks (chunk lanes), or the state carried in (carry lane)
-        P26 V = p26_zero();
-        if (is_chunk) {
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-                V = p26_mul(p26_add(V, p26_words(ct[4 * c], ct[4 * c + 1], ct[4 * c + 2], ct[4 * c + 3], 1u)), r);
-        }
-        if (is_carry) V = state;
-        // fold lanes 0..30 (tree positions 1..31) with r^4, r^8, ..., r^64
-        P26 pw = p26_mul(r, r);
-        pw = p26_mul(pw, pw);
-#pragma unroll
-        for (int k = 0; k < 5; k++) {
-            P26 left = p26_shfl_up(V, 1 << k);
-            if (lane < (1u << k)) left = p26_zero();
-            const P26 t = p26_add(p26_mul(left, pw), V);
-            const uint32_t mask = (2u << k) - 1u;
-            if (((lane + 1u) & mask) == mask && lane != 31u) V = t;
-            if (k < 4) pw = p26_mul(pw, pw);
-        }
-        state = p26_shfl(V, 30);
-        done += F;
-        first = false;
-    } while (!last_round);
+    }
+    for (; t < tiles; t += step) {
+        const uint32_t in_tile = min(T, a.n - t * T);
+        Tile next = load_tile(t + step);
+        uint32_t res_len = 0, res_slot = 0, res_status = BNK_PKT_OK; // of the packet of this lane
+        bool has_counter = !OPEN && cur.slot < a.max_slots;
+        uint64_t res_ctr = cur.ctr;
+        for (uint32_t k = 0; k < in_tile; k++, buf ^= 1u) {
+            const uint32_t off = __shfl_sync(0xffffffffu, cur.off, k), len = __shfl_sync(0xffffffffu, cur.len, k);
+            uint32_t slot = __shfl_sync(0xffffffffu, cur.slot, k);
+            if (k + 1 < in_tile) {
+                fetch(__shfl_sync(0xffffffffu, cur.off, k + 1), __shfl_sync(0xffffffffu, cur.len, k + 1),
+                      __shfl_sync(0xffffffffu, cur.slot, k + 1), buf ^ 1u);
+                copy_async_wait<1>();
+            } else if (t + step < tiles) {
+                load_keypair(next, t + step);
+                fetch(__shfl_sync(0xffffffffu, next.off, 0), __shfl_sync(0xffffffffu, next.len, 0),
+                      __shfl_sync(0xffffffffu, next.slot, 0), buf ^ 1u);
+                copy_async_wait<1>();
+            } else {
+                copy_async_wait<0>();
+            }
+            __syncwarp();
+            uint4 *const stage = stage_all[warp][buf];
+            uint8_t *const stage_bytes = reinterpret_cast<uint8_t *>(stage);
+            Round rd(off, 0);
 
-    // lane 31: the blocks behind the last whole chunk, the length block, the tag
-    uint32_t verdict = 0; // open: 1 = tag mismatch
-    if (lane == 31u) {
-        P26 h = state;
-        const uint32_t nb = (tail_bytes + 15u) >> 4;
+            // ---- what the descriptor says (the same for all lanes) ----
+            uint8_t st = BNK_PKT_OK;
+            uint32_t body = 0, in_len = 0, n_lo = 0, n_hi = 0;
+            if (OPEN) {
+                const bool in_ring = (uint64_t)off + len <= a.ring_bytes, whole = in_ring && len >= BNK_WG_HEADER + BNK_WG_TAG;
+                uint4 hdr = make_uint4(0, 0, 0, 0);
+                if (!(off & 15u) && whole) hdr = stage[stage_at(rd.first)];
+                if (a.demux) {
+                    slot = 0; // descriptors refused below for other reasons
+                    if (!(off & 15u) && whole) slot = demux_index_warp(a.index_keys, a.index_vals, a.index_slots, hdr.y);
+                }
+                if ((off & 15u) || slot >= a.max_slots) st = slot == kSlotNoKeypair ? BNK_PKT_NO_KEYPAIR : BNK_PKT_BAD_DESC;
+                else if (!(a.demux ? a.valid[slot] : __shfl_sync(0xffffffffu, cur.valid, k))) st = BNK_PKT_NO_KEYPAIR;
+                else if (!in_ring) st = BNK_PKT_BAD_DESC;
+                else if (!whole) st = BNK_PKT_MALFORMED;
+                else {
+                    n_lo = hdr.z;
+                    n_hi = hdr.w;
+                    if (lane == k) {
+                        res_ctr = ((uint64_t)hdr.w << 32) | hdr.z;
+                        has_counter = true;
+                    }
+                    if (hdr.x != 4u) st = BNK_PKT_MALFORMED;
+                    body = in_len = len - (BNK_WG_HEADER + BNK_WG_TAG);
+                }
+            } else {
+                const uint64_t ctr = __shfl_sync(0xffffffffu, cur.ctr, k);
+                n_lo = (uint32_t)ctr;
+                n_hi = (uint32_t)(ctr >> 32);
+                body = wg_padded_len(len, a.mtu);
+                in_len = len;
+                if ((off & 15u) || slot >= a.max_slots) st = BNK_PKT_BAD_DESC;
+                else if (!__shfl_sync(0xffffffffu, cur.valid, k)) st = BNK_PKT_NO_KEYPAIR;
+                else if ((uint64_t)off + BNK_WG_HEADER + body + BNK_WG_TAG > a.ring_bytes || body < len) st = BNK_PKT_BAD_DESC;
+                else if (ctr >= BNK_REJECT_AFTER_MESSAGES) st = BNK_PKT_COUNTER_EXHAUSTED;
+            }
+            if (lane == k) {
+                res_slot = slot;
+                res_status = st;
+                res_len = 0;
+            }
+            FlowNote note;
+            if (NOTE && !(off & 15u) && (uint64_t)off + BNK_WG_HEADER + len <= a.ring_bytes) {
+                const uint32_t word = stage_word(stage, rd.body); // the IPv4 header and the ports lie in 64 bytes
+                Parsed p;
+                const uint32_t at = parse_ipv4_words(__shfl_sync(0xffffffffu, word, 0), __shfl_sync(0xffffffffu, word, 2),
+                                                     __shfl_sync(0xffffffffu, word, 3), __shfl_sync(0xffffffffu, word, 4), len, p);
+                const uint32_t ports = __shfl_sync(0xffffffffu, word, (at >> 2) & 15u);
+                if (at != kParseBad && lane == 0) {
+                    if (at) parse_ports(ports, p);
+                    note.begin(a.ft, p, a.now);
+                }
+            }
+            if (st != BNK_PKT_OK) { // the next packet's copies are in the other stage
+                if (NOTE) {
+                    note.place(a.ft);
+                    note.count(a.ft);
+                }
+                __syncwarp();
+                continue;
+            }
+
+            uint32_t key[8];
+            {
+                uint4 ka, kb;
+                if (OPEN && a.demux) {
+                    const uint4 *kp = reinterpret_cast<const uint4 *>(a.keys + (size_t)slot * 8);
+                    ka = kp[0];
+                    kb = kp[1];
+                } else {
+                    ka = key_all[warp][buf][0];
+                    kb = key_all[warp][buf][1];
+                }
+                key[0] = ka.x; key[1] = ka.y; key[2] = ka.z; key[3] = ka.w;
+                key[4] = kb.x; key[5] = kb.y; key[6] = kb.z; key[7] = kb.w;
+            }
+            const uint32_t remote = OPEN ? 0u : __shfl_sync(0xffffffffu, cur.remote, k);
+            P26 r = p26_zero(), state = p26_zero();
+            uint32_t pad[4] = {0, 0, 0, 0}, tag[4];
+            bool forged = false;
+            for (uint32_t rnd = 0;; rnd++) {
+                const uint32_t done = rnd * kRoundBytes;
+                const uint32_t rb = min(body - done, kRoundBytes); // body bytes of this round
+                const bool last = body - done <= kRoundBytes;
+                if (rnd) { // longer packets: the further rounds are fetched when their turn comes
+                    rd = Round(off, rnd);
+                    __syncwarp(); // the stage is read out
+                    const uint32_t bytes = OPEN ? rb + (last ? BNK_WG_TAG : 0u) : (in_len > done ? min(in_len - done, kRoundBytes) : 0u);
+                    const uint32_t end = rd.body + ((bytes + 15u) >> 4);
+                    for (uint32_t q = lane; q < end; q += 32)
+                        if (q >= rd.body) stage[stage_at(q)] = *reinterpret_cast<const uint4 *>(a.in + rd.window + 16u * q);
+                    __syncwarp();
+                }
+                // ---- keystream and cipher: lane 0 block 0, lane j the j-th block of the round ----
+                uint32_t x[16];
+                chacha20_block(x, key, lane == 0 ? 0u : rnd * kRoundBlocks + lane, n_lo, n_hi);
+                if (rnd == 0) {
+                    const uint32_t k0 = __shfl_sync(0xffffffffu, x[0], 0), k1 = __shfl_sync(0xffffffffu, x[1], 0);
+                    const uint32_t k2 = __shfl_sync(0xffffffffu, x[2], 0), k3 = __shfl_sync(0xffffffffu, x[3], 0);
+                    r = p26_words(k0 & 0x0fffffffu, k1 & 0x0ffffffcu, k2 & 0x0ffffffcu, k3 & 0x0ffffffcu, 0u);
 #pragma unroll
-        for (int c = 0; c < 4; c++)
-            if ((uint32_t)c < nb) h = p26_mul(p26_add(h, p26_words(ct[4 * c], ct[4 * c + 1], ct[4 * c + 2], ct[4 * c + 3], 1u)), r);
-        h = p26_mul(p26_add(h, p26_words(0u, 0u, body, 0u, 1u)), r); // le64(0) | le64(body)
-        uint32_t tag[4];
-        p26_finish(h, pad, tag);
-        uint8_t *tagp = data + body;
-        if (!OPEN) {
+                    for (int i = 0; i < 4; i++) pad[i] = __shfl_sync(0xffffffffu, x[4 + i], 0);
+                }
+                const bool works = lane != 0 && (lane - 1u) * 64u < rb;
+                if (works) {
+                    const int in_left = (int)(in_len > done ? min(in_len - done, kRoundBytes) : 0u) - (int)(lane - 1u) * 64;
+                    const int body_left = (int)rb - (int)(lane - 1u) * 64;
 #pragma unroll
-            for (int w = 0; w < 4; w++)
+                    for (int c = 0; c < 4; c++) {
+                        const uint4 v = stage[stage_at(rd.body + 4u * (lane - 1u) + c)];
+                        const uint32_t d[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int k = 0; k < 4; k++) tagp[4 * w + k] = (uint8_t)(tag[w] >> (8 * k));
-        } else {
-            uint32_t diff = 0;
+                        for (int w = 0; w < 4; w++) {
+                            const int at = 16 * c + 4 * w;
+                            x[4 * c + w] = keep_bytes(keep_bytes(d[w], in_left - at) ^ x[4 * c + w], body_left - at);
+                        }
+                    }
+                    if (!OPEN) {
 #pragma unroll
-            for (int w = 0; w < 4; w++)
+                        for (int c = 0; c < 4; c++)
+                            stage[stage_at(rd.body + 4u * (lane - 1u) + c)] =
+                                make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+                    }
+                }
+                if (NOTE && rnd == 0) note.place(a.ft);
+                __syncwarp();
+                // ---- Poly1305 over the ciphertext in the stage ----
+                const uint32_t data_blocks = (rb + 15u) >> 4, blocks = data_blocks + (last ? 1u : 0u);
+                P26 V = p26_zero();
+                {
+                    const int b0 = (int)(4u * lane + blocks) - 128; // the lane's first block; negative: none
+                    if (b0 <= 0 && b0 > -4) V = state;              // (zero in round 0)
 #pragma unroll
-                for (int k = 0; k < 4; k++) diff |= (uint32_t)(tagp[4 * w + k] ^ (uint8_t)(tag[w] >> (8 * k)));
-            verdict = diff != 0;
+                    for (int s = 0; s < 4; s++) {
+                        const int blk = b0 + s;
+                        if (blk < 0) continue;
+                        uint4 m = make_uint4(0u, 0u, body, 0u); // le64(0) | le64(body)
+                        if ((uint32_t)blk < data_blocks) {
+                            m = stage[stage_at(rd.body + blk)];
+                            const int left = (int)rb - 16 * blk;
+                            if (OPEN && left < 16) {
+                                m.x = keep_bytes(m.x, left);
+                                m.y = keep_bytes(m.y, left - 4);
+                                m.z = keep_bytes(m.z, left - 8);
+                                m.w = keep_bytes(m.w, left - 12);
+                            }
+                        }
+                        V = p26_mul(p26_add(V, p26_words(m.x, m.y, m.z, m.w, 1u)), r);
+                    }
+                }
+                P26 pw = p26_mul(r, r);
+                pw = p26_mul(pw, pw);
+                const uint32_t lanes_used = (blocks + 3u) >> 2;
+                for (uint32_t span = 1; span < lanes_used; span <<= 1) {
+                    const P26 sum = p26_add(p26_mul(p26_shfl_up(V, span), pw), V);
+                    if (((lane + 1u) & (2u * span - 1u)) == 0) V = sum;
+                    pw = p26_mul(pw, pw);
+                }
+                state = p26_shfl(V, 31);
+                // ---- tag, output ----
+                if (last) {
+                    p26_finish(state, pad, tag);
+                    const uint32_t tw = (lane & 8u) ? ((lane & 4u) ? tag[3] : tag[2]) : ((lane & 4u) ? tag[1] : tag[0]);
+                    const uint8_t tb = (uint8_t)(tw >> (8u * (lane & 3u)));
+                    const uint32_t at = 16u * rd.body + rb + lane;
+                    uint8_t *const p = stage_bytes + 16u * stage_at(at >> 4) + (at & 15u);
+                    if (OPEN) forged = __any_sync(0xffffffffu, lane < 16u && *p != tb);
+                    else if (lane < 16u) *p = tb;
+                }
+                if (OPEN) {
+                    __syncwarp(); // ciphertext and tag are read
+                    if (works) {
+#pragma unroll
+                        for (int c = 0; c < 4; c++)
+                            stage[stage_at(rd.body + 4u * (lane - 1u) + c)] =
+                                forged ? make_uint4(0, 0, 0, 0) : make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+                    }
+                } else if (rnd == 0 && lane == 0) {
+                    stage[stage_at(rd.first)] = make_uint4(4u, remote, n_lo, n_hi);
+                }
+                __syncwarp();
+                if (OPEN && a.inner && rnd == 0 && !forged) {
+                    const uint32_t word = stage_word(stage, rd.body);
+                    const uint32_t w0 = __shfl_sync(0xffffffffu, word, 0), w3 = __shfl_sync(0xffffffffu, word, 3);
+                    const uint32_t total = ((w0 >> 8) & 0xff00u) | (w0 >> 24); // bytes 2,3 big-endian
+                    const bool is_whole = body >= 20 && ((w0 & 0xffu) >> 4) == 4u && total >= 20 && total <= body;
+                    Parsed p{};
+                    const uint32_t at = parse_ipv4_words(w0, __shfl_sync(0xffffffffu, word, 2), w3, __shfl_sync(0xffffffffu, word, 4),
+                                                         a.inner_cut && is_whole ? total : body, p);
+                    const uint32_t ports = __shfl_sync(0xffffffffu, word, (at >> 2) & 15u);
+                    if (at != kParseBad && at) parse_ports(ports, p);
+                    if (lane == 0)
+                        a.inner[(size_t)t * T + k] =
+                            make_uint4(__byte_perm(w3, 0, 0x0123), (uint32_t)p.sport << 16 | p.dport,
+                                       p.proto | (at != kParseBad ? kInnerParses : 0u) | (is_whole ? kInnerWhole : 0u), total);
+                }
+                const uint32_t out_bytes = OPEN ? rb : rb + (last ? BNK_WG_TAG : 0u);
+                const uint32_t whole_end = rd.body + (out_bytes >> 4), rest = out_bytes & 15u;
+                for (uint32_t q = lane; q < whole_end; q += 32) {
+                    if (q < (OPEN ? rd.body : rd.first)) continue;
+                    const uint4 v = stage[stage_at(q)];
+                    *reinterpret_cast<uint4 *>(a.out + rd.window + 16u * q) = v;
+                    if (a.out2) *reinterpret_cast<uint4 *>(a.out2 + rd.window + 16u * q) = v;
+                }
+                if (lane < rest) {
+                    const uint8_t v = stage_bytes[16u * stage_at(whole_end) + lane];
+                    a.out[rd.window + 16u * whole_end + lane] = v;
+                    if (a.out2) a.out2[rd.window + 16u * whole_end + lane] = v;
+                }
+                if (last) break;
+            }
+            if (OPEN && forged && body > kRoundBytes) { // the earlier rounds' plaintext is out already: wipe it
+                uint8_t *const data = a.out + (size_t)off + BNK_WG_HEADER, *const data2 = a.out2 + (size_t)off + BNK_WG_HEADER;
+                const uint32_t end = body - (body - 1u) % kRoundBytes - 1u; // what lies in the rounds before the last
+                __syncwarp();
+                for (uint32_t q = lane * 16u; q < end; q += 512u) {
+                    *reinterpret_cast<uint4 *>(data + q) = make_uint4(0, 0, 0, 0);
+                    if (a.out2) *reinterpret_cast<uint4 *>(data2 + q) = make_uint4(0, 0, 0, 0);
+                }
+            }
+            if (lane == k) {
+                res_status = OPEN ? (forged ? BNK_PKT_AUTH_FAIL : body ? BNK_PKT_OK : BNK_PKT_KEEPALIVE) : BNK_PKT_OK;
+                res_len = OPEN ? (forged ? 0u : body) : BNK_WG_HEADER + body + BNK_WG_TAG;
+            }
+            if (NOTE) note.count(a.ft);
+            __syncwarp(); // the stage may be filled again
         }
+        const uint32_t i = t * T + lane;
+        if (lane < in_tile) {
+#pragma unroll
+            for (int d = 0; d < 2; d++) {
+                const AeadResults &o = a.res[d];
+                if (o.status) o.status[i] = (uint8_t)res_status;
+                if (o.out_len) o.out_len[i] = res_len;
+                if (o.counter && has_counter) o.counter[i] = res_ctr;
+                if (o.slot) o.slot[i] = res_slot;
+            }
+        }
+        cur = next;
     }
-    if (!OPEN) {
-        if (lane == 0) {
-            *reinterpret_cast<uint4 *>(a.ring + dsc.off) = make_uint4(4u, a.remote_index[dsc.slot], dsc.n_lo, dsc.n_hi);
-            a.status[pkt] = BNK_PKT_OK;
-            a.out_len[pkt] = BNK_WG_HEADER + body + BNK_WG_TAG;
-        }
-    } else {
-        verdict = __shfl_sync(0xffffffffu, verdict, 31);
-        if (verdict) { // forged or damaged: wipe what the fused pass wrote
-            for (uint32_t k = lane * 16u; k + 16u <= body; k += 512u) *reinterpret_cast<uint4 *>(data + k) = make_uint4(0, 0, 0, 0);
-            if (lane == 0)
-                for (uint32_t k = body & ~15u; k < body; k++) data[k] = 0;
-        }
-        if (lane == 0) {
-            a.status[pkt] = verdict ? BNK_PKT_AUTH_FAIL : (body ? BNK_PKT_OK : BNK_PKT_KEEPALIVE);
-            a.out_len[pkt] = verdict ? 0u : body;
-        }
-    }
+    signal_done(a.done, [&] {
+        if (NOTE && a.flow_report) flow_report(flow_ctl(a.ft), a.flow_report);
+    });
 }
 
 // Below this many packets one-packet-per-thread leaves most of the GPU idle and its run time is that of one thread
@@ -725,13 +948,30 @@ __global__ void __launch_bounds__(128) aead_wpp_kernel(const AeadArgs a) {
 #define BNK_WPP_MAX_PACKETS 6144u
 #endif
 
+// Tiles and grid of a warp-per-packet launch.  Rings in device memory (n <= BNK_WPP_MAX_PACKETS): a warp per packet.
+// Rings in host memory: the link is the bound, kHostCtas CTAs keep it busy and more make it slower (see the kernel);
+// from 8 packets a warp on, warps take tiles of 8, whose descriptors are whole 32-byte reads.
+#ifndef BNK_HOST_CTAS
+#define BNK_HOST_CTAS 128u
+#endif
+void wpp_grid(AeadArgs &a, uint32_t &ctas) {
+    const uint32_t all = (a.n + kWppWarps - 1) / kWppWarps;
+    a.tile = 1;
+    ctas = all;
+    if (!a.over_link || all <= BNK_HOST_CTAS) return;
+    ctas = BNK_HOST_CTAS;
+    while (a.tile < 8 && (uint64_t)a.n > (uint64_t)ctas * kWppWarps * a.tile * 4u) a.tile *= 2;
+}
+
 template <bool OPEN>
-cudaError_t launch_aead(const AeadArgs &a, cudaStream_t s, bnk_ctx *ctx) {
+cudaError_t launch_aead(AeadArgs a, cudaStream_t s, bnk_ctx *ctx) {
     if (a.n == 0) return cudaSuccess;
-    const bool wpp = ctx->aead_mode == 2 || (ctx->aead_mode == 0 && a.n <= BNK_WPP_MAX_PACKETS);
+    const bool wpp = a.over_link || ctx->aead_mode == 2 || (ctx->aead_mode == 0 && a.n <= BNK_WPP_MAX_PACKETS);
     if (wpp) {
-        const uint32_t ctas = (a.n + 3) / 4; // 4 warps = 4 packets per CTA
-        cudaError_t e = launch_after_kernel(aead_wpp_kernel<OPEN>, dim3(ctas), dim3(128), s, a);
+        uint32_t ctas;
+        wpp_grid(a, ctas);
+        auto *const kernel = !OPEN && a.note ? aead_wpp_kernel<OPEN, !OPEN> : aead_wpp_kernel<OPEN, false>;
+        cudaError_t e = launch_after_kernel(kernel, dim3(ctas), dim3(32 * kWppWarps), s, a);
         if (e != cudaSuccess) return e;
     } else {
         // one CTA per 128 packets; the hardware hands CTAs to SMs as slots free up, which measured faster

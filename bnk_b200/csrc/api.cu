@@ -8,7 +8,7 @@
 #include <new>
 #include <thread>
 
-#include "bnk_internal.cuh"
+#include "filter_device.cuh"
 
 namespace {
 
@@ -33,6 +33,14 @@ int fail(bnk_ctx *ctx, int code, const char *what, cudaError_t e = cudaSuccess) 
         cudaError_t _e = (call);                                       \
         if (_e != cudaSuccess) return fail((ctx), BNK_ECUDA, #call, _e); \
     } while (0)
+
+inline void cpu_relax() {
+#if defined(__x86_64__) || defined(__i386__)
+    __builtin_ia32_pause();
+#else
+    std::this_thread::yield();
+#endif
+}
 
 bool is_pow2(uint64_t v) { return v && !(v & (v - 1)); }
 
@@ -70,9 +78,25 @@ int begin_submit(bnk_batch *b, uint32_t npkts, bool touches_host = true) {
 struct SubmitScope {
     bnk_batch *b;
     std::shared_lock<std::shared_mutex> tables; // see bnk_ctx::submit_mu
-    explicit SubmitScope(bnk_batch *batch) : b(batch), tables(batch->ctx->submit_mu) { b->stats_pending = false; }
-    ~SubmitScope() { b->in_flight = true; }
+    explicit SubmitScope(bnk_batch *batch) : b(batch), tables(batch->ctx->submit_mu) { b->stats_pending = b->done_watched = false; }
+    ~SubmitScope() {
+        b->in_flight = true;
+        if (!b->counted) b->ctx->in_flight.fetch_add(1, std::memory_order_relaxed);
+        b->counted = true;
+    }
 };
+void submit_over(bnk_batch *b) { // waited for, or going away
+    b->in_flight = false;
+    if (b->counted) b->ctx->in_flight.fetch_sub(1, std::memory_order_relaxed);
+    b->counted = false;
+    if (b->direct_counted) b->ctx->direct_in_flight.fetch_sub(b->direct_counted, std::memory_order_relaxed);
+    b->direct_counted = 0;
+}
+// For the kernel that is the submit's last piece of work: bnk_wait will watch for it.
+Done watch_for(bnk_batch *b) {
+    b->done_watched = true;
+    return Done{b->d_ticket, b->h_done, ++b->done_seq};
+}
 
 // The counters of BNK_F_STATS: one launch behind the submit's last kernel, totals straight into pinned memory.
 cudaError_t tally_if_asked(bnk_batch *b, uint32_t npkts, uint32_t flags, cudaStream_t s) {
@@ -81,41 +105,32 @@ cudaError_t tally_if_asked(bnk_batch *b, uint32_t npkts, uint32_t flags, cudaStr
     return launch_tally(b, npkts, s);
 }
 
-// Small batches skip the copy engines: the kernels read the caller's pinned ring and descriptors through the
-// bus and write the results straight back (pinned memory has the same address on the device).  For a batch of
-// a few hundred KB the four copies and the engine hand-overs either side of the kernels cost more than the
-// kernels themselves.  While a HostAlias lives, the launchers see the host arrays where the device copies
-// would be; the device copies fall behind (dev_stale) until the next full upload.
-// The seal/open kernel of such a batch (one warp per packet) moves its data in 512-byte stretches per load and store
-// instruction; with 16-byte pieces 64 bytes apart every piece was a bus transaction of its own, reads came at
-// ~10 GB/s and the mode stopped paying at a hundred KB and did not scale over threads.  Now, measured on 128 full-size
-// packets: 35 us against 38 per seal, and eight / sixteen host threads with batches of their own move 140 / 144
-// Gbit/s against 118 / 117 through the copy engines (256 packets: 154 / 170 against 155 / 137).  Beyond 256 packets
-// the copy engines win again (512: 184 against 60), hence the two limits.  Serving only the descriptors this way and
-// the ring by copy was measured too and gained nothing.
-constexpr uint32_t kHostDirectMaxPkts = 256;
-// With many such batches in flight at once the mode can collapse (sixteen threads with four 128-packet batches each:
-// 51 Gbit/s in most runs, against 140-150 with two each or with eight threads), so at most kHostDirectInFlight
-// batches of a context run this way at a time and the next ones are copied, which does not degrade.  With the cap,
-// ten runs each: 8 threads x 2 batches median 140 Gbit/s (copies: 117), 16 x 2 152 (115), 16 x 4 127 (118); on a
-// shared host both ways show slow runs now and then.
-constexpr int kHostDirectInFlight = 16;
+// A batch whose results go back to the host need not be copied at all: the kernels read the caller's pinned ring and
+// descriptors through the host link and write the results straight back (pinned memory has the same address on the
+// device).  Copies either side of the kernels run one after the other, each at ~55 GB/s and ~8 us before it moves
+// anything; a kernel that works on the pinned ring moves both directions at once.  While a HostAlias lives, the
+// launchers see the host arrays where the device copies would be; the device copies fall behind (dev_stale) until the
+// next full upload.
+// Measured with plain copies through SMs, 1440-byte pieces read and written in place, against upload, kernel and
+// download in a row: 190 KB 17 us against 33, 1.6 MB 56 against 82, 6.4 MB 177 against 253, 24 MB 613 against 916,
+// 190 MB 4.74 ms against 7.0.  Chunks of one batch over three streams, so that the copy engines run both ways, take
+// 77 us at 1.6 MB, 234 at 6.4 MB, 680 at 24 MB and 4.55 ms at 190 MB: only far up they are the faster form.
+// With several batches in flight the engines overlap the batches' copies with each other (48 GB/s each way together),
+// and many kernels on the link at once slow each other down, so a batch runs this way only if nothing else is in
+// flight, or if all that run this way together stay below kDirectTogether bytes and kDirectBatches batches.
+constexpr uint64_t kDirectTogether = 6ull << 20;
+constexpr int kDirectBatches = 16;
 bool host_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, uint64_t ext) {
     bnk_ctx *ctx = b->ctx;
-    if (!(ctx->host_direct_bytes != 0 && npkts != 0 && npkts <= kHostDirectMaxPkts &&
-          !(flags & (BNK_F_NO_H2D | BNK_F_NO_D2H | BNK_F_USE_OUT_LEN)) && ext <= ctx->host_direct_bytes))
+    if (ctx->host_direct_bytes == 0 || npkts == 0 || (flags & (BNK_F_NO_H2D | BNK_F_NO_D2H | BNK_F_USE_OUT_LEN)) ||
+        ext > ctx->host_direct_bytes)
         return false;
-    if (b->direct_counted) return true; // a second submit on a batch that is already counted
-    if (ctx->direct_in_flight.load(std::memory_order_relaxed) >= kHostDirectInFlight) return false;
-    ctx->direct_in_flight.fetch_add(1, std::memory_order_relaxed);
-    b->direct_counted = true;
+    const uint64_t together = ctx->direct_in_flight.load(std::memory_order_relaxed) - b->direct_counted;
+    const int others = ctx->in_flight.load(std::memory_order_relaxed) - (b->counted ? 1 : 0);
+    if (others > 0 && (together + ext > kDirectTogether || others >= kDirectBatches)) return false;
+    ctx->direct_in_flight.fetch_add(ext - b->direct_counted, std::memory_order_relaxed);
+    b->direct_counted = ext;
     return true;
-}
-void direct_done(bnk_batch *b) {
-    if (b->direct_counted) {
-        b->direct_counted = false;
-        b->ctx->direct_in_flight.fetch_sub(1, std::memory_order_relaxed);
-    }
 }
 struct HostAlias {
     bnk_batch *b;
@@ -165,13 +180,12 @@ cudaError_t desc_copy(bnk_batch *b, size_t n, int first, int last, bool to_devic
 AeadArgs aead_args(bnk_batch *b, uint32_t n, bool open, const uint32_t *order) {
     bnk_ctx *ctx = b->ctx;
     AeadArgs a{};
-    a.ring = b->dev.ring;
+    a.in = a.out = b->dev.ring;
     a.off = b->dev.off;
     a.len = b->dev.len;
     a.slot = b->dev.slot;
     a.counter = b->dev.counter;
-    a.out_len = b->dev.out_len;
-    a.status = b->dev.status;
+    a.res[0] = AeadResults{b->dev.counter, b->dev.out_len, b->dev.status, nullptr};
     a.keys = open ? ctx->kt.recv_keys : ctx->kt.send_keys;
     a.remote_index = ctx->kt.remote_index;
     a.valid = ctx->kt.valid;
@@ -242,8 +256,7 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     ctx->aead_mode = 0;
     if (const char *m = getenv("BNK_AEAD_KERNEL")) // tuning and test aid: tpp | wpp
         ctx->aead_mode = !strcmp(m, "tpp") ? 1 : (!strcmp(m, "wpp") ? 2 : 0);
-    ctx->host_direct_bytes = 384u << 10; // 256 slots of 1456 bytes and their headroom
-
+    ctx->host_direct_bytes = 512u << 20;
     if (const char *m = getenv("BNK_HOST_DIRECT_BYTES")) // largest ring extent served without copies; 0 = never
         ctx->host_direct_bytes = strtoull(m, nullptr, 0);
     if (!prop.unifiedAddressing || !prop.canMapHostMemory) ctx->host_direct_bytes = 0; // pinned memory must have one address
@@ -266,6 +279,7 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     if ((e = dev_alloc_zero(&ctx->kt.recv_keys, k * 8)) != cudaSuccess) return bail("recv_keys", e);
     if ((e = dev_alloc_zero(&ctx->kt.remote_index, k)) != cudaSuccess) return bail("remote_index", e);
     if ((e = dev_alloc_zero(&ctx->kt.send_counter, k)) != cudaSuccess) return bail("send_counter", e);
+    if ((e = dev_alloc_zero(&ctx->kt.arrived, k)) != cudaSuccess) return bail("arrived", e);
     if ((e = dev_alloc_zero(&ctx->kt.replay_last, k)) != cudaSuccess) return bail("replay_last", e);
     if ((e = dev_alloc_zero(&ctx->kt.replay_next, k)) != cudaSuccess) return bail("replay_next", e);
     if ((e = dev_alloc_zero(&ctx->kt.replay_ring, k * cfg->replay_ring_blocks)) != cudaSuccess) return bail("replay_ring", e);
@@ -284,6 +298,7 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     ctx->kt.addr_slots = islots;
     ctx->addr_host.assign(islots, KeypairTables::AddrEntry{});
     if ((e = dev_alloc_zero(&ctx->kt.addr_tab, (size_t)islots)) != cudaSuccess) return bail("addr_tab", e);
+    if ((e = group_kernels_init()) != cudaSuccess) return bail("kernel attributes", e);
     if ((e = filter_tables_alloc(ctx)) != cudaSuccess) return bail("filter tables", e);
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) return bail("sync", e);
     *out = ctx;
@@ -298,6 +313,7 @@ int bnk_ctx_destroy(bnk_ctx *ctx) {
     cudaFree(ctx->kt.recv_keys);
     cudaFree(ctx->kt.remote_index);
     cudaFree(ctx->kt.send_counter);
+    cudaFree(ctx->kt.arrived);
     cudaFree(ctx->kt.replay_last);
     cudaFree(ctx->kt.replay_next);
     cudaFree(ctx->kt.replay_ring);
@@ -627,7 +643,11 @@ int bnk_table_stats_get(bnk_ctx *ctx, bnk_table_stats *out) {
 int bnk_batch_destroy(bnk_batch *b) {
     if (!b) return BNK_EINVAL;
     cudaSetDevice(b->ctx->device);
-    direct_done(b);
+    submit_over(b);
+    if (b->flow_in_flight) {
+        std::lock_guard<std::mutex> g(b->ctx->flow_mu);
+        b->ctx->flow_in_flight--;
+    }
     {
         std::unique_lock<std::shared_mutex> tables(b->ctx->submit_mu); // not while table maintenance walks the registry
         std::lock_guard<std::mutex> g(b->ctx->mu);
@@ -646,6 +666,8 @@ int bnk_batch_destroy(bnk_batch *b) {
     cudaFreeHost(b->h_stats);
     cudaFree(b->d_stats);
     cudaFreeHost(b->h_gso);
+    cudaFreeHost(b->h_done);
+    cudaFree(b->d_ticket);
     DeviceBatch &d = b->dev;
     cudaFree(d.src_addr);
     cudaFree(d.order);
@@ -659,6 +681,7 @@ int bnk_batch_destroy(bnk_batch *b) {
     cudaFree(d.replay_tile_carry);
     cudaFree(d.hist);
     cudaFree(d.len_order);
+    cudaFree(d.inner);
     cudaFree(d.counters32);
     cudaFree(d.gso);
     if (b->k_begin) cudaEventDestroy(b->k_begin);
@@ -720,6 +743,7 @@ int bnk_batch_create(bnk_ctx *ctx, uint32_t max_pkts, uint64_t ring_bytes, bnk_b
     H((void **)&b->h_flow, sizeof(FlowReport));
     H((void **)&b->h_stats, sizeof(bnk_batch_stats));
     H((void **)&b->h_gso, n * sizeof(bnk_gso_super));
+    H((void **)&b->h_done, 128);
     b->host.ring_bytes = ring_bytes;
     b->host.max_pkts = max_pkts;
     DeviceBatch &d = b->dev;
@@ -745,8 +769,10 @@ int bnk_batch_create(bnk_ctx *ctx, uint32_t max_pkts, uint64_t ring_bytes, bnk_b
     D((void **)&d.replay_tile_carry, (size_t)replay_scan_tiles(max_pkts) * 8);
     D((void **)&d.hist, (size_t)512 * group_sort_chunks(max_pkts) * 4); // histogram columns + one row of totals
     D((void **)&d.len_order, n * 4);
+    D((void **)&d.inner, n * sizeof(uint4));
     D((void **)&d.counters32, 2048 * 4);
     D((void **)&d.gso, n * sizeof(bnk_gso_super));
+    D((void **)&b->d_ticket, 128);
     D((void **)&b->d_stats, 20 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->stream, cudaStreamNonBlocking, ctx->prio_high);
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->aux_stream, cudaStreamNonBlocking, ctx->prio_high);
@@ -814,6 +840,62 @@ int bnk_batch_download(bnk_batch *b, uint32_t npkts) {
     return BNK_SUCCESS;
 }
 
+// A seal that works on the pinned ring and descriptors: one launch up to kRankMax packets, else one more in front of
+// it for the counters, and one behind it when expired flows may have to be swept.
+static int seal_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_unix_ns) {
+    bnk_ctx *ctx = b->ctx;
+    cudaStream_t s = b->stream;
+    const bool timed = (flags & BNK_F_TIMED) != 0, stats = (flags & BNK_F_STATS) != 0;
+    const bnk_batch_view &h = b->host;
+    b->dev_stale = true;
+    if (b->order_wait) CK(ctx, cudaStreamWaitEvent(s, b->order_wait, 0));
+    if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
+    AeadArgs a = aead_args(b, npkts, false, nullptr);
+    a.over_link = true;
+    a.in = a.out = h.ring;
+    a.off = h.off;
+    a.len = h.len;
+    a.slot = h.slot;
+    a.counter = h.counter;
+    a.res[0] = AeadResults{nullptr, h.out_len, h.status, nullptr};
+    if (stats) a.res[1] = AeadResults{nullptr, b->dev.out_len, b->dev.status, nullptr};
+    if (flags & BNK_F_ASSIGN_COUNTERS) {
+        a.res[0].counter = h.counter;
+        if (npkts <= kRankMax) {
+            a.send_counter = ctx->kt.send_counter;
+            a.arrived = ctx->kt.arrived;
+        } else {
+            a.counter = b->dev.counter;
+            CK(ctx, launch_assign_counters(b, npkts, h.slot, b->dev.counter, s));
+        }
+    }
+    const bool note = (flags & BNK_F_NOTE_OUTBOUND) && ctx->ft.enforce && ctx->ft.flow_capacity; // filter.go:192-194
+    const bool sweep = note && flow_note_begins(b, npkts, now_unix_ns);
+    const Done done = stats ? Done{} : watch_for(b);
+    if (note) {
+        a.note = true;
+        a.now = now_unix_ns;
+        a.ft = ctx->ft;
+    }
+    if (!sweep) {
+        a.done = done;
+        if (note && done.flag) {
+            a.flow_report = b->h_flow;
+            b->flow_reported = true;
+        }
+    }
+    if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
+    CK(ctx, launch_seal(a, s, ctx));
+    if (timed) CK(ctx, cudaEventRecord(b->a_end, s));
+    if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, done, s));
+    else if (note && !done.flag) CK(ctx, launch_flow_report(b, s));
+    if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
+    b->kernel_timed = b->aead_timed = timed;
+    CK(ctx, tally_if_asked(b, npkts, flags, s));
+    if (b->order_record) CK(ctx, cudaEventRecord(b->order_record, s));
+    return BNK_SUCCESS;
+}
+
 int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_unix_ns) {
     const bool device_only = (flags & BNK_F_NO_H2D) && (flags & BNK_F_NO_D2H);
     int rc = begin_submit(b, npkts, !device_only);
@@ -827,9 +909,8 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     // header room + payload + padding (< 16) + tag
     const bool refresh = b->dev_stale; // the device copies are behind the host arrays: upload whatever the flags say
     const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, 16 + 16 + 16);
-    const bool direct = host_direct(b, npkts, flags, ext);
-    HostAlias alias(b, direct);
-    if (!direct && (!(flags & BNK_F_NO_H2D) || refresh) && n) {
+    if (ctx->aead_mode != 1 && host_direct(b, npkts, flags, ext)) return seal_direct(b, npkts, flags, now_unix_ns);
+    if ((!(flags & BNK_F_NO_H2D) || refresh) && n) {
         if (b->joint_copy) {
             CK(ctx, cudaMemcpyAsync(b->d_desc, b->h_desc, b->desc_room + ext, cudaMemcpyHostToDevice, s));
         } else {
@@ -840,9 +921,11 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     }
     if (b->order_wait) CK(ctx, cudaStreamWaitEvent(s, b->order_wait, 0));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
-    if (flags & BNK_F_NOTE_OUTBOUND) {
+    if ((flags & BNK_F_NOTE_OUTBOUND) && n && ctx->ft.enforce && ctx->ft.flow_capacity) { // filter.go:192-194
+        const bool sweep = flow_note_begins(b, npkts, now_unix_ns);
         CK(ctx, launch_filter_note(b, npkts, now_unix_ns, s));
-        CK(ctx, launch_flow_report(b, s));
+        if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, Done{}, s));
+        else CK(ctx, launch_flow_report(b, s));
     }
     const uint32_t *order = nullptr;
     const bool side_order = (flags & BNK_F_SORT_BY_LENGTH) && (flags & BNK_F_ASSIGN_COUNTERS) && npkts > 4096;
@@ -853,13 +936,15 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
         CK(ctx, cudaEventRecord(b->ev_join, b->aux_stream));
         order = b->dev.len_order;
     }
-    if (flags & BNK_F_ASSIGN_COUNTERS) CK(ctx, launch_assign_counters(b, npkts, s));
+    if (flags & BNK_F_ASSIGN_COUNTERS) CK(ctx, launch_assign_counters(b, npkts, b->dev.slot, b->dev.counter, s));
     if (side_order) {
         CK(ctx, cudaStreamWaitEvent(s, b->ev_join, 0));
     } else if (flags & BNK_F_SORT_BY_LENGTH) {
         CK(ctx, launch_length_order(b, npkts, b->dev.len, false, s));
         order = b->dev.len_order;
     }
+    AeadArgs a = aead_args(b, npkts, false, order);
+    a.res[0].counter = nullptr; // in place already
     const bool side = b->aead_stream && npkts >= ctx->aead_side_stream_from;
     cudaStream_t as = side ? b->aead_stream : s;
     if (side) {
@@ -867,7 +952,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
         CK(ctx, cudaStreamWaitEvent(as, b->ev_aead_go, 0));
     }
     if (timed) CK(ctx, cudaEventRecord(b->a_begin, as));
-    CK(ctx, launch_seal(aead_args(b, npkts, false, order), as, ctx));
+    CK(ctx, launch_seal(a, as, ctx));
     if (timed) CK(ctx, cudaEventRecord(b->a_end, as));
     if (side) {
         CK(ctx, cudaEventRecord(b->ev_aead_done, as));
@@ -878,7 +963,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     b->aead_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
     if (b->order_record) CK(ctx, cudaEventRecord(b->order_record, s));
-    if (!direct && !(flags & BNK_F_NO_D2H) && n) {
+    if (!(flags & BNK_F_NO_D2H) && n) {
         if (b->joint_copy) {
             CK(ctx, cudaMemcpyAsync(b->h_desc, b->d_desc, b->desc_room + ext, cudaMemcpyDeviceToHost, s));
         } else {
@@ -886,6 +971,79 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
             CK(ctx, desc_copy(b, n, D_COUNTER, D_STATUS, false, s));
         }
     }
+    return BNK_SUCCESS;
+}
+
+// An open that works on the pinned ring and descriptors.  What has to wait for the replay window (statuses, lengths)
+// stays on the device until then, with the packets' inner headers, so that no later kernel goes back to the ring.
+static int open_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_unix_ns) {
+    bnk_ctx *ctx = b->ctx;
+    cudaStream_t s = b->stream;
+    const bool timed = (flags & BNK_F_TIMED) != 0, stats = (flags & BNK_F_STATS) != 0;
+    const bool replay = (flags & BNK_F_REPLAY) != 0, checks = (flags & (BNK_F_INNER_CHECK | BNK_F_CHECK_INBOUND)) != 0;
+    const bnk_batch_view &h = b->host;
+    b->dev_stale = true;
+    if (b->order_wait) CK(ctx, cudaStreamWaitEvent(s, b->order_wait, 0));
+    if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
+    AeadArgs a = aead_args(b, npkts, true, nullptr);
+    a.over_link = true;
+    a.in = a.out = h.ring;
+    a.off = h.off;
+    a.len = h.len;
+    a.slot = h.slot;
+    a.res[0] = AeadResults{h.counter, h.out_len, h.status, nullptr};
+    if (flags & BNK_F_DEMUX_INDEX) {
+        a.demux = true;
+        a.index_keys = ctx->kt.index_keys;
+        a.index_vals = ctx->kt.index_vals;
+        a.index_slots = ctx->kt.index_slots;
+        a.res[0].slot = h.slot;
+    }
+    const bool tail = replay || checks;
+    if (tail) {
+        a.res[0].out_len = nullptr;
+        a.res[0].status = nullptr;
+        a.res[1] = AeadResults{b->dev.counter, b->dev.out_len, b->dev.status, b->dev.slot};
+        if (checks) a.inner = b->dev.inner;
+        a.inner_cut = (flags & BNK_F_INNER_CHECK) != 0;
+    } else if (stats) {
+        a.res[1] = AeadResults{nullptr, b->dev.out_len, b->dev.status, nullptr};
+    }
+    // beyond one launch the replay window is a chain of kernels, and the results come back by copy
+    const bool one_launch = npkts <= kGroupMax || !replay;
+    const Done done = stats || !one_launch ? Done{} : watch_for(b);
+    if (!tail) a.done = done;
+    if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
+    CK(ctx, launch_open(a, s, ctx));
+    if (timed) CK(ctx, cudaEventRecord(b->a_end, s));
+    if (tail) {
+        VerdictArgs v{};
+        v.ft = ctx->ft;
+        v.inner = b->dev.inner;
+        v.slot = b->dev.slot;
+        v.allowed_ip = ctx->kt.allowed_ip;
+        v.status = b->dev.status;
+        v.out_len = b->dev.out_len;
+        v.now = now_unix_ns;
+        v.n = npkts;
+        v.inner_check = (flags & BNK_F_INNER_CHECK) != 0;
+        v.check_inbound = (flags & BNK_F_CHECK_INBOUND) != 0;
+        if (v.check_inbound) flow_check_begins(b, now_unix_ns);
+        if (one_launch) {
+            v.host_status = h.status;
+            v.host_out_len = h.out_len;
+            CK(ctx, launch_open_tail(b, npkts, replay, &v, done, s));
+        } else {
+            CK(ctx, launch_group_by_slot(b, npkts, s));
+            CK(ctx, launch_replay(b, npkts, s));
+            if (checks) CK(ctx, launch_verdict(ctx, v, Done{}, s));
+        }
+    }
+    if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
+    b->kernel_timed = b->aead_timed = timed;
+    CK(ctx, tally_if_asked(b, npkts, flags, s));
+    if (b->order_record) CK(ctx, cudaEventRecord(b->order_record, s));
+    if (!one_launch) CK(ctx, desc_copy(b, npkts, D_OUT_LEN, D_STATUS, false, s));
     return BNK_SUCCESS;
 }
 
@@ -900,11 +1058,10 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     const size_t n = npkts;
     const bool refresh = b->dev_stale;
     const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, (flags & BNK_F_USE_OUT_LEN) ? 48 : 0);
-    const bool direct = host_direct(b, npkts, flags, ext);
-    HostAlias alias(b, direct);
+    if (ctx->aead_mode != 1 && host_direct(b, npkts, flags, ext)) return open_direct(b, npkts, flags, now_unix_ns);
     // BNK_F_USE_OUT_LEN reads the lengths a seal left on the device: an upload beside it must not bring the
     // host's out_len along, so it moves the fields one by one instead of the whole slab.
-    if (!direct && (!(flags & BNK_F_NO_H2D) || refresh) && n) {
+    if ((!(flags & BNK_F_NO_H2D) || refresh) && n) {
         if (b->joint_copy && !((flags & BNK_F_USE_OUT_LEN) && !refresh)) {
             CK(ctx, cudaMemcpyAsync(b->d_desc, b->h_desc, b->desc_room + ext, cudaMemcpyHostToDevice, s));
         } else {
@@ -924,12 +1081,12 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
         order = b->dev.len_order;
     }
     oa.order = order;
-    const bool replay_fused = (flags & BNK_F_REPLAY) && replay_is_one_launch(npkts);
-    if ((flags & BNK_F_REPLAY) && !replay_fused) {
+    const bool replay = (flags & BNK_F_REPLAY) && n, one_launch = npkts <= kGroupMax;
+    if (replay && !one_launch) {
         // grouping by keypair needs only the descriptors: it runs on the side stream beside the open kernel
         CK(ctx, cudaEventRecord(b->ev_fork, s));
         CK(ctx, cudaStreamWaitEvent(b->aux_stream, b->ev_fork, 0));
-        CK(ctx, launch_group_by_slot(b, npkts, false, b->aux_stream));
+        CK(ctx, launch_group_by_slot(b, npkts, b->aux_stream));
         CK(ctx, cudaEventRecord(b->ev_join, b->aux_stream));
     }
     const bool side = b->aead_stream && npkts >= ctx->aead_side_stream_from;
@@ -946,19 +1103,22 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
         CK(ctx, cudaStreamWaitEvent(s, b->ev_aead_done, 0));
     }
     b->aead_timed = timed;
-    if (replay_fused) { // small batch: one launch sorts and walks; the stream hand-over would cost more than it hides
-        CK(ctx, launch_group_and_replay(b, npkts, s));
-    } else if (flags & BNK_F_REPLAY) {
+    if (replay && one_launch) {
+        CK(ctx, launch_open_tail(b, npkts, true, nullptr, Done{}, s));
+    } else if (replay) {
         CK(ctx, cudaStreamWaitEvent(s, b->ev_join, 0));
         CK(ctx, launch_replay(b, npkts, s));
     }
     if (flags & BNK_F_INNER_CHECK) CK(ctx, launch_inner_check(b, npkts, s));
-    if (flags & BNK_F_CHECK_INBOUND) CK(ctx, launch_filter_check(b, npkts, now_unix_ns, true, s));
+    if (flags & BNK_F_CHECK_INBOUND) {
+        flow_check_begins(b, now_unix_ns);
+        CK(ctx, launch_filter_check(b, npkts, now_unix_ns, true, s));
+    }
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
     if (b->order_record) CK(ctx, cudaEventRecord(b->order_record, s));
-    if (!direct && !(flags & BNK_F_NO_D2H) && n) {
+    if (!(flags & BNK_F_NO_D2H) && n) {
         if (b->joint_copy) {
             CK(ctx, cudaMemcpyAsync(b->h_desc, b->d_desc, b->desc_room + ext, cudaMemcpyDeviceToHost, s));
         } else {
@@ -994,10 +1154,15 @@ int bnk_filter_note_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t
         }
     }
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
-    CK(ctx, launch_filter_note(b, npkts, now_unix_ns, s));
+    bool sweep = false;
+    if (n && ctx->ft.enforce && ctx->ft.flow_capacity) {
+        sweep = flow_note_begins(b, npkts, now_unix_ns);
+        CK(ctx, launch_filter_note(b, npkts, now_unix_ns, s));
+        if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, Done{}, s));
+    }
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = timed;
-    CK(ctx, launch_flow_report(b, s));
+    if (!sweep) CK(ctx, launch_flow_report(b, s));
     return BNK_SUCCESS;
 }
 
@@ -1025,6 +1190,7 @@ int bnk_filter_check_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_
         }
     }
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
+    flow_check_begins(b, now_unix_ns);
     CK(ctx, launch_filter_check(b, npkts, now_unix_ns, false, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = timed;
@@ -1108,25 +1274,42 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
     return BNK_SUCCESS;
 }
 
+// Watches the word that the submit's last kernel stores.  Like the driver's own wait it keeps the core; after
+// ~200 us, or if the word does not come because the work failed, the driver's wait takes over.
+static bool done_seen(bnk_batch *b, uint64_t timeout_ns) {
+    if (!b->done_watched) return false;
+    const volatile uint32_t *word = b->h_done;
+    const uint64_t turns = timeout_ns / 64 < 4096 ? timeout_ns / 64 : 4096; // a turn is at least ~40 ns
+    for (uint32_t i = 0; *word != b->done_seq; i++) {
+        if (i >= turns) return false;
+        cpu_relax();
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return true;
+}
+
 int bnk_wait(bnk_batch *b, uint64_t timeout_ns) {
     if (!b) return BNK_EINVAL;
     if (!b->in_flight) return BNK_SUCCESS;
     bnk_ctx *ctx = b->ctx;
-    CK(ctx, cudaSetDevice(ctx->device));
-    if (timeout_ns == UINT64_MAX) {
-        CK(ctx, cudaStreamSynchronize(b->stream));
-    } else {
-        const auto deadline = std::chrono::steady_clock::now() + std::chrono::nanoseconds(timeout_ns);
-        for (;;) {
-            cudaError_t e = cudaStreamQuery(b->stream);
-            if (e == cudaSuccess) break;
-            if (e != cudaErrorNotReady) return fail(ctx, BNK_ECUDA, "cudaStreamQuery", e);
-            if (std::chrono::steady_clock::now() >= deadline) return BNK_ETIMEDOUT;
-            std::this_thread::yield();
+    if (!done_seen(b, timeout_ns)) {
+        if (b->done_watched && timeout_ns == 0 && (++b->done_polls & 63u)) return BNK_ETIMEDOUT; // ask the driver now and then
+        CK(ctx, cudaSetDevice(ctx->device));
+        if (timeout_ns == UINT64_MAX) {
+            CK(ctx, cudaStreamSynchronize(b->stream));
+        } else {
+            const auto deadline = std::chrono::steady_clock::now() + std::chrono::nanoseconds(timeout_ns);
+            for (;;) {
+                cudaError_t e = cudaStreamQuery(b->stream);
+                if (e == cudaSuccess) break;
+                if (e != cudaErrorNotReady) return fail(ctx, BNK_ECUDA, "cudaStreamQuery", e);
+                if (std::chrono::steady_clock::now() >= deadline) return BNK_ETIMEDOUT;
+                std::this_thread::yield();
+            }
         }
     }
-    b->in_flight = false;
-    direct_done(b);
+    submit_over(b);
+    if (b->flow_in_flight || b->flow_reported) flow_work_over(b);
     if (b->flow_reported) { // what the device said about the flow table after this batch: input of the next compaction
         b->flow_reported = false;
         for (int c = 0; c < 3; c++) ctx->flow_dead_hint[c] = b->h_flow->dead[c];

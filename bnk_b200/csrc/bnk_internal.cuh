@@ -24,6 +24,7 @@ struct KeypairTables {
     uint32_t *recv_keys;    // [max_keypairs][8]
     uint32_t *remote_index; // [max_keypairs] receiver index written into sealed headers
     uint64_t *send_counter; // [max_keypairs] next nonce to hand out
+    uint32_t *arrived;      // [max_keypairs] scratch of the seal kernel that hands out counters itself, zero between launches
     uint64_t *replay_last;  // [max_keypairs] highest counter accepted
     uint64_t *replay_next;  // [max_keypairs] scratch: the value replay_last takes after the batch in flight
     uint64_t *replay_ring;  // [max_keypairs][ring_blocks] RFC 6479 bitmap ring
@@ -62,7 +63,6 @@ struct FilterTables {
     uint8_t flow_half[3];
     unsigned long long *flow_live;  // device control block (FlowCtl): live entries (Go's len(f.flows)) and more
     long long *flow_special_exp;    // [3] entry for the one key that equals FLOW_EMPTY
-    int *flow_error;       // counts the inserts that found no free slot
 };
 // region of protocol class `cls` that is in use
 __host__ __device__ inline size_t flow_region(const FilterTables &ft, int cls) {
@@ -70,9 +70,11 @@ __host__ __device__ inline size_t flow_region(const FilterTables &ft, int cls) {
 }
 // What a batch's filter work reports back to the host next to the packets (pinned, one per batch).
 struct FlowReport {
-    int error;            // inserts that found no free slot, since the table was last cleared
-    uint32_t used[3];     // slots of the class's region that hold a key, live or deleted
-    uint32_t dead[3];     // of those, deleted ones (reclaimed by compaction)
+    unsigned long long live; // len(f.flows)
+    long long floor;         // no entry's expiry lies below this
+    int error;               // inserts that found no free slot, since the table was last cleared
+    uint32_t used[3];        // slots of the class's region that hold a key, live or deleted
+    uint32_t dead[3];        // of those, deleted ones (reclaimed by compaction)
 };
 
 struct bnk_ctx {
@@ -84,7 +86,8 @@ struct bnk_ctx {
     cudaEvent_t timer_start;
     int sm_count;
     uint64_t host_direct_bytes; // batches up to this ring extent run on the caller's pinned buffers (BNK_HOST_DIRECT_BYTES)
-    std::atomic<int> direct_in_flight{0}; // batches whose last submit ran that way and has not been waited for
+    std::atomic<int> in_flight{0};           // batches submitted and not waited for
+    std::atomic<uint64_t> direct_in_flight{0}; // ring bytes of those that run on the pinned buffers
     int aead_mode; // 0 = choose by batch size, 1 = always thread per packet, 2 = always warp per packet (BNK_AEAD_KERNEL)
     uint32_t aead_side_stream_from; // batches of at least this many packets run seal/open on the low-priority stream (BNK_AEAD_SIDE_STREAM_FROM; 0 = never)
     int prio_low, prio_high;        // stream priority range of the device
@@ -97,6 +100,14 @@ struct bnk_ctx {
     std::shared_mutex submit_mu;
     std::vector<bnk_batch *> batches;       // every live batch of the context (guarded by mu)
     std::atomic<uint32_t> flow_dead_hint[3]; // deleted entries per class as last reported by the device
+    // What the host knows about the flow table without asking: no entry expires before flow_floor, at most
+    // flow_live_most are live.  Every submit with filter work widens them; a report of the device replaces them
+    // unless another such submit has been made since (flow_epoch) or is under way.
+    std::mutex flow_mu;
+    long long flow_floor = 0;
+    uint64_t flow_live_most = 0;
+    uint32_t flow_epoch = 0;
+    int flow_in_flight = 0; // batches whose filter work has not been waited for
     std::atomic<int> flow_errors_seen;       // failed inserts already reported to a caller as BNK_EFULL
     // rule table: two device buffer sets, the one not in use receives the next upload
     struct RuleSet {
@@ -134,6 +145,7 @@ struct DeviceBatch {
     uint64_t *replay_tile_carry; // [tiles]
     uint32_t *hist;       // [512 * chunks] digit-major histograms
     uint32_t *len_order;  // [max_pkts] packet indices ordered by length class
+    uint4 *inner;         // [max_pkts] headers of opened packets on their way to the last checks
     uint32_t *counters32; // small scratch (bins)
     bnk_gso_super *gso;   // [max_pkts] super-packet descriptors of a GSO split
 };
@@ -158,7 +170,12 @@ struct bnk_batch {
     cudaEvent_t k_begin, k_end, t_end, a_begin, a_end;
     bool in_flight;
     bool dev_stale; // a submit ran on the host arrays: the device copies of ring and descriptors are behind
-    bool direct_counted; // this batch is one of ctx->direct_in_flight
+    bool counted;        // this batch is one of ctx->in_flight
+    uint64_t direct_counted; // what it adds to ctx->direct_in_flight
+    // bnk_wait watches *h_done for done_seq when done_watched: the last kernel of the submit stores it (Done)
+    uint32_t *h_done, *d_ticket;
+    uint32_t done_seq, done_polls;
+    bool done_watched;
     bool kernel_timed;
     bool aead_timed;
     bnk_gso_super *h_gso; // pinned staging for the super-packet descriptors
@@ -168,6 +185,8 @@ struct bnk_batch {
     bool joint_copy;   // descriptors and ring move as one copy
     FlowReport *h_flow; // pinned copy of the flow table's state after the batch's filter work
     bool stats_pending; // the last submit was made with BNK_F_STATS
+    uint32_t flow_epoch; // ctx->flow_epoch of the last submit with filter work
+    bool flow_in_flight; // this batch is one of ctx->flow_in_flight
     bool flow_reported; // the last submit queued a copy of the flow table's state into h_flow
     bnk_batch_stats *h_stats; // pinned; written by the tally kernel
     unsigned long long *d_stats; // device accumulators of the tally kernel (zero between launches)
@@ -222,43 +241,95 @@ cudaError_t launch_kernel(bool dependent, void (*kernel)(KArgs...), dim3 grid, d
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+constexpr uint32_t kSlotNoKeypair = 0xfffffffeu; // demux found no keypair for the receiver index
+
 // ---------------------------------------------------------------------------
 // Kernel launchers (each defined next to its kernels).  All are asynchronous on
 // `s` and return the cudaError_t of the launch.
 // ---------------------------------------------------------------------------
-struct AeadArgs {
-    uint8_t *ring;
-    const uint32_t *off;
-    const uint32_t *len;
-    const uint32_t *slot;
+struct AeadResults { // where a packet's outcome goes; null members are left out
     uint64_t *counter;
     uint32_t *out_len;
     uint8_t *status;
+    uint32_t *slot; // open side with demux
+};
+// How a batch's last kernel tells the host that everything before it is done: the CTA that finishes last stores
+// `value` to a pinned word (bnk_wait watches it, which saves the ~3 us a stream synchronisation takes to notice).
+struct Done {
+    uint32_t *ticket; // device, zero between launches
+    uint32_t *flag;   // pinned; null: nobody watches
+    uint32_t value;
+};
+// By all threads of all CTAs, once, at the end; `last_words` runs in one thread when every CTA's stores are visible.
+template <typename F>
+__device__ __forceinline__ void signal_done(const Done &d, F last_words) {
+    if (d.flag == nullptr) return;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence_system(); // the CTA's stores, to host memory too, before its ticket
+    if (gridDim.x != 1 && atomicAdd(d.ticket, 1u) + 1u != gridDim.x) return;
+    *d.ticket = 0u;
+    __threadfence();
+    last_words();
+    __threadfence_system();
+    *(volatile uint32_t *)d.flag = d.value;
+}
+struct AeadArgs {
+    const uint8_t *in;            // ring the input is read from and ...
+    uint8_t *out, *out2;          // ... ring(s) the output goes to; thread per packet: in == out, no out2
+    const uint32_t *off;
+    const uint32_t *len;
+    const uint32_t *slot;
+    const uint64_t *counter;      // seal only
+    AeadResults res[2];           // thread per packet: res[0] only, all members but slot set
     const uint32_t *keys;         // send keys (seal) or receive keys (open)
     const uint32_t *remote_index; // seal only
     const uint8_t *valid;         // per keypair slot: keys present
-    const uint32_t *order;        // optional scheduling permutation, may be null
+    const uint32_t *order;        // thread per packet: optional scheduling permutation, may be null
+    const uint64_t *index_keys;   // with demux: the receiver-index table
+    const uint32_t *index_vals;
+    uint32_t index_slots;
+    bool demux;                   // open, warp per packet: the slot comes from the header's receiver index
+    bool inner_cut;               // packets will be cut to their IPv4 total length
+    uint4 *inner;                 // open, warp per packet: headers of the plaintexts (see VerdictArgs); null: not wanted
+    bool over_link;               // a ring is in host memory
     uint32_t n;
+    uint32_t tile;                // set by the launcher
     uint32_t mtu;
     uint32_t max_slots;
     uint64_t ring_bytes;
+    // Seal of up to kRankMax packets in pinned memory: nonces are handed out by the seal kernel itself (null: from counter[])
+    uint64_t *send_counter;       // [max_slots]
+    uint32_t *arrived;            // [max_slots] packets of the slot that have read their counter; zero between launches
+    // Seal in pinned memory with BNK_F_NOTE_OUTBOUND: the kernel records its packets' flows
+    bool note;
+    long long now;
+    FilterTables ft;
+    FlowReport *flow_report;      // pinned, written before `done`; null: none
+    Done done;
 };
+constexpr uint32_t kRankMax = 256;
 cudaError_t launch_seal(const AeadArgs &a, cudaStream_t s, bnk_ctx *ctx);
 cudaError_t launch_open(const AeadArgs &a, cudaStream_t s, bnk_ctx *ctx);
 
 // group_kernels.cu
-cudaError_t launch_group_by_slot(bnk_batch *b, uint32_t n, bool only_status_ok, cudaStream_t s);
-cudaError_t launch_assign_counters(bnk_batch *b, uint32_t n, cudaStream_t s);
+cudaError_t launch_group_by_slot(bnk_batch *b, uint32_t n, cudaStream_t s);
+// slot / counter: the batch's arrays, wherever they are (device or pinned)
+cudaError_t launch_assign_counters(bnk_batch *b, uint32_t n, const uint32_t *slot, uint64_t *counter, cudaStream_t s);
 cudaError_t launch_replay(bnk_batch *b, uint32_t n, cudaStream_t s);
-bool replay_is_one_launch(uint32_t n); // small batches: grouping and walk fit one CTA
-cudaError_t launch_group_and_replay(bnk_batch *b, uint32_t n, cudaStream_t s); // after the open kernel
+struct VerdictArgs;
+// After the open kernel, up to kGroupMax packets: grouping, replay window (when `replay`) and the last checks in one launch.
+constexpr uint32_t kGroupMax = 32768;
+cudaError_t launch_open_tail(bnk_batch *b, uint32_t n, bool replay, const VerdictArgs *verdict, const Done &done, cudaStream_t s);
+cudaError_t launch_verdict(bnk_ctx *ctx, const VerdictArgs &verdict, const Done &done, cudaStream_t s); // the last checks alone
+cudaError_t group_kernels_init(); // once per context, for the current device
 cudaError_t launch_length_order(bnk_batch *b, uint32_t n, const uint32_t *len, bool open_side, cudaStream_t s);
 uint32_t group_sort_chunks(uint32_t max_pkts);
 uint32_t replay_scan_tiles(uint32_t max_pkts);     // tiles of the running-maximum scan
 uint32_t replay_hash_capacity(uint32_t max_pkts);  // entries of the duplicate-counter table
 
 // filter_kernels.cu
-cudaError_t launch_filter_note(bnk_batch *b, uint32_t n, long long now_ns, cudaStream_t s);
+cudaError_t launch_filter_note(bnk_batch *b, uint32_t n, long long now_ns, cudaStream_t s); // the inserts; no sweep
 cudaError_t launch_filter_check(bnk_batch *b, uint32_t n, long long now_ns, bool only_status_ok, cudaStream_t s);
 cudaError_t filter_tables_alloc(bnk_ctx *ctx);
 void filter_tables_free(bnk_ctx *ctx);
@@ -268,6 +339,12 @@ cudaError_t filter_flow_stats(bnk_ctx *ctx, uint64_t *live, uint32_t used[3], ui
 int filter_flows_export(bnk_ctx *ctx, bnk_flow_entry *out, size_t capacity, size_t *count);
 int filter_flows_import(bnk_ctx *ctx, const bnk_flow_entry *entries, size_t n);
 cudaError_t launch_flow_report(bnk_batch *b, cudaStream_t s); // copies the flow table's control block to b->h_flow
+// A submit is about to record up to n flows at `now` / to check packets at `now`.  The former returns whether the
+// batch may have to sweep expired flows behind its inserts (launch_flow_sweep).
+bool flow_note_begins(bnk_batch *b, uint32_t n, long long now);
+void flow_check_begins(bnk_batch *b, long long now);
+void flow_work_over(bnk_batch *b); // the batch has been waited for; its report, if it made one, is in b->h_flow
+cudaError_t launch_flow_sweep(bnk_batch *b, long long now, const Done &done, cudaStream_t s);
 // Rebuilds the regions whose deleted entries have piled up; called by a submit that feeds the flow table,
 // before it takes submit_mu.  Returns without doing anything in the common case.
 cudaError_t filter_flows_maintain(bnk_batch *b, cudaStream_t s);
@@ -275,10 +352,14 @@ cudaError_t filter_flows_maintain(bnk_batch *b, cudaStream_t s);
 cudaError_t launch_tally(bnk_batch *b, uint32_t n, cudaStream_t s);
 
 // inner_kernels.cu
-constexpr uint32_t kSlotNoKeypair = 0xfffffffeu; // demux found no keypair for the receiver index
 cudaError_t launch_demux_index(bnk_batch *b, uint32_t n, const uint32_t *len, cudaStream_t s);
 cudaError_t launch_inner_check(bnk_batch *b, uint32_t n, cudaStream_t s);
 cudaError_t launch_classify(bnk_batch *b, uint32_t n, cudaStream_t s);
+// nonce of the k-th packet of a run that starts at `base`: never past the message limit
+__device__ __forceinline__ uint64_t saturating_counter(uint64_t base, uint32_t k) {
+    const uint64_t c = base + k;
+    return (c < base || c > BNK_REJECT_AFTER_MESSAGES) ? BNK_REJECT_AFTER_MESSAGES : c;
+}
 __host__ __device__ inline uint32_t addr_hash(uint64_t hi, uint64_t lo, uint32_t port) {
     uint64_t z = hi * 0x9e3779b97f4a7c15ull ^ (lo + 0xbf58476d1ce4e5b9ull) * 0x94d049bb133111ebull ^ ((uint64_t)port << 40);
     z ^= z >> 29;
@@ -290,6 +371,21 @@ __host__ __device__ inline uint32_t index_hash(uint32_t index) {
     z ^= z >> 15;
     z *= 0x85ebca6bu;
     return z ^ (z >> 13);
+}
+// Receiver index -> keypair slot by a whole warp: the 32 places from the index's own on are looked at in one read, so
+// a lookup is one trip to the table however long its probe chain (tables are at most half full).
+__device__ __forceinline__ uint32_t demux_index_warp(const uint64_t *keys, const uint32_t *vals, uint32_t slots, uint32_t index) {
+    const uint64_t key = (1ull << 32) | index;
+    for (uint32_t base = 0; base < slots; base += 32) {
+        const uint32_t h = (index_hash(index) + base + (threadIdx.x & 31u)) & (slots - 1);
+        const uint64_t k = keys[h];
+        const uint32_t v = vals[h];
+        const uint32_t hit = __ballot_sync(0xffffffffu, k == key), empty = __ballot_sync(0xffffffffu, k == 0);
+        const uint32_t at = __ffs(hit) - 1;
+        if (hit && (empty == 0 || at < (uint32_t)__ffs(empty) - 1)) return __shfl_sync(0xffffffffu, v, at);
+        if (empty) break;
+    }
+    return kSlotNoKeypair;
 }
 
 // gso_kernels.cu

@@ -1,0 +1,289 @@
+// Device side of the packet filter: the parser, the rule match and the reply-flow table (filter.Filter's f.flows,
+// internal/filter/filter.go:26-38 of the reference), shared by the filter kernels and by the seal and open kernels
+// that do their packets' filter work in passing.
+//
+// Flows.  Go's map[flowKey]time.Time becomes three open-addressing tables (tcp, udp, icmp) keyed by remote address | remote
+// port | local port, claimed with a 64-bit compare-and-swap.  A deleted entry keeps its key with expiry FLOW_DEAD,
+// which behaves like an absent key for every later lookup.  The live-entry count is kept exactly because the
+// reference's expiry sweep depends on len(flows) > 4096.
+#pragma once
+
+#include <climits>
+
+#include "bnk_internal.cuh"
+
+constexpr unsigned long long FLOW_EMPTY = ~0ull;
+constexpr long long FLOW_DEAD = LLONG_MIN;      // the key is there, the entry is deleted
+constexpr long long FLOW_FRESH = LLONG_MIN + 1; // expiry of a slot no key has used yet
+__host__ __device__ __forceinline__ bool flow_absent(long long exp) { return exp <= FLOW_FRESH; }
+constexpr long long TTL_UDP = 30ll * 1000000000ll;  // filter.go:19
+constexpr long long TTL_TCP = 120ll * 1000000000ll; // filter.go:20
+constexpr long long TTL_ICMP = 30ll * 1000000000ll; // filter.go:21
+constexpr long long TTL_LEAST = TTL_UDP;
+constexpr unsigned long long SWEEP_THRESHOLD = 4096; // filter.go:202
+
+// small device-side control block behind FilterTables::flow_live
+struct FlowCtl {
+    FlowReport rep;             // live count, floor of the expiries, overflow flag, per-class slot counts
+    unsigned long long dropped; // entries the sweep under way has deleted
+    long long next_floor;       // lowest expiry it has left
+    uint32_t ticket;            // CTAs of the sweep that have finished
+    uint32_t moved;             // entries a compaction has re-inserted so far
+};
+__device__ __forceinline__ FlowCtl *flow_ctl(const FilterTables &ft) { return reinterpret_cast<FlowCtl *>(ft.flow_live); }
+
+__host__ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
+    z += 0x9e3779b97f4a7c15ull;
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+    return z ^ (z >> 31);
+}
+
+struct Parsed {
+    uint32_t src, dst;
+    uint16_t sport, dport;
+    uint8_t proto;
+};
+// filter.go:71-106 in two steps, so that the caller can fetch the ports from wherever it has them: w0..w4 are the first
+// twenty bytes (present when len >= 20); returns the byte offset of the ports, 0 when none are needed, or
+// kParseBad for a packet that does not parse.
+constexpr uint32_t kParseBad = 0xffffffffu;
+__device__ __forceinline__ uint32_t parse_ipv4_words(uint32_t w0, uint32_t w2, uint32_t w3, uint32_t w4, uint32_t len, Parsed &out) {
+    if (len < 20) return kParseBad;
+    if (((w0 & 0xffu) >> 4) != 4u) return kParseBad;
+    const uint32_t ihl = (w0 & 0x0fu) * 4u;
+    if (ihl < 20u || len < ihl) return kParseBad;
+    out.proto = (uint8_t)((w2 >> 8) & 0xffu); // byte 9
+    out.src = __byte_perm(w3, 0, 0x0123);     // bytes 12..15, big-endian
+    out.dst = __byte_perm(w4, 0, 0x0123);
+    out.sport = 0;
+    out.dport = 0;
+    const uint32_t body = len - ihl;
+    if (out.proto == 6 || out.proto == 17) return body < 4 ? kParseBad : ihl; // ihl is a multiple of 4
+    if (out.proto == 1) return body >= 1 ? 0u : kParseBad;
+    return kParseBad;
+}
+__device__ __forceinline__ void parse_ports(uint32_t ports, Parsed &out) {
+    out.sport = (uint16_t)(((ports & 0xffu) << 8) | ((ports >> 8) & 0xffu));
+    out.dport = (uint16_t)((((ports >> 16) & 0xffu) << 8) | (ports >> 24));
+}
+
+__device__ __forceinline__ int proto_class(uint8_t proto) { return proto == 6 ? 0 : (proto == 17 ? 1 : 2); }
+__device__ __forceinline__ long long flow_ttl(uint8_t proto) { // filter.go:108-117
+    return proto == 6 ? TTL_TCP : (proto == 1 ? TTL_ICMP : TTL_UDP);
+}
+__device__ __forceinline__ unsigned long long flow_key(uint32_t remote, uint16_t rport, uint16_t lport) {
+    return ((unsigned long long)remote << 32) | ((unsigned long long)rport << 16) | lport;
+}
+
+// One atomic per group of lanes that add to the same counter at the same point of the code, instead of one per
+// lane: a batch of new flows otherwise sends a few hundred thousand atomics to two addresses (300,000 fresh flows
+// took 0.7 ms that way).
+template <typename T>
+__device__ __forceinline__ void add_one_aggregated(T *counter) {
+    const unsigned same = __match_any_sync(__activemask(), (unsigned long long)(uintptr_t)counter);
+    if ((threadIdx.x & 31u) == (unsigned)(__ffs(same) - 1)) atomicAdd(counter, (T)__popc(same));
+}
+// No entry expires before rep.floor: whoever writes an expiry below it lowers it (rare: a fresh expiry lies at least
+// the shortest lifetime ahead, and the floor is where the oldest entry stood at the last sweep).
+__device__ __forceinline__ void flow_keep_floor(FlowCtl *ctl, long long exp) {
+    if (exp < *(volatile long long *)&ctl->rep.floor) atomicMin(&ctl->rep.floor, exp);
+}
+
+// NoteOutbound (filter.go:189-209) of one flow by one thread, in three steps that each start with what the step
+// before has asked memory for, so that a caller can do other work in between.
+struct FlowNote {
+    unsigned long long key = FLOW_EMPTY, old = FLOW_EMPTY;
+    long long exp = 0, prev = 0;
+    uint32_t h = 0;
+    int cls = -1; // -1: nothing to note
+    bool placed = false;
+
+    __device__ __forceinline__ void begin(const FilterTables &ft, const Parsed &p, long long now) {
+        cls = proto_class(p.proto);
+        exp = now + flow_ttl(p.proto);
+        key = flow_key(p.dst, p.dport, p.sport);
+        h = (uint32_t)mix64(key) & (ft.flow_capacity - 1);
+        if (key != FLOW_EMPTY)
+            old = atomicCAS((unsigned long long *)ft.flow_keys + flow_region(ft, cls) + h, FLOW_EMPTY, key);
+    }
+    __device__ __forceinline__ void place(const FilterTables &ft) {
+        if (cls < 0) return;
+        if (key == FLOW_EMPTY) {
+            prev = (long long)atomicExch((unsigned long long *)&ft.flow_special_exp[cls], (unsigned long long)exp);
+            placed = true;
+            return;
+        }
+        unsigned long long *const keys = (unsigned long long *)ft.flow_keys + flow_region(ft, cls);
+        for (uint32_t probe = 1; old != FLOW_EMPTY && old != key; probe++) {
+            if (probe >= ft.flow_capacity) { // table full: the flow is not recorded, the host reports BNK_EFULL
+                atomicAdd(&flow_ctl(ft)->rep.error, 1);
+                return;
+            }
+            h = (h + 1) & (ft.flow_capacity - 1);
+            old = atomicCAS(&keys[h], FLOW_EMPTY, key);
+        }
+        prev = (long long)atomicExch((unsigned long long *)ft.flow_exp + flow_region(ft, cls) + h, (unsigned long long)exp);
+        placed = true;
+    }
+    __device__ __forceinline__ void count(const FilterTables &ft) {
+        if (!placed) return;
+        FlowCtl *const ctl = flow_ctl(ft);
+        if (key != FLOW_EMPTY && old == FLOW_EMPTY) add_one_aggregated(&ctl->rep.used[cls]);
+        if (flow_absent(prev)) add_one_aggregated(&ctl->rep.live);
+        if (key != FLOW_EMPTY && prev == FLOW_DEAD) atomicSub(&ctl->rep.dead[cls], 1u); // a deleted entry is back
+        flow_keep_floor(ctl, exp);
+    }
+};
+
+// The state of the table after a batch, for the host (one thread, when all the batch's filter work is visible).
+__device__ __forceinline__ void flow_report(const FlowCtl *ctl, FlowReport *host) {
+    const volatile FlowReport *const r = &ctl->rep;
+    FlowReport v;
+    v.live = r->live;
+    v.floor = r->floor;
+    v.error = r->error;
+    for (int c = 0; c < 3; c++) {
+        v.used[c] = r->used[c];
+        v.dead[c] = r->dead[c];
+    }
+    *host = v;
+}
+
+// ---- rules ----
+// Slot of a rule key: the key is a 32-bit address and a prefix length, so a 32-bit finaliser (two 32-bit
+// multiplies) spreads it; the 64-bit mixer above costs three times the instructions on a machine without a 64-bit
+// multiplier, and the check kernel hashes once per prefix length and packet.
+__host__ __device__ __forceinline__ uint32_t rule_hash(uint64_t key) {
+    uint32_t x = (uint32_t)key ^ ((uint32_t)(key >> 32) * 0x9e3779b1u);
+    x ^= x >> 16;
+    x *= 0x85ebca6bu;
+    x ^= x >> 13;
+    x *= 0xc2b2ae35u;
+    return x ^ (x >> 16);
+}
+
+__host__ __device__ __forceinline__ uint64_t rule_key(uint32_t len, uint32_t addr) {
+    const uint32_t mask = len == 0 ? 0u : 0xffffffffu << (32 - len);
+    return (1ull << 40) | ((uint64_t)len << 32) | (addr & mask);
+}
+
+// any allowance matches?  acl.go:149-172 over the indexed table
+// (Fetching the first slot of four prefix lengths before looking at any of them, to overlap the round trips, was
+// measured: 10 % slower on configuration 3, where nearly half the packets match at one of the first lengths.)
+__device__ __forceinline__ bool rules_allow(const FilterTables &ft, const Parsed &p) {
+    if (ft.rule_slots == 0) return false;
+    // longest prefixes first: acl.Compile emits /32s (acl.go:98), so a packet that some rule admits is most often
+    // admitted at the first probe; any match allows, the order changes no verdict
+    uint64_t lens = ft.len_mask;
+    while (lens) {
+        const uint32_t len = 63u - (uint32_t)__clzll((long long)lens);
+        lens &= ~(1ull << len);
+        const uint64_t key = rule_key(len, p.src);
+        uint32_t h = rule_hash(key) & (ft.rule_slots - 1);
+        for (uint32_t probe = 0; probe < ft.rule_slots; probe++) {
+            const uint64_t k = ft.rule_keys[h];
+            if (k == 0) break;
+            if (k == key) {
+                const uint2 span = ft.rule_span[h];
+                for (uint32_t e = 0; e < span.y; e++) {
+                    const uint64_t ent = ft.rule_entries[span.x + e];
+                    if ((uint8_t)(ent >> 32) != p.proto) continue;
+                    if (p.proto == 1) return true;
+                    const uint16_t first = (uint16_t)(ent >> 16), last = (uint16_t)ent;
+                    if (p.dport >= first && p.dport <= last) return true;
+                }
+                break;
+            }
+            h = (h + 1) & (ft.rule_slots - 1);
+        }
+    }
+    return false;
+}
+
+// CheckInbound (filter.go:121-147) of a packet that parses, with enforcement on: a rule allows it, or it is the reply to
+// a flow that is alive (the key mirrors NoteOutbound's), which it then keeps alive.
+__device__ __forceinline__ uint8_t filter_verdict(const FilterTables &ft, const Parsed &p, long long now) {
+    if (rules_allow(ft, p)) return BNK_PKT_OK;
+    if (ft.flow_capacity == 0) return BNK_PKT_FILTER_DENY;
+    FlowCtl *const ctl = flow_ctl(ft);
+    const int cls = proto_class(p.proto);
+    const unsigned long long key = flow_key(p.src, p.sport, p.dport);
+    long long *slot_exp = nullptr;
+    if (key == FLOW_EMPTY) {
+        slot_exp = &ft.flow_special_exp[cls];
+    } else {
+        const unsigned long long *const keys = (const unsigned long long *)ft.flow_keys + flow_region(ft, cls);
+        uint32_t h = (uint32_t)mix64(key) & (ft.flow_capacity - 1);
+        for (uint32_t probe = 0; probe < ft.flow_capacity; probe++) {
+            const unsigned long long k = keys[h];
+            if (k == FLOW_EMPTY) break;
+            if (k == key) {
+                slot_exp = ft.flow_exp + flow_region(ft, cls) + h;
+                break;
+            }
+            h = (h + 1) & (ft.flow_capacity - 1);
+        }
+    }
+    if (!slot_exp) return BNK_PKT_FILTER_DENY;
+    const long long exp = *(volatile long long *)slot_exp;
+    if (flow_absent(exp)) return BNK_PKT_FILTER_DENY;
+    if (now < exp) { // strict: time.Before
+        const long long fresh = now + flow_ttl(p.proto);
+        *(volatile long long *)slot_exp = fresh; // keep-alive on traffic
+        flow_keep_floor(ctl, fresh);
+        return BNK_PKT_OK;
+    }
+    const long long prev = (long long)atomicExch((unsigned long long *)slot_exp, (unsigned long long)FLOW_DEAD);
+    if (!flow_absent(prev)) {
+        atomicAdd(&ctl->rep.live, 0ull - 1ull);
+        if (key != FLOW_EMPTY) atomicAdd(&ctl->rep.dead[cls], 1u);
+    }
+    return BNK_PKT_FILTER_DENY;
+}
+
+// ---- the last word on an opened packet ----
+// What the open kernel notes of a plaintext's headers (InnerHeader::of) is all that the checks behind the replay
+// window need, so that they do not go back to the packet: over the host link that would be a read per packet.
+//   x source address   y source port << 16 | destination port   z protocol | flags   w IPv4 total length
+constexpr uint32_t kInnerParses = 1u << 8; // filter.parse accepts it
+constexpr uint32_t kInnerWhole = 1u << 9;  // IPv4, 20 <= total length <= decrypted length
+struct VerdictArgs {
+    FilterTables ft;
+    const uint4 *inner;
+    const uint32_t *slot;
+    const uint32_t *allowed_ip;
+    uint8_t *status;
+    uint32_t *out_len;
+    uint8_t *host_status; // the results' pinned arrays, written besides
+    uint32_t *host_out_len;
+    long long now;
+    uint32_t n;
+    bool inner_check, check_inbound;
+};
+__device__ __forceinline__ void final_verdict(const VerdictArgs &v, uint32_t i) {
+    uint8_t st = *(volatile uint8_t *)&v.status[i];
+    uint32_t l = v.out_len[i];
+    if (st == BNK_PKT_OK && (v.inner_check || v.check_inbound)) {
+        const uint4 h = v.inner[i];
+        if (v.inner_check) { // cut to the IPv4 total length; the source must be the peer's address
+            if ((h.z & kInnerWhole) && h.x != 0 && h.x == v.allowed_ip[v.slot[i]]) l = h.w;
+            else st = BNK_PKT_BAD_INNER;
+        }
+        if (v.check_inbound && st == BNK_PKT_OK && v.ft.enforce) {
+            Parsed p;
+            p.src = h.x;
+            p.dst = 0;
+            p.sport = (uint16_t)(h.y >> 16);
+            p.dport = (uint16_t)h.y;
+            p.proto = (uint8_t)h.z;
+            st = (h.z & kInnerParses) ? filter_verdict(v.ft, p, v.now) : (uint8_t)BNK_PKT_FILTER_DENY;
+        }
+        v.status[i] = st;
+        v.out_len[i] = l;
+    }
+    if (v.host_status) {
+        v.host_status[i] = st;
+        v.host_out_len[i] = l;
+    }
+}

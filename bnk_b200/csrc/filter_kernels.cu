@@ -9,144 +9,26 @@
 // the table once per prefix length that occurs in the rule set (a 33-bit mask) and
 // scans only the allowances of prefixes that contain its source address.
 //
-// Flows.  Go's map[flowKey]time.Time becomes three open-addressing tables (tcp,
-// udp, icmp) keyed by remote address | remote port | local port, claimed with a
-// 64-bit compare-and-swap.  A deleted entry keeps its key with expiry FLOW_DEAD,
-// which behaves like an absent key for every later lookup.  The live-entry count
-// is kept exactly because the reference's expiry sweep depends on len(flows) > 4096.
+// Flows: see filter_device.cuh.
 // Go deletes map entries (filter.go:144, 202-208), so its map is bounded by the live
 // flows; here deleted entries are counted per class, and once they fill a quarter of
 // a class's region the surviving entries are re-inserted into the class's second,
 // empty region and the two swap roles (filter_flows_maintain), between two batches.
 #include <algorithm>
-#include <climits>
 #include <vector>
 
-#include "bnk_internal.cuh"
+#include "filter_device.cuh"
 
 namespace {
-
-constexpr unsigned long long FLOW_EMPTY = ~0ull;
-constexpr long long FLOW_DEAD = LLONG_MIN;      // the key is there, the entry is deleted
-constexpr long long FLOW_FRESH = LLONG_MIN + 1; // expiry of a slot no key has used yet
-__device__ __forceinline__ bool flow_absent(long long exp) { return exp <= FLOW_FRESH; }
-constexpr long long TTL_UDP = 30ll * 1000000000ll;  // filter.go:19
-constexpr long long TTL_TCP = 120ll * 1000000000ll; // filter.go:20
-constexpr long long TTL_ICMP = 30ll * 1000000000ll; // filter.go:21
-constexpr unsigned long long SWEEP_THRESHOLD = 4096; // filter.go:202
-
-// small device-side control block behind FilterTables::flow_live
-struct FlowCtl {
-    unsigned long long live;   // len(f.flows)
-    long long swept_at;        // `now` of the last completed sweep
-    int swept_valid;           // nothing was written at another `now` since that sweep
-    int sweep_now;             // decision for the sweep kernel of this batch
-    FlowReport rep;            // overflow flag and per-class slot counts; copied to the host after a batch
-    uint32_t moved;            // entries a compaction has re-inserted so far
-};
-
-__host__ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
-    z += 0x9e3779b97f4a7c15ull;
-    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
-    z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
-    return z ^ (z >> 31);
-}
-
-// Slot of a rule key: the key is a 32-bit address and a prefix length, so a 32-bit finaliser (two 32-bit
-// multiplies) spreads it; the 64-bit mixer above costs three times the instructions on a machine without a 64-bit
-// multiplier, and the check kernel hashes once per prefix length and packet.
-__host__ __device__ __forceinline__ uint32_t rule_hash(uint64_t key) {
-    uint32_t x = (uint32_t)key ^ ((uint32_t)(key >> 32) * 0x9e3779b1u);
-    x ^= x >> 16;
-    x *= 0x85ebca6bu;
-    x ^= x >> 13;
-    x *= 0xc2b2ae35u;
-    return x ^ (x >> 16);
-}
-
-__host__ __device__ __forceinline__ uint64_t rule_key(uint32_t len, uint32_t addr) {
-    const uint32_t mask = len == 0 ? 0u : 0xffffffffu << (32 - len);
-    return (1ull << 40) | ((uint64_t)len << 32) | (addr & mask);
-}
-
-struct Parsed {
-    uint32_t src, dst;
-    uint16_t sport, dport;
-    uint8_t proto;
-};
 
 // filter.go:71-106.  `p` is 16-byte aligned (packets start 16 bytes into a 16-aligned slot).
 __device__ __forceinline__ bool parse_ipv4(const uint8_t *p, uint32_t len, Parsed &out) {
     if (len < 20) return false;
     const uint4 w = *reinterpret_cast<const uint4 *>(p); // bytes 0..15
-    if (((w.x & 0xffu) >> 4) != 4u) return false;
-    const uint32_t ihl = (w.x & 0x0fu) * 4u;
-    if (ihl < 20u || len < ihl) return false;
-    out.proto = (uint8_t)((w.z >> 8) & 0xffu); // byte 9
-    out.src = __byte_perm(w.w, 0, 0x0123);     // bytes 12..15, big-endian
-    out.dst = __byte_perm(*reinterpret_cast<const uint32_t *>(p + 16), 0, 0x0123);
-    out.sport = 0;
-    out.dport = 0;
-    const uint32_t body = len - ihl;
-    if (out.proto == 6 || out.proto == 17) {
-        if (body < 4) return false;
-        const uint32_t ports = *reinterpret_cast<const uint32_t *>(p + ihl); // ihl is a multiple of 4
-        out.sport = (uint16_t)(((ports & 0xffu) << 8) | ((ports >> 8) & 0xffu));
-        out.dport = (uint16_t)((((ports >> 16) & 0xffu) << 8) | (ports >> 24));
-        return true;
-    }
-    if (out.proto == 1) return body >= 1;
-    return false;
-}
-
-__device__ __forceinline__ int proto_class(uint8_t proto) { return proto == 6 ? 0 : (proto == 17 ? 1 : 2); }
-__device__ __forceinline__ long long flow_ttl(uint8_t proto) { // filter.go:108-117
-    return proto == 6 ? TTL_TCP : (proto == 1 ? TTL_ICMP : TTL_UDP);
-}
-__device__ __forceinline__ unsigned long long flow_key(uint32_t remote, uint16_t rport, uint16_t lport) {
-    return ((unsigned long long)remote << 32) | ((unsigned long long)rport << 16) | lport;
-}
-
-// any allowance matches?  acl.go:149-172 over the indexed table
-// (Fetching the first slot of four prefix lengths before looking at any of them, to overlap the round trips, was
-// measured: 10 % slower on configuration 3, where nearly half the packets match at one of the first lengths.)
-__device__ __forceinline__ bool rules_allow(const FilterTables &ft, const Parsed &p) {
-    if (ft.rule_slots == 0) return false;
-    // longest prefixes first: acl.Compile emits /32s (acl.go:98), so a packet that some rule admits is most often
-    // admitted at the first probe; any match allows, the order changes no verdict
-    uint64_t lens = ft.len_mask;
-    while (lens) {
-        const uint32_t len = 63u - (uint32_t)__clzll((long long)lens);
-        lens &= ~(1ull << len);
-        const uint64_t key = rule_key(len, p.src);
-        uint32_t h = rule_hash(key) & (ft.rule_slots - 1);
-        for (uint32_t probe = 0; probe < ft.rule_slots; probe++) {
-            const uint64_t k = ft.rule_keys[h];
-            if (k == 0) break;
-            if (k == key) {
-                const uint2 span = ft.rule_span[h];
-                for (uint32_t e = 0; e < span.y; e++) {
-                    const uint64_t ent = ft.rule_entries[span.x + e];
-                    if ((uint8_t)(ent >> 32) != p.proto) continue;
-                    if (p.proto == 1) return true;
-                    const uint16_t first = (uint16_t)(ent >> 16), last = (uint16_t)ent;
-                    if (p.dport >= first && p.dport <= last) return true;
-                }
-                break;
-            }
-            h = (h + 1) & (ft.rule_slots - 1);
-        }
-    }
-    return false;
-}
-
-// One atomic per group of lanes that add to the same counter at the same point of the code, instead of one per
-// lane: a batch of new flows otherwise sends a few hundred thousand atomics to two addresses (300,000 fresh flows
-// took 0.7 ms that way).
-template <typename T>
-__device__ __forceinline__ void add_one_aggregated(T *counter) {
-    const unsigned same = __match_any_sync(__activemask(), (unsigned long long)(uintptr_t)counter);
-    if ((threadIdx.x & 31u) == (unsigned)(__ffs(same) - 1)) atomicAdd(counter, (T)__popc(same));
+    const uint32_t at = parse_ipv4_words(w.x, w.z, w.w, *reinterpret_cast<const uint32_t *>(p + 16), len, out);
+    if (at == kParseBad) return false;
+    if (at) parse_ports(*reinterpret_cast<const uint32_t *>(p + at), out);
+    return true;
 }
 
 // ---- NoteOutbound, filter.go:189-209 ----------------------------------------------------
@@ -160,74 +42,79 @@ __global__ void filter_note_kernel(FilterTables ft, const uint8_t *ring, const u
     if ((o & 15u) || (uint64_t)o + 16u + l > ring_bytes) return;
     Parsed p;
     if (!parse_ipv4(ring + o + 16, l, p)) return;
-    FlowCtl *ctl = reinterpret_cast<FlowCtl *>(ft.flow_live);
-    const long long exp = now + flow_ttl(p.proto);
-    const int cls = proto_class(p.proto);
-    const unsigned long long key = flow_key(p.dst, p.dport, p.sport);
-    if (!(ctl->swept_valid && ctl->swept_at == now)) ctl->swept_valid = 0;
-    if (key == FLOW_EMPTY) {
-        const long long prev = (long long)atomicExch((unsigned long long *)&ft.flow_special_exp[cls],
-                                                     (unsigned long long)exp);
-        if (flow_absent(prev)) atomicAdd(&ctl->live, 1ull);
-        return;
-    }
-    unsigned long long *keys = (unsigned long long *)ft.flow_keys + flow_region(ft, cls);
-    long long *exps = ft.flow_exp + flow_region(ft, cls);
-    uint32_t h = (uint32_t)mix64(key) & (ft.flow_capacity - 1);
-    for (uint32_t probe = 0; probe < ft.flow_capacity; probe++) {
-        const unsigned long long old = atomicCAS(&keys[h], FLOW_EMPTY, key);
-        if (old == FLOW_EMPTY || old == key) {
-            if (old == FLOW_EMPTY) add_one_aggregated(&ctl->rep.used[cls]);
-            const long long prev = (long long)atomicExch((unsigned long long *)&exps[h], (unsigned long long)exp);
-            if (flow_absent(prev)) add_one_aggregated(&ctl->live);
-            if (prev == FLOW_DEAD) atomicSub(&ctl->rep.dead[cls], 1u); // a deleted entry is back
-            return;
-        }
-        h = (h + 1) & (ft.flow_capacity - 1);
-    }
-    atomicAdd(ft.flow_error, 1); // table full: the flow is not recorded, the host reports BNK_EFULL
+    FlowNote note;
+    note.begin(ft, p, now);
+    note.place(ft);
+    note.count(ft);
 }
 
-// The reference sweeps expired flows whenever the map holds more than 4096 entries after an
-// insert.  Within one batch (one `now`) that equals: insert everything, then sweep once if
-// the count exceeds the threshold.  A repeat sweep at an unchanged `now` finds nothing.
-__global__ void filter_sweep_decide_kernel(FilterTables ft, long long now) {
+// The reference sweeps expired flows whenever the map holds more than 4096 entries after an insert.  Within one batch
+// (one `now`) that equals: insert everything, then sweep once if the count exceeds the threshold.  A sweep that
+// starts at or before the floor of the expiries would find nothing and does not walk the table; the host, which
+// knows a lower bound of the floor, does not even launch it (flow_note_begins).  One walk reads the expiries of the
+// regions in use (8 bytes a slot) and leaves the floor at the lowest expiry it has seen, or at what an insert that
+// ran beside it can have written.
+__global__ void __launch_bounds__(256) filter_sweep_kernel(const __grid_constant__ FilterTables ft, long long now, FlowReport *report, Done done) {
     let_next_kernel_start();
     wait_for_kernel_in_front();
-    FlowCtl *ctl = reinterpret_cast<FlowCtl *>(ft.flow_live);
-    ctl->sweep_now = (ctl->live > SWEEP_THRESHOLD && !(ctl->swept_valid && ctl->swept_at == now)) ? 1 : 0;
-}
-__global__ void filter_sweep_kernel(FilterTables ft, long long now) {
-    let_next_kernel_start();
-    wait_for_kernel_in_front();
-    FlowCtl *ctl = reinterpret_cast<FlowCtl *>(ft.flow_live);
-    if (!ctl->sweep_now) return;
-    // both regions of every class are walked; the one not in use holds nothing but fresh slots
-    const size_t total = (size_t)6 * ft.flow_capacity;
-    unsigned long long dropped = 0;
-    uint32_t dead[3] = {0, 0, 0};
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total + 3; k += (size_t)gridDim.x * blockDim.x) {
-        long long *e = k < total ? &ft.flow_exp[k] : &ft.flow_special_exp[k - total];
-        const long long exp = *e;
-        if (!flow_absent(exp) && now > exp) {
-            *e = FLOW_DEAD;
-            dropped++;
-            if (k < total) dead[k / ((size_t)2 * ft.flow_capacity)]++;
-        }
+    FlowCtl *const ctl = flow_ctl(ft);
+    __shared__ unsigned long long dropped_s;
+    __shared__ long long floor_s;
+    __shared__ uint32_t dead_s[3];
+    if (threadIdx.x == 0) {
+        dropped_s = 0;
+        floor_s = LLONG_MAX;
+        dead_s[0] = dead_s[1] = dead_s[2] = 0;
     }
-    if (dropped) atomicAdd(&ctl->live, 0ull - dropped);
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-        if (dead[c]) atomicAdd(&ctl->rep.dead[c], dead[c]);
-}
-__global__ void filter_sweep_finish_kernel(FilterTables ft, long long now) {
-    let_next_kernel_start();
-    wait_for_kernel_in_front();
-    FlowCtl *ctl = reinterpret_cast<FlowCtl *>(ft.flow_live);
-    if (ctl->sweep_now) {
-        ctl->swept_at = now;
-        ctl->swept_valid = 1;
-        ctl->sweep_now = 0;
+    __syncthreads();
+    // all CTAs decide alike: neither value changes before the last of them has finished
+    const bool walk = ctl->rep.live > SWEEP_THRESHOLD && now > ctl->rep.floor;
+    if (walk) {
+        const size_t cap = ft.flow_capacity, total = 3 * cap;
+        unsigned long long dropped = 0;
+        long long floor = LLONG_MAX;
+        for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total + 3; k += (size_t)gridDim.x * blockDim.x) {
+            const int cls = k < total ? (int)(k / cap) : 0;
+            long long *const e = k < total ? &ft.flow_exp[flow_region(ft, cls) + (k - cls * cap)] : &ft.flow_special_exp[k - total];
+            const long long exp = *e;
+            if (flow_absent(exp)) continue;
+            if (now > exp) {
+                *e = FLOW_DEAD;
+                dropped++;
+                if (k < total) atomicAdd(&dead_s[cls], 1u);
+            } else if (exp < floor) {
+                floor = exp;
+            }
+        }
+        if (dropped) atomicAdd(&dropped_s, dropped);
+        atomicMin(&floor_s, floor);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (walk) {
+            atomicAdd(&ctl->dropped, dropped_s);
+            atomicMin(&ctl->next_floor, floor_s);
+            for (int c = 0; c < 3; c++)
+                if (dead_s[c]) atomicAdd(&ctl->rep.dead[c], dead_s[c]);
+        }
+        __threadfence();
+        if (atomicAdd(&ctl->ticket, 1u) + 1u == gridDim.x) {
+            __threadfence();
+            if (walk) {
+                atomicAdd(&ctl->rep.live, 0ull - *(volatile unsigned long long *)&ctl->dropped);
+                const long long seen = *(volatile long long *)&ctl->next_floor, beside = now + TTL_LEAST;
+                ctl->rep.floor = seen < beside ? seen : beside;
+                ctl->dropped = 0;
+                ctl->next_floor = LLONG_MAX;
+            }
+            ctl->ticket = 0;
+            __threadfence();
+            if (report) flow_report(ctl, report);
+            if (done.flag) {
+                __threadfence_system();
+                *(volatile uint32_t *)done.flag = done.value;
+            }
+        }
     }
 }
 
@@ -253,52 +140,7 @@ __global__ void filter_check_kernel(FilterTables ft, const uint8_t *ring, const 
         status[i] = BNK_PKT_FILTER_DENY;
         return;
     }
-    if (rules_allow(ft, p)) {
-        status[i] = BNK_PKT_OK;
-        return;
-    }
-    // reply to a flow this node opened?  key mirrors NoteOutbound's
-    FlowCtl *ctl = reinterpret_cast<FlowCtl *>(ft.flow_live);
-    const int cls = proto_class(p.proto);
-    const unsigned long long key = flow_key(p.src, p.sport, p.dport);
-    long long *slot_exp = nullptr;
-    if (ft.flow_capacity == 0) {
-        status[i] = BNK_PKT_FILTER_DENY;
-        return;
-    }
-    if (key == FLOW_EMPTY) {
-        slot_exp = &ft.flow_special_exp[cls];
-    } else {
-        const unsigned long long *keys = (const unsigned long long *)ft.flow_keys + flow_region(ft, cls);
-        uint32_t h = (uint32_t)mix64(key) & (ft.flow_capacity - 1);
-        for (uint32_t probe = 0; probe < ft.flow_capacity; probe++) {
-            const unsigned long long k = keys[h];
-            if (k == FLOW_EMPTY) break;
-            if (k == key) {
-                slot_exp = ft.flow_exp + flow_region(ft, cls) + h;
-                break;
-            }
-            h = (h + 1) & (ft.flow_capacity - 1);
-        }
-    }
-    uint8_t verdict = BNK_PKT_FILTER_DENY;
-    if (slot_exp) {
-        const long long exp = *(volatile long long *)slot_exp;
-        if (!flow_absent(exp)) {
-            if (now < exp) { // strict: time.Before
-                *(volatile long long *)slot_exp = now + flow_ttl(p.proto); // keep-alive on traffic
-                if (!(ctl->swept_valid && ctl->swept_at == now)) ctl->swept_valid = 0;
-                verdict = BNK_PKT_OK;
-            } else {
-                const long long prev = (long long)atomicExch((unsigned long long *)slot_exp, (unsigned long long)FLOW_DEAD);
-                if (!flow_absent(prev)) {
-                    atomicAdd(&ctl->live, 0ull - 1ull);
-                    if (key != FLOW_EMPTY) atomicAdd(&ctl->rep.dead[cls], 1u);
-                }
-            }
-        }
-    }
-    status[i] = verdict;
+    status[i] = filter_verdict(ft, p, now);
 }
 
 __global__ void flows_fill_kernel(FilterTables ft) {
@@ -309,8 +151,9 @@ __global__ void flows_fill_kernel(FilterTables ft) {
     }
     if (blockIdx.x == 0 && threadIdx.x < 3) ft.flow_special_exp[threadIdx.x] = FLOW_FRESH;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        FlowCtl *ctl = reinterpret_cast<FlowCtl *>(ft.flow_live);
-        *ctl = FlowCtl{};
+        FlowCtl v{};
+        v.rep.floor = v.next_floor = LLONG_MAX;
+        *flow_ctl(ft) = v;
     }
 }
 
@@ -318,7 +161,7 @@ __global__ void flows_fill_kernel(FilterTables ft) {
 // other region, which is empty; the host then swaps the roles (filter_flows_maintain).  Expired entries that no
 // sweep or lookup has deleted yet move along: they still count in len(f.flows), which decides the next sweep.
 __global__ void flows_compact_kernel(FilterTables ft, int cls) {
-    FlowCtl *ctl = reinterpret_cast<FlowCtl *>(ft.flow_live);
+    FlowCtl *ctl = flow_ctl(ft);
     const size_t from = flow_region(ft, cls), to = ((size_t)cls * 2 + (ft.flow_half[cls] ^ 1)) * ft.flow_capacity;
     unsigned long long *keys = (unsigned long long *)ft.flow_keys + to;
     long long *exps = ft.flow_exp + to;
@@ -335,7 +178,7 @@ __global__ void flows_compact_kernel(FilterTables ft, int cls) {
             else h = (h + 1) & (ft.flow_capacity - 1);
         }
         if (!placed) {
-            atomicAdd(ft.flow_error, 1);
+            atomicAdd(&ctl->rep.error, 1);
             continue;
         }
         exps[h] = exp;
@@ -345,7 +188,7 @@ __global__ void flows_compact_kernel(FilterTables ft, int cls) {
 }
 // wipes the region the class has just left and books the move
 __global__ void flows_compact_finish_kernel(FilterTables ft, int cls) {
-    FlowCtl *ctl = reinterpret_cast<FlowCtl *>(ft.flow_live);
+    FlowCtl *ctl = flow_ctl(ft);
     const size_t from = flow_region(ft, cls);
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < ft.flow_capacity; k += (size_t)gridDim.x * blockDim.x) {
         ft.flow_keys[from + k] = FLOW_EMPTY;
@@ -409,7 +252,6 @@ cudaError_t filter_tables_alloc(bnk_ctx *ctx) {
     FlowCtl *ctl = nullptr;
     if ((e = cudaMalloc(&ctl, sizeof(FlowCtl))) != cudaSuccess) return e;
     ft.flow_live = reinterpret_cast<unsigned long long *>(ctl);
-    ft.flow_error = &ctl->rep.error;
     if ((e = cudaMalloc(&ft.flow_special_exp, 3 * sizeof(long long))) != cudaSuccess) return e;
     if (cap) {
         if ((e = cudaMalloc(&ft.flow_keys, (size_t)6 * cap * sizeof(uint64_t))) != cudaSuccess) return e;
@@ -450,6 +292,12 @@ cudaError_t filter_flows_clear(bnk_ctx *ctx, cudaStream_t s) {
     ctx->ft.flow_half[0] = ctx->ft.flow_half[1] = ctx->ft.flow_half[2] = 0;
     for (auto &h : ctx->flow_dead_hint) h = 0;
     ctx->flow_errors_seen = 0;
+    {
+        std::lock_guard<std::mutex> g(ctx->flow_mu);
+        ctx->flow_floor = LLONG_MAX;
+        ctx->flow_live_most = 0;
+        ctx->flow_epoch++;
+    }
     flows_fill_kernel<<<ctx->sm_count * 4, 256, 0, s>>>(ctx->ft);
     ctx->launches += 1;
     cudaError_t e = cudaGetLastError();
@@ -461,7 +309,7 @@ cudaError_t filter_flow_stats(bnk_ctx *ctx, uint64_t *live, uint32_t used[3], ui
     FlowCtl ctl;
     cudaError_t e = cudaMemcpy(&ctl, ctx->ft.flow_live, sizeof ctl, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return e;
-    *live = ctl.live;
+    *live = ctl.rep.live;
     for (int c = 0; c < 3; c++) {
         used[c] = ctl.rep.used[c];
         dead[c] = ctl.rep.dead[c];
@@ -494,7 +342,6 @@ cudaError_t flows_download(bnk_ctx *ctx, FlowTablesHost &h) {
 }
 int class_of(uint8_t proto) { return proto == 6 ? 0 : (proto == 17 ? 1 : 2); }
 uint8_t proto_of(int cls) { return cls == 0 ? 6 : (cls == 1 ? 17 : 1); }
-bool absent_host(long long exp) { return exp <= FLOW_FRESH; }
 } // namespace
 
 int filter_flows_export(bnk_ctx *ctx, bnk_flow_entry *out, size_t capacity, size_t *count) {
@@ -517,8 +364,8 @@ int filter_flows_export(bnk_ctx *ctx, bnk_flow_entry *out, size_t capacity, size
     for (int cls = 0; cls < 3; cls++) {
         const size_t base = flow_region(ft, cls);
         for (size_t k = 0; k < ft.flow_capacity; k++)
-            if (h.keys[base + k] != FLOW_EMPTY && !absent_host(h.exp[base + k])) emit(cls, h.keys[base + k], h.exp[base + k]);
-        if (!absent_host(h.special[cls])) emit(cls, FLOW_EMPTY, h.special[cls]);
+            if (h.keys[base + k] != FLOW_EMPTY && !flow_absent(h.exp[base + k])) emit(cls, h.keys[base + k], h.exp[base + k]);
+        if (!flow_absent(h.special[cls])) emit(cls, FLOW_EMPTY, h.special[cls]);
     }
     *count = n;
     return BNK_SUCCESS;
@@ -532,11 +379,11 @@ int filter_flows_import(bnk_ctx *ctx, const bnk_flow_entry *entries, size_t n) {
     for (size_t i = 0; i < n; i++) {
         const bnk_flow_entry &e = entries[i];
         if (e.proto != 6 && e.proto != 17 && e.proto != 1) return BNK_EINVAL;
-        if (absent_host(e.expiry_unix_ns)) return BNK_EINVAL;
+        if (flow_absent(e.expiry_unix_ns)) return BNK_EINVAL;
         const int cls = class_of(e.proto);
         const unsigned long long key = ((unsigned long long)e.remote_addr << 32) | ((unsigned long long)e.remote_port << 16) | e.local_port;
         if (key == FLOW_EMPTY) {
-            if (absent_host(h.special[cls])) h.ctl.live++;
+            if (flow_absent(h.special[cls])) h.ctl.rep.live++;
             h.special[cls] = e.expiry_unix_ns;
             continue;
         }
@@ -552,14 +399,20 @@ int filter_flows_import(bnk_ctx *ctx, const bnk_flow_entry *entries, size_t n) {
                 h.ctl.rep.used[cls]++;
             }
             long long &x = h.exp[base + at];
-            if (absent_host(x)) h.ctl.live++;
+            if (flow_absent(x)) h.ctl.rep.live++;
             if (x == FLOW_DEAD) h.ctl.rep.dead[cls]--;
             x = e.expiry_unix_ns;
             placed = true;
         }
         if (!placed) return BNK_EFULL;
     }
-    h.ctl.swept_valid = 0;
+    h.ctl.rep.floor = LLONG_MIN; // unknown: the next sweep finds it
+    {
+        std::lock_guard<std::mutex> g(ctx->flow_mu);
+        ctx->flow_floor = LLONG_MIN;
+        ctx->flow_live_most = h.ctl.rep.live;
+        ctx->flow_epoch++;
+    }
     const size_t total = (size_t)6 * cap;
     cudaError_t e = cudaSuccess;
     if (total) {
@@ -575,6 +428,45 @@ cudaError_t launch_flow_report(bnk_batch *b, cudaStream_t s) {
     const FlowCtl *ctl = reinterpret_cast<const FlowCtl *>(b->ctx->ft.flow_live);
     b->flow_reported = true;
     return cudaMemcpyAsync(b->h_flow, &ctl->rep, sizeof(FlowReport), cudaMemcpyDeviceToHost, s);
+}
+
+static long long earliest_expiry(long long now) { return now > LLONG_MAX - TTL_LEAST ? LLONG_MAX : now + TTL_LEAST; }
+static void flow_work_begins(bnk_batch *b) {
+    b->flow_epoch = ++b->ctx->flow_epoch;
+    if (!b->flow_in_flight) b->ctx->flow_in_flight++;
+    b->flow_in_flight = true;
+}
+bool flow_note_begins(bnk_batch *b, uint32_t n, long long now) {
+    bnk_ctx *ctx = b->ctx;
+    std::lock_guard<std::mutex> g(ctx->flow_mu);
+    flow_work_begins(b);
+    ctx->flow_live_most += n;
+    const bool sweep = ctx->flow_live_most > SWEEP_THRESHOLD && now > ctx->flow_floor;
+    ctx->flow_floor = std::min(ctx->flow_floor, earliest_expiry(now));
+    return sweep;
+}
+void flow_check_begins(bnk_batch *b, long long now) { // a lookup keeps its flow alive: it writes an expiry too
+    bnk_ctx *ctx = b->ctx;
+    std::lock_guard<std::mutex> g(ctx->flow_mu);
+    flow_work_begins(b);
+    ctx->flow_floor = std::min(ctx->flow_floor, earliest_expiry(now));
+}
+void flow_work_over(bnk_batch *b) {
+    bnk_ctx *ctx = b->ctx;
+    std::lock_guard<std::mutex> g(ctx->flow_mu);
+    if (b->flow_in_flight) ctx->flow_in_flight--;
+    b->flow_in_flight = false;
+    if (!b->flow_reported || ctx->flow_epoch != b->flow_epoch || ctx->flow_in_flight != 0) return;
+    ctx->flow_floor = b->h_flow->floor;
+    ctx->flow_live_most = b->h_flow->live;
+}
+cudaError_t launch_flow_sweep(bnk_batch *b, long long now, const Done &done, cudaStream_t s) {
+    bnk_ctx *ctx = b->ctx;
+    const size_t slots = (size_t)3 * ctx->ft.flow_capacity;
+    const uint32_t grid = (uint32_t)std::min<size_t>(ctx->sm_count * 4, (slots + 1023) / 1024);
+    b->flow_reported = true;
+    ctx->launches += 1;
+    return launch_after_kernel(filter_sweep_kernel, dim3(grid), dim3(256), s, ctx->ft, now, b->h_flow, done);
 }
 
 // Deleted entries keep their slots, so a class whose flows come and go (every connection brings a new source
@@ -736,11 +628,7 @@ cudaError_t launch_filter_note(bnk_batch *b, uint32_t n, long long now_ns, cudaS
     if (n == 0 || !ctx->ft.enforce || ctx->ft.flow_capacity == 0) return cudaSuccess; // filter.go:192-194
     launch_kernel(n <= dependent_launch_up_to(), filter_note_kernel, dim3((n + 255) / 256), dim3(256), s, ctx->ft,
         b->dev.ring, b->dev.off, b->dev.len, n, b->ring_bytes, now_ns);
-    launch_kernel(n <= dependent_launch_up_to(), filter_sweep_decide_kernel, dim3(1), dim3(1), s, ctx->ft, now_ns);
-    launch_kernel(n <= dependent_launch_up_to(), filter_sweep_kernel, dim3(ctx->sm_count * 4), dim3(256), s, ctx->ft,
-        now_ns);
-    launch_kernel(n <= dependent_launch_up_to(), filter_sweep_finish_kernel, dim3(1), dim3(1), s, ctx->ft, now_ns);
-    ctx->launches += 4;
+    ctx->launches += 1;
     return cudaGetLastError();
 }
 

@@ -10,7 +10,13 @@
 // the walk has a parallel form: a packet's nonce is the peer's counter plus its
 // rank in the peer's run, and the window's verdicts over a stretch of packets
 // follow in closed form from the state at the start of the stretch.
-#include "bnk_internal.cuh"
+#include <algorithm>
+
+#include <cooperative_groups.h>
+
+#include "filter_device.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -26,20 +32,13 @@ constexpr uint32_t kBatchMaxChunks = BNK_SORT_MAX_CHUNKS; // ~2 CTAs per SM: eno
 
 struct SortKeySrc {
     const uint32_t *slot;
-    const uint8_t *status;
     uint32_t max_slots;
-    int only_status_ok; // 1: packets whose status is not OK/KEEPALIVE do not take part
 };
 
 // Key of packet i: its keypair slot, or max_slots ("takes no part", sorts last).
 __device__ __forceinline__ uint32_t slot_key(const SortKeySrc &k, uint32_t i) {
     const uint32_t s = k.slot[i];
-    if (s >= k.max_slots) return k.max_slots;
-    if (k.only_status_ok) {
-        const uint8_t st = k.status[i];
-        if (st != BNK_PKT_OK && st != BNK_PKT_KEEPALIVE) return k.max_slots;
-    }
-    return s;
+    return s < k.max_slots ? s : k.max_slots;
 }
 
 // one shared-memory add per distinct digit in the warp instead of one per lane
@@ -247,10 +246,6 @@ __device__ __forceinline__ uint32_t run_start(const uint32_t *keys, uint32_t j) 
     }
     return lo;
 }
-__device__ __forceinline__ uint64_t saturating_counter(uint64_t base, uint32_t k) {
-    const uint64_t c = base + k;
-    return (c < base || c > BNK_REJECT_AFTER_MESSAGES) ? BNK_REJECT_AFTER_MESSAGES : c;
-}
 __global__ void assign_counters_kernel(const uint32_t *keys, const uint32_t *order, uint32_t n, uint32_t max_slots,
                                        const uint64_t *send_counter, uint64_t *counter_out) {
     let_next_kernel_start();
@@ -290,7 +285,7 @@ __global__ void advance_counters_kernel(const uint32_t *keys, uint32_t n, uint32
 //   "repeats an earlier one"    the lowest grouped position holding the same (peer, counter), found with a
 //                               hash table of positions; built only when some packet of the batch lies behind
 //                               its M_j inside the window, which in-order traffic never does.
-// Up to 1024 packets all of this runs in the CTA that sorted them (group_small_kernel); beyond, as kernels in
+// Up to kGroupMax packets all of this runs in the cluster that sorted them (group_kernel); beyond, as kernels in
 // stream order: scan_tiles (also lays the counters out in grouped order), scan_carry, classify, advance (new
 // last, clears), hash_clear, hash_insert, finish (duplicate look-up, verdicts, marks).
 constexpr uint32_t kScanTile = 1024; // grouped positions per CTA: 256 threads x 4
@@ -346,32 +341,40 @@ __device__ __forceinline__ SegMax seg_block_exclusive(SegMax mine, SegMax *part,
     }
     return seg_combine(before, ex);
 }
-// Four consecutive grouped positions per thread.  e[k] = maximum of the values of the same run that lie in
-// front of item k (`carry` stands for what lies in front of the tile); total = the tile as one span.
-__device__ __forceinline__ void tile_running_max(const bool head[4], const uint64_t v[4], uint64_t carry,
-                                                 uint64_t e[4], SegMax *part, SegMax &total) {
+// ITEMS consecutive grouped positions per thread.  e[k] = maximum of the values of the same run that lie in
+// front of item k; total = the tile as one span; what lies in front of the tile comes in with tile_carry.
+struct TileMax {
+    SegMax ex;
+    uint32_t headed; // bit k: a head lies at or before item k inside this thread
+};
+template <int ITEMS, int NW>
+__device__ __forceinline__ TileMax tile_running_max(const bool (&head)[ITEMS], const uint64_t (&v)[ITEMS],
+                                                    uint64_t (&e)[ITEMS], SegMax *part, SegMax &total) {
     SegMax run{0u, 0ull};
-    uint32_t headed = 0; // bit k: a head lies at or before item k inside this thread
+    TileMax t{SegMax{0u, 0ull}, 0u};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         if (head[k]) run = SegMax{1u, 0ull};
         e[k] = run.m;
-        headed |= run.f << k;
+        t.headed |= run.f << k;
         if (v[k] > run.m) run.m = v[k];
     }
-    const SegMax ex = seg_block_exclusive<8>(run, part, total);
-    const uint64_t front = ex.f ? ex.m : (carry > ex.m ? carry : ex.m);
+    t.ex = seg_block_exclusive<NW>(run, part, total);
+    return t;
+}
+template <int ITEMS>
+__device__ __forceinline__ void tile_carry(const TileMax &t, uint64_t carry, uint64_t (&e)[ITEMS]) {
+    const uint64_t front = t.ex.f ? t.ex.m : (carry > t.ex.m ? carry : t.ex.m);
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if (!((headed >> k) & 1u) && front > e[k]) e[k] = front;
+    for (int k = 0; k < ITEMS; ++k)
+        if (!((t.headed >> k) & 1u) && front > e[k]) e[k] = front;
 }
 
 // Counter of grouped position p, or kReplayNoPart.  Authenticated packets at or beyond the message limit are
 // refused here: their verdict does not depend on the window and they leave no trace in it.
-__device__ __forceinline__ uint64_t replay_gather(const ReplayArgs &a, uint32_t p, uint32_t slot) {
+__device__ __forceinline__ uint64_t replay_gather(const ReplayArgs &a, uint32_t p, uint32_t slot, uint32_t pkt) {
     uint64_t c = kReplayNoPart;
     if (slot < a.max_slots) {
-        const uint32_t pkt = a.order[p];
         const uint8_t st = a.status[pkt];
         if (st == BNK_PKT_OK || st == BNK_PKT_KEEPALIVE) {
             c = a.counter[pkt];
@@ -386,7 +389,7 @@ __device__ __forceinline__ uint64_t replay_gather(const ReplayArgs &a, uint32_t 
 }
 // Verdict of position p as far as it can be told without the duplicate search; the last packet of a run also
 // leaves the peer's next `last`.  e = running maximum of the run in front of p.
-__device__ __forceinline__ uint8_t replay_classify(const ReplayArgs &a, uint32_t p, uint32_t slot, uint64_t c, uint64_t e) {
+__device__ __forceinline__ uint8_t replay_classify(const ReplayArgs &a, uint32_t p, uint32_t slot, bool tail, uint64_t c, uint64_t e) {
     if (slot >= a.max_slots) return RP_NOPART;
     const uint64_t rmask = a.ring_blocks - 1, window = (uint64_t)(a.ring_blocks - 1) * 64u;
     const uint64_t last = a.replay_last[slot];
@@ -402,7 +405,7 @@ __device__ __forceinline__ uint8_t replay_classify(const ReplayArgs &a, uint32_t
             st = RP_REJECT;
         else st = RP_PENDING;
     }
-    if (p + 1 == a.n || a.keys[p + 1] != slot) a.replay_next[slot] = top;
+    if (tail) a.replay_next[slot] = top;
     return st;
 }
 // Warp-wide over 32 consecutive positions (p = this lane's): the peers whose run ends here move their window.
@@ -509,8 +512,8 @@ __device__ __forceinline__ void replay_finish_warp(const ReplayArgs &a, uint32_t
 // The tile of the calling CTA (thread t: positions base..base+3): counters gathered when GATHER, else read
 // back; running maximum with `carry` in front; returns the tile as one span.
 template <bool GATHER>
-__device__ __forceinline__ SegMax replay_tile(const ReplayArgs &a, uint32_t base, uint64_t carry, uint32_t slot[4],
-                                              uint64_t c[4], uint64_t e[4], SegMax *part) {
+__device__ __forceinline__ SegMax replay_tile(const ReplayArgs &a, uint32_t base, uint64_t carry, uint32_t (&slot)[4],
+                                              uint64_t (&c)[4], uint64_t (&e)[4], SegMax *part) {
     bool head[4];
     uint64_t v[4];
 #pragma unroll
@@ -523,12 +526,13 @@ __device__ __forceinline__ SegMax replay_tile(const ReplayArgs &a, uint32_t base
         if (p < a.n) {
             slot[k] = a.keys[p];
             head[k] = p == 0 || a.keys[p - 1] != slot[k];
-            c[k] = GATHER ? replay_gather(a, p, slot[k]) : a.sorted_counter[p];
+            c[k] = GATHER ? replay_gather(a, p, slot[k], a.order[p]) : a.sorted_counter[p];
             if (c[k] != kReplayNoPart) v[k] = c[k];
         }
     }
     SegMax total;
-    tile_running_max(head, v, carry, e, part, total);
+    const TileMax t = tile_running_max<4, 8>(head, v, e, part, total);
+    tile_carry<4>(t, carry, e);
     return total;
 }
 
@@ -576,7 +580,8 @@ __global__ void __launch_bounds__(256) replay_classify_kernel(ReplayArgs a, cons
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         if (base + k >= a.n) continue;
-        const uint8_t st = replay_classify(a, base + k, slot[k], c[k], e[k]);
+        const bool tail = base + k + 1 == a.n || a.keys[base + k + 1] != slot[k];
+        const uint8_t st = replay_classify(a, base + k, slot[k], tail, c[k], e[k]);
         a.state[base + k] = st;
         pending |= st == RP_PENDING;
     }
@@ -605,100 +610,123 @@ __global__ void __launch_bounds__(256) replay_finish_kernel(ReplayArgs a) {
     wait_for_kernel_in_front();
     replay_finish_warp(a, blockIdx.x * blockDim.x + threadIdx.x);
 }
-// All of the above for one tile, by the CTA that holds it (n <= kScanTile, 256 threads).
-__device__ __forceinline__ void replay_one_cta(const ReplayArgs &a, SegMax *part) {
-    const uint32_t tid = threadIdx.x;
-    uint32_t slot[4];
-    uint64_t c[4], e[4];
-    replay_tile<true>(a, tid * 4u, 0ull, slot, c, e, part);
-    bool pending = false;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (tid * 4u + k >= a.n) continue;
-        const uint8_t st = replay_classify(a, tid * 4u + k, slot[k], c[k], e[k]);
-        a.state[tid * 4u + k] = st;
-        pending |= st == RP_PENDING;
-    }
-    const bool any_pending = __syncthreads_or(pending); // also: every verdict and next `last` is written
-    for (uint32_t p = tid; p < kScanTile; p += 256u) replay_advance_warp(a, p);
-    if (any_pending) {
-        for (uint32_t i = tid; i <= a.mask; i += 256u) a.table[i] = kHashEmpty;
-        __syncthreads();
-        for (uint32_t p = tid; p < kScanTile; p += 256u) replay_hash_insert_warp(a, p, p < a.n && a.state[p] != RP_NOPART);
-    }
-    __syncthreads(); // clears before marks, inserts before look-ups
-    for (uint32_t p = tid; p < kScanTile; p += 256u) replay_finish_warp(a, p);
+// The last checks alone, one thread per packet.
+__global__ void __launch_bounds__(256) verdict_kernel(const __grid_constant__ VerdictArgs v, Done done) {
+    let_next_kernel_start();
+    wait_for_kernel_in_front();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < v.n) final_verdict(v, i);
+    signal_done(done, [] {});
 }
 
-// --- the whole sort in one CTA, for batches of up to 1024 packets ----------------------
-// Same three steps per digit as above, but keys and indices ping-pong between shared-memory buffers
-// and all passes run inside one launch: a 128-packet batch pays one launch instead of six.
-constexpr uint32_t kSmallMax = 1024;
-// Send counters in the same launch (counter_out != nullptr): with one CTA a barrier separates the reads of
-// the peers' counters from their advance, which takes two launches for larger batches.
-// The replay window of a small batch can follow in the same launch as well (replay_last != nullptr).
-struct SmallCounters {
-    uint64_t *send_counter; // [max_slots]
-    uint64_t *counter_out;  // per packet
-    uint32_t max_slots;
+// --- the whole ordering work of a batch of up to kGroupMax packets in one launch --------
+// The same stable radix sort, the counters or the replay window behind it and the last checks behind that, by one
+// cluster of up to 8 CTAs of 512 threads with 1 to 8 packets a thread.  As kernels in stream order this is up to
+// twenty launches of a few microseconds' work each, and a batch of a few thousand packets spent more time in front of
+// and between them than in them (a 4096-packet open with every check: 20 launches).  Keys and indices ping-pong
+// between shared-memory buffers; the CTAs read each other's digit totals, and the scatter writes into the buffer of
+// the CTA that a position belongs to, through distributed shared memory; cluster barriers stand where kernel
+// boundaries stood.  Up to 256 packets the sort is a count: the place of a packet is the number of packets with a
+// lower key, or the same key and a lower index.
+constexpr uint32_t kGroupThreads = 512, kGroupWarps = kGroupThreads / 32, kGroupCtas = 8;
+static_assert(kGroupMax == kGroupThreads * 8 * kGroupCtas, "8 packets a thread at most");
+
+struct GroupArgs {
+    SortKeySrc src;
+    uint32_t n, passes, digit_bits, max_slots;
+    // counters (send_counter != nullptr)
+    uint64_t *send_counter;
+    uint64_t *counter_out; // per packet
+    // replay window (replay): rp.keys and rp.order are written here
+    uint32_t *keys_out, *order_out;
+    ReplayArgs rp;
+    bool replay;
+    VerdictArgs verdict; // n == 0: none
+    Done done;
 };
-__global__ void __launch_bounds__(kSortThreads) group_small_kernel(SortKeySrc src, uint32_t n, uint32_t passes,
-                                                                   uint32_t digit_bits, uint32_t *keys_out,
-                                                                   uint32_t *vals_out, SmallCounters sc, ReplayArgs rp) {
+
+template <int ITEMS>
+__global__ void __launch_bounds__(kGroupThreads) group_kernel(const __grid_constant__ GroupArgs a) {
     let_next_kernel_start();    // seal side: the seal launch behind may take its place already
     wait_for_kernel_in_front(); // open side: statuses and counters come from the open launch in front
-    constexpr uint32_t TILES = kSmallMax / kSortThreads; // 4
-    __shared__ uint32_t kbuf[2][kSmallMax], vbuf[2][kSmallMax];
-    __shared__ uint32_t cur[kSortWarps][kMaxBins];
-    __shared__ uint32_t base_of[kMaxBins];
-    __shared__ uint32_t warp_sum[kSortWarps];
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t bins = 1u << digit_bits;
-    const uint32_t begin = warp * (32 * TILES);
-    const uint32_t lt = (1u << lane) - 1u;
-    if (n <= kSortThreads) {
-        // One packet per thread at most (the upstream batch is 128): the place of a packet is the number of
-        // packets with a lower key, or the same key and a lower index.  n broadcast reads from shared memory
-        // instead of two radix passes with five barriers each.
-        const uint32_t mine = tid < n ? slot_key(src, tid) : 0xffffffffu;
-        kbuf[0][tid] = mine;
+    constexpr uint32_t kChunk = kGroupThreads * ITEMS; // positions per CTA
+    extern __shared__ __align__(16) uint32_t dyn[];
+    auto kbuf = [&](uint32_t half) { return dyn + half * kChunk; };
+    auto vbuf = [&](uint32_t half) { return dyn + (2 + half) * kChunk; };
+    uint16_t *const cnt = reinterpret_cast<uint16_t *>(dyn + 4 * kChunk); // [kGroupWarps][kMaxBins]
+    __shared__ uint32_t hist[kMaxBins], base_of[kMaxBins], warp_sum[kGroupWarps];
+    __shared__ SegMax part[kGroupWarps];
+    __shared__ SegMax cta_total;
+    __shared__ uint32_t cta_head, cta_pending;
+    const cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ctas = gridDim.x, me = blockIdx.x;
+    auto all_sync = [&] {
+        if (ctas > 1) cluster.sync();
+        else __syncthreads();
+    };
+    const uint32_t first = me * kChunk; // this CTA's positions (and, before the sort, its packets)
+    const uint32_t mine = a.n > first ? min(kChunk, a.n - first) : 0u;
+
+    // ---- sort ----
+    uint32_t f = 0; // which buffer holds the result
+    if (a.n <= 256) { // one CTA
+        const uint32_t key = tid < a.n ? slot_key(a.src, tid) : 0xffffffffu;
+        if (tid < 256) kbuf(0)[tid] = key;
         __syncthreads();
         uint32_t place = 0;
-        for (uint32_t j = 0; j < n; j++) {
-            const uint32_t other = kbuf[0][j];
-            place += (other < mine || (other == mine && j < tid)) ? 1u : 0u;
+        for (uint32_t j = 0; j < a.n; j++) {
+            const uint32_t other = kbuf(0)[j];
+            place += (other < key || (other == key && j < tid)) ? 1u : 0u;
         }
-        if (tid < n) {
-            keys_out[place] = mine;
-            vals_out[place] = tid;
+        f = 1;
+        if (tid < a.n) {
+            kbuf(1)[place] = key;
+            vbuf(1)[place] = tid;
         }
         __syncthreads();
-        passes = 0;
-    }
-    for (uint32_t p = 0; p < passes; p++) {
-        const uint32_t shift = p * digit_bits;
-        const uint32_t *kin = kbuf[p & 1], *vin = vbuf[p & 1];
-        uint32_t *kout = kbuf[(p + 1) & 1], *vout = vbuf[(p + 1) & 1];
-        for (uint32_t d = tid; d < kSortWarps * kMaxBins; d += kSortThreads) (&cur[0][0])[d] = 0;
-        __syncthreads();
-        uint32_t key[TILES], val[TILES];
+    } else {
+        const uint32_t bins = 1u << a.digit_bits, lt = (1u << lane) - 1u;
+        for (uint32_t p = 0; p < a.passes; p++, f ^= 1u) {
+            const uint32_t shift = p * a.digit_bits;
+            for (uint32_t d = tid; d < kGroupWarps * kMaxBins / 8; d += kGroupThreads) reinterpret_cast<uint4 *>(cnt)[d] = make_uint4(0, 0, 0, 0);
+            __syncthreads();
+            uint16_t *const my_cnt = cnt + warp * kMaxBins;
+            uint32_t key[ITEMS], val[ITEMS], rank[ITEMS];
 #pragma unroll
-        for (uint32_t t = 0; t < TILES; t++) {
-            const uint32_t i = begin + t * 32 + lane;
-            const bool have = i < n;
-            key[t] = have ? (p == 0 ? slot_key(src, i) : kin[i]) : 0xffffffffu;
-            val[t] = have ? (p == 0 ? i : vin[i]) : 0u;
-            warp_hist_add(cur[warp], (key[t] >> shift) & (bins - 1), have);
-        }
-        __syncthreads();
-        {   // digit bases: exclusive prefix over the digit totals, two digits per thread
-            const uint32_t d0 = 2 * tid, d1 = 2 * tid + 1;
-            uint32_t v0 = 0, v1 = 0;
-            for (uint32_t w = 0; w < kSortWarps; w++) {
-                if (d0 < bins) v0 += cur[w][d0];
-                if (d1 < bins) v1 += cur[w][d1];
+            for (int t = 0; t < ITEMS; t++) { // a warp owns 32 * ITEMS consecutive packets
+                const uint32_t e = warp * (32 * ITEMS) + t * 32 + lane;
+                const bool have = e < mine;
+                key[t] = have ? (p == 0 ? slot_key(a.src, first + e) : kbuf(f)[e]) : 0xffffffffu;
+                val[t] = have ? (p == 0 ? first + e : vbuf(f)[e]) : 0u;
+                const uint32_t digit = have ? (key[t] >> shift) & (bins - 1) : 0xffffffffu;
+                const uint32_t peers = __match_any_sync(0xffffffffu, digit);
+                rank[t] = __popc(peers & lt);
+                if (have) rank[t] += my_cnt[digit];
+                __syncwarp();
+                if (have && (peers & lt) == 0) my_cnt[digit] += (uint16_t)__popc(peers);
+                __syncwarp();
             }
-            uint32_t incl = v0 + v1;
+            __syncthreads();
+            if (tid < bins) { // counts of the warps -> their starts inside the CTA's share of the digit
+                uint32_t run = 0;
+#pragma unroll
+                for (uint32_t w = 0; w < kGroupWarps; w++) {
+                    const uint32_t c = cnt[w * kMaxBins + tid];
+                    cnt[w * kMaxBins + tid] = (uint16_t)run;
+                    run += c;
+                }
+                hist[tid] = run;
+            }
+            all_sync();
+            uint32_t before = 0, all = 0; // of digit `tid`: in the CTAs in front, in all CTAs
+            if (tid < bins) {
+                for (uint32_t c = 0; c < ctas; c++) {
+                    const uint32_t v = ctas > 1 ? cluster.map_shared_rank(hist, c)[tid] : hist[tid];
+                    if (c < me) before += v;
+                    all += v;
+                }
+            }
+            uint32_t incl = all;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -706,74 +734,144 @@ __global__ void __launch_bounds__(kSortThreads) group_small_kernel(SortKeySrc sr
             }
             if (lane == 31) warp_sum[warp] = incl;
             __syncthreads();
-            uint32_t before = 0;
             for (uint32_t w = 0; w < warp; w++) before += warp_sum[w];
-            const uint32_t excl = before + incl - (v0 + v1);
-            if (d0 < bins) base_of[d0] = excl;
-            if (d1 < bins) base_of[d1] = excl + v0;
-        }
-        __syncthreads();
-        for (uint32_t d = tid; d < bins; d += kSortThreads) {
-            uint32_t run = base_of[d];
+            if (tid < bins) base_of[tid] = before + incl - all;
+            __syncthreads();
 #pragma unroll
-            for (uint32_t w = 0; w < kSortWarps; w++) {
-                const uint32_t c = cur[w][d];
-                cur[w][d] = run;
-                run += c;
-            }
-        }
-        __syncthreads();
-        const bool final_pass = p + 1 == passes;
-        uint32_t *mine = cur[warp];
-#pragma unroll
-        for (uint32_t t = 0; t < TILES; t++) {
-            const bool have = begin + t * 32 + lane < n;
-            const uint32_t digit = have ? ((key[t] >> shift) & (bins - 1)) : 0xffffffffu;
-            const uint32_t peers = __match_any_sync(0xffffffffu, digit);
-            const uint32_t rank = __popc(peers & lt);
-            uint32_t pos = 0;
-            if (have) pos = mine[digit] + rank;
-            __syncwarp();
-            if (have && rank == 0) mine[digit] += __popc(peers);
-            __syncwarp();
-            if (have) {
-                if (final_pass) {
-                    keys_out[pos] = key[t];
-                    vals_out[pos] = val[t];
-                } else {
-                    kout[pos] = key[t];
-                    vout[pos] = val[t];
+            for (int t = 0; t < ITEMS; t++) {
+                const uint32_t e = warp * (32 * ITEMS) + t * 32 + lane;
+                if (e < mine) {
+                    const uint32_t digit = (key[t] >> shift) & (bins - 1);
+                    const uint32_t pos = base_of[digit] + my_cnt[digit] + rank[t], to = pos / kChunk, at = pos % kChunk;
+                    uint32_t *const kout = ctas > 1 ? cluster.map_shared_rank(kbuf(f ^ 1u), to) : kbuf(f ^ 1u);
+                    uint32_t *const vout = ctas > 1 ? cluster.map_shared_rank(vbuf(f ^ 1u), to) : vbuf(f ^ 1u);
+                    kout[at] = key[t];
+                    vout[at] = val[t];
                 }
             }
+            all_sync();
         }
+    }
+
+    // ---- the grouped order: ITEMS consecutive positions a thread ----
+    const uint32_t at0 = tid * ITEMS;
+    uint32_t slot[ITEMS];
+    bool head[ITEMS], tail[ITEMS];
+    {
+        uint32_t prev = 0xffffffffu;
+        if (at0 > 0) prev = kbuf(f)[at0 - 1];
+        else if (me > 0) prev = cluster.map_shared_rank(kbuf(f), me - 1)[kChunk - 1];
+        uint32_t next = 0xffffffffu; // key behind the thread's last position
+        if (at0 + ITEMS < mine) next = kbuf(f)[at0 + ITEMS];
+        else if (at0 + ITEMS == kChunk && first + kChunk < a.n) next = cluster.map_shared_rank(kbuf(f), me + 1)[0];
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            slot[k] = at0 + k < mine ? kbuf(f)[at0 + k] : 0xffffffffu;
+            head[k] = at0 + k < mine && ((first + at0 + k) == 0 || slot[k] != prev);
+            prev = slot[k];
+        }
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++)
+            tail[k] = at0 + k < mine && slot[k] != (k + 1 < ITEMS ? slot[k + 1] : next);
+    }
+
+    if (a.send_counter) {
+        // start of the run a position lies in: running maximum of the head positions (+1; 0 = none yet)
+        uint32_t run = 0;
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++)
+            if (head[k]) run = first + at0 + k + 1;
+        uint32_t incl = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl = max(incl, t);
+        }
+        uint32_t front = __shfl_up_sync(0xffffffffu, incl, 1);
+        if (lane == 0) front = 0;
+        if (lane == 31) warp_sum[warp] = incl;
         __syncthreads();
-    }
-    if (rp.replay_last != nullptr) { // the barrier that closed the last pass makes the sorted arrays visible
-        __shared__ SegMax part[8];
-        replay_one_cta(rp, part);
-    }
-    if (sc.counter_out == nullptr) return;
-    uint64_t next[TILES];
-    uint32_t tail_slot[TILES];
-#pragma unroll
-    for (uint32_t t = 0; t < TILES; t++) {
-        const uint32_t j = t * kSortThreads + tid;
-        tail_slot[t] = 0xffffffffu;
-        if (j >= n) continue;
-        const uint32_t slot = keys_out[j];
-        if (slot >= sc.max_slots) continue;
-        const uint32_t rank = j - run_start(keys_out, j);
-        const uint64_t base = sc.send_counter[slot];
-        sc.counter_out[vals_out[j]] = saturating_counter(base, rank);
-        if (j + 1 == n || keys_out[j + 1] != slot) {
-            tail_slot[t] = slot;
-            next[t] = saturating_counter(base, rank + 1);
+        uint32_t whole = 0;
+        for (uint32_t w = 0; w < kGroupWarps; w++) {
+            if (w < warp) front = max(front, warp_sum[w]);
+            whole = max(whole, warp_sum[w]);
         }
-    }
-    __syncthreads();
+        if (ctas > 1) {
+            if (tid == 0) cta_head = whole;
+            cluster.sync();
+            for (uint32_t c = 0; c < me; c++) front = max(front, *cluster.map_shared_rank(&cta_head, c));
+        }
+        uint64_t next_counter[ITEMS];
 #pragma unroll
-    for (uint32_t t = 0; t < TILES; t++)
-        if (tail_slot[t] != 0xffffffffu) sc.send_counter[tail_slot[t]] = next[t];
+        for (int k = 0; k < ITEMS; k++) {
+            const uint32_t p = first + at0 + k;
+            if (head[k]) front = p + 1;
+            if (at0 + k >= mine || slot[k] >= a.max_slots) continue;
+            const uint64_t base = a.send_counter[slot[k]];
+            const uint32_t rank = p + 1 - front;
+            a.counter_out[vbuf(f)[at0 + k]] = saturating_counter(base, rank);
+            next_counter[k] = saturating_counter(base, rank + 1);
+        }
+        all_sync(); // every counter is read
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++)
+            if (tail[k] && slot[k] < a.max_slots) a.send_counter[slot[k]] = next_counter[k];
+    }
+
+    if (a.replay) {
+        const ReplayArgs &r = a.rp;
+        uint64_t c[ITEMS], e[ITEMS], v[ITEMS];
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            c[k] = kReplayNoPart;
+            v[k] = 0;
+            if (at0 + k < mine) {
+                const uint32_t pkt = vbuf(f)[at0 + k], p = first + at0 + k;
+                a.keys_out[p] = slot[k];
+                a.order_out[p] = pkt;
+                c[k] = replay_gather(r, p, slot[k], pkt);
+                if (c[k] != kReplayNoPart) v[k] = c[k];
+            }
+        }
+        SegMax total;
+        const TileMax t = tile_running_max<ITEMS, kGroupWarps>(head, v, e, part, total);
+        if (tid == 0) {
+            cta_total = total;
+            cta_pending = 0;
+        }
+        all_sync();
+        SegMax reached{0u, 0ull};
+        for (uint32_t q = 0; q < me; q++) reached = seg_combine(reached, *cluster.map_shared_rank(&cta_total, q));
+        tile_carry<ITEMS>(t, reached.m, e);
+        bool pending = false;
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            if (at0 + k >= mine) continue;
+            const uint8_t st = replay_classify(r, first + at0 + k, slot[k], tail[k], c[k], e[k]);
+            r.state[first + at0 + k] = st;
+            pending |= st == RP_PENDING;
+        }
+        if (__syncthreads_or(pending) && tid == 0) cta_pending = 1;
+        all_sync(); // every verdict and next `last` is written
+        bool any_pending = false;
+        for (uint32_t q = 0; q < ctas; q++) any_pending |= (ctas > 1 ? *cluster.map_shared_rank(&cta_pending, q) : cta_pending) != 0;
+        for (uint32_t i = tid; i < kChunk; i += kGroupThreads) replay_advance_warp(r, i < mine ? first + i : a.n);
+        if (any_pending) {
+            for (uint32_t i = me * kGroupThreads + tid; i <= r.mask; i += ctas * kGroupThreads) r.table[i] = kHashEmpty;
+            all_sync();
+            for (uint32_t i = tid; i < kChunk; i += kGroupThreads) {
+                const uint32_t p = first + i;
+                replay_hash_insert_warp(r, p, i < mine && r.state[p] != RP_NOPART);
+            }
+        }
+        all_sync(); // clears before marks, inserts before look-ups
+        for (uint32_t i = tid; i < kChunk; i += kGroupThreads) replay_finish_warp(r, i < mine ? first + i : a.n);
+        if (a.verdict.n) all_sync(); // every refusal is written
+    }
+    if (a.verdict.n)
+        for (uint32_t i = tid; i < mine; i += kGroupThreads) final_verdict(a.verdict, first + i);
+    if (ctas > 1) cluster.sync(); // nobody leaves while another may still look into its shared memory
+    signal_done(a.done, [] {});
 }
 
 // --- scheduling order by length class (mixed packet sizes) ------------------------------
@@ -883,11 +981,6 @@ void sort_pass(const SortKeySrc &src, const uint32_t *kin, const uint32_t *vin, 
 // Stable sort of packet indices 0..n-1 by key.  Returns the number of kernel launches.
 uint32_t group_sort(const SortKeySrc &src, uint32_t n, uint32_t max_chunks, const SortBuffers &sb, cudaStream_t s) {
     const SortPlan plan = plan_for(src.max_slots);
-    if (n <= kSmallMax) {
-        launch_after_kernel(group_small_kernel, dim3(1), dim3(kSortThreads), s, src, n, plan.passes, plan.digit_bits,
-            sb.keys_b, sb.order, SmallCounters{nullptr, nullptr, 0}, ReplayArgs{});
-        return 1;
-    }
     const uint32_t bins = 1u << plan.digit_bits;
     const uint32_t tiles = tiles_for(n, max_chunks);
     const uint32_t chunks = chunks_for(n, tiles);
@@ -912,7 +1005,57 @@ uint32_t group_sort(const SortKeySrc &src, uint32_t n, uint32_t max_chunks, cons
     return 3 * plan.passes;
 }
 
+// Dynamic shared memory of group_kernel<items>.
+constexpr size_t group_smem(uint32_t items) { return (size_t)kGroupThreads * items * 16 + kGroupWarps * kMaxBins * 2; }
+template <int ITEMS>
+cudaError_t launch_group_items(const GroupArgs &a, uint32_t ctas, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kGroupThreads);
+    cfg.dynamicSmemBytes = group_smem(ITEMS);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = ctas;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, group_kernel<ITEMS>, a);
+}
+// One CTA up to 1024 packets, then as many as keep two packets a thread, up to the eight of a portable cluster.
+cudaError_t launch_group(const GroupArgs &a, cudaStream_t s) {
+    uint32_t ctas = 1;
+    while (ctas < kGroupCtas && a.n > ctas * 2 * kGroupThreads) ctas *= 2;
+    const uint32_t per_thread = (a.n + ctas * kGroupThreads - 1) / (ctas * kGroupThreads);
+    if (per_thread <= 1) return launch_group_items<1>(a, ctas, s);
+    if (per_thread <= 2) return launch_group_items<2>(a, ctas, s);
+    if (per_thread <= 4) return launch_group_items<4>(a, ctas, s);
+    return launch_group_items<8>(a, ctas, s);
+}
+cudaError_t launch_counters(bnk_ctx *ctx, const uint32_t *slot, uint32_t n, uint64_t *counter, cudaStream_t s) {
+    const uint32_t max_slots = ctx->cfg.max_keypairs;
+    const SortPlan plan = plan_for(max_slots);
+    GroupArgs g{};
+    g.src = SortKeySrc{slot, max_slots};
+    g.n = n;
+    g.passes = plan.passes;
+    g.digit_bits = plan.digit_bits;
+    g.max_slots = max_slots;
+    g.send_counter = ctx->kt.send_counter;
+    g.counter_out = counter;
+    ctx->launches += 1;
+    return launch_group(g, s);
+}
+
 } // namespace
+
+cudaError_t group_kernels_init() {
+    cudaError_t e = cudaFuncSetAttribute(group_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)group_smem(4));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(group_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)group_smem(8));
+    return e;
+}
 
 // words of histogram scratch a batch of max_pkts packets needs
 uint32_t group_sort_chunks(uint32_t max_pkts) {
@@ -922,34 +1065,28 @@ uint32_t group_sort_chunks(uint32_t max_pkts) {
 
 // Sorts packet indices 0..n-1 by keypair slot, stable.  Leaves the sorted keys in
 // dev.keys_tmp (second half) and the packet indices in dev.order.
-cudaError_t launch_group_by_slot(bnk_batch *b, uint32_t n, bool only_status_ok, cudaStream_t s) {
+cudaError_t launch_group_by_slot(bnk_batch *b, uint32_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     bnk_ctx *ctx = b->ctx;
     DeviceBatch &d = b->dev;
-    SortKeySrc src{d.slot, d.status, ctx->cfg.max_keypairs, only_status_ok ? 1 : 0};
+    SortKeySrc src{d.slot, ctx->cfg.max_keypairs};
     SortBuffers sb{d.keys_tmp, d.keys_tmp + b->max_pkts, d.order_tmp, d.order, d.hist + kMaxBins, d.hist};
     ctx->launches += group_sort(src, n, kBatchMaxChunks, sb, s);
     return cudaGetLastError();
 }
 
-cudaError_t launch_assign_counters(bnk_batch *b, uint32_t n, cudaStream_t s) {
+cudaError_t launch_assign_counters(bnk_batch *b, uint32_t n, const uint32_t *slot, uint64_t *counter, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    if (n <= kSmallMax) { // sort and counters in one launch
-        bnk_ctx *ctx = b->ctx;
-        DeviceBatch &d = b->dev;
-        const SortPlan plan = plan_for(ctx->cfg.max_keypairs);
-        launch_after_kernel(group_small_kernel, dim3(1), dim3(kSortThreads), s,
-            SortKeySrc{d.slot, d.status, ctx->cfg.max_keypairs, 0}, n, plan.passes, plan.digit_bits,
-            d.keys_tmp + b->max_pkts, d.order, SmallCounters{ctx->kt.send_counter, d.counter, ctx->cfg.max_keypairs},
-            ReplayArgs{});
-        ctx->launches += 1;
-        return cudaGetLastError();
-    }
-    cudaError_t e = launch_group_by_slot(b, n, false, s);
-    if (e != cudaSuccess) return e;
+    bnk_ctx *ctx = b->ctx;
     DeviceBatch &d = b->dev;
+    const SortKeySrc src{slot, ctx->cfg.max_keypairs};
+    if (n <= kGroupMax) return launch_counters(ctx, slot, n, counter, s);
+    SortBuffers sb{d.keys_tmp, d.keys_tmp + b->max_pkts, d.order_tmp, d.order, d.hist + kMaxBins, d.hist};
+    ctx->launches += group_sort(src, n, kBatchMaxChunks, sb, s);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
     launch_kernel(n <= dependent_launch_up_to(), assign_counters_kernel, dim3((n + 255) / 256), dim3(256), s,
-        d.keys_tmp + b->max_pkts, d.order, n, b->ctx->cfg.max_keypairs, b->ctx->kt.send_counter, d.counter);
+        d.keys_tmp + b->max_pkts, d.order, n, ctx->cfg.max_keypairs, ctx->kt.send_counter, counter);
     launch_kernel(n <= dependent_launch_up_to(), advance_counters_kernel, dim3((n + 255) / 256), dim3(256), s,
         d.keys_tmp + b->max_pkts, n, b->ctx->cfg.max_keypairs, b->ctx->kt.send_counter);
     b->ctx->launches += 2;
@@ -984,20 +1121,31 @@ static ReplayArgs replay_args(bnk_batch *b, uint32_t n) {
     a.mask = cap - 1;
     return a;
 }
-// Grouping and replay window of a small batch in one launch, for after the open kernel.
-bool replay_is_one_launch(uint32_t n) { return n <= kSmallMax; }
-cudaError_t launch_group_and_replay(bnk_batch *b, uint32_t n, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
+cudaError_t launch_open_tail(bnk_batch *b, uint32_t n, bool replay, const VerdictArgs *verdict, const Done &done, cudaStream_t s) {
     bnk_ctx *ctx = b->ctx;
     DeviceBatch &d = b->dev;
+    if (!replay) return launch_verdict(ctx, *verdict, done, s);
     const SortPlan plan = plan_for(ctx->cfg.max_keypairs);
-    launch_after_kernel(group_small_kernel, dim3(1), dim3(kSortThreads), s,
-        SortKeySrc{d.slot, d.status, ctx->cfg.max_keypairs, 0}, n, plan.passes, plan.digit_bits,
-        d.keys_tmp + b->max_pkts, d.order, SmallCounters{nullptr, nullptr, 0}, replay_args(b, n));
+    GroupArgs g{};
+    g.src = SortKeySrc{d.slot, ctx->cfg.max_keypairs};
+    g.n = n;
+    g.passes = plan.passes;
+    g.digit_bits = plan.digit_bits;
+    g.max_slots = ctx->cfg.max_keypairs;
+    g.keys_out = d.keys_tmp + b->max_pkts;
+    g.order_out = d.order;
+    g.rp = replay_args(b, n);
+    g.replay = true;
+    if (verdict) g.verdict = *verdict;
+    g.done = done;
     ctx->launches += 1;
-    return cudaGetLastError();
+    return launch_group(g, s);
 }
-// Expects launch_group_by_slot(b, n, false, ...) to have completed before this point of stream s.
+cudaError_t launch_verdict(bnk_ctx *ctx, const VerdictArgs &v, const Done &done, cudaStream_t s) {
+    ctx->launches += 1;
+    return launch_after_kernel(verdict_kernel, dim3((v.n + 255) / 256), dim3(256), s, v, done);
+}
+// Expects launch_group_by_slot(b, n, ...) to have completed before this point of stream s.
 cudaError_t launch_replay(bnk_batch *b, uint32_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     DeviceBatch &d = b->dev;
@@ -1039,42 +1187,13 @@ cudaError_t launch_length_order(bnk_batch *b, uint32_t n, const uint32_t *len, b
 // whole device, so one allocation stalls every other batch in flight, and a caller that
 // keeps packets in device buffers of its own (for instance buffers a NIC writes into
 // directly) has no bnk_batch whose creation would have set the grouping scratch aside.
-// For those callers the same grouping kernels run here on a fixed scratch area that is
-// part of the library image: kNoAllocMaxPkts packets at most, 384 KiB held by every GPU
-// that loads the library until the process exits.
-//
-// The area is shared by every call and keeps whatever the previous call left in it.  All
-// regions are written before they are read within one call (the histogram kernel stores
-// every bin of every chunk it later scans, the scatter kernel stores every element below
-// npkts), so nothing needs clearing; calls that overlap on the GPU race on
-// the area and must be ordered by the caller (same stream, or an event between them).
+// For those callers one group_kernel launch sorts in shared memory and writes nothing but their counters and the send
+// counters.
 // ---------------------------------------------------------------------------------------
 namespace {
 
 constexpr uint32_t kNoAllocMaxPkts = BNK_NOALLOC_MAX_PKTS;
-constexpr uint32_t kNoAllocMaxChunks = 31; // (31 chunk columns + 1 row of totals) * 512 bins = the 16384-word histogram region
-constexpr size_t kNoAllocWords = (size_t)5 * kNoAllocMaxPkts + 16384; // 384 KiB
-static_assert((size_t)kMaxBins * (kNoAllocMaxChunks + 1) <= 16384, "histogram region too small");
-
-static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocWords];
-
-constexpr int kNoAllocMaxDevices = 64;
-std::mutex g_noalloc_mu;
-uint32_t *g_noalloc_ptr[kNoAllocMaxDevices] = {};
-
-// Device address of the scratch area on the current device.  In host code the array's name
-// is only a handle, so the address is asked for once per device and remembered.
-cudaError_t noalloc_scratch(int device, uint32_t **out) {
-    std::lock_guard<std::mutex> g(g_noalloc_mu);
-    if (!g_noalloc_ptr[device]) {
-        void *p = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-        if (e != cudaSuccess) return e;
-        g_noalloc_ptr[device] = static_cast<uint32_t *>(p);
-    }
-    *out = g_noalloc_ptr[device];
-    return cudaSuccess;
-}
+static_assert(kNoAllocMaxPkts <= kGroupMax, "one launch");
 
 int noalloc_fail(bnk_ctx *ctx, int code, const char *what, cudaError_t e = cudaSuccess) {
     std::lock_guard<std::mutex> g(ctx->mu);
@@ -1096,27 +1215,10 @@ extern "C" int bnk_assign_counters_noalloc(bnk_ctx *ctx, void *stream, const uin
         return noalloc_fail(ctx, BNK_EINVAL,
                             "bnk_assign_counters_noalloc: npkts exceeds BNK_NOALLOC_MAX_PKTS (16384); split the batch "
                             "or use bnk_seal_submit with BNK_F_ASSIGN_COUNTERS");
-    if (ctx->device < 0 || ctx->device >= kNoAllocMaxDevices)
-        return noalloc_fail(ctx, BNK_EINVAL, "bnk_assign_counters_noalloc: device ordinal above 63");
     if (npkts == 0) return BNK_SUCCESS;
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) return noalloc_fail(ctx, BNK_ECUDA, "cudaSetDevice", e);
-    uint32_t *base = nullptr;
-    if ((e = noalloc_scratch(ctx->device, &base)) != cudaSuccess)
-        return noalloc_fail(ctx, BNK_ECUDA, "cudaGetSymbolAddress(scratch)", e);
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-
-    const uint32_t n = npkts, cap = kNoAllocMaxPkts;
-    uint32_t *keys_a = base, *keys_b = base + cap, *vals_a = base + 2 * cap, *order = base + 3 * cap;
-    uint32_t *hist = base + 5 * cap; // [4*cap, 5*cap) is spare
-    SortKeySrc src{dev_slot, nullptr, ctx->cfg.max_keypairs, 0};
-    SortBuffers sb{keys_a, keys_b, vals_a, order, hist + kMaxBins, hist};
-    const uint32_t sort_launches = group_sort(src, n, kNoAllocMaxChunks, sb, s);
-    launch_kernel(n <= dependent_launch_up_to(), assign_counters_kernel, dim3((n + 255) / 256), dim3(256), s, keys_b,
-        order, n, ctx->cfg.max_keypairs, ctx->kt.send_counter, dev_counter);
-    launch_kernel(n <= dependent_launch_up_to(), advance_counters_kernel, dim3((n + 255) / 256), dim3(256), s, keys_b, n,
-        ctx->cfg.max_keypairs, ctx->kt.send_counter);
-    ctx->launches += sort_launches + 2;
-    if ((e = cudaGetLastError()) != cudaSuccess) return noalloc_fail(ctx, BNK_ECUDA, "kernel launch", e);
+    e = launch_counters(ctx, dev_slot, npkts, dev_counter, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return noalloc_fail(ctx, BNK_ECUDA, "kernel launch", e);
     return BNK_SUCCESS;
 }

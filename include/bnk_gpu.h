@@ -24,9 +24,10 @@
  *     both BNK_F_NO_H2D and BNK_F_NO_D2H only queue kernels on the batch's stream
  *     and may be issued back to back.
  *   - Between a submit and its bnk_wait the batch's host arrays belong to the
- *     library.  Small batches (up to 256 packets and a ring extent of 384 KiB,
- *     environment BNK_HOST_DIRECT_BYTES, 0 = never) are not copied: the kernels
- *     read and write the pinned arrays in place.  The results are the same bytes.
+ *     library.  A batch that asks for both copies and is alone in flight, or small
+ *     enough beside others, is not copied at all: the kernels read and write the
+ *     pinned arrays in place (up to a ring extent of BNK_HOST_DIRECT_BYTES from the
+ *     environment, 0 = never).  The results are the same bytes.
  *   - Send counters and replay windows are per keypair and ordered: batches that
  *     are in flight at the same time must not carry packets of the same keypair
  *     slot when BNK_F_ASSIGN_COUNTERS or BNK_F_REPLAY is used (give each peer's
@@ -294,9 +295,8 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
  * stalls every stream of the device), and a caller that keeps packets in device buffers of its own,
  * such as buffers a NIC writes into directly, has no bnk_batch to lend it grouping scratch.  This
  * entry point does the send-counter stage of bnk_seal_submit(BNK_F_ASSIGN_COUNTERS) on the caller's
- * buffers and allocates nothing: its scratch is a fixed 384 KiB area inside the library image,
- * present on every GPU that loads the library, which limits a call to BNK_NOALLOC_MAX_PKTS packets
- * (more is refused with BNK_EINVAL).
+ * buffers and allocates nothing: it sorts in the GPU's shared memory, which limits a call to
+ * BNK_NOALLOC_MAX_PKTS packets (more is refused with BNK_EINVAL).
  *   dev_slot[i]    (device memory, in)  keypair slot of packet i
  *   dev_counter[i] (device memory, out) the nonce handed to packet i: packets of one slot get
  *                  consecutive values in batch order and the slot's send counter moves past them,
@@ -304,12 +304,8 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
  *                  max_keypairs are left untouched
  *   stream         a cudaStream_t of ctx's device, or NULL for the default stream; the work is
  *                  queued on it and the call returns without waiting.
- * The first call on each device looks up the address of the scratch area (the device must be usable
- * at that moment); make that first call before any stream capture begins.  The scratch is shared by
- * all calls and keeps the previous call's contents; each call overwrites what it reads, so nothing
- * has to be cleared, but two calls whose work overlaps on the GPU would corrupt each other: order
- * them on one stream or with an event.  The same holds against batches in flight that hand out
- * counters for the same keypair slots. */
+ * Calls whose work overlaps on the GPU must not hand out counters for the same keypair slots: order
+ * them on one stream or with an event, also against batches in flight that do. */
 #define BNK_NOALLOC_MAX_PKTS 16384u
 int bnk_assign_counters_noalloc(bnk_ctx *ctx, void *stream, const uint32_t *dev_slot, uint32_t npkts,
                                 uint64_t *dev_counter);

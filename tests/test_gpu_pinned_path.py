@@ -1,0 +1,151 @@
+"""Batches that stay in pinned memory: the warp-per-packet kernel at the edges of its rounds, the one-launch grouping at
+the edges of its splits, and the flow table's sweep, against the CPU checker (bytes, statuses and counters are equal)."""
+import numpy as np
+import pytest
+
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+ROUND = 1984  # payload bytes a warp takes per round
+
+
+def _expected_counters(slots, start, max_slots):
+    """Consecutive per slot in batch order."""
+    out, nxt = np.zeros(len(slots), np.uint64), dict(start)
+    for i, s in enumerate(slots):
+        if s < max_slots:
+            out[i] = nxt.get(int(s), 0)
+            nxt[int(s)] = nxt.get(int(s), 0) + 1
+    return out, nxt
+
+
+# 1 / 256 / 257: nonces inside the seal kernel or by the grouping launch; 512..32768: one, two, four, eight packets a
+# thread and one to eight CTAs; 32769: the chain of kernels.  Keypairs: one, two and three digits.
+@pytest.mark.parametrize("n,n_peers", [(1, 1), (256, 40), (257, 40), (1025, 600), (4097, 5), (8193, 3000), (32768, 300_000),
+                                       (32769, 70)])
+def test_counters_and_replay_at_the_edges_of_a_split(gpu_lib, oracle, n, n_peers):
+    from bnk_b200 import Context
+    from bnk_b200.device import F_ASSIGN_COUNTERS, F_REPLAY, PKT_BAD_DESC
+
+    rng = np.random.default_rng(n)
+    c = Context(max_keypairs=n_peers, mtu=0, flow_capacity=0, replay_ring_blocks=32)
+    try:
+        used = min(n_peers, 200)
+        keys = rng.integers(0, 256, (used, 32), dtype=np.uint8)
+        first = n_peers - used  # the highest slots: every digit of the sort takes part
+        c.set_keypairs(first, keys, keys, np.arange(used, dtype=np.uint32))
+        size, stride = 20, 80
+        b, r = c.batch(n, n * stride), c.batch(n, n * stride)
+        state, start = {}, {}
+        for turn in range(2):
+            slots = (first + np.where(rng.random(n) < 0.3, used - 1, rng.integers(0, used, n))).astype(np.uint32)
+            if n > 8:
+                slots[rng.integers(0, n, 2)] = n_peers  # not a keypair
+            b.ring[:] = rng.integers(0, 256, n * stride, dtype=np.uint8)
+            b.off[:], b.len[:], b.slot[:], b.counter[:] = np.arange(n) * stride, size, slots, 77
+            want_ctr, start = _expected_counters(slots, start, n_peers)
+            real = slots < n_peers
+            key_of = np.where(real, slots - np.uint32(first), 0).astype(np.uint32)
+            ring, st, ln = H.oracle_seal(oracle, keys, np.arange(used), 0, b.ring, b.off, b.len, key_of, want_ctr)
+            b.seal(n, F_ASSIGN_COUNTERS)
+            assert np.array_equal(b.counter[real], want_ctr[real]) and (b.counter[~real] == 77).all()
+            assert np.array_equal(b.status, np.where(real, st, PKT_BAD_DESC)) and np.array_equal(b.out_len, np.where(real, ln, 0))
+            assert H.spans_differ_count(np.array(b.ring), ring, b.off[real], ln[real]) == 0
+            for s in (first, n_peers - 1):
+                assert c.send_counter(s) == start.get(s, 0)
+            # arrival: swaps, and copies of earlier packets in the place of a few
+            order = np.arange(n)
+            for i in rng.integers(0, n, n // 10):
+                j = min(n - 1, int(i) + int(rng.integers(1, 70)))
+                order[[i, j]] = order[[j, i]]
+            again = rng.integers(0, n, n // 50)
+            order[again] = order[np.maximum(again - rng.integers(1, 300, len(again)), 0)]
+            r.ring[:] = np.array(b.ring).reshape(n, stride)[order].reshape(-1)
+            r.off[:], r.len[:], r.slot[:] = b.off, 16 + 32 + 16, slots[order]
+            _, st, ctr, ln = H.oracle_open(oracle, keys, r.ring, r.off, r.len, key_of[order])
+            st[~real[order]] = PKT_BAD_DESC
+            want, state = H.oracle_replay(oracle, 32, r.slot, ctr, st, state)
+            r.open(n, F_REPLAY)
+            assert np.array_equal(r.status, want), np.flatnonzero(r.status != want)[:8]
+            assert np.array_equal(r.out_len[want == 0], ln[want == 0])
+        for s in list(state)[:5]:
+            last, ring = c.replay_export(s)
+            assert last == state[s].last and np.array_equal(ring, state[s].ring())
+    finally:
+        c.close()
+
+
+@pytest.mark.parametrize("copies", [False, True])
+def test_round_edges_and_forgeries_of_long_packets(gpu_lib, oracle, copies):
+    from bnk_b200.device import F_NO_D2H, F_NO_H2D
+
+    from bnk_b200 import Context
+
+    rng = np.random.default_rng(3)
+    lens = np.array([k * ROUND + d for k in (1, 2) for d in (-65, -64, -17, -16, -15, -1, 0, 1, 15, 16, 17, 64)] + [3 * ROUND + 5], np.uint32)
+    n = len(lens)
+    keys = rng.integers(0, 256, (3, 32), dtype=np.uint8)
+    slots = rng.integers(0, 3, n).astype(np.uint32)
+    ctr = rng.integers(0, 2**60, n, dtype=np.uint64)
+    off = H.layout_packed(lens)
+    with Context(max_keypairs=3, mtu=0, flow_capacity=0) as c:
+        c.set_keypairs(0, keys, keys, np.arange(3, dtype=np.uint32))
+        b = c.batch(n, H.ring_bytes_for(off, lens))
+        b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
+        b.off[:], b.len[:], b.slot[:], b.counter[:] = off, lens, slots, ctr
+        plain = np.array(b.ring)
+        ring, st, ln = H.oracle_seal(oracle, keys, np.arange(3), 0, plain, off, lens, slots, ctr)
+
+        def call(f):
+            if not copies:
+                return f(n)
+            b.upload(n)
+            f(n, F_NO_H2D | F_NO_D2H)
+            b.download(n)
+
+        call(b.seal)
+        assert np.array_equal(b.out_len, ln) and H.spans_equal(np.array(b.ring), ring, off, ln) == []
+        hurt = np.arange(n) % 3 == 0  # a byte of the ciphertext, the first or a later round's
+        for i in np.flatnonzero(hurt):
+            b.ring[int(off[i]) + 16 + int(rng.integers(0, lens[i]))] ^= 1
+        b.len[:] = ln
+        want, st, _, _ = H.oracle_open(oracle, keys, b.ring, off, ln, slots)
+        call(b.open)
+        assert np.array_equal(b.status, st) and np.array_equal(st == oracle.AUTH_FAIL, hurt)
+        assert H.spans_equal(np.array(b.ring), want, off, ln - 32, start=16) == []
+
+
+def test_flows_noted_by_the_seal_kernel_and_swept(gpu_lib, oracle):
+    """More than 4096 flows over a clock that passes their lifetimes, noted by seal submits and by filter submits in
+    turn: the table equals the checker's map after every one."""
+    from bnk_b200 import Context, gen
+    from bnk_b200.device import F_ASSIGN_COUNTERS, F_NOTE_OUTBOUND
+
+    sec = 10**9
+    rng = np.random.default_rng(8)
+    with Context(max_keypairs=2, mtu=1420, flow_capacity=1 << 15) as c:
+        keys = rng.integers(0, 256, (2, 32), dtype=np.uint8)
+        c.set_keypairs(0, keys, keys, np.zeros(2, np.uint32))
+        c.acl_set(True, None)
+        f = oracle.Filter()
+        f.set_rules([])
+        now = 1_700_000_000 * sec
+        for turn, (n, step) in enumerate([(100, 1), (3000, 1), (1500, 31), (200, 5), (2500, 20), (257, 40), (64, 120), (1, 1)]):
+            now += step * sec
+            proto = rng.choice(np.array([6, 17, 1], np.uint8), n)
+            h = gen._headers(proto, np.full(n, gen.ip4(100, 64, 0, 1), np.uint64), rng.integers(1 << 30, 1 << 31, n).astype(np.uint64),
+                             rng.integers(1, 65536, n).astype(np.uint64), rng.integers(1, 65536, n).astype(np.uint64))
+            lens = np.full(n, 28, np.uint32)
+            h[n // 2, 0] = 0x65  # not IPv4: nothing to note
+            f.note_batch(np.ascontiguousarray(h), 28, lens, now)
+            b = c.batch(n, n * 80)
+            b.ring.reshape(n, 80)[:, 16:44] = h
+            b.off[:], b.len[:], b.slot[:] = np.arange(n) * 80, lens, rng.integers(0, 3, n)  # slot 2: refused, noted all the same
+            if turn % 3 == 2:
+                b.filter_note(n, now)
+            else:
+                b.seal(n, F_ASSIGN_COUNTERS | F_NOTE_OUTBOUND, now)
+            b.close()
+            assert c.flows_count() == f.flow_count, turn
+            assert H.flows_equal(c.flows_export(), f.flows()), turn
