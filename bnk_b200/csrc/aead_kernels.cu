@@ -21,6 +21,9 @@
 // FMA pipe.  The MAC input is ciphertext | zero pad to 16 | le64(0) | le64(ct_len),
 // RFC 8439 section 2.8 with empty AAD; nonce = 32 zero bits | le64(counter) and the
 // header is le32(4) | le32(receiver index) | le64(counter) (WireGuard whitepaper 5.4.6).
+#include <algorithm>
+#include <cstring>
+
 #include "filter_device.cuh"
 
 namespace {
@@ -64,6 +67,10 @@ __device__ __forceinline__ uint32_t rotl7(uint32_t x) { return __funnelshift_l(x
 // (The first column round of columns 1, 2 and 3 reads constants, key and nonce only, so it is the same for every
 // block of a packet.  Written out as a per-packet precomputation it compiles to the same register count as this
 // form: the compiler already moves those 37 instructions out of the block loop.)
+// UNROLL: double rounds per pass of the loop.  The throughput kernel wants all ten; a warp that computes one block and
+// is done pays for fetching fifteen kilobytes of straight-line code instead (measured for one block of one warp: 1.7 us
+// against 1.0 with one double round per pass).
+template <int UNROLL = 10>
 __device__ __forceinline__ void chacha20_block(uint32_t (&x)[16], const uint32_t (&k)[8], uint32_t blk,
                                                uint32_t n_lo, uint32_t n_hi) {
     x[0] = 0x61707865u;
@@ -76,7 +83,7 @@ __device__ __forceinline__ void chacha20_block(uint32_t (&x)[16], const uint32_t
     x[13] = 0u;
     x[14] = n_lo;
     x[15] = n_hi;
-#pragma unroll
+#pragma unroll UNROLL
     for (int r = 0; r < 10; r++) {
         BNK_QR(x[0], x[4], x[8], x[12])
         BNK_QR(x[1], x[5], x[9], x[13])
@@ -479,17 +486,16 @@ __device__ __forceinline__ P26 p26_mul(const P26 &x, const P26 &y) {
     o.v[4] = (uint32_t)d4 & kM26;
     return o;
 }
-__device__ __forceinline__ P26 p26_shfl(const P26 &x, int src) {
-    P26 o;
-#pragma unroll
-    for (int i = 0; i < 5; i++) o.v[i] = __shfl_sync(0xffffffffu, x.v[i], src);
-    return o;
-}
-__device__ __forceinline__ P26 p26_shfl_up(const P26 &x, int delta) {
-    P26 o;
-#pragma unroll
-    for (int i = 0; i < 5; i++) o.v[i] = __shfl_up_sync(0xffffffffu, x.v[i], delta);
-    return o;
+// limbs of up to 32 bits -> limbs below 2^26 (limb 1 may keep a few extra units)
+__device__ __forceinline__ P26 p26_carry(P26 h) {
+    uint32_t c;
+    c = h.v[0] >> 26; h.v[0] &= kM26; h.v[1] += c;
+    c = h.v[1] >> 26; h.v[1] &= kM26; h.v[2] += c;
+    c = h.v[2] >> 26; h.v[2] &= kM26; h.v[3] += c;
+    c = h.v[3] >> 26; h.v[3] &= kM26; h.v[4] += c;
+    c = h.v[4] >> 26; h.v[4] &= kM26; h.v[0] += c * 5u;
+    c = h.v[0] >> 26; h.v[0] &= kM26; h.v[1] += c;
+    return h;
 }
 // tag = ((h mod p) + pad) mod 2^128
 __device__ __forceinline__ void p26_finish(const P26 &x, const uint32_t (&pad)[4], uint32_t (&tag)[4]) {
@@ -527,19 +533,29 @@ __device__ __forceinline__ void p26_finish(const P26 &x, const uint32_t (&pad)[4
 // round's bytes into shared memory in 16-byte pieces with cp.async, in windows that start on 128-byte lines: over
 // the host link an instruction then asks for whole lines (measured on 4096 x 1440 B, read and written in place:
 // 172 us against 177 with windows at the packet's own 16-byte alignment).  Lane 0 computes cipher block 0 (the
-// one-time Poly1305 key), lane j the round's block j, all in the same pass.  For Poly1305 the round's 16-byte blocks
-// are laid out from the right, four to a lane, the length block last in lane 31, so that every lane runs the same
-// Horner steps from zero (the lane of the first block starts from the state carried in) and a binary tree over the
-// lanes with r^4, r^8 ... folds them; no lane works through a ragged end while the others idle.  What leaves the
-// round is put together in shared memory and written in the same pieces, so ragged ends cost one store instruction.
+// one-time Poly1305 key), lane j the round's block j, all in the same pass; on the seal side that needs no payload and
+// is done while the payload is on its way.  For Poly1305 the round's 16-byte blocks are laid out from the right, four
+// to a lane, the length block last in lane 31, so that every lane runs the same Horner steps from zero (the lane of the
+// first block starts from the state carried in); lane j's sum is then multiplied by r^(4 (31 - j)), which again needs no
+// payload, and the lanes' limbs are added up.  What leaves the round is put together in shared memory and written in
+// the same pieces; bytes behind the end of a message that share its last piece are written back as they were read.
 // A tag is checked before a one-round packet's plaintext is written.
 //
 // A warp takes tiles of a.tile consecutive packets (one in small batches); the descriptors of a tile lie in its
 // lanes, and the next packet's bytes are on their way while one is computed.  Few warps are enough to keep the host
 // link busy, and more of them in flight make it slower (read + write of 4096 x 1440 B: 172 us from 16 CTAs of 8
 // warps, 184 from 148, 225 from 512), so the grid is capped for host-resident rings (wpp_grid).
+//
+// Loops are kept rolled: a warp of a small batch runs its code once, from a cold instruction cache.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kWppWarps = 8;
+constexpr uint32_t kWppWarps = 4; // one per scheduler: the warps of a small batch then share none
+constexpr uint32_t kInlineMax = kRankMax;
+template <bool>
+struct InlineDesc {};
+template <>
+struct InlineDesc<true> {
+    uint32_t off[kInlineMax], len[kInlineMax], slot[kInlineMax];
+};
 constexpr uint32_t kRoundBlocks = 31;
 constexpr uint32_t kRoundBytes = kRoundBlocks * 64;
 constexpr uint32_t kStagePieces = 136; // <= 7 of the first line + header + 124 body + 1 of the tag, rounded to the swizzle's 8
@@ -568,9 +584,9 @@ struct Round {
 };
 
 //
-// Seal batches of up to kRankMax packets in pinned memory hand out their nonces here (a.send_counter): every CTA reads
-// the batch's slots, a warp counts the packets of its slot in front of its own, and of the packets of a slot the one
-// that reads the counter last moves it past them all.  A grouping launch in front costs more than this reading.
+// Seal batches of up to kRankMax packets in pinned memory hand out their nonces here (a.send_counter): a warp counts the
+// packets of its slot in front of its own, and the last packet of a slot moves the counter past them all (SendCounter
+// says why nobody has to wait for that).  A grouping launch in front took 5 us.
 // NOTE: the flows of the packets are recorded from the bytes in the stage, each step of the table's atomics behind a
 // piece of the cipher work.
 // Word `lane` (0..15) of the 64 bytes that start at a piece.
@@ -579,8 +595,28 @@ __device__ __forceinline__ uint32_t stage_word(const uint4 *stage, uint32_t piec
     return reinterpret_cast<const uint32_t *>(&stage[stage_at(piece + ((lane >> 2) & 3u))])[lane & 3u];
 }
 
-template <bool OPEN, bool NOTE>
-__global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __grid_constant__ AeadArgs a) {
+// r^(4 e) for the lane's e = 31 - lane, one bit of e per step: pw goes through r^4, r^8, r^16 ...
+struct LanePower {
+    P26 p, pw;
+    uint32_t bits; // of e still to come
+    __device__ __forceinline__ void begin(const P26 &r) {
+        p = p26_zero();
+        p.v[0] = 1u;
+        pw = p26_mul(r, r);
+        pw = p26_mul(pw, pw);
+        bits = 31u - (threadIdx.x & 31u);
+    }
+    __device__ __forceinline__ void step() {
+        const P26 t = p26_mul(p, pw);
+        if (bits & 1u) p = t;
+        bits >>= 1;
+        pw = p26_mul(pw, pw);
+    }
+};
+
+template <bool OPEN, bool NOTE, bool INLINE>
+__global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __grid_constant__ AeadArgs a,
+                                                                      const __grid_constant__ InlineDesc<INLINE> desc) {
     static_assert(!(OPEN && NOTE), "flows are recorded on the seal side");
     let_next_kernel_start(); // open side: the grouping + replay launch behind may take its place already
     // What a ring in device memory holds may come from the kernel in front; a pinned ring and its descriptors are the
@@ -599,9 +635,15 @@ __global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __gri
         Tile d{0, 0, 0, 0, 0, 0};
         const uint32_t i = t * T + lane;
         if (t < tiles && lane < T && i < a.n) {
-            d.off = a.off[i];
-            d.len = a.len[i];
-            if (!OPEN || !a.demux) d.slot = a.slot[i];
+            if constexpr (INLINE) {
+                d.off = desc.off[i];
+                d.len = desc.len[i];
+                d.slot = desc.slot[i];
+            } else {
+                d.off = a.off[i];
+                d.len = a.len[i];
+                if (!OPEN || !a.demux) d.slot = a.slot[i];
+            }
         }
         return d;
     };
@@ -613,85 +655,96 @@ __global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __gri
             if (!OPEN) d.remote = a.remote_index[d.slot];
         }
     };
-    // Starts the copies of a packet's first round (and of its keys when the slot is known) into stage `buf`.
+    // Starts the copies of a packet's keys (when the slot is known) and of its first round into stage `buf`: two groups.
     auto fetch = [&](uint32_t off, uint32_t len, uint32_t slot, uint32_t buf) {
         uint4 *const stage = stage_all[warp][buf];
+        if ((!OPEN || !a.demux) && slot < a.max_slots && lane < 2)
+            copy_async16(&key_all[warp][buf][lane], a.keys + (size_t)slot * 8 + 4u * lane);
+        copy_async_commit();
         if (!(off & 15u)) {
             const Round r(off, 0);
-            uint32_t from, bytes; // pieces from `from` on, to the piece of byte `bytes` of the body
+            uint32_t from, end, extra = 0xffffffffu; // pieces [from, end), and the piece the message ends in
             bool fits;
             if (OPEN) {
                 from = r.first;
                 fits = len >= BNK_WG_HEADER + BNK_WG_TAG && (uint64_t)off + len <= a.ring_bytes;
                 const uint32_t body = len - (BNK_WG_HEADER + BNK_WG_TAG);
-                bytes = body <= kRoundBytes ? body + BNK_WG_TAG : kRoundBytes;
+                end = r.body + (((body <= kRoundBytes ? body + BNK_WG_TAG : kRoundBytes) + 15u) >> 4);
             } else {
                 from = r.body;
                 fits = (uint64_t)off + BNK_WG_HEADER + len <= a.ring_bytes;
-                bytes = min(len, kRoundBytes);
+                end = r.body + ((min(len, kRoundBytes) + 15u) >> 4);
+                const uint32_t body = wg_padded_len(len, a.mtu);
+                if (body <= kRoundBytes && (body & 15u) && (uint64_t)off + BNK_WG_HEADER + body + BNK_WG_TAG <= a.ring_bytes)
+                    extra = r.body + ((body + BNK_WG_TAG) >> 4);
             }
             if (fits) {
-                const uint32_t end = r.body + ((bytes + 15u) >> 4);
-                for (uint32_t q = lane; q < end; q += 32)
-                    if (q >= from) copy_async16(&stage[stage_at(q)], a.in + r.window + 16u * q);
+#pragma unroll 1
+                for (uint32_t q = lane; q < kStagePieces; q += 32)
+                    if ((q >= from && q < end) || q == extra) copy_async16(&stage[stage_at(q)], a.in + r.window + 16u * q);
             }
         }
-        if ((!OPEN || !a.demux) && slot < a.max_slots && lane < 2)
-            copy_async16(&key_all[warp][buf][lane], a.keys + (size_t)slot * 8 + 4u * lane);
         copy_async_commit();
     };
 
     uint32_t t = blockIdx.x * kWppWarps + warp, buf = 0;
     Tile cur = load_tile(t);
-    __shared__ uint32_t slots[OPEN ? 1 : kRankMax];
-    if (!OPEN && a.send_counter) { // one tile of one packet per warp
-        for (uint32_t i = threadIdx.x; i < a.n; i += blockDim.x) slots[i] = a.slot[i];
-        __syncthreads();
-    }
+    // Loads come back in the order they were issued, also those from the device's own memory behind those over the link:
+    // what hangs on the slot is asked for before the payload, unless the kernel in front has still to write it.
+    __shared__ uint32_t slots[INLINE ? kRankMax : 1];
+    CounterRead counter{};
+    const bool hands_out = INLINE && !OPEN && a.send_counter;
+    if (OPEN || !a.behind_kernel || !a.over_link) load_keypair(cur, t);
+    if (hands_out && t < tiles && lane == 0 && cur.slot < a.max_slots) counter = counter_read(&a.send_counter[cur.slot], a.seal_seq);
     if (t < tiles) fetch(__shfl_sync(0xffffffffu, cur.off, 0), __shfl_sync(0xffffffffu, cur.len, 0),
                          __shfl_sync(0xffffffffu, cur.slot, 0), 0);
     if (a.over_link) wait_for_kernel_in_front();
-    load_keypair(cur, t);
-    if (!OPEN && a.send_counter && t < tiles) {
-        const uint32_t mine = slots[t];
-        uint32_t before = 0, all = 0;
-        for (uint32_t base = 0; base < a.n; base += 32) {
-            const uint32_t same = __ballot_sync(0xffffffffu, base + lane < a.n && slots[base + lane] == mine);
-            all += __popc(same);
-            before += __popc(base + 32 <= t ? same : base > t ? 0u : same & ((1u << (t - base)) - 1u));
-        }
-        if (lane == 0 && mine < a.max_slots) {
-            const uint64_t base = *(volatile uint64_t *)&a.send_counter[mine];
-            cur.ctr = saturating_counter(base, before);
-            __threadfence();
-            if (atomicAdd(&a.arrived[mine], 1u) + 1u == all) { // every packet of the slot has read it
-                a.send_counter[mine] = saturating_counter(base, all);
-                a.arrived[mine] = 0u;
+    if (!OPEN && a.behind_kernel && a.over_link) load_keypair(cur, t);
+    if constexpr (INLINE && !OPEN) {
+        if (hands_out) { // one tile of one packet per warp
+            for (uint32_t i = threadIdx.x; i < a.n; i += blockDim.x) slots[i] = desc.slot[i];
+            __syncthreads();
+            if (t < tiles) {
+                const uint32_t mine = slots[t];
+                uint32_t before = 0, all = 0;
+#pragma unroll 1
+                for (uint32_t base = 0; base < a.n; base += 32) {
+                    const uint32_t same = __ballot_sync(0xffffffffu, base + lane < a.n && slots[base + lane] == mine);
+                    all += __popc(same);
+                    before += __popc(base + 32 <= t ? same : base > t ? 0u : same & ((1u << (t - base)) - 1u));
+                }
+                cur.ctr = saturating_counter(counter.now.value, before);
+                if (before + 1 == all && lane == 0 && mine < a.max_slots) // the last packet of its slot moves the counter on
+                    counter_store(&a.send_counter[mine].e[counter.at ^ 1u],
+                                  SendCounter::Entry{saturating_counter(counter.now.value, all), a.seal_seq});
             }
         }
     }
+    __shared__ uint32_t cta_len[kWppWarps];
+    __shared__ uint64_t cta_ctr[kWppWarps];
+    __shared__ uint8_t cta_status[kWppWarps], cta_has[kWppWarps];
+    const bool by_cta = T == 1 && tiles <= step; // one packet per warp: the CTA's results leave together
     for (; t < tiles; t += step) {
         const uint32_t in_tile = min(T, a.n - t * T);
         Tile next = load_tile(t + step);
         uint32_t res_len = 0, res_slot = 0, res_status = BNK_PKT_OK; // of the packet of this lane
         bool has_counter = !OPEN && cur.slot < a.max_slots;
         uint64_t res_ctr = cur.ctr;
+#pragma unroll 1
         for (uint32_t k = 0; k < in_tile; k++, buf ^= 1u) {
             const uint32_t off = __shfl_sync(0xffffffffu, cur.off, k), len = __shfl_sync(0xffffffffu, cur.len, k);
             uint32_t slot = __shfl_sync(0xffffffffu, cur.slot, k);
+            bool ahead = true; // another packet's two groups are on their way behind this one's
             if (k + 1 < in_tile) {
                 fetch(__shfl_sync(0xffffffffu, cur.off, k + 1), __shfl_sync(0xffffffffu, cur.len, k + 1),
                       __shfl_sync(0xffffffffu, cur.slot, k + 1), buf ^ 1u);
-                copy_async_wait<1>();
             } else if (t + step < tiles) {
                 load_keypair(next, t + step);
                 fetch(__shfl_sync(0xffffffffu, next.off, 0), __shfl_sync(0xffffffffu, next.len, 0),
                       __shfl_sync(0xffffffffu, next.slot, 0), buf ^ 1u);
-                copy_async_wait<1>();
             } else {
-                copy_async_wait<0>();
+                ahead = false;
             }
-            __syncwarp();
             uint4 *const stage = stage_all[warp][buf];
             uint8_t *const stage_bytes = reinterpret_cast<uint8_t *>(stage);
             Round rd(off, 0);
@@ -700,6 +753,9 @@ __global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __gri
             uint8_t st = BNK_PKT_OK;
             uint32_t body = 0, in_len = 0, n_lo = 0, n_hi = 0;
             if (OPEN) {
+                if (ahead) copy_async_wait<2>();
+                else copy_async_wait<0>();
+                __syncwarp();
                 const bool in_ring = (uint64_t)off + len <= a.ring_bytes, whole = in_ring && len >= BNK_WG_HEADER + BNK_WG_TAG;
                 uint4 hdr = make_uint4(0, 0, 0, 0);
                 if (!(off & 15u) && whole) hdr = stage[stage_at(rd.first)];
@@ -738,8 +794,9 @@ __global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __gri
                 res_len = 0;
             }
             FlowNote note;
-            if (NOTE && !(off & 15u) && (uint64_t)off + BNK_WG_HEADER + len <= a.ring_bytes) {
-                const uint32_t word = stage_word(stage, rd.body); // the IPv4 header and the ports lie in 64 bytes
+            auto note_begin = [&] { // the IPv4 header and the ports lie in 64 bytes
+                if (!NOTE || (off & 15u) || (uint64_t)off + BNK_WG_HEADER + len > a.ring_bytes) return;
+                const uint32_t word = stage_word(stage, rd.body);
                 Parsed p;
                 const uint32_t at = parse_ipv4_words(__shfl_sync(0xffffffffu, word, 0), __shfl_sync(0xffffffffu, word, 2),
                                                      __shfl_sync(0xffffffffu, word, 3), __shfl_sync(0xffffffffu, word, 4), len, p);
@@ -748,9 +805,13 @@ __global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __gri
                     if (at) parse_ports(ports, p);
                     note.begin(a.ft, p, a.now);
                 }
-            }
+            };
             if (st != BNK_PKT_OK) { // the next packet's copies are in the other stage
-                if (NOTE) {
+                if (!OPEN) {
+                    if (ahead) copy_async_wait<2>();
+                    else copy_async_wait<0>();
+                    __syncwarp();
+                    note_begin();
                     note.place(a.ft);
                     note.count(a.ft);
                 }
@@ -766,6 +827,11 @@ __global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __gri
                     ka = kp[0];
                     kb = kp[1];
                 } else {
+                    if (!OPEN) {
+                        if (ahead) copy_async_wait<3>();
+                        else copy_async_wait<1>();
+                        __syncwarp();
+                    }
                     ka = key_all[warp][buf][0];
                     kb = key_all[warp][buf][1];
                 }
@@ -774,105 +840,131 @@ __global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __gri
             }
             const uint32_t remote = OPEN ? 0u : __shfl_sync(0xffffffffu, cur.remote, k);
             P26 r = p26_zero(), state = p26_zero();
+            LanePower power;
             uint32_t pad[4] = {0, 0, 0, 0}, tag[4];
             bool forged = false;
+            uint8_t tag_byte = 0;
+#pragma unroll 1
             for (uint32_t rnd = 0;; rnd++) {
                 const uint32_t done = rnd * kRoundBytes;
                 const uint32_t rb = min(body - done, kRoundBytes); // body bytes of this round
                 const bool last = body - done <= kRoundBytes;
-                if (rnd) { // longer packets: the further rounds are fetched when their turn comes
-                    rd = Round(off, rnd);
-                    __syncwarp(); // the stage is read out
-                    const uint32_t bytes = OPEN ? rb + (last ? BNK_WG_TAG : 0u) : (in_len > done ? min(in_len - done, kRoundBytes) : 0u);
-                    const uint32_t end = rd.body + ((bytes + 15u) >> 4);
-                    for (uint32_t q = lane; q < end; q += 32)
-                        if (q >= rd.body) stage[stage_at(q)] = *reinterpret_cast<const uint4 *>(a.in + rd.window + 16u * q);
-                    __syncwarp();
-                }
-                // ---- keystream and cipher: lane 0 block 0, lane j the j-th block of the round ----
+                const uint32_t data_blocks = (rb + 15u) >> 4, blocks = data_blocks + (last ? 1u : 0u);
+                // ---- keystream: lane 0 block 0, lane j the j-th block of the round ----
                 uint32_t x[16];
-                chacha20_block(x, key, lane == 0 ? 0u : rnd * kRoundBlocks + lane, n_lo, n_hi);
+                chacha20_block<1>(x, key, lane == 0 ? 0u : rnd * kRoundBlocks + lane, n_lo, n_hi);
+                uint32_t steps = 0; // of the lanes' powers: as many as there are bits in the number of lanes that hold blocks
                 if (rnd == 0) {
                     const uint32_t k0 = __shfl_sync(0xffffffffu, x[0], 0), k1 = __shfl_sync(0xffffffffu, x[1], 0);
                     const uint32_t k2 = __shfl_sync(0xffffffffu, x[2], 0), k3 = __shfl_sync(0xffffffffu, x[3], 0);
                     r = p26_words(k0 & 0x0fffffffu, k1 & 0x0ffffffcu, k2 & 0x0ffffffcu, k3 & 0x0ffffffcu, 0u);
 #pragma unroll
                     for (int i = 0; i < 4; i++) pad[i] = __shfl_sync(0xffffffffu, x[4 + i], 0);
-                }
-                const bool works = lane != 0 && (lane - 1u) * 64u < rb;
-                if (works) {
-                    const int in_left = (int)(in_len > done ? min(in_len - done, kRoundBytes) : 0u) - (int)(lane - 1u) * 64;
-                    const int body_left = (int)rb - (int)(lane - 1u) * 64;
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const uint4 v = stage[stage_at(rd.body + 4u * (lane - 1u) + c)];
-                        const uint32_t d[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                        for (int w = 0; w < 4; w++) {
-                            const int at = 16 * c + 4 * w;
-                            x[4 * c + w] = keep_bytes(keep_bytes(d[w], in_left - at) ^ x[4 * c + w], body_left - at);
-                        }
-                    }
+                    power.begin(r);
+                    steps = last ? 32u - __clz((blocks + 3u) / 4u - 1u) : 5u;
                     if (!OPEN) {
-#pragma unroll
-                        for (int c = 0; c < 4; c++)
-                            stage[stage_at(rd.body + 4u * (lane - 1u) + c)] =
-                                make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+#pragma unroll 1
+                        for (; steps; steps--) power.step();
+                        if (ahead) copy_async_wait<2>();
+                        else copy_async_wait<0>();
+                        __syncwarp();
+                        note_begin();
                     }
+                } else { // longer packets: the further rounds are fetched when their turn comes
+                    rd = Round(off, rnd);
+                    __syncwarp(); // the stage is read out
+                    const uint32_t bytes = OPEN ? rb + (last ? BNK_WG_TAG : 0u) : (in_len > done ? min(in_len - done, kRoundBytes) : 0u);
+                    const uint32_t end = rd.body + ((bytes + 15u) >> 4);
+                    const uint32_t extra = !OPEN && last && (rb & 15u) ? rd.body + ((rb + BNK_WG_TAG) >> 4) : 0xffffffffu;
+#pragma unroll 1
+                    for (uint32_t q = lane; q < kStagePieces; q += 32)
+                        if ((q >= rd.body && q < end) || q == extra)
+                            stage[stage_at(q)] = *reinterpret_cast<const uint4 *>(a.in + rd.window + 16u * q);
+                    __syncwarp();
+                }
+                // ---- cipher ----
+                const bool works = lane != 0 && (lane - 1u) * 64u < rb;
+                const int body_left = (int)rb - (int)(lane - 1u) * 64;
+                const uint32_t end_at = 16u * rd.body + rb + lane; // byte `lane` behind the round's body, in the stage
+                uint8_t *const end_byte = stage_bytes + 16u * stage_at(end_at >> 4) + (end_at & 15u);
+                const bool in_last_piece = lane < ((0u - rb) & 15u); // it shares the body's last piece
+                if (!OPEN && in_len < body) { // WireGuard's padding: zeros behind the payload
+                    const uint32_t at = in_len + lane - done;
+                    if (lane < 16u && in_len + lane >= done && at < rb)
+                        stage_bytes[16u * stage_at(rd.body + (at >> 4)) + (at & 15u)] = 0;
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    if (!works || 16 * c >= body_left) continue;
+                    uint4 *const p = &stage[stage_at(rd.body + 4u * (lane - 1u) + c)];
+                    const uint4 v = *p;
+                    x[4 * c + 0] ^= v.x;
+                    x[4 * c + 1] ^= v.y;
+                    x[4 * c + 2] ^= v.z;
+                    x[4 * c + 3] ^= v.w;
+                    if (!OPEN) *p = make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+                }
+                if (!OPEN) { // Poly1305 pads its last block with zeros
+                    __syncwarp();
+                    if (in_last_piece) *end_byte = 0;
                 }
                 if (NOTE && rnd == 0) note.place(a.ft);
                 __syncwarp();
                 // ---- Poly1305 over the ciphertext in the stage ----
-                const uint32_t data_blocks = (rb + 15u) >> 4, blocks = data_blocks + (last ? 1u : 0u);
                 P26 V = p26_zero();
-                {
-                    const int b0 = (int)(4u * lane + blocks) - 128; // the lane's first block; negative: none
-                    if (b0 <= 0 && b0 > -4) V = state;              // (zero in round 0)
-#pragma unroll
-                    for (int s = 0; s < 4; s++) {
-                        const int blk = b0 + s;
-                        if (blk < 0) continue;
-                        uint4 m = make_uint4(0u, 0u, body, 0u); // le64(0) | le64(body)
-                        if ((uint32_t)blk < data_blocks) {
-                            m = stage[stage_at(rd.body + blk)];
-                            const int left = (int)rb - 16 * blk;
-                            if (OPEN && left < 16) {
-                                m.x = keep_bytes(m.x, left);
-                                m.y = keep_bytes(m.y, left - 4);
-                                m.z = keep_bytes(m.z, left - 8);
-                                m.w = keep_bytes(m.w, left - 12);
-                            }
+                const int b0 = (int)(4u * lane + blocks) - 128; // the lane's first block; negative: none
+                if (b0 <= 0 && b0 > -4) V = state;              // (zero in round 0)
+#pragma unroll 1
+                for (int s = 0; s < 4; s++) {
+                    const int blk = b0 + s;
+                    uint4 m = make_uint4(0u, 0u, body, 0u); // le64(0) | le64(body)
+                    if (blk >= 0 && (uint32_t)blk < data_blocks) {
+                        m = stage[stage_at(rd.body + blk)];
+                        const int left = (int)rb - 16 * blk;
+                        if (OPEN && left < 16) {
+                            m.x = keep_bytes(m.x, left);
+                            m.y = keep_bytes(m.y, left - 4);
+                            m.z = keep_bytes(m.z, left - 8);
+                            m.w = keep_bytes(m.w, left - 12);
                         }
-                        V = p26_mul(p26_add(V, p26_words(m.x, m.y, m.z, m.w, 1u)), r);
+                    }
+                    const P26 next_v = p26_mul(p26_add(V, p26_words(m.x, m.y, m.z, m.w, 1u)), r);
+                    if (blk >= 0) V = next_v;
+                    if (OPEN && steps) { // beside the Horner step: neither waits for the other
+                        power.step();
+                        steps--;
                     }
                 }
-                P26 pw = p26_mul(r, r);
-                pw = p26_mul(pw, pw);
-                const uint32_t lanes_used = (blocks + 3u) >> 2;
-                for (uint32_t span = 1; span < lanes_used; span <<= 1) {
-                    const P26 sum = p26_add(p26_mul(p26_shfl_up(V, span), pw), V);
-                    if (((lane + 1u) & (2u * span - 1u)) == 0) V = sum;
-                    pw = p26_mul(pw, pw);
+                if (OPEN && steps) power.step();
+                V = p26_mul(V, power.p);
+#pragma unroll
+                for (int d = 16; d; d >>= 1) { // limbs below 2^27: the sum of 32 of them fits a word
+#pragma unroll
+                    for (int i = 0; i < 5; i++) V.v[i] += __shfl_xor_sync(0xffffffffu, V.v[i], d);
                 }
-                state = p26_shfl(V, 31);
+                state = p26_carry(V);
                 // ---- tag, output ----
                 if (last) {
                     p26_finish(state, pad, tag);
                     const uint32_t tw = (lane & 8u) ? ((lane & 4u) ? tag[3] : tag[2]) : ((lane & 4u) ? tag[1] : tag[0]);
                     const uint8_t tb = (uint8_t)(tw >> (8u * (lane & 3u)));
-                    const uint32_t at = 16u * rd.body + rb + lane;
-                    uint8_t *const p = stage_bytes + 16u * stage_at(at >> 4) + (at & 15u);
-                    if (OPEN) forged = __any_sync(0xffffffffu, lane < 16u && *p != tb);
-                    else if (lane < 16u) *p = tb;
+                    if (OPEN) {
+                        tag_byte = *end_byte;
+                        forged = __any_sync(0xffffffffu, lane < 16u && tag_byte != tb);
+                    } else if (lane < 16u) {
+                        *end_byte = tb;
+                    }
                 }
                 if (OPEN) {
                     __syncwarp(); // ciphertext and tag are read
-                    if (works) {
 #pragma unroll
-                        for (int c = 0; c < 4; c++)
+                    for (int c = 0; c < 4; c++)
+                        if (works && 16 * c < body_left)
                             stage[stage_at(rd.body + 4u * (lane - 1u) + c)] =
                                 forged ? make_uint4(0, 0, 0, 0) : make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
-                    }
+                    __syncwarp();
+                    if (last && in_last_piece) *end_byte = tag_byte; // what is not plaintext goes back as it came
                 } else if (rnd == 0 && lane == 0) {
                     stage[stage_at(rd.first)] = make_uint4(4u, remote, n_lo, n_hi);
                 }
@@ -892,18 +984,13 @@ __global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __gri
                             make_uint4(__byte_perm(w3, 0, 0x0123), (uint32_t)p.sport << 16 | p.dport,
                                        p.proto | (at != kParseBad ? kInnerParses : 0u) | (is_whole ? kInnerWhole : 0u), total);
                 }
-                const uint32_t out_bytes = OPEN ? rb : rb + (last ? BNK_WG_TAG : 0u);
-                const uint32_t whole_end = rd.body + (out_bytes >> 4), rest = out_bytes & 15u;
-                for (uint32_t q = lane; q < whole_end; q += 32) {
+                const uint32_t out_end = rd.body + (((OPEN ? rb : rb + (last ? BNK_WG_TAG : 0u)) + 15u) >> 4);
+#pragma unroll 1
+                for (uint32_t q = lane; q < out_end; q += 32) {
                     if (q < (OPEN ? rd.body : rd.first)) continue;
                     const uint4 v = stage[stage_at(q)];
                     *reinterpret_cast<uint4 *>(a.out + rd.window + 16u * q) = v;
                     if (a.out2) *reinterpret_cast<uint4 *>(a.out2 + rd.window + 16u * q) = v;
-                }
-                if (lane < rest) {
-                    const uint8_t v = stage_bytes[16u * stage_at(whole_end) + lane];
-                    a.out[rd.window + 16u * whole_end + lane] = v;
-                    if (a.out2) a.out2[rd.window + 16u * whole_end + lane] = v;
                 }
                 if (last) break;
             }
@@ -923,8 +1010,17 @@ __global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __gri
             if (NOTE) note.count(a.ft);
             __syncwarp(); // the stage may be filled again
         }
-        const uint32_t i = t * T + lane;
-        if (lane < in_tile) {
+        if (by_cta) {
+            if (lane == 0) {
+                cta_len[warp] = res_len;
+                cta_ctr[warp] = res_ctr;
+                cta_status[warp] = (uint8_t)res_status;
+                cta_has[warp] = has_counter;
+                if (a.res[0].slot) a.res[0].slot[t] = res_slot;
+                if (a.res[1].slot) a.res[1].slot[t] = res_slot;
+            }
+        } else if (lane < in_tile) {
+            const uint32_t i = t * T + lane;
 #pragma unroll
             for (int d = 0; d < 2; d++) {
                 const AeadResults &o = a.res[d];
@@ -936,9 +1032,20 @@ __global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __gri
         }
         cur = next;
     }
-    signal_done(a.done, [&] {
-        if (NOTE && a.flow_report) flow_report(flow_ctl(a.ft), a.flow_report);
-    });
+    if (by_cta) {
+        __syncthreads();
+        const uint32_t i = blockIdx.x * kWppWarps + threadIdx.x;
+        if (threadIdx.x < kWppWarps && i < a.n) {
+#pragma unroll
+            for (int d = 0; d < 2; d++) {
+                const AeadResults &o = a.res[d];
+                if (o.status) o.status[i] = cta_status[threadIdx.x];
+                if (o.out_len) o.out_len[i] = cta_len[threadIdx.x];
+                if (o.counter && cta_has[threadIdx.x]) o.counter[i] = cta_ctr[threadIdx.x];
+            }
+        }
+    }
+    signal_done(a.done, NOTE && a.flow_report, [&] { flow_report(flow_ctl(a.ft), a.flow_report); });
 }
 
 // Below this many packets one-packet-per-thread leaves most of the GPU idle and its run time is that of one thread
@@ -949,18 +1056,32 @@ __global__ void __launch_bounds__(32 * kWppWarps, 2) aead_wpp_kernel(const __gri
 #endif
 
 // Tiles and grid of a warp-per-packet launch.  Rings in device memory (n <= BNK_WPP_MAX_PACKETS): a warp per packet.
-// Rings in host memory: the link is the bound, kHostCtas CTAs keep it busy and more make it slower (see the kernel);
-// from 8 packets a warp on, warps take tiles of 8, whose descriptors are whole 32-byte reads.
-#ifndef BNK_HOST_CTAS
-#define BNK_HOST_CTAS 128u
-#endif
+// Rings in host memory: the link is the bound.  With a warp per packet all reads are asked for at once, end together and
+// leave the writes for afterwards, so beyond kLinkWindow bytes a warp takes several packets: 1024 x 1420 B sealed by
+// 32 to 96 CTAs 72 us, by 128 84, by 256 (a packet each) 92; 512 x 1420 46 against 54.  Small packets are bound by what
+// a warp computes, and want more warps: 4096 x 300 B 104 us from 64 CTAs, 77 from 128 to 192, 92 from 512; 131,072 x 64 B
+// 2.6 ms from 64, 1.16 from 256, 1.01 from 512.  Tiles of 2, 4 or 8 make descriptors and results one access.
+constexpr uint64_t kLinkWindow = 64u << 10, kLeastCtas = 64, kMostCtas = 512;
 void wpp_grid(AeadArgs &a, uint32_t &ctas) {
-    const uint32_t all = (a.n + kWppWarps - 1) / kWppWarps;
+    ctas = (a.n + kWppWarps - 1) / kWppWarps;
     a.tile = 1;
-    ctas = all;
-    if (!a.over_link || all <= BNK_HOST_CTAS) return;
-    ctas = BNK_HOST_CTAS;
-    while (a.tile < 8 && (uint64_t)a.n > (uint64_t)ctas * kWppWarps * a.tile * 4u) a.tile *= 2;
+    if (!a.over_link || ctas <= kLeastCtas) return;
+    const uint64_t per_packet = a.link_bytes / a.n + 1;
+    ctas = (uint32_t)std::min<uint64_t>(ctas, std::min(std::max(kLinkWindow / per_packet, kLeastCtas), kMostCtas));
+    while (a.tile < 8 && a.n > ctas * kWppWarps * a.tile) a.tile *= 2;
+}
+template <bool OPEN, bool NOTE>
+cudaError_t launch_wpp(const AeadArgs &a, uint32_t ctas, const HostDesc *h, cudaStream_t s) {
+    // A launch that may start early costs the driver 2.7 us more when the stream's last kernel is just about to end, as it
+    // is when a caller comes back right after its wait; only where a kernel of the same submit is in front does it pay.
+    const bool early = a.behind_kernel;
+    if (h == nullptr)
+        return launch_kernel(early, aead_wpp_kernel<OPEN, NOTE, false>, dim3(ctas), dim3(32 * kWppWarps), s, a, InlineDesc<false>{});
+    InlineDesc<true> d;
+    memcpy(d.off, h->off, a.n * sizeof(uint32_t));
+    memcpy(d.len, h->len, a.n * sizeof(uint32_t));
+    memcpy(d.slot, h->slot, a.n * sizeof(uint32_t));
+    return launch_kernel(early, aead_wpp_kernel<OPEN, NOTE, true>, dim3(ctas), dim3(32 * kWppWarps), s, a, d);
 }
 
 template <bool OPEN>
@@ -970,8 +1091,10 @@ cudaError_t launch_aead(AeadArgs a, cudaStream_t s, bnk_ctx *ctx) {
     if (wpp) {
         uint32_t ctas;
         wpp_grid(a, ctas);
-        auto *const kernel = !OPEN && a.note ? aead_wpp_kernel<OPEN, !OPEN> : aead_wpp_kernel<OPEN, false>;
-        cudaError_t e = launch_after_kernel(kernel, dim3(ctas), dim3(32 * kWppWarps), s, a);
+        // Up to kInlineMax descriptors go with the launch: a read of them over the host link costs 1.4 us before the
+        // first byte of a packet can be asked for.
+        const HostDesc *const h = a.over_link && a.n <= kInlineMax ? &a.host : nullptr;
+        cudaError_t e = !OPEN && a.note ? launch_wpp<OPEN, !OPEN>(a, ctas, h, s) : launch_wpp<OPEN, false>(a, ctas, h, s);
         if (e != cudaSuccess) return e;
     } else {
         // one CTA per 128 packets; the hardware hands CTAs to SMs as slots free up, which measured faster

@@ -51,14 +51,16 @@ cudaError_t dev_alloc_zero(T **p, size_t count) {
     return cudaMemset(*p, 0, count * sizeof(T));
 }
 
-// highest ring byte any of the first n packets can touch (input or output side)
-uint64_t ring_extent(const bnk_batch *b, uint32_t n, uint32_t slack) {
+// highest ring byte any of the first n packets can touch (input or output side), and their bytes
+uint64_t ring_extent(const bnk_batch *b, uint32_t n, uint32_t slack, uint64_t *bytes = nullptr) {
     const uint32_t *off = b->host.off, *len = b->host.len;
-    uint64_t ext = 0;
+    uint64_t ext = 0, sum = 0;
     for (uint32_t i = 0; i < n; i++) {
         const uint64_t e = (uint64_t)off[i] + len[i] + slack;
         if (e > ext) ext = e;
+        sum += len[i];
     }
+    if (bytes) *bytes = sum + (uint64_t)n * slack;
     ext = (ext + 15) & ~15ull;
     return ext > b->ring_bytes ? b->ring_bytes : ext;
 }
@@ -279,7 +281,6 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     if ((e = dev_alloc_zero(&ctx->kt.recv_keys, k * 8)) != cudaSuccess) return bail("recv_keys", e);
     if ((e = dev_alloc_zero(&ctx->kt.remote_index, k)) != cudaSuccess) return bail("remote_index", e);
     if ((e = dev_alloc_zero(&ctx->kt.send_counter, k)) != cudaSuccess) return bail("send_counter", e);
-    if ((e = dev_alloc_zero(&ctx->kt.arrived, k)) != cudaSuccess) return bail("arrived", e);
     if ((e = dev_alloc_zero(&ctx->kt.replay_last, k)) != cudaSuccess) return bail("replay_last", e);
     if ((e = dev_alloc_zero(&ctx->kt.replay_next, k)) != cudaSuccess) return bail("replay_next", e);
     if ((e = dev_alloc_zero(&ctx->kt.replay_ring, k * cfg->replay_ring_blocks)) != cudaSuccess) return bail("replay_ring", e);
@@ -313,7 +314,6 @@ int bnk_ctx_destroy(bnk_ctx *ctx) {
     cudaFree(ctx->kt.recv_keys);
     cudaFree(ctx->kt.remote_index);
     cudaFree(ctx->kt.send_counter);
-    cudaFree(ctx->kt.arrived);
     cudaFree(ctx->kt.replay_last);
     cudaFree(ctx->kt.replay_next);
     cudaFree(ctx->kt.replay_ring);
@@ -347,7 +347,7 @@ int bnk_keypair_set_many(bnk_ctx *ctx, uint32_t first_slot, uint32_t n, const ui
     CK(ctx, cudaMemcpy(ctx->kt.send_keys + (size_t)first_slot * 8, send_keys, (size_t)n * 32, cudaMemcpyHostToDevice));
     CK(ctx, cudaMemcpy(ctx->kt.recv_keys + (size_t)first_slot * 8, recv_keys, (size_t)n * 32, cudaMemcpyHostToDevice));
     CK(ctx, cudaMemcpy(ctx->kt.remote_index + first_slot, remote_index, (size_t)n * 4, cudaMemcpyHostToDevice));
-    CK(ctx, cudaMemset(ctx->kt.send_counter + first_slot, 0, (size_t)n * 8));
+    CK(ctx, cudaMemset(ctx->kt.send_counter + first_slot, 0, (size_t)n * sizeof(SendCounter)));
     CK(ctx, cudaMemset(ctx->kt.replay_last + first_slot, 0, (size_t)n * 8));
     CK(ctx, cudaMemset(ctx->kt.replay_ring + (size_t)first_slot * rb, 0, (size_t)n * rb * 8));
     CK(ctx, cudaMemset(ctx->kt.allowed_ip + first_slot, 0, (size_t)n * 4));
@@ -374,14 +374,17 @@ int bnk_keypair_clear(bnk_ctx *ctx, uint32_t slot) {
 int bnk_send_counter_get(bnk_ctx *ctx, uint32_t slot, uint64_t *counter) {
     if (!ctx || !counter || slot >= ctx->cfg.max_keypairs) return fail(ctx, BNK_EINVAL, "bad slot");
     CK(ctx, cudaSetDevice(ctx->device));
-    CK(ctx, cudaMemcpy(counter, ctx->kt.send_counter + slot, 8, cudaMemcpyDeviceToHost));
+    SendCounter c;
+    CK(ctx, cudaMemcpy(&c, ctx->kt.send_counter + slot, sizeof c, cudaMemcpyDeviceToHost));
+    *counter = c.e[c.e[0].seq >= c.e[1].seq ? 0 : 1].value;
     return BNK_SUCCESS;
 }
 
 int bnk_send_counter_set(bnk_ctx *ctx, uint32_t slot, uint64_t counter) {
     if (!ctx || slot >= ctx->cfg.max_keypairs) return fail(ctx, BNK_EINVAL, "bad slot");
     CK(ctx, cudaSetDevice(ctx->device));
-    CK(ctx, cudaMemcpy(ctx->kt.send_counter + slot, &counter, 8, cudaMemcpyHostToDevice));
+    const SendCounter c{{{counter, 0}, {0, 0}}};
+    CK(ctx, cudaMemcpy(ctx->kt.send_counter + slot, &c, sizeof c, cudaMemcpyHostToDevice));
     return BNK_SUCCESS;
 }
 
@@ -842,7 +845,7 @@ int bnk_batch_download(bnk_batch *b, uint32_t npkts) {
 
 // A seal that works on the pinned ring and descriptors: one launch up to kRankMax packets, else one more in front of
 // it for the counters, and one behind it when expired flows may have to be swept.
-static int seal_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_unix_ns) {
+static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t flags, int64_t now_unix_ns) {
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0, stats = (flags & BNK_F_STATS) != 0;
@@ -852,6 +855,8 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, false, nullptr);
     a.over_link = true;
+    a.host = HostDesc{h.off, h.len, h.slot};
+    a.link_bytes = bytes;
     a.in = a.out = h.ring;
     a.off = h.off;
     a.len = h.len;
@@ -863,9 +868,10 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now
         a.res[0].counter = h.counter;
         if (npkts <= kRankMax) {
             a.send_counter = ctx->kt.send_counter;
-            a.arrived = ctx->kt.arrived;
+            a.seal_seq = ++ctx->seal_seq;
         } else {
             a.counter = b->dev.counter;
+            a.behind_kernel = true;
             CK(ctx, launch_assign_counters(b, npkts, h.slot, b->dev.counter, s));
         }
     }
@@ -908,8 +914,9 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     const size_t n = npkts;
     // header room + payload + padding (< 16) + tag
     const bool refresh = b->dev_stale; // the device copies are behind the host arrays: upload whatever the flags say
-    const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, 16 + 16 + 16);
-    if (ctx->aead_mode != 1 && host_direct(b, npkts, flags, ext)) return seal_direct(b, npkts, flags, now_unix_ns);
+    uint64_t bytes = 0;
+    const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, 16 + 16 + 16, &bytes);
+    if (ctx->aead_mode != 1 && host_direct(b, npkts, flags, ext)) return seal_direct(b, npkts, bytes, flags, now_unix_ns);
     if ((!(flags & BNK_F_NO_H2D) || refresh) && n) {
         if (b->joint_copy) {
             CK(ctx, cudaMemcpyAsync(b->d_desc, b->h_desc, b->desc_room + ext, cudaMemcpyHostToDevice, s));
@@ -945,6 +952,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     }
     AeadArgs a = aead_args(b, npkts, false, order);
     a.res[0].counter = nullptr; // in place already
+    a.behind_kernel = true;
     const bool side = b->aead_stream && npkts >= ctx->aead_side_stream_from;
     cudaStream_t as = side ? b->aead_stream : s;
     if (side) {
@@ -976,7 +984,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
 
 // An open that works on the pinned ring and descriptors.  What has to wait for the replay window (statuses, lengths)
 // stays on the device until then, with the packets' inner headers, so that no later kernel goes back to the ring.
-static int open_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_unix_ns) {
+static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t flags, int64_t now_unix_ns) {
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0, stats = (flags & BNK_F_STATS) != 0;
@@ -987,6 +995,8 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, true, nullptr);
     a.over_link = true;
+    a.host = HostDesc{h.off, h.len, h.slot};
+    a.link_bytes = bytes;
     a.in = a.out = h.ring;
     a.off = h.off;
     a.len = h.len;
@@ -1057,8 +1067,9 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     const bool timed = (flags & BNK_F_TIMED) != 0;
     const size_t n = npkts;
     const bool refresh = b->dev_stale;
-    const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, (flags & BNK_F_USE_OUT_LEN) ? 48 : 0);
-    if (ctx->aead_mode != 1 && host_direct(b, npkts, flags, ext)) return open_direct(b, npkts, flags, now_unix_ns);
+    uint64_t bytes = 0;
+    const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, (flags & BNK_F_USE_OUT_LEN) ? 48 : 0, &bytes);
+    if (ctx->aead_mode != 1 && host_direct(b, npkts, flags, ext)) return open_direct(b, npkts, bytes, flags, now_unix_ns);
     // BNK_F_USE_OUT_LEN reads the lengths a seal left on the device: an upload beside it must not bring the
     // host's out_len along, so it moves the fields one by one instead of the whole slab.
     if ((!(flags & BNK_F_NO_H2D) || refresh) && n) {
@@ -1081,6 +1092,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
         order = b->dev.len_order;
     }
     oa.order = order;
+    oa.behind_kernel = true;
     const bool replay = (flags & BNK_F_REPLAY) && n, one_launch = npkts <= kGroupMax;
     if (replay && !one_launch) {
         // grouping by keypair needs only the descriptors: it runs on the side stream beside the open kernel

@@ -19,12 +19,21 @@
 // lives here, indexed by keypair slot, so that peers shard across GPUs with no
 // exchange: keys, send counter, replay window.
 // ---------------------------------------------------------------------------
+// Next nonce of a keypair.  The packets of one seal launch read it and one of them moves it on, with nothing to order
+// them by: so a launch never writes the entry its packets read.  The entry with the higher `seq` counts; the launch that
+// carries the number q (ctx->seal_seq, rising) looks at entries below q only and writes the other one, as {value, q}.
+// Kernels that separate their reads from their writes by a barrier change the entry in place.
+struct alignas(32) SendCounter {
+    struct alignas(16) Entry {
+        uint64_t value, seq;
+    } e[2];
+};
+
 struct KeypairTables {
     uint32_t *send_keys;    // [max_keypairs][8] little-endian words
     uint32_t *recv_keys;    // [max_keypairs][8]
     uint32_t *remote_index; // [max_keypairs] receiver index written into sealed headers
-    uint64_t *send_counter; // [max_keypairs] next nonce to hand out
-    uint32_t *arrived;      // [max_keypairs] scratch of the seal kernel that hands out counters itself, zero between launches
+    SendCounter *send_counter; // [max_keypairs] next nonce to hand out
     uint64_t *replay_last;  // [max_keypairs] highest counter accepted
     uint64_t *replay_next;  // [max_keypairs] scratch: the value replay_last takes after the batch in flight
     uint64_t *replay_ring;  // [max_keypairs][ring_blocks] RFC 6479 bitmap ring
@@ -92,6 +101,7 @@ struct bnk_ctx {
     uint32_t aead_side_stream_from; // batches of at least this many packets run seal/open on the low-priority stream (BNK_AEAD_SIDE_STREAM_FROM; 0 = never)
     int prio_low, prio_high;        // stream priority range of the device
     std::atomic<uint64_t> launches;
+    std::atomic<uint64_t> seal_seq{0}; // number of the last seal launch that handed out nonces itself (see SendCounter)
     std::mutex mu;
     std::string last_error;
     // Submits hold this shared while they queue their work; whoever changes what running kernels of other
@@ -260,20 +270,28 @@ struct Done {
     uint32_t *flag;   // pinned; null: nobody watches
     uint32_t value;
 };
-// By all threads of all CTAs, once, at the end; `last_words` runs in one thread when every CTA's stores are visible.
+// By all threads of all CTAs, once, at the end; `last_words` (if `has_words`) runs in one thread when every CTA's stores
+// are visible.  A fence that covers host memory takes ~1.5 us, so there is no second one when nothing is said.
 template <typename F>
-__device__ __forceinline__ void signal_done(const Done &d, F last_words) {
+__device__ __forceinline__ void signal_done(const Done &d, bool has_words, F last_words) {
     if (d.flag == nullptr) return;
     __syncthreads();
     if (threadIdx.x != 0) return;
     __threadfence_system(); // the CTA's stores, to host memory too, before its ticket
-    if (gridDim.x != 1 && atomicAdd(d.ticket, 1u) + 1u != gridDim.x) return;
-    *d.ticket = 0u;
-    __threadfence();
-    last_words();
-    __threadfence_system();
+    if (gridDim.x != 1) { // the other CTAs' stores have arrived when their tickets are out: their fences were before
+        if (atomicAdd(d.ticket, 1u) + 1u != gridDim.x) return;
+        *d.ticket = 0u;
+    }
+    if (has_words) {
+        __threadfence();
+        last_words();
+        __threadfence_system();
+    }
     *(volatile uint32_t *)d.flag = d.value;
 }
+struct HostDesc { // the descriptors where the host can read them
+    const uint32_t *off, *len, *slot;
+};
 struct AeadArgs {
     const uint8_t *in;            // ring the input is read from and ...
     uint8_t *out, *out2;          // ... ring(s) the output goes to; thread per packet: in == out, no out2
@@ -292,15 +310,18 @@ struct AeadArgs {
     bool demux;                   // open, warp per packet: the slot comes from the header's receiver index
     bool inner_cut;               // packets will be cut to their IPv4 total length
     uint4 *inner;                 // open, warp per packet: headers of the plaintexts (see VerdictArgs); null: not wanted
+    bool behind_kernel;           // a kernel of the same submit is in front
     bool over_link;               // a ring is in host memory
+    HostDesc host;                // with over_link
+    uint64_t link_bytes;          // with over_link: bytes of the packets
     uint32_t n;
     uint32_t tile;                // set by the launcher
     uint32_t mtu;
     uint32_t max_slots;
     uint64_t ring_bytes;
     // Seal of up to kRankMax packets in pinned memory: nonces are handed out by the seal kernel itself (null: from counter[])
-    uint64_t *send_counter;       // [max_slots]
-    uint32_t *arrived;            // [max_slots] packets of the slot that have read their counter; zero between launches
+    SendCounter *send_counter;    // [max_slots]
+    uint64_t seal_seq;
     // Seal in pinned memory with BNK_F_NOTE_OUTBOUND: the kernel records its packets' flows
     bool note;
     long long now;
@@ -355,6 +376,25 @@ cudaError_t launch_tally(bnk_batch *b, uint32_t n, cudaStream_t s);
 cudaError_t launch_demux_index(bnk_batch *b, uint32_t n, const uint32_t *len, cudaStream_t s);
 cudaError_t launch_inner_check(bnk_batch *b, uint32_t n, cudaStream_t s);
 cudaError_t launch_classify(bnk_batch *b, uint32_t n, cudaStream_t s);
+// One 16-byte entry in one access, from and to the L2 that all SMs share.
+__device__ __forceinline__ SendCounter::Entry counter_load(const SendCounter::Entry *p) {
+    SendCounter::Entry v;
+    asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }" : "=l"(v.value), "=l"(v.seq) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void counter_store(SendCounter::Entry *p, SendCounter::Entry v) {
+    asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(p), "l"(v.value), "l"(v.seq) : "memory");
+}
+struct CounterRead {
+    SendCounter::Entry now;
+    uint32_t at; // which entry that is
+};
+// The entry that counts, of those below `below` (~0: of both).
+__device__ __forceinline__ CounterRead counter_read(const SendCounter *c, uint64_t below) {
+    const SendCounter::Entry a = counter_load(&c->e[0]), b = counter_load(&c->e[1]);
+    const bool first = a.seq < below && (b.seq >= below || a.seq >= b.seq);
+    return CounterRead{first ? a : b, first ? 0u : 1u};
+}
 // nonce of the k-th packet of a run that starts at `base`: never past the message limit
 __device__ __forceinline__ uint64_t saturating_counter(uint64_t base, uint32_t k) {
     const uint64_t c = base + k;

@@ -247,23 +247,24 @@ __device__ __forceinline__ uint32_t run_start(const uint32_t *keys, uint32_t j) 
     return lo;
 }
 __global__ void assign_counters_kernel(const uint32_t *keys, const uint32_t *order, uint32_t n, uint32_t max_slots,
-                                       const uint64_t *send_counter, uint64_t *counter_out) {
+                                       const SendCounter *send_counter, uint64_t *counter_out) {
     let_next_kernel_start();
     wait_for_kernel_in_front();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const uint32_t slot = keys[j];
     if (slot >= max_slots) return;
-    counter_out[order[j]] = saturating_counter(send_counter[slot], j - run_start(keys, j));
+    counter_out[order[j]] = saturating_counter(counter_read(&send_counter[slot], ~0ull).now.value, j - run_start(keys, j));
 }
-__global__ void advance_counters_kernel(const uint32_t *keys, uint32_t n, uint32_t max_slots, uint64_t *send_counter) {
+__global__ void advance_counters_kernel(const uint32_t *keys, uint32_t n, uint32_t max_slots, SendCounter *send_counter) {
     let_next_kernel_start();
     wait_for_kernel_in_front();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const uint32_t slot = keys[j];
     if (slot >= max_slots || (j + 1 < n && keys[j + 1] == slot)) return; // the last packet of a run moves the counter
-    send_counter[slot] = saturating_counter(send_counter[slot], j - run_start(keys, j) + 1);
+    const CounterRead c = counter_read(&send_counter[slot], ~0ull);
+    counter_store(&send_counter[slot].e[c.at], SendCounter::Entry{saturating_counter(c.now.value, j - run_start(keys, j) + 1), c.now.seq});
 }
 
 // --- anti-replay window, RFC 6479 -------------------------------------------------------
@@ -616,7 +617,7 @@ __global__ void __launch_bounds__(256) verdict_kernel(const __grid_constant__ Ve
     wait_for_kernel_in_front();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < v.n) final_verdict(v, i);
-    signal_done(done, [] {});
+    signal_done(done, false, [] {});
 }
 
 // --- the whole ordering work of a batch of up to kGroupMax packets in one launch --------
@@ -635,7 +636,7 @@ struct GroupArgs {
     SortKeySrc src;
     uint32_t n, passes, digit_bits, max_slots;
     // counters (send_counter != nullptr)
-    uint64_t *send_counter;
+    SendCounter *send_counter;
     uint64_t *counter_out; // per packet
     // replay window (replay): rp.keys and rp.order are written here
     uint32_t *keys_out, *order_out;
@@ -801,21 +802,21 @@ __global__ void __launch_bounds__(kGroupThreads) group_kernel(const __grid_const
             cluster.sync();
             for (uint32_t c = 0; c < me; c++) front = max(front, *cluster.map_shared_rank(&cta_head, c));
         }
-        uint64_t next_counter[ITEMS];
+        CounterRead counter[ITEMS];
 #pragma unroll
         for (int k = 0; k < ITEMS; k++) {
             const uint32_t p = first + at0 + k;
             if (head[k]) front = p + 1;
             if (at0 + k >= mine || slot[k] >= a.max_slots) continue;
-            const uint64_t base = a.send_counter[slot[k]];
+            counter[k] = counter_read(&a.send_counter[slot[k]], ~0ull);
             const uint32_t rank = p + 1 - front;
-            a.counter_out[vbuf(f)[at0 + k]] = saturating_counter(base, rank);
-            next_counter[k] = saturating_counter(base, rank + 1);
+            a.counter_out[vbuf(f)[at0 + k]] = saturating_counter(counter[k].now.value, rank);
+            counter[k].now.value = saturating_counter(counter[k].now.value, rank + 1);
         }
         all_sync(); // every counter is read
 #pragma unroll
         for (int k = 0; k < ITEMS; k++)
-            if (tail[k] && slot[k] < a.max_slots) a.send_counter[slot[k]] = next_counter[k];
+            if (tail[k] && slot[k] < a.max_slots) counter_store(&a.send_counter[slot[k]].e[counter[k].at], counter[k].now);
     }
 
     if (a.replay) {
@@ -871,7 +872,7 @@ __global__ void __launch_bounds__(kGroupThreads) group_kernel(const __grid_const
     if (a.verdict.n)
         for (uint32_t i = tid; i < mine; i += kGroupThreads) final_verdict(a.verdict, first + i);
     if (ctas > 1) cluster.sync(); // nobody leaves while another may still look into its shared memory
-    signal_done(a.done, [] {});
+    signal_done(a.done, false, [] {});
 }
 
 // --- scheduling order by length class (mixed packet sizes) ------------------------------
