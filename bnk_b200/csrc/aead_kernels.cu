@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
     let_next_kernel_start(); // open side: the grouping + replay launch behind may take its place already
     // What a ring in device memory holds may come from the kernel in front; a pinned ring and its descriptors are the
     // host's, and only the counters of a seal come from there.
-    if (!a.over_link) wait_for_kernel_in_front();
+    if (!a.from_host) wait_for_kernel_in_front();
     __shared__ __align__(128) uint4 stage_all[kWppWarps][2][kStagePieces];
     __shared__ __align__(16) uint4 key_all[kWppWarps][2][2];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -694,12 +694,12 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
     __shared__ uint32_t slots[INLINE ? kRankMax : 1];
     CounterRead counter{};
     const bool hands_out = INLINE && !OPEN && a.send_counter;
-    if (OPEN || !a.behind_kernel || !a.over_link) load_keypair(cur, t);
+    if (OPEN || !a.behind_kernel || !a.from_host) load_keypair(cur, t);
     if (hands_out && t < tiles && lane == 0 && cur.slot < a.max_slots) counter = counter_read(&a.send_counter[cur.slot], a.seal_seq);
     if (t < tiles) fetch(__shfl_sync(0xffffffffu, cur.off, 0), __shfl_sync(0xffffffffu, cur.len, 0),
                          __shfl_sync(0xffffffffu, cur.slot, 0), 0);
-    if (a.over_link) wait_for_kernel_in_front();
-    if (!OPEN && a.behind_kernel && a.over_link) load_keypair(cur, t);
+    if (a.from_host) wait_for_kernel_in_front();
+    if (!OPEN && a.behind_kernel && a.from_host) load_keypair(cur, t);
     if constexpr (INLINE && !OPEN) {
         if (hands_out) { // one tile of one packet per warp
             for (uint32_t i = threadIdx.x; i < a.n; i += blockDim.x) slots[i] = desc.slot[i];
@@ -984,13 +984,21 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                             make_uint4(__byte_perm(w3, 0, 0x0123), (uint32_t)p.sport << 16 | p.dport,
                                        p.proto | (at != kParseBad ? kInnerParses : 0u) | (is_whole ? kInnerWhole : 0u), total);
                 }
-                const uint32_t out_end = rd.body + (((OPEN ? rb : rb + (last ? BNK_WG_TAG : 0u)) + 15u) >> 4);
+                // The last piece goes out whole where the bytes behind the message were read from the same place.
+                const uint32_t out_bytes = OPEN ? rb : rb + (last ? BNK_WG_TAG : 0u);
+                const bool other_place = a.in != a.out;
+                const uint32_t out_end = rd.body + ((out_bytes + (other_place ? 0u : 15u)) >> 4);
 #pragma unroll 1
                 for (uint32_t q = lane; q < out_end; q += 32) {
                     if (q < (OPEN ? rd.body : rd.first)) continue;
                     const uint4 v = stage[stage_at(q)];
                     *reinterpret_cast<uint4 *>(a.out + rd.window + 16u * q) = v;
                     if (a.out2) *reinterpret_cast<uint4 *>(a.out2 + rd.window + 16u * q) = v;
+                }
+                if (other_place && lane < (out_bytes & 15u)) {
+                    const uint8_t v = stage_bytes[16u * stage_at(out_end) + lane];
+                    a.out[rd.window + 16u * out_end + lane] = v;
+                    if (a.out2) a.out2[rd.window + 16u * out_end + lane] = v;
                 }
                 if (last) break;
             }
@@ -1093,7 +1101,7 @@ cudaError_t launch_aead(AeadArgs a, cudaStream_t s, bnk_ctx *ctx) {
         wpp_grid(a, ctas);
         // Up to kInlineMax descriptors go with the launch: a read of them over the host link costs 1.4 us before the
         // first byte of a packet can be asked for.
-        const HostDesc *const h = a.over_link && a.n <= kInlineMax ? &a.host : nullptr;
+        const HostDesc *const h = a.from_host && a.n <= kInlineMax ? &a.host : nullptr;
         cudaError_t e = !OPEN && a.note ? launch_wpp<OPEN, !OPEN>(a, ctas, h, s) : launch_wpp<OPEN, false>(a, ctas, h, s);
         if (e != cudaSuccess) return e;
     } else {

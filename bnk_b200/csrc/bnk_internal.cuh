@@ -180,6 +180,7 @@ struct bnk_batch {
     cudaEvent_t k_begin, k_end, t_end, a_begin, a_end;
     bool in_flight;
     bool dev_stale; // a submit ran on the host arrays: the device copies of ring and descriptors are behind
+    bool ring_partial;   // of the device ring only packets and super-packets are those of the host ring
     bool counted;        // this batch is one of ctx->in_flight
     uint64_t direct_counted; // what it adds to ctx->direct_in_flight
     // bnk_wait watches *h_done for done_seq when done_watched: the last kernel of the submit stores it (Done)
@@ -312,7 +313,8 @@ struct AeadArgs {
     uint4 *inner;                 // open, warp per packet: headers of the plaintexts (see VerdictArgs); null: not wanted
     bool behind_kernel;           // a kernel of the same submit is in front
     bool over_link;               // a ring is in host memory
-    HostDesc host;                // with over_link
+    bool from_host;               // the ring that is read and the descriptors are
+    HostDesc host;                // with from_host
     uint64_t link_bytes;          // with over_link: bytes of the packets
     uint32_t n;
     uint32_t tile;                // set by the launcher
@@ -350,8 +352,8 @@ uint32_t replay_scan_tiles(uint32_t max_pkts);     // tiles of the running-maxim
 uint32_t replay_hash_capacity(uint32_t max_pkts);  // entries of the duplicate-counter table
 
 // filter_kernels.cu
-cudaError_t launch_filter_note(bnk_batch *b, uint32_t n, long long now_ns, cudaStream_t s); // the inserts; no sweep
-cudaError_t launch_filter_check(bnk_batch *b, uint32_t n, long long now_ns, bool only_status_ok, cudaStream_t s);
+cudaError_t launch_filter_note(bnk_batch *b, uint32_t n, long long now_ns, const Done &done, cudaStream_t s); // the inserts; no sweep
+cudaError_t launch_filter_check(bnk_batch *b, uint32_t n, long long now_ns, bool only_status_ok, const Done &done, cudaStream_t s);
 cudaError_t filter_tables_alloc(bnk_ctx *ctx);
 void filter_tables_free(bnk_ctx *ctx);
 int filter_acl_upload(bnk_ctx *ctx, int enforce, const bnk_acl_tuple *tuples, size_t n);
@@ -375,7 +377,7 @@ cudaError_t launch_tally(bnk_batch *b, uint32_t n, cudaStream_t s);
 // inner_kernels.cu
 cudaError_t launch_demux_index(bnk_batch *b, uint32_t n, const uint32_t *len, cudaStream_t s);
 cudaError_t launch_inner_check(bnk_batch *b, uint32_t n, cudaStream_t s);
-cudaError_t launch_classify(bnk_batch *b, uint32_t n, cudaStream_t s);
+cudaError_t launch_classify(bnk_batch *b, uint32_t n, const Done &done, cudaStream_t s);
 // One 16-byte entry in one access, from and to the L2 that all SMs share.
 __device__ __forceinline__ SendCounter::Entry counter_load(const SendCounter::Entry *p) {
     SendCounter::Entry v;
@@ -430,3 +432,4 @@ __device__ __forceinline__ uint32_t demux_index_warp(const uint64_t *keys, const
 
 // gso_kernels.cu
 cudaError_t launch_gso_split(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, cudaStream_t s);
+cudaError_t launch_slots_to_host(bnk_batch *b, uint32_t n, cudaStream_t s);

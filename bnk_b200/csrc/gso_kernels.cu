@@ -13,8 +13,6 @@
 
 namespace {
 
-__device__ __forceinline__ uint32_t be16(const uint8_t *p) { return ((uint32_t)p[0] << 8) | p[1]; }
-
 // one's-complement sum of big-endian 16-bit words, folded to 16 bits
 __device__ __forceinline__ uint32_t fold16(uint64_t s) {
     s = (s & 0xffffffffull) + (s >> 32);
@@ -95,48 +93,44 @@ __global__ void __launch_bounds__(256) gso_split_kernel(const bnk_gso_super *sup
     }
     if (lane == 0) hdr_sum += sp.proto + (hdr - iph + seg_len);
 
-    // payload copy + sum.  Payload byte i sits at transport offset (hdr - iph + i): when that is odd the
-    // 16-bit words straddle, so sum bytes with their parity weight instead.
+    // payload copy + sum.  The destination starts on a word (headers are whole words); the source starts where the
+    // segments before it end, at any byte of a word, so a word of the payload is cut out of two aligned words of the
+    // source.
     const uint8_t *src = in + data_at;
     uint8_t *dst = out + hdr;
-    const uint32_t parity = (hdr - iph) & 1u;
     uint64_t sum = 0;    // of big-endian 16-bit words
     uint64_t le_sum = 0; // of the payload words as loaded (little-endian): the one's-complement sum commutes with the
                          // byte swap (RFC 1071, 2(B)), so the words are added raw and the folded sum is swapped once
-    if ((((uintptr_t)src | (uintptr_t)dst) & 3u) == 0 && parity == 0) {
-        const uint32_t words = seg_len >> 2;
-        const uint32_t *s32 = reinterpret_cast<const uint32_t *>(src);
-        uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
-        // several loads in flight per lane: the copy is latency-bound otherwise.  (Writing the destination in
-        // aligned 16-byte chunks assembled from two aligned source lines was measured: 17 % slower.)
-        constexpr uint32_t kInFlight = 4; // 2, 4 and 11 measure the same within noise
-        uint32_t i = lane;
-        for (; i + 32u * (kInFlight - 1) < words; i += 32u * kInFlight) {
-            uint32_t w[kInFlight];
+    const uint32_t words = seg_len >> 2, shift = 8u * ((uint32_t)(uintptr_t)src & 3u);
+    const uint32_t *s32 = reinterpret_cast<const uint32_t *>((uintptr_t)src & ~(uintptr_t)3u);
+    uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
+    auto word_at = [&](uint32_t i) { // behind a source that starts on a word there may be no further one
+        const uint32_t lo = s32[i];
+        return shift ? __funnelshift_r(lo, s32[i + 1], shift) : lo;
+    };
+    // several loads in flight per lane: the copy is latency-bound otherwise.  (Writing the destination in
+    // aligned 16-byte chunks assembled from two aligned source lines was measured: 17 % slower.)
+    constexpr uint32_t kInFlight = 4; // 2, 4 and 11 measure the same within noise
+    uint32_t i = lane;
+    for (; i + 32u * (kInFlight - 1) < words; i += 32u * kInFlight) {
+        uint32_t w[kInFlight];
 #pragma unroll
-            for (uint32_t u = 0; u < kInFlight; u++) w[u] = s32[i + 32u * u];
+        for (uint32_t u = 0; u < kInFlight; u++) w[u] = word_at(i + 32u * u);
 #pragma unroll
-            for (uint32_t u = 0; u < kInFlight; u++) {
-                d32[i + 32u * u] = w[u];
-                le_sum += w[u];
-            }
+        for (uint32_t u = 0; u < kInFlight; u++) {
+            d32[i + 32u * u] = w[u];
+            le_sum += w[u];
         }
-        for (; i < words; i += 32) {
-            const uint32_t w = s32[i];
-            d32[i] = w;
-            le_sum += w;
-        }
-        for (uint32_t i = (words << 2) + lane; i < seg_len; i += 32) {
-            const uint8_t v = src[i];
-            dst[i] = v;
-            sum += (i & 1u) ? v : ((uint32_t)v << 8);
-        }
-    } else {
-        for (uint32_t i = lane; i < seg_len; i += 32) {
-            const uint8_t v = src[i];
-            dst[i] = v;
-            sum += ((i + parity) & 1u) ? v : ((uint32_t)v << 8);
-        }
+    }
+    for (; i < words; i += 32) {
+        const uint32_t w = word_at(i);
+        d32[i] = w;
+        le_sum += w;
+    }
+    for (uint32_t i = (words << 2) + lane; i < seg_len; i += 32) {
+        const uint8_t v = src[i];
+        dst[i] = v;
+        sum += (i & 1u) ? v : ((uint32_t)v << 8);
     }
     le_sum = (le_sum & 0xffffffffull) + (le_sum >> 32); // 33 bits: 32 lanes of them still fit
     sum += hdr_sum; // both in 16-bit big-endian words
@@ -169,6 +163,19 @@ __global__ void gso_map_kernel(const bnk_gso_super *supers, uint32_t n_super, ui
         if (sp.first_pkt + k < n_pkts) seg_super[sp.first_pkt + k] = j;
 }
 
+// Packets' slots from the device ring to the pinned one, a warp per packet: header room, what the packet holds and the
+// room behind it.
+__global__ void __launch_bounds__(256) slots_to_host_kernel(const uint8_t *ring, uint8_t *host_ring, const uint32_t *off,
+                                                            const uint32_t *len, const uint32_t *out_len, uint32_t n, uint64_t ring_bytes) {
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const uint64_t begin = off[i] & ~15u;
+    uint64_t end = begin + 64u + max(len[i], out_len[i]);
+    if (end > ring_bytes) end = ring_bytes;
+    for (uint64_t q = begin + 16u * lane; q + 16u <= end; q += 512u)
+        *reinterpret_cast<uint4 *>(host_ring + q) = *reinterpret_cast<const uint4 *>(ring + q);
+}
+
 __global__ void fill_u32_kernel(uint32_t *p, uint32_t n, uint32_t v) {
     let_next_kernel_start();
     wait_for_kernel_in_front();
@@ -189,5 +196,11 @@ cudaError_t launch_gso_split(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, cu
     launch_kernel(n_pkts <= dependent_launch_up_to(), gso_split_kernel, dim3((n_pkts + 7) / 8), dim3(256), s, d.gso,
         n_super, d.ring, d.off, d.len, d.slot, n_pkts, b->ring_bytes, seg_super);
     b->ctx->launches += 3;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_slots_to_host(bnk_batch *b, uint32_t n, cudaStream_t s) {
+    slots_to_host_kernel<<<(n + 7) / 8, 256, 0, s>>>(b->dev.ring, b->host.ring, b->dev.off, b->dev.len, b->dev.out_len, n, b->ring_bytes);
+    b->ctx->launches += 1;
     return cudaGetLastError();
 }

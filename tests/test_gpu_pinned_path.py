@@ -149,3 +149,49 @@ def test_flows_noted_by_the_seal_kernel_and_swept(gpu_lib, oracle):
             b.close()
             assert c.flows_count() == f.flow_count, turn
             assert H.flows_equal(c.flows_export(), f.flows()), turn
+
+
+@pytest.mark.parametrize("busy", [False, True])  # True: another batch in flight, so that the results come back by copy
+def test_split_uploads_super_packets_only(gpu_lib, oracle, busy):
+    """The split and the seal behind it change packets and their room, not what the host ring holds beside them, and the
+    sealed messages are on the device too."""
+    from bnk_b200 import Context
+    from bnk_b200.device import F_ASSIGN_COUNTERS, F_NO_H2D, F_REPLAY, F_USE_OUT_LEN
+    from tests.test_gpu_gso import _plan, _tcp_super
+
+    rng = np.random.default_rng(4)
+    supers, meta = [], []
+    for size, gso in [(40_000, 1251), (9000, 333), (1380, 1380), (7, 2)]:
+        pkt, cs, hdr = _tcp_super(rng, size)
+        supers.append(pkt)
+        meta.append((hdr, gso, cs, 16, 6))
+    stride = 1472
+    sup, seg_len, n, ring_bytes = _plan(supers, meta, stride)
+    want = [s for p, m in zip(supers, meta) for s in oracle.gso_split(p, *m)]
+    key = rng.integers(0, 256, (1, 32), dtype=np.uint8)
+    with Context(max_keypairs=1, mtu=1420, flow_capacity=0) as c:
+        c.set_keypairs(0, key, key, np.array([9], np.uint32))
+        b, other = c.batch(n, ring_bytes + 64), c.batch(1, 2048)
+        other.off[0], other.len[0], other.slot[0], other.counter[0] = 0, 1000, 0, 1 << 40
+        b.ring[:] = 0xEE
+        for j, pkt in enumerate(supers):
+            b.ring[int(sup[j]["src_off"]):int(sup[j]["src_off"]) + len(pkt)] = np.frombuffer(pkt, np.uint8)
+        b.off[:], b.len[:], b.slot[:] = H.layout_fixed(n, stride), seg_len, 0
+        before = np.array(b.ring)
+        b.gso_split(sup, n)
+        if busy:
+            other.seal(1, wait=False)
+        b.seal(n, F_NO_H2D | F_ASSIGN_COUNTERS)
+        assert (b.status == 0).all()
+        room = np.zeros(len(before), bool)
+        for i in range(n):
+            o = int(b.off[i])
+            assert b.message(i) == oracle.wg_seal(key[0].tobytes(), 9, i, want[i], 1420), i
+            room[o:o + 64 + len(want[i]) + 32] = True
+        assert np.array_equal(b.ring[~room], before[~room])
+        b.open(n, F_NO_H2D | F_USE_OUT_LEN | F_REPLAY)
+        assert (b.status == 0).all()
+        for i in range(n):
+            assert b.payload(i)[:len(want[i])] == want[i], i
+        assert np.array_equal(b.ring[~room], before[~room])
+        other.wait()
