@@ -9,6 +9,7 @@
 #include <thread>
 
 #include "filter_device.cuh"
+#include "submit_order.h"
 
 namespace {
 
@@ -223,6 +224,14 @@ AeadArgs aead_args(bnk_batch *b, uint32_t n, bool open, const uint32_t *order) {
 }
 
 } // namespace
+
+int order_begin(bnk_batch *b, bnk_batch *behind) {
+    if (!b->ev_order) CK(b->ctx, cudaEventCreateWithFlags(&b->ev_order, cudaEventDisableTiming));
+    b->order_wait = behind ? behind->ev_order : nullptr;
+    b->order_record = b->ev_order;
+    return BNK_SUCCESS;
+}
+void order_end(bnk_batch *b) { b->order_wait = b->order_record = nullptr; }
 
 extern "C" {
 
@@ -715,6 +724,7 @@ int bnk_batch_destroy(bnk_batch *b) {
     if (b->a_begin) cudaEventDestroy(b->a_begin);
     if (b->a_end) cudaEventDestroy(b->a_end);
     if (b->t_end) cudaEventDestroy(b->t_end);
+    if (b->ev_order) cudaEventDestroy(b->ev_order);
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
     if (b->ev_fence) cudaEventDestroy(b->ev_fence);

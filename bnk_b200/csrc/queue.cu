@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "bnk_internal.cuh"
+#include "submit_order.h"
 
 namespace {
 
@@ -29,7 +30,6 @@ enum State : int { FREE, FILLING, CLOSED, IN_FLIGHT, DONE };
 struct GpuBatch {
     bnk_batch *b = nullptr;
     bnk_batch_view v{};
-    cudaEvent_t kernels_done = nullptr; // recorded behind the batch's last kernel
     std::atomic<int> state{FREE};       // written under the queue's lock; its callers watch it without
     uint32_t reserved = 0;              // packets handed out to callers
     std::atomic<uint32_t> filled{0};    // of those, copied in
@@ -160,11 +160,9 @@ void pump(bnk_queue *q) {
         }
         GpuBatch &g = q->gb[idx];
         // kernels of this batch start behind the kernels of the batch submitted before it
-        g.b->order_wait = prev >= 0 ? q->gb[prev].kernels_done : nullptr;
-        g.b->order_record = g.kernels_done;
-        g.rc = q->cfg.open_side ? bnk_open_submit(g.b, n, q->cfg.flags, g.now) : bnk_seal_submit(g.b, n, q->cfg.flags, g.now);
-        g.b->order_wait = nullptr;
-        g.b->order_record = nullptr;
+        g.rc = submit_behind(g.b, prev >= 0 ? q->gb[prev].b : nullptr, [&] {
+            return q->cfg.open_side ? bnk_open_submit(g.b, n, q->cfg.flags, g.now) : bnk_seal_submit(g.b, n, q->cfg.flags, g.now);
+        });
         {
             Locked lk(q->mu);
             q->inflight.push(idx); // only now may anybody ask the driver about it
@@ -226,7 +224,6 @@ int bnk_queue_destroy(bnk_queue *q) {
             bnk_wait(g.b, UINT64_MAX);
             bnk_batch_destroy(g.b);
         }
-        if (g.kernels_done) cudaEventDestroy(g.kernels_done);
     }
     delete q;
     return BNK_SUCCESS;
@@ -253,7 +250,6 @@ int bnk_queue_create(bnk_ctx *ctx, const bnk_queue_cfg *cfg, bnk_queue **out) {
     for (GpuBatch &g : q->gb) {
         int rc = bnk_batch_create(ctx, cfg->max_pkts, (uint64_t)cfg->max_pkts * q->slot_bytes, &g.b);
         if (rc == BNK_SUCCESS) rc = bnk_batch_view_get(g.b, &g.v);
-        if (rc == BNK_SUCCESS && cudaEventCreateWithFlags(&g.kernels_done, cudaEventDisableTiming) != cudaSuccess) rc = BNK_ECUDA;
         if (rc != BNK_SUCCESS) {
             bnk_queue_destroy(q);
             return rc;
