@@ -81,7 +81,10 @@ int begin_submit(bnk_batch *b, uint32_t npkts, bool touches_host = true) {
 struct SubmitScope {
     bnk_batch *b;
     std::shared_lock<std::shared_mutex> tables; // see bnk_ctx::submit_mu
-    explicit SubmitScope(bnk_batch *batch) : b(batch), tables(batch->ctx->submit_mu) { b->stats_pending = b->done_watched = false; }
+    explicit SubmitScope(bnk_batch *batch) : b(batch), tables(batch->ctx->submit_mu) {
+        b->stats_pending = b->done_watched = false;
+        b->run_stream = b->stream;
+    }
     ~SubmitScope() {
         b->in_flight = true;
         if (!b->counted) b->ctx->in_flight.fetch_add(1, std::memory_order_relaxed);
@@ -227,11 +230,32 @@ AeadArgs aead_args(bnk_batch *b, uint32_t n, bool open, const uint32_t *order) {
 
 int order_begin(bnk_batch *b, bnk_batch *behind) {
     if (!b->ev_order) CK(b->ctx, cudaEventCreateWithFlags(&b->ev_order, cudaEventDisableTiming));
-    b->order_wait = behind ? behind->ev_order : nullptr;
-    b->order_record = b->ev_order;
+    b->ordered = true;
+    b->behind = behind;
     return BNK_SUCCESS;
 }
-void order_end(bnk_batch *b) { b->order_wait = b->order_record = nullptr; }
+void order_end(bnk_batch *b) {
+    b->ordered = false;
+    b->behind = nullptr;
+}
+void batch_set_direct_stream(bnk_batch *b, cudaStream_t s) { b->direct_stream = s; }
+cudaError_t order_stream_create(bnk_ctx *ctx, cudaStream_t *s) {
+    return cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, ctx->prio_high);
+}
+// The kernels of a submit come next on stream s ...
+static cudaError_t order_kernels_begin(bnk_batch *b, cudaStream_t s) {
+    bnk_batch *const p = b->behind;
+    if (!b->ordered || !p || p->run_stream == s) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    if (p->ran_direct) e = cudaEventRecord(p->ev_order, p->run_stream); // nothing but kernels there
+    return e != cudaSuccess ? e : cudaStreamWaitEvent(s, p->ev_order, 0);
+}
+// ... and these were the last of them.
+static cudaError_t order_kernels_end(bnk_batch *b, cudaStream_t s, bool direct) {
+    b->run_stream = s;
+    b->ran_direct = direct;
+    return b->ordered && !direct ? cudaEventRecord(b->ev_order, s) : cudaSuccess;
+}
 
 extern "C" {
 
@@ -694,6 +718,7 @@ int bnk_batch_destroy(bnk_batch *b) {
             }
     }
     if (b->stream) cudaStreamSynchronize(b->stream);
+    if (b->direct_stream) cudaStreamSynchronize(b->direct_stream);
     cudaFreeHost(b->host.src_addr);
     cudaFreeHost(b->h_desc);
     cudaFree(b->d_desc);
@@ -882,12 +907,12 @@ int bnk_batch_download(bnk_batch *b, uint32_t npkts) {
 // segments sealed and stored 0.38 ms, against 0.44 for seal and download in a row.
 static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t flags, int64_t now_unix_ns, bool resident) {
     bnk_ctx *ctx = b->ctx;
-    cudaStream_t s = b->stream;
+    cudaStream_t s = b->direct_stream ? b->direct_stream : b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0, stats = (flags & BNK_F_STATS) != 0;
     const bool assign = (flags & BNK_F_ASSIGN_COUNTERS) != 0;
     const bnk_batch_view &h = b->host;
     const DeviceBatch &d = b->dev;
-    if (b->order_wait) CK(ctx, cudaStreamWaitEvent(s, b->order_wait, 0));
+    CK(ctx, order_kernels_begin(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, false, nullptr);
     a.over_link = true;
@@ -942,7 +967,7 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = b->aead_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
-    if (b->order_record) CK(ctx, cudaEventRecord(b->order_record, s));
+    CK(ctx, order_kernels_end(b, s, true));
     return BNK_SUCCESS;
 }
 
@@ -974,7 +999,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
         }
         b->dev_stale = false;
     }
-    if (b->order_wait) CK(ctx, cudaStreamWaitEvent(s, b->order_wait, 0));
+    CK(ctx, order_kernels_begin(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     if ((flags & BNK_F_NOTE_OUTBOUND) && n && ctx->ft.enforce && ctx->ft.flow_capacity) { // filter.go:192-194
         const bool sweep = flow_note_begins(b, npkts, now_unix_ns);
@@ -1018,7 +1043,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     b->kernel_timed = timed;
     b->aead_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
-    if (b->order_record) CK(ctx, cudaEventRecord(b->order_record, s));
+    CK(ctx, order_kernels_end(b, s, false));
     if (!(flags & BNK_F_NO_D2H) && n) {
         if (b->joint_copy) {
             CK(ctx, ring_down(b, npkts, ext, true, s));
@@ -1034,12 +1059,12 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
 // stays on the device until then, with the packets' inner headers, so that no later kernel goes back to the ring.
 static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t flags, int64_t now_unix_ns) {
     bnk_ctx *ctx = b->ctx;
-    cudaStream_t s = b->stream;
+    cudaStream_t s = b->direct_stream ? b->direct_stream : b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0, stats = (flags & BNK_F_STATS) != 0;
     const bool replay = (flags & BNK_F_REPLAY) != 0, checks = (flags & (BNK_F_INNER_CHECK | BNK_F_CHECK_INBOUND)) != 0;
     const bnk_batch_view &h = b->host;
     b->dev_stale = true;
-    if (b->order_wait) CK(ctx, cudaStreamWaitEvent(s, b->order_wait, 0));
+    CK(ctx, order_kernels_begin(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, true, nullptr);
     a.over_link = a.from_host = true;
@@ -1100,7 +1125,7 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = b->aead_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
-    if (b->order_record) CK(ctx, cudaEventRecord(b->order_record, s));
+    CK(ctx, order_kernels_end(b, s, true));
     if (!one_launch) CK(ctx, desc_copy(b, npkts, D_OUT_LEN, D_STATUS, false, s));
     return BNK_SUCCESS;
 }
@@ -1129,7 +1154,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
         }
         b->dev_stale = false;
     }
-    if (b->order_wait) CK(ctx, cudaStreamWaitEvent(s, b->order_wait, 0));
+    CK(ctx, order_kernels_begin(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     const uint32_t *order = nullptr;
     AeadArgs oa = aead_args(b, npkts, true, nullptr);
@@ -1177,7 +1202,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
-    if (b->order_record) CK(ctx, cudaEventRecord(b->order_record, s));
+    CK(ctx, order_kernels_end(b, s, false));
     if (!(flags & BNK_F_NO_D2H) && n) {
         if (b->joint_copy) {
             CK(ctx, ring_down(b, npkts, ext, true, s));
@@ -1352,11 +1377,11 @@ int bnk_wait(bnk_batch *b, uint64_t timeout_ns) {
         if (b->done_watched && timeout_ns == 0 && (++b->done_polls & 63u)) return BNK_ETIMEDOUT; // ask the driver now and then
         CK(ctx, cudaSetDevice(ctx->device));
         if (timeout_ns == UINT64_MAX) {
-            CK(ctx, cudaStreamSynchronize(b->stream));
+            CK(ctx, cudaStreamSynchronize(b->run_stream));
         } else {
             const auto deadline = std::chrono::steady_clock::now() + std::chrono::nanoseconds(timeout_ns);
             for (;;) {
-                cudaError_t e = cudaStreamQuery(b->stream);
+                cudaError_t e = cudaStreamQuery(b->run_stream);
                 if (e == cudaSuccess) break;
                 if (e != cudaErrorNotReady) return fail(ctx, BNK_ECUDA, "cudaStreamQuery", e);
                 if (std::chrono::steady_clock::now() >= deadline) return BNK_ETIMEDOUT;

@@ -202,9 +202,13 @@ struct bnk_batch {
     bnk_batch_stats *h_stats; // pinned; written by the tally kernel
     unsigned long long *d_stats; // device accumulators of the tally kernel (zero between launches)
     cudaEvent_t ev_fence; // orders this batch's stream against table maintenance on another stream
-    // Set around one submit (submit_order.h): its kernels start behind order_wait and order_record, the batch's ev_order,
-    // is recorded behind the last of them.
-    cudaEvent_t order_wait, order_record, ev_order;
+    // Submits in order over several batches (submit_order.h).  direct_stream: where such a batch runs when it stays in
+    // pinned memory (shared with the batches it is ordered against; null: on its own stream).  run_stream: where the last
+    // submit ran.  ev_order: behind its kernels.
+    cudaStream_t direct_stream, run_stream;
+    bool ordered, ran_direct; // between order_begin and order_end / the last submit ran in pinned memory
+    bnk_batch *behind;
+    cudaEvent_t ev_order;
 };
 
 // Small batches are two dependent launches with little work in each, so the gap between them counts.  A kernel

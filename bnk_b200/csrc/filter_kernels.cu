@@ -491,9 +491,11 @@ cudaError_t filter_flows_maintain(bnk_batch *b, cudaStream_t s) {
     std::unique_lock<std::shared_mutex> tables(ctx->submit_mu);
     cudaError_t e;
     for (bnk_batch *o : ctx->batches) { // everything submitted so far finishes before the move
-        if (o == b) continue;
-        if ((e = cudaEventRecord(o->ev_fence, o->stream)) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(s, o->ev_fence, 0)) != cudaSuccess) return e;
+        for (cudaStream_t os : {o->stream, o->direct_stream}) {
+            if (!os) continue;
+            if ((e = cudaEventRecord(o->ev_fence, os)) != cudaSuccess) return e;
+            if ((e = cudaStreamWaitEvent(s, o->ev_fence, 0)) != cudaSuccess) return e;
+        }
     }
     for (int cls = 0; cls < 3; cls++) {
         if (ctx->flow_dead_hint[cls] < limit) continue;
@@ -506,7 +508,8 @@ cudaError_t filter_flows_maintain(bnk_batch *b, cudaStream_t s) {
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = cudaEventRecord(b->ev_fence, s)) != cudaSuccess) return e;
     for (bnk_batch *o : ctx->batches) // and nothing submitted later starts before it is done
-        if (o != b && (e = cudaStreamWaitEvent(o->stream, b->ev_fence, 0)) != cudaSuccess) return e;
+        for (cudaStream_t os : {o->stream, o->direct_stream})
+            if (os && os != s && (e = cudaStreamWaitEvent(os, b->ev_fence, 0)) != cudaSuccess) return e;
     return cudaSuccess;
 }
 
@@ -613,10 +616,13 @@ int filter_acl_upload(bnk_ctx *ctx, int enforce, const bnk_acl_tuple *tuples, si
         std::unique_lock<std::shared_mutex> tables(ctx->submit_mu); // between two submits
         bnk_ctx::RuleSet &old = ctx->rule_set[ctx->rule_cur];
         for (bnk_batch *b : ctx->batches) { // what has been launched with the old set, per stream
-            cudaEvent_t ev;
-            if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return BNK_ECUDA;
-            cudaEventRecord(ev, b->stream);
-            old.in_use.push_back(ev);
+            for (cudaStream_t bs : {b->stream, b->direct_stream}) {
+                if (!bs) continue;
+                cudaEvent_t ev;
+                if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return BNK_ECUDA;
+                cudaEventRecord(ev, bs);
+                old.in_use.push_back(ev);
+            }
         }
         ft.rule_keys = spare.keys;
         ft.rule_span = spare.span;

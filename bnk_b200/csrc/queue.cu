@@ -99,6 +99,7 @@ struct bnk_queue {
     bnk_ctx *ctx;
     bnk_queue_cfg cfg;
     uint32_t slot_bytes;
+    cudaStream_t stream = nullptr; // of the GPU batches that stay in pinned memory
     std::vector<GpuBatch> gb;
     SpinLock mu;
     uint32_t cur = 0;    // the batch that is filling (or will be, once it is free)
@@ -121,7 +122,10 @@ bool ripe(const bnk_queue *q) {
         c.filled.load(std::memory_order_acquire) != c.reserved)
         return false;
     if (q->inflight.empty()) return true;                                   // the device is idle
-    if (c.reserved >= q->cfg.min_fill) return true;                         // worth a launch
+    // Worth a launch.  With one batch at work and one behind it a third gains the device nothing by being there and the
+    // callers' threads a launch by being larger.
+    const uint32_t fill = q->inflight.count < 2 ? q->cfg.min_fill : std::max(q->cfg.min_fill, q->cfg.max_pkts / 2);
+    if (c.reserved >= fill) return true;
     return std::chrono::steady_clock::now() >= c.first_at + kGatherNs;      // waited long enough
 }
 
@@ -225,6 +229,7 @@ int bnk_queue_destroy(bnk_queue *q) {
             bnk_batch_destroy(g.b);
         }
     }
+    if (q->stream) cudaStreamDestroy(q->stream);
     delete q;
     return BNK_SUCCESS;
 }
@@ -247,9 +252,14 @@ int bnk_queue_create(bnk_ctx *ctx, const bnk_queue_cfg *cfg, bnk_queue **out) {
     q->closed.slot.resize(q->gb.size());
     q->inflight.slot.resize(q->gb.size());
     cudaSetDevice(ctx->device);
+    if (order_stream_create(ctx, &q->stream) != cudaSuccess) {
+        delete q;
+        return BNK_ECUDA;
+    }
     for (GpuBatch &g : q->gb) {
         int rc = bnk_batch_create(ctx, cfg->max_pkts, (uint64_t)cfg->max_pkts * q->slot_bytes, &g.b);
         if (rc == BNK_SUCCESS) rc = bnk_batch_view_get(g.b, &g.v);
+        if (rc == BNK_SUCCESS) batch_set_direct_stream(g.b, q->stream);
         if (rc != BNK_SUCCESS) {
             bnk_queue_destroy(q);
             return rc;
@@ -352,6 +362,7 @@ int bnk_queue_commit(bnk_queue *q, bnk_ticket ticket) {
             rc = BNK_EINVAL;
         }
     g->filled.fetch_add(n, std::memory_order_release);
+    poll(q); // what has come back makes room for what goes
     pump(q);
     return rc;
 }
@@ -400,6 +411,7 @@ int bnk_queue_submit(bnk_queue *q, const uint8_t *const *pkts, const uint32_t *l
         if (len[k]) memcpy(v.ring + (size_t)at * q->slot_bytes + head, pkts[k], len[k]);
     }
     g->filled.fetch_add(n, std::memory_order_release);
+    poll(q); // what has come back makes room for what goes
     pump(q);
     return BNK_SUCCESS;
 }

@@ -326,6 +326,7 @@ struct bnk_mgpu {
     uint32_t piece; // packets per piece of a share
     std::vector<std::vector<bnk_batch *>> batch; // [gpu][Share::kSlots]
     std::vector<std::vector<bnk_batch_view>> view;
+    std::vector<cudaStream_t> stream; // [gpu] of the pieces that stay in pinned memory
     std::vector<bnk_batch *> last; // [gpu] batch of the submit that the next one's kernels have to follow
     std::vector<std::unique_ptr<Worker>> worker;
     std::vector<std::unique_ptr<Crew>> crew;
@@ -370,6 +371,8 @@ int bnk_mgpu_destroy(bnk_mgpu *m) {
     for (std::vector<bnk_batch *> &of_gpu : m->batch)
         for (bnk_batch *b : of_gpu)
             if (b) bnk_batch_destroy(b);
+    for (cudaStream_t s : m->stream)
+        if (s) cudaStreamDestroy(s);
     for (bnk_ctx *c : m->ctx)
         if (c) bnk_ctx_destroy(c);
     delete m;
@@ -395,6 +398,7 @@ int bnk_mgpu_create(const bnk_mgpu_cfg *cfg, bnk_mgpu **out) {
     m->ctx.assign(ng, nullptr);
     m->batch.assign(ng, std::vector<bnk_batch *>(Share::kSlots, nullptr));
     m->view.assign(ng, std::vector<bnk_batch_view>(Share::kSlots));
+    m->stream.assign(ng, nullptr);
     m->last.assign(ng, nullptr);
     m->peer_of_index.Init(cfg->max_peers);
     m->pkts_per_gpu.assign(ng, 0);
@@ -403,9 +407,11 @@ int bnk_mgpu_create(const bnk_mgpu_cfg *cfg, bnk_mgpu **out) {
         c.struct_size = sizeof c;
         c.device_id = cfg->devices[g];
         int rc = bnk_ctx_create(&c, &m->ctx[g]);
+        if (rc == BNK_SUCCESS && order_stream_create(m->ctx[g], &m->stream[g]) != cudaSuccess) rc = BNK_ECUDA;
         for (uint32_t k = 0; k < Share::kSlots; k++) {
             if (rc == BNK_SUCCESS) rc = bnk_batch_create(m->ctx[g], m->piece, (uint64_t)m->piece * m->slot_bytes, &m->batch[g][k]);
             if (rc == BNK_SUCCESS) rc = bnk_batch_view_get(m->batch[g][k], &m->view[g][k]);
+            if (rc == BNK_SUCCESS) batch_set_direct_stream(m->batch[g][k], m->stream[g]);
         }
         if (rc != BNK_SUCCESS) {
             bnk_mgpu_destroy(m);
