@@ -1197,7 +1197,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     if (flags & BNK_F_INNER_CHECK) CK(ctx, launch_inner_check(b, npkts, s));
     if (flags & BNK_F_CHECK_INBOUND) {
         flow_check_begins(b, now_unix_ns);
-        CK(ctx, launch_filter_check(b, npkts, now_unix_ns, true, Done{}, s));
+        CK(ctx, launch_filter_check(b, npkts, now_unix_ns, true, nullptr, Done{}, s));
     }
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = timed;
@@ -1267,13 +1267,14 @@ int bnk_filter_check_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_
     HostAlias alias(b, direct);
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     flow_check_begins(b, now_unix_ns);
-    const Done done = direct && !(flags & BNK_F_STATS) ? watch_for(b) : Done{};
-    CK(ctx, launch_filter_check(b, npkts, now_unix_ns, false, done, s));
+    const bool to_host = !(flags & BNK_F_NO_D2H);
+    const Done done = to_host && npkts && !(flags & BNK_F_STATS) ? watch_for(b) : Done{};
+    uint8_t *const host_status = to_host ? b->host.status : nullptr;
+    if (direct) b->dev.status = alias.saved.status; // the kernel writes to both
+    CK(ctx, launch_filter_check(b, npkts, now_unix_ns, false, host_status, done, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
-    if (!direct && !(flags & BNK_F_NO_D2H) && npkts)
-        CK(ctx, cudaMemcpyAsync(b->host.status, b->dev.status, npkts, cudaMemcpyDeviceToHost, s));
     return BNK_SUCCESS;
 }
 

@@ -54,14 +54,26 @@ struct KeypairTables {
     uint32_t addr_slots;    // power of two
 };
 
+// The allowances of one prefix.  Port ranges (first << 16 | last) are disjoint and in rising order; those of tcp and those
+// of udp each start at a multiple of four in rule_ports and are filled up with kNoPorts to one.
+struct alignas(16) RuleGroup {
+    uint32_t addr, len;         // the prefix (hash table: len 0 = an empty place)
+    uint32_t parent;            // the longest shorter prefix with allowances that contains this one, + 1; bit 31: icmp is allowed
+    uint32_t n_ports;           // tcp's ranges | udp's << 16
+    uint32_t tcp_at, udp_at;    // where they start in rule_ports
+    uint32_t tcp0, udp0;        // the first of each (kNoPorts: none)
+};
+constexpr uint32_t kNoPorts = 0xffff0000u;
+
 // Flattened, indexed ACL and the reply-flow table (filter_kernels.cu).
 struct FilterTables {
-    // rule index: open-addressing table keyed by (prefix_len, masked address)
-    uint64_t *rule_keys;   // [rule_slots] 0 = empty; else (1<<40 | len<<32 | masked addr)
-    uint2 *rule_span;      // [rule_slots] (first entry, entry count) into rule_entries
-    uint64_t *rule_entries; // packed (proto<<32 | first<<16 | last)
-    uint32_t rule_slots;   // power of two (0 when no tuples)
-    uint64_t len_mask;     // bit L set when some tuple has prefix length L (bits 0..32)
+    // rule index (filter_device.cuh), one block of device memory
+    const uint32_t *rule_top;    // [65536] by the upper 16 address bits; null when there are no rules
+    const uint2 *rule_blocks;    // [blocks][256] by the next 8
+    const RuleGroup *rule_long;  // hash table of the prefixes longer than 24
+    uint32_t rule_long_mask;
+    const RuleGroup *rule_groups;
+    const uint32_t *rule_ports;
     int enforce;
     // flow table, one open-addressing region per protocol class (tcp, udp, icmp).  Every class has two
     // regions, [class][half][flow_capacity]; flow_half[class] says which one is in use, the other one is all
@@ -121,10 +133,8 @@ struct bnk_ctx {
     std::atomic<int> flow_errors_seen;       // failed inserts already reported to a caller as BNK_EFULL
     // rule table: two device buffer sets, the one not in use receives the next upload
     struct RuleSet {
-        uint64_t *keys = nullptr;
-        uint2 *span = nullptr;
-        uint64_t *entries = nullptr;
-        size_t slots_cap = 0, entries_cap = 0;
+        uint8_t *mem = nullptr;
+        size_t cap = 0;
         std::vector<cudaEvent_t> in_use; // recorded on every batch stream when the set was retired
     } rule_set[2];
     int rule_cur = 0;
@@ -282,11 +292,12 @@ __device__ __forceinline__ void signal_done(const Done &d, bool has_words, F las
     if (d.flag == nullptr) return;
     __syncthreads();
     if (threadIdx.x != 0) return;
-    __threadfence_system(); // the CTA's stores, to host memory too, before its ticket
-    if (gridDim.x != 1) { // the other CTAs' stores have arrived when their tickets are out: their fences were before
+    if (gridDim.x != 1) {
+        __threadfence();
         if (atomicAdd(d.ticket, 1u) + 1u != gridDim.x) return;
         *d.ticket = 0u;
     }
+    __threadfence_system();
     if (has_words) {
         __threadfence();
         last_words();
@@ -357,7 +368,8 @@ uint32_t replay_hash_capacity(uint32_t max_pkts);  // entries of the duplicate-c
 
 // filter_kernels.cu
 cudaError_t launch_filter_note(bnk_batch *b, uint32_t n, long long now_ns, const Done &done, cudaStream_t s); // the inserts; no sweep
-cudaError_t launch_filter_check(bnk_batch *b, uint32_t n, long long now_ns, bool only_status_ok, const Done &done, cudaStream_t s);
+cudaError_t launch_filter_check(bnk_batch *b, uint32_t n, long long now_ns, bool only_status_ok, uint8_t *host_status,
+                                const Done &done, cudaStream_t s);
 cudaError_t filter_tables_alloc(bnk_ctx *ctx);
 void filter_tables_free(bnk_ctx *ctx);
 int filter_acl_upload(bnk_ctx *ctx, int enforce, const bnk_acl_tuple *tuples, size_t n);

@@ -2,12 +2,9 @@
 // (internal/filter/filter.go of the reference) and acl.CompiledRule.Match
 // (internal/acl/acl.go:149-172), one thread per packet.
 //
-// Rules.  The reference scans every rule for every packet.  The verdict is an OR
-// over rules, so scan order is free; here the flattened allowances
-// (prefix, proto, port range) are grouped by prefix and the groups are put in an
-// open-addressing table keyed by (prefix length, masked address).  A packet probes
-// the table once per prefix length that occurs in the rule set (a 33-bit mask) and
-// scans only the allowances of prefixes that contain its source address.
+// Rules.  The reference scans every rule for every packet.  The verdict is an OR over rules, so scan order is free;
+// here the flattened allowances (prefix, proto, port range) are grouped by prefix and the prefixes are indexed
+// (filter_device.cuh).
 //
 // Flows: see filter_device.cuh.
 // Go deletes map entries (filter.go:144, 202-208), so its map is bounded by the live
@@ -15,17 +12,18 @@
 // a class's region the surviving entries are re-inserted into the class's second,
 // empty region and the two swap roles (filter_flows_maintain), between two batches.
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 #include "filter_device.cuh"
 
 namespace {
 
-// filter.go:71-106 of the packet at ring[o + 16 .. o + 16 + len), which lies in the ring.  Its first 32 bytes, which
+// filter.go:71-106 of the packet at ring[o + 16 .. o + 16 + len), which has to lie in the ring.  Its first 32 bytes, which
 // hold all of a packet without IP options, are asked for together: when the ring is in host memory a dependent read is
 // another trip over the link (8192 whole packets noted and checked: 95 us with three dependent reads, 87 with one).
 __device__ __forceinline__ bool parse_ipv4(const uint8_t *ring, uint32_t o, uint32_t len, uint64_t ring_bytes, Parsed &out) {
-    if (len < 20) return false;
+    if ((o & 15u) || (uint64_t)o + 16u + len > ring_bytes || len < 20) return false;
     const uint8_t *const p = ring + o + 16; // 16-byte aligned
     const bool both = (uint64_t)o + 48 <= ring_bytes;
     const uint4 a = *reinterpret_cast<const uint4 *>(p);
@@ -45,9 +43,8 @@ __global__ void __launch_bounds__(128) filter_note_kernel(const __grid_constant_
     wait_for_kernel_in_front();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
-        const uint32_t o = off[i], l = len[i];
         Parsed p;
-        if (!(o & 15u) && (uint64_t)o + 16u + l <= ring_bytes && parse_ipv4(ring, o, l, ring_bytes, p)) {
+        if (parse_ipv4(ring, off[i], len[i], ring_bytes, p)) {
             FlowNote note;
             note.begin(ft, p, now);
             note.place(ft);
@@ -128,23 +125,32 @@ __global__ void __launch_bounds__(256) filter_sweep_kernel(const __grid_constant
 }
 
 // ---- CheckInbound, filter.go:121-147 -----------------------------------------------------
-// only_status_ok: packets whose status is not BNK_PKT_OK are left alone (open pipeline).
+// only_status_ok: packets whose status is not BNK_PKT_OK are left alone (open pipeline).  host_status (may be null): the
+// results' pinned array, which gets a CTA's 128 statuses as one line: 1,000,000 of them cost 20 us of link time beside
+// the checks instead of a copy of 27 us behind them.
 __global__ void __launch_bounds__(128) filter_check_kernel(const __grid_constant__ FilterTables ft, const uint8_t *ring, const uint32_t *off,
                                     const uint32_t *len, uint8_t *status, uint32_t n, uint64_t ring_bytes,
-                                    long long now, int only_status_ok, Done done) {
+                                    long long now, int only_status_ok, uint8_t *host_status, Done done) {
     let_next_kernel_start();
     wait_for_kernel_in_front();
+    __shared__ uint32_t line[32];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n && !(only_status_ok && status[i] != BNK_PKT_OK)) {
         uint8_t verdict = BNK_PKT_OK; // filter.go:124-126: allow-all passes even unparseable packets
-        if (ft.enforce) {
-            const uint32_t o = off[i], l = len[i];
-            Parsed p;
-            verdict = (o & 15u) || (uint64_t)o + 16u + l > ring_bytes || !parse_ipv4(ring, o, l, ring_bytes, p)
-                          ? (uint8_t)BNK_PKT_FILTER_DENY
-                          : filter_verdict(ft, p, now);
-        }
+        Parsed p;
+        if (ft.enforce)
+            verdict = parse_ipv4(ring, off[i], len[i], ring_bytes, p) ? filter_verdict(ft, p, now) : (uint8_t)BNK_PKT_FILTER_DENY;
         status[i] = verdict;
+        reinterpret_cast<uint8_t *>(line)[threadIdx.x] = verdict;
+    }
+    if (host_status) {
+        __syncthreads();
+        const uint32_t first = blockIdx.x * blockDim.x + 4u * threadIdx.x;
+        if (threadIdx.x < 32) {
+            if (first + 4u <= n) *reinterpret_cast<uint32_t *>(host_status + first) = line[threadIdx.x];
+            else
+                for (uint32_t k = first; k < n; k++) host_status[k] = reinterpret_cast<uint8_t *>(line)[4u * threadIdx.x + (k - first)];
+        }
     }
     signal_done(done, false, [] {});
 }
@@ -177,7 +183,7 @@ __global__ void flows_compact_kernel(FilterTables ft, int cls) {
         if (key == FLOW_EMPTY) continue;
         const long long exp = ft.flow_exp[from + k];
         if (flow_absent(exp)) continue;
-        uint32_t h = (uint32_t)mix64(key) & (ft.flow_capacity - 1);
+        uint32_t h = flow_hash(key) & (ft.flow_capacity - 1);
         bool placed = false; // the target region starts empty and takes fewer entries than it has slots
         for (uint32_t probe = 0; probe < ft.flow_capacity && !placed; probe++) {
             if (atomicCAS(&keys[h], FLOW_EMPTY, key) == FLOW_EMPTY) placed = true;
@@ -249,6 +255,26 @@ __global__ void __launch_bounds__(256) tally_kernel(const uint8_t *status, const
 
 } // namespace
 
+// Where the parts of a rule index lie in its block of memory.
+namespace {
+struct RuleLayout {
+    size_t top = 0, blocks, table, groups, ports, total;
+    RuleLayout(size_t n_blocks, size_t n_slots, size_t n_groups, size_t n_ports) {
+        auto room = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+        blocks = room(65536 * sizeof(uint32_t));
+        table = blocks + room(n_blocks * 256 * sizeof(uint2));
+        groups = table + room(n_slots * sizeof(RuleGroup));
+        ports = groups + room(n_groups * sizeof(RuleGroup));
+        total = ports + room(n_ports * sizeof(uint32_t));
+    }
+};
+size_t rule_long_slots(size_t prefixes) { // a quarter full at most: the lanes of a warp wait for the longest of their walks
+    size_t n = 4;
+    while (n < prefixes * 4) n <<= 1;
+    return n;
+}
+} // namespace
+
 cudaError_t filter_tables_alloc(bnk_ctx *ctx) {
     FilterTables &ft = ctx->ft;
     ft = FilterTables{};
@@ -265,14 +291,10 @@ cudaError_t filter_tables_alloc(bnk_ctx *ctx) {
     }
     // With a stated rule-table capacity both buffer sets are allocated here, and a rule swap allocates nothing.
     if (const size_t cap_t = ctx->cfg.max_acl_tuples) {
-        size_t slots = 16;
-        while (slots < cap_t * 8) slots <<= 1;
+        const size_t bytes = RuleLayout(std::min<size_t>(cap_t, 65536), rule_long_slots(cap_t), cap_t, 4 * cap_t).total;
         for (bnk_ctx::RuleSet &rs : ctx->rule_set) {
-            if ((e = cudaMalloc(&rs.keys, slots * sizeof(uint64_t))) != cudaSuccess) return e;
-            if ((e = cudaMalloc(&rs.span, slots * sizeof(uint2))) != cudaSuccess) return e;
-            if ((e = cudaMalloc(&rs.entries, cap_t * sizeof(uint64_t))) != cudaSuccess) return e;
-            rs.slots_cap = slots;
-            rs.entries_cap = cap_t;
+            if ((e = cudaMalloc(&rs.mem, bytes)) != cudaSuccess) return e;
+            rs.cap = bytes;
         }
     }
     return filter_flows_clear(ctx, ctx->admin_stream);
@@ -285,9 +307,7 @@ void filter_tables_free(bnk_ctx *ctx) {
     cudaFree(ft.flow_keys);
     cudaFree(ft.flow_exp);
     for (bnk_ctx::RuleSet &rs : ctx->rule_set) {
-        cudaFree(rs.keys);
-        cudaFree(rs.span);
-        cudaFree(rs.entries);
+        cudaFree(rs.mem);
         for (cudaEvent_t ev : rs.in_use) cudaEventDestroy(ev);
         rs = bnk_ctx::RuleSet{};
     }
@@ -395,7 +415,7 @@ int filter_flows_import(bnk_ctx *ctx, const bnk_flow_entry *entries, size_t n) {
         }
         if (cap == 0) return BNK_EFULL;
         const size_t base = flow_region(ft, cls);
-        uint32_t at = (uint32_t)mix64(key) & (cap - 1);
+        uint32_t at = flow_hash(key) & (cap - 1);
         bool placed = false;
         for (uint32_t probe = 0; probe < cap && !placed; probe++, at = (at + 1) & (cap - 1)) {
             unsigned long long &k = h.keys[base + at];
@@ -535,48 +555,111 @@ int filter_acl_upload(bnk_ctx *ctx, int enforce, const bnk_acl_tuple *tuples, si
     std::lock_guard<std::mutex> one_at_a_time(ctx->acl_mu);
     FilterTables &ft = ctx->ft;
     struct Item {
-        uint64_t key, ent;
+        uint64_t key, ent; // prefix length << 32 | address;  proto << 32 | first << 16 | last
     };
     std::vector<Item> items;
     items.reserve(n);
-    uint64_t len_mask = 0;
     for (size_t i = 0; i < n; i++) {
         const bnk_acl_tuple &t = tuples[i];
         if (t.prefix_len > 32) return BNK_EINVAL;
         if (t.proto != 6 && t.proto != 17 && t.proto != 1) continue; // can never equal a parsed protocol
         if (t.proto != 1 && t.port_first > t.port_last) continue;    // empty range
-        items.push_back({rule_key(t.prefix_len, t.addr),
+        items.push_back({(uint64_t)t.prefix_len << 32 | (t.addr & prefix_mask(t.prefix_len)),
                          ((uint64_t)t.proto << 32) | ((uint64_t)t.port_first << 16) | t.port_last});
-        len_mask |= 1ull << t.prefix_len;
     }
     std::sort(items.begin(), items.end(), [](const Item &a, const Item &b) {
         return a.key != b.key ? a.key < b.key : a.ent < b.ent;
     });
-    items.erase(std::unique(items.begin(), items.end(),
-                            [](const Item &a, const Item &b) { return a.key == b.key && a.ent == b.ent; }),
-                items.end());
-    size_t groups = 0;
-    for (size_t i = 0; i < items.size(); i++)
-        if (i == 0 || items[i].key != items[i - 1].key) groups++;
-    uint32_t slots = 0;
-    if (groups) {
-        slots = 16;
-        while ((size_t)slots < groups * 8) slots <<= 1; // a quarter full at most: misses end after 1.4 probes on average, and the lanes of a warp wait for the longest of their walks
-    }
-    std::vector<uint64_t> keys(slots, 0);
-    std::vector<uint2> span(slots, make_uint2(0, 0));
-    std::vector<uint64_t> ents(items.size());
+    // groups in the order of rising prefix length, their ranges merged
+    std::vector<RuleGroup> groups;
+    std::vector<uint32_t> ports;
+    size_t n_long = 0;
     for (size_t i = 0; i < items.size();) {
-        size_t j = i;
-        while (j < items.size() && items[j].key == items[i].key) {
-            ents[j] = items[j].ent;
-            j++;
+        const uint64_t key = items[i].key;
+        RuleGroup g{};
+        g.len = (uint32_t)(key >> 32);
+        g.addr = (uint32_t)key;
+        for (; i < items.size() && items[i].key == key && (items[i].ent >> 32) == 1; i++) g.parent = 1u << 31; // icmp ignores ports
+        for (const uint64_t proto : {6, 17}) {
+            uint32_t count = 0, &at = proto == 6 ? g.tcp_at : g.udp_at;
+            at = (uint32_t)ports.size();
+            for (; i < items.size() && items[i].key == key && (items[i].ent >> 32) == proto; i++) {
+                const uint32_t first = (uint32_t)items[i].ent >> 16, last = (uint32_t)items[i].ent & 0xffffu;
+                if (count && first <= (ports.back() & 0xffffu) + 1) { // overlaps or continues the range before it
+                    ports.back() = (ports.back() & 0xffff0000u) | std::max(last, ports.back() & 0xffffu);
+                } else {
+                    ports.push_back(first << 16 | last);
+                    count++;
+                }
+            }
+            (proto == 6 ? g.tcp0 : g.udp0) = count ? ports[at] : kNoPorts;
+            g.n_ports |= count << (proto == 6 ? 0 : 16); // at most 32,768: there is a port between two ranges
+            while (ports.size() & 3) ports.push_back(kNoPorts);
         }
-        uint32_t h = rule_hash(items[i].key) & (slots - 1);
-        while (keys[h]) h = (h + 1) & (slots - 1);
-        keys[h] = items[i].key;
-        span[h] = make_uint2((uint32_t)i, (uint32_t)(j - i));
-        i = j;
+        n_long += g.len > 24;
+        groups.push_back(g);
+    }
+    // The index.  A group's parent is what a lookup of its prefix finds before the group itself is entered.
+    size_t n_blocks = 0;
+    {
+        std::vector<bool> seen(65536, false);
+        for (const RuleGroup &g : groups)
+            if (g.len > 16 && !seen[g.addr >> 16]) {
+                seen[g.addr >> 16] = true;
+                n_blocks++;
+            }
+    }
+    const size_t slots = rule_long_slots(n_long);
+    const RuleLayout at(n_blocks, slots, groups.size(), ports.size());
+    std::vector<uint8_t> image(groups.empty() ? 0 : at.total, 0);
+    if (!groups.empty()) {
+        uint32_t *const top = reinterpret_cast<uint32_t *>(image.data() + at.top);
+        uint2 *const blocks = reinterpret_cast<uint2 *>(image.data() + at.blocks);
+        RuleGroup *const table = reinterpret_cast<RuleGroup *>(image.data() + at.table);
+        const uint32_t mask = (uint32_t)slots - 1;
+        std::vector<uint32_t> number(slots); // group of each place in the table
+        uint32_t used = 0;
+        for (uint32_t k = 0; k < groups.size(); k++) {
+            RuleGroup &g = groups[k];
+            const uint32_t len = g.len, addr = g.addr;
+            uint32_t parent;
+            if (len <= 16) {
+                parent = top[addr >> 16];
+                std::fill_n(top + (addr >> 16), (size_t)1 << (16 - len), k + 1);
+            } else {
+                uint32_t &t = top[addr >> 16];
+                if (!(t & kRuleBlock)) {
+                    std::fill_n(blocks + (size_t)used * 256, 256, make_uint2(t, 0));
+                    t = kRuleBlock | used++;
+                }
+                uint2 *const e = blocks + (size_t)(t & ~kRuleBlock) * 256 + ((addr >> 8) & 255u);
+                parent = e->x;
+                if (len <= 24) {
+                    std::for_each(e, e + ((size_t)1 << (24 - len)), [&](uint2 &v) { v.x = k + 1; });
+                } else {
+                    // is there a longer one than those of up to 24?
+                    bool found = false;
+                    for (uint32_t l = len; !found && l-- > 25;) {
+                        if (!(e->y >> (l - 25) & 1u)) continue;
+                        const uint32_t outer = addr & prefix_mask(l);
+                        uint32_t h = rule_hash(outer, l) & mask;
+                        while (table[h].len && (table[h].addr != outer || table[h].len != l)) h = (h + 1) & mask;
+                        found = table[h].len != 0;
+                        if (found) parent = number[h] + 1;
+                    }
+                    e->y |= 1u << (len - 25);
+                    uint32_t h = rule_hash(addr, len) & mask;
+                    while (table[h].len) h = (h + 1) & mask;
+                    g.parent |= parent;
+                    table[h] = g;
+                    number[h] = k;
+                    continue;
+                }
+            }
+            g.parent |= parent;
+        }
+        memcpy(image.data() + at.groups, groups.data(), groups.size() * sizeof(RuleGroup));
+        if (!ports.empty()) memcpy(image.data() + at.ports, ports.data(), ports.size() * sizeof(uint32_t));
     }
     bnk_ctx::RuleSet &spare = ctx->rule_set[ctx->rule_cur ^ 1];
     // Kernels launched before the previous switch may still be reading the spare set: wait for those (the events
@@ -588,29 +671,15 @@ int filter_acl_upload(bnk_ctx *ctx, int enforce, const bnk_acl_tuple *tuples, si
     spare.in_use.clear();
     // A context created without max_acl_tuples grows the spare set here when a larger table arrives
     // (an allocation can stall the device for a moment; state the capacity to avoid that).
-    if (slots > spare.slots_cap) {
-        cudaFree(spare.keys);
-        cudaFree(spare.span);
-        spare.keys = nullptr;
-        spare.span = nullptr;
-        spare.slots_cap = 0;
-        if (cudaMalloc(&spare.keys, slots * sizeof(uint64_t)) != cudaSuccess) return BNK_ENOMEM;
-        if (cudaMalloc(&spare.span, slots * sizeof(uint2)) != cudaSuccess) return BNK_ENOMEM;
-        spare.slots_cap = slots;
-    }
-    if (ents.size() > spare.entries_cap) {
-        cudaFree(spare.entries);
-        spare.entries = nullptr;
-        spare.entries_cap = 0;
-        if (cudaMalloc(&spare.entries, ents.size() * sizeof(uint64_t)) != cudaSuccess) return BNK_ENOMEM;
-        spare.entries_cap = ents.size();
+    if (image.size() > spare.cap) {
+        cudaFree(spare.mem);
+        spare.mem = nullptr;
+        spare.cap = 0;
+        if (cudaMalloc(&spare.mem, image.size()) != cudaSuccess) return BNK_ENOMEM;
+        spare.cap = image.size();
     }
     cudaStream_t as = ctx->admin_stream;
-    if (slots) {
-        cudaMemcpyAsync(spare.keys, keys.data(), slots * sizeof(uint64_t), cudaMemcpyHostToDevice, as);
-        cudaMemcpyAsync(spare.span, span.data(), slots * sizeof(uint2), cudaMemcpyHostToDevice, as);
-        if (!ents.empty()) cudaMemcpyAsync(spare.entries, ents.data(), ents.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, as);
-    }
+    if (!image.empty()) cudaMemcpyAsync(spare.mem, image.data(), image.size(), cudaMemcpyHostToDevice, as);
     if (cudaStreamSynchronize(as) != cudaSuccess) return BNK_ECUDA;
     {
         std::unique_lock<std::shared_mutex> tables(ctx->submit_mu); // between two submits
@@ -624,11 +693,12 @@ int filter_acl_upload(bnk_ctx *ctx, int enforce, const bnk_acl_tuple *tuples, si
                 old.in_use.push_back(ev);
             }
         }
-        ft.rule_keys = spare.keys;
-        ft.rule_span = spare.span;
-        ft.rule_entries = spare.entries;
-        ft.rule_slots = slots;
-        ft.len_mask = len_mask;
+        ft.rule_top = image.empty() ? nullptr : reinterpret_cast<const uint32_t *>(spare.mem + at.top);
+        ft.rule_blocks = reinterpret_cast<const uint2 *>(spare.mem + at.blocks);
+        ft.rule_long = reinterpret_cast<const RuleGroup *>(spare.mem + at.table);
+        ft.rule_long_mask = (uint32_t)slots - 1;
+        ft.rule_groups = reinterpret_cast<const RuleGroup *>(spare.mem + at.groups);
+        ft.rule_ports = reinterpret_cast<const uint32_t *>(spare.mem + at.ports);
         ft.enforce = enforce ? 1 : 0;
         ctx->rule_cur ^= 1;
     }
@@ -645,13 +715,14 @@ cudaError_t launch_filter_note(bnk_batch *b, uint32_t n, long long now_ns, const
     return cudaGetLastError();
 }
 
-cudaError_t launch_filter_check(bnk_batch *b, uint32_t n, long long now_ns, bool only_status_ok, const Done &done, cudaStream_t s) {
+cudaError_t launch_filter_check(bnk_batch *b, uint32_t n, long long now_ns, bool only_status_ok, uint8_t *host_status,
+                                const Done &done, cudaStream_t s) {
     bnk_ctx *ctx = b->ctx;
     if (n == 0) return cudaSuccess;
     // open pipeline: the packet handed to the filter is the decrypted payload of out_len bytes
     const uint32_t *lens = only_status_ok ? b->dev.out_len : b->dev.len;
     launch_kernel(n <= dependent_launch_up_to(), filter_check_kernel, dim3((n + 127) / 128), dim3(128), s, ctx->ft,
-        b->dev.ring, b->dev.off, lens, b->dev.status, n, b->ring_bytes, now_ns, only_status_ok ? 1 : 0, done);
+        b->dev.ring, b->dev.off, lens, b->dev.status, n, b->ring_bytes, now_ns, only_status_ok ? 1 : 0, host_status, done);
     ctx->launches += 1;
     return cudaGetLastError();
 }

@@ -307,3 +307,52 @@ def test_rule_tables_with_many_prefix_lengths(gpu_lib, oracle, shape):
         f._batch.close()
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 5000])  # a CTA's statuses leave as one line
+def test_nested_prefixes_and_merged_port_ranges(gpu_lib, oracle, n):
+    """Prefixes of every length one inside the other, around the steps of the index (16, 24 bits), each with several port
+    ranges that touch, overlap or leave a port between them: a packet is allowed by whichever contains it."""
+    from bnk_b200 import Context
+    from bnk_b200.device import F_NO_H2D
+    from bnk_b200.filter import CompiledRule, PortRange, flatten_rules
+
+    rng = np.random.default_rng(n)
+    base = RC.ip("100.64.0.0")
+    spots = base + rng.integers(0, 1 << 18, 12)  # prefixes crowd around these
+    rules, chk_rules = [], []
+    for bits in [0] + [int(b) for b in rng.integers(1, 33, 700)] + [15, 16, 17, 23, 24, 25, 31, 32] * 6:
+        addr = int(spots[rng.integers(0, len(spots))]) ^ int(rng.integers(0, 1 << int(rng.integers(1, 20))))
+        addr &= (0xffffffff << (32 - bits)) & 0xffffffff if bits else 0
+        proto = str(rng.choice(["tcp", "udp", "icmp"], p=[0.5, 0.45, 0.05])) if bits > 8 else "udp"
+        at, ranges = int(rng.integers(0, 65536)), []
+        for _ in range(int(rng.integers(1, 6)) if proto != "icmp" else 0):
+            end = min(65535, at + int(rng.choice([0, 1, 5, 300])))
+            ranges.append((at, end))
+            at = min(65535, end + int(rng.choice([0, 1, 2, 40])))
+        rules.append(CompiledRule(srcs=[f"{addr >> 24}.{addr >> 16 & 255}.{addr >> 8 & 255}.{addr & 255}/{bits}"], proto=proto,
+                                  ports=[PortRange(*r) for r in ranges]))
+        chk_rules.append(([(addr, bits)], proto, ranges))
+    chk = oracle.Filter()
+    chk.set_rules(chk_rules)
+    pick = rng.integers(0, len(chk_rules), n)
+    h = np.zeros((n, 28), np.uint8)
+    lens = np.full(n, 28, np.uint32)
+    for i, k in enumerate(pick):  # sources inside and beside a prefix, ports at and beside the ends of a range
+        (addr, bits), = chk_rules[k][0]
+        src = (addr + int(rng.integers(-2, 3)) + int(rng.integers(0, 1 << min(32 - bits, 9)))) & 0xffffffff
+        ends = [e for r in chk_rules[int(rng.choice(pick))][2] for e in r] or [80]
+        port = (int(rng.choice(ends)) + int(rng.integers(-1, 2))) & 0xffff
+        h[i] = np.frombuffer([RC.tcp, RC.udp, lambda a, b, c, d: RC.icmp_echo(a, b, False)][int(rng.integers(0, 3))](src, RC.SELF, 40000, port)[:28], np.uint8)
+    want = chk.check_batch(np.ascontiguousarray(h), 28, lens, RC.T0)
+    with Context(max_keypairs=1, flow_capacity=1 << 10) as c:
+        c.acl_set(True, flatten_rules(rules))
+        b = c.batch(n, n * 48)
+        b.ring.reshape(n, 48)[:, 16:44] = h
+        b.off[:], b.len[:] = np.arange(n) * 48, lens
+        for flags in (0, F_NO_H2D):
+            b.status[:] = 99
+            b.filter_check(n, RC.T0, flags)
+            assert np.array_equal(b.status == 0, want != 0), np.flatnonzero((b.status == 0) != (want != 0))[:5]
+        assert n < 1000 or 200 < (want != 0).sum() < n - 200
+        b.close()
