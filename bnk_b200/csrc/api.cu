@@ -1,6 +1,7 @@
 // C ABI of libbnkgpu.so (declared in include/bnk_gpu.h): contexts, device tables,
 // pinned packet rings with device mirrors, and the submit/wait pipeline that strings
 // host->device copies, the kernels and device->host copies on one CUDA stream per batch.
+#include <algorithm>
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
@@ -9,6 +10,7 @@
 #include <thread>
 
 #include "filter_device.cuh"
+#include "scan.h"
 #include "submit_order.h"
 
 namespace {
@@ -52,17 +54,13 @@ cudaError_t dev_alloc_zero(T **p, size_t count) {
     return cudaMemset(*p, 0, count * sizeof(T));
 }
 
-// highest ring byte any of the first n packets can touch (input or output side), and their bytes
-uint64_t ring_extent(const bnk_batch *b, uint32_t n, uint32_t slack, uint64_t *bytes = nullptr) {
-    const uint32_t *off = b->host.off, *len = b->host.len;
-    uint64_t ext = 0, sum = 0;
-    for (uint32_t i = 0; i < n; i++) {
-        const uint64_t e = (uint64_t)off[i] + len[i] + slack;
-        if (e > ext) ext = e;
-        sum += len[i];
-    }
-    if (bytes) *bytes = sum + (uint64_t)n * slack;
-    ext = (ext + 15) & ~15ull;
+// highest ring byte any of the first n packets can touch (input or output side); their bytes; whether they lie in the
+// ring in order, each with `room` bytes of its own behind it
+uint64_t ring_extent(const bnk_batch *b, uint32_t n, uint32_t slack, uint64_t *bytes = nullptr, uint32_t room = 0, bool *in_order = nullptr) {
+    const PacketScan r = scan_packets(b->host.off, b->host.len, n, room);
+    if (bytes) *bytes = r.sum + (uint64_t)n * slack;
+    if (in_order) *in_order = r.in_order;
+    const uint64_t ext = n ? (r.end + slack + 15) & ~15ull : 0;
     return ext > b->ring_bytes ? b->ring_bytes : ext;
 }
 
@@ -145,6 +143,86 @@ constexpr uint64_t kSparse = 128;
 bool heads_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, uint64_t ext) {
     return (npkts <= 1024 || ext >= kSparse * npkts) && host_direct(b, npkts, flags, 0);
 }
+// A large batch that is alone in flight goes over the link in pieces: while one is worked on, the next comes up and the
+// one before goes down, so both copy engines are busy.  Pieces end on pages of the ring (a copy that starts elsewhere is
+// up to a sixth slower: 190 MB up and down in 8 MB pieces 4.1 ms against 4.9), at most kPieceMost bytes each, with small
+// ones first and last, when one direction has nothing to do yet or any more.  Packets have to lie in the ring in order.
+constexpr uint64_t kPieceLeast = 1ull << 20, kPieceMost = 8ull << 20, kPage = 4096;
+struct Piece {
+    uint32_t first, count;       // packets
+    uint64_t up, up_to;          // ring bytes that come up in front of them
+    uint64_t down, down_to;      // ring bytes nobody works on any more behind them
+};
+class Pieces {
+  public:
+    // `more`: a packet's kernel reads and writes at most len + more bytes from its offset on.  All of them have to be up: a
+    // later copy must not run over what the kernel has written.
+    Pieces(const bnk_batch *b, uint32_t n, uint32_t more, uint64_t ext) : off_(b->host.off), len_(b->host.len), n_(n), more_(more), ext_(ext) {}
+    bool next(Piece &p) {
+        if (at_ == n_) return false;
+        p.first = at_;
+        p.up = up_;
+        p.down = down_;
+        do { // a packet larger than a piece takes several
+            const uint64_t left = ext_ - up_, size = std::min(std::min(kPieceMost, up_ + kPieceLeast), std::max(kPieceLeast, left / 2));
+            up_ = left <= size + size / 2 ? ext_ : (up_ + size) & ~(kPage - 1);
+            if (up_ == ext_) at_ = n_;
+            while (at_ < n_ && (uint64_t)off_[at_] + more_ + len_[at_] <= up_) at_++;
+        } while (at_ == p.first);
+        down_ = at_ == n_ ? ext_ : std::max(down_, std::min(up_, (uint64_t)off_[at_]) & ~(kPage - 1));
+        p.count = at_ - p.first;
+        p.up_to = up_;
+        p.down_to = down_;
+        return true;
+    }
+
+  private:
+    const uint32_t *off_, *len_;
+    uint32_t n_, more_, at_ = 0;
+    uint64_t ext_, up_ = 0, down_ = 0;
+};
+// Below ctx->pieces_from (24 MB) a kernel on the pinned ring is as fast or faster, because the first piece up and the last
+// one down have no company: 16,384 x 1420 B 710 us against 750, 32,768 1390 against 1330, 131,072 5.74 ms against 4.96.
+// With small packets that kernel is bound by what its warps compute, ~7.5 ns a packet, and pieces win earlier: 8192 x
+// 300 B 138 us against 144, 16,384 252 against 233, 131,072 x 64 B 990 against 600.
+constexpr uint32_t kManySmall = 10240, kSmallBytes = 512;
+bool in_pieces(const bnk_batch *b, uint32_t n, uint32_t flags, uint64_t ext, bool in_order) {
+    const uint64_t from = b->ctx->pieces_from;
+    if (ext < from && (n < kManySmall || ext > (uint64_t)n * kSmallBytes || ext < from / 16)) return false;
+    return in_order && b->up_stream && !(flags & (BNK_F_NO_H2D | BNK_F_NO_D2H | BNK_F_USE_OUT_LEN)) &&
+           b->ctx->in_flight.load(std::memory_order_relaxed) == (b->counted ? 1 : 0);
+}
+// Copies a piece up and lets stream s go on behind it / copies down what is done on s.
+cudaError_t piece_up(bnk_batch *b, const Piece &p, cudaStream_t s) {
+    cudaError_t e = cudaMemcpyAsync(b->dev.ring + p.up, b->host.ring + p.up, p.up_to - p.up, cudaMemcpyHostToDevice, b->up_stream);
+    if (e == cudaSuccess) e = cudaEventRecord(b->ev_up, b->up_stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b->ev_up, 0);
+    return e;
+}
+cudaError_t piece_down(bnk_batch *b, const Piece &p, cudaStream_t s) {
+    if (p.down_to == p.down) return cudaSuccess;
+    cudaError_t e = cudaEventRecord(b->ev_down, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(b->down_stream, b->ev_down, 0);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(b->host.ring + p.down, b->dev.ring + p.down, p.down_to - p.down, cudaMemcpyDeviceToHost, b->down_stream);
+    return e;
+}
+cudaError_t pieces_end(bnk_batch *b, cudaStream_t s) { // s is done when the last piece is down
+    cudaError_t e = cudaEventRecord(b->ev_down, b->down_stream);
+    return e != cudaSuccess ? e : cudaStreamWaitEvent(s, b->ev_down, 0);
+}
+AeadArgs piece_args(AeadArgs a, const Piece &p) {
+    a.off += p.first;
+    a.len += p.first;
+    a.slot += p.first;
+    a.counter += p.first;
+    if (a.res[0].counter) a.res[0].counter += p.first;
+    a.res[0].out_len += p.first;
+    a.res[0].status += p.first;
+    a.n = p.count;
+    return a;
+}
+
 struct HostAlias {
     bnk_batch *b;
     DeviceBatch saved;
@@ -318,6 +396,9 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     if (const char *m = getenv("BNK_HOST_DIRECT_BYTES")) // largest ring extent served without copies; 0 = never
         ctx->host_direct_bytes = strtoull(m, nullptr, 0);
     if (!prop.unifiedAddressing || !prop.canMapHostMemory) ctx->host_direct_bytes = 0; // pinned memory must have one address
+    ctx->pieces_from = 24u << 20;
+    if (const char *m = getenv("BNK_PIECES_FROM")) // tuning aid: ring extent from which a batch that is alone goes in pieces
+        ctx->pieces_from = strtoull(m, nullptr, 0);
     ctx->aead_side_stream_from = 1u << 18; // below, the seal/open launch is too short for the hand-over between streams to pay
     if (const char *m = getenv("BNK_AEAD_SIDE_STREAM_FROM")) // tuning aid: 0 = seal/open always on the batch's own stream
         ctx->aead_side_stream_from = (uint32_t)strtoul(m, nullptr, 0);
@@ -750,6 +831,10 @@ int bnk_batch_destroy(bnk_batch *b) {
     if (b->a_end) cudaEventDestroy(b->a_end);
     if (b->t_end) cudaEventDestroy(b->t_end);
     if (b->ev_order) cudaEventDestroy(b->ev_order);
+    if (b->ev_up) cudaEventDestroy(b->ev_up);
+    if (b->ev_down) cudaEventDestroy(b->ev_down);
+    if (b->up_stream) cudaStreamDestroy(b->up_stream);
+    if (b->down_stream) cudaStreamDestroy(b->down_stream);
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
     if (b->ev_fence) cudaEventDestroy(b->ev_fence);
@@ -790,6 +875,7 @@ int bnk_batch_create(bnk_ctx *ctx, uint32_t max_pkts, uint64_t ring_bytes, bnk_b
     const size_t np = b->npad;
     b->desc_room = (25 * np + 255) & ~(size_t)255;
     b->joint_copy = b->desc_room <= 64u * 1024;
+    if (!b->joint_copy) b->desc_room = (b->desc_room + 4095) & ~(size_t)4095; // the ring then starts on a page: see Pieces
     H((void **)&b->h_desc, b->desc_room + ring_bytes);
     if (e == cudaSuccess) {
         b->host.ring = b->h_desc + b->desc_room;
@@ -841,6 +927,12 @@ int bnk_batch_create(bnk_ctx *ctx, uint32_t max_pkts, uint64_t ring_bytes, bnk_b
         e = cudaStreamCreateWithPriority(&b->aead_stream, cudaStreamNonBlocking, ctx->prio_low);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_aead_go, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_aead_done, cudaEventDisableTiming);
+    }
+    if (e == cudaSuccess && (ring_bytes >= ctx->pieces_from || max_pkts >= kManySmall)) {
+        e = cudaStreamCreateWithPriority(&b->up_stream, cudaStreamNonBlocking, ctx->prio_high);
+        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->down_stream, cudaStreamNonBlocking, ctx->prio_high);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_up, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_down, cudaEventDisableTiming);
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
@@ -971,6 +1063,40 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     return BNK_SUCCESS;
 }
 
+static int seal_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flags, int64_t now_unix_ns) {
+    bnk_ctx *ctx = b->ctx;
+    cudaStream_t s = b->stream;
+    const bool timed = (flags & BNK_F_TIMED) != 0;
+    CK(ctx, desc_copy(b, npkts, D_OFF, b->dev_stale ? D_STATUS : (flags & BNK_F_ASSIGN_COUNTERS) ? D_SLOT : D_COUNTER, true, s));
+    b->dev_stale = b->ring_partial = false;
+    CK(ctx, order_kernels_begin(b, s));
+    if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
+    if (flags & BNK_F_ASSIGN_COUNTERS) CK(ctx, launch_assign_counters(b, npkts, b->dev.slot, b->dev.counter, s));
+    AeadArgs a = aead_args(b, npkts, false, nullptr); // (length classes would only be those of a piece, and the link is the bound)
+    a.res[0].counter = nullptr; // in place already
+    a.behind_kernel = true;
+    const bool note = (flags & BNK_F_NOTE_OUTBOUND) && ctx->ft.enforce && ctx->ft.flow_capacity; // filter.go:192-194
+    const bool sweep = note && flow_note_begins(b, npkts, now_unix_ns);
+    if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
+    Piece p;
+    for (Pieces pieces(b, npkts, BNK_WG_HEADER + 16 + BNK_WG_TAG, ext); pieces.next(p);) {
+        CK(ctx, piece_up(b, p, s));
+        if (note) CK(ctx, launch_filter_note(b, p.first, p.count, now_unix_ns, Done{}, s));
+        CK(ctx, launch_seal(piece_args(a, p), s, ctx));
+        CK(ctx, piece_down(b, p, s));
+    }
+    if (timed) CK(ctx, cudaEventRecord(b->a_end, s));
+    if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, Done{}, s));
+    else if (note) CK(ctx, launch_flow_report(b, s));
+    if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
+    b->kernel_timed = b->aead_timed = timed;
+    CK(ctx, tally_if_asked(b, npkts, flags, s));
+    CK(ctx, order_kernels_end(b, s, false));
+    CK(ctx, desc_copy(b, npkts, D_COUNTER, D_STATUS, false, s));
+    CK(ctx, pieces_end(b, s));
+    return BNK_SUCCESS;
+}
+
 int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_unix_ns) {
     const bool device_only = (flags & BNK_F_NO_H2D) && (flags & BNK_F_NO_D2H);
     int rc = begin_submit(b, npkts, !device_only);
@@ -984,7 +1110,9 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     // header room + payload + padding (< 16) + tag
     const bool refresh = b->dev_stale; // the device copies are behind the host arrays: upload whatever the flags say
     uint64_t bytes = 0;
-    const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, 16 + 16 + 16, &bytes);
+    bool in_order = false;
+    const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, 16 + 16 + 16, &bytes, BNK_WG_HEADER + BNK_WG_TAG, &in_order);
+    if (in_pieces(b, npkts, flags, ext, in_order)) return seal_pieces(b, npkts, ext, flags, now_unix_ns);
     if (ctx->aead_mode != 1) {
         if (host_direct(b, npkts, flags, ext)) return seal_direct(b, npkts, bytes, flags, now_unix_ns, false);
         if (!refresh && (flags & BNK_F_NO_H2D) && host_direct(b, npkts, flags & ~BNK_F_NO_H2D, ext))
@@ -1003,7 +1131,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     if ((flags & BNK_F_NOTE_OUTBOUND) && n && ctx->ft.enforce && ctx->ft.flow_capacity) { // filter.go:192-194
         const bool sweep = flow_note_begins(b, npkts, now_unix_ns);
-        CK(ctx, launch_filter_note(b, npkts, now_unix_ns, Done{}, s));
+        CK(ctx, launch_filter_note(b, 0, npkts, now_unix_ns, Done{}, s));
         if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, Done{}, s));
         else CK(ctx, launch_flow_report(b, s));
     }
@@ -1130,6 +1258,46 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     return BNK_SUCCESS;
 }
 
+static int open_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flags, int64_t now_unix_ns) {
+    bnk_ctx *ctx = b->ctx;
+    cudaStream_t s = b->stream;
+    const bool timed = (flags & BNK_F_TIMED) != 0, demux = (flags & BNK_F_DEMUX_INDEX) != 0;
+    CK(ctx, desc_copy(b, npkts, D_OFF, b->dev_stale ? D_STATUS : demux ? D_LEN : D_SLOT, true, s));
+    b->dev_stale = b->ring_partial = false;
+    CK(ctx, order_kernels_begin(b, s));
+    if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
+    AeadArgs a = aead_args(b, npkts, true, nullptr);
+    a.behind_kernel = true;
+    const bool replay = (flags & BNK_F_REPLAY) != 0, one_launch = npkts <= kGroupMax;
+    if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
+    Piece p;
+    for (Pieces pieces(b, npkts, 0, ext); pieces.next(p);) {
+        CK(ctx, piece_up(b, p, s));
+        if (demux) CK(ctx, launch_demux_index(b, p.first, p.count, a.len, s));
+        CK(ctx, launch_open(piece_args(a, p), s, ctx));
+        CK(ctx, piece_down(b, p, s)); // the checks below say which plaintexts count, and change no byte of them
+    }
+    if (timed) CK(ctx, cudaEventRecord(b->a_end, s));
+    if (replay && one_launch) {
+        CK(ctx, launch_open_tail(b, npkts, true, nullptr, Done{}, s));
+    } else if (replay) {
+        CK(ctx, launch_group_by_slot(b, npkts, s));
+        CK(ctx, launch_replay(b, npkts, s));
+    }
+    if (flags & BNK_F_INNER_CHECK) CK(ctx, launch_inner_check(b, npkts, s));
+    if (flags & BNK_F_CHECK_INBOUND) {
+        flow_check_begins(b, now_unix_ns);
+        CK(ctx, launch_filter_check(b, npkts, now_unix_ns, true, nullptr, Done{}, s));
+    }
+    if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
+    b->kernel_timed = b->aead_timed = timed;
+    CK(ctx, tally_if_asked(b, npkts, flags, s));
+    CK(ctx, order_kernels_end(b, s, false));
+    CK(ctx, desc_copy(b, npkts, demux ? D_SLOT : D_COUNTER, D_STATUS, false, s));
+    CK(ctx, pieces_end(b, s));
+    return BNK_SUCCESS;
+}
+
 int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_unix_ns) {
     const bool device_only = (flags & BNK_F_NO_H2D) && (flags & BNK_F_NO_D2H);
     int rc = begin_submit(b, npkts, !device_only);
@@ -1141,7 +1309,9 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     const size_t n = npkts;
     const bool refresh = b->dev_stale;
     uint64_t bytes = 0;
-    const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, (flags & BNK_F_USE_OUT_LEN) ? 48 : 0, &bytes);
+    bool in_order = false;
+    const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, (flags & BNK_F_USE_OUT_LEN) ? 48 : 0, &bytes, 0, &in_order);
+    if (in_pieces(b, npkts, flags, ext, in_order)) return open_pieces(b, npkts, ext, flags, now_unix_ns);
     if (ctx->aead_mode != 1 && host_direct(b, npkts, flags, ext)) return open_direct(b, npkts, bytes, flags, now_unix_ns);
     // BNK_F_USE_OUT_LEN reads the lengths a seal left on the device: an upload beside it must not bring the
     // host's out_len along, so it moves the fields one by one instead of the whole slab.
@@ -1159,7 +1329,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     const uint32_t *order = nullptr;
     AeadArgs oa = aead_args(b, npkts, true, nullptr);
     if (flags & BNK_F_USE_OUT_LEN) oa.len = b->dev.out_len;
-    if (flags & BNK_F_DEMUX_INDEX) CK(ctx, launch_demux_index(b, npkts, oa.len, s));
+    if (flags & BNK_F_DEMUX_INDEX) CK(ctx, launch_demux_index(b, 0, npkts, oa.len, s));
     if (flags & BNK_F_SORT_BY_LENGTH) {
         CK(ctx, launch_length_order(b, npkts, oa.len, true, s));
         order = b->dev.len_order;
@@ -1243,7 +1413,7 @@ int bnk_filter_note_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t
     if (note) {
         const bool sweep = flow_note_begins(b, npkts, now_unix_ns);
         const Done done = watch_for(b);
-        CK(ctx, launch_filter_note(b, npkts, now_unix_ns, sweep ? Done{} : done, s));
+        CK(ctx, launch_filter_note(b, 0, npkts, now_unix_ns, sweep ? Done{} : done, s));
         if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, done, s));
         reported = true;
     }

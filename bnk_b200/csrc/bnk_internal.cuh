@@ -111,6 +111,7 @@ struct bnk_ctx {
     std::atomic<uint64_t> direct_in_flight{0}; // ring bytes of those that run on the pinned buffers
     int aead_mode; // 0 = choose by batch size, 1 = always thread per packet, 2 = always warp per packet (BNK_AEAD_KERNEL)
     uint32_t aead_side_stream_from; // batches of at least this many packets run seal/open on the low-priority stream (BNK_AEAD_SIDE_STREAM_FROM; 0 = never)
+    uint64_t pieces_from;           // ring extent from which a batch that is alone goes over the link in pieces (BNK_PIECES_FROM)
     int prio_low, prio_high;        // stream priority range of the device
     std::atomic<uint64_t> launches;
     std::atomic<uint64_t> seal_seq{0}; // number of the last seal launch that handed out nonces itself (see SendCounter)
@@ -186,6 +187,8 @@ struct bnk_batch {
     // kernel of another.
     cudaStream_t aead_stream;
     cudaEvent_t ev_aead_go, ev_aead_done;
+    cudaStream_t up_stream, down_stream; // of a batch large enough to go over the link in pieces
+    cudaEvent_t ev_up, ev_down;
     cudaEvent_t ev_fork, ev_join;
     cudaEvent_t k_begin, k_end, t_end, a_begin, a_end;
     bool in_flight;
@@ -367,7 +370,8 @@ uint32_t replay_scan_tiles(uint32_t max_pkts);     // tiles of the running-maxim
 uint32_t replay_hash_capacity(uint32_t max_pkts);  // entries of the duplicate-counter table
 
 // filter_kernels.cu
-cudaError_t launch_filter_note(bnk_batch *b, uint32_t n, long long now_ns, const Done &done, cudaStream_t s); // the inserts; no sweep
+// the inserts of packets [first, first + n); no sweep
+cudaError_t launch_filter_note(bnk_batch *b, uint32_t first, uint32_t n, long long now_ns, const Done &done, cudaStream_t s);
 cudaError_t launch_filter_check(bnk_batch *b, uint32_t n, long long now_ns, bool only_status_ok, uint8_t *host_status,
                                 const Done &done, cudaStream_t s);
 cudaError_t filter_tables_alloc(bnk_ctx *ctx);
@@ -391,7 +395,7 @@ cudaError_t filter_flows_maintain(bnk_batch *b, cudaStream_t s);
 cudaError_t launch_tally(bnk_batch *b, uint32_t n, cudaStream_t s);
 
 // inner_kernels.cu
-cudaError_t launch_demux_index(bnk_batch *b, uint32_t n, const uint32_t *len, cudaStream_t s);
+cudaError_t launch_demux_index(bnk_batch *b, uint32_t first, uint32_t n, const uint32_t *len, cudaStream_t s); // packets [first, first + n)
 cudaError_t launch_inner_check(bnk_batch *b, uint32_t n, cudaStream_t s);
 cudaError_t launch_classify(bnk_batch *b, uint32_t n, const Done &done, cudaStream_t s);
 // One 16-byte entry in one access, from and to the L2 that all SMs share.

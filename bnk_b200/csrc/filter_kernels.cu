@@ -705,12 +705,12 @@ int filter_acl_upload(bnk_ctx *ctx, int enforce, const bnk_acl_tuple *tuples, si
     return BNK_SUCCESS;
 }
 
-cudaError_t launch_filter_note(bnk_batch *b, uint32_t n, long long now_ns, const Done &done, cudaStream_t s) {
+cudaError_t launch_filter_note(bnk_batch *b, uint32_t first, uint32_t n, long long now_ns, const Done &done, cudaStream_t s) {
     bnk_ctx *ctx = b->ctx;
     FlowReport *const report = done.flag ? b->h_flow : nullptr;
     if (report) b->flow_reported = true;
     launch_kernel(n <= dependent_launch_up_to(), filter_note_kernel, dim3((n + 127) / 128), dim3(128), s, ctx->ft,
-        b->dev.ring, b->dev.off, b->dev.len, n, b->ring_bytes, now_ns, report, done);
+        b->dev.ring, b->dev.off + first, b->dev.len + first, n, b->ring_bytes, now_ns, report, done);
     ctx->launches += 1;
     return cudaGetLastError();
 }

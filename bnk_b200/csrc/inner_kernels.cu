@@ -125,10 +125,10 @@ cudaError_t launch_classify(bnk_batch *b, uint32_t n, const Done &done, cudaStre
     return cudaGetLastError();
 }
 
-cudaError_t launch_demux_index(bnk_batch *b, uint32_t n, const uint32_t *len, cudaStream_t s) {
+cudaError_t launch_demux_index(bnk_batch *b, uint32_t first, uint32_t n, const uint32_t *len, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     launch_kernel(n <= dependent_launch_up_to(), demux_index_kernel, dim3((n + 255) / 256), dim3(256), s, b->ctx->kt,
-        b->dev.ring, b->dev.off, len, b->dev.slot, n, b->ring_bytes);
+        b->dev.ring, b->dev.off + first, len + first, b->dev.slot + first, n, b->ring_bytes);
     ++b->ctx->launches;
     return cudaGetLastError();
 }
