@@ -228,57 +228,70 @@ __device__ __forceinline__ bool rules_allow(const FilterTables &ft, const Parsed
         g = a.z & 0x7fffffffu;
     }
 }
-// CheckInbound (filter.go:121-147) of a packet that parses, with enforcement on: a rule allows it, or it is the reply to
-// a flow that is alive (the key mirrors NoteOutbound's), which it then keeps alive.
-// The flow table is asked before the rules are looked at, so that the two searches wait for memory together.
-__device__ __forceinline__ uint8_t filter_verdict(const FilterTables &ft, const Parsed &p, long long now) {
-    const int cls = proto_class(p.proto);
-    const unsigned long long key = flow_key(p.src, p.sport, p.dport);
-    const unsigned long long *const keys = (const unsigned long long *)ft.flow_keys + flow_region(ft, cls);
-    long long *exps = ft.flow_exp + flow_region(ft, cls);
-    uint32_t h = flow_hash(key) & (ft.flow_capacity - 1);
-    unsigned long long k = FLOW_EMPTY;
-    long long exp = FLOW_FRESH;
-    FlowCtl *const ctl = flow_ctl(ft);
-    const long long floor = flow_floor(ctl);
-    if (ft.flow_capacity) {
+// The reply-flow half of CheckInbound: is the packet the reply to a flow that is alive (the key mirrors NoteOutbound's)?
+// In two steps, so that the first can wait for memory beside the search of the rules.
+struct FlowReply {
+    unsigned long long key, k;
+    long long exp, floor, *exps;
+    uint32_t h;
+    int cls;
+
+    __device__ __forceinline__ void begin(const FilterTables &ft, const Parsed &p) {
+        cls = proto_class(p.proto);
+        key = flow_key(p.src, p.sport, p.dport);
+        exps = ft.flow_exp + flow_region(ft, cls);
+        h = flow_hash(key) & (ft.flow_capacity - 1);
+        k = FLOW_EMPTY;
+        exp = FLOW_FRESH;
+        floor = flow_floor(flow_ctl(ft));
+        if (ft.flow_capacity == 0) return;
         if (key == FLOW_EMPTY) {
             exps = ft.flow_special_exp;
             h = cls;
         } else {
-            k = *(const volatile unsigned long long *)&keys[h];
+            k = ((const volatile unsigned long long *)ft.flow_keys + flow_region(ft, cls))[h];
         }
         exp = *(volatile long long *)&exps[h];
     }
-    if (rules_allow(ft, p)) return BNK_PKT_OK;
-    if (key != FLOW_EMPTY && k != key) {
-        exp = FLOW_FRESH;
-        for (uint32_t probe = 1; k != FLOW_EMPTY && probe < ft.flow_capacity; probe++) {
-            h = (h + 1) & (ft.flow_capacity - 1);
-            k = keys[h];
-            if (k == key) {
-                exp = *(volatile long long *)&exps[h];
-                break;
+    __device__ __forceinline__ uint8_t finish(const FilterTables &ft, uint8_t proto, long long now) {
+        if (key != FLOW_EMPTY && k != key) {
+            const unsigned long long *const keys = (const unsigned long long *)ft.flow_keys + flow_region(ft, cls);
+            exp = FLOW_FRESH;
+            for (uint32_t probe = 1; k != FLOW_EMPTY && probe < ft.flow_capacity; probe++) {
+                h = (h + 1) & (ft.flow_capacity - 1);
+                k = keys[h];
+                if (k == key) {
+                    exp = *(volatile long long *)&exps[h];
+                    break;
+                }
             }
         }
+        if (flow_absent(exp)) return BNK_PKT_FILTER_DENY;
+        FlowCtl *const ctl = flow_ctl(ft);
+        if (now < exp) { // strict: time.Before
+            const long long fresh = now + flow_ttl(proto);
+            *(volatile long long *)&exps[h] = fresh; // keep-alive on traffic
+            flow_keep_floor(ctl, fresh, floor);
+            return BNK_PKT_OK;
+        }
+        const long long prev = (long long)atomicExch((unsigned long long *)&exps[h], (unsigned long long)FLOW_DEAD);
+        if (!flow_absent(prev)) {
+            atomicAdd(&ctl->rep.live, 0ull - 1ull);
+            if (key != FLOW_EMPTY) atomicAdd(&ctl->rep.dead[cls], 1u);
+        }
+        return BNK_PKT_FILTER_DENY;
     }
-    if (flow_absent(exp)) return BNK_PKT_FILTER_DENY;
-    if (now < exp) { // strict: time.Before
-        const long long fresh = now + flow_ttl(p.proto);
-        *(volatile long long *)&exps[h] = fresh; // keep-alive on traffic
-        flow_keep_floor(ctl, fresh, floor);
-        return BNK_PKT_OK;
-    }
-    const long long prev = (long long)atomicExch((unsigned long long *)&exps[h], (unsigned long long)FLOW_DEAD);
-    if (!flow_absent(prev)) {
-        atomicAdd(&ctl->rep.live, 0ull - 1ull);
-        if (key != FLOW_EMPTY) atomicAdd(&ctl->rep.dead[cls], 1u);
-    }
-    return BNK_PKT_FILTER_DENY;
+};
+// CheckInbound (filter.go:121-147) of a packet that parses, with enforcement on: a rule allows it, or it is a reply.
+__device__ __forceinline__ uint8_t filter_verdict(const FilterTables &ft, const Parsed &p, long long now) {
+    FlowReply reply;
+    reply.begin(ft, p);
+    if (rules_allow(ft, p)) return BNK_PKT_OK;
+    return reply.finish(ft, p.proto, now);
 }
 
 // ---- the last word on an opened packet ----
-// What the open kernel notes of a plaintext's headers (InnerHeader::of) is all that the checks behind the replay
+// What the open kernel notes of a plaintext's headers is all that the checks behind the replay
 // window need, so that they do not go back to the packet: over the host link that would be a read per packet.
 //   x source address   y source port << 16 | destination port   z protocol | flags   w IPv4 total length
 constexpr uint32_t kInnerParses = 1u << 8; // filter.parse accepts it
@@ -296,6 +309,15 @@ struct VerdictArgs {
     uint32_t n;
     bool inner_check, check_inbound;
 };
+__device__ __forceinline__ Parsed inner_parsed(const uint4 &h) {
+    Parsed p;
+    p.src = h.x;
+    p.dst = 0;
+    p.sport = (uint16_t)(h.y >> 16);
+    p.dport = (uint16_t)h.y;
+    p.proto = (uint8_t)h.z;
+    return p;
+}
 __device__ __forceinline__ void final_verdict(const VerdictArgs &v, uint32_t i) {
     uint8_t st = *(volatile uint8_t *)&v.status[i];
     uint32_t l = v.out_len[i];
@@ -305,15 +327,8 @@ __device__ __forceinline__ void final_verdict(const VerdictArgs &v, uint32_t i) 
             if ((h.z & kInnerWhole) && h.x != 0 && h.x == v.allowed_ip[v.slot[i]]) l = h.w;
             else st = BNK_PKT_BAD_INNER;
         }
-        if (v.check_inbound && st == BNK_PKT_OK && v.ft.enforce) {
-            Parsed p;
-            p.src = h.x;
-            p.dst = 0;
-            p.sport = (uint16_t)(h.y >> 16);
-            p.dport = (uint16_t)h.y;
-            p.proto = (uint8_t)h.z;
-            st = (h.z & kInnerParses) ? filter_verdict(v.ft, p, v.now) : (uint8_t)BNK_PKT_FILTER_DENY;
-        }
+        if (v.check_inbound && st == BNK_PKT_OK && v.ft.enforce)
+            st = (h.z & kInnerParses) ? filter_verdict(v.ft, inner_parsed(h), v.now) : (uint8_t)BNK_PKT_FILTER_DENY;
         v.status[i] = st;
         v.out_len[i] = l;
     }

@@ -319,8 +319,11 @@ __device__ __forceinline__ SegMax seg_shfl_up(SegMax v, int o) {
 }
 // Inclusive scan of one value per thread over a CTA of NW warps; returns the exclusive prefix of the calling
 // thread and the total of the CTA.  `part` is NW entries of shared memory.
-template <int NW>
-__device__ __forceinline__ SegMax seg_block_exclusive(SegMax mine, SegMax *part, SegMax &total) {
+struct CtaSync {
+    __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+template <int NW, typename Sync = CtaSync>
+__device__ __forceinline__ SegMax seg_block_exclusive(SegMax mine, SegMax *part, SegMax &total, Sync sync = Sync()) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     SegMax inc = mine;
 #pragma unroll
@@ -330,9 +333,9 @@ __device__ __forceinline__ SegMax seg_block_exclusive(SegMax mine, SegMax *part,
     }
     SegMax ex = seg_shfl_up(inc, 1);
     if (lane == 0) ex = SegMax{0u, 0ull};
-    __syncthreads(); // `part` may still be read from an earlier call
+    sync(); // `part` may still be read from an earlier call
     if (lane == 31) part[warp] = inc;
-    __syncthreads();
+    sync();
     SegMax before{0u, 0ull};
     total = SegMax{0u, 0ull};
 #pragma unroll
@@ -474,21 +477,12 @@ __device__ __forceinline__ bool replay_hash_has_earlier(const ReplayArgs &a, uin
     }
     return false;
 }
-// Warp-wide over 32 consecutive positions: settles the pending verdicts, writes the refusals and marks the
-// ring.  Lanes that hit the same ring word hand their bits to the lowest of them.
-__device__ __forceinline__ void replay_finish_warp(const ReplayArgs &a, uint32_t p) {
+// Warp-wide: marks the accepted counters in the rings.  Lanes that hit the same ring word hand their bits to the lowest
+// of them.
+__device__ __forceinline__ void replay_mark_warp(const ReplayArgs &a, bool accepted, uint32_t slot, uint64_t c) {
     const uint32_t lane = threadIdx.x & 31;
-    uint8_t st = p < a.n ? a.state[p] : (uint8_t)RP_NOPART;
-    uint32_t slot = 0;
-    uint64_t c = 0;
-    if (st != RP_NOPART) {
-        slot = a.keys[p];
-        c = a.sorted_counter[p];
-    }
-    if (st == RP_PENDING) st = replay_hash_has_earlier(a, p, slot, c) ? RP_REJECT : RP_ACCEPT;
-    if (st == RP_REJECT) a.status[a.order[p]] = BNK_PKT_REPLAY;
     const uint64_t rmask = a.ring_blocks - 1;
-    const bool mark = st == RP_ACCEPT && (a.replay_last[slot] >> 6) - (c >> 6) < a.ring_blocks;
+    const bool mark = accepted && (a.replay_last[slot] >> 6) - (c >> 6) < a.ring_blocks;
     const unsigned long long word = mark ? (unsigned long long)slot * a.ring_blocks + ((c >> 6) & rmask) : ~0ull - lane;
     const uint32_t group = __match_any_sync(0xffffffffu, word);
     const bool leader = mark && (uint32_t)(__ffs(group) - 1) == lane;
@@ -509,6 +503,19 @@ __device__ __forceinline__ void replay_finish_warp(const ReplayArgs &a, uint32_t
     } else if (mark) {
         atomicOr(&ring[word], ((unsigned long long)bit_hi << 32) | bit_lo);
     }
+}
+// Warp-wide over 32 consecutive positions: settles the pending verdicts, writes the refusals and marks the ring.
+__device__ __forceinline__ void replay_finish_warp(const ReplayArgs &a, uint32_t p) {
+    uint8_t st = p < a.n ? a.state[p] : (uint8_t)RP_NOPART;
+    uint32_t slot = 0;
+    uint64_t c = 0;
+    if (st != RP_NOPART) {
+        slot = a.keys[p];
+        c = a.sorted_counter[p];
+    }
+    if (st == RP_PENDING) st = replay_hash_has_earlier(a, p, slot, c) ? RP_REJECT : RP_ACCEPT;
+    if (st == RP_REJECT) a.status[a.order[p]] = BNK_PKT_REPLAY;
+    replay_mark_warp(a, st == RP_ACCEPT, slot, c);
 }
 // The tile of the calling CTA (thread t: positions base..base+3): counters gathered when GATHER, else read
 // back; running maximum with `carry` in front; returns the tile as one span.
@@ -622,15 +629,15 @@ __global__ void __launch_bounds__(256) verdict_kernel(const __grid_constant__ Ve
 
 // --- the whole ordering work of a batch of up to kGroupMax packets in one launch --------
 // The same stable radix sort, the counters or the replay window behind it and the last checks behind that, by one
-// cluster of up to 8 CTAs of 512 threads with 1 to 8 packets a thread.  As kernels in stream order this is up to
+// cluster of up to 16 CTAs of 512 threads with 1 to 4 packets a thread.  As kernels in stream order this is up to
 // twenty launches of a few microseconds' work each, and a batch of a few thousand packets spent more time in front of
 // and between them than in them (a 4096-packet open with every check: 20 launches).  Keys and indices ping-pong
 // between shared-memory buffers; the CTAs read each other's digit totals, and the scatter writes into the buffer of
 // the CTA that a position belongs to, through distributed shared memory; cluster barriers stand where kernel
 // boundaries stood.  Up to 256 packets the sort is a count: the place of a packet is the number of packets with a
 // lower key, or the same key and a lower index.
-constexpr uint32_t kGroupThreads = 512, kGroupWarps = kGroupThreads / 32, kGroupCtas = 8;
-static_assert(kGroupMax == kGroupThreads * 8 * kGroupCtas, "8 packets a thread at most");
+constexpr uint32_t kGroupThreads = 512, kGroupWarps = kGroupThreads / 32, kGroupCtas = 16;
+static_assert(kGroupMax == kGroupThreads * 4 * kGroupCtas, "4 packets a thread at most");
 
 struct GroupArgs {
     SortKeySrc src;
@@ -875,6 +882,147 @@ __global__ void __launch_bounds__(kGroupThreads) group_kernel(const __grid_const
     signal_done(a.done, false, [] {});
 }
 
+// --- what follows the open kernel of up to kTailMax packets -----------------------------
+// Here nothing but latency counts, and group_kernel's phases hand each other their results through memory: 10 us for 9
+// packets, 36 for 129 with a hundred rules.  In this one CTA eight warps group the packets and run the replay window
+// in registers and shared memory, while the other eight already look the packets' flows and rules up; who judges a
+// packet then has everything in hand.
+constexpr uint32_t kTailMax = 256;
+struct HalfSync { // of the first 256 threads
+    __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+};
+__global__ void __launch_bounds__(512) open_tail_kernel(const __grid_constant__ ReplayArgs r, const uint32_t *slots,
+                                                        const __grid_constant__ VerdictArgs v, Done done) {
+    let_next_kernel_start();
+    wait_for_kernel_in_front();
+    __shared__ __align__(16) uint32_t key_of[kTailMax];
+    __shared__ uint32_t sorted_key[kTailMax];
+    __shared__ uint64_t sorted_ctr[kTailMax];
+    __shared__ uint8_t sorted_pkt[kTailMax], refused[kTailMax];
+    __shared__ SegMax part[8];
+    const uint32_t tid = threadIdx.x, n = v.n;
+    if (tid < kTailMax) { // ---- the replay window; the steps and their reasons are those of replay_*_kernel ----
+        const HalfSync half_sync;
+        const uint32_t lane = tid & 31;
+        uint32_t key = 0xffffffffu;
+        uint64_t c = kReplayNoPart;
+        bool beyond = false; // authenticated, at or beyond the message limit
+        if (tid < n) {
+            const uint32_t slot = slots[tid];
+            const uint8_t st = *(const volatile uint8_t *)&v.status[tid];
+            const uint64_t ctr = r.counter[tid];
+            key = min(slot, r.max_slots);
+            if (key < r.max_slots && (st == BNK_PKT_OK || st == BNK_PKT_KEEPALIVE)) {
+                beyond = ctr >= BNK_REJECT_AFTER_MESSAGES;
+                if (!beyond) c = ctr;
+            }
+        }
+        key_of[tid] = key;
+        refused[tid] = beyond;
+        half_sync();
+        uint32_t place = 0; // packets with a lower key, or the same key and a lower index
+        for (uint32_t j = 0; j < n; j += 4) {
+            const uint4 other = *reinterpret_cast<const uint4 *>(&key_of[j]);
+            place += (other.x < key + (j < tid)) + (other.y < key + (j + 1 < tid)) + (other.z < key + (j + 2 < tid)) + (other.w < key + (j + 3 < tid));
+        }
+        if (tid < n) {
+            sorted_key[place] = key;
+            sorted_ctr[place] = c;
+            sorted_pkt[place] = (uint8_t)tid;
+        }
+        half_sync();
+        const bool real = tid < n && sorted_key[tid] < r.max_slots; // from here on tid is a grouped position
+        const uint32_t slot = real ? sorted_key[tid] : 0u;
+        const bool head = tid < n && (tid == 0 || sorted_key[tid - 1] != sorted_key[tid]);
+        const bool tail = real && (tid + 1 == n || sorted_key[tid + 1] != slot);
+        c = real ? sorted_ctr[tid] : kReplayNoPart;
+        const uint64_t rmask = r.ring_blocks - 1, window = (uint64_t)(r.ring_blocks - 1) * 64u;
+        uint64_t *const ring = r.replay_ring + (size_t)slot * r.ring_blocks;
+        const uint64_t last = real ? r.replay_last[slot] : 0;
+        const uint64_t word = c != kReplayNoPart ? ring[(c >> 6) & rmask] : 0;
+        SegMax mine{head, c != kReplayNoPart ? c : 0ull}, total;
+        const SegMax ex = seg_block_exclusive<8>(mine, part, total, half_sync);
+        const uint64_t e = head ? 0ull : ex.m, M = e > last ? e : last;
+        uint8_t st = RP_NOPART;
+        uint64_t top = M;
+        if (c != kReplayNoPart) {
+            if (c > M) {
+                st = RP_ACCEPT;
+                top = c;
+            } else if (M - c > window || (c <= last && ((word >> (c & 63u)) & 1ull))) {
+                st = RP_REJECT;
+            } else { // accepted unless an earlier packet of the run has the same counter
+                st = RP_ACCEPT;
+                for (uint32_t q = tid; q-- > 0 && sorted_key[q] == slot;)
+                    if (sorted_ctr[q] == c) {
+                        st = RP_REJECT;
+                        break;
+                    }
+            }
+        }
+        half_sync(); // `last` and the ring are read: the peers whose run ends here move their window
+        uint32_t tails = __ballot_sync(0xffffffffu, tail && top != last);
+        while (tails) {
+            const uint32_t src = __ffs(tails) - 1;
+            tails &= tails - 1;
+            const uint32_t s = __shfl_sync(0xffffffffu, slot, src);
+            const uint64_t from = __shfl_sync(0xffffffffu, last, src) >> 6, to = __shfl_sync(0xffffffffu, top, src) >> 6;
+            const uint64_t steps = to - from < r.ring_blocks ? to - from : r.ring_blocks;
+            for (uint64_t i = lane; i < steps; i += 32) r.replay_ring[(size_t)s * r.ring_blocks + ((from + 1 + i) & rmask)] = 0ull;
+        }
+        if (tail) r.replay_last[slot] = top;
+        half_sync(); // clears before marks
+        replay_mark_warp(r, st == RP_ACCEPT, slot, c);
+        if (st == RP_REJECT) refused[sorted_pkt[tid]] = 1;
+        __syncthreads();
+    } else { // ---- the last checks of packet i ----
+        const uint32_t i = tid - kTailMax;
+        uint8_t st = BNK_PKT_BAD_DESC, found = BNK_PKT_OK; // found: what checks that leave no trace say of it
+        uint32_t l = 0, len = 0;
+        bool ask_flows = false;
+        FlowReply reply;
+        uint8_t proto = 0;
+        if (i < n) {
+            st = *(const volatile uint8_t *)&v.status[i];
+            l = len = v.out_len[i];
+            if (st == BNK_PKT_OK && (v.inner_check || v.check_inbound)) {
+                const uint4 h = v.inner[i];
+                proto = (uint8_t)h.z;
+                if (v.check_inbound && v.ft.enforce) {
+                    if (h.z & kInnerParses) {
+                        const Parsed p = inner_parsed(h);
+                        reply.begin(v.ft, p);
+                        ask_flows = !rules_allow(v.ft, p);
+                    } else {
+                        found = BNK_PKT_FILTER_DENY;
+                    }
+                }
+                if (v.inner_check) { // cut to the IPv4 total length; the source must be the peer's address
+                    if ((h.z & kInnerWhole) && h.x != 0 && h.x == v.allowed_ip[slots[i]]) len = h.w;
+                    else found = BNK_PKT_BAD_INNER;
+                }
+            }
+        }
+        __syncthreads();
+        if (i < n) {
+            uint8_t out = st;
+            if (refused[i]) {
+                out = BNK_PKT_REPLAY;
+                len = l;
+            } else if (st == BNK_PKT_OK) {
+                out = found == BNK_PKT_OK && ask_flows ? reply.finish(v.ft, proto, v.now) : found;
+            }
+            v.status[i] = out;
+            v.out_len[i] = len;
+            if (v.host_status) {
+                v.host_status[i] = out;
+                v.host_out_len[i] = len;
+            }
+        }
+    }
+    signal_done(done, false, [] {});
+}
+
 // --- scheduling order by length class (mixed packet sizes) ------------------------------
 // Packets with the same number of 64-byte cipher blocks end up next to each other so that
 // the lanes of a seal/open warp finish together; classes in falling order of length.  Order inside a class does
@@ -1025,15 +1173,16 @@ cudaError_t launch_group_items(const GroupArgs &a, uint32_t ctas, cudaStream_t s
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, group_kernel<ITEMS>, a);
 }
-// One CTA up to 1024 packets, then as many as keep two packets a thread, up to the eight of a portable cluster.
+// One CTA up to 1024 packets (its barriers are cheaper than a cluster's: 600 opened in 37 us against 41), then as many as
+// give every packet a thread, up to the 16 a cluster can have here (eight CTAs of two packets a thread and more: 2048
+// opened in 54 us against 46, 4096 in 74 against 65, 32,768 in 259 against 243).
 cudaError_t launch_group(const GroupArgs &a, cudaStream_t s) {
     uint32_t ctas = 1;
-    while (ctas < kGroupCtas && a.n > ctas * 2 * kGroupThreads) ctas *= 2;
+    while (ctas < kGroupCtas && a.n > std::max(ctas, 2u / ctas) * kGroupThreads) ctas *= 2;
     const uint32_t per_thread = (a.n + ctas * kGroupThreads - 1) / (ctas * kGroupThreads);
     if (per_thread <= 1) return launch_group_items<1>(a, ctas, s);
     if (per_thread <= 2) return launch_group_items<2>(a, ctas, s);
-    if (per_thread <= 4) return launch_group_items<4>(a, ctas, s);
-    return launch_group_items<8>(a, ctas, s);
+    return launch_group_items<4>(a, ctas, s);
 }
 cudaError_t launch_counters(bnk_ctx *ctx, const uint32_t *slot, uint32_t n, uint64_t *counter, cudaStream_t s) {
     const uint32_t max_slots = ctx->cfg.max_keypairs;
@@ -1054,7 +1203,9 @@ cudaError_t launch_counters(bnk_ctx *ctx, const uint32_t *slot, uint32_t n, uint
 
 cudaError_t group_kernels_init() {
     cudaError_t e = cudaFuncSetAttribute(group_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)group_smem(4));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(group_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)group_smem(8));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(group_kernel<1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(group_kernel<2>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(group_kernel<4>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
 
@@ -1126,6 +1277,15 @@ cudaError_t launch_open_tail(bnk_batch *b, uint32_t n, bool replay, const Verdic
     bnk_ctx *ctx = b->ctx;
     DeviceBatch &d = b->dev;
     if (!replay) return launch_verdict(ctx, *verdict, done, s);
+    if (n <= kTailMax) {
+        VerdictArgs v{};
+        if (verdict) v = *verdict;
+        v.status = d.status;
+        v.out_len = d.out_len;
+        v.n = n;
+        ctx->launches += 1;
+        return launch_after_kernel(open_tail_kernel, dim3(1), dim3(512), s, replay_args(b, n), d.slot, v, done);
+    }
     const SortPlan plan = plan_for(ctx->cfg.max_keypairs);
     GroupArgs g{};
     g.src = SortKeySrc{d.slot, ctx->cfg.max_keypairs};
