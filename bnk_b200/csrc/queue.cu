@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "bnk_internal.cuh"
+#include "packet_copy.h"
 #include "submit_order.h"
 
 namespace {
@@ -408,6 +409,7 @@ int bnk_queue_submit(bnk_queue *q, const uint8_t *const *pkts, const uint32_t *l
         v.off[at] = at * q->slot_bytes;
         v.len[at] = len[k];
         v.slot[at] = slot ? slot[k] : 0u;
+        if (k + 1 < n) copy_comes_next(pkts[k + 1], v.ring + (size_t)(at + 1) * q->slot_bytes + head, len[k + 1]);
         if (len[k]) memcpy(v.ring + (size_t)at * q->slot_bytes + head, pkts[k], len[k]);
     }
     g->filled.fetch_add(n, std::memory_order_release);
@@ -435,6 +437,7 @@ int bnk_queue_wait(bnk_queue *q, bnk_ticket ticket, uint8_t *const *out, uint32_
         out_len[k] = pass ? v.out_len[at] : 0u;
         if (counter) counter[k] = v.counter[at];
         if (slot_out) slot_out[k] = v.slot[at];
+        if (k + 1 < n) copy_comes_next(v.ring + (size_t)(at + 1) * q->slot_bytes, out[k + 1], v.out_len[at + 1]);
         if (out_len[k]) memcpy(out[k], v.ring + (size_t)at * q->slot_bytes + (open_side ? 16u : 0u), out_len[k]);
     }
     release(q, &g);
