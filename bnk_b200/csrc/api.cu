@@ -47,12 +47,38 @@ inline void cpu_relax() {
 
 bool is_pow2(uint64_t v) { return v && !(v & (v - 1)); }
 
-template <typename T>
-cudaError_t dev_alloc_zero(T **p, size_t count) {
-    cudaError_t e = cudaMalloc(p, count * sizeof(T));
-    if (e != cudaSuccess) return e;
-    return cudaMemset(*p, 0, count * sizeof(T));
-}
+// Several zeroed arrays, the first at the beginning, in one allocation: a cudaMalloc or cudaHostAlloc costs tens to
+// hundreds of microseconds however little it allocates, and a program pays that for every batch and context it makes.
+class Slab {
+  public:
+    template <typename T>
+    void add(T **p, size_t count) {
+        parts_.push_back({reinterpret_cast<void **>(p), total_});
+        total_ += (count * sizeof(T) + 255) & ~(size_t)255;
+    }
+    cudaError_t device() {
+        void *base = nullptr;
+        const cudaError_t e = cudaMalloc(&base, total_);
+        if (e != cudaSuccess) return e;
+        place(base);
+        return cudaMemset(base, 0, total_);
+    }
+    cudaError_t pinned() {
+        void *base = nullptr;
+        const cudaError_t e = cudaHostAlloc(&base, total_, cudaHostAllocDefault);
+        if (e != cudaSuccess) return e;
+        place(base);
+        memset(base, 0, total_);
+        return cudaSuccess;
+    }
+
+  private:
+    void place(void *base) {
+        for (const auto &part : parts_) *part.first = static_cast<uint8_t *>(base) + part.second;
+    }
+    std::vector<std::pair<void **, size_t>> parts_;
+    size_t total_ = 0;
+};
 
 // highest ring byte any of the first n packets can touch (input or output side); their bytes; whether they lie in the
 // ring in order, each with `room` bytes of its own behind it
@@ -379,15 +405,18 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     if (e != cudaSuccess) return fail(nullptr, BNK_ECUDA, "no usable CUDA device (there is no CPU fallback)", e);
     if (cfg->device_id < 0 || cfg->device_id >= ndev) return fail(nullptr, BNK_EINVAL, "device_id out of range");
     CK(nullptr, cudaSetDevice(cfg->device_id));
-    cudaDeviceProp prop;
-    CK(nullptr, cudaGetDeviceProperties(&prop, cfg->device_id));
-    if (prop.major != 10) return fail(nullptr, BNK_ECUDA, "device is not sm_100: this library carries sm_100a code only");
+    int major = 0, sms = 0, one_address = 0, maps_host = 0; // (the whole property record takes a millisecond to put together)
+    CK(nullptr, cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, cfg->device_id));
+    CK(nullptr, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device_id));
+    CK(nullptr, cudaDeviceGetAttribute(&one_address, cudaDevAttrUnifiedAddressing, cfg->device_id));
+    CK(nullptr, cudaDeviceGetAttribute(&maps_host, cudaDevAttrCanMapHostMemory, cfg->device_id));
+    if (major != 10) return fail(nullptr, BNK_ECUDA, "device is not sm_100: this library carries sm_100a code only");
 
     bnk_ctx *ctx = new (std::nothrow) bnk_ctx();
     if (!ctx) return fail(nullptr, BNK_ENOMEM, "host allocation failed");
     ctx->cfg = *cfg;
     ctx->device = cfg->device_id;
-    ctx->sm_count = prop.multiProcessorCount;
+    ctx->sm_count = sms;
     ctx->launches = 0;
     ctx->aead_mode = 0;
     if (const char *m = getenv("BNK_AEAD_KERNEL")) // tuning and test aid: tpp | wpp
@@ -395,7 +424,7 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     ctx->host_direct_bytes = 512u << 20;
     if (const char *m = getenv("BNK_HOST_DIRECT_BYTES")) // largest ring extent served without copies; 0 = never
         ctx->host_direct_bytes = strtoull(m, nullptr, 0);
-    if (!prop.unifiedAddressing || !prop.canMapHostMemory) ctx->host_direct_bytes = 0; // pinned memory must have one address
+    if (!one_address || !maps_host) ctx->host_direct_bytes = 0; // pinned memory must have one address
     ctx->pieces_from = 24u << 20;
     if (const char *m = getenv("BNK_PIECES_FROM")) // tuning aid: ring extent from which a batch that is alone goes in pieces
         ctx->pieces_from = strtoull(m, nullptr, 0);
@@ -414,15 +443,16 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     };
     if ((e = cudaStreamCreateWithFlags(&ctx->admin_stream, cudaStreamNonBlocking)) != cudaSuccess) return bail("stream", e);
     if ((e = cudaEventCreate(&ctx->timer_start)) != cudaSuccess) return bail("event", e);
-    if ((e = dev_alloc_zero(&ctx->kt.send_keys, k * 8)) != cudaSuccess) return bail("send_keys", e);
-    if ((e = dev_alloc_zero(&ctx->kt.recv_keys, k * 8)) != cudaSuccess) return bail("recv_keys", e);
-    if ((e = dev_alloc_zero(&ctx->kt.remote_index, k)) != cudaSuccess) return bail("remote_index", e);
-    if ((e = dev_alloc_zero(&ctx->kt.send_counter, k)) != cudaSuccess) return bail("send_counter", e);
-    if ((e = dev_alloc_zero(&ctx->kt.replay_last, k)) != cudaSuccess) return bail("replay_last", e);
-    if ((e = dev_alloc_zero(&ctx->kt.replay_next, k)) != cudaSuccess) return bail("replay_next", e);
-    if ((e = dev_alloc_zero(&ctx->kt.replay_ring, k * cfg->replay_ring_blocks)) != cudaSuccess) return bail("replay_ring", e);
-    if ((e = dev_alloc_zero(&ctx->kt.allowed_ip, k)) != cudaSuccess) return bail("allowed_ip", e);
-    if ((e = dev_alloc_zero(&ctx->kt.valid, k)) != cudaSuccess) return bail("valid", e);
+    Slab tables;
+    tables.add(&ctx->kt.send_keys, k * 8);
+    tables.add(&ctx->kt.recv_keys, k * 8);
+    tables.add(&ctx->kt.remote_index, k);
+    tables.add(&ctx->kt.send_counter, k);
+    tables.add(&ctx->kt.replay_last, k);
+    tables.add(&ctx->kt.replay_next, k);
+    tables.add(&ctx->kt.replay_ring, k * cfg->replay_ring_blocks);
+    tables.add(&ctx->kt.allowed_ip, k);
+    tables.add(&ctx->kt.valid, k);
     uint32_t islots = 16;
     while (islots < 2 * k) islots <<= 1;
     ctx->kt.index_slots = islots;
@@ -431,11 +461,12 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     ctx->index_live = ctx->index_dead = ctx->addr_live = ctx->addr_dead = 0;
     for (auto &h : ctx->flow_dead_hint) h = 0;
     ctx->flow_errors_seen = 0;
-    if ((e = dev_alloc_zero(&ctx->kt.index_keys, (size_t)islots)) != cudaSuccess) return bail("index_keys", e);
-    if ((e = dev_alloc_zero(&ctx->kt.index_vals, (size_t)islots)) != cudaSuccess) return bail("index_vals", e);
+    tables.add(&ctx->kt.index_keys, (size_t)islots);
+    tables.add(&ctx->kt.index_vals, (size_t)islots);
     ctx->kt.addr_slots = islots;
     ctx->addr_host.assign(islots, KeypairTables::AddrEntry{});
-    if ((e = dev_alloc_zero(&ctx->kt.addr_tab, (size_t)islots)) != cudaSuccess) return bail("addr_tab", e);
+    tables.add(&ctx->kt.addr_tab, (size_t)islots);
+    if ((e = tables.device()) != cudaSuccess) return bail("keypair tables", e);
     if ((e = group_kernels_init()) != cudaSuccess) return bail("kernel attributes", e);
     if ((e = filter_tables_alloc(ctx)) != cudaSuccess) return bail("filter tables", e);
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) return bail("sync", e);
@@ -447,18 +478,7 @@ int bnk_ctx_destroy(bnk_ctx *ctx) {
     if (!ctx) return BNK_EINVAL;
     cudaSetDevice(ctx->device);
     cudaDeviceSynchronize();
-    cudaFree(ctx->kt.send_keys);
-    cudaFree(ctx->kt.recv_keys);
-    cudaFree(ctx->kt.remote_index);
-    cudaFree(ctx->kt.send_counter);
-    cudaFree(ctx->kt.replay_last);
-    cudaFree(ctx->kt.replay_next);
-    cudaFree(ctx->kt.replay_ring);
-    cudaFree(ctx->kt.allowed_ip);
-    cudaFree(ctx->kt.valid);
-    cudaFree(ctx->kt.index_keys);
-    cudaFree(ctx->kt.index_vals);
-    cudaFree(ctx->kt.addr_tab);
+    cudaFree(ctx->kt.send_keys); // all of the tables' arrays
     filter_tables_free(ctx);
     if (ctx->timer_start) cudaEventDestroy(ctx->timer_start);
     if (ctx->admin_stream) cudaStreamDestroy(ctx->admin_stream);
@@ -800,31 +820,8 @@ int bnk_batch_destroy(bnk_batch *b) {
     }
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->direct_stream) cudaStreamSynchronize(b->direct_stream);
-    cudaFreeHost(b->host.src_addr);
-    cudaFreeHost(b->h_desc);
-    cudaFree(b->d_desc);
-    cudaFreeHost(b->h_flow);
-    cudaFreeHost(b->h_stats);
-    cudaFree(b->d_stats);
-    cudaFreeHost(b->h_gso);
-    cudaFreeHost(b->h_done);
-    cudaFree(b->d_ticket);
-    DeviceBatch &d = b->dev;
-    cudaFree(d.src_addr);
-    cudaFree(d.order);
-    cudaFree(d.order_tmp);
-    cudaFree(d.keys_tmp);
-    cudaFree(d.sorted_counter);
-    cudaFree(d.replay_state);
-    cudaFree(d.replay_hash);
-    cudaFree(d.replay_tile_head);
-    cudaFree(d.replay_tile_max);
-    cudaFree(d.replay_tile_carry);
-    cudaFree(d.hist);
-    cudaFree(d.len_order);
-    cudaFree(d.inner);
-    cudaFree(d.counters32);
-    cudaFree(d.gso);
+    cudaFreeHost(b->h_desc); // all of the pinned arrays
+    cudaFree(b->d_desc);     // all of the device's
     if (b->k_begin) cudaEventDestroy(b->k_begin);
     if (b->k_end) cudaEventDestroy(b->k_end);
     if (b->a_begin) cudaEventDestroy(b->a_begin);
@@ -860,67 +857,57 @@ int bnk_batch_create(bnk_ctx *ctx, uint32_t max_pkts, uint64_t ring_bytes, bnk_b
     b->ring_bytes = ring_bytes;
     const size_t n = max_pkts;
     cudaError_t e = cudaSuccess;
-    auto H = [&](void **p, size_t bytes) {
-        if (e == cudaSuccess) e = cudaHostAlloc(p, bytes, cudaHostAllocDefault);
-        if (e == cudaSuccess) memset(*p, 0, bytes);
-    };
-    auto D = [&](void **p, size_t bytes) {
-        if (e == cudaSuccess) e = cudaMalloc(p, bytes);
-        if (e == cudaSuccess) e = cudaMemset(*p, 0, bytes);
-    };
     // One slab per side: the descriptor arrays, then the ring.  A batch whose descriptor slab is small moves
     // descriptors and ring with one copy each way (joint_copy); otherwise the descriptor fields a call needs
-    // move as one run or field by field (desc_copy).
+    // move as one run or field by field (desc_copy).  What else the batch needs lies behind.
     b->npad = (max_pkts + 15u) & ~15u;
     const size_t np = b->npad;
     b->desc_room = (25 * np + 255) & ~(size_t)255;
     b->joint_copy = b->desc_room <= 64u * 1024;
     if (!b->joint_copy) b->desc_room = (b->desc_room + 4095) & ~(size_t)4095; // the ring then starts on a page: see Pieces
-    H((void **)&b->h_desc, b->desc_room + ring_bytes);
+    DeviceBatch &d = b->dev;
+    Slab pinned, device;
+    pinned.add(&b->h_desc, b->desc_room + ring_bytes);
+    pinned.add(&b->host.src_addr, n * BNK_SRC_ADDR_STRIDE);
+    pinned.add(&b->h_gso, n);
+    pinned.add(&b->h_flow, 1);
+    pinned.add(&b->h_stats, 1);
+    pinned.add(&b->h_done, 32);
+    e = pinned.pinned();
+    device.add(&b->d_desc, b->desc_room + ring_bytes);
+    device.add(&d.src_addr, n * BNK_SRC_ADDR_STRIDE);
+    device.add(&d.order, n);
+    device.add(&d.order_tmp, n);
+    device.add(&d.keys_tmp, 2 * n);
+    device.add(&d.sorted_counter, n);
+    device.add(&d.replay_state, n);
+    device.add(&d.replay_hash, replay_hash_capacity(max_pkts));
+    device.add(&d.replay_tile_head, (size_t)replay_scan_tiles(max_pkts) + 1);
+    device.add(&d.replay_tile_max, replay_scan_tiles(max_pkts));
+    device.add(&d.replay_tile_carry, replay_scan_tiles(max_pkts));
+    device.add(&d.hist, (size_t)512 * group_sort_chunks(max_pkts)); // histogram columns + one row of totals
+    device.add(&d.len_order, n);
+    device.add(&d.inner, n);
+    device.add(&d.counters32, 2048);
+    device.add(&d.gso, n);
+    device.add(&b->d_ticket, 32);
+    device.add(&b->d_stats, 20);
+    if (e == cudaSuccess) e = device.device();
     if (e == cudaSuccess) {
-        b->host.ring = b->h_desc + b->desc_room;
-        b->host.off = reinterpret_cast<uint32_t *>(b->h_desc);
-        b->host.len = reinterpret_cast<uint32_t *>(b->h_desc + 4 * np);
-        b->host.slot = reinterpret_cast<uint32_t *>(b->h_desc + 8 * np);
-        b->host.counter = reinterpret_cast<uint64_t *>(b->h_desc + 12 * np);
-        b->host.out_len = reinterpret_cast<uint32_t *>(b->h_desc + 20 * np);
-        b->host.status = b->h_desc + 24 * np;
+        auto fields = [&](uint8_t *p, auto &v) {
+            v.ring = p + b->desc_room;
+            v.off = reinterpret_cast<uint32_t *>(p);
+            v.len = reinterpret_cast<uint32_t *>(p + 4 * np);
+            v.slot = reinterpret_cast<uint32_t *>(p + 8 * np);
+            v.counter = reinterpret_cast<uint64_t *>(p + 12 * np);
+            v.out_len = reinterpret_cast<uint32_t *>(p + 20 * np);
+            v.status = p + 24 * np;
+        };
+        fields(b->h_desc, b->host);
+        fields(b->d_desc, d);
     }
-    H((void **)&b->host.src_addr, n * BNK_SRC_ADDR_STRIDE);
-    H((void **)&b->h_flow, sizeof(FlowReport));
-    H((void **)&b->h_stats, sizeof(bnk_batch_stats));
-    H((void **)&b->h_gso, n * sizeof(bnk_gso_super));
-    H((void **)&b->h_done, 128);
     b->host.ring_bytes = ring_bytes;
     b->host.max_pkts = max_pkts;
-    DeviceBatch &d = b->dev;
-    D((void **)&b->d_desc, b->desc_room + ring_bytes);
-    if (e == cudaSuccess) {
-        d.ring = b->d_desc + b->desc_room;
-        d.off = reinterpret_cast<uint32_t *>(b->d_desc);
-        d.len = reinterpret_cast<uint32_t *>(b->d_desc + 4 * np);
-        d.slot = reinterpret_cast<uint32_t *>(b->d_desc + 8 * np);
-        d.counter = reinterpret_cast<uint64_t *>(b->d_desc + 12 * np);
-        d.out_len = reinterpret_cast<uint32_t *>(b->d_desc + 20 * np);
-        d.status = b->d_desc + 24 * np;
-    }
-    D((void **)&d.src_addr, n * BNK_SRC_ADDR_STRIDE);
-    D((void **)&d.order, n * 4);
-    D((void **)&d.order_tmp, n * 4);
-    D((void **)&d.keys_tmp, 2 * n * 4);
-    D((void **)&d.sorted_counter, n * 8);
-    D((void **)&d.replay_state, n);
-    D((void **)&d.replay_hash, (size_t)replay_hash_capacity(max_pkts) * 4);
-    D((void **)&d.replay_tile_head, ((size_t)replay_scan_tiles(max_pkts) + 1) * 4);
-    D((void **)&d.replay_tile_max, (size_t)replay_scan_tiles(max_pkts) * 8);
-    D((void **)&d.replay_tile_carry, (size_t)replay_scan_tiles(max_pkts) * 8);
-    D((void **)&d.hist, (size_t)512 * group_sort_chunks(max_pkts) * 4); // histogram columns + one row of totals
-    D((void **)&d.len_order, n * 4);
-    D((void **)&d.inner, n * sizeof(uint4));
-    D((void **)&d.counters32, 2048 * 4);
-    D((void **)&d.gso, n * sizeof(bnk_gso_super));
-    D((void **)&b->d_ticket, 128);
-    D((void **)&b->d_stats, 20 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->stream, cudaStreamNonBlocking, ctx->prio_high);
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->aux_stream, cudaStreamNonBlocking, ctx->prio_high);
     if (e == cudaSuccess && ctx->aead_side_stream_from && max_pkts >= ctx->aead_side_stream_from && ctx->prio_low != ctx->prio_high) {

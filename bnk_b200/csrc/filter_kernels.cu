@@ -281,13 +281,16 @@ cudaError_t filter_tables_alloc(bnk_ctx *ctx) {
     const uint32_t cap = ctx->cfg.flow_capacity;
     ft.flow_capacity = cap;
     cudaError_t e;
-    FlowCtl *ctl = nullptr;
-    if ((e = cudaMalloc(&ctl, sizeof(FlowCtl))) != cudaSuccess) return e;
-    ft.flow_live = reinterpret_cast<unsigned long long *>(ctl);
-    if ((e = cudaMalloc(&ft.flow_special_exp, 3 * sizeof(long long))) != cudaSuccess) return e;
+    // one block: control block, special entries, keys, expiries
+    const size_t head = 512, keys = (size_t)6 * cap * sizeof(uint64_t);
+    static_assert(sizeof(FlowCtl) <= 256, "control block");
+    uint8_t *mem = nullptr;
+    if ((e = cudaMalloc(&mem, head + 2 * keys)) != cudaSuccess) return e;
+    ft.flow_live = reinterpret_cast<unsigned long long *>(mem);
+    ft.flow_special_exp = reinterpret_cast<long long *>(mem + 256);
     if (cap) {
-        if ((e = cudaMalloc(&ft.flow_keys, (size_t)6 * cap * sizeof(uint64_t))) != cudaSuccess) return e;
-        if ((e = cudaMalloc(&ft.flow_exp, (size_t)6 * cap * sizeof(long long))) != cudaSuccess) return e;
+        ft.flow_keys = reinterpret_cast<uint64_t *>(mem + head);
+        ft.flow_exp = reinterpret_cast<long long *>(mem + head + keys);
     }
     // With a stated rule-table capacity both buffer sets are allocated here, and a rule swap allocates nothing.
     if (const size_t cap_t = ctx->cfg.max_acl_tuples) {
@@ -302,10 +305,7 @@ cudaError_t filter_tables_alloc(bnk_ctx *ctx) {
 
 void filter_tables_free(bnk_ctx *ctx) {
     FilterTables &ft = ctx->ft;
-    cudaFree(ft.flow_live);
-    cudaFree(ft.flow_special_exp);
-    cudaFree(ft.flow_keys);
-    cudaFree(ft.flow_exp);
+    cudaFree(ft.flow_live); // the block's beginning
     for (bnk_ctx::RuleSet &rs : ctx->rule_set) {
         cudaFree(rs.mem);
         for (cudaEvent_t ev : rs.in_use) cudaEventDestroy(ev);
