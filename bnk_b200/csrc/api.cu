@@ -171,9 +171,12 @@ bool heads_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, uint64_t ext) {
 }
 // A large batch that is alone in flight goes over the link in pieces: while one is worked on, the next comes up and the
 // one before goes down, so both copy engines are busy.  Pieces end on pages of the ring (a copy that starts elsewhere is
-// up to a sixth slower: 190 MB up and down in 8 MB pieces 4.1 ms against 4.9), at most kPieceMost bytes each, with small
-// ones first and last, when one direction has nothing to do yet or any more.  Packets have to lie in the ring in order.
-constexpr uint64_t kPieceLeast = 1ull << 20, kPieceMost = 8ull << 20, kPage = 4096;
+// up to a sixth slower: 190 MB up and down in 8 MB pieces 4.1 ms against 4.9), with small ones first and last, when one
+// direction has nothing to do yet or any more.  Between two copies an engine rests ~15 us while the other direction is
+// busy, so the pieces in the middle of a large ring are large: 190 MB sealed in pieces of at most 8 MB 5.0 ms, 16 MB 4.74,
+// 24 MB 4.70, but 47 MB in at most 8 MB 1.35 ms, 24 MB 1.39.  Two streams for each direction share its engine's rate and
+// finish later (5.7 ms).  Packets have to lie in the ring in order.
+constexpr uint64_t kPieceLeast = 1ull << 20, kPieceMost = 8ull << 20, kPieceMostEver = 24ull << 20, kPage = 4096;
 struct Piece {
     uint32_t first, count;       // packets
     uint64_t up, up_to;          // ring bytes that come up in front of them
@@ -183,14 +186,15 @@ class Pieces {
   public:
     // `more`: a packet's kernel reads and writes at most len + more bytes from its offset on.  All of them have to be up: a
     // later copy must not run over what the kernel has written.
-    Pieces(const bnk_batch *b, uint32_t n, uint32_t more, uint64_t ext) : off_(b->host.off), len_(b->host.len), n_(n), more_(more), ext_(ext) {}
+    Pieces(const bnk_batch *b, uint32_t n, uint32_t more, uint64_t ext) : off_(b->host.off), len_(b->host.len), n_(n), more_(more), ext_(ext),
+          most_(std::min(std::max(kPieceMost, ext / 8), kPieceMostEver)) {}
     bool next(Piece &p) {
         if (at_ == n_) return false;
         p.first = at_;
         p.up = up_;
         p.down = down_;
         do { // a packet larger than a piece takes several
-            const uint64_t left = ext_ - up_, size = std::min(std::min(kPieceMost, up_ + kPieceLeast), std::max(kPieceLeast, left / 2));
+            const uint64_t left = ext_ - up_, size = std::min(std::min(most_, up_ + kPieceLeast), std::max(kPieceLeast, left / 2));
             up_ = left <= size + size / 2 ? ext_ : (up_ + size) & ~(kPage - 1);
             if (up_ == ext_) at_ = n_;
             while (at_ < n_ && (uint64_t)off_[at_] + more_ + len_[at_] <= up_) at_++;
@@ -205,7 +209,7 @@ class Pieces {
   private:
     const uint32_t *off_, *len_;
     uint32_t n_, more_, at_ = 0;
-    uint64_t ext_, up_ = 0, down_ = 0;
+    uint64_t ext_, most_, up_ = 0, down_ = 0;
 };
 // Below ctx->pieces_from (24 MB) a kernel on the pinned ring is as fast or faster, because the first piece up and the last
 // one down have no company: 16,384 x 1420 B 710 us against 750, 32,768 1390 against 1330, 131,072 5.74 ms against 4.96.
@@ -218,13 +222,12 @@ bool in_pieces(const bnk_batch *b, uint32_t n, uint32_t flags, uint64_t ext, boo
     return in_order && b->up_stream && !(flags & (BNK_F_NO_H2D | BNK_F_NO_D2H | BNK_F_USE_OUT_LEN)) &&
            b->ctx->in_flight.load(std::memory_order_relaxed) == (b->counted ? 1 : 0);
 }
-// Copies a piece up and lets stream s go on behind it / copies down what is done on s.
-cudaError_t piece_up(bnk_batch *b, const Piece &p, cudaStream_t s) {
-    cudaError_t e = cudaMemcpyAsync(b->dev.ring + p.up, b->host.ring + p.up, p.up_to - p.up, cudaMemcpyHostToDevice, b->up_stream);
-    if (e == cudaSuccess) e = cudaEventRecord(b->ev_up, b->up_stream);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b->ev_up, 0);
-    return e;
+// Copies a piece up (piece_is_up lets stream s go on behind it) / copies down what is done on s.
+cudaError_t piece_up(bnk_batch *b, const Piece &p) {
+    const cudaError_t e = cudaMemcpyAsync(b->dev.ring + p.up, b->host.ring + p.up, p.up_to - p.up, cudaMemcpyHostToDevice, b->up_stream);
+    return e != cudaSuccess ? e : cudaEventRecord(b->ev_up, b->up_stream);
 }
+cudaError_t piece_is_up(bnk_batch *b, cudaStream_t s) { return cudaStreamWaitEvent(s, b->ev_up, 0); }
 cudaError_t piece_down(bnk_batch *b, const Piece &p, cudaStream_t s) {
     if (p.down_to == p.down) return cudaSuccess;
     cudaError_t e = cudaEventRecord(b->ev_down, s);
@@ -1054,6 +1057,10 @@ static int seal_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
+    Pieces pieces(b, npkts, BNK_WG_HEADER + 16 + BNK_WG_TAG, ext);
+    Piece p;
+    pieces.next(p); // the first is on its way while the kernels in front of the first seal are prepared
+    CK(ctx, piece_up(b, p));
     CK(ctx, desc_copy(b, npkts, D_OFF, b->dev_stale ? D_STATUS : (flags & BNK_F_ASSIGN_COUNTERS) ? D_SLOT : D_COUNTER, true, s));
     b->dev_stale = b->ring_partial = false;
     CK(ctx, order_kernels_begin(b, s));
@@ -1065,12 +1072,13 @@ static int seal_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     const bool note = (flags & BNK_F_NOTE_OUTBOUND) && ctx->ft.enforce && ctx->ft.flow_capacity; // filter.go:192-194
     const bool sweep = note && flow_note_begins(b, npkts, now_unix_ns);
     if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
-    Piece p;
-    for (Pieces pieces(b, npkts, BNK_WG_HEADER + 16 + BNK_WG_TAG, ext); pieces.next(p);) {
-        CK(ctx, piece_up(b, p, s));
+    for (bool more = true; more;) {
+        CK(ctx, piece_is_up(b, s));
         if (note) CK(ctx, launch_filter_note(b, p.first, p.count, now_unix_ns, Done{}, s));
         CK(ctx, launch_seal(piece_args(a, p), s, ctx));
         CK(ctx, piece_down(b, p, s));
+        more = pieces.next(p);
+        if (more) CK(ctx, piece_up(b, p));
     }
     if (timed) CK(ctx, cudaEventRecord(b->a_end, s));
     if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, Done{}, s));
@@ -1249,6 +1257,10 @@ static int open_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0, demux = (flags & BNK_F_DEMUX_INDEX) != 0;
+    Pieces pieces(b, npkts, 0, ext);
+    Piece p;
+    pieces.next(p);
+    CK(ctx, piece_up(b, p));
     CK(ctx, desc_copy(b, npkts, D_OFF, b->dev_stale ? D_STATUS : demux ? D_LEN : D_SLOT, true, s));
     b->dev_stale = b->ring_partial = false;
     CK(ctx, order_kernels_begin(b, s));
@@ -1257,12 +1269,13 @@ static int open_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     a.behind_kernel = true;
     const bool replay = (flags & BNK_F_REPLAY) != 0, one_launch = npkts <= kGroupMax;
     if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
-    Piece p;
-    for (Pieces pieces(b, npkts, 0, ext); pieces.next(p);) {
-        CK(ctx, piece_up(b, p, s));
+    for (bool more = true; more;) {
+        CK(ctx, piece_is_up(b, s));
         if (demux) CK(ctx, launch_demux_index(b, p.first, p.count, a.len, s));
         CK(ctx, launch_open(piece_args(a, p), s, ctx));
         CK(ctx, piece_down(b, p, s)); // the checks below say which plaintexts count, and change no byte of them
+        more = pieces.next(p);
+        if (more) CK(ctx, piece_up(b, p));
     }
     if (timed) CK(ctx, cudaEventRecord(b->a_end, s));
     if (replay && one_launch) {
