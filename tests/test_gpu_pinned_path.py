@@ -197,7 +197,7 @@ def test_split_uploads_super_packets_only(gpu_lib, oracle, busy):
         other.wait()
 
 
-@pytest.mark.parametrize("n,sizes", [(4000, (1420, 1404, 1)), (12_000, (64, 300, 0)), (100, (65_000, 30_001, 9))])
+@pytest.mark.parametrize("n,sizes", [(4000, (1420, 1404, 1)), (12_000, (64, 300, 0)), (100, (65_000, 30_001, 9)), (2200, (65_000, 30_001, 9))])
 def test_large_batches_in_pieces(gpu_lib, oracle, n, sizes, monkeypatch):
     """A batch that goes over the link in pieces, packets across the pieces' ends among them, with every option that has
     its own part in the loop: bytes, statuses and flows are the checker's, and nothing beside the packets changes."""
