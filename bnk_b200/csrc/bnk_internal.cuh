@@ -66,6 +66,10 @@ struct alignas(16) RuleGroup {
 constexpr uint32_t kNoPorts = 0xffff0000u;
 
 // Flattened, indexed ACL and the reply-flow table (filter_kernels.cu).
+struct alignas(16) FlowSlot { // key and expiry side by side: a lookup's first probe is one 16-byte load
+    unsigned long long key; // FLOW_EMPTY = all ones
+    long long exp;          // in unix ns; FLOW_DEAD = deleted
+};
 struct FilterTables {
     // rule index (filter_device.cuh), one block of device memory
     const uint32_t *rule_top;    // [65536] by the upper 16 address bits; null when there are no rules
@@ -78,8 +82,7 @@ struct FilterTables {
     // flow table, one open-addressing region per protocol class (tcp, udp, icmp).  Every class has two
     // regions, [class][half][flow_capacity]; flow_half[class] says which one is in use, the other one is all
     // FLOW_EMPTY and receives the surviving entries when the class is compacted (filter_flows_compact).
-    uint64_t *flow_keys;   // [3][2][flow_capacity] FLOW_EMPTY = all ones
-    long long *flow_exp;   // [3][2][flow_capacity] expiry in unix ns; FLOW_DEAD = deleted
+    FlowSlot *flow_slots;   // [3][2][flow_capacity]
     uint32_t flow_capacity; // power of two
     uint8_t flow_half[3];
     unsigned long long *flow_live;  // device control block (FlowCtl): live entries (Go's len(f.flows)) and more

@@ -110,7 +110,7 @@ struct FlowNote {
         key = flow_key(p.dst, p.dport, p.sport);
         h = flow_hash(key) & (ft.flow_capacity - 1);
         if (key != FLOW_EMPTY)
-            old = atomicCAS((unsigned long long *)ft.flow_keys + flow_region(ft, cls) + h, FLOW_EMPTY, key);
+            old = atomicCAS(&ft.flow_slots[flow_region(ft, cls) + h].key, FLOW_EMPTY, key);
     }
     __device__ __forceinline__ void place(const FilterTables &ft) {
         if (cls < 0) return;
@@ -119,16 +119,16 @@ struct FlowNote {
             placed = true;
             return;
         }
-        unsigned long long *const keys = (unsigned long long *)ft.flow_keys + flow_region(ft, cls);
+        FlowSlot *const slots = ft.flow_slots + flow_region(ft, cls);
         for (uint32_t probe = 1; old != FLOW_EMPTY && old != key; probe++) {
             if (probe >= ft.flow_capacity) { // table full: the flow is not recorded, the host reports BNK_EFULL
                 atomicAdd(&flow_ctl(ft)->rep.error, 1);
                 return;
             }
             h = (h + 1) & (ft.flow_capacity - 1);
-            old = atomicCAS(&keys[h], FLOW_EMPTY, key);
+            old = atomicCAS(&slots[h].key, FLOW_EMPTY, key);
         }
-        prev = (long long)atomicExch((unsigned long long *)ft.flow_exp + flow_region(ft, cls) + h, (unsigned long long)exp);
+        prev = (long long)atomicExch((unsigned long long *)&slots[h].exp, (unsigned long long)exp);
         placed = true;
     }
     __device__ __forceinline__ void count(const FilterTables &ft) {
@@ -232,36 +232,36 @@ __device__ __forceinline__ bool rules_allow(const FilterTables &ft, const Parsed
 // In two steps, so that the first can wait for memory beside the search of the rules.
 struct FlowReply {
     unsigned long long key, k;
-    long long exp, floor, *exps;
+    long long exp, *place;
     uint32_t h;
     int cls;
 
     __device__ __forceinline__ void begin(const FilterTables &ft, const Parsed &p) {
         cls = proto_class(p.proto);
         key = flow_key(p.src, p.sport, p.dport);
-        exps = ft.flow_exp + flow_region(ft, cls);
         h = flow_hash(key) & (ft.flow_capacity - 1);
         k = FLOW_EMPTY;
         exp = FLOW_FRESH;
-        floor = flow_floor(flow_ctl(ft));
+        place = &ft.flow_special_exp[cls];
         if (ft.flow_capacity == 0) return;
         if (key == FLOW_EMPTY) {
-            exps = ft.flow_special_exp;
-            h = cls;
+            exp = *(volatile long long *)place;
         } else {
-            k = ((const volatile unsigned long long *)ft.flow_keys + flow_region(ft, cls))[h];
+            FlowSlot *const at = ft.flow_slots + flow_region(ft, cls) + h;
+            place = &at->exp;
+            asm volatile("ld.volatile.global.v2.b64 {%0, %1}, [%2];" : "=l"(k), "=l"(exp) : "l"(__cvta_generic_to_global(at)));
         }
-        exp = *(volatile long long *)&exps[h];
     }
     __device__ __forceinline__ uint8_t finish(const FilterTables &ft, uint8_t proto, long long now) {
         if (key != FLOW_EMPTY && k != key) {
-            const unsigned long long *const keys = (const unsigned long long *)ft.flow_keys + flow_region(ft, cls);
+            FlowSlot *const slots = ft.flow_slots + flow_region(ft, cls);
             exp = FLOW_FRESH;
             for (uint32_t probe = 1; k != FLOW_EMPTY && probe < ft.flow_capacity; probe++) {
                 h = (h + 1) & (ft.flow_capacity - 1);
-                k = keys[h];
+                k = slots[h].key;
                 if (k == key) {
-                    exp = *(volatile long long *)&exps[h];
+                    place = &slots[h].exp;
+                    exp = *(volatile long long *)place;
                     break;
                 }
             }
@@ -270,11 +270,12 @@ struct FlowReply {
         FlowCtl *const ctl = flow_ctl(ft);
         if (now < exp) { // strict: time.Before
             const long long fresh = now + flow_ttl(proto);
-            *(volatile long long *)&exps[h] = fresh; // keep-alive on traffic
-            flow_keep_floor(ctl, fresh, floor);
+            *(volatile long long *)place = fresh; // keep-alive on traffic
+            // The floor may come from L1, one word for all warps: a sweep that raises it meanwhile leaves it below `fresh`.
+            flow_keep_floor(ctl, fresh, ctl->rep.floor);
             return BNK_PKT_OK;
         }
-        const long long prev = (long long)atomicExch((unsigned long long *)&exps[h], (unsigned long long)FLOW_DEAD);
+        const long long prev = (long long)atomicExch((unsigned long long *)place, (unsigned long long)FLOW_DEAD);
         if (!flow_absent(prev)) {
             atomicAdd(&ctl->rep.live, 0ull - 1ull);
             if (key != FLOW_EMPTY) atomicAdd(&ctl->rep.dead[cls], 1u);

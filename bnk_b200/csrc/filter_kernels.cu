@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(128) filter_note_kernel(const __grid_constant_
 // (one `now`) that equals: insert everything, then sweep once if the count exceeds the threshold.  A sweep that
 // starts at or before the floor of the expiries would find nothing and does not walk the table; the host, which
 // knows a lower bound of the floor, does not even launch it (flow_note_begins).  One walk reads the expiries of the
-// regions in use (8 bytes a slot) and leaves the floor at the lowest expiry it has seen, or at what an insert that
+// regions in use and leaves the floor at the lowest expiry it has seen, or at what an insert that
 // ran beside it can have written.
 __global__ void __launch_bounds__(256) filter_sweep_kernel(const __grid_constant__ FilterTables ft, long long now, FlowReport *report, Done done) {
     let_next_kernel_start();
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(256) filter_sweep_kernel(const __grid_constant
         long long floor = LLONG_MAX;
         for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total + 3; k += (size_t)gridDim.x * blockDim.x) {
             const int cls = k < total ? (int)(k / cap) : 0;
-            long long *const e = k < total ? &ft.flow_exp[flow_region(ft, cls) + (k - cls * cap)] : &ft.flow_special_exp[k - total];
+            long long *const e = k < total ? &ft.flow_slots[flow_region(ft, cls) + (k - cls * cap)].exp : &ft.flow_special_exp[k - total];
             const long long exp = *e;
             if (flow_absent(exp)) continue;
             if (now > exp) {
@@ -158,8 +158,7 @@ __global__ void __launch_bounds__(128) filter_check_kernel(const __grid_constant
 __global__ void flows_fill_kernel(FilterTables ft) {
     const size_t total = (size_t)6 * ft.flow_capacity;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
-        ft.flow_keys[k] = FLOW_EMPTY;
-        ft.flow_exp[k] = FLOW_FRESH;
+        ft.flow_slots[k] = FlowSlot{FLOW_EMPTY, FLOW_FRESH};
     }
     if (blockIdx.x == 0 && threadIdx.x < 3) ft.flow_special_exp[threadIdx.x] = FLOW_FRESH;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -175,25 +174,23 @@ __global__ void flows_fill_kernel(FilterTables ft) {
 __global__ void flows_compact_kernel(FilterTables ft, int cls) {
     FlowCtl *ctl = flow_ctl(ft);
     const size_t from = flow_region(ft, cls), to = ((size_t)cls * 2 + (ft.flow_half[cls] ^ 1)) * ft.flow_capacity;
-    unsigned long long *keys = (unsigned long long *)ft.flow_keys + to;
-    long long *exps = ft.flow_exp + to;
+    FlowSlot *const slots = ft.flow_slots + to;
     uint32_t moved = 0;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < ft.flow_capacity; k += (size_t)gridDim.x * blockDim.x) {
-        const unsigned long long key = ft.flow_keys[from + k];
-        if (key == FLOW_EMPTY) continue;
-        const long long exp = ft.flow_exp[from + k];
-        if (flow_absent(exp)) continue;
+        const unsigned long long key = ft.flow_slots[from + k].key;
+        const long long exp = ft.flow_slots[from + k].exp;
+        if (key == FLOW_EMPTY || flow_absent(exp)) continue;
         uint32_t h = flow_hash(key) & (ft.flow_capacity - 1);
         bool placed = false; // the target region starts empty and takes fewer entries than it has slots
         for (uint32_t probe = 0; probe < ft.flow_capacity && !placed; probe++) {
-            if (atomicCAS(&keys[h], FLOW_EMPTY, key) == FLOW_EMPTY) placed = true;
+            if (atomicCAS(&slots[h].key, FLOW_EMPTY, key) == FLOW_EMPTY) placed = true;
             else h = (h + 1) & (ft.flow_capacity - 1);
         }
         if (!placed) {
             atomicAdd(&ctl->rep.error, 1);
             continue;
         }
-        exps[h] = exp;
+        slots[h].exp = exp;
         moved++;
     }
     if (moved) atomicAdd(&ctl->moved, moved);
@@ -203,8 +200,7 @@ __global__ void flows_compact_finish_kernel(FilterTables ft, int cls) {
     FlowCtl *ctl = flow_ctl(ft);
     const size_t from = flow_region(ft, cls);
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < ft.flow_capacity; k += (size_t)gridDim.x * blockDim.x) {
-        ft.flow_keys[from + k] = FLOW_EMPTY;
-        ft.flow_exp[from + k] = FLOW_FRESH;
+        ft.flow_slots[from + k] = FlowSlot{FLOW_EMPTY, FLOW_FRESH};
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         ctl->rep.used[cls] = ctl->moved; // the kernel in front has finished: the count is final
@@ -281,17 +277,14 @@ cudaError_t filter_tables_alloc(bnk_ctx *ctx) {
     const uint32_t cap = ctx->cfg.flow_capacity;
     ft.flow_capacity = cap;
     cudaError_t e;
-    // one block: control block, special entries, keys, expiries
-    const size_t head = 512, keys = (size_t)6 * cap * sizeof(uint64_t);
+    // one block: control block, special entries, slots
+    const size_t head = 512;
     static_assert(sizeof(FlowCtl) <= 256, "control block");
     uint8_t *mem = nullptr;
-    if ((e = cudaMalloc(&mem, head + 2 * keys)) != cudaSuccess) return e;
+    if ((e = cudaMalloc(&mem, head + (size_t)6 * cap * sizeof(FlowSlot))) != cudaSuccess) return e;
     ft.flow_live = reinterpret_cast<unsigned long long *>(mem);
     ft.flow_special_exp = reinterpret_cast<long long *>(mem + 256);
-    if (cap) {
-        ft.flow_keys = reinterpret_cast<uint64_t *>(mem + head);
-        ft.flow_exp = reinterpret_cast<long long *>(mem + head + keys);
-    }
+    if (cap) ft.flow_slots = reinterpret_cast<FlowSlot *>(mem + head);
     // With a stated rule-table capacity both buffer sets are allocated here, and a rule swap allocates nothing.
     if (const size_t cap_t = ctx->cfg.max_acl_tuples) {
         const size_t bytes = RuleLayout(std::min<size_t>(cap_t, 65536), rule_long_slots(cap_t), cap_t, 4 * cap_t).total;
@@ -347,21 +340,16 @@ cudaError_t filter_flow_stats(bnk_ctx *ctx, uint64_t *live, uint32_t used[3], ui
 // path, and the caller has quiesced the context.  The host applies the same hash and the same probing as the kernels.
 namespace {
 struct FlowTablesHost {
-    std::vector<unsigned long long> keys;
-    std::vector<long long> exp;
+    std::vector<FlowSlot> slots;
     long long special[3];
     FlowCtl ctl;
 };
 cudaError_t flows_download(bnk_ctx *ctx, FlowTablesHost &h) {
     const FilterTables &ft = ctx->ft;
     const size_t total = (size_t)6 * ft.flow_capacity;
-    h.keys.resize(total);
-    h.exp.resize(total);
+    h.slots.resize(total);
     cudaError_t e = cudaSuccess;
-    if (total) {
-        e = cudaMemcpy(h.keys.data(), ft.flow_keys, total * sizeof(uint64_t), cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(h.exp.data(), ft.flow_exp, total * sizeof(long long), cudaMemcpyDeviceToHost);
-    }
+    if (total) e = cudaMemcpy(h.slots.data(), ft.flow_slots, total * sizeof(FlowSlot), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(h.special, ft.flow_special_exp, sizeof h.special, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(&h.ctl, ft.flow_live, sizeof h.ctl, cudaMemcpyDeviceToHost);
     return e;
@@ -389,8 +377,10 @@ int filter_flows_export(bnk_ctx *ctx, bnk_flow_entry *out, size_t capacity, size
     };
     for (int cls = 0; cls < 3; cls++) {
         const size_t base = flow_region(ft, cls);
-        for (size_t k = 0; k < ft.flow_capacity; k++)
-            if (h.keys[base + k] != FLOW_EMPTY && !flow_absent(h.exp[base + k])) emit(cls, h.keys[base + k], h.exp[base + k]);
+        for (size_t k = 0; k < ft.flow_capacity; k++) {
+            const FlowSlot &v = h.slots[base + k];
+            if (v.key != FLOW_EMPTY && !flow_absent(v.exp)) emit(cls, v.key, v.exp);
+        }
         if (!flow_absent(h.special[cls])) emit(cls, FLOW_EMPTY, h.special[cls]);
     }
     *count = n;
@@ -418,13 +408,13 @@ int filter_flows_import(bnk_ctx *ctx, const bnk_flow_entry *entries, size_t n) {
         uint32_t at = flow_hash(key) & (cap - 1);
         bool placed = false;
         for (uint32_t probe = 0; probe < cap && !placed; probe++, at = (at + 1) & (cap - 1)) {
-            unsigned long long &k = h.keys[base + at];
+            unsigned long long &k = h.slots[base + at].key;
             if (k != FLOW_EMPTY && k != key) continue;
             if (k == FLOW_EMPTY) {
                 k = key;
                 h.ctl.rep.used[cls]++;
             }
-            long long &x = h.exp[base + at];
+            long long &x = h.slots[base + at].exp;
             if (flow_absent(x)) h.ctl.rep.live++;
             if (x == FLOW_DEAD) h.ctl.rep.dead[cls]--;
             x = e.expiry_unix_ns;
@@ -441,10 +431,7 @@ int filter_flows_import(bnk_ctx *ctx, const bnk_flow_entry *entries, size_t n) {
     }
     const size_t total = (size_t)6 * cap;
     cudaError_t e = cudaSuccess;
-    if (total) {
-        e = cudaMemcpy(ft.flow_keys, h.keys.data(), total * sizeof(uint64_t), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(ft.flow_exp, h.exp.data(), total * sizeof(long long), cudaMemcpyHostToDevice);
-    }
+    if (total) e = cudaMemcpy(ft.flow_slots, h.slots.data(), total * sizeof(FlowSlot), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(ft.flow_special_exp, h.special, sizeof h.special, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(ft.flow_live, &h.ctl, sizeof h.ctl, cudaMemcpyHostToDevice);
     return e == cudaSuccess ? BNK_SUCCESS : BNK_ECUDA;
