@@ -7,6 +7,7 @@
 #include <stdlib.h>
 
 #include <atomic>
+#include <memory>
 #include <mutex>
 #include <shared_mutex>
 #include <string>
@@ -101,6 +102,7 @@ struct FlowReport {
     uint32_t dead[3];        // of those, deleted ones (reclaimed by compaction)
 };
 
+class CopyCrew;
 struct bnk_ctx {
     bnk_cfg cfg;
     int device;
@@ -125,6 +127,7 @@ struct bnk_ctx {
     // (rule table) holds it exclusively.
     std::shared_mutex submit_mu;
     std::vector<bnk_batch *> batches;       // every live batch of the context (guarded by mu)
+    std::shared_ptr<CopyCrew> crew;         // helpers of its queues' copies, made with the first queue (guarded by mu)
     std::atomic<uint32_t> flow_dead_hint[3]; // deleted entries per class as last reported by the device
     // What the host knows about the flow table without asking: no entry expires before flow_floor, at most
     // flow_live_most are live.  Every submit with filter work widens them; a report of the device replaces them
