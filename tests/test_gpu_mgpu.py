@@ -156,3 +156,30 @@ def test_dispatcher_runs_the_filter_of_the_peers_gpu(gpu_lib, oracle):
         assert np.array_equal(got_who, who)
         assert st.reshape(n_peers, 4).tolist() == [[PKT_OK, PKT_OK, PKT_FILTER_DENY, PKT_FILTER_DENY]] * n_peers
         assert pts[0] == inner[0] and pts[1] == inner[1]
+
+
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 2560, 2561])
+def test_refused_packets_around_the_shared_look(gpu_lib, n):
+    """Calls of which several threads read the descriptors and headers: the first and last packet of every stretch of 512
+    are refused on the host, everything else comes back as it went in."""
+    from bnk_b200.device import PKT_NO_KEYPAIR, PKT_OK
+    from bnk_b200.mgpu import MultiGpu
+
+    rng = np.random.default_rng(n)
+    keys = rng.integers(0, 256, (5, 32), dtype=np.uint8)
+    with MultiGpu([0], max_peers=5, max_pkts_per_gpu=1024) as m:
+        for p in range(4):
+            m.peer_set(p, keys[p].tobytes(), keys[p].tobytes(), 0x100 + p, 0x100 + p)
+        pkts = [rng.integers(0, 256, int(k), dtype=np.uint8).tobytes() for k in rng.integers(1, 100, n)]
+        peers = rng.integers(0, 4, n).astype(np.uint32)
+        edge = np.zeros(n, bool)
+        edge[0::512] = edge[511::512] = edge[-1] = True
+        msgs, st, _ = m.seal(pkts, np.where(edge, 4, peers).astype(np.uint32))  # peer 4 is not set
+        assert np.array_equal(st == PKT_NO_KEYPAIR, edge) and (st[~edge] == PKT_OK).all()
+        msgs, st, _ = m.seal(pkts, peers)
+        assert (st == PKT_OK).all()
+        inbound = [x[:4] + b"\xff\xff\xff\x7f" + x[8:] if e else x for x, e in zip(msgs, edge)]
+        plain, st, _, who = m.open(inbound)
+        assert np.array_equal(st == PKT_NO_KEYPAIR, edge) and (st[~edge] == PKT_OK).all()
+        for i in np.flatnonzero(~edge):
+            assert who[i] == peers[i] and plain[i][:len(pkts[i])] == pkts[i], i
