@@ -76,6 +76,11 @@ def test_counters_and_replay_at_the_edges_of_a_split(gpu_lib, oracle, n, n_peers
         c.close()
 
 
+@pytest.mark.parametrize("n", [16, 17, 64, 65, 160, 161])  # sizes of the descriptors that go along with a launch
+def test_counters_and_replay_at_the_edges_of_inline_descriptors(gpu_lib, oracle, n):
+    test_counters_and_replay_at_the_edges_of_a_split(gpu_lib, oracle, n, 40)
+
+
 @pytest.mark.parametrize("copies", [False, True])
 def test_round_edges_and_forgeries_of_long_packets(gpu_lib, oracle, copies):
     from bnk_b200.device import F_NO_D2H, F_NO_H2D
