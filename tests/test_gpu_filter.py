@@ -356,3 +356,39 @@ def test_nested_prefixes_and_merged_port_ranges(gpu_lib, oracle, n):
             assert np.array_equal(b.status == 0, want != 0), np.flatnonzero((b.status == 0) != (want != 0))[:5]
         assert n < 1000 or 200 < (want != 0).sum() < n - 200
         b.close()
+
+
+@pytest.mark.parametrize("n", [1025, 16384, 16385, 49152, 49153, 180000])  # a stretch of descriptors: 16,384, then double
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_packets_close_together_go_up_stretch_by_stretch(gpu_lib, oracle, n, shuffled):
+    """Headers 48 bytes apart, in ring order and not, on a device copy that holds others: every verdict is that of the
+    header the host wrote."""
+    from bnk_b200 import Context
+
+    rng = np.random.default_rng(n)
+    rule = ([(RC.ip("100.64.1.0"), 24)], "udp", [(1000, 1999)])
+    chk = oracle.Filter()
+    chk.set_rules([rule])
+    h = np.zeros((n, 28), np.uint8)
+    h[:] = np.frombuffer(RC.udp(RC.ip("100.64.1.1"), RC.SELF, 40000, 1000)[:28], np.uint8)
+    h[:, 14] = rng.integers(1, 3, n)              # the source's third byte: in the prefix or beside it
+    port = rng.integers(500, 2500, n)
+    h[:, 22], h[:, 23] = port >> 8, port & 255
+    lens = np.full(n, 28, np.uint32)
+    want = chk.check_batch(h, 28, lens, RC.T0) != 0
+    from bnk_b200.filter import CompiledRule, PortRange, flatten_rules
+
+    with Context(max_keypairs=1, flow_capacity=1 << 10) as c:
+        c.acl_set(True, flatten_rules([CompiledRule(srcs=["100.64.1.0/24"], proto="udp", ports=[PortRange(1000, 1999)])]))
+        b = c.batch(n, n * 48)
+        place = rng.permutation(n) if shuffled else np.arange(n)
+        b.off[:], b.len[:] = place * 48, lens
+        slots = b.ring.reshape(n, 48)
+        slots[:] = 0
+        b.filter_check(n, RC.T0)                  # the device's copy: headers that nothing allows
+        assert (b.status != 0).all()
+        slots[place, 16:44] = h
+        b.filter_check(n, RC.T0)
+        assert np.array_equal(b.status == 0, want), np.flatnonzero((b.status == 0) != want)[:5]
+        assert 0.1 < want.mean() < 0.4
+        b.close()
