@@ -147,9 +147,14 @@ cudaError_t tally_if_asked(bnk_batch *b, uint32_t npkts, uint32_t flags, cudaStr
 // 77 us at 1.6 MB, 234 at 6.4 MB, 680 at 24 MB and 4.55 ms at 190 MB: only far up they are the faster form.
 // With several batches in flight the engines overlap the batches' copies with each other (48 GB/s each way together),
 // and many kernels on the link at once slow each other down, so a batch runs this way only if nothing else is in
-// flight, or if all that run this way together stay below kDirectTogether bytes and kDirectBatches batches.
+// flight, or if all that run this way together stay below kDirectTogether bytes and few others are in flight: for a
+// batch of more than 384 KB three, because SMs move 28-33 GB/s each way over the link and the engines, kept busy by that
+// many batches, 46-48.  Queue of 1024-packet batches, Gbit/s with up to sixteen others / three / none in place beyond
+// 384 KB: 32 callers x 4 calls 195 / 255 / 243, 16 x 4 193 / 205 / 197, 16 x 2 (smaller batches) 182 / 170 / 146 (the last
+// column by an earlier build).
 constexpr uint64_t kDirectTogether = 6ull << 20;
-constexpr int kDirectBatches = 16;
+constexpr uint64_t kDirectSmall = 384u << 10;
+constexpr int kDirectBatches = 16, kDirectLarge = 3;
 bool host_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, uint64_t ext) {
     bnk_ctx *ctx = b->ctx;
     if (ctx->host_direct_bytes == 0 || npkts == 0 || (flags & (BNK_F_NO_H2D | BNK_F_NO_D2H | BNK_F_USE_OUT_LEN)) ||
@@ -157,7 +162,8 @@ bool host_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, uint64_t ext) {
         return false;
     const uint64_t together = ctx->direct_in_flight.load(std::memory_order_relaxed) - b->direct_counted;
     const int others = ctx->in_flight.load(std::memory_order_relaxed) - (b->counted ? 1 : 0);
-    if (others > 0 && (together + ext > kDirectTogether || others >= kDirectBatches)) return false;
+    const int most = ext > kDirectSmall ? kDirectLarge : kDirectBatches;
+    if (others > 0 && (together + ext > kDirectTogether || others >= most)) return false;
     ctx->direct_in_flight.fetch_add(ext - b->direct_counted, std::memory_order_relaxed);
     b->direct_counted = ext;
     return true;
