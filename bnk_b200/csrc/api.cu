@@ -1504,6 +1504,7 @@ int bnk_classify_submit(bnk_batch *b, uint32_t npkts, uint32_t flags) {
     return BNK_SUCCESS;
 }
 
+constexpr uint32_t kPlainRuns = 16; // copies of plain packets between a split's segments
 int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_super, uint32_t n_pkts,
                          uint32_t flags) {
     int rc = begin_submit(b, n_pkts, true); // the descriptor staging area is host memory in any case
@@ -1518,17 +1519,42 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
         const bool refresh = b->dev_stale;
         b->dev_stale = false;
         // The segments' slots are written on the device: of the ring only the super-packets have to go up, in one copy when
-        // they lie close together.  (Device copies that are behind the host arrays catch up as a whole.)
+        // they lie close together, and the packets that are no super-packet's segments, each run of them in a copy of its
+        // own.  (Device copies that are behind the host arrays catch up as a whole, and so does a batch that is cut into
+        // many runs, whose plain packets are spread over most of the ring, or whose super-packets are not in batch order.)
         uint64_t ext = ring_extent(b, n_pkts, 16 + 16 + 16), from = ~0ull, to = 0, sum = 0;
+        struct {
+            uint64_t at, to;
+        } run[kPlainRuns];
+        uint32_t runs = 0, next = 0; // packets below `next` are dealt with
+        uint64_t plain_bytes = 0;
+        bool whole = refresh || n_super == 0;
+        auto plain_up_to = [&](uint32_t end) {
+            if (next >= end || whole) return;
+            uint64_t lo = ~0ull, hi = 0;
+            for (uint32_t i = next; i < end; i++) {
+                lo = std::min<uint64_t>(lo, b->host.off[i]);
+                hi = std::max(hi, (uint64_t)b->host.off[i] + b->host.len[i] + 16 + 16 + 16);
+            }
+            lo &= ~63ull;
+            hi = std::min<uint64_t>((hi + 15) & ~15ull, b->ring_bytes);
+            if (lo >= hi) return;
+            if (runs == kPlainRuns || (plain_bytes += hi - lo) > ext / 2) whole = true;
+            else run[runs++] = {lo, hi};
+        };
         for (uint32_t j = 0; j < n_super; j++) {
             const uint64_t at = supers[j].src_off, e = at + supers[j].src_len;
             if (e > b->ring_bytes) return fail(ctx, BNK_EINVAL, "super-packet lies outside the ring");
             if (at < from) from = at;
             if (e > to) to = e;
             sum += supers[j].src_len;
+            if (supers[j].first_pkt < next) whole = true;
+            plain_up_to(std::min(supers[j].first_pkt, n_pkts));
+            next = (uint32_t)std::min<uint64_t>((uint64_t)supers[j].first_pkt + supers[j].n_pkts, n_pkts);
         }
+        plain_up_to(n_pkts);
         from &= ~63ull;
-        b->ring_partial = !(refresh || n_super == 0 || to - from > 2 * sum + 65536);
+        b->ring_partial = !(whole || to - from > 2 * sum + 65536);
         if (!b->ring_partial) {
             from = 0;
             if (to < ext) to = ext;
@@ -1536,6 +1562,8 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
         to = (to + 15) & ~15ull;
         if (to > b->ring_bytes) to = b->ring_bytes;
         if (to > from) CK(ctx, cudaMemcpyAsync(b->dev.ring + from, b->host.ring + from, to - from, cudaMemcpyHostToDevice, s));
+        for (uint32_t k = 0; b->ring_partial && k < runs; k++)
+            CK(ctx, cudaMemcpyAsync(b->dev.ring + run[k].at, b->host.ring + run[k].at, run[k].to - run[k].at, cudaMemcpyHostToDevice, s));
         if (n && refresh) {
             CK(ctx, desc_copy(b, n, D_OFF, D_STATUS, true, s));
         } else if (n) {

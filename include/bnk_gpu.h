@@ -271,10 +271,11 @@ int bnk_classify_submit(bnk_batch *b, uint32_t npkts, uint32_t flags);
  * Super-packet j is ring[src_off .. src_off+src_len); its segments are packets first_pkt .. first_pkt +
  * n_pkts - 1 of the batch, whose off[], len[] (= hdr_len + segment payload) and slot[] the caller has
  * filled; each segment is written at ring[off+16], ready for bnk_seal_submit(... BNK_F_NO_H2D ...).
- * The submit copies ring, descriptors and `supers` to the device unless BNK_F_NO_H2D is given, and
- * copies nothing back.  A segment whose descriptor does not match the split (wrong len, out of range,
- * unsupported header layout) has its device-side slot[] set to an invalid keypair, so the seal that
- * follows reports BNK_PKT_BAD_DESC for it. */
+ * Packets that are no super-packet's segments stay as they are, so one batch may hold both.  The submit
+ * copies the super-packets, those other packets, the descriptors and `supers` to the device unless
+ * BNK_F_NO_H2D is given, and copies nothing back.  A segment whose descriptor does not match the split
+ * (wrong len, out of range, unsupported header layout) has its device-side slot[] set to an invalid
+ * keypair, so the seal that follows reports BNK_PKT_BAD_DESC for it. */
 typedef struct bnk_gso_super {
     uint32_t src_off;     /* 4-byte aligned */
     uint32_t src_len;

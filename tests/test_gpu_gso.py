@@ -298,3 +298,66 @@ def test_config5_full_size_every_segment(gpu_lib, oracle):
     finally:
         tx.close()
         rx.close()
+
+
+# where plain packets stand beside segments; "many": more runs than are copied one by one; "back": super-packets not in batch order
+@pytest.mark.parametrize("order", ["front", "between", "behind", "all", "many", "back"])
+@pytest.mark.parametrize("busy", [False, True])  # True: another batch in flight, so that the results come back by copy
+def test_plain_packets_beside_segments(gpu_lib, oracle, order, busy):
+    """A batch of segments and packets that are none, on a device ring that holds another batch's bytes: every packet is
+    sealed from what the host ring holds, and its flow is noted."""
+    from bnk_b200 import Context
+    from bnk_b200.device import F_ASSIGN_COUNTERS, F_NO_D2H, F_NO_H2D, F_NOTE_OUTBOUND, GSO_SUPER_DTYPE
+
+    rng = np.random.default_rng(len(order))
+    plan = {"front": "ppS", "between": "SpS", "behind": "SSpp", "all": "pSppSp", "many": "pS" * 20 + "p", "back": "SpSp"}[order]
+    packets, segs_of, gso = [], [], 700
+    for kind in plan:
+        if kind == "S":
+            pkt, cs, hdr = _tcp_super(rng, int(rng.integers(gso, 9 * gso)))
+            segs = oracle.gso_split(pkt, hdr, gso, cs, 16, 6)
+            segs_of.append((len(packets), pkt, cs, hdr, len(segs)))
+            packets += segs
+        else:
+            pkt, _, _ = _tcp_super(rng, int(rng.integers(0, 1300)))
+            packets.append(pkt)
+    n, stride = len(packets), 1472
+    sup = np.zeros(len(segs_of), GSO_SUPER_DTYPE)
+    at = n * stride
+    for j, (first, pkt, cs, hdr, count) in enumerate(segs_of if order != "back" else segs_of[::-1]):
+        sup[j]["src_off"], sup[j]["src_len"], sup[j]["first_pkt"], sup[j]["n_pkts"] = at, len(pkt), first, count
+        sup[j]["hdr_len"], sup[j]["gso_size"], sup[j]["csum_start"], sup[j]["csum_offset"], sup[j]["proto"] = hdr, gso, cs, 16, 6
+        at += (len(pkt) + 15) & ~15
+    key, now = rng.integers(0, 256, (1, 32), dtype=np.uint8), RC.T0
+    with Context(max_keypairs=1, mtu=1420, flow_capacity=1 << 12) as c:
+        c.set_keypairs(0, key, key, np.array([9], np.uint32))
+        c.acl_set(True, None)
+        f = oracle.Filter()
+        f.set_rules([])
+        b, other = c.batch(n, at + 64), c.batch(1, 2048)
+        other.off[0], other.len[0], other.slot[0], other.counter[0] = 0, 1000, 0, 1 << 40
+        b.off[:], b.slot[:] = H.layout_fixed(n, stride), 0
+        b.len[:] = 1400
+        for i in range(n):  # the use before this one: other packets, in the same places
+            pkt, _, _ = _tcp_super(rng, 1360)
+            b.ring[i * stride + 16:i * stride + 16 + 1400] = np.frombuffer(pkt, np.uint8)
+        b.upload(n)
+        b.seal(n, F_NO_H2D | F_NO_D2H)
+        b.ring[:] = 0
+        b.len[:] = [len(p) for p in packets]
+        for j, (first, pkt, cs, hdr, count) in enumerate(segs_of):
+            o = int(sup["src_off"][list(sup["first_pkt"]).index(first)])
+            b.ring[o:o + len(pkt)] = np.frombuffer(pkt, np.uint8)
+        segments = np.concatenate([np.arange(first, first + count) for first, _, _, _, count in segs_of])
+        for i in np.setdiff1d(np.arange(n), segments):
+            b.ring[i * stride + 16:i * stride + 16 + len(packets[i])] = np.frombuffer(packets[i], np.uint8)
+        b.gso_split(sup, n)
+        if busy:
+            other.seal(1, wait=False)
+        b.seal(n, F_NO_H2D | F_NOTE_OUTBOUND | F_ASSIGN_COUNTERS, now)
+        other.wait()
+        assert (b.status == 0).all()
+        for i in range(n):
+            assert b.message(i) == oracle.wg_seal(key[0].tobytes(), 9, i, packets[i], 1420), i
+            f.note_outbound(packets[i], now)
+        assert H.flows_equal(c.flows_export(), f.flows())
