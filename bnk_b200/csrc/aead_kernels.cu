@@ -215,16 +215,6 @@ __device__ __forceinline__ uint32_t keep_bytes(uint32_t w, int k) {
     return w & ((1u << (8 * k)) - 1u);
 }
 
-// WireGuard padding: up to a multiple of 16, never beyond the MTU; a packet
-// longer than the MTU is padded as if only its last MTU-sized unit counted.
-__device__ __forceinline__ uint32_t wg_padded_len(uint32_t len, uint32_t mtu) {
-    if (mtu == 0) return (len + 15u) & ~15u;
-    uint32_t last = len > mtu ? len % mtu : len;
-    uint32_t padded = (last + 15u) & ~15u;
-    if (padded > mtu) padded = mtu;
-    return len + (padded - last);
-}
-
 // ---------------------------------------------------------------------------
 // Descriptor of one packet, validated; the outcome of a refused packet is recorded here.
 // ---------------------------------------------------------------------------

@@ -321,7 +321,7 @@ cudaError_t ring_up(bnk_batch *b, uint64_t ext, bool joint, cudaStream_t s) {
 cudaError_t ring_down(bnk_batch *b, uint32_t n, uint64_t ext, bool joint, cudaStream_t s) {
     if (b->ring_partial) { // what lies between the packets stays the host's
         const cudaError_t e = joint ? desc_copy(b, n, D_OFF, D_STATUS, false, s) : cudaSuccess;
-        return e != cudaSuccess ? e : launch_slots_to_host(b, n, s);
+        return e != cudaSuccess ? e : launch_packets_to_host(b, n, s);
     }
     if (joint) return cudaMemcpyAsync(b->h_desc, b->d_desc, b->desc_room + ext, cudaMemcpyDeviceToHost, s);
     return ext ? cudaMemcpyAsync(b->host.ring, b->dev.ring, ext, cudaMemcpyDeviceToHost, s) : cudaSuccess;
@@ -1016,6 +1016,7 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     a.out = h.ring;
     a.res[0] = AeadResults{assign ? h.counter : nullptr, h.out_len, h.status, nullptr};
     if (resident) {
+        b->split_sealed = std::max(b->split_sealed, npkts);
         a.out2 = d.ring;
         a.res[1] = AeadResults{nullptr, d.out_len, d.status, nullptr}; // the counters are there
         if (!assign) a.res[0].counter = h.counter;
@@ -1171,6 +1172,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     }
     if (timed) CK(ctx, cudaEventRecord(b->a_begin, as));
     CK(ctx, launch_seal(a, as, ctx));
+    b->split_sealed = std::max(b->split_sealed, npkts);
     if (timed) CK(ctx, cudaEventRecord(b->a_end, as));
     if (side) {
         CK(ctx, cudaEventRecord(b->ev_aead_done, as));
@@ -1555,6 +1557,7 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
         plain_up_to(n_pkts);
         from &= ~63ull;
         b->ring_partial = !(whole || to - from > 2 * sum + 65536);
+        b->split_sealed = 0;
         if (!b->ring_partial) {
             from = 0;
             if (to < ext) to = ext;

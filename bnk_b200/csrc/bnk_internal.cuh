@@ -200,6 +200,7 @@ struct bnk_batch {
     bool in_flight;
     bool dev_stale; // a submit ran on the host arrays: the device copies of ring and descriptors are behind
     bool ring_partial;   // of the device ring only packets and super-packets are those of the host ring
+    uint32_t split_sealed; // with ring_partial: that many packets have been sealed since the split
     bool counted;        // this batch is one of ctx->in_flight
     uint64_t direct_counted; // what it adds to ctx->direct_in_flight
     // bnk_wait watches *h_done for done_seq when done_watched: the last kernel of the submit stores it (Done)
@@ -276,6 +277,16 @@ cudaError_t launch_kernel(bool dependent, void (*kernel)(KArgs...), dim3 grid, d
 }
 
 constexpr uint32_t kSlotNoKeypair = 0xfffffffeu; // demux found no keypair for the receiver index
+
+// WireGuard padding: up to a multiple of 16, never beyond the MTU; a packet
+// longer than the MTU is padded as if only its last MTU-sized unit counted.
+__device__ __forceinline__ uint32_t wg_padded_len(uint32_t len, uint32_t mtu) {
+    if (mtu == 0) return (len + 15u) & ~15u;
+    uint32_t last = len > mtu ? len % mtu : len;
+    uint32_t padded = (last + 15u) & ~15u;
+    if (padded > mtu) padded = mtu;
+    return len + (padded - last);
+}
 
 // ---------------------------------------------------------------------------
 // Kernel launchers (each defined next to its kernels).  All are asynchronous on
@@ -458,4 +469,4 @@ __device__ __forceinline__ uint32_t demux_index_warp(const uint64_t *keys, const
 
 // gso_kernels.cu
 cudaError_t launch_gso_split(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, cudaStream_t s);
-cudaError_t launch_slots_to_host(bnk_batch *b, uint32_t n, cudaStream_t s);
+cudaError_t launch_packets_to_host(bnk_batch *b, uint32_t n, cudaStream_t s);

@@ -163,17 +163,25 @@ __global__ void gso_map_kernel(const bnk_gso_super *supers, uint32_t n_super, ui
         if (sp.first_pkt + k < n_pkts) seg_super[sp.first_pkt + k] = j;
 }
 
-// Packets' slots from the device ring to the pinned one, a warp per packet: header room, what the packet holds and the
-// room behind it.
-__global__ void __launch_bounds__(256) slots_to_host_kernel(const uint8_t *ring, uint8_t *host_ring, const uint32_t *off,
-                                                            const uint32_t *len, const uint32_t *out_len, uint32_t n, uint64_t ring_bytes) {
+// What the device has made of the packets of a split, to the pinned ring, a warp per packet: the packet, or once a seal has
+// run the message.  A packet that the split or the seal refused leaves no bytes.
+__global__ void __launch_bounds__(256) packets_to_host_kernel(const uint8_t *ring, uint8_t *host_ring, const uint32_t *off,
+                                                              const uint32_t *len, const uint32_t *slot, const uint8_t *status,
+                                                              uint32_t n, uint64_t ring_bytes, uint32_t max_slots, uint32_t mtu, uint32_t sealed) {
     const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (i >= n) return;
-    const uint64_t begin = off[i] & ~15u;
-    uint64_t end = begin + 64u + max(len[i], out_len[i]);
-    if (end > ring_bytes) end = ring_bytes;
-    for (uint64_t q = begin + 16u * lane; q + 16u <= end; q += 512u)
-        *reinterpret_cast<uint4 *>(host_ring + q) = *reinterpret_cast<const uint4 *>(ring + q);
+    if (i >= n || slot[i] >= max_slots || (off[i] & 15u)) return;
+    uint64_t at = off[i] + 16ull;
+    uint32_t bytes = len[i];
+    const uint8_t st = i < sealed ? status[i] : (uint8_t)BNK_PKT_BAD_DESC;
+    if (st != BNK_PKT_BAD_DESC && st != BNK_PKT_NO_KEYPAIR && st != BNK_PKT_COUNTER_EXHAUSTED && st != BNK_PKT_MALFORMED) {
+        at -= 16u;
+        bytes = 16u + wg_padded_len(bytes, mtu) + 16u;
+    }
+    if (at + bytes > ring_bytes) return;
+    for (uint32_t q = 16u * lane; q + 16u <= bytes; q += 512u)
+        *reinterpret_cast<uint4 *>(host_ring + at + q) = *reinterpret_cast<const uint4 *>(ring + at + q);
+    const uint32_t tail = (bytes & ~15u) + lane;
+    if (tail < bytes) host_ring[at + tail] = ring[at + tail];
 }
 
 __global__ void fill_u32_kernel(uint32_t *p, uint32_t n, uint32_t v) {
@@ -199,8 +207,10 @@ cudaError_t launch_gso_split(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, cu
     return cudaGetLastError();
 }
 
-cudaError_t launch_slots_to_host(bnk_batch *b, uint32_t n, cudaStream_t s) {
-    slots_to_host_kernel<<<(n + 7) / 8, 256, 0, s>>>(b->dev.ring, b->host.ring, b->dev.off, b->dev.len, b->dev.out_len, n, b->ring_bytes);
+cudaError_t launch_packets_to_host(bnk_batch *b, uint32_t n, cudaStream_t s) {
+    const bnk_cfg &cfg = b->ctx->cfg;
+    packets_to_host_kernel<<<(n + 7) / 8, 256, 0, s>>>(b->dev.ring, b->host.ring, b->dev.off, b->dev.len, b->dev.slot, b->dev.status, n,
+                                                       b->ring_bytes, cfg.max_keypairs, cfg.mtu, b->split_sealed);
     b->ctx->launches += 1;
     return cudaGetLastError();
 }

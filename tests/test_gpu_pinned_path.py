@@ -156,50 +156,70 @@ def test_flows_noted_by_the_seal_kernel_and_swept(gpu_lib, oracle):
             assert H.flows_equal(c.flows_export(), f.flows()), turn
 
 
-@pytest.mark.parametrize("busy", [False, True])  # True: another batch in flight, so that the results come back by copy
-def test_split_uploads_super_packets_only(gpu_lib, oracle, busy):
-    """The split and the seal behind it change packets and their room, not what the host ring holds beside them, and the
-    sealed messages are on the device too."""
+@pytest.mark.parametrize("copied", [False, True])  # how the results come back
+def test_split_uploads_super_packets_only(gpu_lib, oracle, copied, monkeypatch):
+    """The split and the seal behind it change packets, then messages, and not a byte beside them in the host ring, where
+    slots stand back to back and device memory holds another use's bytes; a refused segment changes none.  The sealed
+    messages are on the device too."""
     from bnk_b200 import Context
-    from bnk_b200.device import F_ASSIGN_COUNTERS, F_NO_H2D, F_REPLAY, F_USE_OUT_LEN
+    from bnk_b200.device import F_ASSIGN_COUNTERS, F_NO_H2D, F_REPLAY, F_USE_OUT_LEN, PKT_BAD_DESC, PKT_NO_KEYPAIR
     from tests.test_gpu_gso import _plan, _tcp_super
 
+    if copied:
+        monkeypatch.setenv("BNK_HOST_DIRECT_BYTES", "0")
     rng = np.random.default_rng(4)
     supers, meta = [], []
     for size, gso in [(40_000, 1251), (9000, 333), (1380, 1380), (7, 2)]:
         pkt, cs, hdr = _tcp_super(rng, size)
         supers.append(pkt)
         meta.append((hdr, gso, cs, 16, 6))
-    stride = 1472
-    sup, seg_len, n, ring_bytes = _plan(supers, meta, stride)
+    sup, seg_len, n, ring_bytes = _plan(supers, meta, 1472)
     want = [s for p, m in zip(supers, meta) for s in oracle.gso_split(p, *m)]
     key = rng.integers(0, 256, (1, 32), dtype=np.uint8)
-    with Context(max_keypairs=1, mtu=1420, flow_capacity=0) as c:
+    with Context(max_keypairs=2, mtu=1420, flow_capacity=0) as c:
         c.set_keypairs(0, key, key, np.array([9], np.uint32))
-        b, other = c.batch(n, ring_bytes + 64), c.batch(1, 2048)
-        other.off[0], other.len[0], other.slot[0], other.counter[0] = 0, 1000, 0, 1 << 40
+        b = c.batch(n, ring_bytes + 64)
+        off = H.layout_packed(seg_len, slack=48)
+        off += (np.arange(n) >= n // 2).astype(np.uint32) * 64  # a gap in the middle
+        b.off[:], b.len[:], b.slot[:] = off, 1400, 0
+        b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
+        b.upload(n)
         b.ring[:] = 0xEE
         for j, pkt in enumerate(supers):
             b.ring[int(sup[j]["src_off"]):int(sup[j]["src_off"]) + len(pkt)] = np.frombuffer(pkt, np.uint8)
-        b.off[:], b.len[:], b.slot[:] = H.layout_fixed(n, stride), seg_len, 0
+        b.len[:] = seg_len
+        b.len[3] += 1   # does not match the split
+        b.slot[5] = 1   # no keys there
         before = np.array(b.ring)
         b.gso_split(sup, n)
-        if busy:
-            other.seal(1, wait=False)
+        if copied:  # (a download between the two: the packets themselves)
+            b.download(n)
+            expect = np.array(before)
+            for i in np.delete(np.arange(n), 3):
+                expect[off[i] + 16:off[i] + 16 + len(want[i])] = np.frombuffer(want[i], np.uint8)
+            assert np.array_equal(b.ring, expect)
+            b.ring[:] = before
         b.seal(n, F_NO_H2D | F_ASSIGN_COUNTERS)
-        assert (b.status == 0).all()
-        room = np.zeros(len(before), bool)
+        assert b.status[3] == PKT_BAD_DESC and b.status[5] == PKT_NO_KEYPAIR
+        good = np.delete(np.arange(n), [3, 5])
+        assert (b.status[good] == 0).all()
+        expect, ctr = np.array(before), 0
         for i in range(n):
-            o = int(b.off[i])
-            assert b.message(i) == oracle.wg_seal(key[0].tobytes(), 9, i, want[i], 1420), i
-            room[o:o + 64 + len(want[i]) + 32] = True
-        assert np.array_equal(b.ring[~room], before[~room])
+            if i not in (3, 5):
+                msg = oracle.wg_seal(key[0].tobytes(), 9, ctr, want[i], 1420)
+                expect[off[i]:off[i] + len(msg)] = np.frombuffer(msg, np.uint8)
+            ctr += i not in (3, 5)
+        if copied:  # of the segment that the seal refused, what the split has made of it
+            expect[off[5] + 16:off[5] + 16 + len(want[5])] = np.frombuffer(want[5], np.uint8)
+        assert np.array_equal(b.ring, expect)
         b.open(n, F_NO_H2D | F_USE_OUT_LEN | F_REPLAY)
-        assert (b.status == 0).all()
-        for i in range(n):
+        assert (b.status[good] == 0).all()
+        room = np.zeros(len(before), bool)
+        for i in good:
             assert b.payload(i)[:len(want[i])] == want[i], i
+            room[off[i]:off[i] + 32 + ((len(want[i]) + 15) & ~15)] = True
+        room[off[5] + 16:off[5] + 16 + len(want[5])] = True
         assert np.array_equal(b.ring[~room], before[~room])
-        other.wait()
 
 
 @pytest.mark.parametrize("n,sizes", [(4000, (1420, 1404, 1)), (12_000, (64, 300, 0)), (100, (65_000, 30_001, 9)), (2200, (65_000, 30_001, 9))])
