@@ -93,7 +93,7 @@ uint64_t ring_extent(const bnk_batch *b, uint32_t n, uint32_t slack, uint64_t *b
 int begin_submit(bnk_batch *b, uint32_t npkts, bool touches_host = true) {
     if (!b) return BNK_EINVAL;
     if (npkts > b->max_pkts) return fail(b->ctx, BNK_EINVAL, "npkts exceeds the batch capacity");
-    if (b->in_flight && (touches_host || b->dev_stale))
+    if (b->in_flight && (touches_host || b->stale_pkts))
         return fail(b->ctx, BNK_EBUSY, "batch has work in flight; call bnk_wait first");
     CK(b->ctx, cudaSetDevice(b->ctx->device));
     return BNK_SUCCESS;
@@ -139,8 +139,8 @@ cudaError_t tally_if_asked(bnk_batch *b, uint32_t npkts, uint32_t flags, cudaStr
 // descriptors through the host link and write the results straight back (pinned memory has the same address on the
 // device).  Copies either side of the kernels run one after the other, each at ~55 GB/s and ~8 us before it moves
 // anything; a kernel that works on the pinned ring moves both directions at once.  While a HostAlias lives, the
-// launchers see the host arrays where the device copies would be; the device copies fall behind (dev_stale) until the
-// next full upload.
+// launchers see the host arrays where the device copies would be; the device copies fall behind (stale_pkts) until
+// catch_up or an upload of as many packets.
 // Measured with plain copies through SMs, 1440-byte pieces read and written in place, against upload, kernel and
 // download in a row: 190 KB 17 us against 33, 1.6 MB 56 against 82, 6.4 MB 177 against 253, 24 MB 613 against 916,
 // 190 MB 4.74 ms against 7.0.  Chunks of one batch over three streams, so that the copy engines run both ways, take
@@ -270,7 +270,7 @@ struct HostAlias {
     bnk_batch *b;
     DeviceBatch saved;
     bool on;
-    HostAlias(bnk_batch *batch, bool enable) : b(batch), saved(batch->dev), on(enable) {
+    HostAlias(bnk_batch *batch, bool enable, uint32_t n) : b(batch), saved(batch->dev), on(enable) {
         if (!on) return;
         DeviceBatch &d = b->dev;
         const bnk_batch_view &h = b->host;
@@ -282,7 +282,7 @@ struct HostAlias {
         d.out_len = h.out_len;
         d.status = h.status;
         d.src_addr = h.src_addr;
-        b->dev_stale = true;
+        b->stale_pkts = std::max(b->stale_pkts, n);
     }
     ~HostAlias() {
         if (on) b->dev = saved;
@@ -313,18 +313,47 @@ cudaError_t desc_copy(bnk_batch *b, size_t n, int first, int last, bool to_devic
 }
 
 // The ring and, when they travel together, the descriptors.
+void ring_is_up(bnk_batch *b, uint64_t ext) {
+    if (ext >= b->partial_to) b->partial_to = 0;
+}
 cudaError_t ring_up(bnk_batch *b, uint64_t ext, bool joint, cudaStream_t s) {
-    b->ring_partial = false;
+    ring_is_up(b, ext);
     if (joint) return cudaMemcpyAsync(b->d_desc, b->h_desc, b->desc_room + ext, cudaMemcpyHostToDevice, s);
     return ext ? cudaMemcpyAsync(b->dev.ring, b->host.ring, ext, cudaMemcpyHostToDevice, s) : cudaSuccess;
 }
 cudaError_t ring_down(bnk_batch *b, uint32_t n, uint64_t ext, bool joint, cudaStream_t s) {
-    if (b->ring_partial) { // what lies between the packets stays the host's
+    if (b->partial_to) { // what lies between the packets stays the host's
         const cudaError_t e = joint ? desc_copy(b, n, D_OFF, D_STATUS, false, s) : cudaSuccess;
         return e != cudaSuccess ? e : launch_packets_to_host(b, n, s);
     }
     if (joint) return cudaMemcpyAsync(b->h_desc, b->d_desc, b->desc_room + ext, cudaMemcpyDeviceToHost, s);
     return ext ? cudaMemcpyAsync(b->host.ring, b->dev.ring, ext, cudaMemcpyDeviceToHost, s) : cudaSuccess;
+}
+
+// Brings the device copies up to the host arrays where submits have run on those.  An upload of as many packets with all
+// descriptor fields does the same.
+constexpr uint32_t kMostRoom = 16 + 16 + 16; // header, padding and tag around a payload
+cudaError_t catch_up(bnk_batch *b, cudaStream_t s) {
+    const uint32_t n = b->stale_pkts;
+    if (n == 0) return cudaSuccess;
+    const uint64_t ext = ring_extent(b, n, kMostRoom);
+    cudaError_t e = ring_up(b, ext, b->joint_copy, s);
+    if (e == cudaSuccess && !b->joint_copy) e = desc_copy(b, n, D_OFF, D_STATUS, true, s);
+    if (e == cudaSuccess && b->stale_src)
+        e = cudaMemcpyAsync(b->dev.src_addr, b->host.src_addr, (size_t)b->stale_src * BNK_SRC_ADDR_STRIDE, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) b->stale_pkts = b->stale_src = 0;
+    return e;
+}
+// In front of a submit's own upload of n packets, if it makes one: what that does not cover catches up first.  Returns in
+// `all` whether the upload has to bring every descriptor field (and is then to be followed by caught_up).
+cudaError_t catch_up_beside(bnk_batch *b, uint32_t n, bool uploads, cudaStream_t s, bool &all) {
+    const bool covers = uploads && n >= b->stale_pkts && b->stale_src == 0;
+    const cudaError_t e = covers ? cudaSuccess : catch_up(b, s);
+    all = b->stale_pkts != 0;
+    return e;
+}
+void caught_up(bnk_batch *b, uint32_t n) {
+    if (n >= b->stale_pkts && b->stale_src == 0) b->stale_pkts = 0;
 }
 
 AeadArgs aead_args(bnk_batch *b, uint32_t n, bool open, const uint32_t *order) {
@@ -973,12 +1002,14 @@ int bnk_batch_upload(bnk_batch *b, uint32_t npkts) {
     SubmitScope scope(b);
     bnk_ctx *ctx = b->ctx;
     const size_t n = npkts;
+    bool all;
+    CK(ctx, catch_up_beside(b, npkts, true, b->stream, all));
     const uint64_t ext = ring_extent(b, npkts, 64);
     CK(ctx, ring_up(b, ext, false, b->stream));
     if (n) {
-        CK(ctx, desc_copy(b, n, D_OFF, b->dev_stale ? D_STATUS : D_COUNTER, true, b->stream));
+        CK(ctx, desc_copy(b, n, D_OFF, all ? D_STATUS : D_COUNTER, true, b->stream));
     }
-    b->dev_stale = false;
+    caught_up(b, npkts);
     return BNK_SUCCESS;
 }
 
@@ -988,7 +1019,7 @@ int bnk_batch_download(bnk_batch *b, uint32_t npkts) {
     SubmitScope scope(b);
     bnk_ctx *ctx = b->ctx;
     const size_t n = npkts;
-    if (b->dev_stale) return BNK_SUCCESS; // the last submit already left its results in the host arrays
+    if (b->stale_pkts) return BNK_SUCCESS; // the last submit already left its results in the host arrays
     const uint64_t ext = ring_extent(b, npkts, 64);
     if (n) {
         CK(ctx, ring_down(b, npkts, ext, false, b->stream));
@@ -1021,7 +1052,7 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
         a.res[1] = AeadResults{nullptr, d.out_len, d.status, nullptr}; // the counters are there
         if (!assign) a.res[0].counter = h.counter;
     } else {
-        b->dev_stale = true;
+        b->stale_pkts = std::max(b->stale_pkts, npkts);
         a.from_host = true;
         a.host = HostDesc{h.off, h.len, h.slot};
         a.in = h.ring;
@@ -1076,8 +1107,9 @@ static int seal_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     Piece p;
     pieces.next(p); // the first is on its way while the kernels in front of the first seal are prepared
     CK(ctx, piece_up(b, p));
-    CK(ctx, desc_copy(b, npkts, D_OFF, b->dev_stale ? D_STATUS : (flags & BNK_F_ASSIGN_COUNTERS) ? D_SLOT : D_COUNTER, true, s));
-    b->dev_stale = b->ring_partial = false;
+    CK(ctx, desc_copy(b, npkts, D_OFF, b->stale_pkts ? D_STATUS : (flags & BNK_F_ASSIGN_COUNTERS) ? D_SLOT : D_COUNTER, true, s));
+    caught_up(b, npkts); // (more of them stay behind: the host arrays will hold this call's results as well)
+    ring_is_up(b, ext);
     CK(ctx, order_kernels_begin(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     if (flags & BNK_F_ASSIGN_COUNTERS) CK(ctx, launch_assign_counters(b, npkts, b->dev.slot, b->dev.counter, s));
@@ -1117,25 +1149,22 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
     const size_t n = npkts;
-    // header room + payload + padding (< 16) + tag
-    const bool refresh = b->dev_stale; // the device copies are behind the host arrays: upload whatever the flags say
     uint64_t bytes = 0;
     bool in_order = false;
-    const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, 16 + 16 + 16, &bytes, BNK_WG_HEADER + BNK_WG_TAG, &in_order);
+    const uint64_t ext = device_only ? 0 : ring_extent(b, npkts, kMostRoom, &bytes, BNK_WG_HEADER + BNK_WG_TAG, &in_order);
     if (in_pieces(b, npkts, flags, ext, in_order)) return seal_pieces(b, npkts, ext, flags, now_unix_ns);
     if (ctx->aead_mode != 1) {
         if (host_direct(b, npkts, flags, ext)) return seal_direct(b, npkts, bytes, flags, now_unix_ns, false);
-        if (!refresh && (flags & BNK_F_NO_H2D) && host_direct(b, npkts, flags & ~BNK_F_NO_H2D, ext))
+        if (!b->stale_pkts && (flags & BNK_F_NO_H2D) && host_direct(b, npkts, flags & ~BNK_F_NO_H2D, ext))
             return seal_direct(b, npkts, bytes, flags, now_unix_ns, true);
     }
-    if ((!(flags & BNK_F_NO_H2D) || refresh) && n) {
-        if (b->joint_copy) {
-            CK(ctx, ring_up(b, ext, true, s));
-        } else {
-            CK(ctx, ring_up(b, ext, false, s));
-            CK(ctx, desc_copy(b, n, D_OFF, refresh ? D_STATUS : (flags & BNK_F_ASSIGN_COUNTERS) ? D_SLOT : D_COUNTER, true, s));
-        }
-        b->dev_stale = false;
+    bool all;
+    CK(ctx, catch_up_beside(b, npkts, !(flags & BNK_F_NO_H2D), s, all));
+    if (!(flags & BNK_F_NO_H2D) && n) {
+        CK(ctx, ring_up(b, ext, b->joint_copy, s));
+        if (!b->joint_copy)
+            CK(ctx, desc_copy(b, n, D_OFF, all ? D_STATUS : (flags & BNK_F_ASSIGN_COUNTERS) ? D_SLOT : D_COUNTER, true, s));
+        caught_up(b, npkts);
     }
     CK(ctx, order_kernels_begin(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
@@ -1202,7 +1231,7 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     const bool timed = (flags & BNK_F_TIMED) != 0, stats = (flags & BNK_F_STATS) != 0;
     const bool replay = (flags & BNK_F_REPLAY) != 0, checks = (flags & (BNK_F_INNER_CHECK | BNK_F_CHECK_INBOUND)) != 0;
     const bnk_batch_view &h = b->host;
-    b->dev_stale = true;
+    b->stale_pkts = std::max(b->stale_pkts, npkts);
     CK(ctx, order_kernels_begin(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, true, nullptr);
@@ -1277,8 +1306,9 @@ static int open_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     Piece p;
     pieces.next(p);
     CK(ctx, piece_up(b, p));
-    CK(ctx, desc_copy(b, npkts, D_OFF, b->dev_stale ? D_STATUS : demux ? D_LEN : D_SLOT, true, s));
-    b->dev_stale = b->ring_partial = false;
+    CK(ctx, desc_copy(b, npkts, D_OFF, b->stale_pkts ? D_STATUS : demux ? D_LEN : D_SLOT, true, s));
+    caught_up(b, npkts);
+    ring_is_up(b, ext);
     CK(ctx, order_kernels_begin(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, true, nullptr);
@@ -1323,22 +1353,20 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
     const size_t n = npkts;
-    const bool refresh = b->dev_stale;
     uint64_t bytes = 0;
     bool in_order = false;
-    const uint64_t ext = (device_only && !refresh) ? 0 : ring_extent(b, npkts, (flags & BNK_F_USE_OUT_LEN) ? 48 : 0, &bytes, 0, &in_order);
+    const uint64_t ext = device_only ? 0 : ring_extent(b, npkts, (flags & BNK_F_USE_OUT_LEN) || b->stale_pkts ? kMostRoom : 0, &bytes, 0, &in_order);
     if (in_pieces(b, npkts, flags, ext, in_order)) return open_pieces(b, npkts, ext, flags, now_unix_ns);
     if (ctx->aead_mode != 1 && host_direct(b, npkts, flags, ext)) return open_direct(b, npkts, bytes, flags, now_unix_ns);
     // BNK_F_USE_OUT_LEN reads the lengths a seal left on the device: an upload beside it must not bring the
     // host's out_len along, so it moves the fields one by one instead of the whole slab.
-    if ((!(flags & BNK_F_NO_H2D) || refresh) && n) {
-        if (b->joint_copy && !((flags & BNK_F_USE_OUT_LEN) && !refresh)) {
-            CK(ctx, ring_up(b, ext, true, s));
-        } else {
-            CK(ctx, ring_up(b, ext, false, s));
-            CK(ctx, desc_copy(b, n, D_OFF, refresh ? D_STATUS : (flags & BNK_F_DEMUX_INDEX) ? D_LEN : D_SLOT, true, s));
-        }
-        b->dev_stale = false;
+    bool all;
+    CK(ctx, catch_up_beside(b, npkts, !(flags & BNK_F_NO_H2D), s, all));
+    if (!(flags & BNK_F_NO_H2D) && n) {
+        const bool joint = b->joint_copy && (all || !(flags & BNK_F_USE_OUT_LEN));
+        CK(ctx, ring_up(b, ext, joint, s));
+        if (!joint) CK(ctx, desc_copy(b, n, D_OFF, all ? D_STATUS : (flags & BNK_F_DEMUX_INDEX) ? D_LEN : D_SLOT, true, s));
+        caught_up(b, npkts);
     }
     CK(ctx, order_kernels_begin(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
@@ -1408,9 +1436,8 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
 // needs 920 at 55 GB/s; 300,000 495 and 378, 30,000 69 and 58.
 static int upload_heads(bnk_batch *b, uint32_t n, cudaStream_t s) {
     bnk_ctx *ctx = b->ctx;
-    // after a submit that ran on the host arrays every device descriptor field is behind
-    CK(ctx, desc_copy(b, n, D_OFF, b->dev_stale ? D_STATUS : D_LEN, true, s));
-    b->ring_partial = false;
+    CK(ctx, catch_up(b, s));
+    CK(ctx, desc_copy(b, n, D_OFF, D_LEN, true, s));
     uint64_t up = 0, ext = 0;
     for (uint32_t at = 0, k = kHeadsFirst; at < n; at += k, k = std::min(2 * k, kHeadsMost)) {
         k = std::min(k, n - at);
@@ -1422,7 +1449,7 @@ static int upload_heads(bnk_batch *b, uint32_t n, cudaStream_t s) {
             up = to;
         }
     }
-    b->dev_stale = false;
+    ring_is_up(b, up);
     return BNK_SUCCESS;
 }
 
@@ -1434,10 +1461,11 @@ int bnk_filter_note_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
-    const bool upload = npkts && (!(flags & BNK_F_NO_H2D) || b->dev_stale);
+    const bool upload = npkts && !(flags & BNK_F_NO_H2D);
     const bool direct = upload && heads_direct(b, npkts, flags);
+    if (npkts && !upload) CK(ctx, catch_up(b, s));
     if (!direct && upload && (rc = upload_heads(b, npkts, s)) != BNK_SUCCESS) return rc;
-    HostAlias alias(b, direct);
+    HostAlias alias(b, direct, npkts);
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     const bool note = npkts && ctx->ft.enforce && ctx->ft.flow_capacity; // filter.go:192-194
     bool reported = false;
@@ -1461,10 +1489,11 @@ int bnk_filter_check_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
-    const bool upload = npkts && (!(flags & BNK_F_NO_H2D) || b->dev_stale);
+    const bool upload = npkts && !(flags & BNK_F_NO_H2D);
     const bool direct = upload && heads_direct(b, npkts, flags);
+    if (npkts && !upload) CK(ctx, catch_up(b, s));
     if (!direct && upload && (rc = upload_heads(b, npkts, s)) != BNK_SUCCESS) return rc;
-    HostAlias alias(b, direct);
+    HostAlias alias(b, direct, npkts);
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     flow_check_begins(b, now_unix_ns);
     const bool to_host = !(flags & BNK_F_NO_D2H);
@@ -1486,13 +1515,15 @@ int bnk_classify_submit(bnk_batch *b, uint32_t npkts, uint32_t flags) {
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
     const size_t n = npkts;
-    const bool upload = n && (!(flags & BNK_F_NO_H2D) || b->dev_stale);
+    const bool upload = n && !(flags & BNK_F_NO_H2D);
     const bool direct = upload && heads_direct(b, npkts, flags);
+    if (direct) b->stale_src = std::max(b->stale_src, npkts);
+    if (npkts && !upload) CK(ctx, catch_up(b, s));
     if (!direct && upload) {
         if ((rc = upload_heads(b, npkts, s)) != BNK_SUCCESS) return rc;
         CK(ctx, cudaMemcpyAsync(b->dev.src_addr, b->host.src_addr, n * BNK_SRC_ADDR_STRIDE, cudaMemcpyHostToDevice, s));
     }
-    HostAlias alias(b, direct);
+    HostAlias alias(b, direct, npkts);
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     const Done done = direct && !(flags & BNK_F_STATS) ? watch_for(b) : Done{};
     CK(ctx, launch_classify(b, npkts, done, s));
@@ -1517,20 +1548,20 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
     const bool timed = (flags & BNK_F_TIMED) != 0;
     if (n_super > b->max_pkts || (n_super && !supers)) return fail(ctx, BNK_EINVAL, "bad super-packet list");
     const size_t n = n_pkts;
-    if (!(flags & BNK_F_NO_H2D) || b->dev_stale) {
-        const bool refresh = b->dev_stale;
-        b->dev_stale = false;
+    const bool refresh = b->stale_pkts != 0;
+    CK(ctx, catch_up(b, s));
+    if (!(flags & BNK_F_NO_H2D) || refresh) {
         // The segments' slots are written on the device: of the ring only the super-packets have to go up, in one copy when
         // they lie close together, and the packets that are no super-packet's segments, each run of them in a copy of its
-        // own.  (Device copies that are behind the host arrays catch up as a whole, and so does a batch that is cut into
-        // many runs, whose plain packets are spread over most of the ring, or whose super-packets are not in batch order.)
+        // own.  (The whole ring goes up for a batch that is cut into many runs, whose plain packets are spread over most of
+        // the ring, or whose super-packets are not in batch order.)
         uint64_t ext = ring_extent(b, n_pkts, 16 + 16 + 16), from = ~0ull, to = 0, sum = 0;
         struct {
             uint64_t at, to;
         } run[kPlainRuns];
         uint32_t runs = 0, next = 0; // packets below `next` are dealt with
         uint64_t plain_bytes = 0;
-        bool whole = refresh || n_super == 0;
+        bool whole = n_super == 0;
         auto plain_up_to = [&](uint32_t end) {
             if (next >= end || whole) return;
             uint64_t lo = ~0ull, hi = 0;
@@ -1556,22 +1587,20 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
         }
         plain_up_to(n_pkts);
         from &= ~63ull;
-        b->ring_partial = !(whole || to - from > 2 * sum + 65536);
+        whole = whole || to - from > 2 * sum + 65536;
         b->split_sealed = 0;
-        if (!b->ring_partial) {
+        if (whole) {
             from = 0;
             if (to < ext) to = ext;
         }
         to = (to + 15) & ~15ull;
         if (to > b->ring_bytes) to = b->ring_bytes;
+        if (whole) ring_is_up(b, to);
+        else b->partial_to = std::max({b->partial_to, ext, to});
         if (to > from) CK(ctx, cudaMemcpyAsync(b->dev.ring + from, b->host.ring + from, to - from, cudaMemcpyHostToDevice, s));
-        for (uint32_t k = 0; b->ring_partial && k < runs; k++)
+        for (uint32_t k = 0; !whole && k < runs; k++)
             CK(ctx, cudaMemcpyAsync(b->dev.ring + run[k].at, b->host.ring + run[k].at, run[k].to - run[k].at, cudaMemcpyHostToDevice, s));
-        if (n && refresh) {
-            CK(ctx, desc_copy(b, n, D_OFF, D_STATUS, true, s));
-        } else if (n) {
-            CK(ctx, desc_copy(b, n, D_OFF, D_SLOT, true, s));
-        }
+        if (n) CK(ctx, desc_copy(b, n, D_OFF, D_SLOT, true, s));
     }
     if (n_super) {
         memcpy(b->h_gso, supers, (size_t)n_super * sizeof(bnk_gso_super));

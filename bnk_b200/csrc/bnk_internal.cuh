@@ -198,9 +198,11 @@ struct bnk_batch {
     cudaEvent_t ev_fork, ev_join;
     cudaEvent_t k_begin, k_end, t_end, a_begin, a_end;
     bool in_flight;
-    bool dev_stale; // a submit ran on the host arrays: the device copies of ring and descriptors are behind
-    bool ring_partial;   // of the device ring only packets and super-packets are those of the host ring
-    uint32_t split_sealed; // with ring_partial: that many packets have been sealed since the split
+    // Submits ran on the host arrays: the device copies of the first `stale_pkts` packets and descriptors (of the first
+    // `stale_src` source addresses) are behind.
+    uint32_t stale_pkts, stale_src;
+    uint64_t partial_to;   // below this place of the device ring only packets and super-packets are those of the host ring
+    uint32_t split_sealed; // with partial_to: that many packets have been sealed since the split
     bool counted;        // this batch is one of ctx->in_flight
     uint64_t direct_counted; // what it adds to ctx->direct_in_flight
     // bnk_wait watches *h_done for done_seq when done_watched: the last kernel of the submit stores it (Done)

@@ -159,3 +159,53 @@ def test_classify_and_gso_after_a_batch_without_copies(gpu_lib, oracle):
         b.close()
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("between", ["seal", "open", "upload", "note", "check", "classify", "classify all", "split"])
+def test_a_small_call_between_does_not_hide_what_is_behind(gpu_lib, oracle, between):
+    """1000 packets sealed in place, then a copied call for ten of the batch, then all of them from the device: the ring and
+    the descriptors that the device works on are those of the host arrays, beyond the ten too."""
+    from bnk_b200.device import F_NO_D2H, F_NO_H2D, F_USE_OUT_LEN, GSO_SUPER_DTYPE
+
+    n, few, size = 1000, 10, 300
+    rng = np.random.default_rng(3)
+    keys = rng.integers(0, 256, (2, 32), dtype=np.uint8)
+    c = _context(1 << 20, max_keypairs=8, mtu=1420, flow_capacity=16)
+    try:
+        c.set_keypairs(0, keys, keys, np.arange(2, dtype=np.uint32))
+        for p in range(2):
+            c.addr_set(bytes(10) + b"\xff\xff" + bytes([10, 0, 0, 1 + p]), 51820, p)
+        b = c.batch(n, n * 352)
+        b.off[:], b.len[:], b.slot[:], b.counter[:] = np.arange(n) * 352, size, rng.integers(0, 2, n), np.arange(n)
+        b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
+        b.src_addr[:, 10:12], b.src_addr[:, 12:16], b.src_addr[:, 16:18] = 255, (10, 0, 0, 2), (51820 >> 8, 51820 & 255)
+        plain = np.array(b.ring).reshape(n, 352)[:, 16:16 + size]
+        b.seal(n)
+        if between.startswith("classify"):
+            if between == "classify all":
+                slot = np.array(b.slot)
+                b.classify(n)  # in place: the device has no source addresses
+                b.slot[:] = slot
+                b.upload(few)
+            else:
+                b.classify(few, F_NO_D2H)
+        elif between == "split":
+            b.gso_split(np.zeros(0, GSO_SUPER_DTYPE), few)
+        elif between == "upload":
+            b.upload(few)
+        elif between == "note":
+            b.filter_note(few, 0, F_NO_D2H)
+        elif between == "check":
+            b.filter_check(few, 0, F_NO_D2H)
+        else:
+            getattr(b, between)(few, F_NO_D2H)
+        if between == "classify all":
+            b.classify(n, F_NO_H2D)
+            assert (b.slot == 1).all() and (b.status == 0).all()
+            return
+        b.open(n, F_NO_H2D | F_USE_OUT_LEN | F_NO_D2H)
+        b.download(n)
+        assert (b.status[few:] == 0).all() and (b.out_len[few:] == 304).all()
+        assert np.array_equal(b.ring.reshape(n, 352)[few:, 16:16 + size], plain[few:])
+    finally:
+        c.close()
