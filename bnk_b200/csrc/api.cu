@@ -93,7 +93,7 @@ uint64_t ring_extent(const bnk_batch *b, uint32_t n, uint32_t slack, uint64_t *b
 int begin_submit(bnk_batch *b, uint32_t npkts, bool touches_host = true) {
     if (!b) return BNK_EINVAL;
     if (npkts > b->max_pkts) return fail(b->ctx, BNK_EINVAL, "npkts exceeds the batch capacity");
-    if (b->in_flight && (touches_host || b->stale_pkts))
+    if (b->in_flight && touches_host)
         return fail(b->ctx, BNK_EBUSY, "batch has work in flight; call bnk_wait first");
     CK(b->ctx, cudaSetDevice(b->ctx->device));
     return BNK_SUCCESS;
@@ -331,7 +331,8 @@ cudaError_t ring_down(bnk_batch *b, uint32_t n, uint64_t ext, bool joint, cudaSt
 }
 
 // Brings the device copies up to the host arrays where submits have run on those.  An upload of as many packets with all
-// descriptor fields does the same.
+// descriptor fields does the same.  One of those submits may still be in flight, in front on this stream (a submit that
+// leaves the host arrays alone needs no wait in between): what is read here on the host, off[] and len[], no kernel writes.
 constexpr uint32_t kMostRoom = 16 + 16 + 16; // header, padding and tag around a payload
 cudaError_t catch_up(bnk_batch *b, cudaStream_t s) {
     const uint32_t n = b->stale_pkts;
