@@ -851,10 +851,7 @@ int bnk_batch_destroy(bnk_batch *b) {
     if (!b) return BNK_EINVAL;
     cudaSetDevice(b->ctx->device);
     submit_over(b);
-    if (b->flow_in_flight) {
-        std::lock_guard<std::mutex> g(b->ctx->flow_mu);
-        b->ctx->flow_in_flight--;
-    }
+    b->ctx->flow_bounds.over(b->flow_work, nullptr);
     {
         std::unique_lock<std::shared_mutex> tables(b->ctx->submit_mu); // not while table maintenance walks the registry
         std::lock_guard<std::mutex> g(b->ctx->mu);
@@ -1074,7 +1071,7 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
         }
     }
     const bool note = (flags & BNK_F_NOTE_OUTBOUND) && ctx->ft.enforce && ctx->ft.flow_capacity; // filter.go:192-194
-    const bool sweep = note && flow_note_begins(b, npkts, now_unix_ns);
+    const bool sweep = note && ctx->flow_bounds.note_begins(b->flow_work, npkts, now_unix_ns);
     const Done done = stats ? Done{} : watch_for(b);
     if (note) {
         a.note = true;
@@ -1118,7 +1115,7 @@ static int seal_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     a.res[0].counter = nullptr; // in place already
     a.behind_kernel = true;
     const bool note = (flags & BNK_F_NOTE_OUTBOUND) && ctx->ft.enforce && ctx->ft.flow_capacity; // filter.go:192-194
-    const bool sweep = note && flow_note_begins(b, npkts, now_unix_ns);
+    const bool sweep = note && ctx->flow_bounds.note_begins(b->flow_work, npkts, now_unix_ns);
     if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
     for (bool more = true; more;) {
         CK(ctx, piece_is_up(b, s));
@@ -1170,7 +1167,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     CK(ctx, order_kernels_begin(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     if ((flags & BNK_F_NOTE_OUTBOUND) && n && ctx->ft.enforce && ctx->ft.flow_capacity) { // filter.go:192-194
-        const bool sweep = flow_note_begins(b, npkts, now_unix_ns);
+        const bool sweep = ctx->flow_bounds.note_begins(b->flow_work, npkts, now_unix_ns);
         CK(ctx, launch_filter_note(b, 0, npkts, now_unix_ns, Done{}, s));
         if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, Done{}, s));
         else CK(ctx, launch_flow_report(b, s));
@@ -1280,7 +1277,7 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
         v.n = npkts;
         v.inner_check = (flags & BNK_F_INNER_CHECK) != 0;
         v.check_inbound = (flags & BNK_F_CHECK_INBOUND) != 0;
-        if (v.check_inbound) flow_check_begins(b, now_unix_ns);
+        if (v.check_inbound) ctx->flow_bounds.check_begins(b->flow_work, now_unix_ns);
         if (one_launch) {
             v.host_status = h.status;
             v.host_out_len = h.out_len;
@@ -1333,7 +1330,7 @@ static int open_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     }
     if (flags & BNK_F_INNER_CHECK) CK(ctx, launch_inner_check(b, npkts, s));
     if (flags & BNK_F_CHECK_INBOUND) {
-        flow_check_begins(b, now_unix_ns);
+        ctx->flow_bounds.check_begins(b->flow_work, now_unix_ns);
         CK(ctx, launch_filter_check(b, npkts, now_unix_ns, true, nullptr, Done{}, s));
     }
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
@@ -1411,7 +1408,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     }
     if (flags & BNK_F_INNER_CHECK) CK(ctx, launch_inner_check(b, npkts, s));
     if (flags & BNK_F_CHECK_INBOUND) {
-        flow_check_begins(b, now_unix_ns);
+        ctx->flow_bounds.check_begins(b->flow_work, now_unix_ns);
         CK(ctx, launch_filter_check(b, npkts, now_unix_ns, true, nullptr, Done{}, s));
     }
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
@@ -1471,7 +1468,7 @@ int bnk_filter_note_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t
     const bool note = npkts && ctx->ft.enforce && ctx->ft.flow_capacity; // filter.go:192-194
     bool reported = false;
     if (note) {
-        const bool sweep = flow_note_begins(b, npkts, now_unix_ns);
+        const bool sweep = ctx->flow_bounds.note_begins(b->flow_work, npkts, now_unix_ns);
         const Done done = watch_for(b);
         CK(ctx, launch_filter_note(b, 0, npkts, now_unix_ns, sweep ? Done{} : done, s));
         if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, done, s));
@@ -1496,7 +1493,7 @@ int bnk_filter_check_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_
     if (!direct && upload && (rc = upload_heads(b, npkts, s)) != BNK_SUCCESS) return rc;
     HostAlias alias(b, direct, npkts);
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
-    flow_check_begins(b, now_unix_ns);
+    ctx->flow_bounds.check_begins(b->flow_work, now_unix_ns);
     const bool to_host = !(flags & BNK_F_NO_D2H);
     const Done done = to_host && npkts && !(flags & BNK_F_STATS) ? watch_for(b) : Done{};
     uint8_t *const host_status = to_host ? b->host.status : nullptr;
@@ -1649,7 +1646,7 @@ int bnk_wait(bnk_batch *b, uint64_t timeout_ns) {
         }
     }
     submit_over(b);
-    if (b->flow_in_flight || b->flow_reported) flow_work_over(b);
+    if (b->flow_work.on) ctx->flow_bounds.over(b->flow_work, b->flow_reported ? b->h_flow : nullptr);
     if (b->flow_reported) { // what the device said about the flow table after this batch: input of the next compaction
         b->flow_reported = false;
         for (int c = 0; c < 3; c++) ctx->flow_dead_hint[c] = b->h_flow->dead[c];

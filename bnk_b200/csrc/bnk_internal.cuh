@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/bnk_gpu.h"
+#include "flow_bounds.h"
 
 // ---------------------------------------------------------------------------
 // Device-resident tables of one context (one GPU).  All per-peer mutable state
@@ -93,15 +94,6 @@ struct FilterTables {
 __host__ __device__ inline size_t flow_region(const FilterTables &ft, int cls) {
     return ((size_t)cls * 2 + ft.flow_half[cls]) * ft.flow_capacity;
 }
-// What a batch's filter work reports back to the host next to the packets (pinned, one per batch).
-struct FlowReport {
-    unsigned long long live; // len(f.flows)
-    long long floor;         // no entry's expiry lies below this
-    int error;               // inserts that found no free slot, since the table was last cleared
-    uint32_t used[3];        // slots of the class's region that hold a key, live or deleted
-    uint32_t dead[3];        // of those, deleted ones (reclaimed by compaction)
-};
-
 class CopyCrew;
 struct bnk_ctx {
     bnk_cfg cfg;
@@ -129,14 +121,7 @@ struct bnk_ctx {
     std::vector<bnk_batch *> batches;       // every live batch of the context (guarded by mu)
     std::shared_ptr<CopyCrew> crew;         // helpers of its queues' copies, made with the first queue (guarded by mu)
     std::atomic<uint32_t> flow_dead_hint[3]; // deleted entries per class as last reported by the device
-    // What the host knows about the flow table without asking: no entry expires before flow_floor, at most
-    // flow_live_most are live.  Every submit with filter work widens them; a report of the device replaces them
-    // unless another such submit has been made since (flow_epoch) or is under way.
-    std::mutex flow_mu;
-    long long flow_floor = 0;
-    uint64_t flow_live_most = 0;
-    uint32_t flow_epoch = 0;
-    int flow_in_flight = 0; // batches whose filter work has not been waited for
+    FlowBounds flow_bounds;
     std::atomic<int> flow_errors_seen;       // failed inserts already reported to a caller as BNK_EFULL
     // rule table: two device buffer sets, the one not in use receives the next upload
     struct RuleSet {
@@ -218,8 +203,7 @@ struct bnk_batch {
     bool joint_copy;   // descriptors and ring move as one copy
     FlowReport *h_flow; // pinned copy of the flow table's state after the batch's filter work
     bool stats_pending; // the last submit was made with BNK_F_STATS
-    uint32_t flow_epoch; // ctx->flow_epoch of the last submit with filter work
-    bool flow_in_flight; // this batch is one of ctx->flow_in_flight
+    FlowWork flow_work; // its filter work that has not been waited for
     bool flow_reported; // the last submit queued a copy of the flow table's state into h_flow
     bnk_batch_stats *h_stats; // pinned; written by the tally kernel
     unsigned long long *d_stats; // device accumulators of the tally kernel (zero between launches)
@@ -401,11 +385,6 @@ cudaError_t filter_flow_stats(bnk_ctx *ctx, uint64_t *live, uint32_t used[3], ui
 int filter_flows_export(bnk_ctx *ctx, bnk_flow_entry *out, size_t capacity, size_t *count);
 int filter_flows_import(bnk_ctx *ctx, const bnk_flow_entry *entries, size_t n);
 cudaError_t launch_flow_report(bnk_batch *b, cudaStream_t s); // copies the flow table's control block to b->h_flow
-// A submit is about to record up to n flows at `now` / to check packets at `now`.  The former returns whether the
-// batch may have to sweep expired flows behind its inserts (launch_flow_sweep).
-bool flow_note_begins(bnk_batch *b, uint32_t n, long long now);
-void flow_check_begins(bnk_batch *b, long long now);
-void flow_work_over(bnk_batch *b); // the batch has been waited for; its report, if it made one, is in b->h_flow
 cudaError_t launch_flow_sweep(bnk_batch *b, long long now, const Done &done, cudaStream_t s);
 // Rebuilds the regions whose deleted entries have piled up; called by a submit that feeds the flow table,
 // before it takes submit_mu.  Returns without doing anything in the common case.

@@ -19,8 +19,8 @@ __host__ __device__ __forceinline__ bool flow_absent(long long exp) { return exp
 constexpr long long TTL_UDP = 30ll * 1000000000ll;  // filter.go:19
 constexpr long long TTL_TCP = 120ll * 1000000000ll; // filter.go:20
 constexpr long long TTL_ICMP = 30ll * 1000000000ll; // filter.go:21
-constexpr long long TTL_LEAST = TTL_UDP;
-constexpr unsigned long long SWEEP_THRESHOLD = 4096; // filter.go:202
+constexpr long long TTL_LEAST = FlowBounds::kTtlLeast;
+constexpr unsigned long long SWEEP_THRESHOLD = FlowBounds::kSweepThreshold;
 
 // small device-side control block behind FilterTables::flow_live
 struct FlowCtl {

@@ -311,12 +311,7 @@ cudaError_t filter_flows_clear(bnk_ctx *ctx, cudaStream_t s) {
     ctx->ft.flow_half[0] = ctx->ft.flow_half[1] = ctx->ft.flow_half[2] = 0;
     for (auto &h : ctx->flow_dead_hint) h = 0;
     ctx->flow_errors_seen = 0;
-    {
-        std::lock_guard<std::mutex> g(ctx->flow_mu);
-        ctx->flow_floor = LLONG_MAX;
-        ctx->flow_live_most = 0;
-        ctx->flow_epoch++;
-    }
+    ctx->flow_bounds.set(LLONG_MAX, 0);
     flows_fill_kernel<<<ctx->sm_count * 4, 256, 0, s>>>(ctx->ft);
     ctx->launches += 1;
     cudaError_t e = cudaGetLastError();
@@ -423,12 +418,7 @@ int filter_flows_import(bnk_ctx *ctx, const bnk_flow_entry *entries, size_t n) {
         if (!placed) return BNK_EFULL;
     }
     h.ctl.rep.floor = LLONG_MIN; // unknown: the next sweep finds it
-    {
-        std::lock_guard<std::mutex> g(ctx->flow_mu);
-        ctx->flow_floor = LLONG_MIN;
-        ctx->flow_live_most = h.ctl.rep.live;
-        ctx->flow_epoch++;
-    }
+    ctx->flow_bounds.set(LLONG_MIN, h.ctl.rep.live);
     const size_t total = (size_t)6 * cap;
     cudaError_t e = cudaSuccess;
     if (total) e = cudaMemcpy(ft.flow_slots, h.slots.data(), total * sizeof(FlowSlot), cudaMemcpyHostToDevice);
@@ -443,36 +433,6 @@ cudaError_t launch_flow_report(bnk_batch *b, cudaStream_t s) {
     return cudaMemcpyAsync(b->h_flow, &ctl->rep, sizeof(FlowReport), cudaMemcpyDeviceToHost, s);
 }
 
-static long long earliest_expiry(long long now) { return now > LLONG_MAX - TTL_LEAST ? LLONG_MAX : now + TTL_LEAST; }
-static void flow_work_begins(bnk_batch *b) {
-    b->flow_epoch = ++b->ctx->flow_epoch;
-    if (!b->flow_in_flight) b->ctx->flow_in_flight++;
-    b->flow_in_flight = true;
-}
-bool flow_note_begins(bnk_batch *b, uint32_t n, long long now) {
-    bnk_ctx *ctx = b->ctx;
-    std::lock_guard<std::mutex> g(ctx->flow_mu);
-    flow_work_begins(b);
-    ctx->flow_live_most += n;
-    const bool sweep = ctx->flow_live_most > SWEEP_THRESHOLD && now > ctx->flow_floor;
-    ctx->flow_floor = std::min(ctx->flow_floor, earliest_expiry(now));
-    return sweep;
-}
-void flow_check_begins(bnk_batch *b, long long now) { // a lookup keeps its flow alive: it writes an expiry too
-    bnk_ctx *ctx = b->ctx;
-    std::lock_guard<std::mutex> g(ctx->flow_mu);
-    flow_work_begins(b);
-    ctx->flow_floor = std::min(ctx->flow_floor, earliest_expiry(now));
-}
-void flow_work_over(bnk_batch *b) {
-    bnk_ctx *ctx = b->ctx;
-    std::lock_guard<std::mutex> g(ctx->flow_mu);
-    if (b->flow_in_flight) ctx->flow_in_flight--;
-    b->flow_in_flight = false;
-    if (!b->flow_reported || ctx->flow_epoch != b->flow_epoch || ctx->flow_in_flight != 0) return;
-    ctx->flow_floor = b->h_flow->floor;
-    ctx->flow_live_most = b->h_flow->live;
-}
 cudaError_t launch_flow_sweep(bnk_batch *b, long long now, const Done &done, cudaStream_t s) {
     bnk_ctx *ctx = b->ctx;
     const size_t slots = (size_t)3 * ctx->ft.flow_capacity;
