@@ -490,6 +490,7 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     };
     if ((e = cudaStreamCreateWithFlags(&ctx->admin_stream, cudaStreamNonBlocking)) != cudaSuccess) return bail("stream", e);
     if ((e = cudaEventCreate(&ctx->timer_start)) != cudaSuccess) return bail("event", e);
+    if ((e = cudaEventCreateWithFlags(&ctx->ev_sweep, cudaEventDisableTiming)) != cudaSuccess) return bail("event", e);
     Slab tables;
     tables.add(&ctx->kt.send_keys, k * 8);
     tables.add(&ctx->kt.recv_keys, k * 8);
@@ -528,6 +529,7 @@ int bnk_ctx_destroy(bnk_ctx *ctx) {
     cudaFree(ctx->kt.send_keys); // all of the tables' arrays
     filter_tables_free(ctx);
     if (ctx->timer_start) cudaEventDestroy(ctx->timer_start);
+    if (ctx->ev_sweep) cudaEventDestroy(ctx->ev_sweep);
     if (ctx->admin_stream) cudaStreamDestroy(ctx->admin_stream);
     delete ctx;
     return BNK_SUCCESS;
@@ -1071,7 +1073,8 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
         }
     }
     const bool note = (flags & BNK_F_NOTE_OUTBOUND) && ctx->ft.enforce && ctx->ft.flow_capacity; // filter.go:192-194
-    const bool sweep = note && ctx->flow_bounds.note_begins(b->flow_work, npkts, now_unix_ns);
+    bool sweep = false;
+    if (note) CK(ctx, flow_note_begins(b, npkts, now_unix_ns, s, sweep));
     const Done done = stats ? Done{} : watch_for(b);
     if (note) {
         a.note = true;
@@ -1115,7 +1118,8 @@ static int seal_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     a.res[0].counter = nullptr; // in place already
     a.behind_kernel = true;
     const bool note = (flags & BNK_F_NOTE_OUTBOUND) && ctx->ft.enforce && ctx->ft.flow_capacity; // filter.go:192-194
-    const bool sweep = note && ctx->flow_bounds.note_begins(b->flow_work, npkts, now_unix_ns);
+    bool sweep = false;
+    if (note) CK(ctx, flow_note_begins(b, npkts, now_unix_ns, s, sweep));
     if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
     for (bool more = true; more;) {
         CK(ctx, piece_is_up(b, s));
@@ -1167,7 +1171,8 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     CK(ctx, order_kernels_begin(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     if ((flags & BNK_F_NOTE_OUTBOUND) && n && ctx->ft.enforce && ctx->ft.flow_capacity) { // filter.go:192-194
-        const bool sweep = ctx->flow_bounds.note_begins(b->flow_work, npkts, now_unix_ns);
+        bool sweep;
+        CK(ctx, flow_note_begins(b, npkts, now_unix_ns, s, sweep));
         CK(ctx, launch_filter_note(b, 0, npkts, now_unix_ns, Done{}, s));
         if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, Done{}, s));
         else CK(ctx, launch_flow_report(b, s));
@@ -1277,7 +1282,7 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
         v.n = npkts;
         v.inner_check = (flags & BNK_F_INNER_CHECK) != 0;
         v.check_inbound = (flags & BNK_F_CHECK_INBOUND) != 0;
-        if (v.check_inbound) ctx->flow_bounds.check_begins(b->flow_work, now_unix_ns);
+        if (v.check_inbound) CK(ctx, flow_check_begins(b, now_unix_ns, s));
         if (one_launch) {
             v.host_status = h.status;
             v.host_out_len = h.out_len;
@@ -1330,7 +1335,7 @@ static int open_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     }
     if (flags & BNK_F_INNER_CHECK) CK(ctx, launch_inner_check(b, npkts, s));
     if (flags & BNK_F_CHECK_INBOUND) {
-        ctx->flow_bounds.check_begins(b->flow_work, now_unix_ns);
+        CK(ctx, flow_check_begins(b, now_unix_ns, s));
         CK(ctx, launch_filter_check(b, npkts, now_unix_ns, true, nullptr, Done{}, s));
     }
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
@@ -1408,7 +1413,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     }
     if (flags & BNK_F_INNER_CHECK) CK(ctx, launch_inner_check(b, npkts, s));
     if (flags & BNK_F_CHECK_INBOUND) {
-        ctx->flow_bounds.check_begins(b->flow_work, now_unix_ns);
+        CK(ctx, flow_check_begins(b, now_unix_ns, s));
         CK(ctx, launch_filter_check(b, npkts, now_unix_ns, true, nullptr, Done{}, s));
     }
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
@@ -1468,7 +1473,8 @@ int bnk_filter_note_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t
     const bool note = npkts && ctx->ft.enforce && ctx->ft.flow_capacity; // filter.go:192-194
     bool reported = false;
     if (note) {
-        const bool sweep = ctx->flow_bounds.note_begins(b->flow_work, npkts, now_unix_ns);
+        bool sweep;
+        CK(ctx, flow_note_begins(b, npkts, now_unix_ns, s, sweep));
         const Done done = watch_for(b);
         CK(ctx, launch_filter_note(b, 0, npkts, now_unix_ns, sweep ? Done{} : done, s));
         if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, done, s));
@@ -1493,7 +1499,7 @@ int bnk_filter_check_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_
     if (!direct && upload && (rc = upload_heads(b, npkts, s)) != BNK_SUCCESS) return rc;
     HostAlias alias(b, direct, npkts);
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
-    ctx->flow_bounds.check_begins(b->flow_work, now_unix_ns);
+    CK(ctx, flow_check_begins(b, now_unix_ns, s));
     const bool to_host = !(flags & BNK_F_NO_D2H);
     const Done done = to_host && npkts && !(flags & BNK_F_STATS) ? watch_for(b) : Done{};
     uint8_t *const host_status = to_host ? b->host.status : nullptr;

@@ -122,6 +122,10 @@ struct bnk_ctx {
     std::shared_ptr<CopyCrew> crew;         // helpers of its queues' copies, made with the first queue (guarded by mu)
     std::atomic<uint32_t> flow_dead_hint[3]; // deleted entries per class as last reported by the device
     FlowBounds flow_bounds;
+    // Sweeps of the flow table run one behind the other, and work with an older clock than one of them behind it.
+    std::mutex sweep_mu;
+    cudaEvent_t ev_sweep;                  // behind the last one
+    std::atomic<long long> sweep_now;      // latest clock of any
     std::atomic<int> flow_errors_seen;       // failed inserts already reported to a caller as BNK_EFULL
     // rule table: two device buffer sets, the one not in use receives the next upload
     struct RuleSet {
@@ -385,6 +389,10 @@ cudaError_t filter_flow_stats(bnk_ctx *ctx, uint64_t *live, uint32_t used[3], ui
 int filter_flows_export(bnk_ctx *ctx, bnk_flow_entry *out, size_t capacity, size_t *count);
 int filter_flows_import(bnk_ctx *ctx, const bnk_flow_entry *entries, size_t n);
 cudaError_t launch_flow_report(bnk_batch *b, cudaStream_t s); // copies the flow table's control block to b->h_flow
+// A submit is about to record up to n flows at `now` / to check packets at `now`, on stream s.  The former says whether the
+// batch may have to sweep expired flows behind its inserts (launch_flow_sweep).
+cudaError_t flow_note_begins(bnk_batch *b, uint32_t n, long long now, cudaStream_t s, bool &sweep);
+cudaError_t flow_check_begins(bnk_batch *b, long long now, cudaStream_t s);
 cudaError_t launch_flow_sweep(bnk_batch *b, long long now, const Done &done, cudaStream_t s);
 // Rebuilds the regions whose deleted entries have piled up; called by a submit that feeds the flow table,
 // before it takes submit_mu.  Returns without doing anything in the common case.

@@ -28,6 +28,7 @@ struct FlowCtl {
     unsigned long long dropped; // entries the sweep under way has deleted
     long long next_floor;       // lowest expiry it has left
     uint32_t ticket;            // CTAs of the sweep that have finished
+    uint32_t decided;           // 2: the sweep under way walks the table, 1: it does not, 0: no CTA has looked yet
     uint32_t moved;             // entries a compaction has re-inserted so far
 };
 __device__ __forceinline__ FlowCtl *flow_ctl(const FilterTables &ft) { return reinterpret_cast<FlowCtl *>(ft.flow_live); }
@@ -275,8 +276,8 @@ struct FlowReply {
             flow_keep_floor(ctl, fresh, ctl->rep.floor);
             return BNK_PKT_OK;
         }
-        const long long prev = (long long)atomicExch((unsigned long long *)place, (unsigned long long)FLOW_DEAD);
-        if (!flow_absent(prev)) {
+        // (not if another batch has recorded the flow again meanwhile)
+        if ((long long)atomicCAS((unsigned long long *)place, (unsigned long long)exp, (unsigned long long)FLOW_DEAD) == exp) {
             atomicAdd(&ctl->rep.live, 0ull - 1ull);
             if (key != FLOW_EMPTY) atomicAdd(&ctl->rep.dead[cls], 1u);
         }

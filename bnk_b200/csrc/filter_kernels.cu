@@ -58,23 +58,28 @@ __global__ void __launch_bounds__(128) filter_note_kernel(const __grid_constant_
 // (one `now`) that equals: insert everything, then sweep once if the count exceeds the threshold.  A sweep that
 // starts at or before the floor of the expiries would find nothing and does not walk the table; the host, which
 // knows a lower bound of the floor, does not even launch it (flow_note_begins).  One walk reads the expiries of the
-// regions in use and leaves the floor at the lowest expiry it has seen, or at what an insert that
-// ran beside it can have written.
-__global__ void __launch_bounds__(256) filter_sweep_kernel(const __grid_constant__ FilterTables ft, long long now, FlowReport *report, Done done) {
+// regions in use and leaves the floor at the lowest expiry it has seen, or at `beside`, which is what inserts and lookups
+// that run beside it write at least.  Sweeps never run side by side (launch_flow_sweep); inserts and lookups may, so an
+// entry is dropped only if it still is the one that was looked at.
+__global__ void __launch_bounds__(256) filter_sweep_kernel(const __grid_constant__ FilterTables ft, long long now, long long beside,
+                                                           FlowReport *report, Done done) {
     let_next_kernel_start();
     wait_for_kernel_in_front();
     FlowCtl *const ctl = flow_ctl(ft);
     __shared__ unsigned long long dropped_s;
     __shared__ long long floor_s;
     __shared__ uint32_t dead_s[3];
-    if (threadIdx.x == 0) {
+    __shared__ bool walk_s;
+    if (threadIdx.x == 0) { // the first CTA to look decides for all: others insert and count meanwhile
+        const uint32_t mine = *(volatile unsigned long long *)&ctl->rep.live > SWEEP_THRESHOLD && now > flow_floor(ctl) ? 2u : 1u;
+        const uint32_t first = atomicCAS(&ctl->decided, 0u, mine);
+        walk_s = (first ? first : mine) == 2u;
         dropped_s = 0;
         floor_s = LLONG_MAX;
         dead_s[0] = dead_s[1] = dead_s[2] = 0;
     }
     __syncthreads();
-    // all CTAs decide alike: neither value changes before the last of them has finished
-    const bool walk = ctl->rep.live > SWEEP_THRESHOLD && now > ctl->rep.floor;
+    const bool walk = walk_s;
     if (walk) {
         const size_t cap = ft.flow_capacity, total = 3 * cap;
         unsigned long long dropped = 0;
@@ -85,7 +90,7 @@ __global__ void __launch_bounds__(256) filter_sweep_kernel(const __grid_constant
             const long long exp = *e;
             if (flow_absent(exp)) continue;
             if (now > exp) {
-                *e = FLOW_DEAD;
+                if ((long long)atomicCAS((unsigned long long *)e, (unsigned long long)exp, (unsigned long long)FLOW_DEAD) != exp) continue;
                 dropped++;
                 if (k < total) atomicAdd(&dead_s[cls], 1u);
             } else if (exp < floor) {
@@ -108,12 +113,12 @@ __global__ void __launch_bounds__(256) filter_sweep_kernel(const __grid_constant
             __threadfence();
             if (walk) {
                 atomicAdd(&ctl->rep.live, 0ull - *(volatile unsigned long long *)&ctl->dropped);
-                const long long seen = *(volatile long long *)&ctl->next_floor, beside = now + TTL_LEAST;
+                const long long seen = *(volatile long long *)&ctl->next_floor;
                 ctl->rep.floor = seen < beside ? seen : beside;
                 ctl->dropped = 0;
                 ctl->next_floor = LLONG_MAX;
             }
-            ctl->ticket = 0;
+            ctl->ticket = ctl->decided = 0;
             __threadfence();
             if (report) flow_report(ctl, report);
             if (done.flag) {
@@ -312,6 +317,7 @@ cudaError_t filter_flows_clear(bnk_ctx *ctx, cudaStream_t s) {
     for (auto &h : ctx->flow_dead_hint) h = 0;
     ctx->flow_errors_seen = 0;
     ctx->flow_bounds.set(LLONG_MAX, 0);
+    ctx->sweep_now = LLONG_MIN;
     flows_fill_kernel<<<ctx->sm_count * 4, 256, 0, s>>>(ctx->ft);
     ctx->launches += 1;
     cudaError_t e = cudaGetLastError();
@@ -433,13 +439,38 @@ cudaError_t launch_flow_report(bnk_batch *b, cudaStream_t s) {
     return cudaMemcpyAsync(b->h_flow, &ctl->rep, sizeof(FlowReport), cudaMemcpyDeviceToHost, s);
 }
 
+// Who has a clock behind that of a sweep waits for it.  (Clocks rise but for the order in which threads come by, so this is
+// rare.)  Looked at behind flow_bounds' entry: a sweep that does not see that has left its clock here before.
+static cudaError_t behind_newer_sweep(bnk_ctx *ctx, long long now, cudaStream_t s) {
+    if (now >= ctx->sweep_now.load()) return cudaSuccess;
+    std::lock_guard<std::mutex> g(ctx->sweep_mu); // its event is recorded
+    return cudaStreamWaitEvent(s, ctx->ev_sweep, 0);
+}
+cudaError_t flow_note_begins(bnk_batch *b, uint32_t n, long long now, cudaStream_t s, bool &sweep) {
+    sweep = b->ctx->flow_bounds.note_begins(b->flow_work, n, now);
+    return behind_newer_sweep(b->ctx, now, s);
+}
+cudaError_t flow_check_begins(bnk_batch *b, long long now, cudaStream_t s) {
+    b->ctx->flow_bounds.check_begins(b->flow_work, now);
+    return behind_newer_sweep(b->ctx, now, s);
+}
 cudaError_t launch_flow_sweep(bnk_batch *b, long long now, const Done &done, cudaStream_t s) {
     bnk_ctx *ctx = b->ctx;
+    std::lock_guard<std::mutex> g(ctx->sweep_mu);
+    const long long latest = ctx->sweep_now.load();
+    if (latest != LLONG_MIN) {
+        const cudaError_t e = cudaStreamWaitEvent(s, ctx->ev_sweep, 0);
+        if (e != cudaSuccess) return e;
+    }
+    ctx->sweep_now.store(std::max(latest, now));
+    const long long beside = ctx->flow_bounds.beside(now);
     const size_t slots = (size_t)3 * ctx->ft.flow_capacity;
     const uint32_t grid = (uint32_t)std::min<size_t>(ctx->sm_count * 4, (slots + 1023) / 1024);
     b->flow_reported = true;
     ctx->launches += 1;
-    return launch_after_kernel(filter_sweep_kernel, dim3(grid), dim3(256), s, ctx->ft, now, b->h_flow, done);
+    const cudaError_t e = launch_after_kernel(filter_sweep_kernel, dim3(grid), dim3(256), s, ctx->ft, now, beside, b->h_flow, done);
+    const cudaError_t r = cudaEventRecord(ctx->ev_sweep, s);
+    return e != cudaSuccess ? e : r;
 }
 
 // Deleted entries keep their slots, so a class whose flows come and go (every connection brings a new source

@@ -27,6 +27,7 @@ struct FlowReport {
 // A batch's filter work between its submit and its wait (zero to start with).
 struct FlowWork {
     FlowWork *next;
+    long long now; // lowest clock of its submits
     bool on, notes;
 };
 
@@ -40,7 +41,7 @@ class FlowBounds {
     // to be swept behind its inserts.
     bool note_begins(FlowWork &w, uint32_t n, long long now) {
         std::lock_guard<std::mutex> g(mu_);
-        begins(w);
+        begins(w, now);
         w.notes = true;
         live_most_ += n;
         const bool sweep = live_most_ > kSweepThreshold && now > floor_;
@@ -49,9 +50,15 @@ class FlowBounds {
     }
     void check_begins(FlowWork &w, long long now) { // a lookup keeps its flow alive: it writes an expiry too
         std::lock_guard<std::mutex> g(mu_);
-        begins(w);
+        begins(w, now);
         floor_ = std::min(floor_, earliest(now));
         group_floor_ = std::min(group_floor_, earliest(now));
+    }
+    // Lowest expiry that work in flight beside a sweep at `now` can write.
+    long long beside(long long now) {
+        std::lock_guard<std::mutex> g(mu_);
+        for (const FlowWork *w = first_; w; w = w->next) now = std::min(now, w->now);
+        return earliest(now);
     }
     // The batch has been waited for; `report` (may be null) was taken behind all of its work.
     void over(FlowWork &w, const FlowReport *report) {
@@ -94,10 +101,12 @@ class FlowBounds {
         group_floor_ = LLONG_MAX;
         group_reported_ = group_lost_ = false;
     }
-    void begins(FlowWork &w) {
-        if (w.on) return;
-        w = FlowWork{first_, true, false};
-        first_ = &w;
+    void begins(FlowWork &w, long long now) {
+        if (!w.on) {
+            w = FlowWork{first_, now, true, false};
+            first_ = &w;
+        }
+        w.now = std::min(w.now, now);
     }
     std::mutex mu_;
     FlowWork *first_ = nullptr; // in flight

@@ -308,3 +308,64 @@ def test_batch_counters_equal_a_count_of_the_statuses(gpu_lib, oracle, n):
         b.close()
     finally:
         c.close()
+
+
+# ---------------------------------------------------------------------------------------------
+# sweeps beside other work
+# ---------------------------------------------------------------------------------------------
+def _flow_headers(first, n):
+    from bnk_b200 import gen
+
+    k = first + np.arange(n, dtype=np.uint64)
+    return gen._headers(np.full(n, 17, np.uint8), np.full(n, gen.ip4(100, 64, 0, 1), np.uint64), (np.uint64(1 << 30) + (k >> np.uint64(15))),
+                        np.full(n, 53, np.uint64), np.uint64(1) + (k & np.uint64(0x7fff)))
+
+
+def _flow_batch(c, first, n):
+    b = c.batch(n, n * 48)
+    b.ring.reshape(n, 48)[:, 16:44] = _flow_headers(first, n)
+    b.off[:], b.len[:] = np.arange(n) * 48, 28
+    return b
+
+
+def test_sweeps_of_two_batches_in_flight_count_every_entry_once(gpu_lib):
+    from bnk_b200 import Context
+
+    sec = 10**9
+    with Context(max_keypairs=1, flow_capacity=1 << 22) as c:  # a walk takes longer than the next submit
+        c.acl_set(True, None)
+        seed, a, b = _flow_batch(c, 0, 60_000), _flow_batch(c, 100_000, 1), _flow_batch(c, 200_000, 1)
+        for turn in range(12):
+            now = RC.T0 + turn * 100 * sec
+            c.flows_clear()
+            seed.filter_note(60_000, now)
+            a.filter_note(1, now + 31 * sec, wait=False)
+            b.filter_note(1, now + 32 * sec, wait=False)
+            (a if turn % 2 else b).wait()
+            a.wait()
+            b.wait()
+            assert len(c.flows_export()) == 2 and c.flows_count() == 2, (turn, c.flows_count(), len(c.flows_export()))
+
+
+def test_flows_of_an_older_clock_beside_a_sweep_expire_in_time(gpu_lib):
+    """A batch whose clock lies behind that of a sweep under way: its flows, gone by their own clock, are swept when that
+    has passed, in whatever order the two ran."""
+    from bnk_b200 import Context
+
+    sec = 10**9
+    with Context(max_keypairs=1, flow_capacity=1 << 20) as c:
+        c.acl_set(True, None)
+        seed, late, sweep, after = _flow_batch(c, 0, 20_000), _flow_batch(c, 50_000, 6000), _flow_batch(c, 100_000, 1), _flow_batch(c, 200_000, 1)
+        for turn in range(16):
+            now = RC.T0 + turn * 1000 * sec
+            c.flows_clear()
+            seed.filter_note(20_000, now)
+            first, second = (sweep, late) if turn % 2 else (late, sweep)
+            for b in (first, second):
+                b.filter_note(len(b.off), now + (60 if b is sweep else 40) * sec, wait=False)
+            (second if turn % 4 < 2 else first).wait()
+            late.wait()
+            sweep.wait()
+            assert len(c.flows_export()) == c.flows_count() == 6001, turn
+            after.filter_note(1, now + 80 * sec)  # the 6000 went at + 70
+            assert len(c.flows_export()) == c.flows_count() == 2, (turn, c.flows_count())
