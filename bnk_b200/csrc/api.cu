@@ -543,6 +543,11 @@ int bnk_ctx_synchronize(bnk_ctx *ctx) {
 }
 
 /* ---- keypairs ---- */
+// cudaMemset returns before the memory is set, and the batches' streams do not wait for the default stream.
+static int memsets_over(bnk_ctx *ctx) {
+    CK(ctx, cudaStreamSynchronize(cudaStreamLegacy));
+    return BNK_SUCCESS;
+}
 int bnk_keypair_set_many(bnk_ctx *ctx, uint32_t first_slot, uint32_t n, const uint8_t *send_keys,
                          const uint8_t *recv_keys, const uint32_t *remote_index) {
     if (!ctx || !send_keys || !recv_keys || !remote_index) return fail(ctx, BNK_EINVAL, "null argument");
@@ -558,7 +563,7 @@ int bnk_keypair_set_many(bnk_ctx *ctx, uint32_t first_slot, uint32_t n, const ui
     CK(ctx, cudaMemset(ctx->kt.replay_ring + (size_t)first_slot * rb, 0, (size_t)n * rb * 8));
     CK(ctx, cudaMemset(ctx->kt.allowed_ip + first_slot, 0, (size_t)n * 4));
     CK(ctx, cudaMemset(ctx->kt.valid + first_slot, 1, (size_t)n));
-    return BNK_SUCCESS;
+    return memsets_over(ctx);
 }
 
 int bnk_keypair_set(bnk_ctx *ctx, uint32_t slot, const uint8_t send_key[32], const uint8_t recv_key[32],
@@ -574,7 +579,8 @@ int bnk_keypair_clear(bnk_ctx *ctx, uint32_t slot) {
     if (rc != BNK_SUCCESS) return rc;
     // no keys: seal and open refuse the slot with BNK_PKT_NO_KEYPAIR, and no receiver index leads to it any more
     CK(ctx, cudaMemset(ctx->kt.valid + slot, 0, 1));
-    return index_drop_slot(ctx, slot);
+    rc = memsets_over(ctx);
+    return rc != BNK_SUCCESS ? rc : index_drop_slot(ctx, slot);
 }
 
 int bnk_send_counter_get(bnk_ctx *ctx, uint32_t slot, uint64_t *counter) {

@@ -310,6 +310,27 @@ def test_batch_counters_equal_a_count_of_the_statuses(gpu_lib, oracle, n):
         c.close()
 
 
+def test_keypairs_are_in_place_when_the_call_returns(gpu_lib):
+    """A submit right behind bnk_keypair_set_many finds all of the slots' state set, however much of it there is."""
+    from bnk_b200 import Context
+    from bnk_b200.device import F_ASSIGN_COUNTERS, PKT_NO_KEYPAIR
+
+    n = 65_536
+    keys = np.random.default_rng(1).integers(0, 256, (n, 32), dtype=np.uint8)
+    index = np.zeros(n, np.uint32)
+    with Context(max_keypairs=n, mtu=1420, flow_capacity=0, replay_ring_blocks=1024) as c:
+        b = c.batch(1, 2048)
+        for turn in range(5):
+            b.off[0], b.len[0], b.slot[0] = 0, 64, n - 1
+            c.set_keypairs(0, keys, keys, index)
+            b.seal(1, F_ASSIGN_COUNTERS)
+            assert (b.status[0], b.counter[0]) == (0, 0), turn
+            c.set_send_counter(n - 1, 7)
+            c.clear_keypair(n - 1)
+            b.seal(1, F_ASSIGN_COUNTERS)
+            assert b.status[0] == PKT_NO_KEYPAIR
+
+
 # ---------------------------------------------------------------------------------------------
 # sweeps beside other work
 # ---------------------------------------------------------------------------------------------
