@@ -232,6 +232,7 @@ class Pieces {
 constexpr uint32_t kManySmall = 10240, kSmallBytes = 512;
 bool in_pieces(const bnk_batch *b, uint32_t n, uint32_t flags, uint64_t ext, bool in_order) {
     const uint64_t from = b->ctx->pieces_from;
+    if (n == 0) return false;
     if (ext < from && (n < kManySmall || ext > (uint64_t)n * kSmallBytes || ext < from / 16)) return false;
     return in_order && b->up_stream && !(flags & (BNK_F_NO_H2D | BNK_F_NO_D2H | BNK_F_USE_OUT_LEN)) &&
            b->ctx->in_flight.load(std::memory_order_relaxed) == (b->counted ? 1 : 0);

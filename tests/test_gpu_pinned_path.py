@@ -269,3 +269,17 @@ def test_large_batches_in_pieces(gpu_lib, oracle, n, sizes, monkeypatch):
         assert np.array_equal(b.status, st) and np.array_equal(b.slot, slots) and np.array_equal(b.counter, ctr)
         assert np.array_equal(b.out_len, ln2) and np.array_equal(b.ring, want)
         assert set(np.flatnonzero(st == oracle.AUTH_FAIL)) == set(hurt)
+
+
+def test_nothing_to_send_in_pieces(gpu_lib, monkeypatch):
+    """An empty batch has no pieces, whatever size they start from."""
+    from bnk_b200 import Context
+    from bnk_b200.device import F_STATS
+
+    monkeypatch.setenv("BNK_PIECES_FROM", "0")
+    with Context(max_keypairs=1, flow_capacity=0) as c:
+        b = c.batch(4, 4096)
+        for f in (b.seal, b.open):
+            f(0, F_STATS)
+            assert b.stats()["packets"] == 0
+            f(0)
