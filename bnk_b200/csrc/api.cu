@@ -10,6 +10,7 @@
 #include <thread>
 
 #include "filter_device.cuh"
+#include "pieces.h"
 #include "scan.h"
 #include "submit_order.h"
 
@@ -183,48 +184,6 @@ bool heads_direct(bnk_batch *b, uint32_t npkts, uint32_t flags) {
     }
     return host_direct(b, npkts, flags, 0);
 }
-// A large batch that is alone in flight goes over the link in pieces: while one is worked on, the next comes up and the
-// one before goes down, so both copy engines are busy.  Pieces end on pages of the ring (a copy that starts elsewhere is
-// up to a sixth slower: 190 MB up and down in 8 MB pieces 4.1 ms against 4.9), with small ones first and last, when one
-// direction has nothing to do yet or any more.  Between two copies an engine rests ~15 us while the other direction is
-// busy, so the pieces in the middle of a large ring are large: 190 MB sealed in pieces of at most 8 MB 5.0 ms, 16 MB 4.74,
-// 24 MB 4.70, but 47 MB in at most 8 MB 1.35 ms, 24 MB 1.39.  Two streams for each direction share its engine's rate and
-// finish later (5.7 ms).  Packets have to lie in the ring in order.
-constexpr uint64_t kPieceLeast = 1ull << 20, kPieceMost = 8ull << 20, kPieceMostEver = 24ull << 20, kPage = 4096;
-struct Piece {
-    uint32_t first, count;       // packets
-    uint64_t up, up_to;          // ring bytes that come up in front of them
-    uint64_t down, down_to;      // ring bytes nobody works on any more behind them
-};
-class Pieces {
-  public:
-    // `more`: a packet's kernel reads and writes at most len + more bytes from its offset on.  All of them have to be up: a
-    // later copy must not run over what the kernel has written.
-    Pieces(const bnk_batch *b, uint32_t n, uint32_t more, uint64_t ext) : off_(b->host.off), len_(b->host.len), n_(n), more_(more), ext_(ext),
-          most_(std::min(std::max(kPieceMost, ext / 8), kPieceMostEver)) {}
-    bool next(Piece &p) {
-        if (at_ == n_) return false;
-        p.first = at_;
-        p.up = up_;
-        p.down = down_;
-        do { // a packet larger than a piece takes several
-            const uint64_t left = ext_ - up_, size = std::min(std::min(most_, up_ + kPieceLeast), std::max(kPieceLeast, left / 2));
-            up_ = left <= size + size / 2 ? ext_ : (up_ + size) & ~(kPage - 1);
-            if (up_ == ext_) at_ = n_;
-            while (at_ < n_ && (uint64_t)off_[at_] + more_ + len_[at_] <= up_) at_++;
-        } while (at_ == p.first);
-        down_ = at_ == n_ ? ext_ : std::max(down_, std::min(up_, (uint64_t)off_[at_]) & ~(kPage - 1));
-        p.count = at_ - p.first;
-        p.up_to = up_;
-        p.down_to = down_;
-        return true;
-    }
-
-  private:
-    const uint32_t *off_, *len_;
-    uint32_t n_, more_, at_ = 0;
-    uint64_t ext_, most_, up_ = 0, down_ = 0;
-};
 // Below ctx->pieces_from (24 MB) a kernel on the pinned ring is as fast or faster, because the first piece up and the last
 // one down have no company: 16,384 x 1420 B 710 us against 750, 32,768 1390 against 1330, 131,072 5.74 ms against 4.96.
 // With small packets that kernel is bound by what its warps compute, ~7.5 ns a packet, and pieces win earlier: 8192 x
@@ -234,26 +193,8 @@ bool in_pieces(const bnk_batch *b, uint32_t n, uint32_t flags, uint64_t ext, boo
     const uint64_t from = b->ctx->pieces_from;
     if (n == 0) return false;
     if (ext < from && (n < kManySmall || ext > (uint64_t)n * kSmallBytes || ext < from / 16)) return false;
-    return in_order && b->up_stream && !(flags & (BNK_F_NO_H2D | BNK_F_NO_D2H | BNK_F_USE_OUT_LEN)) &&
+    return in_order && b->pieces.up && !(flags & (BNK_F_NO_H2D | BNK_F_NO_D2H | BNK_F_USE_OUT_LEN)) &&
            b->ctx->in_flight.load(std::memory_order_relaxed) == (b->counted ? 1 : 0);
-}
-// Copies a piece up (piece_is_up lets stream s go on behind it) / copies down what is done on s.
-cudaError_t piece_up(bnk_batch *b, const Piece &p) {
-    const cudaError_t e = cudaMemcpyAsync(b->dev.ring + p.up, b->host.ring + p.up, p.up_to - p.up, cudaMemcpyHostToDevice, b->up_stream);
-    return e != cudaSuccess ? e : cudaEventRecord(b->ev_up, b->up_stream);
-}
-cudaError_t piece_is_up(bnk_batch *b, cudaStream_t s) { return cudaStreamWaitEvent(s, b->ev_up, 0); }
-cudaError_t piece_down(bnk_batch *b, const Piece &p, cudaStream_t s) {
-    if (p.down_to == p.down) return cudaSuccess;
-    cudaError_t e = cudaEventRecord(b->ev_down, s);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(b->down_stream, b->ev_down, 0);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(b->host.ring + p.down, b->dev.ring + p.down, p.down_to - p.down, cudaMemcpyDeviceToHost, b->down_stream);
-    return e;
-}
-cudaError_t pieces_end(bnk_batch *b, cudaStream_t s) { // s is done when the last piece is down
-    cudaError_t e = cudaEventRecord(b->ev_down, b->down_stream);
-    return e != cudaSuccess ? e : cudaStreamWaitEvent(s, b->ev_down, 0);
 }
 AeadArgs piece_args(AeadArgs a, const Piece &p) {
     a.off += p.first;
@@ -873,6 +814,8 @@ int bnk_batch_destroy(bnk_batch *b) {
     }
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->direct_stream) cudaStreamSynchronize(b->direct_stream);
+    for (cudaStream_t side : {b->aux_stream, b->aead_stream, b->pieces.up, b->pieces.down})
+        if (side) cudaStreamSynchronize(side);
     cudaFreeHost(b->h_desc); // all of the pinned arrays
     cudaFree(b->d_desc);     // all of the device's
     if (b->k_begin) cudaEventDestroy(b->k_begin);
@@ -881,10 +824,10 @@ int bnk_batch_destroy(bnk_batch *b) {
     if (b->a_end) cudaEventDestroy(b->a_end);
     if (b->t_end) cudaEventDestroy(b->t_end);
     if (b->ev_order) cudaEventDestroy(b->ev_order);
-    if (b->ev_up) cudaEventDestroy(b->ev_up);
-    if (b->ev_down) cudaEventDestroy(b->ev_down);
-    if (b->up_stream) cudaStreamDestroy(b->up_stream);
-    if (b->down_stream) cudaStreamDestroy(b->down_stream);
+    if (b->pieces.ev_up) cudaEventDestroy(b->pieces.ev_up);
+    if (b->pieces.ev_down) cudaEventDestroy(b->pieces.ev_down);
+    if (b->pieces.up) cudaStreamDestroy(b->pieces.up);
+    if (b->pieces.down) cudaStreamDestroy(b->pieces.down);
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
     if (b->ev_fence) cudaEventDestroy(b->ev_fence);
@@ -969,10 +912,10 @@ int bnk_batch_create(bnk_ctx *ctx, uint32_t max_pkts, uint64_t ring_bytes, bnk_b
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_aead_done, cudaEventDisableTiming);
     }
     if (e == cudaSuccess && (ring_bytes >= ctx->pieces_from || max_pkts >= kManySmall)) {
-        e = cudaStreamCreateWithPriority(&b->up_stream, cudaStreamNonBlocking, ctx->prio_high);
-        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->down_stream, cudaStreamNonBlocking, ctx->prio_high);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_up, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_down, cudaEventDisableTiming);
+        e = cudaStreamCreateWithPriority(&b->pieces.up, cudaStreamNonBlocking, ctx->prio_high);
+        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->pieces.down, cudaStreamNonBlocking, ctx->prio_high);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->pieces.ev_up, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->pieces.ev_down, cudaEventDisableTiming);
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
@@ -1111,10 +1054,11 @@ static int seal_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
-    Pieces pieces(b, npkts, BNK_WG_HEADER + 16 + BNK_WG_TAG, ext);
+    Pieces pieces(b->host.off, b->host.len, npkts, kMostRoom, ext);
+    PieceCopies copies(b->pieces, b->dev.ring, b->host.ring, s);
     Piece p;
     pieces.next(p); // the first is on its way while the kernels in front of the first seal are prepared
-    CK(ctx, piece_up(b, p));
+    CK(ctx, copies.up(p));
     CK(ctx, desc_copy(b, npkts, D_OFF, b->stale_pkts ? D_STATUS : (flags & BNK_F_ASSIGN_COUNTERS) ? D_SLOT : D_COUNTER, true, s));
     caught_up(b, npkts); // (more of them stay behind: the host arrays will hold this call's results as well)
     ring_is_up(b, ext);
@@ -1129,12 +1073,12 @@ static int seal_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     if (note) CK(ctx, flow_note_begins(b, npkts, now_unix_ns, s, sweep));
     if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
     for (bool more = true; more;) {
-        CK(ctx, piece_is_up(b, s));
+        CK(ctx, copies.is_up());
         if (note) CK(ctx, launch_filter_note(b, p.first, p.count, now_unix_ns, Done{}, s));
         CK(ctx, launch_seal(piece_args(a, p), s, ctx));
-        CK(ctx, piece_down(b, p, s));
+        CK(ctx, copies.down(p));
         more = pieces.next(p);
-        if (more) CK(ctx, piece_up(b, p));
+        if (more) CK(ctx, copies.up(p));
     }
     if (timed) CK(ctx, cudaEventRecord(b->a_end, s));
     if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, Done{}, s));
@@ -1144,7 +1088,7 @@ static int seal_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     CK(ctx, tally_if_asked(b, npkts, flags, s));
     CK(ctx, order_kernels_end(b, s, false));
     CK(ctx, desc_copy(b, npkts, D_COUNTER, D_STATUS, false, s));
-    CK(ctx, pieces_end(b, s));
+    CK(ctx, copies.join());
     return BNK_SUCCESS;
 }
 
@@ -1312,10 +1256,11 @@ static int open_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0, demux = (flags & BNK_F_DEMUX_INDEX) != 0;
-    Pieces pieces(b, npkts, 0, ext);
+    Pieces pieces(b->host.off, b->host.len, npkts, 0, ext);
+    PieceCopies copies(b->pieces, b->dev.ring, b->host.ring, s);
     Piece p;
     pieces.next(p);
-    CK(ctx, piece_up(b, p));
+    CK(ctx, copies.up(p));
     CK(ctx, desc_copy(b, npkts, D_OFF, b->stale_pkts ? D_STATUS : demux ? D_LEN : D_SLOT, true, s));
     caught_up(b, npkts);
     ring_is_up(b, ext);
@@ -1326,12 +1271,12 @@ static int open_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     const bool replay = (flags & BNK_F_REPLAY) != 0, one_launch = npkts <= kGroupMax;
     if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
     for (bool more = true; more;) {
-        CK(ctx, piece_is_up(b, s));
+        CK(ctx, copies.is_up());
         if (demux) CK(ctx, launch_demux_index(b, p.first, p.count, a.len, s));
         CK(ctx, launch_open(piece_args(a, p), s, ctx));
-        CK(ctx, piece_down(b, p, s)); // the checks below say which plaintexts count, and change no byte of them
+        CK(ctx, copies.down(p)); // the checks below say which plaintexts count, and change no byte of them
         more = pieces.next(p);
-        if (more) CK(ctx, piece_up(b, p));
+        if (more) CK(ctx, copies.up(p));
     }
     if (timed) CK(ctx, cudaEventRecord(b->a_end, s));
     if (replay && one_launch) {
@@ -1350,7 +1295,7 @@ static int open_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     CK(ctx, tally_if_asked(b, npkts, flags, s));
     CK(ctx, order_kernels_end(b, s, false));
     CK(ctx, desc_copy(b, npkts, demux ? D_SLOT : D_COUNTER, D_STATUS, false, s));
-    CK(ctx, pieces_end(b, s));
+    CK(ctx, copies.join());
     return BNK_SUCCESS;
 }
 

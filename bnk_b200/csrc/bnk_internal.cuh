@@ -15,6 +15,7 @@
 
 #include "../../include/bnk_gpu.h"
 #include "flow_bounds.h"
+#include "pieces.h"
 
 // ---------------------------------------------------------------------------
 // Device-resident tables of one context (one GPU).  All per-peer mutable state
@@ -182,8 +183,7 @@ struct bnk_batch {
     // kernel of another.
     cudaStream_t aead_stream;
     cudaEvent_t ev_aead_go, ev_aead_done;
-    cudaStream_t up_stream, down_stream; // of a batch large enough to go over the link in pieces
-    cudaEvent_t ev_up, ev_down;
+    PieceStreams pieces; // of a batch large enough to go over the link that way
     cudaEvent_t ev_fork, ev_join;
     cudaEvent_t k_begin, k_end, t_end, a_begin, a_end;
     bool in_flight;
