@@ -108,7 +108,7 @@ struct SubmitScope {
     std::shared_lock<std::shared_mutex> tables; // see bnk_ctx::submit_mu
     explicit SubmitScope(bnk_batch *batch) : b(batch), tables(batch->ctx->submit_mu) {
         b->stats_pending = b->done_watched = false;
-        b->run_stream = b->stream;
+        b->order.begins(b->stream);
     }
     ~SubmitScope() {
         b->in_flight = true;
@@ -322,12 +322,13 @@ AeadArgs aead_args(bnk_batch *b, uint32_t n, bool open, const uint32_t *order) {
 } // namespace
 
 int order_begin(bnk_batch *b, bnk_batch *behind) {
-    if (!b->ev_order) CK(b->ctx, cudaEventCreateWithFlags(&b->ev_order, cudaEventDisableTiming));
-    b->ordered = true;
     b->behind = behind;
+    if (!b->order.ev) CK(b->ctx, cudaEventCreateWithFlags(&b->order.ev, cudaEventDisableTiming));
+    b->ordered = true;
     return BNK_SUCCESS;
 }
-void order_end(bnk_batch *b) {
+void order_end(bnk_batch *b, int rc) {
+    if (rc != BNK_SUCCESS && b->behind) SubmitOrder::failed_behind(b->behind->order);
     b->ordered = false;
     b->behind = nullptr;
 }
@@ -335,20 +336,12 @@ void batch_set_direct_stream(bnk_batch *b, cudaStream_t s) { b->direct_stream = 
 cudaError_t order_stream_create(bnk_ctx *ctx, cudaStream_t *s) {
     return cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, ctx->prio_high);
 }
-// The kernels of a submit come next on stream s ...
-static cudaError_t order_kernels_begin(bnk_batch *b, cudaStream_t s) {
-    bnk_batch *const p = b->behind;
-    if (!b->ordered || !p || p->run_stream == s) return cudaSuccess;
-    cudaError_t e = cudaSuccess;
-    if (p->ran_direct) e = cudaEventRecord(p->ev_order, p->run_stream); // nothing but kernels there
-    return e != cudaSuccess ? e : cudaStreamWaitEvent(s, p->ev_order, 0);
+// The submit's kernels come next, on the stream it has begun on ...
+static cudaError_t order_kernels_begin(bnk_batch *b) {
+    return b->ordered && b->behind ? b->order.follow(b->behind->order) : cudaSuccess;
 }
-// ... and these were the last of them.
-static cudaError_t order_kernels_end(bnk_batch *b, cudaStream_t s, bool direct) {
-    b->run_stream = s;
-    b->ran_direct = direct;
-    return b->ordered && !direct ? cudaEventRecord(b->ev_order, s) : cudaSuccess;
-}
+// ... and these were the last of them; copies may follow.
+static cudaError_t order_kernels_end(bnk_batch *b) { return b->ordered ? b->order.kernels_end() : cudaSuccess; }
 
 extern "C" {
 
@@ -823,7 +816,7 @@ int bnk_batch_destroy(bnk_batch *b) {
     if (b->a_begin) cudaEventDestroy(b->a_begin);
     if (b->a_end) cudaEventDestroy(b->a_end);
     if (b->t_end) cudaEventDestroy(b->t_end);
-    if (b->ev_order) cudaEventDestroy(b->ev_order);
+    if (b->order.ev) cudaEventDestroy(b->order.ev);
     if (b->pieces.ev_up) cudaEventDestroy(b->pieces.ev_up);
     if (b->pieces.ev_down) cudaEventDestroy(b->pieces.ev_down);
     if (b->pieces.up) cudaStreamDestroy(b->pieces.up);
@@ -985,11 +978,12 @@ int bnk_batch_download(bnk_batch *b, uint32_t npkts) {
 static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t flags, int64_t now_unix_ns, bool resident) {
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->direct_stream ? b->direct_stream : b->stream;
+    b->order.begins(s);
     const bool timed = (flags & BNK_F_TIMED) != 0, stats = (flags & BNK_F_STATS) != 0;
     const bool assign = (flags & BNK_F_ASSIGN_COUNTERS) != 0;
     const bnk_batch_view &h = b->host;
     const DeviceBatch &d = b->dev;
-    CK(ctx, order_kernels_begin(b, s));
+    CK(ctx, order_kernels_begin(b));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, false, nullptr);
     a.over_link = true;
@@ -1046,7 +1040,6 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = b->aead_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
-    CK(ctx, order_kernels_end(b, s, true));
     return BNK_SUCCESS;
 }
 
@@ -1062,7 +1055,7 @@ static int seal_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     CK(ctx, desc_copy(b, npkts, D_OFF, b->stale_pkts ? D_STATUS : (flags & BNK_F_ASSIGN_COUNTERS) ? D_SLOT : D_COUNTER, true, s));
     caught_up(b, npkts); // (more of them stay behind: the host arrays will hold this call's results as well)
     ring_is_up(b, ext);
-    CK(ctx, order_kernels_begin(b, s));
+    CK(ctx, order_kernels_begin(b));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     if (flags & BNK_F_ASSIGN_COUNTERS) CK(ctx, launch_assign_counters(b, npkts, b->dev.slot, b->dev.counter, s));
     AeadArgs a = aead_args(b, npkts, false, nullptr); // (length classes would only be those of a piece, and the link is the bound)
@@ -1086,7 +1079,7 @@ static int seal_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = b->aead_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
-    CK(ctx, order_kernels_end(b, s, false));
+    CK(ctx, order_kernels_end(b));
     CK(ctx, desc_copy(b, npkts, D_COUNTER, D_STATUS, false, s));
     CK(ctx, copies.join());
     return BNK_SUCCESS;
@@ -1119,7 +1112,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
             CK(ctx, desc_copy(b, n, D_OFF, all ? D_STATUS : (flags & BNK_F_ASSIGN_COUNTERS) ? D_SLOT : D_COUNTER, true, s));
         caught_up(b, npkts);
     }
-    CK(ctx, order_kernels_begin(b, s));
+    CK(ctx, order_kernels_begin(b));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     if ((flags & BNK_F_NOTE_OUTBOUND) && n && ctx->ft.enforce && ctx->ft.flow_capacity) { // filter.go:192-194
         bool sweep;
@@ -1165,7 +1158,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     b->kernel_timed = timed;
     b->aead_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
-    CK(ctx, order_kernels_end(b, s, false));
+    CK(ctx, order_kernels_end(b));
     if (!(flags & BNK_F_NO_D2H) && n) {
         if (b->joint_copy) {
             CK(ctx, ring_down(b, npkts, ext, true, s));
@@ -1182,11 +1175,12 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
 static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t flags, int64_t now_unix_ns) {
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->direct_stream ? b->direct_stream : b->stream;
+    b->order.begins(s);
     const bool timed = (flags & BNK_F_TIMED) != 0, stats = (flags & BNK_F_STATS) != 0;
     const bool replay = (flags & BNK_F_REPLAY) != 0, checks = (flags & (BNK_F_INNER_CHECK | BNK_F_CHECK_INBOUND)) != 0;
     const bnk_batch_view &h = b->host;
     b->stale_pkts = std::max(b->stale_pkts, npkts);
-    CK(ctx, order_kernels_begin(b, s));
+    CK(ctx, order_kernels_begin(b));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, true, nullptr);
     a.over_link = a.from_host = true;
@@ -1247,7 +1241,6 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = b->aead_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
-    CK(ctx, order_kernels_end(b, s, true));
     if (!one_launch) CK(ctx, desc_copy(b, npkts, D_OUT_LEN, D_STATUS, false, s));
     return BNK_SUCCESS;
 }
@@ -1264,7 +1257,7 @@ static int open_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     CK(ctx, desc_copy(b, npkts, D_OFF, b->stale_pkts ? D_STATUS : demux ? D_LEN : D_SLOT, true, s));
     caught_up(b, npkts);
     ring_is_up(b, ext);
-    CK(ctx, order_kernels_begin(b, s));
+    CK(ctx, order_kernels_begin(b));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, true, nullptr);
     a.behind_kernel = true;
@@ -1293,7 +1286,7 @@ static int open_pieces(bnk_batch *b, uint32_t npkts, uint64_t ext, uint32_t flag
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = b->aead_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
-    CK(ctx, order_kernels_end(b, s, false));
+    CK(ctx, order_kernels_end(b));
     CK(ctx, desc_copy(b, npkts, demux ? D_SLOT : D_COUNTER, D_STATUS, false, s));
     CK(ctx, copies.join());
     return BNK_SUCCESS;
@@ -1323,7 +1316,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
         if (!joint) CK(ctx, desc_copy(b, n, D_OFF, all ? D_STATUS : (flags & BNK_F_DEMUX_INDEX) ? D_LEN : D_SLOT, true, s));
         caught_up(b, npkts);
     }
-    CK(ctx, order_kernels_begin(b, s));
+    CK(ctx, order_kernels_begin(b));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     const uint32_t *order = nullptr;
     AeadArgs oa = aead_args(b, npkts, true, nullptr);
@@ -1371,7 +1364,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
-    CK(ctx, order_kernels_end(b, s, false));
+    CK(ctx, order_kernels_end(b));
     if (!(flags & BNK_F_NO_D2H) && n) {
         if (b->joint_copy) {
             CK(ctx, ring_down(b, npkts, ext, true, s));
@@ -1591,11 +1584,11 @@ int bnk_wait(bnk_batch *b, uint64_t timeout_ns) {
         if (b->done_watched && timeout_ns == 0 && (++b->done_polls & 63u)) return BNK_ETIMEDOUT; // ask the driver now and then
         CK(ctx, cudaSetDevice(ctx->device));
         if (timeout_ns == UINT64_MAX) {
-            CK(ctx, cudaStreamSynchronize(b->run_stream));
+            CK(ctx, cudaStreamSynchronize(b->order.run));
         } else {
             const auto deadline = std::chrono::steady_clock::now() + std::chrono::nanoseconds(timeout_ns);
             for (;;) {
-                cudaError_t e = cudaStreamQuery(b->run_stream);
+                cudaError_t e = cudaStreamQuery(b->order.run);
                 if (e == cudaSuccess) break;
                 if (e != cudaErrorNotReady) return fail(ctx, BNK_ECUDA, "cudaStreamQuery", e);
                 if (std::chrono::steady_clock::now() >= deadline) return BNK_ETIMEDOUT;

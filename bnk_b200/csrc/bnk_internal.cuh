@@ -16,6 +16,7 @@
 #include "../../include/bnk_gpu.h"
 #include "flow_bounds.h"
 #include "pieces.h"
+#include "submit_order.h"
 
 // ---------------------------------------------------------------------------
 // Device-resident tables of one context (one GPU).  All per-peer mutable state
@@ -213,12 +214,11 @@ struct bnk_batch {
     unsigned long long *d_stats; // device accumulators of the tally kernel (zero between launches)
     cudaEvent_t ev_fence; // orders this batch's stream against table maintenance on another stream
     // Submits in order over several batches (submit_order.h).  direct_stream: where such a batch runs when it stays in
-    // pinned memory (shared with the batches it is ordered against; null: on its own stream).  run_stream: where the last
-    // submit ran.  ev_order: behind its kernels.
-    cudaStream_t direct_stream, run_stream;
-    bool ordered, ran_direct; // between order_begin and order_end / the last submit ran in pinned memory
+    // pinned memory (shared with the batches it is ordered against; null: on its own stream).
+    cudaStream_t direct_stream;
+    SubmitOrder order;
+    bool ordered; // between order_begin and order_end
     bnk_batch *behind;
-    cudaEvent_t ev_order;
 };
 
 // Small batches are two dependent launches with little work in each, so the gap between them counts.  A kernel

@@ -1,4 +1,4 @@
-"""The order of a submit's copies and kernels over its streams (csrc/pieces.h) with a CUDA runtime that
+"""The order of a submit's copies and kernels over its streams (csrc/pieces.h, csrc/submit_order.h) with a CUDA runtime that
 only keeps lists: every stream runs its operations in order, a stream that is waited for runs and the others only as far as
 its events ask, and any call may fail.  Host code only."""
 import os
@@ -58,6 +58,7 @@ inline cudaError_t cudaStreamSynchronize(cudaStream_t st) {
 """
 PROGRAM = r"""
 #include "pieces.h"
+#include "submit_order.h"
 #include <cstdio>
 #include <cstdlib>
 #include <random>
@@ -116,7 +117,50 @@ static int pieces_test(uint32_t seed) {
     }
     return 0;
 }
-int main(int, char **argv) { return pieces_test(atoi(argv[2])); }
+// Submits of batches in turn, in place on the shared stream or copied on their own, some failing half way: what is queued of a
+// submit's kernels runs behind all kernels of those in front, and waiting for a batch waits for its kernels.
+static int order_test(uint32_t seed) {
+    std::mt19937 rng(seed);
+    Stream shared, own[3];
+    Event ev[3];
+    SubmitOrder o[3] = {{&own[0], &ev[0], false}, {&own[1], &ev[1], false}, {&own[2], &ev[2], false}};
+    std::vector<int> ran;
+    int queued = 0, last = -1;
+    for (int turn = 0; turn < 400; turn++) {
+        const int b = turn % 3;
+        cudaStreamSynchronize(o[b].run); // its earlier submit is waited for
+        const bool direct = rng() % 2;
+        std::vector<int> mine;
+        const bool ok = [&] {
+            SubmitOrder &x = o[b];
+            x.begins(&own[b]);
+            if (direct) x.begins(&shared);
+            if (rng() % 4 == 0) calls_left = rng() % 3;
+            if (last >= 0 && x.follow(o[last]) != cudaSuccess) return false;
+            for (int k = 0; k < 2; k++) {
+                if (rng() % 8 == 0) return false; // a launch fails
+                const int id = queued++;
+                mine.push_back(id);
+                x.run->ops.push_back({[&ran, id] { ran.push_back(id); }});
+            }
+            if (direct) return true;
+            if (x.kernels_end() != cudaSuccess) return false;
+            x.run->ops.push_back({[] {}}); // the copy down
+            return true;
+        }();
+        calls_left = 1 << 30;
+        if (!ok && last >= 0) SubmitOrder::failed_behind(o[last]);
+        last = b;
+        if (rng() % 3 == 0) {
+            cudaStreamSynchronize(o[b].run);
+            for (int id : mine) { bool in = false; for (int r : ran) in |= r == id; if (!in) return printf("waited for, not run: %d\n", id), 1; }
+        }
+    }
+    for (Stream *st : {&shared, &own[0], &own[1], &own[2]}) cudaStreamSynchronize(st);
+    for (size_t i = 1; i < ran.size(); i++) if (ran[i] < ran[i - 1]) return printf("%d behind %d\n", ran[i], ran[i - 1]), 1;
+    return (int)ran.size() != queued;
+}
+int main(int, char **argv) { return argv[1][0] == 'p' ? pieces_test(atoi(argv[2])) : order_test(atoi(argv[2])); }
 """
 
 
@@ -131,7 +175,7 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("seed", range(6))
-@pytest.mark.parametrize("what", ["pieces"])
+@pytest.mark.parametrize("what", ["pieces", "order"])
 def test_streams(program, what, seed):
     out = subprocess.run([program, what, str(seed)], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
