@@ -1064,6 +1064,9 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
 // 12,032 x 1420 B in 421 us by 64 CTAs, 395 by 128, 375 by 444 and more.
 constexpr uint64_t kLinkWindow = 64u << 10, kLeastCtas = 64, kMostCtas = 512;
 constexpr uint32_t kStoreCtas = 592;
+// The seal kernel hands out nonces for one packet per warp, counted over one tile of the whole batch: a batch of that size
+// has to get a warp for every packet.
+static_assert(kRankMax <= kLeastCtas * kWppWarps, "batches that hand out their own nonces run a packet per warp");
 void wpp_grid(AeadArgs &a, uint32_t &ctas) {
     ctas = (a.n + kWppWarps - 1) / kWppWarps;
     a.tile = 1;
