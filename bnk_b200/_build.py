@@ -38,7 +38,7 @@ def bench_sources() -> list[str]:
 
 def _deps() -> list[str]:
     inc = os.path.join(os.path.dirname(PKG_DIR), "include", "bnk_gpu.h")
-    return sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(HOST, "*.hpp")) + [inc]
+    return sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(HOST, "*.h*")) + [inc]
 
 
 def _bench_deps() -> list[str]:

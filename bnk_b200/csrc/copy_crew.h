@@ -13,8 +13,8 @@
 #include <chrono>
 #include <condition_variable>
 #include <cstdint>
+#include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -22,8 +22,9 @@ class CopyCrew {
   public:
     explicit CopyCrew(uint32_t helpers) {
         try {
+            threads_.reserve(helpers);
             for (uint32_t i = 0; i < helpers; i++) threads_.emplace_back([this] { help(); });
-        } catch (const std::system_error &) { // as many as the process may have
+        } catch (const std::exception &) { // as many as the process may have
         }
     }
     ~CopyCrew() {

@@ -262,13 +262,16 @@ int bnk_queue_create(bnk_ctx *ctx, const bnk_queue_cfg *cfg, bnk_queue **out) {
     if (!cfg->open_side) q->cfg.flags |= BNK_F_ASSIGN_COUNTERS;
     if (q->cfg.min_fill == 0) q->cfg.min_fill = std::min(128u, (cfg->max_pkts + 3) / 4); // one upstream batch
     q->slot_bytes = (16u + ((cfg->max_packet + 15u) & ~15u) + 16u + 15u) & ~15u;
-    q->gb = std::vector<GpuBatch>(cfg->depth + kRotationExtra);
-    q->closed.slot.resize(q->gb.size());
-    q->inflight.slot.resize(q->gb.size());
-    {
+    try {
+        q->gb = std::vector<GpuBatch>(cfg->depth + kRotationExtra);
+        q->closed.slot.resize(q->gb.size());
+        q->inflight.slot.resize(q->gb.size());
         std::lock_guard<std::mutex> g(ctx->mu);
-        if (!ctx->crew) ctx->crew.reset(new CopyCrew(CopyCrew::helpers_for(std::thread::hardware_concurrency())));
+        if (!ctx->crew) ctx->crew = std::make_shared<CopyCrew>(CopyCrew::helpers_for(std::thread::hardware_concurrency()));
         q->crew = ctx->crew.get();
+    } catch (const std::exception &) { // no memory
+        delete q;
+        return BNK_ENOMEM;
     }
     cudaSetDevice(ctx->device);
     if (order_stream_create(ctx, &q->stream) != cudaSuccess) {

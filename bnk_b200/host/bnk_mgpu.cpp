@@ -22,6 +22,7 @@
 #include "../../include/bnk_gpu.h"
 #include "../csrc/packet_copy.h"
 #include "../csrc/submit_order.h"
+#include "crew.h"
 
 extern "C" int bnk_place_peers(const uint64_t *load, uint32_t n_peers, uint32_t n_gpus, uint32_t max_per_gpu,
                                uint32_t *gpu_of, uint32_t *slot_of, uint64_t *load_per_gpu) {
@@ -63,67 +64,9 @@ extern "C" int bnk_place_peers(const uint64_t *load, uint32_t n_peers, uint32_t 
 
 namespace {
 
+using namespace crew;
+
 constexpr uint32_t kNoPeer = 0xffffffffu;
-
-// One host thread per GPU: runs the jobs posted to it in order.
-class Worker {
-  public:
-    Worker() : thread_([this] { Run(); }) {}
-    ~Worker() {
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            stop_ = true;
-        }
-        cv_.notify_all();
-        thread_.join();
-    }
-    void Post(std::function<void()> job) {
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            jobs_.push(std::move(job));
-        }
-        cv_.notify_all();
-    }
-
-  private:
-    void Run() {
-        for (;;) {
-            std::function<void()> job;
-            {
-                std::unique_lock<std::mutex> g(mu_);
-                cv_.wait(g, [this] { return stop_ || !jobs_.empty(); });
-                if (jobs_.empty()) return;
-                job = std::move(jobs_.front());
-                jobs_.pop();
-            }
-            job();
-        }
-    }
-    std::mutex mu_;
-    std::condition_variable cv_;
-    std::queue<std::function<void()>> jobs_;
-    bool stop_ = false;
-    std::thread thread_;
-};
-
-// counts the per-GPU jobs of one call down
-class Latch {
-  public:
-    explicit Latch(int n) : left_(n) {}
-    void Done() {
-        std::lock_guard<std::mutex> g(mu_);
-        if (--left_ == 0) cv_.notify_all();
-    }
-    void Wait() {
-        std::unique_lock<std::mutex> g(mu_);
-        cv_.wait(g, [this] { return left_ <= 0; });
-    }
-
-  private:
-    std::mutex mu_;
-    std::condition_variable cv_;
-    int left_;
-};
 
 struct PeerInfo {
     bool set = false;
@@ -170,187 +113,6 @@ class IndexTable {
     std::vector<uint64_t> slots_;
 };
 
-inline void Pause() {
-#if defined(__x86_64__) || defined(__i386__)
-    __builtin_ia32_pause();
-#else
-    std::this_thread::yield();
-#endif
-}
-
-// Work of one thread that others may join.
-struct Task {
-    virtual ~Task() = default;
-    virtual int Drive() = 0; // the calling thread; returns when all is done
-    virtual void Help() = 0; // any other
-};
-
-// f(first, last) over [0, n) in stretches, whoever is free taking the next one.
-struct Stretches : Task {
-    static constexpr uint32_t kStretch = 512;
-    const uint32_t n;
-    const std::function<void(uint32_t, uint32_t)> f;
-    std::atomic<uint32_t> next{0}, done{0};
-    Stretches(uint32_t n_, std::function<void(uint32_t, uint32_t)> f_) : n(n_), f(std::move(f_)) {}
-    int Drive() override {
-        Help();
-        for (uint32_t idle = 0; done.load(std::memory_order_acquire) < n;) {
-            if (++idle < 4000) Pause();
-            else std::this_thread::yield();
-        }
-        return BNK_SUCCESS;
-    }
-    void Help() override {
-        for (;;) {
-            const uint32_t at = next.fetch_add(kStretch, std::memory_order_relaxed);
-            if (at >= n) return;
-            const uint32_t to = std::min(n, at + kStretch);
-            f(at, to);
-            done.fetch_add(to - at, std::memory_order_release);
-        }
-    }
-};
-
-// A GPU's share of one call in pieces: while one piece is on the GPU the next is copied into the pinned ring of another
-// batch and the one before is copied out, by several threads.  (One batch, one thread, one step after the other: 24,576 x
-// 1420 B sealed and opened in 21.8 ms, of which the GPU worked 3.)
-struct Share : Task {
-    static constexpr uint32_t kSlots = 4;  // pinned batches in rotation
-    static constexpr uint32_t kAhead = 2;  // pieces on the GPU at once: one works, one waits behind it
-    static constexpr uint32_t kChunk = 32; // packets a thread copies at a time
-    uint32_t n, piece, pieces, chunks; // packets, packets per piece, pieces, chunks per piece
-    std::function<void(uint32_t slot, uint32_t at, uint32_t first, uint32_t cnt)> in, out; // packets [first, +cnt) of the share, at `at` of the slot's batch
-    std::function<int(uint32_t slot, uint32_t piece, uint32_t cnt)> submit;
-    std::function<int(uint32_t slot)> poll;                                                // BNK_ETIMEDOUT: not yet
-    std::atomic<uint32_t> in_next{0}, out_next{0}, gpu_done{0}, out_done{0};
-    std::vector<std::atomic<uint32_t>> in_left, out_left;
-    std::atomic<bool> stop{false};
-
-    Share(uint32_t n_, uint32_t piece_)
-        : n(n_), piece(piece_), pieces((n_ + piece_ - 1) / piece_), chunks((piece_ + kChunk - 1) / kChunk), in_left(pieces), out_left(pieces) {
-        for (uint32_t p = 0; p < pieces; p++) {
-            in_left[p].store(chunks, std::memory_order_relaxed);
-            out_left[p].store(chunks, std::memory_order_relaxed);
-        }
-    }
-    uint32_t Count(uint32_t p) const { return std::min(piece, n - p * piece); }
-    void Chunk(uint32_t t, const std::function<void(uint32_t, uint32_t, uint32_t, uint32_t)> &f) const {
-        const uint32_t p = t / chunks, at = t % chunks * kChunk, cnt = Count(p);
-        if (at < cnt) f(p % kSlots, at, p * piece + at, std::min(kChunk, cnt - at));
-    }
-    // One copy, if there is one to do.
-    bool Copy() {
-        uint32_t t = out_next.load(std::memory_order_relaxed);
-        if (t / chunks < gpu_done.load(std::memory_order_acquire) && t < pieces * chunks) {
-            if (!out_next.compare_exchange_strong(t, t + 1, std::memory_order_acq_rel)) return true;
-            Chunk(t, out);
-            if (out_left[t / chunks].fetch_sub(1, std::memory_order_acq_rel) == 1) out_done.fetch_add(1, std::memory_order_release);
-            return true;
-        }
-        t = in_next.load(std::memory_order_relaxed);
-        if (t < pieces * chunks) {
-            const uint32_t p = t / chunks;
-            if (p >= kSlots && out_left[p - kSlots].load(std::memory_order_acquire) != 0) return false; // its ring is taken
-            if (!in_next.compare_exchange_strong(t, t + 1, std::memory_order_acq_rel)) return true;
-            Chunk(t, in);
-            in_left[p].fetch_sub(1, std::memory_order_acq_rel);
-            return true;
-        }
-        return false;
-    }
-    bool Over() const { return stop.load(std::memory_order_acquire) || out_done.load(std::memory_order_acquire) == pieces; }
-    // The thread that drives the GPU; copies in between.  Returns the first error.
-    int Drive() override {
-        int rc = BNK_SUCCESS;
-        uint32_t sent = 0, back = 0, idle = 0;
-        while (!Over()) {
-            if ((rc == BNK_SUCCESS || rc == BNK_EFULL) && sent < pieces && sent - back < kAhead && in_left[sent].load(std::memory_order_acquire) == 0) {
-                const int r = submit(sent % kSlots, sent, Count(sent));
-                sent++; // whatever was queued before an error has to be waited for as well
-                if (r != BNK_SUCCESS) rc = r;
-            }
-            if (back < sent) { // BNK_EFULL (flows that found no place) is an outcome, the results are valid
-                const int r = poll(back % kSlots);
-                if (r != BNK_ETIMEDOUT) {
-                    back++;
-                    if (rc == BNK_SUCCESS || rc == BNK_EFULL) rc = r != BNK_SUCCESS ? r : rc;
-                    if (rc == BNK_SUCCESS || rc == BNK_EFULL) gpu_done.store(back, std::memory_order_release);
-                }
-            } else if (rc != BNK_SUCCESS && rc != BNK_EFULL) {
-                stop.store(true, std::memory_order_release);
-            }
-            Turn(idle);
-        }
-        return rc;
-    }
-    void Help() override {
-        for (uint32_t idle = 0; !Over();) Turn(idle);
-    }
-    void Turn(uint32_t &idle) {
-        if (Copy()) idle = 0;
-        else if (++idle < 4000) Pause();
-        else std::this_thread::yield(); // more threads than cores, or a GPU that is far behind
-    }
-};
-
-// Threads that help with the copies of one GPU's shares.  They sleep between calls, after a moment of looking for the next.
-class Crew {
-  public:
-    explicit Crew(uint32_t helpers) {
-        for (uint32_t i = 0; i < helpers; i++) threads_.emplace_back([this] { Run(); });
-    }
-    ~Crew() {
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            stop_.store(true);
-        }
-        cv_.notify_all();
-        for (std::thread &t : threads_) t.join();
-    }
-    int Do(Task &t) {
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            task_ = &t;
-            calls_.fetch_add(1);
-        }
-        cv_.notify_all();
-        const int rc = t.Drive();
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            task_ = nullptr; // who has not come yet need not come
-        }
-        while (inside_.load(std::memory_order_acquire) != 0) Pause();
-        return rc;
-    }
-
-  private:
-    void Run() {
-        uint64_t seen = 0;
-        for (;;) {
-            for (int i = 0; i < 1000 && calls_.load(std::memory_order_relaxed) == seen && !stop_.load(std::memory_order_relaxed); i++) Pause();
-            Task *t;
-            {
-                std::unique_lock<std::mutex> g(mu_);
-                cv_.wait(g, [&] { return stop_.load() || calls_.load() != seen; });
-                if (stop_.load()) return;
-                seen = calls_.load();
-                t = task_;
-                if (t) inside_.fetch_add(1, std::memory_order_acq_rel);
-            }
-            if (!t) continue;
-            t->Help();
-            inside_.fetch_sub(1, std::memory_order_acq_rel);
-        }
-    }
-    std::mutex mu_;
-    std::condition_variable cv_;
-    Task *task_ = nullptr;
-    std::atomic<uint64_t> calls_{0};
-    std::atomic<bool> stop_{false};
-    std::atomic<int> inside_{0};
-    std::vector<std::thread> threads_;
-};
-
 } // namespace
 
 struct bnk_mgpu {
@@ -363,7 +125,7 @@ struct bnk_mgpu {
     std::vector<cudaStream_t> stream; // [gpu] of the pieces that stay in pinned memory
     std::vector<bnk_batch *> last; // [gpu] batch of the submit that the next one's kernels have to follow
     std::vector<std::unique_ptr<Worker>> worker;
-    std::vector<std::unique_ptr<Crew>> crew;
+    std::vector<std::unique_ptr<Crew>> helpers;
     std::vector<uint32_t> gpu_of, slot_of;
     std::vector<PeerInfo> peer;
     IndexTable peer_of_index; // receiver index -> peer
@@ -387,7 +149,7 @@ template <typename F>
 void over_packets(bnk_mgpu *m, uint32_t n, F f) {
     if (n < kShareFrom) return f(0, n);
     Stretches all(n, f);
-    m->crew[0]->Do(all);
+    m->helpers[0]->Do(all);
 }
 
 // Per-GPU lists of packet numbers in batch order (stable: a peer's packets keep their order), and what every peer carries.
@@ -417,7 +179,7 @@ const char *bnk_mgpu_last_error_string(bnk_mgpu *m) { return m ? m->last_error.c
 int bnk_mgpu_destroy(bnk_mgpu *m) {
     if (!m) return BNK_EINVAL;
     m->worker.clear(); // joins the threads
-    m->crew.clear();
+    m->helpers.clear();
     for (std::vector<bnk_batch *> &of_gpu : m->batch)
         for (bnk_batch *b : of_gpu)
             if (b) bnk_batch_destroy(b);
@@ -429,14 +191,7 @@ int bnk_mgpu_destroy(bnk_mgpu *m) {
     return BNK_SUCCESS;
 }
 
-int bnk_mgpu_create(const bnk_mgpu_cfg *cfg, bnk_mgpu **out) {
-    if (!cfg || !out || cfg->struct_size != sizeof(bnk_mgpu_cfg) || cfg->n_devices == 0 || !cfg->devices ||
-        cfg->max_pkts_per_gpu == 0 || cfg->max_peers == 0 || cfg->max_packet == 0)
-        return BNK_EINVAL;
-    *out = nullptr;
-    if ((uint64_t)cfg->n_devices * cfg->ctx.max_keypairs < cfg->max_peers) return BNK_EINVAL;
-    bnk_mgpu *m = new (std::nothrow) bnk_mgpu();
-    if (!m) return BNK_ENOMEM;
+static int build(bnk_mgpu *m, const bnk_mgpu_cfg *cfg) {
     m->cfg = *cfg;
     m->cfg.devices = nullptr;
     m->slot_bytes = (16u + ((cfg->max_packet + 15u) & ~15u) + 16u + 15u) & ~15u;
@@ -444,7 +199,7 @@ int bnk_mgpu_create(const bnk_mgpu_cfg *cfg, bnk_mgpu **out) {
     // A piece is about three megabytes of ring: the GPU then works ~100 us on it, and two of them may stay in pinned memory.
     m->piece = std::min(cfg->max_pkts_per_gpu, std::min(2048u, std::max(64u, (3u << 20) / m->slot_bytes)));
     const uint32_t cores = std::max(1u, std::thread::hardware_concurrency());
-    const uint32_t helpers = std::min(8u, cores / ng > 1 ? cores / ng - 1 : 0u); // 24,576 x 1420 B sealed and opened: 4.9 ms with 4, 4.1 with 6, 3.8 with 8, 3.6 with 14
+    const uint32_t n_helpers = std::min(8u, cores / ng > 1 ? cores / ng - 1 : 0u); // 24,576 x 1420 B sealed and opened: 4.9 ms with 4, 4.1 with 6, 3.8 with 8, 3.6 with 14
     m->ctx.assign(ng, nullptr);
     m->batch.assign(ng, std::vector<bnk_batch *>(Share::kSlots, nullptr));
     m->view.assign(ng, std::vector<bnk_batch_view>(Share::kSlots));
@@ -463,25 +218,35 @@ int bnk_mgpu_create(const bnk_mgpu_cfg *cfg, bnk_mgpu **out) {
             if (rc == BNK_SUCCESS) rc = bnk_batch_view_get(m->batch[g][k], &m->view[g][k]);
             if (rc == BNK_SUCCESS) batch_set_direct_stream(m->batch[g][k], m->stream[g]);
         }
-        if (rc != BNK_SUCCESS) {
-            bnk_mgpu_destroy(m);
-            return rc;
-        }
-        m->worker.emplace_back(new Worker());
-        m->crew.emplace_back(new Crew(helpers));
+        if (rc != BNK_SUCCESS) return rc;
+        m->worker.push_back(std::make_unique<Worker>());
+        m->helpers.push_back(std::make_unique<Crew>(n_helpers));
     }
     m->gpu_of.assign(cfg->max_peers, 0);
     m->slot_of.assign(cfg->max_peers, 0);
     m->peer.assign(cfg->max_peers, PeerInfo{});
     m->pkts_per_peer.assign(cfg->max_peers, 0);
     m->bytes_per_peer.assign(cfg->max_peers, 0);
-    const int rc = bnk_place_peers(nullptr, cfg->max_peers, ng, cfg->ctx.max_keypairs, m->gpu_of.data(), m->slot_of.data(), nullptr);
-    if (rc != BNK_SUCCESS) {
-        bnk_mgpu_destroy(m);
+    return bnk_place_peers(nullptr, cfg->max_peers, ng, cfg->ctx.max_keypairs, m->gpu_of.data(), m->slot_of.data(), nullptr);
+}
+
+int bnk_mgpu_create(const bnk_mgpu_cfg *cfg, bnk_mgpu **out) {
+    if (!cfg || !out || cfg->struct_size != sizeof(bnk_mgpu_cfg) || cfg->n_devices == 0 || !cfg->devices ||
+        cfg->max_pkts_per_gpu == 0 || cfg->max_peers == 0 || cfg->max_packet == 0)
+        return BNK_EINVAL;
+    *out = nullptr;
+    if ((uint64_t)cfg->n_devices * cfg->ctx.max_keypairs < cfg->max_peers) return BNK_EINVAL;
+    bnk_mgpu *m = new (std::nothrow) bnk_mgpu();
+    if (!m) return BNK_ENOMEM;
+    try {
+        const int rc = build(m, cfg);
+        if (rc == BNK_SUCCESS) *out = m;
+        else bnk_mgpu_destroy(m);
         return rc;
+    } catch (const std::exception &) { // no memory or no thread
+        bnk_mgpu_destroy(m);
+        return BNK_ENOMEM;
     }
-    *out = m;
-    return BNK_SUCCESS;
 }
 
 bnk_ctx *bnk_mgpu_ctx(bnk_mgpu *m, uint32_t g) { return (m && g < m->ctx.size()) ? m->ctx[g] : nullptr; }
@@ -578,7 +343,7 @@ static int run_shares(bnk_mgpu *m, const std::vector<std::vector<uint32_t>> &lis
         if (!lists[g].empty()) own = g;
     Latch latch(busy - 1);
     std::vector<int> rcs(ng, BNK_SUCCESS);
-    auto job = [&](uint32_t g) {
+    auto work = [&](uint32_t g) {
         const std::vector<uint32_t> &l = lists[g];
         const uint32_t n = (uint32_t)l.size();
         m->last[g] = nullptr; // nothing is in flight between calls
@@ -597,16 +362,28 @@ static int run_shares(bnk_mgpu *m, const std::vector<std::vector<uint32_t>> &lis
         };
         s.poll = [&](uint32_t slot) { return bnk_wait(m->batch[g][slot], 0); };
         // waking the helpers takes longer than copying half a megabyte
-        rcs[g] = bytes / (uint32_t)busy < (512u << 10) ? s.Drive() : m->crew[g]->Do(s);
+        rcs[g] = bytes / (uint32_t)busy < (512u << 10) ? s.Drive() : m->helpers[g]->Do(s);
+    };
+    auto job = [&](uint32_t g) {
+        try {
+            work(g);
+        } catch (const std::exception &) { // no memory, before anything was submitted
+            rcs[g] = BNK_ENOMEM;
+        }
     };
     for (uint32_t g = 0; g < ng; g++) {
         if (lists[g].empty()) continue;
         m->pkts_per_gpu[g] += lists[g].size();
         if (g == own) continue;
-        m->worker[g]->Post([&, g] {
-            job(g);
+        try {
+            m->worker[g]->Post([&, g] {
+                job(g);
+                latch.Done();
+            });
+        } catch (const std::exception &) {
+            rcs[g] = BNK_ENOMEM;
             latch.Done();
-        });
+        }
     }
     job(own);
     latch.Wait();
@@ -617,7 +394,7 @@ static int run_shares(bnk_mgpu *m, const std::vector<std::vector<uint32_t>> &lis
 
 int bnk_mgpu_seal(bnk_mgpu *m, const uint8_t *const *pkts, const uint32_t *len, const uint32_t *peer, uint32_t n,
                   uint32_t flags, int64_t now_unix_ns, uint8_t *const *out, uint32_t *out_len, uint64_t *counter,
-                  uint8_t *status) {
+                  uint8_t *status) try {
     if (!m || (n && (!pkts || !len || !peer || !out || !out_len || !status))) return BNK_EINVAL;
     std::lock_guard<std::mutex> guard(m->mu);
     std::vector<uint32_t> peer_of_pkt(n);
@@ -651,11 +428,13 @@ int bnk_mgpu_seal(bnk_mgpu *m, const uint8_t *const *pkts, const uint32_t *len, 
             if (j != i) copy_comes_next(v.ring + (size_t)(k + 1) * m->slot_bytes, out[j], v.out_len[k + 1]);
             if (v.out_len[k]) memcpy(out[i], v.ring + (size_t)k * m->slot_bytes, v.out_len[k]);
         });
+} catch (const std::exception &) { // no memory
+    return BNK_ENOMEM;
 }
 
 int bnk_mgpu_open(bnk_mgpu *m, const uint8_t *const *msgs, const uint32_t *len, uint32_t n, uint32_t flags,
                   int64_t now_unix_ns, uint8_t *const *out, uint32_t *out_len, uint64_t *counter, uint32_t *peer_out,
-                  uint8_t *status) {
+                  uint8_t *status) try {
     if (!m || (n && (!msgs || !len || !out || !out_len || !status))) return BNK_EINVAL;
     std::lock_guard<std::mutex> guard(m->mu);
     std::vector<uint32_t> peer_of_pkt(n, kNoPeer);
@@ -709,6 +488,8 @@ int bnk_mgpu_open(bnk_mgpu *m, const uint8_t *const *msgs, const uint32_t *len, 
             if (j != i) copy_comes_next(v.ring + (size_t)(k + 1) * m->slot_bytes, out[j], v.out_len[k + 1]);
             if (out_len[i]) memcpy(out[i], v.ring + (size_t)k * m->slot_bytes + 16, out_len[i]);
         });
+} catch (const std::exception &) {
+    return BNK_ENOMEM;
 }
 
 } // extern "C"
