@@ -423,7 +423,7 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
         bnk_ctx_destroy(ctx);
         return rc;
     };
-    if ((e = cudaStreamCreateWithFlags(&ctx->admin_stream, cudaStreamNonBlocking)) != cudaSuccess) return bail("stream", e);
+    if ((e = cudaStreamCreateWithPriority(&ctx->admin_stream, cudaStreamNonBlocking, ctx->prio_high)) != cudaSuccess) return bail("stream", e);
     if ((e = cudaEventCreate(&ctx->timer_start)) != cudaSuccess) return bail("event", e);
     if ((e = cudaEventCreateWithFlags(&ctx->ev_sweep, cudaEventDisableTiming)) != cudaSuccess) return bail("event", e);
     Slab tables;

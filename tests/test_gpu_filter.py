@@ -309,6 +309,49 @@ def test_rule_tables_with_many_prefix_lengths(gpu_lib, oracle, shape):
         c.close()
 
 
+@pytest.mark.parametrize("room", [False, True])  # True: both buffers of the index were made with the context
+@pytest.mark.parametrize("shape", ["hosts anywhere", "hosts of one stretch", "networks anywhere", "every length", "short only"])
+def test_rule_tables_over_the_whole_address_space(gpu_lib, oracle, shape, room):
+    """Tables whose prefixes lie anywhere (a block of the index for nearly every 65,536 addresses) or all in one such
+    stretch, the first and the last address among them, set one after the other in one context."""
+    from bnk_b200 import Context
+    from bnk_b200.device import ACL_TUPLE_DTYPE
+
+    rng = np.random.default_rng(len(shape))
+    k = 90_000 if shape == "hosts anywhere" else 8000
+    bits = {"hosts": np.full(k, 32), "networks": rng.integers(17, 25, k), "every": rng.integers(0, 33, k), "short": rng.integers(13, 17, k)}[shape.split()[0]]
+    if shape == "every length":
+        bits[bits < 9] += 12  # (or everything is allowed)
+    addr = rng.integers(0, 1 << 32, k)
+    if shape == "hosts of one stretch":
+        addr = 0xC0A80000 + rng.integers(0, 1 << 16, k)
+    addr[:2] = 0, 0xFFFFFFFF
+    if shape == "every length":
+        addr[k // 2:] = addr[:k // 2] ^ rng.integers(0, 1 << 12, k // 2)  # one inside the other
+    addr &= (0xFFFFFFFF << (32 - bits)) & 0xFFFFFFFF
+    n = 6000
+    h = np.zeros((n, 28), np.uint8)
+    for i in range(n):
+        src = int(addr[rng.integers(0, k)] if i > 3 else (0, 0xFFFFFFFF, 0x80000000, 0x0000FFFF)[i])
+        src = (src + int(rng.choice([0, 0, 1, 255, 256, 65535, 1 << 20]))) & 0xFFFFFFFF
+        h[i] = np.frombuffer(RC.tcp(src, RC.SELF, 40000, 443)[:28], np.uint8)
+    lens = np.full(n, 28, np.uint32)
+    with Context(max_keypairs=1, flow_capacity=16, max_acl_tuples=100_000 if room else 0) as c:
+        b = c.batch(n, n * 48)
+        b.ring.reshape(n, 48)[:, 16:44] = h
+        b.off[:], b.len[:] = np.arange(n) * 48, lens
+        for part in (slice(0, k), slice(0, k // 3), slice(0, 1), slice(0, 0), slice(k // 2, k)):
+            t = np.zeros(len(addr[part]), ACL_TUPLE_DTYPE)
+            t["addr"], t["prefix_len"], t["proto"], t["port_first"], t["port_last"] = addr[part], bits[part], 6, 443, 443
+            c.acl_set(True, t)
+            chk = oracle.Filter()
+            chk.set_rules([([(int(x), int(y)) for x, y in zip(addr[part], bits[part])], "tcp", [(443, 443)])])
+            want = chk.check_batch_mt(np.ascontiguousarray(h), 28, lens, RC.T0)
+            b.filter_check(n, RC.T0)
+            assert np.array_equal(b.status == 0, want != 0), np.flatnonzero((b.status == 0) != (want != 0))[:5]
+            assert len(t) < 4000 or 500 < (want != 0).sum() < n
+
+
 @pytest.mark.parametrize("n", [1, 127, 128, 129, 5000])  # a CTA's statuses leave as one line
 def test_nested_prefixes_and_merged_port_ranges(gpu_lib, oracle, n):
     """Prefixes of every length one inside the other, around the steps of the index (16, 24 bits), each with several port
