@@ -287,10 +287,11 @@ cudaError_t catch_up(bnk_batch *b, cudaStream_t s) {
     if (e == cudaSuccess) b->stale_pkts = b->stale_src = 0;
     return e;
 }
-// In front of a submit's own upload of n packets, if it makes one: what that does not cover catches up first.  Returns in
-// `all` whether the upload has to bring every descriptor field (and is then to be followed by caught_up).
-cudaError_t catch_up_beside(bnk_batch *b, uint32_t n, bool uploads, cudaStream_t s, bool &all) {
-    const bool covers = uploads && n >= b->stale_pkts && b->stale_src == 0;
+// In front of a submit's own upload of n packets, if it makes one: what that does not cover catches up first.  Not so when the
+// results come down: the host arrays then hold all there is, and what is behind may stay so.  Returns in `all` whether the
+// upload has to bring every descriptor field (and is then to be followed by caught_up).
+cudaError_t catch_up_beside(bnk_batch *b, uint32_t n, bool uploads, bool results_down, cudaStream_t s, bool &all) {
+    const bool covers = uploads && (results_down || (n >= b->stale_pkts && b->stale_src == 0));
     const cudaError_t e = covers ? cudaSuccess : catch_up(b, s);
     all = b->stale_pkts != 0;
     return e;
@@ -946,7 +947,7 @@ int bnk_batch_upload(bnk_batch *b, uint32_t npkts) {
     bnk_ctx *ctx = b->ctx;
     const size_t n = npkts;
     bool all;
-    CK(ctx, catch_up_beside(b, npkts, true, b->stream, all));
+    CK(ctx, catch_up_beside(b, npkts, true, false, b->stream, all));
     const uint64_t ext = ring_extent(b, npkts, 64);
     CK(ctx, ring_up(b, ext, false, b->stream));
     if (n) {
@@ -1105,7 +1106,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
             return seal_direct(b, npkts, bytes, flags, now_unix_ns, true);
     }
     bool all;
-    CK(ctx, catch_up_beside(b, npkts, !(flags & BNK_F_NO_H2D), s, all));
+    CK(ctx, catch_up_beside(b, npkts, !(flags & BNK_F_NO_H2D), !(flags & BNK_F_NO_D2H), s, all));
     if (!(flags & BNK_F_NO_H2D) && n) {
         CK(ctx, ring_up(b, ext, b->joint_copy, s));
         if (!b->joint_copy)
@@ -1309,7 +1310,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     // BNK_F_USE_OUT_LEN reads the lengths a seal left on the device: an upload beside it must not bring the
     // host's out_len along, so it moves the fields one by one instead of the whole slab.
     bool all;
-    CK(ctx, catch_up_beside(b, npkts, !(flags & BNK_F_NO_H2D), s, all));
+    CK(ctx, catch_up_beside(b, npkts, !(flags & BNK_F_NO_H2D), !(flags & BNK_F_NO_D2H), s, all));
     if (!(flags & BNK_F_NO_H2D) && n) {
         const bool joint = b->joint_copy && (all || !(flags & BNK_F_USE_OUT_LEN));
         CK(ctx, ring_up(b, ext, joint, s));
@@ -1382,9 +1383,9 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
 // while the next is looked through; pieces end on pages like those of a large batch.  (The highest byte only grows, so
 // packets in any order are covered.)  900,000 headers checked 1337 us with the pass in front, 1023 so, of which the link
 // needs 920 at 55 GB/s; 300,000 495 and 378, 30,000 69 and 58.
-static int upload_heads(bnk_batch *b, uint32_t n, cudaStream_t s) {
+static int upload_heads(bnk_batch *b, uint32_t n, bool results_down, cudaStream_t s) {
     bnk_ctx *ctx = b->ctx;
-    CK(ctx, catch_up(b, s));
+    if (!results_down) CK(ctx, catch_up(b, s)); // (see catch_up_beside)
     CK(ctx, desc_copy(b, n, D_OFF, D_LEN, true, s));
     uint64_t up = 0, ext = 0;
     for (uint32_t at = 0, k = kHeadsFirst; at < n; at += k, k = std::min(2 * k, kHeadsMost)) {
@@ -1412,7 +1413,7 @@ int bnk_filter_note_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t
     const bool upload = npkts && !(flags & BNK_F_NO_H2D);
     const bool direct = upload && heads_direct(b, npkts, flags);
     if (npkts && !upload) CK(ctx, catch_up(b, s));
-    if (!direct && upload && (rc = upload_heads(b, npkts, s)) != BNK_SUCCESS) return rc;
+    if (!direct && upload && (rc = upload_heads(b, npkts, true, s)) != BNK_SUCCESS) return rc;
     HostAlias alias(b, direct, npkts);
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     const bool note = npkts && ctx->ft.enforce && ctx->ft.flow_capacity; // filter.go:192-194
@@ -1441,7 +1442,7 @@ int bnk_filter_check_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_
     const bool upload = npkts && !(flags & BNK_F_NO_H2D);
     const bool direct = upload && heads_direct(b, npkts, flags);
     if (npkts && !upload) CK(ctx, catch_up(b, s));
-    if (!direct && upload && (rc = upload_heads(b, npkts, s)) != BNK_SUCCESS) return rc;
+    if (!direct && upload && (rc = upload_heads(b, npkts, !(flags & BNK_F_NO_D2H), s)) != BNK_SUCCESS) return rc;
     HostAlias alias(b, direct, npkts);
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     CK(ctx, flow_check_begins(b, now_unix_ns, s));
@@ -1469,7 +1470,7 @@ int bnk_classify_submit(bnk_batch *b, uint32_t npkts, uint32_t flags) {
     if (direct) b->stale_src = std::max(b->stale_src, npkts);
     if (npkts && !upload) CK(ctx, catch_up(b, s));
     if (!direct && upload) {
-        if ((rc = upload_heads(b, npkts, s)) != BNK_SUCCESS) return rc;
+        if ((rc = upload_heads(b, npkts, !(flags & BNK_F_NO_D2H), s)) != BNK_SUCCESS) return rc;
         CK(ctx, cudaMemcpyAsync(b->dev.src_addr, b->host.src_addr, n * BNK_SRC_ADDR_STRIDE, cudaMemcpyHostToDevice, s));
     }
     HostAlias alias(b, direct, npkts);

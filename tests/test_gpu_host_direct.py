@@ -161,7 +161,7 @@ def test_classify_and_gso_after_a_batch_without_copies(gpu_lib, oracle):
         c.close()
 
 
-@pytest.mark.parametrize("between", ["seal", "open", "upload", "note", "check", "classify", "classify all", "split"])
+@pytest.mark.parametrize("between", ["seal", "open", "upload", "note", "check", "classify", "classify all", "split", "copied seal"])
 def test_a_small_call_between_does_not_hide_what_is_behind(gpu_lib, oracle, between):
     """1000 packets sealed in place, then a copied call for ten of the batch, then all of them from the device: the ring and
     the descriptors that the device works on are those of the host arrays, beyond the ten too."""
@@ -191,6 +191,15 @@ def test_a_small_call_between_does_not_hide_what_is_behind(gpu_lib, oracle, betw
                 b.classify(few, F_NO_D2H)
         elif between == "split":
             b.gso_split(np.zeros(0, GSO_SUPER_DTYPE), few)
+        elif between == "copied seal":  # results come down: nothing has to catch up for it, everything for what follows
+            b.len[:few] = 200
+            others = [c.batch(600, 600 * 800) for _ in range(4)]
+            for o in others:
+                o.seal(600, wait=False)
+            b.seal(few)
+            b.len[:few] = b.out_len[:few] - 32
+            for o in others:
+                o.wait()
         elif between == "upload":
             b.upload(few)
         elif between == "note":
