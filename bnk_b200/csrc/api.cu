@@ -146,16 +146,19 @@ cudaError_t tally_if_asked(bnk_batch *b, uint32_t npkts, uint32_t flags, cudaStr
 // download in a row: 190 KB 17 us against 33, 1.6 MB 56 against 82, 6.4 MB 177 against 253, 24 MB 613 against 916,
 // 190 MB 4.74 ms against 7.0.  Chunks of one batch over three streams, so that the copy engines run both ways, take
 // 77 us at 1.6 MB, 234 at 6.4 MB, 680 at 24 MB and 4.55 ms at 190 MB: only far up they are the faster form.
-// With several batches in flight the engines overlap the batches' copies with each other (48 GB/s each way together),
-// and many kernels on the link at once slow each other down, so a batch runs this way only if nothing else is in
-// flight, or if all that run this way together stay below kDirectTogether bytes and few others are in flight: for a
-// batch of more than 384 KB three, because SMs move 28-33 GB/s each way over the link and the engines, kept busy by that
-// many batches, 46-48.  Queue of 1024-packet batches, Gbit/s with up to sixteen others / three / none in place beyond
-// 384 KB: 32 callers x 4 calls 195 / 255 / 243, 16 x 4 193 / 205 / 197, 16 x 2 (smaller batches) 182 / 170 / 146 (the last
-// column by an earlier build).
+// With several batches in flight the engines overlap the batches' copies with each other (48 GB/s each way together), so a
+// large batch runs this way only if nothing else is in flight, or if all that run this way together stay below
+// kDirectTogether bytes and at most two others are in flight: SMs move 28-33 GB/s each way over the link and the engines,
+// kept busy by that many batches, 46-48.  Queue of 1024-packet batches, Gbit/s with up to fifteen others / two in place
+// beyond 384 KB: 32 callers x 4 calls 195 / 255, 16 x 4 193 / 205, 16 x 2 (smaller batches) 182 / 170.
+// A small batch always does.  Its copies are too small for the engines, and in-place kernels beside copied batches are
+// slower than either alone.  128 x 1420 B a batch, threads x batches each in flight, Gbit/s with at most 16 in place / all
+// (best of five to seven; a host that stalls halves single runs): 16 x 1 176 / 177, 12 x 2 118 / 187, 16 x 2 118 / 196, 8 x
+// 4 121 / 199, 16 x 4 112 / 195, 32 x 2 97 / 160, 16 x 8 106 / 171, 32 x 4 93 / 148; 256 x 1420 B 16 x 2 146 / 222, 32 x 4 97 /
+// 198; 128 x 300 B 16 x 2 40 / 95.
 constexpr uint64_t kDirectTogether = 6ull << 20;
 constexpr uint64_t kDirectSmall = 384u << 10;
-constexpr int kDirectBatches = 16, kDirectLarge = 3;
+constexpr int kDirectOthers = 2;
 bool host_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, uint64_t ext) {
     bnk_ctx *ctx = b->ctx;
     if (ctx->host_direct_bytes == 0 || npkts == 0 || (flags & (BNK_F_NO_H2D | BNK_F_NO_D2H | BNK_F_USE_OUT_LEN)) ||
@@ -163,8 +166,7 @@ bool host_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, uint64_t ext) {
         return false;
     const uint64_t together = ctx->direct_in_flight.load(std::memory_order_relaxed) - b->direct_counted;
     const int others = ctx->in_flight.load(std::memory_order_relaxed) - (b->counted ? 1 : 0);
-    const int most = ext > kDirectSmall ? kDirectLarge : kDirectBatches;
-    if (others > 0 && (together + ext > kDirectTogether || others >= most)) return false;
+    if (ext > kDirectSmall && others > 0 && (together + ext > kDirectTogether || others > kDirectOthers)) return false;
     ctx->direct_in_flight.fetch_add(ext - b->direct_counted, std::memory_order_relaxed);
     b->direct_counted = ext;
     return true;
