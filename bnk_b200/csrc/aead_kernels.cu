@@ -1089,8 +1089,10 @@ cudaError_t launch_wpp(const AeadArgs &a, uint32_t ctas, const HostDesc *h, cuda
         memcpy(d.slot, h->slot, a.n * sizeof(uint32_t));
         return launch_kernel(early, kernel, dim3(ctas), dim3(32 * kWppWarps), s, a, d);
     };
-    // A few packets, half an upstream batch, one with what arrived twice, and as many as there may be.  With room for 256
-    // alone nine packets of 300 B took 57.7 us sealed and opened, 128 x 1420 B 24.2 sealed; with these 54.0 and 23.4.
+    // The cost of a launch grows with its parameters, 12 bytes a packet here: a quarter of a kilobyte, three quarters, two and
+    // three kilobytes.  160 leaves a read of the upstream size (128) room for what a receive call brings beyond it.  With
+    // room for 256 alone nine packets of 300 B took 57.7 us sealed and opened, 128 x 1420 B 24.2 sealed; with these 54.0
+    // and 23.4.
     if (a.n <= 16) return with(InlineDesc<16>{}, aead_wpp_kernel<OPEN, NOTE, 16>);
     if (a.n <= 64) return with(InlineDesc<64>{}, aead_wpp_kernel<OPEN, NOTE, 64>);
     if (a.n <= 160) return with(InlineDesc<160>{}, aead_wpp_kernel<OPEN, NOTE, 160>);

@@ -404,17 +404,20 @@ int bnk_queue_stats_get(bnk_queue *q, uint64_t *gpu_batches, uint64_t *packets, 
 int bnk_place_peers(const uint64_t *load, uint32_t n_peers, uint32_t n_gpus, uint32_t max_per_gpu, uint32_t *gpu_of,
                     uint32_t *slot_of, uint64_t *load_per_gpu);
 
-/* The dispatcher: one context per listed device, driven by one host thread each.  It stands where the
+/* The dispatcher: one context per listed device, driven by one host thread each, with helper threads for the
+ * copies between the caller's buffers and the pinned rings (as many as the process may have).  It stands where the
  * reference's device.NewDevice stands when a box has several GPUs: bnk_mgpu_seal / bnk_mgpu_open take one
  * mixed batch in the caller's buffers (a tun.Device.Read or conn.ReceiveFunc batch, or many of them), route
  * every packet to its peer's GPU, keep batch order inside each peer, run the per-GPU submits side by side and
- * hand the results back in the caller's order.  Plain cudaMemcpyAsync per GPU; no peer access, no collective. */
+ * hand the results back in the caller's order.  A GPU's share of a call goes in pieces, several of them under way at
+ * once: out[i] may be where packet i of the input lies, but must not overlap another packet's input.  No peer access,
+ * no collective. */
 typedef struct bnk_mgpu bnk_mgpu;
 typedef struct bnk_mgpu_cfg {
     uint32_t struct_size;       /* sizeof(bnk_mgpu_cfg) */
     uint32_t n_devices;
     const int32_t *devices;     /* CUDA ordinals; one listed twice gets two contexts (for tests on one GPU) */
-    uint32_t max_pkts_per_gpu;  /* packets one submit of one GPU carries; longer batches go in rounds */
+    uint32_t max_pkts_per_gpu;  /* most packets one submit of one GPU carries; a share goes in pieces of about 3 MB at most */
     uint32_t max_packet;        /* longest plaintext packet */
     uint32_t max_peers;         /* peers numbered 0 .. max_peers-1 */
     uint32_t reserved;
@@ -438,8 +441,8 @@ int bnk_mgpu_acl_set(bnk_mgpu *m, int enforce, const bnk_acl_tuple *tuples, size
 /* Seals packets pkts[i][0 .. len[i]) of peer peer[i]; the message goes to out[i] (room for len + 48 bytes),
  * its length to out_len[i], the nonce used to counter[i] (may be NULL), the outcome to status[i].  flags as for
  * bnk_seal_submit; counters are always taken from the peers' send counters.  A peer that is not set yields
- * BNK_PKT_NO_KEYPAIR.  Blocks until every GPU has finished.  One GPU's share is worked on by the calling thread
- * itself (with a single busy GPU nothing is handed to another thread); like the other calls of the library this
+ * BNK_PKT_NO_KEYPAIR.  Blocks until every GPU has finished.  One GPU's share is driven by the calling thread
+ * itself, with helpers for the copies from half a megabyte a GPU on; like the other calls of the library this
  * leaves the thread's current CUDA device set to a GPU of the dispatcher. */
 int bnk_mgpu_seal(bnk_mgpu *m, const uint8_t *const *pkts, const uint32_t *len, const uint32_t *peer, uint32_t n,
                   uint32_t flags, int64_t now_unix_ns, uint8_t *const *out, uint32_t *out_len, uint64_t *counter,

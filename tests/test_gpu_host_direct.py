@@ -1,4 +1,4 @@
-"""Small batches run on the caller's pinned buffers (no copies); larger ones through the copy engines.  Both
+"""Batches run on the caller's pinned buffers (no copies) or through the copy engines.  Both
 ways must give the same bytes, and a batch that ran without copies must still chain into device-resident calls."""
 import os
 
@@ -34,7 +34,7 @@ def _load(b, rng, n, n_peers):
     return off, sizes
 
 
-@pytest.mark.parametrize("n", [1, 7, 64, 200, 256, 300])  # 300: beyond the mode's packet limit, copied both times
+@pytest.mark.parametrize("n", [1, 7, 64, 200, 256, 300])  # 300: more than go along with a launch
 def test_same_bytes_with_and_without_copies(gpu_lib, oracle, n):
     from bnk_b200.device import F_ASSIGN_COUNTERS, F_REPLAY
 

@@ -20,9 +20,10 @@ def _expected_counters(slots, start, max_slots):
     return out, nxt
 
 
-# 1 / 256 / 257: nonces inside the seal kernel or by the grouping launch; 512..32768: one, two, four, eight packets a
-# thread and one to eight CTAs; 32769: the chain of kernels.  Keypairs: one, two and three digits.
-@pytest.mark.parametrize("n,n_peers", [(1, 1), (256, 40), (257, 40), (1025, 600), (4097, 5), (8193, 3000), (32768, 300_000),
+# 1 / 256 / 257: nonces inside the seal kernel or by the grouping launch; up to 1024 one CTA with one or two packets a thread,
+# then 4, 8, 16 CTAs with one and 16 with two and four; 32769: the chain of kernels.  Keypairs: one, two and three digits.
+@pytest.mark.parametrize("n,n_peers", [(1, 1), (256, 40), (257, 40), (512, 3), (513, 3), (1024, 600), (1025, 600), (2048, 9), (2049, 2000),
+                                       (4096, 5), (4097, 5), (8192, 700), (8193, 3000), (16_384, 50), (16_385, 600_000), (32768, 300_000),
                                        (32769, 70)])
 def test_counters_and_replay_at_the_edges_of_a_split(gpu_lib, oracle, n, n_peers):
     from bnk_b200 import Context
