@@ -435,3 +435,54 @@ def test_packets_close_together_go_up_stretch_by_stretch(gpu_lib, oracle, n, shu
         assert np.array_equal(b.status == 0, want), np.flatnonzero((b.status == 0) != want)[:5]
         assert 0.1 < want.mean() < 0.4
         b.close()
+
+
+@pytest.mark.parametrize("n", [1, 511, 512, 513, 799])  # from 512 on, two lanes read a head that lies in pinned memory
+def test_heads_of_packets_anywhere_in_the_ring(gpu_lib, oracle, n):
+    """Whole packets in any order, at every 16 bytes of a line and up to the ring's last byte, some with IP options (ports
+    beyond the first 32 bytes), some cut short, misplaced or outside the ring: flows and verdicts are the checker's."""
+    from bnk_b200 import Context
+    from bnk_b200.filter import CompiledRule, PortRange, flatten_rules
+    from tests.helpers import flows_equal
+
+    rng = np.random.default_rng(n)
+
+    def packet(src, dst, sport, dport):
+        p = bytearray([RC.udp, RC.tcp][int(rng.integers(0, 2))](src, dst, sport, dport)[:28])
+        words = int(rng.choice([5, 5, 5, 6, 7, 8, 15]))  # options between the header and the ports
+        p[0] = 0x40 | words
+        p = p[:20] + bytes(rng.integers(0, 256, 4 * words - 20, dtype=np.uint8)) + p[20:] + bytes(int(rng.integers(0, 200)))
+        return bytes(p[:int(rng.choice([0, 1, 19, 20, 4 * words, 4 * words + 3, 4 * words + 4]))] if rng.random() < 0.1 else p)
+
+    peers = RC.ip("100.64.1.0") + rng.integers(0, 4, n)
+    out = [packet(RC.SELF, int(p), 1000 + i, 53) for i, p in enumerate(peers)]
+    into = [packet(int(p), RC.SELF, int(rng.choice([53, 54, 77])), 1000 + i) for i, p in enumerate(peers)]
+    chk = oracle.Filter()
+    chk.set_rules([([(RC.ip("100.64.1.2"), 32)], "tcp", [(1000, 1000 + n // 2)])])
+    with Context(max_keypairs=1, flow_capacity=1 << 12) as c:
+        c.acl_set(True, flatten_rules([CompiledRule(srcs=["100.64.1.2/32"], proto="tcp", ports=[PortRange(1000, 1000 + n // 2)])]))
+        for inbound, pkts in ((False, out), (True, into)):
+            order = rng.permutation(n)
+            off, at = np.zeros(n, np.uint32), 0
+            for i in order:
+                off[i] = at
+                at += 16 + ((len(pkts[i]) + 15) & ~15) + 16 * int(rng.integers(0, 9))
+            ring = at - int(at - off[order[-1]] - 16 - ((len(pkts[order[-1]]) + 15) & ~15))  # the last packet ends where the ring does
+            b = c.batch(n, ring)
+            for i in range(n):
+                b.ring[int(off[i]) + 16:int(off[i]) + 16 + len(pkts[i])] = np.frombuffer(pkts[i], np.uint8)
+            wrong = rng.random(n) < 0.05
+            bad = np.where(rng.random(n) < 0.5, off + 4, ring & 0xFFFFFFF0).astype(np.uint32)  # misplaced, or nothing behind it
+            b.off[:], b.len[:] = np.where(wrong, bad, off), [len(p) for p in pkts]
+            if inbound:
+                b.filter_check(n, RC.T0 + 1)
+                want = np.array([not w and chk.check_inbound(p, RC.T0 + 1) for w, p in zip(wrong, pkts)])
+                assert np.array_equal(b.status == 0, want), np.flatnonzero((b.status == 0) != want)[:5]
+                assert n < 500 or 0.1 * n < want.sum() < 0.5 * n  # a sixth replies, a sixteenth by the rule
+            else:
+                b.filter_note(n, RC.T0)
+                for w, p in zip(wrong, pkts):
+                    if not w:
+                        chk.note_outbound(p, RC.T0)
+            assert flows_equal(c.flows_export(), chk.flows())
+            b.close()
