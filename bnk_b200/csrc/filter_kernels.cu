@@ -19,44 +19,49 @@
 
 namespace {
 
-// filter.go:71-106 of a packet per lane: the one at ring[o + 16 .. o + 16 + len), which has to lie in the ring (`have`: the
-// lane has one).  By all lanes of a warp.  Its first 32 bytes, which hold all of a packet without IP options, are asked for
-// together: when the ring is in host memory a dependent read is another trip over the link (8192 whole packets noted and
-// checked: 95 us with three dependent reads, 87 with one).
-// PAIRS: two lanes ask for a packet's two 16-byte halves in one instruction, so that halves in different sectors of one line
-// are one request to the link all the same; a lane that asks for both makes two of them.  8192 whole packets noted and checked
-// (two calls) 98 -> 76 us, 16,000 x 400 B 158 -> 106.  A ring on the device (1,000,000 headers 47.4 us, with pairs 48.3) and
-// few packets (60 noted and checked 32.9 us, 33.9) are not bound by requests, and the exchange between the lanes costs.
+// filter.go:71-106 of the packet at ring[o + 16 .. o + 16 + len), which has to lie in the ring.  Its first 32 bytes, which
+// hold all of a packet without IP options, are asked for together: when the ring is in host memory a dependent read is
+// another trip over the link (8192 whole packets noted and checked: 95 us with three dependent reads, 87 with one).
+__device__ __forceinline__ bool parse_ipv4(const uint8_t *ring, uint32_t o, uint32_t len, uint64_t ring_bytes, Parsed &out) {
+    if ((o & 15u) || (uint64_t)o + 16u + len > ring_bytes || len < 20) return false;
+    const uint8_t *const p = ring + o + 16; // 16-byte aligned
+    const bool both = (uint64_t)o + 48 <= ring_bytes;
+    const uint4 a = *reinterpret_cast<const uint4 *>(p);
+    uint4 b = make_uint4(0, 0, 0, 0);
+    if (both) b = *reinterpret_cast<const uint4 *>(p + 16);
+    else b.x = *reinterpret_cast<const uint32_t *>(p + 16);
+    const uint32_t at = parse_ipv4_words(a.x, a.z, a.w, b.x, len, out);
+    if (at == kParseBad) return false;
+    if (at) parse_ports(both && at == 20 ? b.y : *reinterpret_cast<const uint32_t *>(p + at), out);
+    return true;
+}
+// The same for a packet per lane (`have`: the lane has one), by all lanes of a warp: two lanes ask for a packet's two 16-byte
+// halves in one instruction, so that halves in different sectors of one line are one request to the link all the same; a
+// lane that asks for both makes two of them.  8192 whole packets noted and checked (two calls) 98 -> 76 us, 16,000 x 400 B
+// 158 -> 106.  A ring on the device (1,000,000 headers 47.4 us, with pairs 48.3) and few packets (60 noted and checked 32.9
+// us, 33.9) are not bound by requests, and the exchange between the lanes costs.  (One parser for both, taking the two
+// halves, made the plain kernels up to 1 us slower on a few packets: those keep the code above.)
 constexpr uint32_t kPairsFrom = 512;
 struct HeadStage { // of one warp
     uint4 half[32][2];
 };
-template <bool PAIRS>
-__device__ __forceinline__ bool parse_ipv4_warp(HeadStage *stage, const uint8_t *ring, bool have, uint32_t o, uint32_t len, uint64_t ring_bytes,
-                                                Parsed &out) {
+__device__ __forceinline__ bool parse_ipv4_pairs(HeadStage &stage, const uint8_t *ring, bool have, uint32_t o, uint32_t len, uint64_t ring_bytes,
+                                                 Parsed &out) {
     // (offsets and the ring's size are multiples of 16, so 20 bytes in the ring behind o + 16 are 32)
     have = have && !(o & 15u) && (uint64_t)o + 16u + len <= ring_bytes && len >= 20;
-    uint4 a = make_uint4(0, 0, 0, 0), b = a;
-    if (PAIRS) {
-        const uint32_t lane = threadIdx.x & 31u, with = __ballot_sync(0xffffffffu, have);
-        uint4 v[2];
+    const uint32_t lane = threadIdx.x & 31u, with = __ballot_sync(0xffffffffu, have);
+    uint4 v[2];
 #pragma unroll
-        for (uint32_t h = 0; h < 2; h++) {
-            const uint32_t p = 16u * h + (lane >> 1), at = __shfl_sync(0xffffffffu, o, p);
-            v[h] = make_uint4(0, 0, 0, 0);
-            if ((with >> p) & 1u) v[h] = *reinterpret_cast<const uint4 *>(ring + at + 16u + 16u * (lane & 1u)); // 16-byte aligned
-        }
-#pragma unroll
-        for (uint32_t h = 0; h < 2; h++) stage->half[16u * h + (lane >> 1)][lane & 1u] = v[h];
-        __syncwarp();
-        a = stage->half[lane][0];
-        b = stage->half[lane][1];
-    } else if (have) {
-        const uint4 *const p = reinterpret_cast<const uint4 *>(ring + o + 16u);
-        a = p[0];
-        b = p[1];
+    for (uint32_t h = 0; h < 2; h++) {
+        const uint32_t p = 16u * h + (lane >> 1), at = __shfl_sync(0xffffffffu, o, p);
+        v[h] = make_uint4(0, 0, 0, 0);
+        if ((with >> p) & 1u) v[h] = *reinterpret_cast<const uint4 *>(ring + at + 16u + 16u * (lane & 1u)); // 16-byte aligned
     }
+#pragma unroll
+    for (uint32_t h = 0; h < 2; h++) stage.half[16u * h + (lane >> 1)][lane & 1u] = v[h];
+    __syncwarp();
     if (!have) return false;
+    const uint4 a = stage.half[lane][0], b = stage.half[lane][1];
     const uint32_t at = parse_ipv4_words(a.x, a.z, a.w, b.x, len, out);
     if (at == kParseBad) return false;
     if (at) parse_ports(at == 20 ? b.y : *reinterpret_cast<const uint32_t *>(ring + o + 16u + at), out);
@@ -69,10 +74,16 @@ __global__ void __launch_bounds__(128) filter_note_kernel(const __grid_constant_
                                    const uint32_t *len, uint32_t n, uint64_t ring_bytes, long long now, FlowReport *report, Done done) {
     let_next_kernel_start();
     wait_for_kernel_in_front();
-    __shared__ HeadStage heads[PAIRS ? 4 : 1];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     Parsed p;
-    if (parse_ipv4_warp<PAIRS>(&heads[PAIRS ? threadIdx.x >> 5 : 0u], ring, i < n, i < n ? off[i] : 0u, i < n ? len[i] : 0u, ring_bytes, p)) {
+    bool parses;
+    if constexpr (PAIRS) {
+        __shared__ HeadStage heads[4];
+        parses = parse_ipv4_pairs(heads[threadIdx.x >> 5], ring, i < n, i < n ? off[i] : 0u, i < n ? len[i] : 0u, ring_bytes, p);
+    } else {
+        parses = i < n && parse_ipv4(ring, off[i], len[i], ring_bytes, p);
+    }
+    if (parses) {
         FlowNote note;
         note.begin(ft, p, now);
         note.place(ft);
@@ -167,16 +178,23 @@ __global__ void __launch_bounds__(128) filter_check_kernel(const __grid_constant
     let_next_kernel_start();
     wait_for_kernel_in_front();
     __shared__ uint32_t line[32];
-    __shared__ HeadStage heads[PAIRS ? 4 : 1];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool have = i < n && !(only_status_ok && status[i] != BNK_PKT_OK);
-    Parsed p;
-    bool parses = false;
-    if (ft.enforce)
-        parses = parse_ipv4_warp<PAIRS>(&heads[PAIRS ? threadIdx.x >> 5 : 0u], ring, have, have ? off[i] : 0u, have ? len[i] : 0u, ring_bytes, p);
+    uint8_t verdict = BNK_PKT_OK; // filter.go:124-126: allow-all passes even unparseable packets
+    if constexpr (PAIRS) {
+        __shared__ HeadStage heads[4];
+        Parsed p;
+        if (ft.enforce && !parse_ipv4_pairs(heads[threadIdx.x >> 5], ring, have, have ? off[i] : 0u, have ? len[i] : 0u, ring_bytes, p))
+            verdict = BNK_PKT_FILTER_DENY;
+        else if (ft.enforce)
+            verdict = filter_verdict(ft, p, now);
+    }
     if (have) {
-        uint8_t verdict = BNK_PKT_OK; // filter.go:124-126: allow-all passes even unparseable packets
-        if (ft.enforce) verdict = parses ? filter_verdict(ft, p, now) : (uint8_t)BNK_PKT_FILTER_DENY;
+        if constexpr (!PAIRS) {
+            Parsed p;
+            if (ft.enforce)
+                verdict = parse_ipv4(ring, off[i], len[i], ring_bytes, p) ? filter_verdict(ft, p, now) : (uint8_t)BNK_PKT_FILTER_DENY;
+        }
         status[i] = verdict;
         reinterpret_cast<uint8_t *>(line)[threadIdx.x] = verdict;
     }
