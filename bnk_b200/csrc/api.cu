@@ -118,10 +118,23 @@ struct SubmitScope {
 };
 void submit_over(bnk_batch *b) { // waited for, or going away
     b->in_flight = false;
+    launch_graph_give(b->graph);
+    b->graph = nullptr;
     if (b->counted) b->ctx->in_flight.fetch_sub(1, std::memory_order_relaxed);
     b->counted = false;
     if (b->direct_counted) b->ctx->direct_in_flight.fetch_sub(b->direct_counted, std::memory_order_relaxed);
     b->direct_counted = 0;
+}
+// Launches what a submit has gathered (launch.h).  Through a graph while at most two other batches are in flight; more of
+// them come from several threads.
+constexpr int kGraphOthers = 2;
+bool few_in_flight(const bnk_batch *b) {
+    return b->ctx->launch_graphs && b->ctx->in_flight.load(std::memory_order_relaxed) - (b->counted ? 1 : 0) <= kGraphOthers;
+}
+cudaError_t send_launches(bnk_batch *b, Launches &all) {
+    launch_graph_give(b->graph); // (of a submit that nobody waited for)
+    b->graph = nullptr;
+    return all.send(b->graph);
 }
 // For the kernel that is the submit's last piece of work: bnk_wait will watch for it.
 Done watch_for(bnk_batch *b) {
@@ -413,6 +426,9 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     ctx->pieces_from = 24u << 20;
     if (const char *m = getenv("BNK_PIECES_FROM")) // tuning aid: ring extent from which a batch that is alone goes in pieces
         ctx->pieces_from = strtoull(m, nullptr, 0);
+    ctx->launch_graphs = true;
+    if (const char *m = getenv("BNK_LAUNCH_GRAPHS")) // tuning and test aid: 0 = every launch by itself
+        ctx->launch_graphs = strtoul(m, nullptr, 0) != 0;
     ctx->aead_side_stream_from = 1u << 18; // below, the seal/open launch is too short for the hand-over between streams to pay
     if (const char *m = getenv("BNK_AEAD_SIDE_STREAM_FROM")) // tuning aid: 0 = seal/open always on the batch's own stream
         ctx->aead_side_stream_from = (uint32_t)strtoul(m, nullptr, 0);
@@ -420,6 +436,7 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     cudaDeviceGetStreamPriorityRange(&ctx->prio_low, &ctx->prio_high);
     ctx->kt = KeypairTables{};
     ctx->ft = FilterTables{};
+    launch_graphs_context(ctx->device, true);
     const size_t k = cfg->max_keypairs;
     auto bail = [&](const char *what, cudaError_t err) {
         int rc = fail(nullptr, BNK_ECUDA, what, err);
@@ -464,6 +481,7 @@ int bnk_ctx_destroy(bnk_ctx *ctx) {
     if (!ctx) return BNK_EINVAL;
     cudaSetDevice(ctx->device);
     cudaDeviceSynchronize();
+    launch_graphs_context(ctx->device, false);
     cudaFree(ctx->kt.send_keys); // all of the tables' arrays
     filter_tables_free(ctx);
     if (ctx->timer_start) cudaEventDestroy(ctx->timer_start);
@@ -987,6 +1005,7 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     const bnk_batch_view &h = b->host;
     const DeviceBatch &d = b->dev;
     CK(ctx, order_kernels_begin(b));
+    Launches all(s, !timed && !stats && few_in_flight(b));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, false, nullptr);
     a.over_link = true;
@@ -1038,6 +1057,8 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
     CK(ctx, launch_seal(a, s, ctx));
     if (timed) CK(ctx, cudaEventRecord(b->a_end, s));
+    if (!sweep) CK(ctx, send_launches(b, all));
+    else CK(ctx, all.stop()); // more than launches follow
     if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, done, s));
     else if (note && !done.flag) CK(ctx, launch_flow_report(b, s));
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
@@ -1183,7 +1204,9 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     const bool replay = (flags & BNK_F_REPLAY) != 0, checks = (flags & (BNK_F_INNER_CHECK | BNK_F_CHECK_INBOUND)) != 0;
     const bnk_batch_view &h = b->host;
     b->stale_pkts = std::max(b->stale_pkts, npkts);
+    const bool one_launch = npkts <= kGroupMax || !replay; // behind the open kernel
     CK(ctx, order_kernels_begin(b));
+    Launches all(s, !timed && !stats && one_launch && few_in_flight(b));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, true, nullptr);
     a.over_link = a.from_host = true;
@@ -1212,7 +1235,6 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
         a.res[1] = AeadResults{nullptr, b->dev.out_len, b->dev.status, nullptr};
     }
     // beyond one launch the replay window is a chain of kernels, and the results come back by copy
-    const bool one_launch = npkts <= kGroupMax || !replay;
     const Done done = stats || !one_launch ? Done{} : watch_for(b);
     if (!tail) a.done = done;
     if (timed) CK(ctx, cudaEventRecord(b->a_begin, s));
@@ -1241,6 +1263,7 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
             if (checks) CK(ctx, launch_verdict(ctx, v, Done{}, s));
         }
     }
+    CK(ctx, send_launches(b, all));
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = b->aead_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
@@ -1424,7 +1447,9 @@ int bnk_filter_note_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t
         bool sweep;
         CK(ctx, flow_note_begins(b, npkts, now_unix_ns, s, sweep));
         const Done done = watch_for(b);
+        Launches all(s, !timed && !sweep && few_in_flight(b));
         CK(ctx, launch_filter_note(b, 0, npkts, now_unix_ns, sweep ? Done{} : done, s));
+        CK(ctx, send_launches(b, all));
         if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, done, s));
         reported = true;
     }
@@ -1452,7 +1477,9 @@ int bnk_filter_check_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_
     const Done done = to_host && npkts && !(flags & BNK_F_STATS) ? watch_for(b) : Done{};
     uint8_t *const host_status = to_host ? b->host.status : nullptr;
     if (direct) b->dev.status = alias.saved.status; // the kernel writes to both
+    Launches all(s, !timed && few_in_flight(b));
     CK(ctx, launch_filter_check(b, npkts, now_unix_ns, false, host_status, done, s));
+    CK(ctx, send_launches(b, all));
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));
@@ -1478,7 +1505,9 @@ int bnk_classify_submit(bnk_batch *b, uint32_t npkts, uint32_t flags) {
     HostAlias alias(b, direct, npkts);
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     const Done done = direct && !(flags & BNK_F_STATS) ? watch_for(b) : Done{};
+    Launches all(s, !timed && few_in_flight(b));
     CK(ctx, launch_classify(b, npkts, done, s));
+    CK(ctx, send_launches(b, all));
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
     b->kernel_timed = timed;
     CK(ctx, tally_if_asked(b, npkts, flags, s));

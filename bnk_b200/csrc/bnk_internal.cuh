@@ -15,6 +15,7 @@
 
 #include "../../include/bnk_gpu.h"
 #include "flow_bounds.h"
+#include "launch.h"
 #include "pieces.h"
 #include "submit_order.h"
 
@@ -108,6 +109,7 @@ struct bnk_ctx {
     uint64_t host_direct_bytes; // batches up to this ring extent run on the caller's pinned buffers (BNK_HOST_DIRECT_BYTES)
     std::atomic<int> in_flight{0};           // batches submitted and not waited for
     std::atomic<uint64_t> direct_in_flight{0}; // ring bytes of those that run on the pinned buffers
+    bool launch_graphs; // BNK_LAUNCH_GRAPHS
     int aead_mode; // 0 = choose by batch size, 1 = always thread per packet, 2 = always warp per packet (BNK_AEAD_KERNEL)
     uint32_t aead_side_stream_from; // batches of at least this many packets run seal/open on the low-priority stream (BNK_AEAD_SIDE_STREAM_FROM; 0 = never)
     uint64_t pieces_from;           // ring extent from which a batch that is alone goes over the link in pieces (BNK_PIECES_FROM)
@@ -199,6 +201,7 @@ struct bnk_batch {
     uint32_t *h_done, *d_ticket;
     uint32_t done_seq, done_polls;
     bool done_watched;
+    LaunchGraph *graph;  // what the submit in flight was launched through
     bool kernel_timed;
     bool aead_timed;
     bnk_gso_super *h_gso; // pinned staging for the super-packet descriptors
@@ -242,28 +245,14 @@ inline uint32_t dependent_launch_up_to() {
     }();
     return v;
 }
-template <typename... KArgs, typename... Args>
-cudaError_t launch_after_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+template <typename... KArgs>
+cudaError_t launch_after_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, const typename AsIs<KArgs>::type &...args) {
+    return launch_shape(LaunchShape{nullptr, grid, block, 0, 1, true}, kernel, s, args...);
 }
 // the same launch with the ordinary full dependency when `dependent` is false
-template <typename... KArgs, typename... Args>
-cudaError_t launch_kernel(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
-    if (dependent) return launch_after_kernel(kernel, grid, block, s, args...);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.stream = s;
-    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+template <typename... KArgs>
+cudaError_t launch_kernel(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, const typename AsIs<KArgs>::type &...args) {
+    return launch_shape(LaunchShape{nullptr, grid, block, 0, 1, dependent}, kernel, s, args...);
 }
 
 constexpr uint32_t kSlotNoKeypair = 0xfffffffeu; // demux found no keypair for the receiver index

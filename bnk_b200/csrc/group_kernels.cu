@@ -1158,20 +1158,7 @@ uint32_t group_sort(const SortKeySrc &src, uint32_t n, uint32_t max_chunks, cons
 constexpr size_t group_smem(uint32_t items) { return (size_t)kGroupThreads * items * 16 + kGroupWarps * kMaxBins * 2; }
 template <int ITEMS>
 cudaError_t launch_group_items(const GroupArgs &a, uint32_t ctas, cudaStream_t s) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(kGroupThreads);
-    cfg.dynamicSmemBytes = group_smem(ITEMS);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = ctas;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, group_kernel<ITEMS>, a);
+    return launch_shape(LaunchShape{nullptr, dim3(ctas), dim3(kGroupThreads), (uint32_t)group_smem(ITEMS), ctas, true}, group_kernel<ITEMS>, s, a);
 }
 // One CTA up to 1024 packets (its barriers are cheaper than a cluster's: 600 opened in 37 us against 41), then as many as
 // give every packet a thread, up to the 16 a cluster can have here (eight CTAs of two packets a thread and more: 2048

@@ -1,0 +1,248 @@
+// Launches and their graphs (launch.h).
+#include "launch.h"
+
+#include <string.h>
+
+#include <mutex>
+#include <new>
+#include <vector>
+
+namespace {
+
+thread_local Launches *t_gathering = nullptr;
+
+cudaError_t launch_now(const LaunchShape &k, void *const *args, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = k.grid;
+    cfg.blockDim = k.block;
+    cfg.dynamicSmemBytes = k.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
+    if (k.behind) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (k.cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = k.cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        cfg.numAttrs++;
+    }
+    return cudaLaunchKernelExC(&cfg, k.fn, const_cast<void **>(args));
+}
+
+} // namespace
+
+// What a graph cannot change: its kernels, their clusters, whether the second is a dependent launch.
+struct LaunchGraph {
+    uint32_t n;
+    const void *fn[2];
+    uint32_t cluster[2];
+    bool behind;
+    bool taken;
+    int device;
+    cudaGraphExec_t exec;
+    cudaGraph_t graph;
+    cudaGraphNode_t node[2];
+    bool is(const LaunchGraph &o) const {
+        return n == o.n && fn[0] == o.fn[0] && fn[1] == o.fn[1] && cluster[0] == o.cluster[0] && cluster[1] == o.cluster[1] && behind == o.behind;
+    }
+};
+
+namespace {
+
+// The graphs of one device, used by all its contexts.  A graph belongs to one submit at a time, from its launch until that
+// has been waited for.  One is made (50 us, 250 for two kernels, 100 KB) when its kernels are asked for the fourth time and
+// none is free, so that a program that calls once or twice does not pay for it.
+class GraphPool {
+  public:
+    LaunchGraph *take(const LaunchGraph &want) {
+        std::lock_guard<std::mutex> g(mu_);
+        for (LaunchGraph *e : made_)
+            if (!e->taken && e->is(want)) {
+                e->taken = true;
+                return e;
+            }
+        if (made_.size() + making_ >= kMost) return nullptr;
+        for (Asked &a : asked_)
+            if (a.what.is(want)) {
+                if (++a.times < kFrom) return nullptr;
+                making_++;
+                return &make_;
+            }
+        if (asked_.size() < 4 * kMost) asked_.push_back({want, 1});
+        return nullptr;
+    }
+    static bool to_be_made(const LaunchGraph *g) { return g == &make_; }
+    void made(LaunchGraph *g) { // null: it could not be
+        std::lock_guard<std::mutex> l(mu_);
+        making_--;
+        if (g) made_.push_back(g);
+    }
+    void failed(const LaunchGraph &want) { // not again
+        std::lock_guard<std::mutex> l(mu_);
+        for (Asked &a : asked_)
+            if (a.what.is(want)) a.times = INT32_MIN;
+    }
+    void give(LaunchGraph *g) {
+        std::lock_guard<std::mutex> l(mu_);
+        g->taken = false;
+    }
+    void context(bool comes) {
+        std::lock_guard<std::mutex> l(mu_);
+        contexts_ += comes ? 1 : -1;
+        if (contexts_ > 0) return;
+        for (LaunchGraph *e : made_) {
+            cudaGraphExecDestroy(e->exec);
+            cudaGraphDestroy(e->graph);
+            delete e;
+        }
+        made_.clear();
+        asked_.clear();
+    }
+
+  private:
+    static constexpr size_t kMost = 48;
+    static constexpr int32_t kFrom = 4;
+    struct Asked {
+        LaunchGraph what;
+        int32_t times;
+    };
+    static LaunchGraph make_; // "there is room for one more"
+    std::mutex mu_;
+    std::vector<LaunchGraph *> made_;
+    std::vector<Asked> asked_;
+    size_t making_ = 0;
+    int contexts_ = 0;
+};
+LaunchGraph GraphPool::make_{};
+constexpr int kDevices = 64;
+GraphPool *pools() {
+    static GraphPool *const all = new GraphPool[kDevices]; // (never destroyed: the driver may be gone before)
+    return all;
+}
+
+} // namespace
+
+void launch_graphs_context(int device, bool comes) {
+    if (device >= 0 && device < kDevices) pools()[device].context(comes);
+}
+void launch_graph_give(LaunchGraph *g) {
+    if (g) pools()[g->device].give(g);
+}
+
+Launches::Launches(cudaStream_t s, bool gather) : s_(s), gathering_(gather), outer_(t_gathering) { t_gathering = this; }
+Launches::~Launches() { t_gathering = outer_; }
+
+bool Launches::add(const LaunchShape &shape, void *const *args, const uint32_t *sizes, uint32_t n) {
+    if (!gathering_ || n_ == kMost || n > kArgs) return false;
+    One &o = one_[n_];
+    uint32_t at = 0;
+    for (uint32_t i = 0; i < n; i++) {
+        if (at + sizes[i] > kStore) return false;
+        o.args[i] = o.store + at;
+        memcpy(o.store + at, args[i], sizes[i]);
+        at = (at + sizes[i] + 15u) & ~15u;
+    }
+    o.shape = shape;
+    n_++;
+    return true;
+}
+
+cudaError_t launch_any(const LaunchShape &shape, void *const *args, const uint32_t *sizes, uint32_t n, cudaStream_t s) {
+    Launches *const l = t_gathering;
+    if (l && l->s_ == s) {
+        if (l->add(shape, args, sizes, n)) return cudaSuccess;
+        const cudaError_t e = l->stop(); // in order
+        if (e != cudaSuccess) return e;
+    }
+    return launch_now(shape, args, s);
+}
+
+// A graph of the n gathered launches' kernels, made if need be.
+LaunchGraph *Launches::graph(uint32_t n) {
+    int device = 0;
+    if (n == 0 || cudaGetDevice(&device) != cudaSuccess || device >= kDevices) return nullptr;
+    GraphPool &pool = pools()[device];
+    LaunchGraph want{};
+    want.n = n;
+    for (uint32_t i = 0; i < n; i++) {
+        want.fn[i] = one_[i].shape.fn;
+        want.cluster[i] = one_[i].shape.cluster;
+    }
+    want.behind = n == 2 && one_[1].shape.behind; // (of the first: nothing is in front, or it is waited for)
+    want.device = device;
+    LaunchGraph *g = pool.take(want);
+    if (!GraphPool::to_be_made(g)) return g;
+    g = new (std::nothrow) LaunchGraph(want);
+    cudaStream_t s = nullptr;
+    int low = 0, high = 0; // the priority that batches' streams have
+    cudaError_t e = g ? cudaDeviceGetStreamPriorityRange(&low, &high) : cudaErrorMemoryAllocation;
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, high);
+    if (e == cudaSuccess) e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+        for (uint32_t i = 0; i < n && e == cudaSuccess; i++) {
+            LaunchShape k = one_[i].shape;
+            k.behind = k.behind && i > 0;
+            e = launch_now(k, one_[i].args, s);
+        }
+        const cudaError_t end = cudaStreamEndCapture(s, &g->graph);
+        if (e == cudaSuccess) e = end;
+    }
+    size_t roots = 1, nodes = 2;
+    cudaGraphNode_t node[2] = {};
+    if (e == cudaSuccess) e = cudaGraphGetRootNodes(g->graph, &g->node[0], &roots);
+    if (e == cudaSuccess) e = cudaGraphGetNodes(g->graph, node, &nodes);
+    if (e == cudaSuccess && (roots != 1 || nodes != n)) e = cudaErrorUnknown;
+    if (e == cudaSuccess) {
+        g->node[1] = node[0] == g->node[0] ? node[1] : node[0];
+        e = cudaGraphInstantiate(&g->exec, g->graph, 0);
+    }
+    if (s) cudaStreamDestroy(s);
+    if (e != cudaSuccess) {
+        if (g && g->graph) cudaGraphDestroy(g->graph);
+        delete g;
+        g = nullptr;
+        (void)cudaGetLastError();
+        pool.failed(want);
+    } else {
+        g->taken = true;
+    }
+    pool.made(g);
+    return g;
+}
+
+cudaError_t Launches::send(LaunchGraph *&taken) {
+    LaunchGraph *const g = graph(n_);
+    if (!g) return stop();
+    cudaError_t e = cudaSuccess;
+    for (uint32_t i = 0; i < n_ && e == cudaSuccess; i++) {
+        cudaKernelNodeParams p = {};
+        p.func = const_cast<void *>(one_[i].shape.fn);
+        p.gridDim = one_[i].shape.grid;
+        p.blockDim = one_[i].shape.block;
+        p.sharedMemBytes = one_[i].shape.smem;
+        p.kernelParams = one_[i].args;
+        e = cudaGraphExecKernelNodeSetParams(g->exec, g->node[i], &p);
+    }
+    if (e == cudaSuccess) e = cudaGraphLaunch(g->exec, s_);
+    if (e != cudaSuccess) {
+        launch_graph_give(g);
+        (void)cudaGetLastError();
+        return stop();
+    }
+    taken = g;
+    n_ = 0;
+    gathering_ = false;
+    return cudaSuccess;
+}
+
+cudaError_t Launches::stop() {
+    const uint32_t n = n_;
+    n_ = 0;
+    gathering_ = false;
+    cudaError_t e = cudaSuccess;
+    for (uint32_t i = 0; i < n && e == cudaSuccess; i++) e = launch_now(one_[i].shape, one_[i].args, s_);
+    return e;
+}

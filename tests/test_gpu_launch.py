@@ -1,0 +1,148 @@
+"""Submits whose kernels are launched together through an executable graph (from the fourth of a kind on) do what they do
+launch by launch: the same bytes, counters, verdicts and flows, in whatever order kinds and sizes come."""
+import os
+
+import numpy as np
+import pytest
+
+from tests import helpers as H
+from tests import reference_cases as RC
+
+pytestmark = pytest.mark.gpu
+
+
+def _context(graphs, **kw):
+    from bnk_b200 import Context
+
+    old = os.environ.get("BNK_LAUNCH_GRAPHS")
+    os.environ["BNK_LAUNCH_GRAPHS"] = str(graphs)
+    try:
+        return Context(**kw)
+    finally:
+        if old is None:
+            del os.environ["BNK_LAUNCH_GRAPHS"]
+        else:
+            os.environ["BNK_LAUNCH_GRAPHS"] = old
+
+
+def _passes(c, sizes, seed):
+    """Rounds of note, seal (with flows), open (index, replay, inner header, rules), check and classify on one context."""
+    from bnk_b200.device import F_ASSIGN_COUNTERS, F_CHECK_INBOUND, F_DEMUX_INDEX, F_INNER_CHECK, F_NOTE_OUTBOUND, F_REPLAY
+    from bnk_b200.filter import CompiledRule, PortRange, flatten_rules
+
+    rng = np.random.default_rng(seed)
+    peers = 7
+    keys = rng.integers(0, 256, (peers, 32), dtype=np.uint8)
+    c.set_keypairs(0, keys, keys, np.arange(peers, dtype=np.uint32) + 100)
+    addr = [RC.ip("100.64.7.0") + p for p in range(peers)]
+    for p in range(peers):
+        c.index_set(100 + p, p)
+        c.set_allowed_ip(p, addr[p])
+        c.addr_set(bytes(10) + b"\xff\xff" + bytes([10, 0, 0, p]), 4000, p)
+    c.acl_set(True, flatten_rules([CompiledRule(srcs=["100.64.7.0/30"], proto="udp", ports=[PortRange(1, 30000)])]))
+    most = max(sizes)
+    batches = [c.batch(most, most * 400) for _ in range(2)]
+    got = []
+    for r, n in enumerate(sizes):
+        b, o = batches[r % 2], batches[1 - r % 2]
+        now = RC.T0 + r * RC.SEC
+        off = (np.arange(n, dtype=np.uint64) * 400).astype(np.uint32)
+        slot = rng.integers(0, peers, n)
+        lens = rng.integers(28, 340, n)
+        b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
+        for i in range(n):
+            p = RC.udp(addr[slot[i]], RC.SELF, int(rng.integers(1, 9)), int(rng.integers(1, 60000)))[:28]
+            p = p[:2] + int(lens[i]).to_bytes(2, "big") + p[4:]
+            b.ring[int(off[i]) + 16:int(off[i]) + 44] = np.frombuffer(p, np.uint8)
+        b.off[:n], b.len[:n], b.slot[:n] = off, lens, slot
+        b.filter_note(n, now)
+        b.seal(n, F_ASSIGN_COUNTERS | (F_NOTE_OUTBOUND if r % 3 else 0), now)
+        got += [np.array(b.ring[:n * 400]), np.array(b.counter[:n]), np.array(b.out_len[:n]), np.array(b.status[:n])]
+        o.ring[:n * 400] = b.ring[:n * 400]
+        o.off[:n], o.len[:n] = off, b.out_len[:n]
+        if n > 3:
+            o.ring[int(off[n // 2]) + 20] ^= 1
+        if r % 4 == 3 and n > 1:  # a message twice
+            o.ring[:400] = o.ring[400:800]
+            o.len[0] = o.len[1]
+        o.open(n, F_DEMUX_INDEX | F_REPLAY | ((F_INNER_CHECK | F_CHECK_INBOUND) if r % 2 else 0), now)
+        got += [np.array(o.ring[:n * 400]), np.array(o.counter[:n]), np.array(o.out_len[:n]), np.array(o.status[:n]), np.array(o.slot[:n])]
+        b.len[:n] = lens
+        b.src_addr[:n] = 0
+        b.src_addr[:n, 10:12], b.src_addr[:n, 12], b.src_addr[:n, 15], b.src_addr[:n, 16], b.src_addr[:n, 17] = 255, 10, slot, 15, 160
+        b.ring[off.astype(np.int64)] = 4
+        b.slot[:n] = 99
+        b.classify(n)
+        got += [np.array(b.status[:n]), np.array(b.slot[:n])]
+        o.len[:n] = lens
+        o.filter_check(n, now)
+        got.append(np.array(o.status[:n]))
+    got.append(c.flows_export())
+    for b in batches:
+        b.close()
+    return got
+
+
+@pytest.mark.parametrize("sizes", [[1] * 10, [16, 17] * 6, [64, 65, 64] * 4, [160, 161] * 5, [256, 257] * 5, [700, 1025] * 5,
+                                   [3, 300, 3, 3, 2000, 3, 300, 300, 3, 300, 2000, 2000, 2000, 3]], ids=str)
+def test_same_results_launch_by_launch_and_through_graphs(gpu_lib, sizes):
+    results = []
+    for graphs in (0, 1, 1):  # the third context finds the second one's graphs gone
+        with _context(graphs, max_keypairs=8, mtu=1420, flow_capacity=1 << 14) as c:
+            results.append(_passes(c, sizes, len(sizes)))
+    for other in results[1:]:
+        for x, y in zip(results[0], other):
+            assert np.array_equal(x, y)
+
+
+def test_batches_in_flight_and_contexts_beside_each_other(gpu_lib, oracle):
+    """Graphs are shared by the contexts of a device: two contexts with up to four submits each in flight, one context closed
+    on the way, every message the checker's."""
+    from bnk_b200.device import F_ASSIGN_COUNTERS
+
+    rng = np.random.default_rng(4)
+    keys = rng.integers(0, 256, (1, 32), dtype=np.uint8)
+    n = 40
+    off = H.layout_fixed(n, 256)
+    lens = rng.integers(0, 200, n).astype(np.uint32)
+    made = [_context(1, max_keypairs=1, flow_capacity=0) for _ in range(2)]
+    counter = [0, 0]
+    batches = []
+    for c in made:
+        c.set_keypairs(0, keys, keys, np.array([5], np.uint32))
+        batches.append([c.batch(n, n * 256) for _ in range(4)])
+    for r in range(24):
+        at_once = 1 + r % 4
+        if r == 16:
+            for b in batches.pop():
+                b.close()
+            made.pop().close()
+        want = []
+        for k in range(len(made)):
+            for b in batches[k][:at_once]:
+                b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
+                b.off[:], b.len[:], b.slot[:] = off, lens, 0
+                ctr = np.arange(counter[k], counter[k] + n, dtype=np.uint64)
+                counter[k] += n
+                want.append((b, H.oracle_seal(oracle, keys, np.array([5]), 1420, b.ring, off, lens, np.zeros(n), ctr)))
+        for k in range(len(made)):
+            for b in batches[k][:at_once]:
+                b.seal(n, F_ASSIGN_COUNTERS, wait=False)
+                b.wait()  # (nonces are handed out in this order)
+        for b, (ring, st, ln) in want:
+            assert np.array_equal(b.status, st) and np.array_equal(b.out_len, ln)
+            assert H.spans_equal(np.array(b.ring), ring, off, ln) == []
+    # and without a wait in between, which takes the nonces in submit order as well: all on one context, stream by stream
+    for r in range(8):
+        for b in batches[0]:
+            b.off[:], b.len[:], b.slot[:], b.counter[:] = off, lens, 0, np.arange(n) + 1000 * r
+        plain = [np.array(b.ring) for b in batches[0]]
+        for b in batches[0]:
+            b.seal(n, wait=False)
+        for b, p in zip(batches[0], plain):
+            b.wait()
+            ring, st, ln = H.oracle_seal(oracle, keys, np.array([5]), 1420, p, off, lens, np.zeros(n), np.arange(n) + 1000 * r)
+            assert np.array_equal(b.out_len, ln) and H.spans_equal(np.array(b.ring), ring, off, ln) == []
+    for b in batches[0]:
+        b.close()
+    made[0].close()
