@@ -447,4 +447,10 @@ __device__ __forceinline__ uint32_t demux_index_warp(const uint64_t *keys, const
 
 // gso_kernels.cu
 cudaError_t launch_gso_split(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, cudaStream_t s);
+// The same with the descriptors and b->h_gso still in pinned memory: prepare, then the split, with the super-packets up or from
+// the pinned ring.
+bool gso_split_fits(const bnk_gso_super *supers, uint32_t n_super, uint32_t n_pkts, uint64_t ring_bytes);
+cudaError_t launch_gso_prepare(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, cudaStream_t s);
+cudaError_t launch_gso_split_up(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, const Done &done, cudaStream_t s);
+cudaError_t launch_gso_split_in_place(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, const Done &done, cudaStream_t s);
 cudaError_t launch_packets_to_host(bnk_batch *b, uint32_t n, cudaStream_t s);

@@ -1,0 +1,34 @@
+// Bulk copies between shared and global memory (a ring's on the device or the host's), by one thread; addresses and sizes are
+// multiples of 16.  What comes in counts its bytes on an mbarrier of shared memory.  Over the link the copy engine of the SM
+// asks for whole lines wherever the bytes start: 16,384 x 1440 B read 1456 bytes apart 488 us, in 16-byte pieces by the
+// lanes of a warp 875 (1536 bytes apart 498 either way).
+#pragma once
+
+#include <stdint.h>
+
+__device__ __forceinline__ uint32_t shared_at(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(uint64_t *bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_at(bar)) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint64_t *bar, uint32_t bytes) { // the phase ends when that many have come
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_at(bar)), "r"(bytes) : "memory");
+}
+// False: it has not come after so many turns (80 ms at the least), which no link that works takes.
+__device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
+    for (uint32_t turn = 0; turn < (1u << 22); turn++) {
+        uint32_t over;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(over)
+                     : "r"(shared_at(bar)), "r"(parity)
+                     : "memory");
+        if (over) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void bulk_in(void *smem, const void *gmem, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(shared_at(smem)),
+                 "l"(__cvta_generic_to_global(gmem)), "r"(bytes), "r"(shared_at(bar))
+                 : "memory");
+}
+// Between this thread's own accesses to shared memory and the bulk copies that follow.
+__device__ __forceinline__ void bulk_fence_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }

@@ -10,6 +10,7 @@
 //   - transport checksum recomputed over pseudo header + transport header + payload.
 // The work is a copy with a running one's-complement sum: HBM-bound, ~2 x segment bytes of traffic.
 #include "bnk_internal.cuh"
+#include "bulk.cuh"
 
 namespace {
 
@@ -23,16 +24,42 @@ __device__ __forceinline__ uint32_t fold16(uint64_t s) {
     return t;
 }
 
-__global__ void __launch_bounds__(256) gso_split_kernel(const bnk_gso_super *supers, uint32_t n_super, uint8_t *ring,
-                                                        const uint32_t *off, const uint32_t *len, uint32_t *slot,
-                                                        uint32_t n_pkts, uint64_t ring_bytes, const uint32_t *seg_super) {
-    let_next_kernel_start();
-    wait_for_kernel_in_front();
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= n_pkts) return;
-    const uint32_t pkt = warp;
-    const uint32_t j = seg_super[pkt];
-    if (j >= n_super) return; // not a segment of any super-packet: left alone
+struct SplitArgs {
+    const bnk_gso_super *supers;
+    uint32_t n_super;
+    uint8_t *ring;
+    const uint32_t *off, *len;
+    uint32_t *slot;
+    uint32_t n_pkts;
+    uint64_t ring_bytes;
+    const uint32_t *seg_super;
+    const uint8_t *host_ring; // FROM_HOST
+    Done done;
+};
+constexpr uint32_t kSplitWarps = 8;
+constexpr uint32_t kSplitWindow = 2048; // FROM_HOST: a segment's payload, from the 16 bytes it starts in to those it ends in
+
+// One segment, or packet that is none, by a warp.  FROM_HOST: the payload comes from the caller's pinned ring, in one bulk copy,
+// and goes to the super-packet's place in the device ring besides (each word by the segment its first byte belongs to), which an
+// upload would have filled; the headers are there already (gso_prepare_kernel).
+template <bool FROM_HOST>
+__device__ __forceinline__ void split_packet(const SplitArgs &a, uint32_t pkt, uint4 *stage, uint64_t *bar) {
+    const bnk_gso_super *const supers = a.supers;
+    const uint32_t n_super = a.n_super;
+    uint8_t *const ring = a.ring;
+    const uint32_t *const off = a.off, *const len = a.len;
+    uint32_t *const slot = a.slot;
+    const uint64_t ring_bytes = a.ring_bytes;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t j = a.seg_super[pkt];
+    if (j >= n_super) { // not a segment of any super-packet: left alone
+        if (!FROM_HOST) return;
+        const uint32_t o = off[pkt], bytes = len[pkt];
+        if ((o & 15u) || (uint64_t)o + 16 + bytes > ring_bytes) return;
+        for (uint32_t q = 16u * lane; q < 16u + bytes; q += 512u)
+            *reinterpret_cast<uint4 *>(ring + o + q) = *reinterpret_cast<const uint4 *>(a.host_ring + o + q);
+        return;
+    }
     const bnk_gso_super sp = supers[j];
     const uint32_t k = pkt - sp.first_pkt;
     const uint32_t hdr = sp.hdr_len, iph = sp.csum_start;
@@ -43,6 +70,26 @@ __global__ void __launch_bounds__(256) gso_split_kernel(const bnk_gso_super *sup
               (sp.csum_offset & 1u) == 0 && hdr <= 128u; // one header word per lane
     uint32_t seg_len = 0, total = 0;
     const uint32_t o = off[pkt];
+    const uint64_t at = (uint64_t)sp.src_off + data_at; // of the payload, in the ring
+    const uint8_t *payload = ring + at;
+    if (FROM_HOST) { // (of such super-packets the host knows that they are whole and each segment fits the window)
+        const uint64_t from = at & ~15ull, end = at + min((uint32_t)sp.gso_size, sp.src_len - data_at);
+        const uint32_t bytes = (uint32_t)(((end + 15u) & ~15ull) - from);
+        if (lane == 0) {
+            bar_expect(bar, bytes);
+            bulk_in(stage, a.host_ring + from, bytes, bar);
+        }
+        if (!__all_sync(0xffffffffu, bar_wait(bar, 0))) ok = false; // (nothing else is read into the stage)
+        __syncwarp();
+        payload = reinterpret_cast<const uint8_t *>(stage) + (at - from);
+        const uint64_t word0 = (at + 3u) & ~3ull, whole = (uint64_t)sp.src_off + sp.src_len;
+        for (uint64_t w = word0 + 4u * lane; w < end; w += 128u) {
+            const uint8_t *const v = reinterpret_cast<const uint8_t *>(stage) + (w - from);
+            if (w + 4u <= whole) *reinterpret_cast<uint32_t *>(ring + w) = *reinterpret_cast<const uint32_t *>(v);
+            else
+                for (uint64_t b = w; b < whole; b++) ring[b] = v[b - w];
+        }
+    }
     if (ok) {
         seg_len = min((uint32_t)sp.gso_size, sp.src_len - data_at);
         total = hdr + seg_len;
@@ -96,7 +143,7 @@ __global__ void __launch_bounds__(256) gso_split_kernel(const bnk_gso_super *sup
     // payload copy + sum.  The destination starts on a word (headers are whole words); the source starts where the
     // segments before it end, at any byte of a word, so a word of the payload is cut out of two aligned words of the
     // source.
-    const uint8_t *src = in + data_at;
+    const uint8_t *src = payload;
     uint8_t *dst = out + hdr;
     uint64_t sum = 0;    // of big-endian 16-bit words
     uint64_t le_sum = 0; // of the payload words as loaded (little-endian): the one's-complement sum commutes with the
@@ -152,6 +199,65 @@ __global__ void __launch_bounds__(256) gso_split_kernel(const bnk_gso_super *sup
     }
 }
 
+template <bool FROM_HOST>
+__global__ void __launch_bounds__(32 * kSplitWarps) gso_split_kernel(const __grid_constant__ SplitArgs a) {
+    let_next_kernel_start();
+    __shared__ __align__(128) uint4 stage[FROM_HOST ? kSplitWarps : 1][kSplitWindow / 16];
+    __shared__ __align__(8) uint64_t bar[kSplitWarps];
+    const uint32_t warp = threadIdx.x >> 5, pkt = blockIdx.x * kSplitWarps + warp;
+    if (FROM_HOST) {
+        if ((threadIdx.x & 31u) == 0) bar_init(&bar[warp]);
+        bulk_fence_shared();
+        __syncwarp();
+    }
+    wait_for_kernel_in_front();
+    if (pkt < a.n_pkts) split_packet<FROM_HOST>(a, pkt, stage[FROM_HOST ? warp : 0], &bar[warp]);
+    signal_done(a.done, false, [] {});
+}
+
+// In front of a split that reads the caller's pinned ring: what an upload would have brought of the descriptors, the super-packets'
+// descriptors and headers, and the map from segment to super-packet.  (The super-packets come in batch order.)  A thread per
+// packet, then a warp per super-packet.
+struct PrepareArgs {
+    const uint32_t *host_off, *host_len, *host_slot;
+    uint32_t *off, *len, *slot, n_pkts;
+    const bnk_gso_super *host_supers;
+    bnk_gso_super *supers;
+    uint32_t n_super;
+    const uint8_t *host_ring;
+    uint8_t *ring;
+    uint32_t *seg_super;
+};
+__global__ void __launch_bounds__(256) gso_prepare_kernel(const __grid_constant__ PrepareArgs a) {
+    let_next_kernel_start();
+    wait_for_kernel_in_front();
+    const uint32_t packet_ctas = (a.n_pkts + 255u) / 256u, lane = threadIdx.x & 31;
+    if (blockIdx.x < packet_ctas) {
+        const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+        if (i >= a.n_pkts) return;
+        const uint32_t o = a.host_off[i], l = a.host_len[i], s = a.host_slot[i];
+        a.off[i] = o;
+        a.len[i] = l;
+        a.slot[i] = s;
+        return;
+    }
+    const uint32_t j = (blockIdx.x - packet_ctas) * 8u + (threadIdx.x >> 5);
+    if (j >= a.n_super) return;
+    constexpr uint32_t kWords = sizeof(bnk_gso_super) / 4;
+    static_assert(sizeof(bnk_gso_super) == 4 * kWords && kWords <= 16, "two descriptors in the lanes of a warp");
+    uint32_t w = 0; // lanes 0..: this one's words, lanes 16..: those of the one in front
+    if (lane < kWords) w = reinterpret_cast<const uint32_t *>(a.host_supers + j)[lane];
+    else if (j > 0 && lane >= 16u && lane < 16u + kWords) w = reinterpret_cast<const uint32_t *>(a.host_supers + j - 1)[lane - 16u];
+    if (lane < kWords) reinterpret_cast<uint32_t *>(a.supers + j)[lane] = w;
+    const uint32_t src = __shfl_sync(0xffffffffu, w, 0), first = __shfl_sync(0xffffffffu, w, 2), n = __shfl_sync(0xffffffffu, w, 3);
+    const uint32_t hdr = __shfl_sync(0xffffffffu, w, 4) & 0xffffu; // words of the header, 32 at most
+    const uint32_t before = __shfl_sync(0xffffffffu, w, 18) + __shfl_sync(0xffffffffu, w, 19); // where the one in front ends
+    if (4u * lane < hdr) reinterpret_cast<uint32_t *>(a.ring + src)[lane] = reinterpret_cast<const uint32_t *>(a.host_ring + src)[lane];
+    for (uint32_t k = before + lane; k < first + n; k += 32) a.seg_super[k] = k < first ? a.n_super : j;
+    if (j + 1 == a.n_super)
+        for (uint32_t k = first + n + lane; k < a.n_pkts; k += 32) a.seg_super[k] = a.n_super;
+}
+
 // segment -> super-packet index (n_super for packets that belong to none)
 __global__ void gso_map_kernel(const bnk_gso_super *supers, uint32_t n_super, uint32_t n_pkts, uint32_t *seg_super) {
     let_next_kernel_start();
@@ -201,9 +307,46 @@ cudaError_t launch_gso_split(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, cu
         seg_super, n_pkts, n_super);
     launch_kernel(n_pkts <= dependent_launch_up_to(), gso_map_kernel, dim3((n_super + 127) / 128), dim3(128), s, d.gso,
         n_super, n_pkts, seg_super);
-    launch_kernel(n_pkts <= dependent_launch_up_to(), gso_split_kernel, dim3((n_pkts + 7) / 8), dim3(256), s, d.gso,
-        n_super, d.ring, d.off, d.len, d.slot, n_pkts, b->ring_bytes, seg_super);
-    b->ctx->launches += 3;
+    b->ctx->launches += 2;
+    return launch_gso_split_up(b, n_super, n_pkts, Done{}, s);
+}
+
+cudaError_t launch_gso_split_up(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, const Done &done, cudaStream_t s) {
+    DeviceBatch &d = b->dev;
+    const SplitArgs a{d.gso, n_super, d.ring, d.off, d.len, d.slot, n_pkts, b->ring_bytes, d.order_tmp, nullptr, done};
+    launch_kernel(n_pkts <= dependent_launch_up_to(), gso_split_kernel<false>, dim3((n_pkts + kSplitWarps - 1) / kSplitWarps),
+        dim3(32 * kSplitWarps), s, a);
+    b->ctx->launches += 1;
+    return cudaGetLastError();
+}
+
+// Whether gso_split_kernel<true> can take them: in batch order, whole, and every segment in one window.
+bool gso_split_fits(const bnk_gso_super *supers, uint32_t n_super, uint32_t n_pkts, uint64_t ring_bytes) {
+    uint64_t next = 0;
+    for (uint32_t j = 0; j < n_super; j++) {
+        const bnk_gso_super &p = supers[j];
+        const uint64_t segs = p.n_pkts, payload = (uint64_t)p.src_len - p.hdr_len;
+        if (p.first_pkt < next || p.first_pkt + segs > n_pkts || segs == 0 || (p.src_off & 3u) || (uint64_t)p.src_off + p.src_len > ring_bytes ||
+            (p.hdr_len & 3u) || p.hdr_len > 128u || p.hdr_len >= p.src_len || p.gso_size == 0 || p.gso_size + 32u > kSplitWindow ||
+            segs != (payload + p.gso_size - 1) / p.gso_size)
+            return false;
+        next = p.first_pkt + segs;
+    }
+    return n_super != 0;
+}
+cudaError_t launch_gso_prepare(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, cudaStream_t s) {
+    DeviceBatch &d = b->dev;
+    const bnk_batch_view &h = b->host;
+    const PrepareArgs p{h.off, h.len, h.slot, d.off, d.len, d.slot, n_pkts, b->h_gso, d.gso, n_super, h.ring, d.ring, d.order_tmp};
+    launch_kernel(false, gso_prepare_kernel, dim3((n_pkts + 255) / 256 + (n_super + 7) / 8), dim3(256), s, p);
+    b->ctx->launches += 1;
+    return cudaGetLastError();
+}
+cudaError_t launch_gso_split_in_place(bnk_batch *b, uint32_t n_super, uint32_t n_pkts, const Done &done, cudaStream_t s) {
+    DeviceBatch &d = b->dev;
+    const SplitArgs a{d.gso, n_super, d.ring, d.off, d.len, d.slot, n_pkts, b->ring_bytes, d.order_tmp, b->host.ring, done};
+    launch_kernel(true, gso_split_kernel<true>, dim3((n_pkts + kSplitWarps - 1) / kSplitWarps), dim3(32 * kSplitWarps), s, a);
+    b->ctx->launches += 1;
     return cudaGetLastError();
 }
 

@@ -359,3 +359,71 @@ def test_plain_packets_beside_segments(gpu_lib, oracle, order, copied, monkeypat
             assert b.message(i) == oracle.wg_seal(key[0].tobytes(), 9, i, packets[i], 1420), i
             f.note_outbound(packets[i], now)
         assert H.flows_equal(c.flows_export(), f.flows())
+
+
+@pytest.mark.parametrize("layout", ["one", "window", "beyond the window", "plain between", "beside their segments", "any order", "many", "copied"])
+def test_split_where_the_super_packets_lie_in_the_host_ring(gpu_lib, oracle, layout):
+    """Super-packets read in place, copied up in front of the split or copied with the ring: the segments and plain packets
+    on the device are the checker's, and so are those of a second split on the device alone, when the host ring holds
+    something else."""
+    from bnk_b200 import Context
+    from bnk_b200.device import F_NO_H2D
+
+    rng = np.random.default_rng(len(layout))
+    plans = {"one": [(1, 1)], "window": [(2016 * 3 + 1, 2016), (2015 * 2, 2015), (17, 16)], "beyond the window": [(2017 * 3, 2017), (9001, 1400)],
+             "plain between": [(7000, 1380), (3, 2), (5000, 501)], "beside their segments": [(9000, 1377), (4444, 536)],
+             "any order": [(5000, 1201), (4000, 999), (30, 7)], "many": [(int(rng.integers(1, 40)) * 61, int(rng.integers(30, 1400))) for _ in range(300)],
+             "copied": [(60_000, 1380)] * 50}[layout]  # "copied": 3 MB
+    supers, meta = [], []
+    for i, (size, gso) in enumerate(plans):
+        if i % 2:
+            pkt, cs, hdr = _udp_super(rng, size)
+            meta.append((hdr, gso, cs, 6, 17))
+        else:
+            pkt, cs, hdr = _tcp_super(rng, size, ihl=5 + i % 3)
+            meta.append((hdr, gso, cs, 16, 6))
+        supers.append(pkt)
+    sup, seg_len, n, end = _plan(supers, meta, 2144)
+    want = [s for p, m in zip(supers, meta) for s in oracle.gso_split(p, *m)]
+    off = np.arange(n, dtype=np.int64) * 2144
+    if layout == "plain between":  # in front of, between and behind the super-packets' segments
+        at = [0, int(sup[1]["first_pkt"]), n, n]
+        for k in reversed(at):
+            want.insert(k, rng.integers(0, 256, int(rng.integers(0, 1500)), dtype=np.uint8).tobytes())
+            for s in sup:
+                s["first_pkt"] += int(s["first_pkt"]) >= k
+        n = len(want)
+        seg_len = np.array([len(w) for w in want], np.uint32)
+        off = np.arange(n, dtype=np.int64) * 2144
+        sup["src_off"] += 4 * 2144
+        end += 4 * 2144
+    elif layout == "beside their segments":  # the first super-packet lies between its segments and those of the second
+        k = int(sup[1]["first_pkt"])
+        sup[0]["src_off"] = k * 2144 + 4
+        off[k:] += 16384
+        sup[1]["src_off"] += 16384
+        end += 16384
+    elif layout == "any order":
+        sup = sup[[2, 0, 1]]  # listed in another order than their segments are
+        supers = [supers[k] for k in (2, 0, 1)]
+    ring = int(end) + 4096 & ~15
+    with Context(max_keypairs=2, mtu=0, flow_capacity=0) as c:
+        b = c.batch(n, ring)
+        b.ring[:] = 0xA5
+        b.off[:], b.len[:], b.slot[:] = off, seg_len, 1
+        b.upload(n)
+        for s, pkt in zip(sup, supers):
+            b.ring[int(s["src_off"]):int(s["src_off"]) + len(pkt)] = np.frombuffer(pkt, np.uint8)
+        plain = np.ones(n, bool)
+        for s in sup:
+            plain[int(s["first_pkt"]):int(s["first_pkt"]) + int(s["n_pkts"])] = False
+        for i in np.flatnonzero(plain):
+            b.ring[off[i] + 16:off[i] + 16 + seg_len[i]] = np.frombuffer(want[i], np.uint8)
+        for flags in (0, F_NO_H2D):
+            b.gso_split(sup, n, flags)
+            b.ring[:] = 0x77
+            b.download(n)
+            for i in range(n):
+                assert b.ring[off[i] + 16:off[i] + 16 + len(want[i])].tobytes() == want[i], (flags, i)
+            assert (b.slot == 1).all()
+        b.close()
