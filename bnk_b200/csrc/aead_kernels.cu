@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "bulk.cuh"
 #include "filter_device.cuh"
 
 namespace {
@@ -519,21 +520,23 @@ __device__ __forceinline__ void p26_finish(const P26 &x, const uint32_t (&pad)[4
 // batches that stay in the caller's pinned memory (AeadArgs::in / out are then host addresses and the host link is
 // the bound).
 //
-// A round covers up to 31 cipher blocks (1984 payload bytes; a full-size packet is one round).  The warp brings the
-// round's bytes into shared memory in 16-byte pieces with cp.async, in windows that start on 128-byte lines: over
-// the host link an instruction then asks for whole lines (measured on 4096 x 1440 B, read and written in place:
-// 172 us against 177 with windows at the packet's own 16-byte alignment).  Lane 0 computes cipher block 0 (the
+// A round covers up to 31 cipher blocks (1984 payload bytes; a full-size packet is one round).  One thread brings the
+// round's bytes into shared memory with one bulk copy, and sends what leaves the round, put together in shared memory, with
+// another: bytes behind the end of a message that share its last 16 are written back as they were read.  Over the link the
+// copy engine of the SM asks for whole lines wherever a packet starts.  16-byte pieces asked for by the lanes do so only
+// where the packets start on 32-byte sectors (plain copy through shared memory, 16,384 x 1440 B read and written: 1456 bytes
+// apart 1030 us in pieces, 650 in bulk; 1536 bytes apart 645 either way; 4096 x 1440 B 1472 apart 186 and 165).
+// Lane 0 computes cipher block 0 (the
 // one-time Poly1305 key), lane j the round's block j, all in the same pass; on the seal side that needs no payload and
 // is done while the payload is on its way.  For Poly1305 the round's 16-byte blocks are laid out from the right, four
 // to a lane, the length block last in lane 31, so that every lane runs the same Horner steps from zero (the lane of the
 // first block starts from the state carried in); lane j's sum is then multiplied by r^(4 (31 - j)), which again needs no
-// payload, and the lanes' limbs are added up.  What leaves the round is put together in shared memory and written in
-// the same pieces; bytes behind the end of a message that share its last piece are written back as they were read.
+// payload, and the lanes' limbs are added up.
 // A tag is checked before a one-round packet's plaintext is written.
 //
 // A warp takes tiles of a.tile consecutive packets (one in small batches); the descriptors of a tile lie in its
 // lanes, and the next packet's bytes are on their way while one is computed.  Few warps are enough to keep the host
-// link busy, and more of them in flight make it slower (read + write of 4096 x 1440 B: 172 us from 16 CTAs of 8
+// link busy, and more of them in flight make it slower (read + write of 4096 x 1440 B in pieces: 172 us from 16 CTAs of 8
 // warps, 184 from 148, 225 from 512), so the grid is capped for host-resident rings (wpp_grid).
 //
 // Loops are kept rolled: a warp of a small batch runs its code once, from a cold instruction cache.
@@ -549,11 +552,9 @@ template <>
 struct InlineDesc<0> {};
 constexpr uint32_t kRoundBlocks = 31;
 constexpr uint32_t kRoundBytes = kRoundBlocks * 64;
-constexpr uint32_t kStagePieces = 136; // <= 7 of the first line + header + 124 body + 1 of the tag, rounded to the swizzle's 8
+constexpr uint32_t kStagePieces = 128; // header, 124 of the body, 2 that the tag may touch, rounded up to a line (no swizzle: a
+                                       // bulk copy fills it, and the four-way bank conflicts of the lanes' loads are 0.1 us of 5)
 
-// Lane j reads its four pieces 4j .. 4j+3 with 16-byte loads: the plain layout would put eight lanes on two bank
-// groups; flipping the low bits of the piece number by its line number spreads them over all eight.
-__device__ __forceinline__ uint32_t stage_at(uint32_t piece) { return piece ^ ((piece >> 3) & 3u); }
 __device__ __forceinline__ void copy_async16(void *smem, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
 }
@@ -561,16 +562,14 @@ __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.com
 template <int LEFT>
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
-// The pieces of round `rnd` of a packet: where they lie and how many there are.
+// Round `rnd` of a packet: its first byte in the ring (the header's in round 0), and which 16-byte piece of the stage its
+// first body byte is.
 struct Round {
-    uint64_t window;  // ring offset of the 128-byte line the first piece lies in
-    uint32_t first;   // piece number (from the window) of the header (round 0) or of the round's first body byte
-    uint32_t body;    // piece number of the round's first body byte
+    uint64_t at;
+    uint32_t body;
     __device__ __forceinline__ Round(uint32_t off, uint32_t rnd) {
-        const uint64_t at = rnd == 0 ? (uint64_t)off : (uint64_t)off + BNK_WG_HEADER + (uint64_t)rnd * kRoundBytes;
-        window = at & ~127ull;
-        first = (uint32_t)(at & 127u) >> 4;
-        body = first + (rnd == 0 ? 1u : 0u);
+        at = rnd == 0 ? (uint64_t)off : (uint64_t)off + BNK_WG_HEADER + (uint64_t)rnd * kRoundBytes;
+        body = rnd == 0 ? 1u : 0u;
     }
 };
 
@@ -583,7 +582,7 @@ struct Round {
 // Word `lane` (0..15) of the 64 bytes that start at a piece.
 __device__ __forceinline__ uint32_t stage_word(const uint4 *stage, uint32_t piece) {
     const uint32_t lane = threadIdx.x & 31;
-    return reinterpret_cast<const uint32_t *>(&stage[stage_at(piece + ((lane >> 2) & 3u))])[lane & 3u];
+    return reinterpret_cast<const uint32_t *>(&stage[piece])[lane & 15u];
 }
 
 // r^(4 e) for the lane's e = 31 - lane, one bit of e per step: pw goes through r^4, r^8, r^16 ...
@@ -615,8 +614,15 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
     if (!a.from_host) wait_for_kernel_in_front();
     __shared__ __align__(128) uint4 stage_all[kWppWarps][2][kStagePieces];
     __shared__ __align__(16) uint4 key_all[kWppWarps][2][2];
+    __shared__ __align__(8) uint64_t bar_all[kWppWarps][2];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t T = a.tile, tiles = (a.n + T - 1) / T, step = gridDim.x * kWppWarps;
+    const uint32_t T = INLINE ? 1u : a.tile, tiles = (a.n + T - 1) / T, step = gridDim.x * kWppWarps;
+    uint32_t parity = 0;  // bit b: of the phase that stage b's next wait is for
+    uint32_t awaited = 0; // bit b: copies into stage b are on their way
+    bool broken = false;  // what was asked for has not come: nothing is read or written any more
+    if (lane < 2) bar_init(&bar_all[warp][lane]);
+    bulk_fence_shared();
+    __syncwarp();
 
     struct Tile { // one packet's descriptor in each of the first T lanes
         uint32_t off, len, slot, valid, remote;
@@ -646,36 +652,49 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
             if (!OPEN) d.remote = a.remote_index[d.slot];
         }
     };
-    // Starts the copies of a packet's keys (when the slot is known) and of its first round into stage `buf`: two groups.
+    // Starts the copies of a packet's keys (when the slot is known) and of its first round into stage `buf`, which has been read
+    // out.  The round is one copy: it reaches the link as whole lines wherever the packet starts, and takes one instruction.
+    // HEADER_FIRST: a message's header comes with the keys besides.  Nonce and receiver index are all that the keystream and
+    // Poly1305's powers need, and they are computed while the rest is on its way, as on the seal side: 128 x 1420 B opened by
+    // receiver index 24.5 us -> 22.8, 9 x 300 B with everything on 21.1 -> 19.9.  (With the rest in pieces
+    // asked for by the lanes this gains nothing where the slot has to be looked up: loads come back in the order they were
+    // issued, those of the index table behind the packet's.  With many packets it would be a request more for each.)
+    constexpr bool HEADER_FIRST = OPEN && INLINE != 0;
+    __shared__ uint4 header_all[HEADER_FIRST ? kWppWarps : 1];
     auto fetch = [&](uint32_t off, uint32_t len, uint32_t slot, uint32_t buf) {
-        uint4 *const stage = stage_all[warp][buf];
         if ((!OPEN || !a.demux) && slot < a.max_slots && lane < 2)
             copy_async16(&key_all[warp][buf][lane], a.keys + (size_t)slot * 8 + 4u * lane);
+        if (HEADER_FIRST && lane == 0 && !(off & 15u) && len >= BNK_WG_HEADER + BNK_WG_TAG && (uint64_t)off + len <= a.ring_bytes)
+            copy_async16(&header_all[warp], a.in + off);
         copy_async_commit();
+        if (broken) return;
+        awaited |= 1u << buf;
+        if (lane != 0) return;
+        const Round r(off, 0);
+        uint32_t from = 0, end = 0; // pieces
         if (!(off & 15u)) {
-            const Round r(off, 0);
-            uint32_t from, end, extra = 0xffffffffu; // pieces [from, end), and the piece the message ends in
-            bool fits;
             if (OPEN) {
-                from = r.first;
-                fits = len >= BNK_WG_HEADER + BNK_WG_TAG && (uint64_t)off + len <= a.ring_bytes;
                 const uint32_t body = len - (BNK_WG_HEADER + BNK_WG_TAG);
-                end = r.body + (((body <= kRoundBytes ? body + BNK_WG_TAG : kRoundBytes) + 15u) >> 4);
-            } else {
+                if (len >= BNK_WG_HEADER + BNK_WG_TAG && (uint64_t)off + len <= a.ring_bytes)
+                    end = r.body + (((body <= kRoundBytes ? body + BNK_WG_TAG : kRoundBytes) + 15u) >> 4);
+            } else if ((uint64_t)off + BNK_WG_HEADER + len <= a.ring_bytes) {
                 from = r.body;
-                fits = (uint64_t)off + BNK_WG_HEADER + len <= a.ring_bytes;
                 end = r.body + ((min(len, kRoundBytes) + 15u) >> 4);
-                const uint32_t body = wg_padded_len(len, a.mtu);
+                const uint32_t body = wg_padded_len(len, a.mtu); // a message that ends inside a piece: as far as that
                 if (body <= kRoundBytes && (body & 15u) && (uint64_t)off + BNK_WG_HEADER + body + BNK_WG_TAG <= a.ring_bytes)
-                    extra = r.body + ((body + BNK_WG_TAG) >> 4);
-            }
-            if (fits) {
-#pragma unroll 1
-                for (uint32_t q = lane; q < kStagePieces; q += 32)
-                    if ((q >= from && q < end) || q == extra) copy_async16(&stage[stage_at(q)], a.in + r.window + 16u * q);
+                    end = r.body + ((body + BNK_WG_TAG + 15u) >> 4);
             }
         }
-        copy_async_commit();
+        bar_expect(&bar_all[warp][buf], 16u * (end - from));
+        if (end > from) bulk_in(&stage_all[warp][buf][from], a.in + r.at + 16u * from, 16u * (end - from), &bar_all[warp][buf]);
+    };
+    auto arrived = [&](uint32_t buf) { // the packet is in the stage
+        if (!broken) broken = !bar_wait(&bar_all[warp][buf], (parity >> buf) & 1u);
+        broken = __any_sync(0xffffffffu, broken);
+        if (broken) return;
+        parity ^= 1u << buf;
+        awaited &= ~(1u << buf);
+        __syncwarp();
     };
 
     uint32_t t = blockIdx.x * kWppWarps + warp, buf = 0;
@@ -725,7 +744,9 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
         for (uint32_t k = 0; k < in_tile; k++, buf ^= 1u) {
             const uint32_t off = __shfl_sync(0xffffffffu, cur.off, k), len = __shfl_sync(0xffffffffu, cur.len, k);
             uint32_t slot = __shfl_sync(0xffffffffu, cur.slot, k);
-            bool ahead = true; // another packet's two groups are on their way behind this one's
+            bool ahead = true; // another packet's copies are on their way behind this one's
+            if (lane == 0) bulk_out_read(); // of the other stage, which the packet before has left
+            __syncwarp();
             if (k + 1 < in_tile) {
                 fetch(__shfl_sync(0xffffffffu, cur.off, k + 1), __shfl_sync(0xffffffffu, cur.len, k + 1),
                       __shfl_sync(0xffffffffu, cur.slot, k + 1), buf ^ 1u);
@@ -743,19 +764,28 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
             // ---- what the descriptor says (the same for all lanes) ----
             uint8_t st = BNK_PKT_OK;
             uint32_t body = 0, in_len = 0, n_lo = 0, n_hi = 0;
+            uint4 ka = make_uint4(0, 0, 0, 0), kb = ka; // the keys, and whether there are any, of a slot that is looked up
+            uint8_t valid = 0;
             if (OPEN) {
-                if (ahead) copy_async_wait<2>();
+                if (ahead) copy_async_wait<1>();
                 else copy_async_wait<0>();
                 __syncwarp();
+                if (!HEADER_FIRST) arrived(buf);
                 const bool in_ring = (uint64_t)off + len <= a.ring_bytes, whole = in_ring && len >= BNK_WG_HEADER + BNK_WG_TAG;
                 uint4 hdr = make_uint4(0, 0, 0, 0);
-                if (!(off & 15u) && whole) hdr = stage[stage_at(rd.first)];
+                if (!(off & 15u) && whole) hdr = HEADER_FIRST ? header_all[warp] : stage[0];
                 if (a.demux) {
                     slot = 0; // descriptors refused below for other reasons
                     if (!(off & 15u) && whole) slot = demux_index_warp(a.index_keys, a.index_vals, a.index_slots, hdr.y);
+                    if (slot < a.max_slots) { // asked for together
+                        const uint4 *const kp = reinterpret_cast<const uint4 *>(a.keys + (size_t)slot * 8);
+                        valid = a.valid[slot];
+                        ka = kp[0];
+                        kb = kp[1];
+                    }
                 }
-                if ((off & 15u) || slot >= a.max_slots) st = slot == kSlotNoKeypair ? BNK_PKT_NO_KEYPAIR : BNK_PKT_BAD_DESC;
-                else if (!(a.demux ? a.valid[slot] : __shfl_sync(0xffffffffu, cur.valid, k))) st = BNK_PKT_NO_KEYPAIR;
+                if (broken || (off & 15u) || slot >= a.max_slots) st = slot == kSlotNoKeypair ? BNK_PKT_NO_KEYPAIR : BNK_PKT_BAD_DESC;
+                else if (!(a.demux ? valid : __shfl_sync(0xffffffffu, cur.valid, k))) st = BNK_PKT_NO_KEYPAIR;
                 else if (!in_ring) st = BNK_PKT_BAD_DESC;
                 else if (!whole) st = BNK_PKT_MALFORMED;
                 else {
@@ -786,7 +816,7 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
             }
             FlowNote note;
             auto note_begin = [&] { // the IPv4 header and the ports lie in 64 bytes
-                if (!NOTE || (off & 15u) || (uint64_t)off + BNK_WG_HEADER + len > a.ring_bytes) return;
+                if (!NOTE || broken || (off & 15u) || (uint64_t)off + BNK_WG_HEADER + len > a.ring_bytes) return;
                 const uint32_t word = stage_word(stage, rd.body);
                 Parsed p;
                 const uint32_t at = parse_ipv4_words(__shfl_sync(0xffffffffu, word, 0), __shfl_sync(0xffffffffu, word, 2),
@@ -798,10 +828,9 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                 }
             };
             if (st != BNK_PKT_OK) { // the next packet's copies are in the other stage
+                if (HEADER_FIRST) arrived(buf);
                 if (!OPEN) {
-                    if (ahead) copy_async_wait<2>();
-                    else copy_async_wait<0>();
-                    __syncwarp();
+                    arrived(buf);
                     note_begin();
                     note.place(a.ft);
                     note.count(a.ft);
@@ -812,15 +841,10 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
 
             uint32_t key[8];
             {
-                uint4 ka, kb;
-                if (OPEN && a.demux) {
-                    const uint4 *kp = reinterpret_cast<const uint4 *>(a.keys + (size_t)slot * 8);
-                    ka = kp[0];
-                    kb = kp[1];
-                } else {
+                if (!OPEN || !a.demux) {
                     if (!OPEN) {
-                        if (ahead) copy_async_wait<3>();
-                        else copy_async_wait<1>();
+                        if (ahead) copy_async_wait<1>();
+                        else copy_async_wait<0>();
                         __syncwarp();
                     }
                     ka = key_all[warp][buf][0];
@@ -853,42 +877,44 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                     for (int i = 0; i < 4; i++) pad[i] = __shfl_sync(0xffffffffu, x[4 + i], 0);
                     power.begin(r);
                     steps = last ? 32u - __clz((blocks + 3u) / 4u - 1u) : 5u;
-                    if (!OPEN) {
+                    if (!OPEN || HEADER_FIRST) {
 #pragma unroll 1
                         for (; steps; steps--) power.step();
-                        if (ahead) copy_async_wait<2>();
-                        else copy_async_wait<0>();
-                        __syncwarp();
+                        arrived(buf);
                         note_begin();
                     }
                 } else { // longer packets: the further rounds are fetched when their turn comes
                     rd = Round(off, rnd);
-                    __syncwarp(); // the stage is read out
                     const uint32_t bytes = OPEN ? rb + (last ? BNK_WG_TAG : 0u) : (in_len > done ? min(in_len - done, kRoundBytes) : 0u);
-                    const uint32_t end = rd.body + ((bytes + 15u) >> 4);
-                    const uint32_t extra = !OPEN && last && (rb & 15u) ? rd.body + ((rb + BNK_WG_TAG) >> 4) : 0xffffffffu;
-#pragma unroll 1
-                    for (uint32_t q = lane; q < kStagePieces; q += 32)
-                        if ((q >= rd.body && q < end) || q == extra)
-                            stage[stage_at(q)] = *reinterpret_cast<const uint4 *>(a.in + rd.window + 16u * q);
+                    const bool to_tag = !OPEN && last && (rb & 15u);
+                    const uint32_t end = rd.body + (((to_tag ? rb + BNK_WG_TAG : bytes) + 15u) >> 4);
                     __syncwarp();
+                    if (!broken) {
+                        awaited |= 1u << buf;
+                        if (lane == 0) {
+                            bulk_out_read();
+                            bar_expect(&bar_all[warp][buf], 16u * end);
+                            if (end) bulk_in(stage, a.in + rd.at, 16u * end, &bar_all[warp][buf]);
+                        }
+                    }
+                    arrived(buf);
                 }
                 // ---- cipher ----
                 const bool works = lane != 0 && (lane - 1u) * 64u < rb;
                 const int body_left = (int)rb - (int)(lane - 1u) * 64;
                 const uint32_t end_at = 16u * rd.body + rb + lane; // byte `lane` behind the round's body, in the stage
-                uint8_t *const end_byte = stage_bytes + 16u * stage_at(end_at >> 4) + (end_at & 15u);
+                uint8_t *const end_byte = stage_bytes + end_at;
                 const bool in_last_piece = lane < ((0u - rb) & 15u); // it shares the body's last piece
                 if (!OPEN && in_len < body) { // WireGuard's padding: zeros behind the payload
                     const uint32_t at = in_len + lane - done;
                     if (lane < 16u && in_len + lane >= done && at < rb)
-                        stage_bytes[16u * stage_at(rd.body + (at >> 4)) + (at & 15u)] = 0;
+                        stage_bytes[16u * rd.body + at] = 0;
                     __syncwarp();
                 }
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     if (!works || 16 * c >= body_left) continue;
-                    uint4 *const p = &stage[stage_at(rd.body + 4u * (lane - 1u) + c)];
+                    uint4 *const p = &stage[rd.body + 4u * (lane - 1u) + c];
                     const uint4 v = *p;
                     x[4 * c + 0] ^= v.x;
                     x[4 * c + 1] ^= v.y;
@@ -911,7 +937,7 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                     const int blk = b0 + s;
                     uint4 m = make_uint4(0u, 0u, body, 0u); // le64(0) | le64(body)
                     if (blk >= 0 && (uint32_t)blk < data_blocks) {
-                        m = stage[stage_at(rd.body + blk)];
+                        m = stage[rd.body + blk];
                         const int left = (int)rb - 16 * blk;
                         if (OPEN && left < 16) {
                             m.x = keep_bytes(m.x, left);
@@ -942,7 +968,7 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                     const uint8_t tb = (uint8_t)(tw >> (8u * (lane & 3u)));
                     if (OPEN) {
                         tag_byte = *end_byte;
-                        forged = __any_sync(0xffffffffu, lane < 16u && tag_byte != tb);
+                        forged = __any_sync(0xffffffffu, lane < 16u && tag_byte != tb) || broken;
                     } else if (lane < 16u) {
                         *end_byte = tb;
                     }
@@ -952,12 +978,12 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
 #pragma unroll
                     for (int c = 0; c < 4; c++)
                         if (works && 16 * c < body_left)
-                            stage[stage_at(rd.body + 4u * (lane - 1u) + c)] =
+                            stage[rd.body + 4u * (lane - 1u) + c] =
                                 forged ? make_uint4(0, 0, 0, 0) : make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
                     __syncwarp();
                     if (last && in_last_piece) *end_byte = tag_byte; // what is not plaintext goes back as it came
                 } else if (rnd == 0 && lane == 0) {
-                    stage[stage_at(rd.first)] = make_uint4(4u, remote, n_lo, n_hi);
+                    stage[0] = make_uint4(4u, remote, n_lo, n_hi);
                 }
                 __syncwarp();
                 if (OPEN && a.inner && rnd == 0 && !forged) {
@@ -979,30 +1005,35 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                 const uint32_t out_bytes = OPEN ? rb : rb + (last ? BNK_WG_TAG : 0u);
                 const bool other_place = a.in != a.out;
                 const uint32_t out_end = rd.body + ((out_bytes + (other_place ? 0u : 15u)) >> 4);
-#pragma unroll 1
-                for (uint32_t q = lane; q < out_end; q += 32) {
-                    if (q < (OPEN ? rd.body : rd.first)) continue;
-                    const uint4 v = stage[stage_at(q)];
-                    *reinterpret_cast<uint4 *>(a.out + rd.window + 16u * q) = v;
-                    if (a.out2) *reinterpret_cast<uint4 *>(a.out2 + rd.window + 16u * q) = v;
+                const uint32_t out_from = OPEN ? rd.body : 0u; // (the open side's header stays)
+                bulk_fence_shared();
+                __syncwarp();
+                if (lane == 0 && out_end > out_from && !broken) {
+                    bulk_out(a.out + rd.at + 16u * out_from, &stage[out_from], 16u * (out_end - out_from));
+                    if (a.out2) bulk_out(a.out2 + rd.at + 16u * out_from, &stage[out_from], 16u * (out_end - out_from));
+                    bulk_out_commit();
                 }
-                if (other_place && lane < (out_bytes & 15u)) {
-                    const uint8_t v = stage_bytes[16u * stage_at(out_end) + lane];
-                    a.out[rd.window + 16u * out_end + lane] = v;
-                    if (a.out2) a.out2[rd.window + 16u * out_end + lane] = v;
+                if (other_place && lane < (out_bytes & 15u) && !broken) {
+                    const uint8_t v = stage_bytes[16u * out_end + lane];
+                    a.out[rd.at + 16u * out_end + lane] = v;
+                    if (a.out2) a.out2[rd.at + 16u * out_end + lane] = v;
                 }
                 if (last) break;
             }
             if (OPEN && forged && body > kRoundBytes) { // the earlier rounds' plaintext is out already: wipe it
                 uint8_t *const data = a.out + (size_t)off + BNK_WG_HEADER, *const data2 = a.out2 + (size_t)off + BNK_WG_HEADER;
                 const uint32_t end = body - (body - 1u) % kRoundBytes - 1u; // what lies in the rounds before the last
+                if (lane == 0) bulk_out_done(); // it is, and the zeros come behind it
+                bulk_fence();
                 __syncwarp();
                 for (uint32_t q = lane * 16u; q < end; q += 512u) {
                     *reinterpret_cast<uint4 *>(data + q) = make_uint4(0, 0, 0, 0);
                     if (a.out2) *reinterpret_cast<uint4 *>(data2 + q) = make_uint4(0, 0, 0, 0);
                 }
             }
-            if (lane == k) {
+            if (lane == k && broken) {
+                res_status = BNK_PKT_BAD_DESC;
+            } else if (lane == k) {
                 res_status = OPEN ? (forged ? BNK_PKT_AUTH_FAIL : body ? BNK_PKT_OK : BNK_PKT_KEEPALIVE) : BNK_PKT_OK;
                 res_len = OPEN ? (forged ? 0u : body) : BNK_WG_HEADER + body + BNK_WG_TAG;
             }
@@ -1031,6 +1062,9 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
         }
         cur = next;
     }
+    if (lane == 0) bulk_out_done();
+    for (uint32_t b = 0; broken && b < 2; b++) // a copy that is still on its way must not meet the next kernel's shared memory
+        if ((awaited >> b) & 1u) bar_wait(&bar_all[warp][b], (parity >> b) & 1u);
     if (by_cta) {
         __syncthreads();
         const uint32_t i = blockIdx.x * kWppWarps + threadIdx.x;
@@ -1063,7 +1097,7 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
 // Packets on the device whose messages go to the host as well only store over the link, and all warps that fit help:
 // 12,032 x 1420 B in 421 us by 64 CTAs, 395 by 128, 375 by 444 and more.
 constexpr uint64_t kLinkWindow = 64u << 10, kLeastCtas = 64, kMostCtas = 512;
-constexpr uint32_t kStoreCtas = 592;
+constexpr uint32_t kStoreCtas = 592, kEvenCtas = 96;
 // The seal kernel hands out nonces for one packet per warp, counted over one tile of the whole batch: a batch of that size
 // has to get a warp for every packet.
 static_assert(kRankMax <= kLeastCtas * kWppWarps, "batches that hand out their own nonces run a packet per warp");
@@ -1075,6 +1109,13 @@ void wpp_grid(AeadArgs &a, uint32_t &ctas) {
     if (!a.from_host) ctas = std::min(ctas, kStoreCtas);
     else ctas = (uint32_t)std::min<uint64_t>(ctas, std::min(std::max(kLinkWindow / per_packet, kLeastCtas), kMostCtas));
     while (a.tile < 8 && a.n > ctas * kWppWarps * a.tile) a.tile *= 2;
+    // Warps that all take as many tiles end together: 8000 x 1420 B are four rounds for 64 CTAs, of which the last has most of
+    // them idle, and three for 84 (sealed 382 us and 363, opened 396 and 374; 15,000 of them 691 and 670, 711 and 656).
+    const uint32_t tiles = (a.n + a.tile - 1) / a.tile;
+    if (a.from_host && tiles > ctas * kWppWarps) {
+        const uint32_t rounds = (tiles + std::max(ctas, kEvenCtas) * kWppWarps - 1) / (std::max(ctas, kEvenCtas) * kWppWarps);
+        ctas = (tiles + rounds * kWppWarps - 1) / (rounds * kWppWarps);
+    }
 }
 template <bool OPEN, bool NOTE>
 cudaError_t launch_wpp(const AeadArgs &a, uint32_t ctas, const HostDesc *h, cudaStream_t s) {

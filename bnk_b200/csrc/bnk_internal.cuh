@@ -284,8 +284,10 @@ struct Done {
     uint32_t *flag;   // pinned; null: nobody watches
     uint32_t value;
 };
-// By all threads of all CTAs, once, at the end; `last_words` (if `has_words`) runs in one thread when every CTA's stores
-// are visible.  A fence that covers host memory takes ~1.5 us, so there is no second one when nothing is said.
+// By all threads of all CTAs, once, at the end; `last_words` (if `has_words`) runs in one thread when every CTA's work is
+// visible on the device.  There is one fence that covers host memory, which takes 1.7 us (one in front of the last words as
+// well: a packet sealed with its flow noted 18.9 us, without it 16.4).  Finding out who is last takes 0.75 us, but with a word
+// per CTA, all watched by the host, every CTA has that fence: 128 x 1420 B sealed by 32 CTAs 19.7 us, so 23.0.
 template <typename F>
 __device__ __forceinline__ void signal_done(const Done &d, bool has_words, F last_words) {
     if (d.flag == nullptr) return;
@@ -296,12 +298,11 @@ __device__ __forceinline__ void signal_done(const Done &d, bool has_words, F las
         if (atomicAdd(d.ticket, 1u) + 1u != gridDim.x) return;
         *d.ticket = 0u;
     }
-    __threadfence_system();
     if (has_words) {
         __threadfence();
         last_words();
-        __threadfence_system();
     }
+    __threadfence_system();
     *(volatile uint32_t *)d.flag = d.value;
 }
 struct HostDesc { // the descriptors where the host can read them

@@ -30,5 +30,14 @@ __device__ __forceinline__ void bulk_in(void *smem, const void *gmem, uint32_t b
                  "l"(__cvta_generic_to_global(gmem)), "r"(bytes), "r"(shared_at(bar))
                  : "memory");
 }
+__device__ __forceinline__ void bulk_out(void *gmem, const void *smem, uint32_t bytes) { // counted per thread
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(__cvta_generic_to_global(gmem)), "r"(shared_at(smem)),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_out_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_out_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); } // shared memory may change
+__device__ __forceinline__ void bulk_out_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }      // it is all where it belongs
+__device__ __forceinline__ void bulk_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
 // Between this thread's own accesses to shared memory and the bulk copies that follow.
 __device__ __forceinline__ void bulk_fence_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
