@@ -486,3 +486,13 @@ def test_heads_of_packets_anywhere_in_the_ring(gpu_lib, oracle, n):
                         chk.note_outbound(p, RC.T0)
             assert flows_equal(c.flows_export(), chk.flows())
             b.close()
+
+
+@pytest.mark.parametrize("n", [1, 1025, 16385, 49153])
+def test_packets_close_together_where_nothing_is_read_in_place(gpu_lib, oracle, n, monkeypatch):
+    """The copies that bring heads up when pinned memory may not be read by the kernels."""
+    monkeypatch.setenv("BNK_HOST_DIRECT_BYTES", "0")
+    if n > 1:
+        return test_packets_close_together_go_up_stretch_by_stretch(gpu_lib, oracle, n, True)
+    for k in (1, 511, 799):
+        test_heads_of_packets_anywhere_in_the_ring(gpu_lib, oracle, k)
