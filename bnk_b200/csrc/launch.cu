@@ -160,6 +160,15 @@ cudaError_t launch_any(const LaunchShape &shape, void *const *args, const uint32
     return launch_now(shape, args, s);
 }
 
+static cudaKernelNodeParams node_params(const LaunchShape &k, void **args) {
+    cudaKernelNodeParams p = {};
+    p.func = const_cast<void *>(k.fn);
+    p.gridDim = k.grid;
+    p.blockDim = k.block;
+    p.sharedMemBytes = k.smem;
+    p.kernelParams = args;
+    return p;
+}
 // A graph of the n gathered launches' kernels, made if need be.
 LaunchGraph *Launches::graph(uint32_t n) {
     int device = 0;
@@ -175,31 +184,34 @@ LaunchGraph *Launches::graph(uint32_t n) {
     want.device = device;
     LaunchGraph *g = pool.take(want);
     if (!GraphPool::to_be_made(g)) return g;
+    // Put together node by node: with a stream captured instead, cuCtxSynchronize of another thread (which a batch's creation
+    // calls) crashed now and then.
     g = new (std::nothrow) LaunchGraph(want);
-    cudaStream_t s = nullptr;
     int low = 0, high = 0; // the priority that batches' streams have
     cudaError_t e = g ? cudaDeviceGetStreamPriorityRange(&low, &high) : cudaErrorMemoryAllocation;
-    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, high);
-    if (e == cudaSuccess) e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        for (uint32_t i = 0; i < n && e == cudaSuccess; i++) {
-            LaunchShape k = one_[i].shape;
-            k.behind = k.behind && i > 0;
-            e = launch_now(k, one_[i].args, s);
+    if (e == cudaSuccess) e = cudaGraphCreate(&g->graph, 0);
+    for (uint32_t i = 0; i < n && e == cudaSuccess; i++) {
+        const cudaKernelNodeParams p = node_params(one_[i].shape, one_[i].args);
+        e = cudaGraphAddKernelNode(&g->node[i], g->graph, nullptr, 0, &p);
+        cudaLaunchAttributeValue v = {};
+        v.priority = high;
+        if (e == cudaSuccess) e = cudaGraphKernelNodeSetAttribute(g->node[i], cudaLaunchAttributePriority, &v);
+        if (e == cudaSuccess && want.cluster[i] > 1) {
+            v = {};
+            v.clusterDim.x = want.cluster[i];
+            v.clusterDim.y = v.clusterDim.z = 1;
+            e = cudaGraphKernelNodeSetAttribute(g->node[i], cudaLaunchAttributeClusterDimension, &v);
         }
-        const cudaError_t end = cudaStreamEndCapture(s, &g->graph);
-        if (e == cudaSuccess) e = end;
     }
-    size_t roots = 1, nodes = 2;
-    cudaGraphNode_t node[2] = {};
-    if (e == cudaSuccess) e = cudaGraphGetRootNodes(g->graph, &g->node[0], &roots);
-    if (e == cudaSuccess) e = cudaGraphGetNodes(g->graph, node, &nodes);
-    if (e == cudaSuccess && (roots != 1 || nodes != n)) e = cudaErrorUnknown;
-    if (e == cudaSuccess) {
-        g->node[1] = node[0] == g->node[0] ? node[1] : node[0];
-        e = cudaGraphInstantiate(&g->exec, g->graph, 0);
+    if (e == cudaSuccess && n == 2) {
+        cudaGraphEdgeData edge = {};
+        if (want.behind) {
+            edge.type = cudaGraphDependencyTypeProgrammatic;
+            edge.from_port = cudaGraphKernelNodePortProgrammatic;
+        }
+        e = cudaGraphAddDependencies_v2(g->graph, &g->node[0], &g->node[1], &edge, 1);
     }
-    if (s) cudaStreamDestroy(s);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, g->graph, 0);
     if (e != cudaSuccess) {
         if (g && g->graph) cudaGraphDestroy(g->graph);
         delete g;
@@ -218,12 +230,7 @@ cudaError_t Launches::send(LaunchGraph *&taken) {
     if (!g) return stop();
     cudaError_t e = cudaSuccess;
     for (uint32_t i = 0; i < n_ && e == cudaSuccess; i++) {
-        cudaKernelNodeParams p = {};
-        p.func = const_cast<void *>(one_[i].shape.fn);
-        p.gridDim = one_[i].shape.grid;
-        p.blockDim = one_[i].shape.block;
-        p.sharedMemBytes = one_[i].shape.smem;
-        p.kernelParams = one_[i].args;
+        const cudaKernelNodeParams p = node_params(one_[i].shape, one_[i].args);
         e = cudaGraphExecKernelNodeSetParams(g->exec, g->node[i], &p);
     }
     if (e == cudaSuccess) e = cudaGraphLaunch(g->exec, s_);

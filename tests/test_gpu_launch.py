@@ -146,3 +146,16 @@ def test_batches_in_flight_and_contexts_beside_each_other(gpu_lib, oracle):
     for b in batches[0]:
         b.close()
     made[0].close()
+
+
+def test_graphs_made_while_other_threads_create_batches(gpu_lib):
+    """Six threads make their batches, which synchronises the device, while the first of them already submit and their graphs
+    are made; a process each time, as graphs are made once."""
+    import subprocess
+
+    from bnk_b200 import _build
+
+    exe = _build.build_mt_stress()
+    for _ in range(6):
+        res = subprocess.run([exe, "6", "10", "128", "1420", "4"], capture_output=True, text=True, timeout=120)
+        assert res.returncode == 0 and res.stdout.startswith("OK"), (res.returncode, res.stdout[-500:] + res.stderr[-2000:])
