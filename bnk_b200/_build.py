@@ -110,6 +110,26 @@ def build_mt_stress(force: bool = False) -> str:
     return _build_cpp(os.path.join(HOST, "apps", "mt_stress.cpp"), os.path.join(HOST, "apps", "mt_stress"), force)
 
 
+LOST_BYTES, LOST_TURNS = 720, 64
+
+
+def lost_copies_path() -> str:
+    return os.path.join(os.path.dirname(PKG_DIR), "build", "lost_copies", "libbnkgpu.so")
+
+
+def build_lost_copies(force: bool = False) -> str:
+    """libbnkgpu.so for the tests of what happens when a copy over the link does not come: its kernels never ask for bulk
+    copies of LOST_BYTES, and their waits give up after LOST_TURNS turns."""
+    lib = lost_copies_path()
+    if force or _stale(lib, _deps()):
+        os.makedirs(os.path.dirname(lib), exist_ok=True)
+        cmd = [nvcc_path(), *NVCC_FLAGS, f"-DBNK_BULK_LOST={LOST_BYTES}u", f"-DBNK_BULK_TURNS={LOST_TURNS}u", "-o", lib, *sources()]
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
+    return lib
+
+
 SAN_FLAGS = {"asan": "-fsanitize=address,-fsanitize=undefined", "tsan": "-fsanitize=thread"}
 
 

@@ -245,12 +245,16 @@ def lib() -> C.CDLL:
             f"{path} is missing: build it with `python -m bnk_b200._build` (needs nvcc). "
             "bnk_b200 has no CPU fallback."
         )
+    _LIB = load(path)
+    return _LIB
+
+
+def load(path: str) -> C.CDLL:
     L = C.CDLL(path)
     for name, (res, args) in SYMBOLS.items():
         fn = getattr(L, name)
         fn.restype = res
         fn.argtypes = args
-    _LIB = L
     return L
 
 

@@ -6,6 +6,11 @@
 
 #include <stdint.h>
 
+// How often a wait looks before it gives up.  (A build for tests has it give up soon, and BNK_BULK_LOST set: copies of that many
+// bytes are never asked for, which is what a link that has stopped looks like from here.)
+#ifndef BNK_BULK_TURNS
+#define BNK_BULK_TURNS (1u << 22)
+#endif
 __device__ __forceinline__ uint32_t shared_at(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void bar_init(uint64_t *bar) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_at(bar)) : "memory");
@@ -15,7 +20,7 @@ __device__ __forceinline__ void bar_expect(uint64_t *bar, uint32_t bytes) { // t
 }
 // False: it has not come after so many turns (80 ms at the least), which no link that works takes.
 __device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
-    for (uint32_t turn = 0; turn < (1u << 22); turn++) {
+    for (uint32_t turn = 0; turn < BNK_BULK_TURNS; turn++) {
         uint32_t over;
         asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
                      : "=r"(over)
@@ -26,6 +31,9 @@ __device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
     return false;
 }
 __device__ __forceinline__ void bulk_in(void *smem, const void *gmem, uint32_t bytes, uint64_t *bar) {
+#ifdef BNK_BULK_LOST
+    if (bytes == BNK_BULK_LOST) return;
+#endif
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(shared_at(smem)),
                  "l"(__cvta_generic_to_global(gmem)), "r"(bytes), "r"(shared_at(bar))
                  : "memory");

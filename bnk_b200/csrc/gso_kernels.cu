@@ -72,6 +72,7 @@ __device__ __forceinline__ void split_packet(const SplitArgs &a, uint32_t pkt, u
     const uint32_t o = off[pkt];
     const uint64_t at = (uint64_t)sp.src_off + data_at; // of the payload, in the ring
     const uint8_t *payload = ring + at;
+    bool came = true;
     if (FROM_HOST) { // (of such super-packets the host knows that they are whole and each segment fits the window)
         const uint64_t from = at & ~15ull, end = at + min((uint32_t)sp.gso_size, sp.src_len - data_at);
         const uint32_t bytes = (uint32_t)(((end + 15u) & ~15ull) - from);
@@ -79,24 +80,25 @@ __device__ __forceinline__ void split_packet(const SplitArgs &a, uint32_t pkt, u
             bar_expect(bar, bytes);
             bulk_in(stage, a.host_ring + from, bytes, bar);
         }
-        if (!__all_sync(0xffffffffu, bar_wait(bar, 0))) ok = false; // (nothing else is read into the stage)
+        came = __all_sync(0xffffffffu, bar_wait(bar, 0));
         __syncwarp();
         payload = reinterpret_cast<const uint8_t *>(stage) + (at - from);
         const uint64_t word0 = (at + 3u) & ~3ull, whole = (uint64_t)sp.src_off + sp.src_len;
-        for (uint64_t w = word0 + 4u * lane; w < end; w += 128u) {
+        for (uint64_t w = word0 + 4u * lane; came && w < end; w += 128u) {
             const uint8_t *const v = reinterpret_cast<const uint8_t *>(stage) + (w - from);
             if (w + 4u <= whole) *reinterpret_cast<uint32_t *>(ring + w) = *reinterpret_cast<const uint32_t *>(v);
             else
                 for (uint64_t b = w; b < whole; b++) ring[b] = v[b - w];
         }
     }
-    if (ok) {
+    if (ok && came) {
         seg_len = min((uint32_t)sp.gso_size, sp.src_len - data_at);
         total = hdr + seg_len;
         ok = len[pkt] == total && (o & 15u) == 0 && (uint64_t)o + 16 + total + 32 <= ring_bytes && total <= 65535u;
     }
-    if (!ok) {
+    if (!ok || !came) {
         if (lane == 0) slot[pkt] = 0xffffffffu; // the seal that follows reports BNK_PKT_BAD_DESC for it
+        if (FROM_HOST && !came) bar_wait(bar, 0); // a copy that is still on its way must not meet the next kernel's shared memory
         return;
     }
     const uint8_t *in = ring + sp.src_off;
