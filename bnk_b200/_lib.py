@@ -13,7 +13,7 @@ from . import _build
 SUCCESS, EINVAL, ENOMEM, ECUDA, ETIMEDOUT, EBUSY, EFULL = 0, -1, -2, -3, -4, -5, -6
 
 PKT_OK, PKT_AUTH_FAIL, PKT_REPLAY, PKT_FILTER_DENY, PKT_MALFORMED, PKT_KEEPALIVE, PKT_COUNTER_EXHAUSTED, PKT_BAD_DESC = range(8)
-PKT_NO_KEYPAIR, PKT_BAD_INNER = 8, 9
+PKT_NO_KEYPAIR, PKT_BAD_INNER, PKT_NOT_READ = 8, 9, 13
 
 F_NO_H2D = 1 << 0
 F_NO_D2H = 1 << 1

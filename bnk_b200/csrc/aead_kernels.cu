@@ -784,7 +784,8 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                         kb = kp[1];
                     }
                 }
-                if (broken || (off & 15u) || slot >= a.max_slots) st = slot == kSlotNoKeypair ? BNK_PKT_NO_KEYPAIR : BNK_PKT_BAD_DESC;
+                if (broken) st = BNK_PKT_NOT_READ;
+                else if ((off & 15u) || slot >= a.max_slots) st = slot == kSlotNoKeypair ? BNK_PKT_NO_KEYPAIR : BNK_PKT_BAD_DESC;
                 else if (!(a.demux ? valid : __shfl_sync(0xffffffffu, cur.valid, k))) st = BNK_PKT_NO_KEYPAIR;
                 else if (!in_ring) st = BNK_PKT_BAD_DESC;
                 else if (!whole) st = BNK_PKT_MALFORMED;
@@ -1032,7 +1033,7 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                 }
             }
             if (lane == k && broken) {
-                res_status = BNK_PKT_BAD_DESC;
+                res_status = BNK_PKT_NOT_READ;
             } else if (lane == k) {
                 res_status = OPEN ? (forged ? BNK_PKT_AUTH_FAIL : body ? BNK_PKT_OK : BNK_PKT_KEEPALIVE) : BNK_PKT_OK;
                 res_len = OPEN ? (forged ? 0u : body) : BNK_WG_HEADER + body + BNK_WG_TAG;

@@ -281,7 +281,8 @@ __global__ void __launch_bounds__(256) packets_to_host_kernel(const uint8_t *rin
     uint64_t at = off[i] + 16ull;
     uint32_t bytes = len[i];
     const uint8_t st = i < sealed ? status[i] : (uint8_t)BNK_PKT_BAD_DESC;
-    if (st != BNK_PKT_BAD_DESC && st != BNK_PKT_NO_KEYPAIR && st != BNK_PKT_COUNTER_EXHAUSTED && st != BNK_PKT_MALFORMED) {
+    if (st != BNK_PKT_BAD_DESC && st != BNK_PKT_NO_KEYPAIR && st != BNK_PKT_COUNTER_EXHAUSTED && st != BNK_PKT_MALFORMED &&
+        st != BNK_PKT_NOT_READ) {
         at -= 16u;
         bytes = 16u + wg_padded_len(bytes, mtu) + 16u;
     }

@@ -28,6 +28,7 @@ from ._lib import (  # noqa: F401  (re-exported)
     PKT_BAD_DESC,
     PKT_BAD_INNER,
     PKT_NO_KEYPAIR,
+    PKT_NOT_READ,
     PKT_COUNTER_EXHAUSTED,
     PKT_FILTER_DENY,
     PKT_KEEPALIVE,

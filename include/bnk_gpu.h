@@ -70,6 +70,11 @@ extern "C" {
                                        BNK_F_DEMUX_INDEX the receiver index in the header maps to no keypair */
 #define BNK_PKT_BAD_INNER 9         /* BNK_F_INNER_CHECK: decrypted packet is not IPv4, lies about its length,
                                        or does not come from the peer's allowed address */
+#define BNK_PKT_NOT_READ 13         /* a fault of the host link, not of the packet: its bytes did not come within the time a
+                                       kernel waits for them (tenths of a second), or did not for a packet that the same
+                                       warp was to work on first.  out_len is 0.  The ring holds what it held, but for
+                                       packets beyond 1984 bytes: of those the stretches in front are sealed already, or
+                                       zeros where they were opened.  A nonce handed out to the packet stays unused. */
 
 #define BNK_WG_HEADER 16u
 #define BNK_WG_TAG 16u
@@ -274,8 +279,9 @@ int bnk_classify_submit(bnk_batch *b, uint32_t npkts, uint32_t flags);
  * Packets that are no super-packet's segments stay as they are, so one batch may hold both.  The submit
  * copies the super-packets, those other packets, the descriptors and `supers` to the device unless
  * BNK_F_NO_H2D is given, and copies nothing back.  A segment whose descriptor does not match the split
- * (wrong len, out of range, unsupported header layout) has its device-side slot[] set to an invalid
- * keypair, so the seal that follows reports BNK_PKT_BAD_DESC for it. */
+ * (wrong len, out of range, unsupported header layout), or whose bytes did not come over the link in time
+ * (see BNK_PKT_NOT_READ), has its device-side slot[] set to an invalid keypair, so the seal that follows
+ * reports BNK_PKT_BAD_DESC for it. */
 typedef struct bnk_gso_super {
     uint32_t src_off;     /* 4-byte aligned */
     uint32_t src_len;

@@ -5,7 +5,9 @@ import os
 import numpy as np
 import pytest
 
+from bnk_b200.filter import CompiledRule, PortRange, flatten_rules
 from tests import helpers as H
+from tests import reference_cases as RC
 
 pytestmark = pytest.mark.gpu
 
@@ -71,4 +73,78 @@ def test_split_leaves_out_what_did_not_come(lossy, oracle):
             assert b.ring[off[i] + 16:off[i] + 16 + lens[i]].tobytes() == w, i
         b.seal(n, F_NO_H2D)
         assert list(np.flatnonzero(b.status)) == [5] and b.out_len[5] == 0
+        b.close()
+
+
+ROUND = 1984  # payload bytes a warp takes per round
+
+
+# 8: a warp each, the descriptors with the launch and the header of a message ahead; 1024: tiles of four, so up to three packets
+# lie behind the one that does not come; long: its second round does not come
+@pytest.mark.parametrize("n,lost,long", [(8, 3, False), (8, 0, True), (256, 255, False), (1024, 513, False), (1024, 515, True)])
+def test_seal_and_open_refuse_what_did_not_come(lossy, oracle, n, lost, long):
+    from bnk_b200 import Context
+    from bnk_b200.device import F_ASSIGN_COUNTERS, F_NOTE_OUTBOUND, F_REPLAY, PKT_NOT_READ
+
+    rng = np.random.default_rng(n + lost)
+    peers, stride, now = 5, 4096, RC.T0
+    keys = rng.integers(0, 256, (peers, 32), dtype=np.uint8)
+    off, slot = H.layout_fixed(n, stride), rng.integers(0, peers, n).astype(np.uint32)
+    refused = np.arange(n) == lost if n <= 256 else (np.arange(n) >= lost) & (np.arange(n) < lost // 4 * 4 + 4)
+    with Context(max_keypairs=peers, mtu=0, flow_capacity=1 << 12, replay_ring_blocks=32) as c:
+        c.set_keypairs(0, keys, keys, np.arange(peers, dtype=np.uint32))
+        c.acl_set(True, flatten_rules([CompiledRule(srcs=["10.0.0.0/8"], proto="udp", ports=[PortRange(1, 9)])]))
+        b = c.batch(n, n * stride)
+        b.off[:], b.slot[:] = off, slot
+
+        def lay_out(lens):
+            b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
+            for i in range(n):
+                p = RC.udp(RC.SELF, RC.ip("10.0.0.0") + i, 7, 8)[:28]
+                b.ring[off[i] + 16:off[i] + 44] = np.frombuffer(p[:2] + int(lens[i]).to_bytes(2, "big") + p[4:], np.uint8)
+            b.len[:] = lens
+            return np.array(b.ring)
+
+        # ---- sealed ----
+        lens = np.full(n, 1104, np.uint32)
+        lens[lost] = (ROUND if long else 0) + lossy - 9
+        ctr = np.array([np.count_nonzero(slot[:i] == slot[i]) for i in range(n)], np.uint64)
+        plain = lay_out(lens)
+        ring, st, ln = H.oracle_seal(oracle, keys, np.arange(peers), 0, plain, off, lens, slot, ctr)
+        b.seal(n, F_ASSIGN_COUNTERS | F_NOTE_OUTBOUND, now)
+        assert np.array_equal(b.status, np.where(refused, PKT_NOT_READ, st))
+        assert np.array_equal(b.out_len, np.where(refused, 0, ln))
+        assert H.spans_equal(np.array(b.ring), ring, off[~refused], ln[~refused]) == []
+        kept = off + (16 + ROUND) * (long & (np.arange(n) == lost)).astype(np.uint32)  # the first round of a long message is out
+        assert H.spans_equal(np.array(b.ring), plain, kept[refused], off[refused] + stride - kept[refused]) == []
+        if long:
+            assert H.spans_equal(np.array(b.ring), ring, off[[lost]], [16 + ROUND]) == []
+        assert c.flows_count() == n - refused.sum() + long  # (its flow is in the first round)
+
+        # ---- opened ----
+        lens[lost] = (ROUND if long else 0) + lossy - 32 + (16 if long else 0)
+        plain = lay_out(lens)
+        ctr += 1000
+        ring, st, ln = H.oracle_seal(oracle, keys, np.arange(peers), 0, plain, off, lens, slot, ctr)
+        b.ring[:], b.len[:] = ring, ln
+        want_ring, st, got_ctr, want_ln = H.oracle_open(oracle, keys, ring, off, ln, slot)
+        b.open(n, F_REPLAY)
+        st[refused] = PKT_NOT_READ
+        want, state = H.oracle_replay(oracle, 32, slot, got_ctr, st)
+        assert np.array_equal(b.status, want) and np.array_equal(b.out_len, np.where(refused, 0, want_ln))
+        assert H.spans_equal(np.array(b.ring), want_ring, off[~refused], want_ln[~refused], 16) == []
+        if long:
+            ring[off[lost] + 16:off[lost] + 16 + ROUND] = 0
+        assert H.spans_equal(np.array(b.ring), ring, off[refused], [stride] * refused.sum()) == []
+        for s, r in state.items():
+            last, words = c.replay_export(s)
+            assert last == r.last and np.array_equal(words, r.ring())
+
+        # ---- and the next submit is as any other ----
+        lens[lost] = 700 if not long else ROUND + 732  # (copies of 704 and 736 bytes)
+        plain = lay_out(lens)
+        ring, st, ln = H.oracle_seal(oracle, keys, np.arange(peers), 0, plain, off, lens, slot, ctr)
+        b.counter[:] = ctr
+        b.seal(n)
+        assert np.array_equal(b.status, st) and H.spans_equal(np.array(b.ring), ring, off, ln) == []
         b.close()
