@@ -654,17 +654,18 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
     };
     // Starts the copies of a packet's keys (when the slot is known) and of its first round into stage `buf`, which has been read
     // out.  The round is one copy: it reaches the link as whole lines wherever the packet starts, and takes one instruction.
-    // HEADER_FIRST: a message's header comes with the keys besides.  Nonce and receiver index are all that the keystream and
+    // header_first: a message's header comes with the keys besides.  Nonce and receiver index are all that the keystream and
     // Poly1305's powers need, and they are computed while the rest is on its way, as on the seal side: 128 x 1420 B opened by
     // receiver index 24.5 us -> 22.8, 9 x 300 B with everything on 21.1 -> 19.9.  (With the rest in pieces
     // asked for by the lanes this gains nothing where the slot has to be looked up: loads come back in the order they were
-    // issued, those of the index table behind the packet's.  With many packets it would be a request more for each.)
-    constexpr bool HEADER_FIRST = OPEN && INLINE != 0;
-    __shared__ uint4 header_all[HEADER_FIRST ? kWppWarps : 1];
+    // issued, those of the index table behind the packet's.)  It is a request more for each packet, which many threads feel:
+    // see open_direct.
+    const bool header_first = OPEN && INLINE != 0 && a.header_first;
+    __shared__ uint4 header_all[OPEN && INLINE != 0 ? kWppWarps : 1];
     auto fetch = [&](uint32_t off, uint32_t len, uint32_t slot, uint32_t buf) {
         if ((!OPEN || !a.demux) && slot < a.max_slots && lane < 2)
             copy_async16(&key_all[warp][buf][lane], a.keys + (size_t)slot * 8 + 4u * lane);
-        if (HEADER_FIRST && lane == 0 && !(off & 15u) && len >= BNK_WG_HEADER + BNK_WG_TAG && (uint64_t)off + len <= a.ring_bytes)
+        if (header_first && lane == 0 && !(off & 15u) && len >= BNK_WG_HEADER + BNK_WG_TAG && (uint64_t)off + len <= a.ring_bytes)
             copy_async16(&header_all[warp], a.in + off);
         copy_async_commit();
         if (broken) return;
@@ -770,10 +771,10 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                 if (ahead) copy_async_wait<1>();
                 else copy_async_wait<0>();
                 __syncwarp();
-                if (!HEADER_FIRST) arrived(buf);
+                if (!header_first) arrived(buf);
                 const bool in_ring = (uint64_t)off + len <= a.ring_bytes, whole = in_ring && len >= BNK_WG_HEADER + BNK_WG_TAG;
                 uint4 hdr = make_uint4(0, 0, 0, 0);
-                if (!(off & 15u) && whole) hdr = HEADER_FIRST ? header_all[warp] : stage[0];
+                if (!(off & 15u) && whole) hdr = header_first ? header_all[warp] : stage[0];
                 if (a.demux) {
                     slot = 0; // descriptors refused below for other reasons
                     if (!(off & 15u) && whole) slot = demux_index_warp(a.index_keys, a.index_vals, a.index_slots, hdr.y);
@@ -829,7 +830,7 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                 }
             };
             if (st != BNK_PKT_OK) { // the next packet's copies are in the other stage
-                if (HEADER_FIRST) arrived(buf);
+                if (header_first) arrived(buf);
                 if (!OPEN) {
                     arrived(buf);
                     note_begin();
@@ -878,7 +879,7 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                     for (int i = 0; i < 4; i++) pad[i] = __shfl_sync(0xffffffffu, x[4 + i], 0);
                     power.begin(r);
                     steps = last ? 32u - __clz((blocks + 3u) / 4u - 1u) : 5u;
-                    if (!OPEN || HEADER_FIRST) {
+                    if (!OPEN || header_first) {
 #pragma unroll 1
                         for (; steps; steps--) power.step();
                         arrived(buf);

@@ -125,12 +125,13 @@ void submit_over(bnk_batch *b) { // waited for, or going away
     if (b->direct_counted) b->ctx->direct_in_flight.fetch_sub(b->direct_counted, std::memory_order_relaxed);
     b->direct_counted = 0;
 }
-// Launches what a submit has gathered (launch.h).  Through a graph while at most two other batches are in flight; more of
-// them come from several threads.
-constexpr int kGraphOthers = 2;
+// At most two other batches are in flight; more of them come from several threads.
+constexpr int kFewOthers = 2;
 bool few_in_flight(const bnk_batch *b) {
-    return b->ctx->launch_graphs && b->ctx->in_flight.load(std::memory_order_relaxed) - (b->counted ? 1 : 0) <= kGraphOthers;
+    return b->ctx->in_flight.load(std::memory_order_relaxed) - (b->counted ? 1 : 0) <= kFewOthers;
 }
+// Launches what a submit has gathered (launch.h), through a graph while few batches are in flight.
+bool through_graph(const bnk_batch *b) { return b->ctx->launch_graphs && few_in_flight(b); }
 cudaError_t send_launches(bnk_batch *b, Launches &all) {
     launch_graph_give(b->graph); // (of a submit that nobody waited for)
     b->graph = nullptr;
@@ -997,7 +998,7 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     const bnk_batch_view &h = b->host;
     const DeviceBatch &d = b->dev;
     CK(ctx, order_kernels_begin(b));
-    Launches all(s, !timed && !stats && few_in_flight(b));
+    Launches all(s, !timed && !stats && through_graph(b));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, false, nullptr);
     a.over_link = true;
@@ -1198,10 +1199,13 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     b->stale_pkts = std::max(b->stale_pkts, npkts);
     const bool one_launch = npkts <= kGroupMax || !replay; // behind the open kernel
     CK(ctx, order_kernels_begin(b));
-    Launches all(s, !timed && !stats && one_launch && few_in_flight(b));
+    Launches all(s, !timed && !stats && one_launch && through_graph(b));
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, true, nullptr);
     a.over_link = a.from_host = true;
+    // With many batches in flight the link is the bound, and the headers' own requests take a share of it: 128 x 1420 B sealed and
+    // opened, threads x batches, Gbit/s with the headers first / without: 8 x 2 177 / 181, 8 x 4 191 / 201, 16 x 4 200 / 214.
+    a.header_first = few_in_flight(b);
     a.host = HostDesc{h.off, h.len, h.slot};
     a.link_bytes = bytes;
     a.in = a.out = h.ring;
@@ -1439,7 +1443,7 @@ int bnk_filter_note_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t
         bool sweep;
         CK(ctx, flow_note_begins(b, npkts, now_unix_ns, s, sweep));
         const Done done = watch_for(b);
-        Launches all(s, !timed && !sweep && few_in_flight(b));
+        Launches all(s, !timed && !sweep && through_graph(b));
         CK(ctx, launch_filter_note(b, 0, npkts, now_unix_ns, sweep ? Done{} : done, s));
         CK(ctx, send_launches(b, all));
         if (sweep) CK(ctx, launch_flow_sweep(b, now_unix_ns, done, s));
@@ -1469,7 +1473,7 @@ int bnk_filter_check_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_
     const Done done = to_host && npkts && !(flags & BNK_F_STATS) ? watch_for(b) : Done{};
     uint8_t *const host_status = to_host ? b->host.status : nullptr;
     if (direct) b->dev.status = alias.saved.status; // the kernel writes to both
-    Launches all(s, !timed && few_in_flight(b));
+    Launches all(s, !timed && through_graph(b));
     CK(ctx, launch_filter_check(b, npkts, now_unix_ns, false, host_status, done, s));
     CK(ctx, send_launches(b, all));
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
@@ -1497,7 +1501,7 @@ int bnk_classify_submit(bnk_batch *b, uint32_t npkts, uint32_t flags) {
     HostAlias alias(b, direct, npkts);
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     const Done done = direct && !(flags & BNK_F_STATS) ? watch_for(b) : Done{};
-    Launches all(s, !timed && few_in_flight(b));
+    Launches all(s, !timed && through_graph(b));
     CK(ctx, launch_classify(b, npkts, done, s));
     CK(ctx, send_launches(b, all));
     if (timed) CK(ctx, cudaEventRecord(b->k_end, s));
@@ -1543,7 +1547,7 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
             b->split_sealed = 0;
             b->partial_to = std::max({b->partial_to, ring_extent(b, n_pkts, kMostRoom), to});
             memcpy(b->h_gso, supers, (size_t)n_super * sizeof(bnk_gso_super));
-            Launches all(s, in_place && !timed && few_in_flight(b));
+            Launches all(s, in_place && !timed && through_graph(b));
             if (!in_place) { // the rest beside the copy
                 CK(ctx, cudaEventRecord(b->ev_fork, s));
                 CK(ctx, cudaStreamWaitEvent(b->aux_stream, b->ev_fork, 0));

@@ -329,6 +329,7 @@ struct AeadArgs {
     bool behind_kernel;           // a kernel of the same submit is in front
     bool over_link;               // a ring is in host memory
     bool from_host;               // the ring that is read and the descriptors are
+    bool header_first;            // open of up to kRankMax packets with from_host: their headers are asked for ahead of them
     HostDesc host;                // with from_host
     uint64_t link_bytes;          // with over_link: bytes of the packets
     uint32_t n;
