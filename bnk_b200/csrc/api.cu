@@ -1519,7 +1519,10 @@ constexpr uint32_t kPlainRuns = 16; // copies of plain packets between a split's
 // split and sealed (two calls) 61.8 -> 47.4 us, 460 of 950 B 69.8 -> 57.3.  SMs read 48 GB/s over the link, the copy engine 55:
 // 2400 of 1380 B (3.3 MB) 194.7 in place and 188.9 with a copy in front, 12,032 (17 MB) 768 and 733.  (In pieces, each split
 // while the next comes up, 763: every piece costs the engine more than the split of all takes.)
-constexpr uint64_t kSplitInPlace = 5ull << 19;
+// That kernel also brings up the packets that are no segments.  Up to kSplitWithPlain bytes with those it is ahead of their upload:
+// two segments and 800 of 1420 B split 39 us and 53, 2500 (3.7 MB) 96 and 101, 5000 (7.3 MB) 170 and 168, 50,000 1506 and 1430;
+// 40,000 of 64 B (4.5 MB, with 48 for each) 142 and 170.
+constexpr uint64_t kSplitInPlace = 5ull << 19, kSplitWithPlain = 2 * kSplitInPlace;
 int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_super, uint32_t n_pkts,
                          uint32_t flags) {
     int rc = begin_submit(b, n_pkts, true); // the descriptor staging area is host memory in any case
@@ -1531,21 +1534,25 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
     if (n_super > b->max_pkts || (n_super && !supers)) return fail(ctx, BNK_EINVAL, "bad super-packet list");
     const size_t n = n_pkts;
     const bool refresh = b->stale_pkts != 0;
+    uint64_t ext = 0; // where the packets end, once they have been looked through
     CK(ctx, catch_up(b, s));
     if (!(flags & BNK_F_NO_H2D) && !refresh && gso_split_fits(supers, n_super, n_pkts, b->ring_bytes)) {
-        uint64_t from = ~0ull, to = 0, sum = 0, segs = 0;
+        uint64_t from = ~0ull, to = 0, sum = 0, segs = 0, of_segs = 0, of_all; // (bytes of segments and of all packets, with their room)
         for (uint32_t j = 0; j < n_super; j++) {
             from = std::min<uint64_t>(from, supers[j].src_off);
             to = std::max(to, (uint64_t)supers[j].src_off + supers[j].src_len);
             sum += supers[j].src_len;
             segs += supers[j].n_pkts;
+            of_segs += supers[j].src_len - supers[j].hdr_len + supers[j].n_pkts * (uint64_t)(supers[j].hdr_len + kMostRoom);
         }
         from &= ~63ull;
         to = std::min<uint64_t>((to + 15) & ~15ull, b->ring_bytes);
-        const bool in_place = sum <= kSplitInPlace && host_direct(b, n_pkts, 0, sum);
+        ext = ring_extent(b, n_pkts, kMostRoom, &of_all);
+        const uint64_t over_link = sum + (segs < n_pkts && of_all > of_segs ? of_all - of_segs : 0);
+        const bool in_place = sum <= kSplitInPlace && over_link <= kSplitWithPlain && host_direct(b, n_pkts, 0, over_link);
         if (in_place || (sum > kSplitInPlace && ctx->host_direct_bytes && segs == n_pkts && to - from <= 2 * sum + 65536)) {
             b->split_sealed = 0;
-            b->partial_to = std::max({b->partial_to, ring_extent(b, n_pkts, kMostRoom), to});
+            b->partial_to = std::max({b->partial_to, ext, to});
             memcpy(b->h_gso, supers, (size_t)n_super * sizeof(bnk_gso_super));
             Launches all(s, in_place && !timed && through_graph(b));
             if (!in_place) { // the rest beside the copy
@@ -1573,7 +1580,8 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
         // they lie close together, and the packets that are no super-packet's segments, each run of them in a copy of its
         // own.  (The whole ring goes up for a batch that is cut into many runs, whose plain packets are spread over most of
         // the ring, or whose super-packets are not in batch order.)
-        uint64_t ext = ring_extent(b, n_pkts, 16 + 16 + 16), from = ~0ull, to = 0, sum = 0;
+        uint64_t from = ~0ull, to = 0, sum = 0;
+        if (ext == 0) ext = ring_extent(b, n_pkts, kMostRoom);
         struct {
             uint64_t at, to;
         } run[kPlainRuns];

@@ -427,3 +427,38 @@ def test_split_where_the_super_packets_lie_in_the_host_ring(gpu_lib, oracle, lay
                 assert b.ring[off[i] + 16:off[i] + 16 + len(want[i])].tobytes() == want[i], (flags, i)
             assert (b.slot == 1).all()
         b.close()
+
+
+@pytest.mark.parametrize("plain,launches", [(40, 2), (3560, 2), (3580, 3)])  # on both sides of 5 MB
+def test_split_of_a_small_super_packet_among_many_plain_packets(gpu_lib, oracle, plain, launches):
+    """Packets that are no segments count when it is decided whether the kernel that splits reads the host ring itself (two
+    launches) or what it needs goes up by copy (three); the device holds the same packets either way."""
+    from bnk_b200 import Context
+    from bnk_b200.device import GSO_SUPER_DTYPE
+
+    rng = np.random.default_rng(plain)
+    pkt, cs, hdr = _tcp_super(rng, 2000)
+    want = oracle.gso_split(pkt, hdr, 1380, cs, 16, 6)
+    n, stride, size = plain + len(want), 1472, 1420
+    off = H.layout_fixed(n, stride)
+    sup = np.zeros(1, GSO_SUPER_DTYPE)
+    sup["src_off"], sup["src_len"], sup["n_pkts"], sup["hdr_len"], sup["gso_size"] = n * stride, len(pkt), len(want), hdr, 1380
+    sup["csum_start"], sup["csum_offset"], sup["proto"] = cs, 16, 6
+    with Context(max_keypairs=1, mtu=0, flow_capacity=0) as c:
+        b = c.batch(n, n * stride + 4096)
+        b.ring[:] = 0x11
+        b.off[:], b.len[:], b.slot[:] = off, size, 0
+        b.len[:len(want)] = [len(w) for w in want]
+        b.upload(n)
+        held = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
+        held[n * stride:n * stride + len(pkt)] = np.frombuffer(pkt, np.uint8)
+        b.ring[:] = held
+        before = c.launch_count()
+        b.gso_split(sup, n)
+        assert c.launch_count() - before == launches
+        b.ring[:] = 0x77
+        b.download(n)
+        for i, w in enumerate(want):
+            assert b.ring[off[i] + 16:off[i] + 16 + len(w)].tobytes() == w
+        assert H.spans_equal(np.array(b.ring), held, off[len(want):], [size] * plain, 16) == []
+        b.close()
