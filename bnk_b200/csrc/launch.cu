@@ -3,9 +3,9 @@
 
 #include <string.h>
 
+#include <atomic>
 #include <mutex>
 #include <new>
-#include <vector>
 
 namespace {
 
@@ -54,36 +54,35 @@ namespace {
 
 // The graphs of one device, used by all its contexts.  A graph belongs to one submit at a time, from its launch until that
 // has been waited for.  One is made (50 us, 250 for two kernels, 100 KB) when its kernels are asked for the fourth time and
-// none is free, so that a program that calls once or twice does not pay for it.
+// none is free, so that a program that calls once or twice does not pay for it.  What is kept here is kept in place: a submit
+// of a process without memory to spare goes launch by launch.
 class GraphPool {
   public:
     LaunchGraph *take(const LaunchGraph &want) {
         std::lock_guard<std::mutex> g(mu_);
-        for (LaunchGraph *e : made_)
-            if (!e->taken && e->is(want)) {
-                e->taken = true;
-                return e;
+        for (uint32_t i = 0; i < made_n_; i++)
+            if (!made_[i]->taken && made_[i]->is(want)) {
+                made_[i]->taken = true;
+                return made_[i];
             }
-        if (made_.size() + making_ >= kMost) return nullptr;
-        for (Asked &a : asked_)
-            if (a.what.is(want)) {
-                if (++a.times < kFrom) return nullptr;
-                making_++;
-                return &make_;
-            }
-        if (asked_.size() < 4 * kMost) asked_.push_back({want, 1});
+        if (made_n_ + making_ >= kMost) return nullptr;
+        if (Asked *a = asked(want)) {
+            if (++a->times < kFrom) return nullptr;
+            making_++;
+            return &make_;
+        }
+        if (asked_n_ < kMostAsked) asked_[asked_n_++] = {want, 1};
         return nullptr;
     }
     static bool to_be_made(const LaunchGraph *g) { return g == &make_; }
     void made(LaunchGraph *g) { // null: it could not be
         std::lock_guard<std::mutex> l(mu_);
         making_--;
-        if (g) made_.push_back(g);
+        if (g) made_[made_n_++] = g;
     }
     void failed(const LaunchGraph &want) { // not again
         std::lock_guard<std::mutex> l(mu_);
-        for (Asked &a : asked_)
-            if (a.what.is(want)) a.times = INT32_MIN;
+        if (Asked *a = asked(want)) a->times = INT32_MIN;
     }
     void give(LaunchGraph *g) {
         std::lock_guard<std::mutex> l(mu_);
@@ -93,43 +92,50 @@ class GraphPool {
         std::lock_guard<std::mutex> l(mu_);
         contexts_ += comes ? 1 : -1;
         if (contexts_ > 0) return;
-        for (LaunchGraph *e : made_) {
-            cudaGraphExecDestroy(e->exec);
-            cudaGraphDestroy(e->graph);
-            delete e;
+        for (uint32_t i = 0; i < made_n_; i++) {
+            cudaGraphExecDestroy(made_[i]->exec);
+            cudaGraphDestroy(made_[i]->graph);
+            delete made_[i];
         }
-        made_.clear();
-        asked_.clear();
+        made_n_ = asked_n_ = 0;
     }
 
   private:
-    static constexpr size_t kMost = 48;
+    static constexpr uint32_t kMost = 48, kMostAsked = 4 * kMost;
     static constexpr int32_t kFrom = 4;
     struct Asked {
         LaunchGraph what;
         int32_t times;
     };
+    Asked *asked(const LaunchGraph &want) {
+        for (uint32_t i = 0; i < asked_n_; i++)
+            if (asked_[i].what.is(want)) return &asked_[i];
+        return nullptr;
+    }
     static LaunchGraph make_; // "there is room for one more"
     std::mutex mu_;
-    std::vector<LaunchGraph *> made_;
-    std::vector<Asked> asked_;
-    size_t making_ = 0;
+    LaunchGraph *made_[kMost];
+    Asked asked_[kMostAsked];
+    uint32_t made_n_ = 0, asked_n_ = 0, making_ = 0;
     int contexts_ = 0;
 };
 LaunchGraph GraphPool::make_{};
+// Made with a device's first context and never destroyed (the driver may be gone before); null if there was no memory for it.
 constexpr int kDevices = 64;
-GraphPool *pools() {
-    static GraphPool *const all = new GraphPool[kDevices]; // (never destroyed: the driver may be gone before)
-    return all;
-}
+std::atomic<GraphPool *> pools[kDevices];
+GraphPool *pool_of(int device) { return device >= 0 && device < kDevices ? pools[device].load(std::memory_order_acquire) : nullptr; }
 
 } // namespace
 
 void launch_graphs_context(int device, bool comes) {
-    if (device >= 0 && device < kDevices) pools()[device].context(comes);
+    if (comes && device >= 0 && device < kDevices && !pool_of(device)) {
+        GraphPool *none = nullptr, *const made = new (std::nothrow) GraphPool;
+        if (!pools[device].compare_exchange_strong(none, made)) delete made;
+    }
+    if (GraphPool *const p = pool_of(device)) p->context(comes);
 }
 void launch_graph_give(LaunchGraph *g) {
-    if (g) pools()[g->device].give(g);
+    if (g) pool_of(g->device)->give(g);
 }
 
 Launches::Launches(cudaStream_t s, bool gather) : s_(s), gathering_(gather), outer_(t_gathering) { t_gathering = this; }
@@ -172,8 +178,9 @@ static cudaKernelNodeParams node_params(const LaunchShape &k, void **args) {
 // A graph of the n gathered launches' kernels, made if need be.
 LaunchGraph *Launches::graph(uint32_t n) {
     int device = 0;
-    if (n == 0 || cudaGetDevice(&device) != cudaSuccess || device >= kDevices) return nullptr;
-    GraphPool &pool = pools()[device];
+    GraphPool *const p = n != 0 && cudaGetDevice(&device) == cudaSuccess ? pool_of(device) : nullptr;
+    if (!p) return nullptr;
+    GraphPool &pool = *p;
     LaunchGraph want{};
     want.n = n;
     for (uint32_t i = 0; i < n; i++) {
