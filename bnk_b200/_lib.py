@@ -206,6 +206,7 @@ SYMBOLS = {
     "bnk_batch_last_kernel_ms": (_i, [_vp, C.POINTER(C.c_float)]),
     "bnk_batch_last_aead_ms": (_i, [_vp, C.POINTER(C.c_float)]),
     "bnk_kernel_launch_count": (_i, [_vp, C.POINTER(_u64)]),
+    "bnk_graph_launch_count": (_i, [_vp, C.POINTER(_u64)]),
 }
 # include/bnk_gpu_bench.h, exported by libbnkgpu_bench.so
 BENCH_SYMBOLS = {

@@ -135,7 +135,9 @@ bool through_graph(const bnk_batch *b) { return b->ctx->launch_graphs && few_in_
 cudaError_t send_launches(bnk_batch *b, Launches &all) {
     launch_graph_give(b->graph); // (of a submit that nobody waited for)
     b->graph = nullptr;
-    return all.send(b->graph);
+    const cudaError_t e = all.send(b->graph);
+    if (b->graph) b->ctx->graph_launches.fetch_add(1, std::memory_order_relaxed);
+    return e;
 }
 // For the kernel that is the submit's last piece of work: bnk_wait will watch for it.
 Done watch_for(bnk_batch *b) {
@@ -408,7 +410,7 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     ctx->cfg = *cfg;
     ctx->device = cfg->device_id;
     ctx->sm_count = sms;
-    ctx->launches = 0;
+    ctx->launches = ctx->graph_launches = 0;
     ctx->aead_mode = 0;
     if (const char *m = getenv("BNK_AEAD_KERNEL")) // tuning and test aid: tpp | wpp
         ctx->aead_mode = !strcmp(m, "tpp") ? 1 : (!strcmp(m, "wpp") ? 2 : 0);
@@ -1716,6 +1718,12 @@ int bnk_batch_last_aead_ms(bnk_batch *b, float *ms) {
 int bnk_kernel_launch_count(bnk_ctx *ctx, uint64_t *count) {
     if (!ctx || !count) return BNK_EINVAL;
     *count = ctx->launches.load();
+    return BNK_SUCCESS;
+}
+
+int bnk_graph_launch_count(bnk_ctx *ctx, uint64_t *count) {
+    if (!ctx || !count) return BNK_EINVAL;
+    *count = ctx->graph_launches.load();
     return BNK_SUCCESS;
 }
 

@@ -114,7 +114,7 @@ struct bnk_ctx {
     uint32_t aead_side_stream_from; // batches of at least this many packets run seal/open on the low-priority stream (BNK_AEAD_SIDE_STREAM_FROM; 0 = never)
     uint64_t pieces_from;           // ring extent from which a batch that is alone goes over the link in pieces (BNK_PIECES_FROM)
     int prio_low, prio_high;        // stream priority range of the device
-    std::atomic<uint64_t> launches;
+    std::atomic<uint64_t> launches, graph_launches;
     std::atomic<uint64_t> seal_seq{0}; // number of the last seal launch that handed out nonces itself (see SendCounter)
     std::mutex mu;
     std::string last_error;

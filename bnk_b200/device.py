@@ -190,6 +190,11 @@ class Context:
         self._ck(_lib.lib().bnk_kernel_launch_count(self._h, C.byref(v)))
         return v.value
 
+    def graph_launch_count(self) -> int:
+        v = C.c_uint64()
+        self._ck(_lib.lib().bnk_graph_launch_count(self._h, C.byref(v)))
+        return v.value
+
     def probe_int_throughput(self, mix: int) -> float:
         v = C.c_double()
         self._ck(_lib.bench_lib().bnk_probe_int_throughput(self._h, mix, C.byref(v)))

@@ -473,6 +473,8 @@ int bnk_batch_last_kernel_ms(bnk_batch *b, float *ms);
 int bnk_batch_last_aead_ms(bnk_batch *b, float *ms);
 /* Number of kernels this library has launched on the context since creation. */
 int bnk_kernel_launch_count(bnk_ctx *ctx, uint64_t *count);
+/* Number of submits on the context whose kernels went out together, through an executable graph. */
+int bnk_graph_launch_count(bnk_ctx *ctx, uint64_t *count);
 
 #ifdef __cplusplus
 }

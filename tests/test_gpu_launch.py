@@ -90,6 +90,7 @@ def test_same_results_launch_by_launch_and_through_graphs(gpu_lib, sizes):
     for graphs in (0, 1, 1):  # the third context finds the second one's graphs gone
         with _context(graphs, max_keypairs=8, mtu=1420, flow_capacity=1 << 14) as c:
             results.append(_passes(c, sizes, len(sizes)))
+            assert (c.graph_launch_count() > 0) == bool(graphs)
     for other in results[1:]:
         for x, y in zip(results[0], other):
             assert np.array_equal(x, y)
