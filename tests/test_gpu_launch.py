@@ -97,53 +97,47 @@ def test_same_results_launch_by_launch_and_through_graphs(gpu_lib, sizes):
 
 
 def test_batches_in_flight_and_contexts_beside_each_other(gpu_lib, oracle):
-    """Graphs are shared by the contexts of a device: two contexts with up to four submits each in flight, one context closed
-    on the way, every message the checker's."""
-    from bnk_b200.device import F_ASSIGN_COUNTERS
-
+    """Graphs are shared by the contexts of a device: two contexts with up to four submits each in flight at once, sealed and
+    opened, one context closed while the other's are in flight, every message and plaintext the checker's."""
     rng = np.random.default_rng(4)
-    keys = rng.integers(0, 256, (1, 32), dtype=np.uint8)
-    n = 40
-    off = H.layout_fixed(n, 256)
-    lens = rng.integers(0, 200, n).astype(np.uint32)
-    made = [_context(1, max_keypairs=1, flow_capacity=0) for _ in range(2)]
-    counter = [0, 0]
+    peers, n = 3, 40
+    keys = [rng.integers(0, 256, (peers, 32), dtype=np.uint8) for _ in range(2)]
+    off, slot = H.layout_fixed(n, 256), rng.integers(0, peers, n).astype(np.uint32)
+    ridx = np.arange(peers, dtype=np.uint32) + 5
+    made = [_context(1, max_keypairs=peers, flow_capacity=0) for _ in range(2)]
     batches = []
-    for c in made:
-        c.set_keypairs(0, keys, keys, np.array([5], np.uint32))
+    for c, k in zip(made, keys):
+        c.set_keypairs(0, k, k, ridx)
         batches.append([c.batch(n, n * 256) for _ in range(4)])
     for r in range(24):
-        at_once = 1 + r % 4
-        if r == 16:
-            for b in batches.pop():
-                b.close()
-            made.pop().close()
+        use = [(k, b) for k in range(len(made)) for b in batches[k][:1 + r % 4]]
         want = []
-        for k in range(len(made)):
-            for b in batches[k][:at_once]:
-                b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
-                b.off[:], b.len[:], b.slot[:] = off, lens, 0
-                ctr = np.arange(counter[k], counter[k] + n, dtype=np.uint64)
-                counter[k] += n
-                want.append((b, H.oracle_seal(oracle, keys, np.array([5]), 1420, b.ring, off, lens, np.zeros(n), ctr)))
-        for k in range(len(made)):
-            for b in batches[k][:at_once]:
-                b.seal(n, F_ASSIGN_COUNTERS, wait=False)
-                b.wait()  # (nonces are handed out in this order)
-        for b, (ring, st, ln) in want:
+        for k, b in use:
+            b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
+            b.off[:], b.len[:], b.slot[:] = off, rng.integers(0, 200, n), slot
+            b.counter[:] = rng.integers(0, 2**60, n, dtype=np.uint64)
+            want.append((np.array(b.ring), *H.oracle_seal(oracle, keys[k], ridx, 1420, b.ring, off, b.len, slot, b.counter)))
+        for k, b in use:
+            b.seal(n, wait=False)
+        for (k, b), (plain, ring, st, ln) in zip(use, want):
+            b.wait()
             assert np.array_equal(b.status, st) and np.array_equal(b.out_len, ln)
             assert H.spans_equal(np.array(b.ring), ring, off, ln) == []
-    # and without a wait in between, which takes the nonces in submit order as well: all on one context, stream by stream
-    for r in range(8):
-        for b in batches[0]:
-            b.off[:], b.len[:], b.slot[:], b.counter[:] = off, lens, 0, np.arange(n) + 1000 * r
-        plain = [np.array(b.ring) for b in batches[0]]
-        for b in batches[0]:
-            b.seal(n, wait=False)
-        for b, p in zip(batches[0], plain):
-            b.wait()
-            ring, st, ln = H.oracle_seal(oracle, keys, np.array([5]), 1420, p, off, lens, np.zeros(n), np.arange(n) + 1000 * r)
-            assert np.array_equal(b.out_len, ln) and H.spans_equal(np.array(b.ring), ring, off, ln) == []
+            b.len[:] = ln
+        for k, b in use:
+            b.open(n, wait=False)
+        for i, ((k, b), (plain, ring, st, ln)) in reversed(list(enumerate(zip(use, want)))):
+            b.wait()  # the second context's first
+            ring, st, ctr, out = H.oracle_open(oracle, keys[k], ring, off, ln, slot)
+            assert np.array_equal(b.status, st) and np.array_equal(b.counter, ctr) and np.array_equal(b.out_len, out)
+            assert H.spans_equal(np.array(b.ring), ring, off, out, 16) == []
+            if r == 15 and i == 4:  # four of the first context are in flight
+                for x in batches.pop():
+                    x.close()
+                gone = made.pop()
+                assert gone.graph_launch_count() > 20
+                gone.close()
+    assert made[0].graph_launch_count() > 50
     for b in batches[0]:
         b.close()
     made[0].close()
