@@ -191,9 +191,36 @@ bool host_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, uint64_t ext) {
 // the link takes ~2.6 ns per request, fewer where packets share lines, and a copy costs 6-8 us before it moves anything.
 // Headers 48 bytes apart checked, copied first / in place: 2000 28.8 us / 17.0, 16,000 40.8 / 32, 80,000 121 / 108, 800,000 908 /
 // 896; packets of 64 B noted and checked, 2000 76 / 36, 16,000 132 / 85; datagrams of 28 B classified, 5000 59 / 23, 50,000 178 /
-// 117.  (With a lane asking for both halves of a head, copying was ahead below 128 bytes a packet from 1024 packets on.)
+// 117.  With other batches in flight as well, Mpackets/s copied / in place, threads x headers 48 bytes apart: 4 x 2000 159 / 344, 8 x
+// 16,000 590 / 772, 8 x 200,000 808 / 913, 8 x 500,000 814 / 931, but 2 x 1,000,000 942 / 916.  (With a lane asking for both halves
+// of a head, copying was ahead below 128 bytes a packet from 1024 packets on.)
+// A program that goes on with such packets on the device (BNK_F_NO_H2D) then waits for their copy after all.  From the second time
+// on they go up in front of the look at their heads: 2000 x 64 B checked and then sealed 68 us with the copy behind, 53 in front,
+// 16,000 163 and 153, 300,000 2267 and 1922.
+constexpr uint64_t kDense = 128;
 constexpr uint32_t kHeadsFirst = 16384, kHeadsMost = 131072, kHeadSlack = 16; // see upload_heads
-bool heads_direct(bnk_batch *b, uint32_t npkts, uint32_t flags) { return host_direct(b, npkts, flags, 0); }
+constexpr uint32_t kDenseFrom = 1024;
+bool heads_are_dense(const bnk_batch *b, uint32_t npkts) {
+    if (npkts <= kDenseFrom) return false;
+    const auto end = [&](uint32_t i) { return (uint64_t)b->host.off[i] + b->host.len[i]; };
+    if (!b->heads_go_up) return end(npkts - 1) < kDense * npkts; // (a guess will do, and a look at more is a microsecond)
+    // Some seventy packets of a batch in any order come within an eighth of the extent; only if they leave a doubt are all of the
+    // descriptors looked through.
+    uint64_t seen = end(npkts - 1);
+    for (uint32_t i = 0; i < npkts; i += npkts / 64) seen = std::max(seen, end(i));
+    return seen * 8 < kDense * npkts * 7 || ring_extent(b, npkts, kHeadSlack) < kDense * npkts;
+}
+// By every submit, with its flags, in front of anything else.
+void behind_heads(bnk_batch *b, uint32_t flags) {
+    if (b->heads == Heads::in_place && (flags & BNK_F_NO_H2D)) b->heads_go_up = true;
+    if (b->heads == Heads::copied && !(flags & BNK_F_NO_H2D)) b->heads_go_up = false;
+    b->heads = Heads::none;
+}
+bool heads_direct(bnk_batch *b, uint32_t npkts, uint32_t flags) {
+    const bool dense = heads_are_dense(b, npkts), direct = !(dense && b->heads_go_up) && host_direct(b, npkts, flags, 0);
+    if (dense) b->heads = direct ? Heads::in_place : Heads::copied;
+    return direct;
+}
 // Below ctx->pieces_from (24 MB) a kernel on the pinned ring is as fast or faster, because the first piece up and the last
 // one down have no company: 16,384 x 1420 B 710 us against 750, 32,768 1390 against 1330, 131,072 5.74 ms against 4.96.
 // With small packets that kernel is bound by what its warps compute, ~7.5 ns a packet, and pieces win earlier: 8192 x
@@ -1110,6 +1137,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     if (rc) return rc;
     if (flags & BNK_F_NOTE_OUTBOUND) CK(b->ctx, filter_flows_maintain(b, b->stream));
     SubmitScope scope(b);
+    behind_heads(b, flags);
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
@@ -1321,6 +1349,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     int rc = begin_submit(b, npkts, !device_only);
     if (rc) return rc;
     SubmitScope scope(b);
+    behind_heads(b, flags);
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
@@ -1409,7 +1438,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
 static int upload_heads(bnk_batch *b, uint32_t n, bool results_down, cudaStream_t s) {
     bnk_ctx *ctx = b->ctx;
     if (!results_down) CK(ctx, catch_up(b, s)); // (see catch_up_beside)
-    CK(ctx, desc_copy(b, n, D_OFF, D_LEN, true, s));
+    CK(ctx, desc_copy(b, n, D_OFF, b->heads_go_up && results_down ? D_STATUS : D_LEN, true, s)); // (all that a catch-up would bring)
     uint64_t up = 0, ext = 0;
     for (uint32_t at = 0, k = kHeadsFirst; at < n; at += k, k = std::min(2 * k, kHeadsMost)) {
         k = std::min(k, n - at);
@@ -1430,6 +1459,7 @@ int bnk_filter_note_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t
     if (rc) return rc;
     CK(b->ctx, filter_flows_maintain(b, b->stream));
     SubmitScope scope(b);
+    behind_heads(b, flags);
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
@@ -1461,6 +1491,7 @@ int bnk_filter_check_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_
     int rc = begin_submit(b, npkts);
     if (rc) return rc;
     SubmitScope scope(b);
+    behind_heads(b, flags);
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
@@ -1488,6 +1519,7 @@ int bnk_classify_submit(bnk_batch *b, uint32_t npkts, uint32_t flags) {
     int rc = begin_submit(b, npkts);
     if (rc) return rc;
     SubmitScope scope(b);
+    behind_heads(b, flags);
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
@@ -1530,6 +1562,7 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
     int rc = begin_submit(b, n_pkts, true); // the descriptor staging area is host memory in any case
     if (rc) return rc;
     SubmitScope scope(b);
+    behind_heads(b, flags);
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;

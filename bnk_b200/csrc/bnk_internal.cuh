@@ -170,6 +170,7 @@ struct DeviceBatch {
     bnk_gso_super *gso;   // [max_pkts] super-packet descriptors of a GSO split
 };
 
+enum class Heads : uint8_t { none, in_place, copied }; // a submit that looks at the heads of many packets that lie close together
 struct bnk_batch {
     bnk_ctx *ctx;
     uint32_t max_pkts;
@@ -193,6 +194,8 @@ struct bnk_batch {
     // Submits ran on the host arrays: the device copies of the first `stale_pkts` packets and descriptors (of the first
     // `stale_src` source addresses) are behind.
     uint32_t stale_pkts, stale_src;
+    Heads heads;           // what the last submit was, and ...
+    bool heads_go_up;      // ... whether such submits leave the packets on the device (see heads_direct)
     uint64_t partial_to;   // below this place of the device ring only packets and super-packets are those of the host ring
     uint32_t split_sealed; // with partial_to: that many packets have been sealed since the split
     bool counted;        // this batch is one of ctx->in_flight

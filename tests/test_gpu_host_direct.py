@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from tests import helpers as H
+from tests import reference_cases as RC
 
 pytestmark = pytest.mark.gpu
 
@@ -244,3 +245,51 @@ def test_device_only_submits_need_no_wait(gpu_lib, oracle, n, size):
         assert sum(c.send_counter(p) for p in range(2)) == 2 * n
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("stride", [96, 512])  # packets that lie close together, and not
+@pytest.mark.parametrize("look", ["note", "check", "classify"])
+def test_heads_looked_at_and_then_sealed_on_the_device(gpu_lib, oracle, look, stride):
+    """A look at the packets' heads, then a seal that takes the packets from the device: where the heads are read in place the
+    packets go up behind the look, and from the second time on in front of it.  Every round has other packets, keypairs and
+    nonces; some have the seal take the packets from the host."""
+    from bnk_b200 import Context
+    from bnk_b200.device import F_NO_H2D
+    from bnk_b200.filter import CompiledRule, PortRange, flatten_rules
+
+    rng = np.random.default_rng(stride)
+    n, peers, size = 1500, 4, 60
+    keys = rng.integers(0, 256, (peers, 32), dtype=np.uint8)
+    off = H.layout_fixed(n, stride)
+    with Context(max_keypairs=peers, mtu=0, flow_capacity=1 << 14) as c:
+        c.set_keypairs(0, keys, keys, np.arange(peers, dtype=np.uint32))
+        c.acl_set(True, flatten_rules([CompiledRule(srcs=["100.64.0.0/16"], proto="udp", ports=[PortRange(1, 30000)])]))
+        b = c.batch(n, n * stride)
+        f = oracle.Filter()
+        f.set_rules([([(RC.ip("100.64.0.0"), 16)], "udp", [(1, 30000)])])
+        for r, on_device in enumerate([True, True, True, False, True, False, False, True]):
+            now = RC.T0 + r * RC.SEC
+            b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
+            packets = [RC.udp(RC.ip("100.64.0.0") + int(rng.integers(0, 1 << 17)), RC.SELF, int(rng.integers(1, 9)), int(rng.integers(1, 60000)))[:28]
+                       for _ in range(n)]
+            for o, p in zip(off, packets):
+                b.ring[o + 16:o + 44] = np.frombuffer(p, np.uint8)
+            b.off[:], b.len[:], b.slot[:] = off, size, rng.integers(0, peers, n)
+            b.counter[:] = rng.integers(0, 2**60, n, dtype=np.uint64)
+            if look == "note":
+                b.filter_note(n, now)
+                for p in packets:
+                    f.note_outbound(p, now)
+                assert H.flows_equal(c.flows_export(), f.flows())
+            elif look == "check":
+                b.filter_check(n, now)
+                assert np.array_equal(b.status == 0, [f.check_inbound(p, now) for p in packets])
+            else:
+                slots = np.array(b.slot)
+                b.classify(n)
+                b.slot[:] = slots  # (an output of the call for known peers, of whom there are none)
+            ring, st, ln = H.oracle_seal(oracle, keys, np.arange(peers), 0, b.ring, off, b.len, b.slot, b.counter)
+            b.seal(n, F_NO_H2D if on_device else 0)
+            assert np.array_equal(b.status, st) and np.array_equal(b.out_len, ln)
+            assert H.spans_differ_count(np.array(b.ring), ring, off, ln) == 0, r
+        b.close()
