@@ -6,10 +6,11 @@
 
 #include <stdint.h>
 
-// How often a wait looks before it gives up.  (A build for tests has it give up soon, and BNK_BULK_LOST set: copies of that many
-// bytes are never asked for, which is what a link that has stopped looks like from here.)
+// How often a wait looks before it gives up.  A look that finds nothing takes 4 us, in which the warp sleeps, so that is half a
+// second.  (A build for tests has it give up soon, and BNK_BULK_LOST set: copies of that many bytes are never asked for, which is
+// what a link that has stopped looks like from here.)
 #ifndef BNK_BULK_TURNS
-#define BNK_BULK_TURNS (1u << 22)
+#define BNK_BULK_TURNS (1u << 17)
 #endif
 __device__ __forceinline__ uint32_t shared_at(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void bar_init(uint64_t *bar) {
@@ -18,7 +19,7 @@ __device__ __forceinline__ void bar_init(uint64_t *bar) {
 __device__ __forceinline__ void bar_expect(uint64_t *bar, uint32_t bytes) { // the phase ends when that many have come
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_at(bar)), "r"(bytes) : "memory");
 }
-// False: it has not come after so many turns (80 ms at the least), which no link that works takes.
+// False: it has not come after so many turns, which no link that works takes.
 __device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
     for (uint32_t turn = 0; turn < BNK_BULK_TURNS; turn++) {
         uint32_t over;

@@ -71,7 +71,7 @@ extern "C" {
 #define BNK_PKT_BAD_INNER 9         /* BNK_F_INNER_CHECK: decrypted packet is not IPv4, lies about its length,
                                        or does not come from the peer's allowed address */
 #define BNK_PKT_NOT_READ 13         /* a fault of the host link, not of the packet: its bytes did not come within the time a
-                                       kernel waits for them (tenths of a second), or did not for a packet that the same
+                                       kernel waits for them (half a second), or did not for a packet that the same
                                        warp was to work on first.  out_len is 0.  The ring holds what it held, but for
                                        packets beyond 1984 bytes: of those the stretches in front are sealed already, or
                                        zeros where they were opened.  A nonce handed out to the packet stays unused. */

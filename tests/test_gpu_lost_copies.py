@@ -148,3 +148,28 @@ def test_seal_and_open_refuse_what_did_not_come(lossy, oracle, n, lost, long):
         b.seal(n)
         assert np.array_equal(b.status, st) and H.spans_equal(np.array(b.ring), ring, off, ln) == []
         b.close()
+
+
+def test_a_wait_gives_up_after_a_time_that_callers_can_bear(lossy):
+    """From the time that this build's waits take, that of the product's: between a tenth of a second, far above what a busy link
+    keeps a packet waiting, and two seconds."""
+    import re
+
+    from bnk_b200 import Context, _build
+    from bnk_b200.device import F_TIMED, PKT_NOT_READ
+
+    text = open(os.path.join(_build.CSRC, "bulk.cuh")).read()
+    turns = 1 << int(re.search(r"#define BNK_BULK_TURNS \(1u << (\d+)\)", text)[1])
+    with Context(max_keypairs=1, mtu=0, flow_capacity=0) as c:
+        key = np.zeros((1, 32), np.uint8)
+        c.set_keypairs(0, key, key, np.zeros(1, np.uint32))
+        b = c.batch(1, 1024)
+        took = []
+        for size, status in [(lossy, PKT_NOT_READ)] * 3 + [(lossy + 16, 0)] * 3:
+            b.off[:], b.len[:], b.slot[:] = 0, size, 0
+            b.seal(1, F_TIMED)
+            assert b.status[0] == status
+            took.append(b.last_kernel_ms())
+        seconds = (min(took[:3]) - min(took[3:])) / 1e3 / (2 * _build.LOST_TURNS) * turns  # (it waits twice)
+        assert 0.1 < seconds < 2, seconds
+        b.close()
