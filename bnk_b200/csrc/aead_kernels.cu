@@ -1111,8 +1111,10 @@ void wpp_grid(AeadArgs &a, uint32_t &ctas) {
     if (!a.from_host) ctas = std::min(ctas, kStoreCtas);
     else ctas = (uint32_t)std::min<uint64_t>(ctas, std::min(std::max(kLinkWindow / per_packet, kLeastCtas), kMostCtas));
     while (a.tile < 8 && a.n > ctas * kWppWarps * a.tile) a.tile *= 2;
-    // Warps that all take as many tiles end together: 8000 x 1420 B are four rounds for 64 CTAs, of which the last has most of
-    // them idle, and three for 84 (sealed 382 us and 363, opened 396 and 374; 15,000 of them 691 and 670, 711 and 656).
+    // Warps that all take as many tiles end together: 9000 x 1420 B are 1125 tiles, five rounds for 64 CTAs, the last with 101 of its
+    // 256 warps busy, and three for 94 (sealed 421 us and 394, opened 408 and 389); 15,000 are eight rounds and five (671 and 638, 660
+    // and 627).  Where the last round is nearly full there is nothing to gain: 8000 (232 of 256 warps) 362 us, by 84 CTAs 361.  More
+    // CTAs than kEvenCtas gain nothing more: 12,000 by 94 (four rounds) 515, by 128 (three) 514; 15,000 by 94 638, by 128 634.
     const uint32_t tiles = (a.n + a.tile - 1) / a.tile;
     if (a.from_host && tiles > ctas * kWppWarps) {
         const uint32_t rounds = (tiles + std::max(ctas, kEvenCtas) * kWppWarps - 1) / (std::max(ctas, kEvenCtas) * kWppWarps);

@@ -164,7 +164,7 @@ cudaError_t tally_if_asked(bnk_batch *b, uint32_t npkts, uint32_t flags, cudaStr
 // 77 us at 1.6 MB, 234 at 6.4 MB, 680 at 24 MB and 4.55 ms at 190 MB: only far up they are the faster form.
 // With several batches in flight the engines overlap the batches' copies with each other (48 GB/s each way together), so a
 // large batch runs this way only if nothing else is in flight, or if all that run this way together stay below
-// kDirectTogether bytes and at most two others are in flight: SMs move 28-33 GB/s each way over the link and the engines,
+// kDirectTogether bytes and at most two others are in flight: SMs move 28-35 GB/s each way over the link and the engines,
 // kept busy by that many batches, 46-48.  Queue of 1024-packet batches, Gbit/s with up to fifteen others / two in place
 // beyond 384 KB: 32 callers x 4 calls 195 / 255, 16 x 4 193 / 205, 16 x 2 (smaller batches) 182 / 170.
 // A small batch always does.  Its copies are too small for the engines, and in-place kernels beside copied batches are
@@ -188,7 +188,8 @@ bool host_direct(bnk_batch *b, uint32_t npkts, uint32_t flags, uint64_t ext) {
     return true;
 }
 // Calls that look at the first bytes of each packet only read them in place, however many there are and however close together:
-// the link takes ~2.6 ns per request, fewer where packets share lines, and a copy costs 6-8 us before it moves anything.
+// the link takes ~2.2 ns per head (65,536 of them 1472 bytes apart 156 us, 64 bytes apart 110: requests are lines), and a copy costs
+// 6-8 us before it moves anything.
 // Headers 48 bytes apart checked, copied first / in place: 2000 28.8 us / 17.0, 16,000 40.8 / 32, 80,000 121 / 108, 800,000 908 /
 // 896; packets of 64 B noted and checked, 2000 76 / 36, 16,000 132 / 85; datagrams of 28 B classified, 5000 59 / 23, 50,000 178 /
 // 117.  With other batches in flight as well, Mpackets/s copied / in place, threads x headers 48 bytes apart: 4 x 2000 159 / 344, 8 x

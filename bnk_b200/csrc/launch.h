@@ -6,6 +6,8 @@
 // the second a dependent launch: 9.1 and 6.6).  With several threads at it the two are alike or the graph is behind (8
 // threads 9.9 and 10.0 us a round, 16 threads 10.1 and 10.9, but 4 threads 9.3 and 7.0), and a change of the kernel in such a graph
 // costs what it saves (7.05 against 7.1).  So: few batches in flight, and a graph for every kernel or pair of kernels.
+// Of a whole call, from submit to the end of the wait: 5 x 92 B sealed 15.0 us without and 14.4 with a graph, opened (two kernels)
+// 20.9 and 17.2; 128 x 1420 B sealed 18.6 either way, opened 28.1 and 21.5.
 #pragma once
 
 #include <cuda_runtime.h>

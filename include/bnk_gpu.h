@@ -27,7 +27,17 @@
  *     library.  A batch that asks for both copies and is alone in flight, or small
  *     enough beside others, is not copied at all: the kernels read and write the
  *     pinned arrays in place (up to a ring extent of BNK_HOST_DIRECT_BYTES from the
- *     environment, 0 = never).  The results are the same bytes.
+ *     environment, 0 = never).  The results are the same bytes.  What such a submit
+ *     works on is not on the device behind it: a call with BNK_F_NO_H2D that follows
+ *     brings it there first, so the host arrays stay as they are until that call.
+ *   - A program's first submit of a kind (call, options, size class) loads its kernels,
+ *     0.1 to 2 ms, and of a kind with few batches in flight the fourth makes the
+ *     executable graph through which they are launched from then on: 0.1 to 0.3 ms and
+ *     100 KB of device memory, again for each further one in flight, at most 48 per
+ *     device, kept until its last context goes; submits of other threads wait as
+ *     long.  A packet loop that cannot bear that makes a few submits of its kinds
+ *     beforehand, or sets BNK_LAUNCH_GRAPHS=0 in the environment of bnk_ctx_create,
+ *     and none is made.
  *   - Send counters and replay windows are per keypair and ordered: batches that
  *     are in flight at the same time must not carry packets of the same keypair
  *     slot when BNK_F_ASSIGN_COUNTERS or BNK_F_REPLAY is used (give each peer's
