@@ -604,6 +604,131 @@ struct LanePower {
     }
 };
 
+// Poly1305's r and pad out of cipher block 0, which lane 0 holds.
+__device__ __forceinline__ P26 one_time_key(const uint32_t (&x)[16], uint32_t (&pad)[4]) {
+    const uint32_t k0 = __shfl_sync(0xffffffffu, x[0], 0), k1 = __shfl_sync(0xffffffffu, x[1], 0);
+    const uint32_t k2 = __shfl_sync(0xffffffffu, x[2], 0), k3 = __shfl_sync(0xffffffffu, x[3], 0);
+#pragma unroll
+    for (int i = 0; i < 4; i++) pad[i] = __shfl_sync(0xffffffffu, x[4 + i], 0);
+    return p26_words(k0 & 0x0fffffffu, k1 & 0x0ffffffcu, k2 & 0x0ffffffcu, k3 & 0x0ffffffcu, 0u);
+}
+// What a lane does with its part of one round: `data` is the stage at the round's body of rb bytes, x the lane's keystream,
+// `steps` what is left of the powers, beside() runs between the cipher and Poly1305.  The body's ciphertext or plaintext and, on
+// the seal side, the tag are in the stage afterwards.  True: the tag is wrong, and the body is zeros.
+template <bool OPEN, typename F>
+__device__ __forceinline__ bool cipher_and_mac(uint4 *const data, uint32_t rb, uint32_t body, bool last, uint32_t (&x)[16], const P26 &r,
+                                               P26 &state, LanePower &power, uint32_t steps, const uint32_t (&pad)[4], bool broken, F beside) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t data_blocks = (rb + 15u) >> 4, blocks = data_blocks + (last ? 1u : 0u);
+    const bool works = lane != 0 && (lane - 1u) * 64u < rb;
+    const int body_left = (int)rb - (int)(lane - 1u) * 64;
+    uint8_t *const end_byte = reinterpret_cast<uint8_t *>(data) + rb + lane; // byte `lane` behind the round's body
+    const bool in_last_piece = lane < ((0u - rb) & 15u);                    // it shares the body's last piece
+    uint8_t tag_byte = 0;
+    bool forged = false;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        if (!works || 16 * c >= body_left) continue;
+        uint4 *const p = &data[4u * (lane - 1u) + c];
+        const uint4 v = *p;
+        x[4 * c + 0] ^= v.x;
+        x[4 * c + 1] ^= v.y;
+        x[4 * c + 2] ^= v.z;
+        x[4 * c + 3] ^= v.w;
+        if (!OPEN) *p = make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+    }
+    if (!OPEN) { // Poly1305 pads its last block with zeros
+        __syncwarp();
+        if (in_last_piece) *end_byte = 0;
+    }
+    beside();
+    __syncwarp();
+    // ---- Poly1305 over the ciphertext in the stage ----
+    P26 V = p26_zero();
+    const int b0 = (int)(4u * lane + blocks) - 128; // the lane's first block; negative: none
+    if (b0 <= 0 && b0 > -4) V = state;              // (zero in round 0)
+#pragma unroll 1
+    for (int s = 0; s < 4; s++) {
+        const int blk = b0 + s;
+        uint4 m = make_uint4(0u, 0u, body, 0u); // le64(0) | le64(body)
+        if (blk >= 0 && (uint32_t)blk < data_blocks) {
+            m = data[blk];
+            const int left = (int)rb - 16 * blk;
+            if (OPEN && left < 16) {
+                m.x = keep_bytes(m.x, left);
+                m.y = keep_bytes(m.y, left - 4);
+                m.z = keep_bytes(m.z, left - 8);
+                m.w = keep_bytes(m.w, left - 12);
+            }
+        }
+        const P26 next_v = p26_mul(p26_add(V, p26_words(m.x, m.y, m.z, m.w, 1u)), r);
+        if (blk >= 0) V = next_v;
+        if (OPEN && steps) { // beside the Horner step: neither waits for the other
+            power.step();
+            steps--;
+        }
+    }
+    if (OPEN && steps) power.step();
+    V = p26_mul(V, power.p);
+#pragma unroll
+    for (int d = 16; d; d >>= 1) { // limbs below 2^27: the sum of 32 of them fits a word
+#pragma unroll
+        for (int i = 0; i < 5; i++) V.v[i] += __shfl_xor_sync(0xffffffffu, V.v[i], d);
+    }
+    state = p26_carry(V);
+    // ---- tag, output ----
+    if (last) {
+        uint32_t tag[4];
+        p26_finish(state, pad, tag);
+        const uint32_t tw = (lane & 8u) ? ((lane & 4u) ? tag[3] : tag[2]) : ((lane & 4u) ? tag[1] : tag[0]);
+        const uint8_t tb = (uint8_t)(tw >> (8u * (lane & 3u)));
+        if (OPEN) {
+            tag_byte = *end_byte;
+            forged = __any_sync(0xffffffffu, lane < 16u && tag_byte != tb) || broken;
+        } else if (lane < 16u) {
+            *end_byte = tb;
+        }
+    }
+    if (OPEN) {
+        __syncwarp(); // ciphertext and tag are read
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            if (works && 16 * c < body_left)
+                data[4u * (lane - 1u) + c] =
+                    forged ? make_uint4(0, 0, 0, 0) : make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+        __syncwarp();
+        if (last && in_last_piece) *end_byte = tag_byte; // what is not plaintext goes back as it came
+    }
+    return forged;
+}
+// The flow of a packet whose payload starts at stage[piece] (the IPv4 header and the ports lie in 64 bytes).
+__device__ __forceinline__ void note_head(FlowNote &note, const AeadArgs &a, const uint4 *stage, uint32_t piece, uint32_t len) {
+    const uint32_t word = stage_word(stage, piece);
+    Parsed p;
+    const uint32_t at = parse_ipv4_words(__shfl_sync(0xffffffffu, word, 0), __shfl_sync(0xffffffffu, word, 2),
+                                         __shfl_sync(0xffffffffu, word, 3), __shfl_sync(0xffffffffu, word, 4), len, p);
+    const uint32_t ports = __shfl_sync(0xffffffffu, word, (at >> 2) & 15u);
+    if (at != kParseBad && (threadIdx.x & 31) == 0) {
+        if (at) parse_ports(ports, p);
+        note.begin(a.ft, p, a.now);
+    }
+}
+// What the last checks want of the plaintext of `body` bytes that starts at stage[piece].
+__device__ __forceinline__ void inner_head(const AeadArgs &a, const uint4 *stage, uint32_t piece, uint32_t body, size_t pkt) {
+    const uint32_t word = stage_word(stage, piece);
+    const uint32_t w0 = __shfl_sync(0xffffffffu, word, 0), w3 = __shfl_sync(0xffffffffu, word, 3);
+    const uint32_t total = ((w0 >> 8) & 0xff00u) | (w0 >> 24); // bytes 2,3 big-endian
+    const bool is_whole = body >= 20 && ((w0 & 0xffu) >> 4) == 4u && total >= 20 && total <= body;
+    Parsed p{};
+    const uint32_t at = parse_ipv4_words(w0, __shfl_sync(0xffffffffu, word, 2), w3, __shfl_sync(0xffffffffu, word, 4),
+                                         a.inner_cut && is_whole ? total : body, p);
+    const uint32_t ports = __shfl_sync(0xffffffffu, word, (at >> 2) & 15u);
+    if (at != kParseBad && at) parse_ports(ports, p);
+    if ((threadIdx.x & 31) == 0)
+        a.inner[pkt] = make_uint4(__byte_perm(w3, 0, 0x0123), (uint32_t)p.sport << 16 | p.dport,
+                                  p.proto | (at != kParseBad ? kInnerParses : 0u) | (is_whole ? kInnerWhole : 0u), total);
+}
+
 template <bool OPEN, bool NOTE, uint32_t INLINE>
 __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __grid_constant__ AeadArgs a,
                                                                       const __grid_constant__ InlineDesc<INLINE> desc) {
@@ -817,17 +942,9 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                 res_len = 0;
             }
             FlowNote note;
-            auto note_begin = [&] { // the IPv4 header and the ports lie in 64 bytes
+            auto note_begin = [&] {
                 if (!NOTE || broken || (off & 15u) || (uint64_t)off + BNK_WG_HEADER + len > a.ring_bytes) return;
-                const uint32_t word = stage_word(stage, rd.body);
-                Parsed p;
-                const uint32_t at = parse_ipv4_words(__shfl_sync(0xffffffffu, word, 0), __shfl_sync(0xffffffffu, word, 2),
-                                                     __shfl_sync(0xffffffffu, word, 3), __shfl_sync(0xffffffffu, word, 4), len, p);
-                const uint32_t ports = __shfl_sync(0xffffffffu, word, (at >> 2) & 15u);
-                if (at != kParseBad && lane == 0) {
-                    if (at) parse_ports(ports, p);
-                    note.begin(a.ft, p, a.now);
-                }
+                note_head(note, a, stage, rd.body, len);
             };
             if (st != BNK_PKT_OK) { // the next packet's copies are in the other stage
                 if (header_first) arrived(buf);
@@ -858,25 +975,20 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
             const uint32_t remote = OPEN ? 0u : __shfl_sync(0xffffffffu, cur.remote, k);
             P26 r = p26_zero(), state = p26_zero();
             LanePower power;
-            uint32_t pad[4] = {0, 0, 0, 0}, tag[4];
+            uint32_t pad[4] = {0, 0, 0, 0};
             bool forged = false;
-            uint8_t tag_byte = 0;
 #pragma unroll 1
             for (uint32_t rnd = 0;; rnd++) {
                 const uint32_t done = rnd * kRoundBytes;
                 const uint32_t rb = min(body - done, kRoundBytes); // body bytes of this round
                 const bool last = body - done <= kRoundBytes;
-                const uint32_t data_blocks = (rb + 15u) >> 4, blocks = data_blocks + (last ? 1u : 0u);
+                const uint32_t blocks = ((rb + 15u) >> 4) + (last ? 1u : 0u);
                 // ---- keystream: lane 0 block 0, lane j the j-th block of the round ----
                 uint32_t x[16];
                 chacha20_block<1>(x, key, lane == 0 ? 0u : rnd * kRoundBlocks + lane, n_lo, n_hi);
                 uint32_t steps = 0; // of the lanes' powers: as many as there are bits in the number of lanes that hold blocks
                 if (rnd == 0) {
-                    const uint32_t k0 = __shfl_sync(0xffffffffu, x[0], 0), k1 = __shfl_sync(0xffffffffu, x[1], 0);
-                    const uint32_t k2 = __shfl_sync(0xffffffffu, x[2], 0), k3 = __shfl_sync(0xffffffffu, x[3], 0);
-                    r = p26_words(k0 & 0x0fffffffu, k1 & 0x0ffffffcu, k2 & 0x0ffffffcu, k3 & 0x0ffffffcu, 0u);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) pad[i] = __shfl_sync(0xffffffffu, x[4 + i], 0);
+                    r = one_time_key(x, pad);
                     power.begin(r);
                     steps = last ? 32u - __clz((blocks + 3u) / 4u - 1u) : 5u;
                     if (!OPEN || header_first) {
@@ -902,107 +1014,20 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                     arrived(buf);
                 }
                 // ---- cipher ----
-                const bool works = lane != 0 && (lane - 1u) * 64u < rb;
-                const int body_left = (int)rb - (int)(lane - 1u) * 64;
-                const uint32_t end_at = 16u * rd.body + rb + lane; // byte `lane` behind the round's body, in the stage
-                uint8_t *const end_byte = stage_bytes + end_at;
-                const bool in_last_piece = lane < ((0u - rb) & 15u); // it shares the body's last piece
                 if (!OPEN && in_len < body) { // WireGuard's padding: zeros behind the payload
                     const uint32_t at = in_len + lane - done;
                     if (lane < 16u && in_len + lane >= done && at < rb)
                         stage_bytes[16u * rd.body + at] = 0;
                     __syncwarp();
                 }
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    if (!works || 16 * c >= body_left) continue;
-                    uint4 *const p = &stage[rd.body + 4u * (lane - 1u) + c];
-                    const uint4 v = *p;
-                    x[4 * c + 0] ^= v.x;
-                    x[4 * c + 1] ^= v.y;
-                    x[4 * c + 2] ^= v.z;
-                    x[4 * c + 3] ^= v.w;
-                    if (!OPEN) *p = make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
-                }
-                if (!OPEN) { // Poly1305 pads its last block with zeros
-                    __syncwarp();
-                    if (in_last_piece) *end_byte = 0;
-                }
-                if (NOTE && rnd == 0) note.place(a.ft);
-                __syncwarp();
-                // ---- Poly1305 over the ciphertext in the stage ----
-                P26 V = p26_zero();
-                const int b0 = (int)(4u * lane + blocks) - 128; // the lane's first block; negative: none
-                if (b0 <= 0 && b0 > -4) V = state;              // (zero in round 0)
-#pragma unroll 1
-                for (int s = 0; s < 4; s++) {
-                    const int blk = b0 + s;
-                    uint4 m = make_uint4(0u, 0u, body, 0u); // le64(0) | le64(body)
-                    if (blk >= 0 && (uint32_t)blk < data_blocks) {
-                        m = stage[rd.body + blk];
-                        const int left = (int)rb - 16 * blk;
-                        if (OPEN && left < 16) {
-                            m.x = keep_bytes(m.x, left);
-                            m.y = keep_bytes(m.y, left - 4);
-                            m.z = keep_bytes(m.z, left - 8);
-                            m.w = keep_bytes(m.w, left - 12);
-                        }
-                    }
-                    const P26 next_v = p26_mul(p26_add(V, p26_words(m.x, m.y, m.z, m.w, 1u)), r);
-                    if (blk >= 0) V = next_v;
-                    if (OPEN && steps) { // beside the Horner step: neither waits for the other
-                        power.step();
-                        steps--;
-                    }
-                }
-                if (OPEN && steps) power.step();
-                V = p26_mul(V, power.p);
-#pragma unroll
-                for (int d = 16; d; d >>= 1) { // limbs below 2^27: the sum of 32 of them fits a word
-#pragma unroll
-                    for (int i = 0; i < 5; i++) V.v[i] += __shfl_xor_sync(0xffffffffu, V.v[i], d);
-                }
-                state = p26_carry(V);
-                // ---- tag, output ----
-                if (last) {
-                    p26_finish(state, pad, tag);
-                    const uint32_t tw = (lane & 8u) ? ((lane & 4u) ? tag[3] : tag[2]) : ((lane & 4u) ? tag[1] : tag[0]);
-                    const uint8_t tb = (uint8_t)(tw >> (8u * (lane & 3u)));
-                    if (OPEN) {
-                        tag_byte = *end_byte;
-                        forged = __any_sync(0xffffffffu, lane < 16u && tag_byte != tb) || broken;
-                    } else if (lane < 16u) {
-                        *end_byte = tb;
-                    }
-                }
-                if (OPEN) {
-                    __syncwarp(); // ciphertext and tag are read
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        if (works && 16 * c < body_left)
-                            stage[rd.body + 4u * (lane - 1u) + c] =
-                                forged ? make_uint4(0, 0, 0, 0) : make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
-                    __syncwarp();
-                    if (last && in_last_piece) *end_byte = tag_byte; // what is not plaintext goes back as it came
-                } else if (rnd == 0 && lane == 0) {
+                forged = cipher_and_mac<OPEN>(&stage[rd.body], rb, body, last, x, r, state, power, steps, pad, broken, [&] {
+                    if (NOTE && rnd == 0) note.place(a.ft);
+                });
+                if (!OPEN && rnd == 0 && lane == 0) {
                     stage[0] = make_uint4(4u, remote, n_lo, n_hi);
                 }
                 __syncwarp();
-                if (OPEN && a.inner && rnd == 0 && !forged) {
-                    const uint32_t word = stage_word(stage, rd.body);
-                    const uint32_t w0 = __shfl_sync(0xffffffffu, word, 0), w3 = __shfl_sync(0xffffffffu, word, 3);
-                    const uint32_t total = ((w0 >> 8) & 0xff00u) | (w0 >> 24); // bytes 2,3 big-endian
-                    const bool is_whole = body >= 20 && ((w0 & 0xffu) >> 4) == 4u && total >= 20 && total <= body;
-                    Parsed p{};
-                    const uint32_t at = parse_ipv4_words(w0, __shfl_sync(0xffffffffu, word, 2), w3, __shfl_sync(0xffffffffu, word, 4),
-                                                         a.inner_cut && is_whole ? total : body, p);
-                    const uint32_t ports = __shfl_sync(0xffffffffu, word, (at >> 2) & 15u);
-                    if (at != kParseBad && at) parse_ports(ports, p);
-                    if (lane == 0)
-                        a.inner[(size_t)t * T + k] =
-                            make_uint4(__byte_perm(w3, 0, 0x0123), (uint32_t)p.sport << 16 | p.dport,
-                                       p.proto | (at != kParseBad ? kInnerParses : 0u) | (is_whole ? kInnerWhole : 0u), total);
-                }
+                if (OPEN && a.inner && rnd == 0 && !forged) inner_head(a, stage, rd.body, body, (size_t)t * T + k);
                 // The last piece goes out whole where the bytes behind the message were read from the same place.
                 const uint32_t out_bytes = OPEN ? rb : rb + (last ? BNK_WG_TAG : 0u);
                 const bool other_place = a.in != a.out;
@@ -1083,6 +1108,353 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
     signal_done(a.done, NOTE && a.flow_report, [&] { flow_report(flow_ctl(a.ft), a.flow_report); });
 }
 
+// ---------------------------------------------------------------------------
+// Kernel 3, a stream of packets through each CTA: batches beyond kRankMax packets in pinned memory whose packets lie close
+// together in the ring.
+//
+// There the link is the bound (without any cipher work kernel 2 takes as long), and what counts is how it is asked: in whole
+// lines, few of them twice, and with about half a megabyte outstanding in all.  So the first warp brings neighbouring packets up
+// as one copy, up to kStreamRun bytes of them, into one of kStreamStages stages, the other warps take the packets of a stage one
+// by one, and the whole stretch goes back as one copy: bytes between packets as they were read.  The warps that compute are as
+// many whatever the size of the packets, which a warp that fetched for itself could not have: with kernel 2's warp for each few
+// packets either the requests of all of them are on the link at once, and the writes come afterwards, or small packets wait
+// for warps.  At most kStreamAhead copies of a CTA are on their way up, however many of its stages are worked on.
+// Plain copies in place, us for 1024 / 4096 / 12,000 packets of 1420 B 1472 apart: a packet at a time, two for each of 256 warps
+// 62 / 176 / 482, two neighbours at a time, three stages in 64 CTAs 53 / 164 / 453; with 16 neighbours in 16 CTAs, as many
+// bytes, 58 / 169 / 455, in 64 61 / 202 / 499.  9000 of 64 B: a packet at a time 74, 32 at a time 40.
+//
+// A CTA's packets lie next to each other, which counts when a core has just written them: the open of 1024 x 1420 B 67 us, with
+// tiles dealt out in turn 75 (12,000 alike either way, 493 and 490).  A tile of a.tile packets is what the first warp has in its
+// lanes: descriptors, of two tiles further ahead as well, since they come over the link behind all that has been asked for; and
+// results, until a tile's leave together.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kStreamWarps = 17, kStreamWorkers = kStreamWarps - 1;
+constexpr uint32_t kStreamStages = 6, kStreamAhead = 2, kStreamRun = 3200;
+constexpr uint32_t kStreamGap = 16;        // what may lie between neighbours: no message, wherever its descriptor is, fits in there
+constexpr uint32_t kStreamIdle = 1u << 25; // turns of the first warp in which nothing has happened: seconds
+static_assert(kStreamRun >= kRoundBytes + BNK_WG_HEADER + 2 * BNK_WG_TAG && kStreamRun % 128 == 0, "a packet of one round fits");
+struct StreamRun { // neighbours in a stage
+    uint32_t count;        // 0: no more come
+    uint32_t first, base;  // the first one, and where it starts in the ring
+    uint32_t bytes;        // in the stage; 0: of a packet that lies outside of the ring
+    uint32_t turn;         // the worker that takes the first
+    bool asked, ends_tile; // asked: the bytes are, or were, on their way
+    uint32_t off[32], len[32], slot[32];
+    uint64_t counter[32]; // of a seal; then the results
+    uint32_t out_len[32];
+    uint8_t status[32], has_counter[32];
+};
+struct StreamShared {
+    alignas(128) uint4 stage[kStreamStages][(kStreamRun + 64) / 16]; // (a look at a packet's head may go 64 bytes beyond its start)
+    StreamRun run[kStreamStages];
+    uint64_t ready[kStreamStages], full[kStreamStages], over[kStreamStages]; // a run is described, has come, is worked on
+};
+// A wait for another warp of the CTA, whose own waits for copies end after bar_wait's time.
+__device__ __forceinline__ bool bar_wait_warp(uint64_t *bar, uint32_t parity) {
+    for (uint32_t k = 0; k < 2 * kStreamStages + 2; k++)
+        if (bar_wait(bar, parity)) return true;
+    return false;
+}
+
+// The first warp.
+template <bool OPEN>
+__device__ __forceinline__ void stream_feed(const AeadArgs &a, StreamShared &sh) {
+    const uint32_t lane = threadIdx.x & 31, T = a.tile, all = (a.n + T - 1) / T, share = (all + gridDim.x - 1) / gridDim.x;
+    uint32_t t = blockIdx.x * share; // the tile that is given out
+    const uint32_t tiles = min(all, t + share);
+    struct Tile { // a packet's descriptor in each of the first T lanes
+        uint32_t off, len, slot;
+        uint64_t ctr;
+    };
+    auto load_tile = [&](uint32_t t) {
+        Tile d{0, 0, 0, 0};
+        const uint32_t i = t * T + lane;
+        if (t < tiles && lane < T && i < a.n) {
+            d.off = a.off[i];
+            d.len = a.len[i];
+            if (!OPEN || !a.demux) d.slot = a.slot[i];
+            if (!OPEN && !a.behind_kernel) d.ctr = a.counter[i]; // the host's
+        }
+        return d;
+    };
+    uint32_t j = 0; // the tile's next packet
+    Tile cur = load_tile(t), next = load_tile(t + 1), after = load_tile(t + 2);
+    uint32_t end = 0; // of this lane's packet in the ring, in whole pieces; 0: outside of it
+    bool joins = false; // it can come with the one in front
+    auto look = [&] {
+        const uint64_t room = OPEN ? cur.len : (uint64_t)BNK_WG_HEADER + cur.len;
+        end = 0;
+        if (lane < T && t * T + lane < a.n && !(cur.off & 15u) && cur.off + room <= a.ring_bytes && (!OPEN || cur.len >= BNK_WG_HEADER + BNK_WG_TAG)) {
+            const uint32_t body = OPEN ? cur.len - (BNK_WG_HEADER + BNK_WG_TAG) : wg_padded_len(cur.len, a.mtu);
+            const uint64_t message = (uint64_t)BNK_WG_HEADER + body + BNK_WG_TAG;
+            const uint64_t size = cur.off + message <= a.ring_bytes && message > room ? message : room;
+            if (body <= kRoundBytes && size <= kStreamRun) end = cur.off + (((uint32_t)size + 15u) & ~15u);
+        }
+        const uint32_t before = __shfl_up_sync(0xffffffffu, end, 1);
+        joins = lane > 0 && end && before && cur.off >= before && cur.off - before <= kStreamGap;
+    };
+    look();
+    // Runs are given to the stages in turn: `asked` of them have been, `sent` are on their way back (or have nothing to send).
+    uint32_t turn = 0, asked = 0, sent = 0;
+    bool fetches = true; // until a copy does not come
+    const auto passed = [&](uint64_t *bars, uint32_t run) { // the same for all lanes
+        const bool v = __any_sync(0xffffffffu, bar_test(&bars[run % kStreamStages], run / kStreamStages & 1u));
+        __syncwarp();
+        return v;
+    };
+    auto ask = [&] {
+        const uint32_t s = asked % kStreamStages, in_tile = min(T, a.n - t * T), base = __shfl_sync(0xffffffffu, cur.off, j);
+        StreamRun &r = sh.run[s];
+        const uint32_t chain = __ballot_sync(0xffffffffu, lane > j && lane < in_tile && joins && end - base <= kStreamRun) >> j >> 1;
+        const uint32_t count = (uint32_t)__ffs(~chain); // and the first itself
+        const uint32_t to = __shfl_sync(0xffffffffu, end, j + count - 1), bytes = to ? to - base : 0u;
+        if (lane >= j && lane < j + count) {
+            r.off[lane - j] = cur.off;
+            r.len[lane - j] = cur.len;
+            r.slot[lane - j] = cur.slot;
+            if (!OPEN) r.counter[lane - j] = cur.ctr;
+        }
+        if (lane == 0) {
+            r.count = count;
+            r.first = t * T + j;
+            r.base = base;
+            r.bytes = bytes;
+            r.turn = turn;
+            r.asked = fetches;
+            r.ends_tile = j + count == in_tile;
+            if (fetches) {
+                bar_expect(&sh.full[s], bytes);
+                if (bytes) bulk_in(sh.stage[s], a.in + base, bytes, &sh.full[s]);
+            }
+        }
+        __syncwarp();
+        if (lane == 0) bar_arrive(&sh.ready[s]);
+        asked++;
+        turn = (turn + count) % kStreamWorkers;
+        j += count;
+        if (j < in_tile) return;
+        t++;
+        j = 0;
+        cur = next;
+        next = after;
+        after = load_tile(t + 2);
+        look();
+    };
+    uint32_t res_len = 0, res_status = BNK_PKT_OK, res_slot = 0, res_has = 0;
+    uint64_t res_ctr = 0;
+    auto send = [&] { // the oldest run, which has been worked on
+        StreamRun &r = sh.run[sent % kStreamStages];
+        const uint32_t count = r.count, first = r.first & (T - 1), k = lane - first;
+        if (lane >= first && k < count) {
+            res_len = r.out_len[k];
+            res_status = r.status[k];
+            res_slot = r.slot[k];
+            res_ctr = r.counter[k];
+            res_has = r.has_counter[k];
+        }
+        // (No worker waits for a packet that is refused for its descriptor; and where one has given up, the bytes are as they came.)
+        const bool whole = __any_sync(0xffffffffu, r.asked && bar_wait(&sh.full[sent % kStreamStages], sent / kStreamStages & 1u));
+        if (!whole) fetches = false;
+        if (lane == 0) {
+            if (whole && r.bytes) bulk_out(a.out + r.base, sh.stage[sent % kStreamStages], r.bytes);
+            bulk_out_commit();
+        }
+        if (r.ends_tile && lane < first + count) {
+            const uint32_t i = r.first - first + lane;
+#pragma unroll
+            for (int d = 0; d < 2; d++) {
+                const AeadResults &o = a.res[d];
+                if (o.status) o.status[i] = (uint8_t)res_status;
+                if (o.out_len) o.out_len[i] = res_len;
+                if (o.counter && res_has) o.counter[i] = res_ctr;
+                if (o.slot) o.slot[i] = res_slot;
+            }
+        }
+        __syncwarp();
+        sent++;
+    };
+    for (uint32_t idle = 0; (t < tiles || sent < asked) && idle < kStreamIdle;) {
+        // a stage is free, or will be as soon as the copy out of it has read it, and not too much is on its way
+        const bool room = asked < kStreamStages || asked - kStreamStages < sent;
+        if (t < tiles && room && (!fetches || asked < kStreamAhead || passed(sh.full, asked - kStreamAhead))) {
+            if (asked >= kStreamStages && lane == 0) {
+                if (sent - (asked - kStreamStages) >= 2) bulk_out_read_but_last();
+                else bulk_out_read();
+            }
+            __syncwarp();
+            ask();
+            idle = 0;
+        } else if (sent < asked && passed(sh.over, sent)) {
+            send();
+            idle = 0;
+        } else {
+            __nanosleep(32);
+            idle++;
+        }
+    }
+    if (lane == 0) { // no more come: in the stage that every worker looks at next
+        sh.run[asked % kStreamStages].count = 0;
+        bar_arrive(&sh.ready[asked % kStreamStages]);
+        bulk_out_done();
+    }
+    for (uint32_t run = sent; run < asked; run++) // a copy that is still on its way must not meet the next kernel's shared memory
+        if (sh.run[run % kStreamStages].asked) bar_wait(&sh.full[run % kStreamStages], run / kStreamStages & 1u);
+}
+
+// The others.
+template <bool OPEN, bool NOTE>
+__device__ __forceinline__ void stream_work(const AeadArgs &a, StreamShared &sh, uint32_t worker) {
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t s = 0, parity = 0;;) {
+        StreamRun &r = sh.run[s];
+        if (!bar_wait_warp(&sh.ready[s], parity)) return;
+        const uint32_t count = r.count;
+        if (count == 0) return;
+#pragma unroll 1
+        for (uint32_t k = (worker + kStreamWorkers - r.turn) % kStreamWorkers; k < count; k += kStreamWorkers) {
+            const uint32_t off = r.off[k], len = r.len[k], pkt = r.first + k;
+            uint32_t slot = r.slot[k];
+            const bool in_stage = r.bytes != 0;
+            uint4 *const stage = sh.stage[s] + (in_stage ? (off - r.base) >> 4 : 0u); // the header, and then the body
+            bool broken = false, looked = false;
+            auto arrived = [&] {
+                if (!looked) broken = !r.asked || !bar_wait(&sh.full[s], parity);
+                looked = true;
+                broken = __any_sync(0xffffffffu, broken);
+                __syncwarp();
+            };
+            // ---- what the descriptor says (the same for all lanes) ----
+            uint8_t st = BNK_PKT_OK, valid = 0;
+            uint32_t body = 0, n_lo = 0, n_hi = 0, remote = 0;
+            uint64_t ctr = 0;
+            uint4 ka = make_uint4(0, 0, 0, 0), kb = ka;
+            bool has_counter = !OPEN && slot < a.max_slots;
+            auto load_keypair = [&] { // asked for together
+                if (slot >= a.max_slots) return;
+                const uint4 *const kp = reinterpret_cast<const uint4 *>(a.keys + (size_t)slot * 8);
+                valid = a.valid[slot];
+                ka = kp[0];
+                kb = kp[1];
+                if (!OPEN) remote = a.remote_index[slot];
+            };
+            if (OPEN) {
+                if (!a.demux) load_keypair();
+                arrived();
+                const bool in_ring = (uint64_t)off + len <= a.ring_bytes, whole = in_ring && len >= BNK_WG_HEADER + BNK_WG_TAG;
+                uint4 hdr = make_uint4(0, 0, 0, 0);
+                if (in_stage) hdr = stage[0];
+                if (a.demux) {
+                    slot = 0; // descriptors refused below for other reasons
+                    if (in_stage) slot = demux_index_warp(a.index_keys, a.index_vals, a.index_slots, hdr.y);
+                    load_keypair();
+                }
+                if (broken) st = BNK_PKT_NOT_READ;
+                else if ((off & 15u) || slot >= a.max_slots) st = slot == kSlotNoKeypair ? BNK_PKT_NO_KEYPAIR : BNK_PKT_BAD_DESC;
+                else if (!valid) st = BNK_PKT_NO_KEYPAIR;
+                else if (!in_ring) st = BNK_PKT_BAD_DESC;
+                else if (!whole) st = BNK_PKT_MALFORMED;
+                else if (!in_stage) st = BNK_PKT_BAD_DESC; // (longer than the host has said)
+                else {
+                    n_lo = hdr.z;
+                    n_hi = hdr.w;
+                    ctr = ((uint64_t)hdr.w << 32) | hdr.z;
+                    has_counter = true;
+                    if (hdr.x != 4u) st = BNK_PKT_MALFORMED;
+                    body = len - (BNK_WG_HEADER + BNK_WG_TAG);
+                }
+            } else {
+                ctr = a.behind_kernel ? a.counter[pkt] : r.counter[k];
+                load_keypair();
+                n_lo = (uint32_t)ctr;
+                n_hi = (uint32_t)(ctr >> 32);
+                body = wg_padded_len(len, a.mtu);
+                if ((off & 15u) || slot >= a.max_slots) st = BNK_PKT_BAD_DESC;
+                else if (!valid) st = BNK_PKT_NO_KEYPAIR;
+                else if ((uint64_t)off + BNK_WG_HEADER + body + BNK_WG_TAG > a.ring_bytes || body < len || !in_stage) st = BNK_PKT_BAD_DESC;
+                else if (ctr >= BNK_REJECT_AFTER_MESSAGES) st = BNK_PKT_COUNTER_EXHAUSTED;
+            }
+            FlowNote note;
+            auto note_begin = [&] {
+                if (NOTE && !broken && in_stage) note_head(note, a, stage, 1, len);
+            };
+            bool forged = false;
+            if (st != BNK_PKT_OK) {
+                if (NOTE) {
+                    arrived();
+                    note_begin();
+                    note.place(a.ft);
+                }
+            } else {
+                const uint32_t key[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
+                const uint32_t blocks = ((body + 15u) >> 4) + 1u;
+                uint32_t x[16], pad[4];
+                chacha20_block<1>(x, key, lane, n_lo, n_hi); // lane 0 the one-time key, lane j the body's block j
+                const P26 rr = one_time_key(x, pad);
+                LanePower power;
+                power.begin(rr);
+                uint32_t steps = 32u - __clz((blocks + 3u) / 4u - 1u);
+                if (!OPEN) {
+#pragma unroll 1
+                    for (; steps; steps--) power.step();
+                    arrived();
+                    note_begin();
+                }
+                if (!broken) {
+                    if (!OPEN && len < body) { // WireGuard's padding: zeros behind the payload
+                        if (lane < 16u && len + lane < body) reinterpret_cast<uint8_t *>(stage + 1)[len + lane] = 0;
+                        __syncwarp();
+                    }
+                    P26 state = p26_zero();
+                    forged = cipher_and_mac<OPEN>(stage + 1, body, body, true, x, rr, state, power, steps, pad, false, [&] {
+                        if (NOTE) note.place(a.ft);
+                    });
+                    if (!OPEN && lane == 0) stage[0] = make_uint4(4u, remote, n_lo, n_hi);
+                    __syncwarp();
+                    if (OPEN && a.inner && !forged) inner_head(a, stage, 1, body, pkt);
+                }
+            }
+            if (NOTE) note.count(a.ft);
+            __syncwarp();
+            if (lane == 0) {
+                const bool good = st == BNK_PKT_OK && !broken && !forged;
+                r.status[k] = st != BNK_PKT_OK ? st : broken ? BNK_PKT_NOT_READ : forged ? BNK_PKT_AUTH_FAIL : OPEN && body == 0 ? BNK_PKT_KEEPALIVE : BNK_PKT_OK;
+                r.out_len[k] = !good ? 0u : OPEN ? body : BNK_WG_HEADER + body + BNK_WG_TAG;
+                r.slot[k] = slot;
+                r.counter[k] = ctr;
+                r.has_counter[k] = has_counter;
+            }
+        }
+        bulk_fence_shared();
+        __syncwarp();
+        if (lane == 0) bar_arrive(&sh.over[s]);
+        if (++s == kStreamStages) {
+            s = 0;
+            parity ^= 1u;
+        }
+    }
+}
+
+template <bool OPEN, bool NOTE>
+__global__ void __launch_bounds__(32 * kStreamWarps, 1) aead_stream_kernel(const __grid_constant__ AeadArgs a) {
+    static_assert(!(OPEN && NOTE), "flows are recorded on the seal side");
+    let_next_kernel_start();
+    __shared__ StreamShared sh;
+    if (threadIdx.x < kStreamStages) {
+        bar_init(&sh.ready[threadIdx.x]);
+        bar_init(&sh.full[threadIdx.x]);
+        bar_init(&sh.over[threadIdx.x], kStreamWorkers);
+    }
+    bulk_fence_shared();
+    __syncthreads();
+    if (threadIdx.x < 32) { // what it reads is the host's
+        stream_feed<OPEN>(a, sh);
+    } else {
+        wait_for_kernel_in_front();
+        stream_work<OPEN, NOTE>(a, sh, (threadIdx.x >> 5) - 1u);
+    }
+    signal_done(a.done, NOTE && a.flow_report, [&] { flow_report(flow_ctl(a.ft), a.flow_report); });
+}
+
 // Below this many packets one-packet-per-thread leaves most of the GPU idle and its run time is that of one thread
 // walking one packet (~39 us for 1420 B) whatever the batch size; one warp per packet takes ~13 us up to 2,400
 // packets and then grows by ~14 us per 2,400 more.  Measured crossover on B200: between 6,000 and 7,000 packets.
@@ -1144,9 +1516,42 @@ cudaError_t launch_wpp(const AeadArgs &a, uint32_t ctas, const HostDesc *h, cuda
     return with(InlineDesc<kRankMax>{}, aead_wpp_kernel<OPEN, NOTE, kRankMax>);
 }
 
+// Tiles and grid of kernel 3.  With small packets every SM helps, 9000 x 64 B sealed by 96 CTAs 84 us, by 148 72; large ones
+// have as much outstanding as the link takes with fewer: 12,000 x 1420 B by 64 504 us, by 96 482, by 148 491.  Tiles of 16 are
+// worth a CTA each, smaller ones of 4 at the least spread a batch that has fewer than kStreamTiles of them.
+// Below kStreamFrom bytes kernel 2 is as fast: 1000 mixed packets (360 KB) sealed 29.5 us and 30.4, opened 34.3 and 35.3; 512 x 1420 B
+// (730 KB) sealed 38.0 and 35.3.  An open works on a stage for longer, as nothing of it can be done beforehand, and of large packets
+// few are at hand in a CTA: 1500 x 1000 B, whole path, 105.1 us and 106.7, 4096 x 700 B (2.9 MB) 152.0 and 154.4, 2000 x 1420 B (2.8 MB) 148.3
+// and 148.0, but 4096 x 1420 B opened 197 and 188, 12,000 518 and 500; small ones 9000 x 64 B 80 and 73.
+// Sealed, kernel 2 and this one: 1024 x 1420 B 66 us and 61, 4096 201 and 183, 12,000 535 and 490, 9000 x 64 B 83 and 74, whole path
+// 10,000 mixed 176 and 158.
+constexpr uint64_t kStreamFrom = 512u << 10, kStreamOpenFrom = 4u << 20;
+constexpr uint32_t kStreamCtas = 96, kStreamCtasSmall = 148, kStreamTiles = 64, kSmallPacket = 512;
+bool small_packets(const AeadArgs &a) { return a.link_bytes <= (uint64_t)kSmallPacket * a.n; }
+bool in_stream(const AeadArgs &a, bool open) {
+    return a.from_host && a.dense && a.n > kRankMax && a.link_bytes >= (open && !small_packets(a) ? kStreamOpenFrom : kStreamFrom);
+}
+void stream_grid(AeadArgs &a, uint32_t &ctas) {
+    const uint32_t most = small_packets(a) ? kStreamCtasSmall : kStreamCtas;
+    a.tile = 16;
+    while (a.tile > 4 && a.n < kStreamTiles * a.tile) a.tile /= 2;
+    const uint32_t tiles = (a.n + a.tile - 1) / a.tile, rounds = (tiles + most - 1) / most;
+    ctas = (tiles + rounds - 1) / rounds;
+}
+
 template <bool OPEN>
 cudaError_t launch_aead(AeadArgs a, cudaStream_t s, bnk_ctx *ctx) {
     if (a.n == 0) return cudaSuccess;
+    if (in_stream(a, OPEN)) {
+        uint32_t ctas;
+        stream_grid(a, ctas);
+        const dim3 grid(ctas), block(32 * kStreamWarps);
+        const cudaError_t e = !OPEN && a.note ? launch_kernel(a.behind_kernel, aead_stream_kernel<OPEN, !OPEN>, grid, block, s, a)
+                                              : launch_kernel(a.behind_kernel, aead_stream_kernel<OPEN, false>, grid, block, s, a);
+        if (e != cudaSuccess) return e;
+        ++ctx->launches;
+        return cudaGetLastError();
+    }
     const bool wpp = a.over_link || ctx->aead_mode == 2 || (ctx->aead_mode == 0 && a.n <= BNK_WPP_MAX_PACKETS);
     if (wpp) {
         uint32_t ctas;

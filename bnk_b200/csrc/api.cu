@@ -81,12 +81,23 @@ class Slab {
     size_t total_ = 0;
 };
 
-// highest ring byte any of the first n packets can touch (input or output side); their bytes; whether they lie in the
-// ring in order, each with `room` bytes of its own behind it
-uint64_t ring_extent(const bnk_batch *b, uint32_t n, uint32_t slack, uint64_t *bytes = nullptr, uint32_t room = 0, bool *in_order = nullptr) {
+constexpr uint32_t kMostRoom = 16 + 16 + 16; // header, padding and tag around a payload
+// What a submit's way depends on besides.
+struct Layout {
+    uint64_t bytes = 0;    // of the packets
+    bool in_order = false; // they lie in the ring in order, each with its own room behind it
+    bool dense = false;    // at most about a quarter of their stretch of it lies between them, and none is longer than kDenseLongest
+};
+// highest ring byte any of the first n packets can touch (input or output side); with `room` bytes of its own behind each
+constexpr uint32_t kDenseLongest = 1969; // a message, with its padding, of one round in the kernels' terms
+uint64_t ring_extent(const bnk_batch *b, uint32_t n, uint32_t slack, Layout *l = nullptr, uint32_t room = 0) {
     const PacketScan r = scan_packets(b->host.off, b->host.len, n, room);
-    if (bytes) *bytes = r.sum + (uint64_t)n * slack;
-    if (in_order) *in_order = r.in_order;
+    if (l) {
+        const uint64_t from = n ? std::min<uint64_t>(b->host.off[0], r.end) : 0, with_room = r.sum + (uint64_t)n * kMostRoom;
+        l->bytes = r.sum + (uint64_t)n * slack;
+        l->in_order = r.in_order;
+        l->dense = r.longest <= kDenseLongest && 4 * with_room >= 3 * (r.end - from);
+    }
     const uint64_t ext = n ? (r.end + slack + 15) & ~15ull : 0;
     return ext > b->ring_bytes ? b->ring_bytes : ext;
 }
@@ -313,7 +324,6 @@ cudaError_t ring_down(bnk_batch *b, uint32_t n, uint64_t ext, bool joint, cudaSt
 // Brings the device copies up to the host arrays where submits have run on those.  An upload of as many packets with all
 // descriptor fields does the same.  One of those submits may still be in flight, in front on this stream (a submit that
 // leaves the host arrays alone needs no wait in between): what is read here on the host, off[] and len[], no kernel writes.
-constexpr uint32_t kMostRoom = 16 + 16 + 16; // header, padding and tag around a payload
 cudaError_t catch_up(bnk_batch *b, cudaStream_t s) {
     const uint32_t n = b->stale_pkts;
     if (n == 0) return cudaSuccess;
@@ -1019,7 +1029,7 @@ int bnk_batch_download(bnk_batch *b, uint32_t npkts) {
 // it for the counters, and one behind it when expired flows may have to be swept.  With `resident` the packets and
 // descriptors are those on the device (BNK_F_NO_H2D), and the messages go to both rings as they are made: 17 MB of
 // segments sealed and stored 0.38 ms, against 0.44 for seal and download in a row.
-static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t flags, int64_t now_unix_ns, bool resident) {
+static int seal_direct(bnk_batch *b, uint32_t npkts, const Layout &lay, uint32_t flags, int64_t now_unix_ns, bool resident) {
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->direct_stream ? b->direct_stream : b->stream;
     b->order.begins(s);
@@ -1032,7 +1042,7 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     if (timed) CK(ctx, cudaEventRecord(b->k_begin, s));
     AeadArgs a = aead_args(b, npkts, false, nullptr);
     a.over_link = true;
-    a.link_bytes = bytes;
+    a.link_bytes = lay.bytes;
     a.out = h.ring;
     a.res[0] = AeadResults{assign ? h.counter : nullptr, h.out_len, h.status, nullptr};
     if (resident) {
@@ -1043,6 +1053,7 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     } else {
         b->stale_pkts = std::max(b->stale_pkts, npkts);
         a.from_host = true;
+        a.dense = lay.dense;
         a.host = HostDesc{h.off, h.len, h.slot};
         a.in = h.ring;
         a.off = h.off;
@@ -1143,14 +1154,13 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
     const size_t n = npkts;
-    uint64_t bytes = 0;
-    bool in_order = false;
-    const uint64_t ext = device_only ? 0 : ring_extent(b, npkts, kMostRoom, &bytes, BNK_WG_HEADER + BNK_WG_TAG, &in_order);
-    if (in_pieces(b, npkts, flags, ext, in_order)) return seal_pieces(b, npkts, ext, flags, now_unix_ns);
+    Layout lay;
+    const uint64_t ext = device_only ? 0 : ring_extent(b, npkts, kMostRoom, &lay, BNK_WG_HEADER + BNK_WG_TAG);
+    if (in_pieces(b, npkts, flags, ext, lay.in_order)) return seal_pieces(b, npkts, ext, flags, now_unix_ns);
     if (ctx->aead_mode != 1) {
-        if (host_direct(b, npkts, flags, ext)) return seal_direct(b, npkts, bytes, flags, now_unix_ns, false);
+        if (host_direct(b, npkts, flags, ext)) return seal_direct(b, npkts, lay, flags, now_unix_ns, false);
         if (!b->stale_pkts && (flags & BNK_F_NO_H2D) && host_direct(b, npkts, flags & ~BNK_F_NO_H2D, ext))
-            return seal_direct(b, npkts, bytes, flags, now_unix_ns, true);
+            return seal_direct(b, npkts, lay, flags, now_unix_ns, true);
     }
     bool all;
     CK(ctx, catch_up_beside(b, npkts, !(flags & BNK_F_NO_H2D), !(flags & BNK_F_NO_D2H), s, all));
@@ -1220,7 +1230,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
 
 // An open that works on the pinned ring and descriptors.  What has to wait for the replay window (statuses, lengths)
 // stays on the device until then, with the packets' inner headers, so that no later kernel goes back to the ring.
-static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t flags, int64_t now_unix_ns) {
+static int open_direct(bnk_batch *b, uint32_t npkts, const Layout &lay, uint32_t flags, int64_t now_unix_ns) {
     bnk_ctx *ctx = b->ctx;
     cudaStream_t s = b->direct_stream ? b->direct_stream : b->stream;
     b->order.begins(s);
@@ -1238,7 +1248,8 @@ static int open_direct(bnk_batch *b, uint32_t npkts, uint64_t bytes, uint32_t fl
     // opened, threads x batches, Gbit/s with the headers first / without: 8 x 2 177 / 181, 8 x 4 191 / 201, 16 x 4 200 / 214.
     a.header_first = few_in_flight(b);
     a.host = HostDesc{h.off, h.len, h.slot};
-    a.link_bytes = bytes;
+    a.link_bytes = lay.bytes;
+    a.dense = lay.dense;
     a.in = a.out = h.ring;
     a.off = h.off;
     a.len = h.len;
@@ -1355,11 +1366,10 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     cudaStream_t s = b->stream;
     const bool timed = (flags & BNK_F_TIMED) != 0;
     const size_t n = npkts;
-    uint64_t bytes = 0;
-    bool in_order = false;
-    const uint64_t ext = device_only ? 0 : ring_extent(b, npkts, (flags & BNK_F_USE_OUT_LEN) || b->stale_pkts ? kMostRoom : 0, &bytes, 0, &in_order);
-    if (in_pieces(b, npkts, flags, ext, in_order)) return open_pieces(b, npkts, ext, flags, now_unix_ns);
-    if (ctx->aead_mode != 1 && host_direct(b, npkts, flags, ext)) return open_direct(b, npkts, bytes, flags, now_unix_ns);
+    Layout lay;
+    const uint64_t ext = device_only ? 0 : ring_extent(b, npkts, (flags & BNK_F_USE_OUT_LEN) || b->stale_pkts ? kMostRoom : 0, &lay);
+    if (in_pieces(b, npkts, flags, ext, lay.in_order)) return open_pieces(b, npkts, ext, flags, now_unix_ns);
+    if (ctx->aead_mode != 1 && host_direct(b, npkts, flags, ext)) return open_direct(b, npkts, lay, flags, now_unix_ns);
     // BNK_F_USE_OUT_LEN reads the lengths a seal left on the device: an upload beside it must not bring the
     // host's out_len along, so it moves the fields one by one instead of the whole slab.
     bool all;
@@ -1573,7 +1583,8 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
     uint64_t ext = 0; // where the packets end, once they have been looked through
     CK(ctx, catch_up(b, s));
     if (!(flags & BNK_F_NO_H2D) && !refresh && gso_split_fits(supers, n_super, n_pkts, b->ring_bytes)) {
-        uint64_t from = ~0ull, to = 0, sum = 0, segs = 0, of_segs = 0, of_all; // (bytes of segments and of all packets, with their room)
+        uint64_t from = ~0ull, to = 0, sum = 0, segs = 0, of_segs = 0; // (bytes of segments, with their room)
+        Layout all;
         for (uint32_t j = 0; j < n_super; j++) {
             from = std::min<uint64_t>(from, supers[j].src_off);
             to = std::max(to, (uint64_t)supers[j].src_off + supers[j].src_len);
@@ -1583,8 +1594,8 @@ int bnk_gso_split_submit(bnk_batch *b, const bnk_gso_super *supers, uint32_t n_s
         }
         from &= ~63ull;
         to = std::min<uint64_t>((to + 15) & ~15ull, b->ring_bytes);
-        ext = ring_extent(b, n_pkts, kMostRoom, &of_all);
-        const uint64_t over_link = sum + (segs < n_pkts && of_all > of_segs ? of_all - of_segs : 0);
+        ext = ring_extent(b, n_pkts, kMostRoom, &all);
+        const uint64_t over_link = sum + (segs < n_pkts && all.bytes > of_segs ? all.bytes - of_segs : 0);
         const bool in_place = sum <= kSplitInPlace && over_link <= kSplitWithPlain && host_direct(b, n_pkts, 0, over_link);
         if (in_place || (sum > kSplitInPlace && ctx->host_direct_bytes && segs == n_pkts && to - from <= 2 * sum + 65536)) {
             b->split_sealed = 0;

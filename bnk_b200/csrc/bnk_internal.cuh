@@ -335,6 +335,7 @@ struct AeadArgs {
     bool header_first;            // open of up to kRankMax packets with from_host: their headers are asked for ahead of them
     HostDesc host;                // with from_host
     uint64_t link_bytes;          // with over_link: bytes of the packets
+    bool dense;                   // with from_host: short packets, one behind the other with little between them
     uint32_t n;
     uint32_t tile;                // set by the launcher
     uint32_t mtu;

@@ -13,8 +13,19 @@
 #define BNK_BULK_TURNS (1u << 17)
 #endif
 __device__ __forceinline__ uint32_t shared_at(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void bar_init(uint64_t *bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_at(bar)) : "memory");
+__device__ __forceinline__ void bar_init(uint64_t *bar, uint32_t arrivals = 1) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_at(bar)), "r"(arrivals) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(shared_at(bar)) : "memory");
+}
+__device__ __forceinline__ bool bar_test(uint64_t *bar, uint32_t parity) { // is the phase over?
+    uint32_t over;
+    asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(over)
+                 : "r"(shared_at(bar)), "r"(parity)
+                 : "memory");
+    return over;
 }
 __device__ __forceinline__ void bar_expect(uint64_t *bar, uint32_t bytes) { // the phase ends when that many have come
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_at(bar)), "r"(bytes) : "memory");
@@ -46,6 +57,7 @@ __device__ __forceinline__ void bulk_out(void *gmem, const void *smem, uint32_t 
 }
 __device__ __forceinline__ void bulk_out_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_out_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); } // shared memory may change
+__device__ __forceinline__ void bulk_out_read_but_last() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 __device__ __forceinline__ void bulk_out_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }      // it is all where it belongs
 __device__ __forceinline__ void bulk_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
 // Between this thread's own accesses to shared memory and the bulk copies that follow.

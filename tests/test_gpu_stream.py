@@ -1,0 +1,129 @@
+"""Batches in pinned memory whose packets lie close together: several cross the link as one copy, so what is checked is where
+such a stretch begins and ends, and that nothing but the messages changes, against the CPU checker."""
+import numpy as np
+import pytest
+
+from tests import helpers as H
+from tests import reference_cases as RC
+
+pytestmark = pytest.mark.gpu
+
+LONGEST = 1969  # of the packets that go this way
+
+
+# Tiles of 4 to 16 packets, a last one that is not full; sizes whose neighbours just fill a stretch of 3200 bytes and do not (1504 and
+# 1552 with their room), the smallest and the longest, whole pieces and parts of them; packets apart, out of order, and with nothing
+# between them; 16 small ones a stretch for more CTAs.
+@pytest.mark.parametrize("mtu", [0, 1420])
+@pytest.mark.parametrize("n,sizes,gaps", [
+    (400, (1456, 1504, 1505, 1552, 1568, 1969), (0, 16)),
+    (513, (LONGEST, 0, 1, 15, 16, 17, 63, 64, 65, 1968, 1953), (0, 16, 32)),
+    (1025, (1420, 576, 64, 1419), (0, 16, 0, 0, 48)),
+    (1503, tuple(range(300, 800, 7)), (0,)),
+    (9001, (64, 40, 52, 28), (0, 16)),
+])
+def test_seal_and_open_of_neighbours(gpu_lib, oracle, n, sizes, gaps, mtu):
+    from bnk_b200 import Context
+    from bnk_b200.device import (F_ASSIGN_COUNTERS, F_DEMUX_INDEX, F_NOTE_OUTBOUND, PKT_AUTH_FAIL, PKT_BAD_DESC, PKT_COUNTER_EXHAUSTED,
+                                 PKT_MALFORMED, PKT_NO_KEYPAIR)
+    from bnk_b200.filter import CompiledRule, PortRange, flatten_rules
+
+    rng = np.random.default_rng(n + mtu)
+    peers, now = 7, RC.T0
+    keys = rng.integers(0, 256, (peers, 32), dtype=np.uint8)
+    lens = rng.choice(np.asarray(sizes, np.uint32), n)
+    lens[:len(sizes)] = sizes
+    last = lens.astype(np.int64) % mtu if mtu else lens.astype(np.int64)  # padded is the last unit, as far as the MTU
+    body = lens - last + (np.minimum((last + 15) & ~15, mtu) if mtu else (last + 15) & ~15)
+    room = ((body + 32 + 15) & ~15) + rng.choice(np.asarray(gaps), n)
+    at = np.concatenate([[0], np.cumsum(room)])
+    off, ring_bytes = at[:-1].astype(np.uint32), int(at[-1]) + 16
+    order = np.arange(n)
+    for i in rng.integers(0, n - 1, n // 25):
+        order[[i, i + 1]] = order[[i + 1, i]]
+    off, lens = off[order], lens[order]
+    slot = rng.integers(0, peers, n).astype(np.uint32)
+    refused = rng.choice(n, 6, replace=False)
+    with Context(max_keypairs=peers + 1, mtu=mtu, flow_capacity=1 << 15) as c:
+        c.set_keypairs(0, keys, keys, 100 + np.arange(peers, dtype=np.uint32))
+        c.acl_set(True, flatten_rules([CompiledRule(srcs=["10.0.0.0/8"], proto="udp", ports=[PortRange(1, 9)])]))
+        for p in range(peers):
+            c.index_set(100 + p, p)
+        b = c.batch(n, ring_bytes)
+        b.ring[:] = rng.integers(0, 256, ring_bytes, dtype=np.uint8)
+        noted = np.flatnonzero(lens >= 28)[:3000]
+        b.ring[off + 16] = 0  # no IPv4
+        for i in noted:
+            p = RC.udp(RC.SELF, RC.ip("10.0.0.0") + int(i), 7, 8)[:28]
+            b.ring[off[i] + 16:off[i] + 44] = np.frombuffer(p[:2] + int(lens[i]).to_bytes(2, "big") + p[4:], np.uint8)
+
+        def geometry(o, ln, sl):  # a place that is no place, one past the ring, no slot, a slot without keys
+            o, ln, sl = o.copy(), ln.copy(), sl.copy()
+            o[refused[0]] += 4
+            o[refused[1]] = (ring_bytes - 16) & ~15
+            sl[refused[2]], sl[refused[3]] = peers + 1, peers
+            return o, ln, sl
+
+        # ---- sealed: nonces of the caller's, then the library's own with the flows noted ----
+        plain = np.array(b.ring)
+        for own in (False, True):
+            b.ring[:] = plain
+            ctr = rng.integers(0, 2**60, n, dtype=np.uint64)
+            ctr[refused[4]] = 2**64 - 2**13 - 1
+            o, ln, sl = geometry(off, lens, slot)
+            b.off[:], b.len[:], b.slot[:] = o, ln, sl
+            if own:
+                ctr = np.array([c.send_counter(p) for p in range(peers + 1)] + [0], np.uint64)[sl] + np.array(
+                    [np.count_nonzero(sl[:i] == sl[i]) for i in range(n)], np.uint64)
+                b.seal(n, F_ASSIGN_COUNTERS | F_NOTE_OUTBOUND, now)
+                assert np.array_equal(b.counter[sl <= peers], ctr[sl <= peers])
+            else:
+                b.counter[:] = ctr
+                b.seal(n)
+            bad = refused[:4 if own else 5]
+            good = np.ones(n, bool)
+            good[bad] = False
+            want = np.zeros(n, np.uint8)
+            want[bad[:3]], want[bad[3]] = PKT_BAD_DESC, PKT_NO_KEYPAIR
+            if not own:
+                want[bad[4]] = PKT_COUNTER_EXHAUSTED
+            ring, st, length = H.oracle_seal(oracle, keys, 100 + np.arange(peers), mtu, plain, off[good], lens[good], slot[good], ctr[good])
+            assert (st == 0).all() and np.array_equal(b.status, want) and np.array_equal(b.out_len[good], length) and not b.out_len[bad].any()
+            assert np.array_equal(b.ring, ring)  # between the messages nothing has changed either
+        assert c.flows_count() == len(set(noted) - set(refused[:2]))
+
+        # ---- opened, the slot given and looked up ----
+        sealed = np.array(ring)
+        back = np.flatnonzero(good)
+        m = len(back)
+        off, slot = off[back], slot[back]
+        hurt = rng.random(m) < 0.05
+        for i in np.flatnonzero(hurt):  # anywhere behind the header
+            sealed[int(off[i]) + 16 + int(rng.integers(0, length[i] - 16))] ^= 1
+        odd = rng.choice(np.flatnonzero(~hurt), 3, replace=False)
+        sealed[off[odd[0]]] = 5              # no transport message
+        length[odd[1]] = 31                  # too short for one
+        for demux in (False, True):
+            o = off.copy()
+            o[odd[2]] += 8
+            b.ring[:] = sealed
+            b.off[:m], b.len[:m], b.slot[:m], b.slot[odd[1]] = o, length, slot, slot[odd[1]]
+            b.open(m, F_DEMUX_INDEX if demux else 0)
+            fine = np.ones(m, bool)
+            fine[odd] = False
+            ring, st, ctr, ln = H.oracle_open(oracle, keys, sealed, off[fine], length[fine], slot[fine])
+            want = np.zeros(m, np.uint8)
+            want[fine], want[odd] = st, (PKT_MALFORMED, PKT_MALFORMED, PKT_BAD_DESC)
+            assert np.count_nonzero(st == PKT_AUTH_FAIL) == np.count_nonzero(hurt)
+            assert np.array_equal(b.status[:m], want)
+            assert np.array_equal(b.out_len[:m][fine], ln) and not b.out_len[odd].any() and np.array_equal(b.counter[:m][fine], ctr)
+            if demux:
+                assert np.array_equal(b.slot[:m][fine], slot[fine])
+            ok = want == 0
+            assert H.spans_equal(np.array(b.ring), ring, off[ok], b.out_len[:m][ok], 16) == []
+            assert H.spans_differ_count(np.zeros_like(ring), np.array(b.ring), off[hurt], b.len[:m][hurt] - 32, 16) == 0  # forged: wiped
+            changed = np.zeros(ring_bytes, bool)
+            for x, k in zip(off[fine], length[fine]):
+                changed[x + 16:x + k - 16] = True
+            assert np.array_equal(np.array(b.ring)[~changed], sealed[~changed])
+        b.close()
