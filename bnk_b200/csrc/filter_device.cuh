@@ -320,6 +320,33 @@ __device__ __forceinline__ Parsed inner_parsed(const uint4 &h) {
     p.proto = (uint8_t)h.z;
     return p;
 }
+// The last checks of packet i, which has been opened, as far as they leave no trace: its status and length, and whether it still
+// depends on its flow (reply.finish).
+__device__ __forceinline__ void checks_begin(const VerdictArgs &v, uint32_t i, uint32_t slot, uint8_t &found, uint32_t &len, uint8_t &proto,
+                                             FlowReply &reply, bool &ask_flows) {
+    found = BNK_PKT_OK;
+    if (!v.inner_check && !v.check_inbound) return;
+    const uint4 h = v.inner[i];
+    const uint32_t allowed_ip = v.inner_check ? v.allowed_ip[slot] : 0u;
+    proto = (uint8_t)h.z;
+    if (v.check_inbound && v.ft.enforce) {
+        if (h.z & kInnerParses) {
+            const Parsed p = inner_parsed(h);
+            reply.begin(v.ft, p);
+            ask_flows = !rules_allow(v.ft, p);
+        } else {
+            found = BNK_PKT_FILTER_DENY;
+        }
+    }
+    if (v.inner_check) { // cut to the IPv4 total length; the source must be the peer's address
+        if ((h.z & kInnerWhole) && h.x != 0 && h.x == allowed_ip) {
+            len = h.w;
+        } else {
+            found = BNK_PKT_BAD_INNER;
+            ask_flows = false;
+        }
+    }
+}
 __device__ __forceinline__ void final_verdict(const VerdictArgs &v, uint32_t i) {
     uint8_t st = *(volatile uint8_t *)&v.status[i];
     uint32_t l = v.out_len[i];

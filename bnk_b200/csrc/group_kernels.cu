@@ -645,16 +645,20 @@ struct GroupArgs {
     // counters (send_counter != nullptr)
     SendCounter *send_counter;
     uint64_t *counter_out; // per packet
-    // replay window (replay): rp.keys and rp.order are written here
-    uint32_t *keys_out, *order_out;
+    // replay window (replay): rp.keys are written here
+    uint32_t *keys_out;
     ReplayArgs rp;
     bool replay;
     VerdictArgs verdict; // n == 0: none
     Done done;
 };
 
+// A packet behind its window's top looks through so many of its peer's packets in front of it for its counter; only where that is
+// not all of them is the table of positions built.  Opened with everything on, us with the table always / so: 2068 mixed packets of 256
+// peers 88 / 82, 4136 109 / 103, 10,100 201 / 193, 16,160 of 1000 peers 287 / 262; of 8 peers, whose runs are longer, 4136 106 / 112.
+constexpr uint32_t kLookBack = 64;
 template <int ITEMS>
-__global__ void __launch_bounds__(kGroupThreads) group_kernel(const __grid_constant__ GroupArgs a) {
+__global__ void __launch_bounds__(kGroupThreads, 1) group_kernel(const __grid_constant__ GroupArgs a) {
     let_next_kernel_start();    // seal side: the seal launch behind may take its place already
     wait_for_kernel_in_front(); // open side: statuses and counters come from the open launch in front
     constexpr uint32_t kChunk = kGroupThreads * ITEMS; // positions per CTA
@@ -674,6 +678,8 @@ __global__ void __launch_bounds__(kGroupThreads) group_kernel(const __grid_const
     };
     const uint32_t first = me * kChunk; // this CTA's positions (and, before the sort, its packets)
     const uint32_t mine = a.n > first ? min(kChunk, a.n - first) : 0u;
+    if (a.replay) // (in case some packet turns out to need the table)
+        for (uint32_t i = me * kGroupThreads + tid; i <= a.rp.mask; i += ctas * kGroupThreads) a.rp.table[i] = kHashEmpty;
 
     // ---- sort ----
     uint32_t f = 0; // which buffer holds the result
@@ -826,19 +832,39 @@ __global__ void __launch_bounds__(kGroupThreads) group_kernel(const __grid_const
             if (tail[k] && slot[k] < a.max_slots) counter_store(&a.send_counter[slot[k]].e[counter[k].at], counter[k].now);
     }
 
+    // The window and the last checks wait for memory and for one another, so a thread keeps what it knows of its positions, asks
+    // for all that nothing else has to be known for in front of a barrier, and the barriers are as few as the window's definition
+    // wants: one for the running maximum, one behind the reads of the old window, one behind its move, one to put the results in
+    // the packets' order.  (Each phase reading what the one before had left in memory, with a thread of its own: 2068 packets of 256
+    // peers 33 us from the open kernel's end, now 22.)
     if (a.replay) {
         const ReplayArgs &r = a.rp;
-        uint64_t c[ITEMS], e[ITEMS], v[ITEMS];
+        const uint64_t rmask = r.ring_blocks - 1, window = (uint64_t)(r.ring_blocks - 1) * 64u;
+        uint64_t c[ITEMS], e[ITEMS], v[ITEMS], last[ITEMS];
+        uint32_t pkt[ITEMS];
+        uint8_t had[ITEMS], st[ITEMS]; // the packet's status so far; what the window says
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) { // asked for together
+            pkt[k] = 0;
+            c[k] = last[k] = 0;
+            had[k] = BNK_PKT_BAD_DESC;
+            if (at0 + k >= mine) continue;
+            pkt[k] = vbuf(f)[at0 + k];
+            had[k] = r.status[pkt[k]];
+            c[k] = r.counter[pkt[k]];
+            if (slot[k] < r.max_slots) last[k] = r.replay_last[slot[k]];
+        }
 #pragma unroll
         for (int k = 0; k < ITEMS; k++) {
-            c[k] = kReplayNoPart;
-            v[k] = 0;
+            const bool authentic = at0 + k < mine && slot[k] < r.max_slots && (had[k] == BNK_PKT_OK || had[k] == BNK_PKT_KEEPALIVE);
+            st[k] = authentic && c[k] >= BNK_REJECT_AFTER_MESSAGES ? RP_REJECT : RP_NOPART; // (whatever the window holds, and without a trace)
+            if (!authentic || st[k] == RP_REJECT) c[k] = kReplayNoPart;
+            v[k] = c[k] != kReplayNoPart ? c[k] : 0ull;
             if (at0 + k < mine) {
-                const uint32_t pkt = vbuf(f)[at0 + k], p = first + at0 + k;
-                a.keys_out[p] = slot[k];
-                a.order_out[p] = pkt;
-                c[k] = replay_gather(r, p, slot[k], pkt);
-                if (c[k] != kReplayNoPart) v[k] = c[k];
+                a.keys_out[first + at0 + k] = slot[k];
+                r.sorted_counter[first + at0 + k] = c[k];
+                kbuf(f ^ 1u)[at0 + k] = (uint32_t)c[k]; // the counters in grouped order, beside the slots in kbuf(f)
+                vbuf(f ^ 1u)[at0 + k] = (uint32_t)(c[k] >> 32);
             }
         }
         SegMax total;
@@ -853,38 +879,109 @@ __global__ void __launch_bounds__(kGroupThreads) group_kernel(const __grid_const
         tile_carry<ITEMS>(t, reached.m, e);
         bool pending = false;
 #pragma unroll
-        for (int k = 0; k < ITEMS; k++) {
-            if (at0 + k >= mine) continue;
-            const uint8_t st = replay_classify(r, first + at0 + k, slot[k], tail[k], c[k], e[k]);
-            r.state[first + at0 + k] = st;
-            pending |= st == RP_PENDING;
-        }
-        if (__syncthreads_or(pending) && tid == 0) cta_pending = 1;
-        all_sync(); // every verdict and next `last` is written
-        bool any_pending = false;
-        for (uint32_t q = 0; q < ctas; q++) any_pending |= (ctas > 1 ? *cluster.map_shared_rank(&cta_pending, q) : cta_pending) != 0;
-        for (uint32_t i = tid; i < kChunk; i += kGroupThreads) replay_advance_warp(r, i < mine ? first + i : a.n);
-        if (any_pending) {
-            for (uint32_t i = me * kGroupThreads + tid; i <= r.mask; i += ctas * kGroupThreads) r.table[i] = kHashEmpty;
-            all_sync();
-            for (uint32_t i = tid; i < kChunk; i += kGroupThreads) {
-                const uint32_t p = first + i;
-                replay_hash_insert_warp(r, p, i < mine && r.state[p] != RP_NOPART);
+        for (int k = 0; k < ITEMS; k++) { // e becomes the peer's `last` behind this packet
+            e[k] = e[k] > last[k] ? e[k] : last[k];
+            if (c[k] == kReplayNoPart) continue;
+            if (c[k] > e[k]) {
+                st[k] = RP_ACCEPT;
+                e[k] = c[k];
+            } else if (e[k] - c[k] > window ||
+                       (c[k] <= last[k] && ((r.replay_ring[(size_t)slot[k] * r.ring_blocks + ((c[k] >> 6) & rmask)] >> (c[k] & 63u)) & 1ull))) {
+                st[k] = RP_REJECT;
+            } else { // accepted unless an earlier packet of the run has the same counter
+                st[k] = RP_PENDING;
+                const uint32_t at = at0 + k; // of this CTA; what lies in front of it is the end of the one before
+                const auto looks = [&](const uint32_t *keys, const uint32_t *lo, const uint32_t *hi, uint32_t from, uint32_t to) {
+#pragma unroll 1
+                    for (uint32_t q = from; q-- > to;) {
+                        if (keys[q] != slot[k]) return RP_ACCEPT; // the run has started behind it
+                        if (lo[q] == (uint32_t)c[k] && hi[q] == (uint32_t)(c[k] >> 32)) return RP_REJECT;
+                    }
+                    return RP_PENDING;
+                };
+                const uint32_t *const keys = at >= kLookBack || me == 0 ? kbuf(f) : cluster.map_shared_rank(kbuf(f), me - 1);
+                if (first + at < kLookBack || keys[(at - kLookBack) % kChunk] != slot[k]) { // the run starts within reach
+                    st[k] = looks(kbuf(f), kbuf(f ^ 1u), vbuf(f ^ 1u), at, at > kLookBack ? at - kLookBack : 0u);
+                    if (st[k] == RP_PENDING && me > 0)
+                        st[k] = looks(cluster.map_shared_rank(kbuf(f), me - 1), cluster.map_shared_rank(kbuf(f ^ 1u), me - 1),
+                                      cluster.map_shared_rank(vbuf(f ^ 1u), me - 1), kChunk, kChunk - (kLookBack - at));
+                    if (st[k] == RP_PENDING) st[k] = RP_ACCEPT; // (it is the batch's first)
+                }
+                pending |= st[k] == RP_PENDING;
             }
         }
+        if (__syncthreads_or(pending) && tid == 0) cta_pending = 1;
+        all_sync(); // `last` and the rings are read
+        bool any_pending = false;
+        for (uint32_t q = 0; q < ctas; q++) any_pending |= (ctas > 1 ? *cluster.map_shared_rank(&cta_pending, q) : cta_pending) != 0;
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) { // the peers whose run ends here move their window, a lane each but for large steps
+            const bool moves = tail[k] && slot[k] < r.max_slots;
+            const uint64_t from = last[k] >> 6, passed = (e[k] >> 6) - from, steps = !moves ? 0u : passed < r.ring_blocks ? passed : r.ring_blocks;
+            uint64_t *const ring = r.replay_ring + (moves ? (size_t)slot[k] * r.ring_blocks : 0u);
+            if (steps <= 8)
+                for (uint64_t i = 1; i <= steps; i++) ring[(from + i) & rmask] = 0ull;
+            uint32_t large = __ballot_sync(0xffffffffu, steps > 8);
+            while (large) {
+                const uint32_t src = __ffs(large) - 1;
+                large &= large - 1;
+                uint64_t *const of = reinterpret_cast<uint64_t *>(__shfl_sync(0xffffffffu, (unsigned long long)ring, src));
+                const uint64_t at = __shfl_sync(0xffffffffu, from, src), many = __shfl_sync(0xffffffffu, steps, src);
+                for (uint64_t i = lane + 1; i <= many; i += 32) of[(at + i) & rmask] = 0ull;
+            }
+            if (moves) r.replay_last[slot[k]] = e[k];
+            if (any_pending) replay_hash_insert_warp(r, first + at0 + k, c[k] != kReplayNoPart);
+        }
+        // The last checks want much of memory too, and none of it depends on what is being written.
+        const VerdictArgs &w = a.verdict;
+        uint32_t len[ITEMS], whole[ITEMS];
+        uint8_t found[ITEMS], proto[ITEMS];
+        FlowReply reply[ITEMS];
+        bool ask_flows[ITEMS];
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            len[k] = whole[k] = proto[k] = 0;
+            found[k] = had[k];
+            ask_flows[k] = false;
+            if (w.n == 0 || at0 + k >= mine) continue;
+            len[k] = whole[k] = w.out_len[pkt[k]];
+            if (had[k] == BNK_PKT_OK && st[k] != RP_REJECT) checks_begin(w, pkt[k], slot[k], found[k], len[k], proto[k], reply[k], ask_flows[k]);
+        }
         all_sync(); // clears before marks, inserts before look-ups
-        for (uint32_t i = tid; i < kChunk; i += kGroupThreads) replay_finish_warp(r, i < mine ? first + i : a.n);
-        if (a.verdict.n) all_sync(); // every refusal is written
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            if (st[k] == RP_PENDING) st[k] = replay_hash_has_earlier(r, first + at0 + k, slot[k], c[k]) ? RP_REJECT : RP_ACCEPT;
+            replay_mark_warp(r, st[k] == RP_ACCEPT, slot[k], c[k]);
+            if (at0 + k >= mine) continue;
+            if (st[k] == RP_REJECT) {
+                found[k] = BNK_PKT_REPLAY;
+                len[k] = whole[k];
+            } else if (ask_flows[k]) {
+                found[k] = reply[k].finish(w.ft, proto[k], w.now);
+            }
+            r.status[pkt[k]] = found[k];
+            if (w.n == 0) continue;
+            w.out_len[pkt[k]] = len[k];
+            if (w.host_status) { // to whose packet it is, so that what goes to the host goes in whole lines
+                const uint32_t to = pkt[k] / kChunk, at = pkt[k] % kChunk;
+                (ctas > 1 ? cluster.map_shared_rank(kbuf(f ^ 1u), to) : kbuf(f ^ 1u))[at] = len[k];
+                (ctas > 1 ? cluster.map_shared_rank(vbuf(f ^ 1u), to) : vbuf(f ^ 1u))[at] = found[k];
+            }
+        }
+        if (w.n && w.host_status) {
+            all_sync();
+            for (uint32_t i = tid; i < mine; i += kGroupThreads) {
+                w.host_status[first + i] = (uint8_t)vbuf(f ^ 1u)[i];
+                w.host_out_len[first + i] = kbuf(f ^ 1u)[i];
+            }
+        }
     }
-    if (a.verdict.n)
-        for (uint32_t i = tid; i < mine; i += kGroupThreads) final_verdict(a.verdict, first + i);
-    if (ctas > 1) cluster.sync(); // nobody leaves while another may still look into its shared memory
+    // (Nobody has looked into another's shared memory since the last barrier.)
     signal_done(a.done, false, [] {});
 }
 
 // --- what follows the open kernel of up to kTailMax packets -----------------------------
-// Here nothing but latency counts, and group_kernel's phases hand each other their results through memory: 10 us for 9
-// packets, 36 for 129 with a hundred rules.  In this one CTA eight warps group the packets and run the replay window
+// Here nothing but latency counts, and group_kernel's phases wait for one another.  In this one CTA eight warps group the packets and run the replay window
 // in registers and shared memory, while the other eight already look the packets' flows and rules up; who judges a
 // packet then has everything in hand.
 constexpr uint32_t kTailMax = 256;
@@ -985,23 +1082,7 @@ __global__ void __launch_bounds__(512) open_tail_kernel(const __grid_constant__ 
         if (i < n) {
             st = *(const volatile uint8_t *)&v.status[i];
             l = len = v.out_len[i];
-            if (st == BNK_PKT_OK && (v.inner_check || v.check_inbound)) {
-                const uint4 h = v.inner[i];
-                proto = (uint8_t)h.z;
-                if (v.check_inbound && v.ft.enforce) {
-                    if (h.z & kInnerParses) {
-                        const Parsed p = inner_parsed(h);
-                        reply.begin(v.ft, p);
-                        ask_flows = !rules_allow(v.ft, p);
-                    } else {
-                        found = BNK_PKT_FILTER_DENY;
-                    }
-                }
-                if (v.inner_check) { // cut to the IPv4 total length; the source must be the peer's address
-                    if ((h.z & kInnerWhole) && h.x != 0 && h.x == v.allowed_ip[slots[i]]) len = h.w;
-                    else found = BNK_PKT_BAD_INNER;
-                }
-            }
+            if (st == BNK_PKT_OK) checks_begin(v, i, slots[i], found, len, proto, reply, ask_flows);
         }
         __syncthreads();
         if (i < n) {
@@ -1281,7 +1362,6 @@ cudaError_t launch_open_tail(bnk_batch *b, uint32_t n, bool replay, const Verdic
     g.digit_bits = plan.digit_bits;
     g.max_slots = ctx->cfg.max_keypairs;
     g.keys_out = d.keys_tmp + b->max_pkts;
-    g.order_out = d.order;
     g.rp = replay_args(b, n);
     g.replay = true;
     if (verdict) g.verdict = *verdict;

@@ -300,3 +300,45 @@ def test_send_counters_small_batches(gpu_lib, n):
         b.close()
     finally:
         c.close()
+
+
+# One CTA, then clusters of them with one and two packets a thread: runs are cut anywhere by the CTAs' shares of the grouped order.
+@pytest.mark.parametrize("n", [1000, 2049, 9000])
+@pytest.mark.parametrize("most", [66, 64, 300])
+def test_replay_of_runs_about_as_long_as_a_look_back(gpu_lib, oracle, n, most):
+    """Peers with one packet to `most`: the last packets of a run repeat its first, its second and its last but one, or come late
+    for the first time, so an earlier copy lies 60 to 65 packets in front, or a run's length away, or nowhere."""
+    from bnk_b200 import Context
+    from bnk_b200.device import F_REPLAY
+
+    rng = np.random.default_rng(n + most)
+    runs, left = [], n
+    while left:
+        runs.append(min(left, int(rng.integers(62, most + 1)) if most < 100 or rng.random() < 0.5 else int(rng.integers(1, most + 1))))
+        left -= runs[-1]
+    peers = len(runs)
+    keys = rng.integers(0, 256, (peers, 32), dtype=np.uint8)
+    slots = rng.permutation(np.repeat(np.arange(peers, dtype=np.uint32), runs))
+    counters = np.zeros(n, np.uint64)
+    for s in range(peers):
+        at = np.flatnonzero(slots == s)
+        c = 1000 + 2 * np.arange(len(at))
+        if len(at) > 6:
+            c[-1], c[-2], c[-3], c[-4] = c[0], c[1], c[-5], 1001
+        counters[at] = c
+    with Context(max_keypairs=peers, replay_ring_blocks=32, mtu=0, flow_capacity=0) as c:
+        c.set_keypairs(0, keys, keys, np.ones(peers, np.uint32))
+        msgs, lengths, off = _sealed_ring(oracle, keys, slots, counters, np.full(n, 16), rng)
+        b = c.batch(n, H.ring_bytes_for(off, lengths))
+        state = {}
+        for turn in range(2):  # and once more: all of them are marked
+            H.fill_payloads(b.ring, off, msgs, headroom=0)
+            b.off[:], b.len[:], b.slot[:] = off, lengths, slots
+            _, st, ctr, _ = H.oracle_open(oracle, keys, b.ring, off, lengths, slots)
+            want, state = H.oracle_replay(oracle, 32, slots, ctr, st, state)
+            b.open(n, F_REPLAY)
+            assert np.array_equal(b.status, want), np.flatnonzero(b.status != want)[:8]
+        for s in range(0, peers, 7):
+            last, ring = c.replay_export(s)
+            assert last == state[s].last and np.array_equal(ring, state[s].ring())
+        b.close()
