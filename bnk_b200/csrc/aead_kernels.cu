@@ -714,7 +714,7 @@ __device__ __forceinline__ void note_head(FlowNote &note, const AeadArgs &a, con
     }
 }
 // What the last checks want of the plaintext of `body` bytes that starts at stage[piece].
-__device__ __forceinline__ void inner_head(const AeadArgs &a, const uint4 *stage, uint32_t piece, uint32_t body, size_t pkt) {
+__device__ __forceinline__ uint4 inner_head(const AeadArgs &a, const uint4 *stage, uint32_t piece, uint32_t body) {
     const uint32_t word = stage_word(stage, piece);
     const uint32_t w0 = __shfl_sync(0xffffffffu, word, 0), w3 = __shfl_sync(0xffffffffu, word, 3);
     const uint32_t total = ((w0 >> 8) & 0xff00u) | (w0 >> 24); // bytes 2,3 big-endian
@@ -724,9 +724,8 @@ __device__ __forceinline__ void inner_head(const AeadArgs &a, const uint4 *stage
                                          a.inner_cut && is_whole ? total : body, p);
     const uint32_t ports = __shfl_sync(0xffffffffu, word, (at >> 2) & 15u);
     if (at != kParseBad && at) parse_ports(ports, p);
-    if ((threadIdx.x & 31) == 0)
-        a.inner[pkt] = make_uint4(__byte_perm(w3, 0, 0x0123), (uint32_t)p.sport << 16 | p.dport,
-                                  p.proto | (at != kParseBad ? kInnerParses : 0u) | (is_whole ? kInnerWhole : 0u), total);
+    return make_uint4(__byte_perm(w3, 0, 0x0123), (uint32_t)p.sport << 16 | p.dport,
+                      p.proto | (at != kParseBad ? kInnerParses : 0u) | (is_whole ? kInnerWhole : 0u), total);
 }
 
 template <bool OPEN, bool NOTE, uint32_t INLINE>
@@ -1027,7 +1026,10 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
                     stage[0] = make_uint4(4u, remote, n_lo, n_hi);
                 }
                 __syncwarp();
-                if (OPEN && a.inner && rnd == 0 && !forged) inner_head(a, stage, rd.body, body, (size_t)t * T + k);
+                if (OPEN && a.inner && rnd == 0 && !forged) {
+                    const uint4 inner = inner_head(a, stage, rd.body, body);
+                    if (lane == 0) a.inner[(size_t)t * T + k] = inner;
+                }
                 // The last piece goes out whole where the bytes behind the message were read from the same place.
                 const uint32_t out_bytes = OPEN ? rb : rb + (last ? BNK_WG_TAG : 0u);
                 const bool other_place = a.in != a.out;
@@ -1310,6 +1312,8 @@ __device__ __forceinline__ void stream_work(const AeadArgs &a, StreamShared &sh,
         if (!bar_wait_warp(&sh.ready[s], parity)) return;
         const uint32_t count = r.count;
         if (count == 0) return;
+        uint4 inner = make_uint4(0, 0, 0, 0); // the n-th of this run's plaintexts of this warp in lane n
+        uint32_t inner_of = 0, n_inner = 0;
 #pragma unroll 1
         for (uint32_t k = (worker + kStreamWorkers - r.turn) % kStreamWorkers; k < count; k += kStreamWorkers) {
             const uint32_t off = r.off[k], len = r.len[k], pkt = r.first + k;
@@ -1410,7 +1414,14 @@ __device__ __forceinline__ void stream_work(const AeadArgs &a, StreamShared &sh,
                     });
                     if (!OPEN && lane == 0) stage[0] = make_uint4(4u, remote, n_lo, n_hi);
                     __syncwarp();
-                    if (OPEN && a.inner && !forged) inner_head(a, stage, 1, body, pkt);
+                    if (OPEN && a.inner && !forged) {
+                        const uint4 v = inner_head(a, stage, 1, body);
+                        if (lane == n_inner) {
+                            inner = v;
+                            inner_of = pkt;
+                        }
+                        n_inner++;
+                    }
                 }
             }
             if (NOTE) note.count(a.ft);
@@ -1427,6 +1438,14 @@ __device__ __forceinline__ void stream_work(const AeadArgs &a, StreamShared &sh,
         bulk_fence_shared();
         __syncwarp();
         if (lane == 0) bar_arrive(&sh.over[s]);
+        // The rules are asked while the link is busy, and nothing waits for the answer but the last checks: 10,100 mixed packets opened
+        // with everything on 190 us, with the rules asked there 193, 16,160 259 and 262.
+        if (OPEN && lane < n_inner) {
+            if (a.judge && (inner.z & kInnerParses))
+                inner.z |= kInnerJudged | (rules_allow(a.ft, inner_parsed(inner)) ? kInnerAllowed : 0u);
+            a.inner[inner_of] = inner;
+        }
+        __syncwarp();
         if (++s == kStreamStages) {
             s = 0;
             parity ^= 1u;
@@ -1525,11 +1544,13 @@ cudaError_t launch_wpp(const AeadArgs &a, uint32_t ctas, const HostDesc *h, cuda
 // and 148.0, but 4096 x 1420 B opened 197 and 188, 12,000 518 and 500; small ones 9000 x 64 B 80 and 73.
 // Sealed, kernel 2 and this one: 1024 x 1420 B 66 us and 61, 4096 201 and 183, 12,000 535 and 490, 9000 x 64 B 83 and 74, whole path
 // 10,000 mixed 176 and 158.
-constexpr uint64_t kStreamFrom = 512u << 10, kStreamOpenFrom = 4u << 20;
+// 2048 mixed packets (840 KB) are on the line: sealed 47 us, 45 to 50.
+constexpr uint64_t kStreamFrom = 512u << 10, kStreamSmallFrom = 896u << 10, kStreamOpenFrom = 4u << 20;
 constexpr uint32_t kStreamCtas = 96, kStreamCtasSmall = 148, kStreamTiles = 64, kSmallPacket = 512;
 bool small_packets(const AeadArgs &a) { return a.link_bytes <= (uint64_t)kSmallPacket * a.n; }
 bool in_stream(const AeadArgs &a, bool open) {
-    return a.from_host && a.dense && a.n > kRankMax && a.link_bytes >= (open && !small_packets(a) ? kStreamOpenFrom : kStreamFrom);
+    const uint64_t from = open == small_packets(a) ? kStreamFrom : open ? kStreamOpenFrom : kStreamSmallFrom;
+    return a.from_host && a.dense && a.n > kRankMax && a.link_bytes >= from;
 }
 void stream_grid(AeadArgs &a, uint32_t &ctas) {
     const uint32_t most = small_packets(a) ? kStreamCtasSmall : kStreamCtas;

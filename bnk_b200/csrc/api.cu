@@ -1269,6 +1269,8 @@ static int open_direct(bnk_batch *b, uint32_t npkts, const Layout &lay, uint32_t
         a.res[1] = AeadResults{b->dev.counter, b->dev.out_len, b->dev.status, b->dev.slot};
         if (checks) a.inner = b->dev.inner;
         a.inner_cut = (flags & BNK_F_INNER_CHECK) != 0;
+        a.ft = ctx->ft;
+        a.judge = (flags & BNK_F_CHECK_INBOUND) && ctx->ft.enforce;
     } else if (stats) {
         a.res[1] = AeadResults{nullptr, b->dev.out_len, b->dev.status, nullptr};
     }

@@ -298,6 +298,7 @@ __device__ __forceinline__ uint8_t filter_verdict(const FilterTables &ft, const 
 //   x source address   y source port << 16 | destination port   z protocol | flags   w IPv4 total length
 constexpr uint32_t kInnerParses = 1u << 8; // filter.parse accepts it
 constexpr uint32_t kInnerWhole = 1u << 9;  // IPv4, 20 <= total length <= decrypted length
+constexpr uint32_t kInnerJudged = 1u << 10, kInnerAllowed = 1u << 11; // the rules have been asked already, and allow it
 struct VerdictArgs {
     FilterTables ft;
     const uint4 *inner;
@@ -333,7 +334,7 @@ __device__ __forceinline__ void checks_begin(const VerdictArgs &v, uint32_t i, u
         if (h.z & kInnerParses) {
             const Parsed p = inner_parsed(h);
             reply.begin(v.ft, p);
-            ask_flows = !rules_allow(v.ft, p);
+            ask_flows = !((h.z & kInnerJudged) ? (h.z & kInnerAllowed) != 0 : rules_allow(v.ft, p));
         } else {
             found = BNK_PKT_FILTER_DENY;
         }
