@@ -61,7 +61,7 @@ struct KeypairTables {
 
 // The allowances of one prefix.  Port ranges (first << 16 | last) are disjoint and in rising order; those of tcp and those
 // of udp each start at a multiple of four in rule_ports and are filled up with kNoPorts to one.
-struct alignas(16) RuleGroup {
+struct alignas(32) RuleGroup {
     uint32_t addr, len;         // the prefix (hash table: len 0 = an empty place)
     uint32_t parent;            // the longest shorter prefix with allowances that contains this one, + 1; bit 31: icmp is allowed
     uint32_t n_ports;           // tcp's ranges | udp's << 16

