@@ -1482,7 +1482,8 @@ __global__ void __launch_bounds__(32 * kStreamWarps, 1) aead_stream_kernel(const
 #endif
 
 // Tiles and grid of a warp-per-packet launch.  Rings in device memory (n <= BNK_WPP_MAX_PACKETS): a warp per packet.
-// Rings in host memory: the link is the bound.  With a warp per packet all reads are asked for at once, end together and
+// Rings in host memory: the link is the bound (and packets that lie close together go through kernel 3, see in_stream; the figures here
+// are of 1472 bytes apart, as longer ones and ones further apart behave).  With a warp per packet all reads are asked for at once, end together and
 // leave the writes for afterwards, so beyond kLinkWindow bytes a warp takes several packets: 1024 x 1420 B sealed by
 // 32 to 96 CTAs 72 us, by 128 84, by 256 (a packet each) 92; 512 x 1420 46 against 54.  Small packets are bound by what
 // a warp computes, and want more warps: 4096 x 300 B 104 us from 64 CTAs, 77 from 128 to 192, 92 from 512; 131,072 x 64 B
