@@ -1,5 +1,5 @@
 """Batches in pinned memory whose packets lie close together: several cross the link as one copy, so what is checked is where
-such a stretch begins and ends, and that nothing but the messages changes, against the CPU checker."""
+such a stretch begins and ends, and that nothing but the messages changes, against the oracle."""
 import numpy as np
 import pytest
 
