@@ -1117,7 +1117,8 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
 // There the link is the bound (without any cipher work kernel 2 takes as long), and what counts is how it is asked: in whole
 // lines, few of them twice, and with about half a megabyte outstanding in all.  So the first warp brings neighbouring packets up
 // as one copy, up to kStreamRun bytes of them, into one of kStreamStages stages, the other warps take the packets of a stage one
-// by one, and the whole stretch goes back as one copy: bytes between packets as they were read.  The warps that compute are as
+// by one, and the whole stretch goes back as one copy: bytes between packets as they were read.  Packets that are refused stay out of
+// it, as their descriptors may name bytes of another packet, which has been worked on meanwhile.  The warps that compute are as
 // many whatever the size of the packets, which a warp that fetched for itself could not have: with kernel 2's warp for each few
 // packets either the requests of all of them are on the link at once, and the writes come afterwards, or small packets wait
 // for warps.  At most kStreamAhead copies of a CTA are on their way up, however many of its stages are worked on.
@@ -1141,10 +1142,10 @@ struct StreamRun { // neighbours in a stage
     uint32_t bytes;        // in the stage; 0: of a packet that lies outside of the ring
     uint32_t turn;         // the worker that takes the first
     bool asked, ends_tile; // asked: the bytes are, or were, on their way
-    uint32_t off[32], len[32], slot[32];
+    uint32_t off[32], len[32], slot[32], end[32];
     uint64_t counter[32]; // of a seal; then the results
     uint32_t out_len[32];
-    uint8_t status[32], has_counter[32];
+    uint8_t status[32], has_counter[32], worked_on[32];
 };
 struct StreamShared {
     alignas(128) uint4 stage[kStreamStages][(kStreamRun + 64) / 16]; // (a look at a packet's head may go 64 bytes beyond its start)
@@ -1214,6 +1215,7 @@ __device__ __forceinline__ void stream_feed(const AeadArgs &a, StreamShared &sh)
             r.off[lane - j] = cur.off;
             r.len[lane - j] = cur.len;
             r.slot[lane - j] = cur.slot;
+            r.end[lane - j] = end;
             if (!OPEN) r.counter[lane - j] = cur.ctr;
         }
         if (lane == 0) {
@@ -1257,8 +1259,13 @@ __device__ __forceinline__ void stream_feed(const AeadArgs &a, StreamShared &sh)
         // (No worker waits for a packet that is refused for its descriptor; and where one has given up, the bytes are as they came.)
         const bool whole = __any_sync(0xffffffffu, r.asked && bar_wait(&sh.full[sent % kStreamStages], sent / kStreamStages & 1u));
         if (!whole) fetches = false;
+        const uint32_t goes = __ballot_sync(0xffffffffu, whole && lane < count && r.worked_on[lane]);
         if (lane == 0) {
-            if (whole && r.bytes) bulk_out(a.out + r.base, sh.stage[sent % kStreamStages], r.bytes);
+            for (uint32_t left = goes; left;) { // as a rule one copy of all of them
+                const uint32_t k = __ffs(left) - 1, many = __ffs(~(left >> k)) - 1, from = r.off[k] - r.base; // (a run has at most 16)
+                bulk_out(a.out + r.off[k], sh.stage[sent % kStreamStages] + from / 16, r.end[k + many - 1] - r.off[k]);
+                left &= ~(((1u << many) - 1u) << k);
+            }
             bulk_out_commit();
         }
         if (r.ends_tile && lane < first + count) {
@@ -1433,6 +1440,7 @@ __device__ __forceinline__ void stream_work(const AeadArgs &a, StreamShared &sh,
                 r.slot[k] = slot;
                 r.counter[k] = ctr;
                 r.has_counter[k] = has_counter;
+                r.worked_on[k] = st == BNK_PKT_OK && !broken;
             }
         }
         bulk_fence_shared();

@@ -27,7 +27,10 @@
  *     library.  A batch that asks for both copies and is alone in flight, or small
  *     enough beside others, is not copied at all: the kernels read and write the
  *     pinned arrays in place (up to a ring extent of BNK_HOST_DIRECT_BYTES from the
- *     environment, 0 = never).  The results are the same bytes.  What such a submit
+ *     environment, 0 = never).  The results are the same bytes; of the ring, what lies
+ *     between two packets of the batch may be written as well, as it was read.  A packet
+ *     that is refused for its descriptor or its keypair is not written, and may name
+ *     bytes of another one.  What such a submit
  *     works on is not on the device behind it: a call with BNK_F_NO_H2D that follows
  *     brings it there first, so the host arrays stay as they are until that call.
  *   - A program's first submit of a kind (call, options, size class) loads its kernels,

@@ -127,3 +127,45 @@ def test_seal_and_open_of_neighbours(gpu_lib, oracle, n, sizes, gaps, mtu):
                 changed[x + 16:x + k - 16] = True
             assert np.array_equal(np.array(b.ring)[~changed], sealed[~changed])
         b.close()
+
+
+@pytest.mark.parametrize("n,size", [(4096, 1420), (9000, 64)])
+def test_refused_descriptors_may_name_bytes_of_others(gpu_lib, oracle, n, size):
+    """Some descriptors of a batch are placeholders that are refused, of no slot or of one without keys, and name a place at which
+    another packet lies.  That packet is sealed and opened as if they were not there, whichever of the two is looked at first."""
+    from bnk_b200 import Context
+    from bnk_b200.device import PKT_BAD_DESC, PKT_NO_KEYPAIR
+
+    rng = np.random.default_rng(n)
+    peers, step = 5, (size + 47) // 16 * 16
+    keys = rng.integers(0, 256, (peers, 32), dtype=np.uint8)
+    good = rng.random(n) < 0.8
+    off = np.zeros(n, np.uint32)
+    off[good] = np.arange(good.sum()) * step
+    # what a placeholder names: the first packet of the ring, the one behind its neighbour in front, or any
+    names = rng.choice(3, n)
+    behind = np.minimum(np.cumsum(good), good.sum() - 1) * step
+    off[~good] = np.choose(names, [np.zeros(n), behind, rng.integers(0, good.sum(), n) * step])[~good]
+    slot = np.where(good, rng.integers(0, peers, n), peers + rng.integers(0, 2, n)).astype(np.uint32)
+    refused = np.where(slot == peers, PKT_NO_KEYPAIR, PKT_BAD_DESC)[~good]
+    with Context(max_keypairs=peers + 1, mtu=0, flow_capacity=0) as c:
+        c.set_keypairs(0, keys, keys, np.arange(peers, dtype=np.uint32))
+        b = c.batch(n, int(good.sum()) * step)
+        for rep in range(8):
+            b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
+            b.off[:], b.len[:], b.slot[:] = off, np.where(good, size, rng.choice([0, size], n)), slot
+            b.counter[:] = rng.integers(0, 2**60, n, dtype=np.uint64)
+            ctr = np.array(b.counter)
+            ring, st, ln = H.oracle_seal(oracle, keys, np.arange(peers), 0, b.ring, off[good], b.len[good], slot[good], ctr[good])
+            b.seal(n)
+            assert np.array_equal(b.status[good], st) and np.array_equal(b.status[~good], refused)
+            assert np.array_equal(b.out_len[good], ln) and not b.out_len[~good].any()
+            assert np.array_equal(b.ring, ring), rep
+            b.len[:] = step
+            want, st, got, ln = H.oracle_open(oracle, keys, ring, off[good], b.len[good], slot[good])
+            assert (st == 0).all()
+            b.open(n)
+            assert np.array_equal(b.status[good], st) and np.array_equal(b.status[~good], refused)
+            assert np.array_equal(b.out_len[good], ln) and np.array_equal(b.counter[good], got)
+            assert H.spans_differ_count(np.array(b.ring), want, off[good], ln, 16) == 0, rep
+        b.close()
