@@ -110,20 +110,22 @@ def build_mt_stress(force: bool = False) -> str:
     return _build_cpp(os.path.join(HOST, "apps", "mt_stress.cpp"), os.path.join(HOST, "apps", "mt_stress"), force)
 
 
-LOST_BYTES, LOST_TURNS = 720, 64
+LOST_BYTES, LOST_TURNS, SOON = 720, 64, 40
 
 
-def lost_copies_path() -> str:
-    return os.path.join(os.path.dirname(PKG_DIR), "build", "lost_copies", "libbnkgpu.so")
+def lost_copies_path(gives_up: bool = False) -> str:
+    return os.path.join(os.path.dirname(PKG_DIR), "build", "gives_up" if gives_up else "lost_copies", "libbnkgpu.so")
 
 
-def build_lost_copies(force: bool = False) -> str:
+def build_lost_copies(force: bool = False, gives_up: bool = False) -> str:
     """libbnkgpu.so for the tests of what happens when a copy over the link does not come: its kernels never ask for bulk
-    copies of LOST_BYTES, and their waits give up after LOST_TURNS turns."""
-    lib = lost_copies_path()
+    copies of LOST_BYTES, and their waits give up after LOST_TURNS turns.  With gives_up the warp that hands packets out
+    gives up after SOON turns without anything to do, which is before most copies can have come."""
+    lib = lost_copies_path(gives_up)
     if force or _stale(lib, _deps()):
         os.makedirs(os.path.dirname(lib), exist_ok=True)
-        cmd = [nvcc_path(), *NVCC_FLAGS, f"-DBNK_BULK_LOST={LOST_BYTES}u", f"-DBNK_BULK_TURNS={LOST_TURNS}u", "-o", lib, *sources()]
+        defs = [f"-DBNK_BULK_LOST={LOST_BYTES}u", f"-DBNK_BULK_TURNS={LOST_TURNS}u"] + ([f"-DBNK_STREAM_IDLE={SOON}u"] if gives_up else [])
+        cmd = [nvcc_path(), *NVCC_FLAGS, *defs, "-o", lib, *sources()]
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)

@@ -1134,7 +1134,10 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
 constexpr uint32_t kStreamWarps = 17, kStreamWorkers = kStreamWarps - 1;
 constexpr uint32_t kStreamStages = 6, kStreamAhead = 2, kStreamRun = 3200;
 constexpr uint32_t kStreamGap = 16;        // what may lie between neighbours: no message, wherever its descriptor is, fits in there
-constexpr uint32_t kStreamIdle = 1u << 25; // turns of the first warp in which nothing has happened: seconds
+// Turns of the first warp in which nothing has happened: seconds.  (A build for tests has it give up at once.)
+#ifndef BNK_STREAM_IDLE
+#define BNK_STREAM_IDLE (1u << 25)
+#endif
 static_assert(kStreamRun >= kRoundBytes + BNK_WG_HEADER + 2 * BNK_WG_TAG && kStreamRun % 128 == 0, "a packet of one round fits");
 struct StreamRun { // neighbours in a stage
     uint32_t count;        // 0: no more come
@@ -1151,11 +1154,14 @@ struct StreamShared {
     alignas(128) uint4 stage[kStreamStages][(kStreamRun + 64) / 16]; // (a look at a packet's head may go 64 bytes beyond its start)
     StreamRun run[kStreamStages];
     uint64_t ready[kStreamStages], full[kStreamStages], over[kStreamStages]; // a run is described, has come, is worked on
+    volatile bool ended; // no more runs come
 };
-// A wait for another warp of the CTA, whose own waits for copies end after bar_wait's time.
-__device__ __forceinline__ bool bar_wait_warp(uint64_t *bar, uint32_t parity) {
-    for (uint32_t k = 0; k < 2 * kStreamStages + 2; k++)
+// A wait for the first warp, whose own waits for copies end after bar_wait's time.
+__device__ __forceinline__ bool bar_wait_warp(const StreamShared &sh, uint64_t *bar, uint32_t parity) {
+    for (uint32_t k = 0; k < 2 * kStreamStages + 2; k++) {
         if (bar_wait(bar, parity)) return true;
+        if (sh.ended) return false;
+    }
     return false;
 }
 
@@ -1246,6 +1252,16 @@ __device__ __forceinline__ void stream_feed(const AeadArgs &a, StreamShared &sh)
     };
     uint32_t res_len = 0, res_status = BNK_PKT_OK, res_slot = 0, res_has = 0;
     uint64_t res_ctr = 0;
+    auto put_results = [&](uint32_t i) {
+#pragma unroll
+        for (int d = 0; d < 2; d++) {
+            const AeadResults &o = a.res[d];
+            if (o.status) o.status[i] = (uint8_t)res_status;
+            if (o.out_len) o.out_len[i] = res_len;
+            if (o.counter && res_has) o.counter[i] = res_ctr;
+            if (o.slot) o.slot[i] = res_slot;
+        }
+    };
     auto send = [&] { // the oldest run, which has been worked on
         StreamRun &r = sh.run[sent % kStreamStages];
         const uint32_t count = r.count, first = r.first & (T - 1), k = lane - first;
@@ -1268,21 +1284,11 @@ __device__ __forceinline__ void stream_feed(const AeadArgs &a, StreamShared &sh)
             }
             bulk_out_commit();
         }
-        if (r.ends_tile && lane < first + count) {
-            const uint32_t i = r.first - first + lane;
-#pragma unroll
-            for (int d = 0; d < 2; d++) {
-                const AeadResults &o = a.res[d];
-                if (o.status) o.status[i] = (uint8_t)res_status;
-                if (o.out_len) o.out_len[i] = res_len;
-                if (o.counter && res_has) o.counter[i] = res_ctr;
-                if (o.slot) o.slot[i] = res_slot;
-            }
-        }
+        if (r.ends_tile && lane < first + count) put_results(r.first - first + lane);
         __syncwarp();
         sent++;
     };
-    for (uint32_t idle = 0; (t < tiles || sent < asked) && idle < kStreamIdle;) {
+    for (uint32_t idle = 0; (t < tiles || sent < asked) && idle < BNK_STREAM_IDLE;) {
         // a stage is free, or will be as soon as the copy out of it has read it, and not too much is on its way
         const bool room = asked < kStreamStages || asked - kStreamStages < sent;
         if (t < tiles && room && (!fetches || asked < kStreamAhead || passed(sh.full, asked - kStreamAhead))) {
@@ -1301,13 +1307,29 @@ __device__ __forceinline__ void stream_feed(const AeadArgs &a, StreamShared &sh)
             idle++;
         }
     }
-    if (lane == 0) { // no more come: in the stage that every worker looks at next
-        sh.run[asked % kStreamStages].count = 0;
-        bar_arrive(&sh.ready[asked % kStreamStages]);
+    if (lane == 0) {
+        sh.ended = true;
+        if (asked < kStreamStages || asked - kStreamStages < sent) { // in the stage that every worker looks at next
+            sh.run[asked % kStreamStages].count = 0;
+            bar_arrive(&sh.ready[asked % kStreamStages]);
+        }
         bulk_out_done();
     }
     for (uint32_t run = sent; run < asked; run++) // a copy that is still on its way must not meet the next kernel's shared memory
         if (sh.run[run % kStreamStages].asked) bar_wait(&sh.full[run % kStreamStages], run / kStreamStages & 1u);
+    const uint32_t left = sent < asked ? sh.run[sent % kStreamStages].first : t * T + j, all_mine = min(a.n, tiles * T);
+    if (left >= all_mine) return;
+    // It has given up.  The results of the last tile that are known, and for all that has not been sent what it is.
+    wait_for_kernel_in_front();
+    if (lane < (left & (T - 1))) put_results((left & ~(T - 1)) + lane);
+    for (uint32_t i = left + lane; i < all_mine; i += 32) {
+        res_status = BNK_PKT_NOT_READ;
+        res_len = 0;
+        res_slot = OPEN && a.demux ? 0u : a.slot[i];
+        res_has = !OPEN && res_slot < a.max_slots;
+        if (!OPEN) res_ctr = a.counter[i];
+        put_results(i);
+    }
 }
 
 // The others.
@@ -1316,7 +1338,7 @@ __device__ __forceinline__ void stream_work(const AeadArgs &a, StreamShared &sh,
     const uint32_t lane = threadIdx.x & 31;
     for (uint32_t s = 0, parity = 0;;) {
         StreamRun &r = sh.run[s];
-        if (!bar_wait_warp(&sh.ready[s], parity)) return;
+        if (!bar_wait_warp(sh, &sh.ready[s], parity)) return;
         const uint32_t count = r.count;
         if (count == 0) return;
         uint4 inner = make_uint4(0, 0, 0, 0); // the n-th of this run's plaintexts of this warp in lane n
@@ -1471,6 +1493,7 @@ __global__ void __launch_bounds__(32 * kStreamWarps, 1) aead_stream_kernel(const
         bar_init(&sh.full[threadIdx.x]);
         bar_init(&sh.over[threadIdx.x], kStreamWorkers);
     }
+    if (threadIdx.x == 0) sh.ended = false;
     bulk_fence_shared();
     __syncthreads();
     if (threadIdx.x < 32) { // what it reads is the host's

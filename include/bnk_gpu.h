@@ -85,7 +85,9 @@ extern "C" {
                                        or does not come from the peer's allowed address */
 #define BNK_PKT_NOT_READ 13         /* a fault of the host link, not of the packet: its bytes did not come within the time a
                                        kernel waits for them (half a second), or did not for a packet that the same
-                                       warp was to work on first.  out_len is 0.  The ring holds what it held, but for
+                                       warp was to work on first, or, where neighbouring packets cross the link as one
+                                       copy, for one in front of it in the same stretch of the batch (a fiftieth of it at
+                                       most).  out_len is 0.  The ring holds what it held, but for
                                        packets beyond 1984 bytes: of those the stretches in front are sealed already, or
                                        zeros where they were opened.  A nonce handed out to the packet stays unused. */
 

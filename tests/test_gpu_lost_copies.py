@@ -12,14 +12,23 @@ from tests import reference_cases as RC
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture
-def lossy(gpu_lib, monkeypatch):
+def _load(monkeypatch, **kind):
     from bnk_b200 import _build, _lib
 
-    if not os.path.exists(_build.lost_copies_path()):
-        _build.build_lost_copies()
-    monkeypatch.setattr(_lib, "_LIB", _lib.load(_build.lost_copies_path()))
+    if not os.path.exists(_build.lost_copies_path(**kind)):
+        _build.build_lost_copies(**kind)
+    monkeypatch.setattr(_lib, "_LIB", _lib.load(_build.lost_copies_path(**kind)))
     return _build.LOST_BYTES
+
+
+@pytest.fixture
+def lossy(gpu_lib, monkeypatch):
+    return _load(monkeypatch)
+
+
+@pytest.fixture
+def gives_up(gpu_lib, monkeypatch):
+    return _load(monkeypatch, gives_up=True)
 
 
 def test_split_leaves_out_what_did_not_come(lossy, oracle):
@@ -147,6 +156,119 @@ def test_seal_and_open_refuse_what_did_not_come(lossy, oracle, n, lost, long):
         b.counter[:] = ctr
         b.seal(n)
         assert np.array_equal(b.status, st) and H.spans_equal(np.array(b.ring), ring, off, ln) == []
+        b.close()
+
+
+def _dense(c, oracle, keys, n, sizes, gaps, rng, first=0, ring_bytes=0):
+    """A batch whose packets lie close together, its payloads and what sealing makes of it."""
+    room = (sizes.astype(np.int64) + 47) // 16 * 16
+    off = np.concatenate([[0], np.cumsum(room + gaps)])
+    b = c.batch(n, max(int(off[-1]), ring_bytes))
+    b.off[:], b.len[:], b.slot[:] = off[:-1], sizes, rng.integers(0, len(keys), n)
+    b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
+    ctr = np.array([first + np.count_nonzero(b.slot[:i] == b.slot[i]) for i in range(n)], np.uint64)
+    ring, st, ln = H.oracle_seal(oracle, keys, np.arange(len(keys)), 0, b.ring, b.off, b.len, b.slot, ctr)
+    assert (st == 0).all()
+    return b, np.array(b.ring), ring, ln, ctr
+
+
+# Packets of 1136 bytes, two a copy; the one that does not come lies by itself.  Tiles of 16 packets, one or three to a CTA: the
+# copy behind the one that does not come is on its way already, and what would come next is not asked for.  (So few are opened by
+# another kernel.)
+@pytest.mark.parametrize("n,lost,stretch", [(1024, 518, 16), (1024, 1023, 16), (4096, 3 * 48 + 17, 48), (4096, 4095, 48)])
+def test_neighbours_of_what_did_not_come(lossy, oracle, n, lost, stretch):
+    from bnk_b200 import Context
+    from bnk_b200.device import F_ASSIGN_COUNTERS, F_REPLAY, PKT_NOT_READ
+
+    rng = np.random.default_rng(n + lost)
+    peers = 5
+    keys = rng.integers(0, 256, (peers, 32), dtype=np.uint8)
+    sizes, gaps = np.full(n, 1104, np.uint32), np.zeros(n, np.int64)
+    sizes[lost] = lossy - 32
+    gaps[max(lost - 1, 0)] = gaps[lost] = 32
+    runs, tile = [], 16  # as they are asked for from the stretch's first packet on
+    for t in range(lost // stretch * stretch, min(lost // stretch * stretch + stretch, n), tile):
+        at, end = t, min(t + tile, n)
+        while at < end:
+            more = 2 if at + 1 < end and lost not in (at, at + 1) else 1
+            runs.append(range(at, at + more))
+            at += more
+    which = next(k for k, r in enumerate(runs) if lost in r)
+    refused = np.zeros(n, bool)
+    for k, r in enumerate(runs):
+        refused[list(r)] = k == which or k > which + 1
+    with Context(max_keypairs=peers, mtu=0, flow_capacity=0, replay_ring_blocks=32) as c:
+        c.set_keypairs(0, keys, keys, np.arange(peers, dtype=np.uint32))
+        b, plain, ring, ln, ctr = _dense(c, oracle, keys, n, sizes, gaps, rng)
+        b.status[:], b.out_len[:] = 0, 7
+        b.seal(n, F_ASSIGN_COUNTERS)
+        assert np.array_equal(b.status, np.where(refused, PKT_NOT_READ, 0)) and np.array_equal(b.out_len, np.where(refused, 0, ln))
+        assert np.array_equal(b.counter, ctr)
+        assert H.spans_equal(np.array(b.ring), ring, b.off[~refused], ln[~refused]) == []
+        assert H.spans_equal(np.array(b.ring), plain, b.off[refused], ln[refused]) == []
+        if n < 4096:
+            return
+        b.ring[:], b.len[:] = ring, ln
+        want_ring, st, got, want_ln = H.oracle_open(oracle, keys, ring, b.off, ln, b.slot)
+        b.open(n, F_REPLAY)
+        want, state = H.oracle_replay(oracle, 32, b.slot, got, np.where(refused, PKT_NOT_READ, st))
+        assert np.array_equal(b.status, want) and np.array_equal(b.out_len, np.where(refused, 0, want_ln))
+        assert H.spans_equal(np.array(b.ring), want_ring, b.off[~refused], want_ln[~refused], 16) == []
+        assert H.spans_equal(np.array(b.ring), ring, b.off[refused], ln[refused]) == []
+        for s, r in state.items():
+            last, words = c.replay_export(s)
+            assert last == r.last and np.array_equal(words, r.ring())
+        b.close()
+
+
+@pytest.mark.parametrize("n", [4096, 5003])
+def test_what_has_not_been_handed_out_is_refused(gives_up, oracle, n):
+    """The warp that hands packets out gives up in the middle of the batch: what it has not sent back is refused, whatever the arrays
+    held before, nothing of it is written, and the replay window does not take it for opened."""
+    from bnk_b200 import Context
+    from bnk_b200.device import F_ASSIGN_COUNTERS, F_REPLAY, PKT_NOT_READ
+
+    rng = np.random.default_rng(n)
+    peers = 5
+    keys = rng.integers(0, 256, (peers, 32), dtype=np.uint8)
+    with Context(max_keypairs=peers, mtu=0, flow_capacity=0, replay_ring_blocks=32) as c:
+        c.set_keypairs(0, keys, keys, np.arange(peers, dtype=np.uint32))
+        b, plain, ring, ln, ctr = _dense(c, oracle, keys, n, np.full(n, 1104, np.uint32), np.zeros(n, np.int64), rng, 5000, 2048 * n)
+        for p in range(peers):
+            c.set_send_counter(p, 5000)
+        b.status[:], b.out_len[:] = 0, 7
+        b.seal(n, F_ASSIGN_COUNTERS)
+        refused = np.array(b.status) == PKT_NOT_READ
+        assert refused.any() and not b.status[~refused].any()
+        assert np.array_equal(b.out_len, np.where(refused, 0, ln)) and np.array_equal(b.counter, ctr)
+        assert H.spans_equal(np.array(b.ring), ring, b.off[~refused], ln[~refused]) == []
+        assert H.spans_equal(np.array(b.ring), plain, b.off[refused], ln[refused]) == []
+        want_ring, st, got, want_ln = H.oracle_open(oracle, keys, ring, b.off, ln, b.slot)
+        # on the device, authentic packets everywhere: another kernel opens them, as they lie far apart
+        dense = np.array(b.off)
+        apart = H.layout_fixed(n, 2048)
+        ctr -= np.uint64(5000)
+        for i in range(n):
+            b.ring[apart[i] + 16:apart[i] + 1120] = 0
+        wide, st_wide, ln_wide = H.oracle_seal(oracle, keys, np.arange(peers), 0, b.ring, apart, b.len, b.slot, ctr)
+        b.ring[:], b.off[:], b.len[:] = wide, apart, ln_wide
+        b.open(n, F_REPLAY)
+        _, state = H.oracle_replay(oracle, 32, b.slot, ctr, st_wide)
+        assert not b.status.any()
+        # and now neighbours, of counters that the window has not seen
+        b.off[:] = dense
+        for rep in range(2):
+            b.ring[:], b.len[:], b.status[:] = ring, ln, 0
+            b.open(n, F_REPLAY)
+            refused = np.array(b.status) == PKT_NOT_READ
+            assert refused.any()
+            want, state = H.oracle_replay(oracle, 32, b.slot, got, np.where(refused, PKT_NOT_READ, st), state)
+            assert np.array_equal(b.status, want) and np.array_equal(b.out_len, np.where(refused, 0, want_ln))
+            assert H.spans_equal(np.array(b.ring), want_ring, b.off[~refused], want_ln[~refused], 16) == []
+            assert H.spans_equal(np.array(b.ring), ring, b.off[refused], ln[refused]) == []
+            for s, r in state.items():
+                last, words = c.replay_export(s)
+                assert last == r.last and np.array_equal(words, r.ring())
         b.close()
 
 
