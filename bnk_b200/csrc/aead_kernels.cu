@@ -26,6 +26,7 @@
 
 #include "bulk.cuh"
 #include "filter_device.cuh"
+#include "layout.h"
 
 namespace {
 
@@ -1133,7 +1134,7 @@ __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __gri
 // ---------------------------------------------------------------------------
 constexpr uint32_t kStreamWarps = 17, kStreamWorkers = kStreamWarps - 1;
 constexpr uint32_t kStreamStages = 6, kStreamAhead = 2, kStreamRun = 3200;
-constexpr uint32_t kStreamGap = 16;        // what may lie between neighbours: no message, wherever its descriptor is, fits in there
+constexpr uint32_t kStreamGap = kJoinGap;  // what may lie between neighbours: no message, wherever its descriptor is, fits in there
 // Turns of the first warp in which nothing has happened: seconds.  (A build for tests has it give up at once.)
 #ifndef BNK_STREAM_IDLE
 #define BNK_STREAM_IDLE (1u << 25)
@@ -1513,7 +1514,7 @@ __global__ void __launch_bounds__(32 * kStreamWarps, 1) aead_stream_kernel(const
 #endif
 
 // Tiles and grid of a warp-per-packet launch.  Rings in device memory (n <= BNK_WPP_MAX_PACKETS): a warp per packet.
-// Rings in host memory: the link is the bound (and packets that lie close together go through kernel 3, see in_stream; the figures here
+// Rings in host memory: the link is the bound (and packets that lie close together go through kernel 3, see in_stream in layout.h; the figures here
 // are of 1472 bytes apart, as longer ones and ones further apart behave).  With a warp per packet all reads are asked for at once, end together and
 // leave the writes for afterwards, so beyond kLinkWindow bytes a warp takes several packets: 1024 x 1420 B sealed by
 // 32 to 96 CTAs 72 us, by 128 84, by 256 (a packet each) 92; 512 x 1420 46 against 54.  Small packets are bound by what
@@ -1570,22 +1571,10 @@ cudaError_t launch_wpp(const AeadArgs &a, uint32_t ctas, const HostDesc *h, cuda
 // Tiles and grid of kernel 3.  With small packets every SM helps, 9000 x 64 B sealed by 96 CTAs 84 us, by 148 72; large ones
 // have as much outstanding as the link takes with fewer: 12,000 x 1420 B by 64 504 us, by 96 482, by 148 491.  Tiles of 16 are
 // worth a CTA each, smaller ones of 4 at the least spread a batch that has fewer than kStreamTiles of them.
-// Below kStreamFrom bytes kernel 2 is as fast: 1000 mixed packets (360 KB) sealed 29.5 us and 30.4, opened 34.3 and 35.3; 512 x 1420 B
-// (730 KB) sealed 38.0 and 35.3.  An open works on a stage for longer, as nothing of it can be done beforehand, and of large packets
-// few are at hand in a CTA: 1500 x 1000 B, whole path, 105.1 us and 106.7, 4096 x 700 B (2.9 MB) 152.0 and 154.4, 2000 x 1420 B (2.8 MB) 148.3
-// and 148.0, but 4096 x 1420 B opened 197 and 188, 12,000 518 and 500; small ones 9000 x 64 B 80 and 73.
-// Sealed, kernel 2 and this one: 1024 x 1420 B 66 us and 61, 4096 201 and 183, 12,000 535 and 490, 9000 x 64 B 83 and 74, whole path
-// 10,000 mixed 176 and 158.
-// 2048 mixed packets (840 KB) are on the line: sealed 47 us, 45 to 50.
-constexpr uint64_t kStreamFrom = 512u << 10, kStreamSmallFrom = 896u << 10, kStreamOpenFrom = 4u << 20;
-constexpr uint32_t kStreamCtas = 96, kStreamCtasSmall = 148, kStreamTiles = 64, kSmallPacket = 512;
-bool small_packets(const AeadArgs &a) { return a.link_bytes <= (uint64_t)kSmallPacket * a.n; }
-bool in_stream(const AeadArgs &a, bool open) {
-    const uint64_t from = open == small_packets(a) ? kStreamFrom : open ? kStreamOpenFrom : kStreamSmallFrom;
-    return a.from_host && a.dense && a.n > kRankMax && a.link_bytes >= from;
-}
+constexpr uint32_t kStreamCtas = 96, kStreamCtasSmall = 148, kStreamTiles = 64;
+static_assert(kStreamPackets >= kRankMax, "it hands out no nonces itself");
 void stream_grid(AeadArgs &a, uint32_t &ctas) {
-    const uint32_t most = small_packets(a) ? kStreamCtasSmall : kStreamCtas;
+    const uint32_t most = a.link_bytes <= (uint64_t)kSmallPacket * a.n ? kStreamCtasSmall : kStreamCtas;
     a.tile = 16;
     while (a.tile > 4 && a.n < kStreamTiles * a.tile) a.tile /= 2;
     const uint32_t tiles = (a.n + a.tile - 1) / a.tile, rounds = (tiles + most - 1) / most;
@@ -1595,7 +1584,7 @@ void stream_grid(AeadArgs &a, uint32_t &ctas) {
 template <bool OPEN>
 cudaError_t launch_aead(AeadArgs a, cudaStream_t s, bnk_ctx *ctx) {
     if (a.n == 0) return cudaSuccess;
-    if (in_stream(a, OPEN)) {
+    if (a.stream) {
         uint32_t ctas;
         stream_grid(a, ctas);
         const dim3 grid(ctas), block(32 * kStreamWarps);

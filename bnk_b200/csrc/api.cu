@@ -10,8 +10,8 @@
 #include <thread>
 
 #include "filter_device.cuh"
+#include "layout.h"
 #include "pieces.h"
-#include "scan.h"
 #include "submit_order.h"
 
 namespace {
@@ -81,23 +81,10 @@ class Slab {
     size_t total_ = 0;
 };
 
-constexpr uint32_t kMostRoom = 16 + 16 + 16; // header, padding and tag around a payload
-// What a submit's way depends on besides.
-struct Layout {
-    uint64_t bytes = 0;    // of the packets
-    bool in_order = false; // they lie in the ring in order, each with its own room behind it
-    bool dense = false;    // at most about a quarter of their stretch of it lies between them, and none is longer than kDenseLongest
-};
 // highest ring byte any of the first n packets can touch (input or output side); with `room` bytes of its own behind each
-constexpr uint32_t kDenseLongest = 1969; // a message, with its padding, of one round in the kernels' terms
 uint64_t ring_extent(const bnk_batch *b, uint32_t n, uint32_t slack, Layout *l = nullptr, uint32_t room = 0) {
     const PacketScan r = scan_packets(b->host.off, b->host.len, n, room);
-    if (l) {
-        const uint64_t from = n ? std::min<uint64_t>(b->host.off[0], r.end) : 0, with_room = r.sum + (uint64_t)n * kMostRoom;
-        l->bytes = r.sum + (uint64_t)n * slack;
-        l->in_order = r.in_order;
-        l->dense = r.longest <= kDenseLongest && 4 * with_room >= 3 * (r.end - from);
-    }
+    if (l) *l = layout_of(r, n, slack);
     const uint64_t ext = n ? (r.end + slack + 15) & ~15ull : 0;
     return ext > b->ring_bytes ? b->ring_bytes : ext;
 }
@@ -237,17 +224,16 @@ bool heads_direct(bnk_batch *b, uint32_t npkts, uint32_t flags) {
 // one down have no company: 16,384 x 1420 B 710 us against 750, 32,768 1390 against 1330, 131,072 5.74 ms against 4.96.
 // With small packets that kernel is bound by what its warps compute, ~7.5 ns a packet, and pieces win earlier: 8192 x
 // 300 B 138 us against 144, 16,384 252 against 233, 131,072 x 64 B 990 against 600.
-// Packets that lie close together go up and down by neighbours, and that kernel is ahead up to ctx->dense_pieces_from (64 MB) whatever their size; sealed, pieces /
+// Packets that lie close together go up and down by neighbours (see in_stream), and that kernel is ahead up to ctx->stream_pieces_from (64 MB); sealed, pieces /
 // in place: 11,000 mixed 204 us and 161, 16,000 262 and 222, 30,000 449 and 400, 20,000 x 64 B 144 and 126, 40,000 x 300 B 508 and 483,
 // 18,000 x 1420 B 815 and 741, 32,768 (48 MB) 1358 and 1315, 48,000 (71 MB) 1935 and 1916, 65,536 (96 MB) 2517 and 2595; opened 16,000 mixed
 // 264 and 221, 32,768 x 1420 B 1385 and 1342, 65,536 2535 and 2597.
-constexpr uint32_t kManySmall = 10240, kSmallBytes = 512;
-bool in_pieces(const bnk_batch *b, uint32_t n, uint32_t flags, uint64_t ext, const Layout &lay) {
+bool in_pieces(const bnk_batch *b, uint32_t n, uint32_t flags, uint64_t ext, const Layout &lay, bool open) {
     const bnk_ctx *const ctx = b->ctx;
-    const bool dense = lay.dense && ctx->aead_mode != 1 && ext <= ctx->host_direct_bytes;
-    const uint64_t from = dense ? ctx->dense_pieces_from : ctx->pieces_from;
+    const bool stream = in_stream(lay, n, open) && ctx->aead_mode != 1 && ext <= ctx->host_direct_bytes;
+    const uint64_t from = stream ? ctx->stream_pieces_from : ctx->pieces_from;
     if (n == 0) return false;
-    if (ext < from && (dense || n < kManySmall || ext > (uint64_t)n * kSmallBytes || ext < from / 16)) return false;
+    if (ext < from && (stream || n < kManySmall || ext > (uint64_t)n * kSmallPacket || ext < from / 16)) return false;
     return lay.in_order && b->pieces.up && !(flags & (BNK_F_NO_H2D | BNK_F_NO_D2H | BNK_F_USE_OUT_LEN)) &&
            ctx->in_flight.load(std::memory_order_relaxed) == (b->counted ? 1 : 0);
 }
@@ -463,9 +449,9 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
         ctx->host_direct_bytes = strtoull(m, nullptr, 0);
     if (!one_address || !maps_host) ctx->host_direct_bytes = 0; // pinned memory must have one address
     ctx->pieces_from = 24u << 20;
-    ctx->dense_pieces_from = 64u << 20;
+    ctx->stream_pieces_from = 64u << 20;
     if (const char *m = getenv("BNK_PIECES_FROM")) // tuning aid: ring extent from which a batch that is alone goes in pieces
-        ctx->pieces_from = ctx->dense_pieces_from = strtoull(m, nullptr, 0);
+        ctx->pieces_from = ctx->stream_pieces_from = strtoull(m, nullptr, 0);
     ctx->launch_graphs = true;
     if (const char *m = getenv("BNK_LAUNCH_GRAPHS")) // tuning and test aid: 0 = every launch by itself
         ctx->launch_graphs = strtoul(m, nullptr, 0) != 0;
@@ -1060,7 +1046,7 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, const Layout &lay, uint32_t
     } else {
         b->stale_pkts = std::max(b->stale_pkts, npkts);
         a.from_host = true;
-        a.dense = lay.dense;
+        a.stream = in_stream(lay, npkts, false);
         a.host = HostDesc{h.off, h.len, h.slot};
         a.in = h.ring;
         a.off = h.off;
@@ -1163,7 +1149,7 @@ int bnk_seal_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     const size_t n = npkts;
     Layout lay;
     const uint64_t ext = device_only ? 0 : ring_extent(b, npkts, kMostRoom, &lay, BNK_WG_HEADER + BNK_WG_TAG);
-    if (in_pieces(b, npkts, flags, ext, lay)) return seal_pieces(b, npkts, ext, flags, now_unix_ns);
+    if (in_pieces(b, npkts, flags, ext, lay, false)) return seal_pieces(b, npkts, ext, flags, now_unix_ns);
     if (ctx->aead_mode != 1) {
         if (host_direct(b, npkts, flags, ext)) return seal_direct(b, npkts, lay, flags, now_unix_ns, false);
         if (!b->stale_pkts && (flags & BNK_F_NO_H2D) && host_direct(b, npkts, flags & ~BNK_F_NO_H2D, ext))
@@ -1256,7 +1242,7 @@ static int open_direct(bnk_batch *b, uint32_t npkts, const Layout &lay, uint32_t
     a.header_first = few_in_flight(b);
     a.host = HostDesc{h.off, h.len, h.slot};
     a.link_bytes = lay.bytes;
-    a.dense = lay.dense;
+    a.stream = in_stream(lay, npkts, true);
     a.in = a.out = h.ring;
     a.off = h.off;
     a.len = h.len;
@@ -1377,7 +1363,7 @@ int bnk_open_submit(bnk_batch *b, uint32_t npkts, uint32_t flags, int64_t now_un
     const size_t n = npkts;
     Layout lay;
     const uint64_t ext = device_only ? 0 : ring_extent(b, npkts, (flags & BNK_F_USE_OUT_LEN) || b->stale_pkts ? kMostRoom : 0, &lay);
-    if (in_pieces(b, npkts, flags, ext, lay)) return open_pieces(b, npkts, ext, flags, now_unix_ns);
+    if (in_pieces(b, npkts, flags, ext, lay, true)) return open_pieces(b, npkts, ext, flags, now_unix_ns);
     if (ctx->aead_mode != 1 && host_direct(b, npkts, flags, ext)) return open_direct(b, npkts, lay, flags, now_unix_ns);
     // BNK_F_USE_OUT_LEN reads the lengths a seal left on the device: an upload beside it must not bring the
     // host's out_len along, so it moves the fields one by one instead of the whole slab.

@@ -112,8 +112,8 @@ struct bnk_ctx {
     bool launch_graphs; // BNK_LAUNCH_GRAPHS
     int aead_mode; // 0 = choose by batch size, 1 = always thread per packet, 2 = always warp per packet (BNK_AEAD_KERNEL)
     uint32_t aead_side_stream_from; // batches of at least this many packets run seal/open on the low-priority stream (BNK_AEAD_SIDE_STREAM_FROM; 0 = never)
-    // ring extent from which a batch that is alone goes over the link in pieces (BNK_PIECES_FROM), of packets that lie close together
-    uint64_t pieces_from, dense_pieces_from;
+    // ring extent from which a batch that is alone goes over the link in pieces (BNK_PIECES_FROM); of batches for aead_stream_kernel
+    uint64_t pieces_from, stream_pieces_from;
     int prio_low, prio_high;        // stream priority range of the device
     std::atomic<uint64_t> launches, graph_launches;
     std::atomic<uint64_t> seal_seq{0}; // number of the last seal launch that handed out nonces itself (see SendCounter)
@@ -336,7 +336,7 @@ struct AeadArgs {
     bool header_first;            // open of up to kRankMax packets with from_host: their headers are asked for ahead of them
     HostDesc host;                // with from_host
     uint64_t link_bytes;          // with over_link: bytes of the packets
-    bool dense;                   // with from_host: short packets, one behind the other with little between them
+    bool stream;                  // with from_host: it is a batch for kernel 3 (see in_stream)
     uint32_t n;
     uint32_t tile;                // set by the launcher
     uint32_t mtu;
