@@ -230,7 +230,7 @@ bool heads_direct(bnk_batch *b, uint32_t npkts, uint32_t flags) {
 // 264 and 221, 32,768 x 1420 B 1385 and 1342, 65,536 2535 and 2597.
 bool in_pieces(const bnk_batch *b, uint32_t n, uint32_t flags, uint64_t ext, const Layout &lay, bool open) {
     const bnk_ctx *const ctx = b->ctx;
-    const bool stream = in_stream(lay, n, open) && ctx->aead_mode != 1 && ext <= ctx->host_direct_bytes;
+    const bool stream = in_stream(lay, n, open) && ctx->aead_mode == 0 && ext <= ctx->host_direct_bytes;
     const uint64_t from = stream ? ctx->stream_pieces_from : ctx->pieces_from;
     if (n == 0) return false;
     if (ext < from && (stream || n < kManySmall || ext > (uint64_t)n * kSmallPacket || ext < from / 16)) return false;
@@ -1046,7 +1046,7 @@ static int seal_direct(bnk_batch *b, uint32_t npkts, const Layout &lay, uint32_t
     } else {
         b->stale_pkts = std::max(b->stale_pkts, npkts);
         a.from_host = true;
-        a.stream = in_stream(lay, npkts, false);
+        a.stream = ctx->aead_mode == 0 && in_stream(lay, npkts, false);
         a.host = HostDesc{h.off, h.len, h.slot};
         a.in = h.ring;
         a.off = h.off;
@@ -1242,7 +1242,7 @@ static int open_direct(bnk_batch *b, uint32_t npkts, const Layout &lay, uint32_t
     a.header_first = few_in_flight(b);
     a.host = HostDesc{h.off, h.len, h.slot};
     a.link_bytes = lay.bytes;
-    a.stream = in_stream(lay, npkts, true);
+    a.stream = ctx->aead_mode == 0 && in_stream(lay, npkts, true);
     a.in = a.out = h.ring;
     a.off = h.off;
     a.len = h.len;

@@ -110,7 +110,7 @@ struct bnk_ctx {
     std::atomic<int> in_flight{0};           // batches submitted and not waited for
     std::atomic<uint64_t> direct_in_flight{0}; // ring bytes of those that run on the pinned buffers
     bool launch_graphs; // BNK_LAUNCH_GRAPHS
-    int aead_mode; // 0 = choose by batch size, 1 = always thread per packet, 2 = always warp per packet (BNK_AEAD_KERNEL)
+    int aead_mode; // 0 = choose by batch size and layout, 1 = always thread per packet, 2 = always warp per packet (BNK_AEAD_KERNEL)
     uint32_t aead_side_stream_from; // batches of at least this many packets run seal/open on the low-priority stream (BNK_AEAD_SIDE_STREAM_FROM; 0 = never)
     // ring extent from which a batch that is alone goes over the link in pieces (BNK_PIECES_FROM); of batches for aead_stream_kernel
     uint64_t pieces_from, stream_pieces_from;

@@ -89,14 +89,17 @@ ROUND = 1984  # payload bytes a warp takes per round
 
 
 # 8: a warp each, the descriptors with the launch and the header of a message ahead; 1024: tiles of four, so up to three packets
-# lie behind the one that does not come; long: its second round does not come
-@pytest.mark.parametrize("n,lost,long", [(8, 3, False), (8, 0, True), (256, 255, False), (1024, 513, False), (1024, 515, True)])
-def test_seal_and_open_refuse_what_did_not_come(lossy, oracle, n, lost, long):
+# lie behind the one that does not come; long: its second round does not come; and neighbours with this kernel asked for
+@pytest.mark.parametrize("n,lost,long,stride", [(8, 3, False, 4096), (8, 0, True, 4096), (256, 255, False, 4096), (1024, 513, False, 4096),
+                                                (1024, 515, True, 4096), (1024, 514, False, 1152)])
+def test_seal_and_open_refuse_what_did_not_come(lossy, oracle, monkeypatch, n, lost, long, stride):
     from bnk_b200 import Context
     from bnk_b200.device import F_ASSIGN_COUNTERS, F_NOTE_OUTBOUND, F_REPLAY, PKT_NOT_READ
 
+    if stride < 4096:
+        monkeypatch.setenv("BNK_AEAD_KERNEL", "wpp")  # read when a context is created
     rng = np.random.default_rng(n + lost)
-    peers, stride, now = 5, 4096, RC.T0
+    peers, now = 5, RC.T0
     keys = rng.integers(0, 256, (peers, 32), dtype=np.uint8)
     off, slot = H.layout_fixed(n, stride), rng.integers(0, peers, n).astype(np.uint32)
     refused = np.arange(n) == lost if n <= 256 else (np.arange(n) >= lost) & (np.arange(n) < lost // 4 * 4 + 4)
