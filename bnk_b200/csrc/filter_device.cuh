@@ -370,13 +370,11 @@ __device__ __forceinline__ void final_verdict(const VerdictArgs &v, uint32_t i) 
     uint8_t st = *(volatile uint8_t *)&v.status[i];
     uint32_t l = v.out_len[i];
     if (st == BNK_PKT_OK && (v.inner_check || v.check_inbound)) {
-        const uint4 h = v.inner[i];
-        if (v.inner_check) { // cut to the IPv4 total length; the source must be the peer's address
-            if ((h.z & kInnerWhole) && h.x != 0 && h.x == v.allowed_ip[v.slot[i]]) l = h.w;
-            else st = BNK_PKT_BAD_INNER;
-        }
-        if (v.check_inbound && st == BNK_PKT_OK && v.ft.enforce)
-            st = (h.z & kInnerParses) ? filter_verdict(v.ft, inner_parsed(h), v.now) : (uint8_t)BNK_PKT_FILTER_DENY;
+        uint8_t proto = 0;
+        FlowReply reply;
+        bool ask_flows = false;
+        checks_begin(v, i, v.inner_check ? v.slot[i] : 0u, st, l, proto, reply, ask_flows);
+        if (ask_flows) st = reply.finish(v.ft, proto, v.now);
         v.status[i] = st;
         v.out_len[i] = l;
     }

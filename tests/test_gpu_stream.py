@@ -169,3 +169,95 @@ def test_refused_descriptors_may_name_bytes_of_others(gpu_lib, oracle, n, size):
             assert np.array_equal(b.out_len[good], ln) and np.array_equal(b.counter[good], got)
             assert H.spans_differ_count(np.array(b.ring), want, off[good], ln, 16) == 0, rep
         b.close()
+
+
+# Few and many peers: runs of a peer's packets that are longer than what the window looks back, and shorter; one cluster's work, and more
+# than it takes; without the window the last checks run by themselves.
+@pytest.mark.parametrize("n,peers,replay", [(5000, 7, True), (5000, 200, True), (5000, 200, False), (36_000, 300, True), (36_000, 300, False)])
+def test_everything_on_behind_small_neighbours(gpu_lib, oracle, n, peers, replay):
+    """Small packets that cross the link together, out of order, a few twice, a few damaged: receiver index, window, inner header, rules
+    and reply flows say what the oracle says, and leave the same windows and flows behind."""
+    from bnk_b200 import Context
+    from bnk_b200.device import F_CHECK_INBOUND, F_DEMUX_INDEX, F_INNER_CHECK, F_REPLAY, PKT_BAD_INNER, PKT_FILTER_DENY, PKT_REPLAY
+    from bnk_b200.filter import CompiledRule, PortRange, flatten_rules
+
+    rng = np.random.default_rng(n + peers)
+    keys = rng.integers(0, 256, (peers, 32), dtype=np.uint8)
+    addr = RC.ip("100.64.0.0") + 16 + np.arange(peers) * 3
+    rules = [("100.64.0.0/25", "udp", [(1, 20000), (40000, 50000)]), ("100.64.0.0/10", "tcp", [(22, 22), (50000, 60000)]), ("100.64.1.0/24", "icmp", [])]
+    rules += [(f"100.64.{(k >> 8) & 255}.{k & 255}/32", "udp", [(20000, 30000 + k)]) for k in range(16, 16 + 3 * peers, 5)]
+    # the packets, each from its peer's address but for some, and what the node has sent before
+    m = n - n // 50
+    slot = rng.integers(0, peers, m).astype(np.uint32)
+    lens = rng.integers(28, 200, m)
+    size = (lens + 47) // 16 * 16
+    off = np.concatenate([[0], np.cumsum(size)])
+    ring = rng.integers(0, 256, int(off[-1]), dtype=np.uint8)
+    f = oracle.Filter()
+    f.set_rules([([(RC.ip(s.split("/")[0]), int(s.split("/")[1]))], p, r) for s, p, r in rules])
+    sent = []
+    for i in range(m):
+        src, sport, dport, kind = int(addr[slot[i]]), int(rng.integers(1, 9)), int(rng.integers(1, 65536)), rng.integers(0, 10)
+        if rng.random() < 0.03:
+            src += 1
+        if kind == 0:
+            p = RC.icmp_echo(src, RC.SELF, True)
+        elif kind < 4 and lens[i] >= 40:
+            p = RC.tcp(src, RC.SELF, sport, dport)
+        else:
+            p = RC.udp(src, RC.SELF, sport, dport)
+        if rng.random() < 0.3:
+            sent.append(RC.icmp_echo(RC.SELF, src, False) if kind == 0 else (RC.tcp if kind < 4 and lens[i] >= 40 else RC.udp)(RC.SELF, src, dport, sport))
+        p = p[:2] + int(lens[i] + (rng.random() < 0.02)).to_bytes(2, "big") + p[4:]
+        ring[off[i] + 16:off[i] + 16 + len(p)] = np.frombuffer(p, np.uint8)
+    ctr = np.zeros(m, np.uint64)
+    for p in range(peers):
+        ctr[slot == p] = np.arange(np.count_nonzero(slot == p))
+    sealed, st, ln = H.oracle_seal(oracle, keys, np.arange(peers), 0, ring, off[:-1], lens, slot, ctr)
+    assert (st == 0).all() and np.array_equal(ln, size)
+    # as they arrive
+    order = np.argsort(np.arange(m) + np.where(rng.random(m) < 0.1, rng.integers(0, 300, m), 0), kind="stable")
+    came = np.insert(order, rng.integers(0, m, n - m), rng.integers(0, m, n - m))
+    at = np.concatenate([[0], np.cumsum(ln[came])]).astype(np.int64)
+    ring = np.concatenate([sealed[off[i]:off[i] + ln[i]] for i in came])
+    for i in rng.choice(n, n // 100, replace=False):
+        ring[at[i] + 16 + int(rng.integers(0, ln[came[i]] - 16))] ^= 1
+    off, lens, slot = at[:-1].astype(np.uint32), ln[came], slot[came]
+    now = RC.T0
+    plain, st, got, pt_len = H.oracle_open(oracle, keys, ring, off, lens, slot)
+    want, state = H.oracle_replay(oracle, 32, slot, got, st) if replay else (st, {})
+    for p in sent:
+        f.note_outbound(p, now)
+    for i in np.flatnonzero(want == oracle.OK):
+        p = plain[off[i] + 16:off[i] + 16 + pt_len[i]].tobytes()
+        total = oracle.inner_check(p, int(addr[slot[i]]))
+        if total is None:
+            want[i] = PKT_BAD_INNER
+        else:
+            pt_len[i] = total
+            if not f.check_inbound(p[:total], now + RC.SEC):
+                want[i] = PKT_FILTER_DENY
+    with Context(max_keypairs=peers, mtu=0, flow_capacity=1 << 16, replay_ring_blocks=32) as c:
+        c.set_keypairs(0, keys, keys, np.arange(peers, dtype=np.uint32))
+        for p in range(peers):
+            c.index_set(p, p)
+            c.set_allowed_ip(p, int(addr[p]))
+        c.acl_set(True, flatten_rules([CompiledRule(srcs=[s], proto=p, ports=[PortRange(*x) for x in r]) for s, p, r in rules]))
+        note = c.batch(len(sent), 64 * len(sent))
+        note.put_packets(sent, 64)
+        note.filter_note(len(sent), now)
+        b = c.batch(n, len(ring) + 64)
+        b.ring[:len(ring)] = ring
+        b.off[:], b.len[:], b.slot[:] = off, lens, 0xFFFFFFFF
+        b.open(n, F_DEMUX_INDEX | F_INNER_CHECK | F_CHECK_INBOUND | (F_REPLAY if replay else 0), now + RC.SEC)
+        assert np.array_equal(b.status, want) and np.array_equal(b.out_len, pt_len)
+        for s in (0, oracle.AUTH_FAIL, PKT_BAD_INNER, PKT_FILTER_DENY) + ((PKT_REPLAY,) if replay else ()):
+            assert np.count_nonzero(want == s) > 20, s
+        ok = want == 0
+        assert np.array_equal(b.slot, slot) and H.spans_differ_count(np.array(b.ring), plain, off[ok], pt_len[ok], 16) == 0
+        for s, r in state.items():
+            last, words = c.replay_export(s)
+            assert last == r.last and np.array_equal(words, r.ring())
+        assert H.flows_equal(c.flows_export(), f.flows())
+        note.close()
+        b.close()
