@@ -1484,8 +1484,16 @@ __device__ __forceinline__ void stream_work(const AeadArgs &a, StreamShared &sh,
     }
 }
 
+// A CTA stays on its SM until the batch ends, and another call's packets should not have to wait for that.  A quarter of an SM, which has
+// five of the 17 warps, has 16,384 registers: with 72 each (and a few in local memory) a warp of kernel 2 of up to 128 still fits beside
+// them, with the 94 that the kernel would take it does not; and both have to want the same share of the SM for shared memory (see
+// aead_kernels_init).  300 packets with own nonces beside other calls' batches sealed over and over, median and 99th of a hundred,
+// as it was / so: 9000 x 64 B 55 and 61 us / 43 and 51, 16,000 x 64 B 89 and 96 / 63 and 85, 16,000 mixed 29 and 199 / 31 and 148,
+// 40,000 mixed 49 and 427 / 52 and 178 (by packet or in pieces 43 and 69, 34 and 109, 33 and 117, 49 and 160).  The batches
+// themselves take the same time.
+constexpr int kStreamShare = 44; // of a hundred: 100 KB, which is what kernel 2's four CTAs get
 template <bool OPEN, bool NOTE>
-__global__ void __launch_bounds__(32 * kStreamWarps, 1) aead_stream_kernel(const __grid_constant__ AeadArgs a) {
+__global__ void __maxnreg__(72) aead_stream_kernel(const __grid_constant__ AeadArgs a) {
     static_assert(!(OPEN && NOTE), "flows are recorded on the seal side");
     let_next_kernel_start();
     __shared__ StreamShared sh;
@@ -1568,26 +1576,15 @@ cudaError_t launch_wpp(const AeadArgs &a, uint32_t ctas, const HostDesc *h, cuda
     return with(InlineDesc<kRankMax>{}, aead_wpp_kernel<OPEN, NOTE, kRankMax>);
 }
 
-// Tiles and grid of kernel 3.  With small packets every SM helps, 9000 x 64 B sealed by 96 CTAs 84 us, by 148 72; large ones
-// have as much outstanding as the link takes with fewer: 12,000 x 1420 B by 64 504 us, by 96 482, by 148 491.  Tiles of 16 are
-// worth a CTA each, smaller ones of 4 at the least spread a batch that has fewer than kStreamTiles of them.
-constexpr uint32_t kStreamCtas = 96, kStreamCtasSmall = 148, kStreamTiles = 64;
 static_assert(kStreamPackets >= kRankMax, "it hands out no nonces itself");
-void stream_grid(AeadArgs &a, uint32_t &ctas) {
-    const uint32_t most = a.link_bytes <= (uint64_t)kSmallPacket * a.n ? kStreamCtasSmall : kStreamCtas;
-    a.tile = 16;
-    while (a.tile > 4 && a.n < kStreamTiles * a.tile) a.tile /= 2;
-    const uint32_t tiles = (a.n + a.tile - 1) / a.tile, rounds = (tiles + most - 1) / most;
-    ctas = (tiles + rounds - 1) / rounds;
-}
 
 template <bool OPEN>
 cudaError_t launch_aead(AeadArgs a, cudaStream_t s, bnk_ctx *ctx) {
     if (a.n == 0) return cudaSuccess;
     if (a.stream) {
-        uint32_t ctas;
-        stream_grid(a, ctas);
-        const dim3 grid(ctas), block(32 * kStreamWarps);
+        const StreamGrid g = stream_grid(a.n, a.link_bytes);
+        a.tile = g.tile;
+        const dim3 grid(g.ctas), block(32 * kStreamWarps);
         const cudaError_t e = !OPEN && a.note ? launch_kernel(a.behind_kernel, aead_stream_kernel<OPEN, !OPEN>, grid, block, s, a)
                                               : launch_kernel(a.behind_kernel, aead_stream_kernel<OPEN, false>, grid, block, s, a);
         if (e != cudaSuccess) return e;
@@ -1615,5 +1612,12 @@ cudaError_t launch_aead(AeadArgs a, cudaStream_t s, bnk_ctx *ctx) {
 
 } // namespace
 
+cudaError_t aead_kernels_init() {
+    const auto share = [](auto kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kStreamShare); };
+    cudaError_t e = share(aead_stream_kernel<false, false>);
+    if (e == cudaSuccess) e = share(aead_stream_kernel<false, true>);
+    if (e == cudaSuccess) e = share(aead_stream_kernel<true, false>);
+    return e;
+}
 cudaError_t launch_seal(const AeadArgs &a, cudaStream_t s, bnk_ctx *ctx) { return launch_aead<false>(a, s, ctx); }
 cudaError_t launch_open(const AeadArgs &a, cudaStream_t s, bnk_ctx *ctx) { return launch_aead<true>(a, s, ctx); }

@@ -496,7 +496,7 @@ int bnk_ctx_create(const bnk_cfg *cfg, bnk_ctx **out) {
     ctx->addr_host.assign(islots, KeypairTables::AddrEntry{});
     tables.add(&ctx->kt.addr_tab, (size_t)islots);
     if ((e = tables.device()) != cudaSuccess) return bail("keypair tables", e);
-    if ((e = group_kernels_init()) != cudaSuccess) return bail("kernel attributes", e);
+    if ((e = group_kernels_init()) != cudaSuccess || (e = aead_kernels_init()) != cudaSuccess) return bail("kernel attributes", e);
     if ((e = filter_tables_alloc(ctx)) != cudaSuccess) return bail("filter tables", e);
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) return bail("sync", e);
     *out = ctx;

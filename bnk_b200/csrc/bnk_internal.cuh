@@ -368,6 +368,7 @@ constexpr uint32_t kGroupMax = 32768;
 cudaError_t launch_open_tail(bnk_batch *b, uint32_t n, bool replay, const VerdictArgs *verdict, const Done &done, cudaStream_t s);
 cudaError_t launch_verdict(bnk_ctx *ctx, const VerdictArgs &verdict, const Done &done, cudaStream_t s); // the last checks alone
 cudaError_t group_kernels_init(); // once per context, for the current device
+cudaError_t aead_kernels_init();
 cudaError_t launch_length_order(bnk_batch *b, uint32_t n, const uint32_t *len, bool open_side, cudaStream_t s);
 uint32_t group_sort_chunks(uint32_t max_pkts);
 uint32_t replay_scan_tiles(uint32_t max_pkts);     // tiles of the running-maximum scan

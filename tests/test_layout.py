@@ -15,6 +15,14 @@ extern "C" void look(const uint32_t *off, const uint32_t *len, uint32_t n, int o
     const uint64_t v[] = {r.end, r.sum, r.longest, r.lowest, r.joined, r.in_order, l.dense, n && in_stream(l, n, open)};
     for (int i = 0; i < 8; i++) out[i] = v[i];
 }
+// tile and CTAs, and whether every tile has one that takes it, as the kernel deals them out
+extern "C" void grid(uint32_t n, uint64_t bytes, uint32_t *out) {
+    const StreamGrid g = stream_grid(n, bytes);
+    const uint32_t tiles = (n + g.tile - 1) / g.tile, share = (tiles + g.ctas - 1) / g.ctas;
+    out[0] = g.tile;
+    out[1] = g.ctas;
+    out[2] = (uint64_t)g.ctas * share >= tiles;
+}
 """
 ROOM = {False: 32, True: 0}  # behind a payload that is sealed; behind a message that is opened
 
@@ -26,7 +34,8 @@ def look(tmp_path_factory):
     so = str(d / "look.so")
     subprocess.run(["g++", "-std=c++17", "-O3", "-fPIC", "-shared", "-I", ROOT, "-o", so, str(d / "look.cpp"),
                     os.path.join(ROOT, "bnk_b200", "host", "scan.cpp")], check=True)
-    f = C.CDLL(so).look
+    lib = C.CDLL(so)
+    f = lib.look
 
     def call(off, length, opened):
         off, length = np.ascontiguousarray(off, np.uint32), np.ascontiguousarray(length, np.uint32)
@@ -35,6 +44,7 @@ def look(tmp_path_factory):
           out.ctypes.data_as(C.c_void_p))
         return dict(zip(("end", "sum", "longest", "lowest", "joined", "in_order", "dense", "stream"), map(int, out)))
 
+    call.lib = lib
     return call
 
 
@@ -84,3 +94,12 @@ def test_batches_whose_packets_join_go_by_neighbours(look, opened):
     got = look(*_lies(4096, 1300 + extra, 1472), opened)
     assert got["dense"] and got["stream"] == (not opened)
     assert look(*_lies(20_000, 1300 + extra, 1472), opened)["stream"]
+
+
+@pytest.mark.parametrize("size", [60, 1420])
+def test_grid_leaves_room_for_other_calls(look, size):
+    out = (C.c_uint32 * 3)()
+    for n in [*range(257, 3000), *range(3000, 1_000_000, 997)]:
+        look.lib.grid(C.c_uint32(n), C.c_uint64(n * size), out)
+        tile, ctas, covered = out
+        assert tile in (4, 8, 16) and covered and 40 < ctas <= 143, n  # of 148 SMs
