@@ -221,14 +221,16 @@ def test_a_small_call_between_does_not_hide_what_is_behind(gpu_lib, oracle, betw
         c.close()
 
 
-@pytest.mark.parametrize("n,size", [(48, 300), (1000, 300), (12_000, 64)])  # in place twice, in pieces
-def test_device_only_submits_need_no_wait(gpu_lib, oracle, n, size):
+@pytest.mark.parametrize("n,size,pieces_from", [(48, 300, None), (1000, 300, None), (12_000, 64, None), (24_000, 64, 1 << 20)])  # in place, and in pieces
+def test_device_only_submits_need_no_wait(gpu_lib, oracle, monkeypatch, n, size, pieces_from):
     """A submit that touches no host array may follow any other without a wait in between."""
     from bnk_b200.device import F_ASSIGN_COUNTERS, F_NO_D2H, F_NO_H2D, F_REPLAY, F_USE_OUT_LEN
 
     rng = np.random.default_rng(n)
     stride = 48 + (size + 15) // 16 * 16
     keys = rng.integers(0, 256, (2, 32), dtype=np.uint8)
+    if pieces_from:
+        monkeypatch.setenv("BNK_PIECES_FROM", str(pieces_from))
     c = _context(512 << 20, max_keypairs=2, mtu=1420, flow_capacity=0)
     try:
         c.set_keypairs(0, keys, keys, np.arange(2, dtype=np.uint32))
@@ -236,7 +238,10 @@ def test_device_only_submits_need_no_wait(gpu_lib, oracle, n, size):
         b.off[:], b.len[:], b.slot[:] = np.arange(n) * stride, size, rng.integers(0, 2, n)
         b.ring[:] = rng.integers(0, 256, b.ring_bytes, dtype=np.uint8)
         plain = np.array(b.ring).reshape(n, stride)[:, 16:16 + size]
+        launched = c.launch_count()
         b.seal(n, F_ASSIGN_COUNTERS, wait=False)
+        launched = c.launch_count() - launched  # for the nonces, up to 256 packets none, and for the packets, of pieces each one
+        assert launched == 1 + (n > 256) if not pieces_from else launched > 2
         b.open(n, F_NO_H2D | F_NO_D2H | F_USE_OUT_LEN | F_REPLAY, wait=False)
         b.seal(n, F_NO_H2D | F_NO_D2H | F_ASSIGN_COUNTERS, wait=False)
         b.open(n, F_NO_H2D | F_NO_D2H | F_USE_OUT_LEN | F_REPLAY)
