@@ -574,12 +574,6 @@ struct Round {
     }
 };
 
-//
-// Seal batches of up to kRankMax packets in pinned memory hand out their nonces here (a.send_counter): a warp counts the
-// packets of its slot in front of its own, and the last packet of a slot moves the counter past them all (SendCounter
-// says why nobody has to wait for that).  A grouping launch in front took 5 us.
-// NOTE: the flows of the packets are recorded from the bytes in the stage, each step of the table's atomics behind a
-// piece of the cipher work.
 // Word `lane` (0..15) of the 64 bytes that start at a piece.
 __device__ __forceinline__ uint32_t stage_word(const uint4 *stage, uint32_t piece) {
     const uint32_t lane = threadIdx.x & 31;
@@ -729,6 +723,11 @@ __device__ __forceinline__ uint4 inner_head(const AeadArgs &a, const uint4 *stag
                       p.proto | (at != kParseBad ? kInnerParses : 0u) | (is_whole ? kInnerWhole : 0u), total);
 }
 
+// Seal batches of up to kRankMax packets in pinned memory hand out their nonces here (a.send_counter): a warp counts the
+// packets of its slot in front of its own, and the last packet of a slot moves the counter past them all (SendCounter
+// says why nobody has to wait for that).  A grouping launch in front took 5 us.
+// NOTE: the flows of the packets are recorded from the bytes in the stage, each step of the table's atomics behind a
+// piece of the cipher work.
 template <bool OPEN, bool NOTE, uint32_t INLINE>
 __global__ void __launch_bounds__(32 * kWppWarps, 4) aead_wpp_kernel(const __grid_constant__ AeadArgs a,
                                                                       const __grid_constant__ InlineDesc<INLINE> desc) {

@@ -227,7 +227,8 @@ bool heads_direct(bnk_batch *b, uint32_t npkts, uint32_t flags) {
 // Packets that lie close together go up and down by neighbours (see in_stream), and that kernel is ahead up to ctx->stream_pieces_from (64 MB); sealed, pieces /
 // in place: 11,000 mixed 204 us and 161, 16,000 262 and 222, 30,000 449 and 400, 20,000 x 64 B 144 and 126, 40,000 x 300 B 508 and 483,
 // 18,000 x 1420 B 815 and 741, 32,768 (48 MB) 1358 and 1315, 48,000 (71 MB) 1935 and 1916, 65,536 (96 MB) 2517 and 2595; opened 16,000 mixed
-// 264 and 221, 32,768 x 1420 B 1385 and 1342, 65,536 2535 and 2597.
+// 264 and 221, 32,768 x 1420 B 1385 and 1342, 65,536 2535 and 2597.  Of two in turn the second is copied while the first is in place, which
+// is no slower than both in pieces or copied: 24,000 x 1420 B 833 us a batch and 838, 32,768 1115 and 1125, 30,000 mixed 340 and 338.
 bool in_pieces(const bnk_batch *b, uint32_t n, uint32_t flags, uint64_t ext, const Layout &lay, bool open) {
     const bnk_ctx *const ctx = b->ctx;
     const bool stream = in_stream(lay, n, open) && ctx->aead_mode == 0 && ext <= ctx->host_direct_bytes;
