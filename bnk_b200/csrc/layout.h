@@ -40,17 +40,26 @@ inline Layout layout_of(const PacketScan &r, uint32_t n, uint32_t slack) {
 // 73 / 80, 65 67 / 76, all 56 / 73.  None joined: 9000 x 200 B 103 / 113 and 105 / 110, x 300 B 116 / 123 and 120 / 127, x 1000 B
 // 297 / 288 and 288 / 299, 4096 x 1300 B in slots of 1472 175 / 174 and 169 / 178, 12,000 x 1420 B 525 / 517 and 499 / 520; 30 of a hundred
 // joined: 9000 x 1000 B 296 / 303 and 282 / 295, 12,000 x 1420 B 524 / 521 and 495 / 508.
-// Where the other way would be pieces (see in_pieces) or very many warps, it takes less: 20,000 x 64 B, none joined, 156 / 166 and 179 /
-// 192, 35 of a hundred 149 / 159 and 151 / 166, half 143 / 157 and 132 / 143; none joined x 100 B 183 / 206 and 180 / 196, x 150 B 211 / 223 and 186 / 207, x 300 B in
-// slots of 400 329 / 317 and 254 / 267, 1056 to 1408 B in slots of 1472 881 / 900 and 726 / 748, x 1420 B 891 / 910 and 819 / 848.
+// Of very many small packets the other way is pieces (see in_pieces), which copy what lies between them as well and of which each has its own
+// start; the more packets, the less that counts.  None joined, in pieces and in the stream: 11,000 x 64 B 107 / 123 and 113 / 122, x 100 B 136 /
+// 146 and 114 / 124; 15,000 x 200 B 202 / 217 and 169 / 185; 20,000 x 64 B 159 / 173 and 189 / 207, x 128 B 191 / 212 and 198 / 217, x 150 B 217 / 228 and
+// 202 / 216, x 300 B in slots of 400 329 / 317 and 254 / 267; 40,000 x 100 B 324 / 338 and 370 / 392, x 150 B 384 / 401 and 395 / 416, x 200 B 432 / 450 and 412 /
+// 439; 80,000 x 200 B 782 / 807 and 816 / 869, x 250 B 865 / 899 and 870 / 916, x 300 B 993 / 1009 and 909 / 944; 64 B of which half join, 20,000 146 / 161
+// and 135 / 150, 40,000 250 / 262 and 257 / 285.  In no order it is by packet: 16,000 x 150 B 160 / 166 and 171 / 188, x 200 B 160 / 171 and 174 / 187, x 250 B
+// 204 / 209 and 196 / 213, x 300 B 225 / 230 and 211 / 226.
+// And of large ones beyond 24 MB, none joined: 20,000 of 1056 to 1408 B in slots of 1472 881 / 900 and 726 / 748, x 1420 B 891 / 910 and 819 / 848.
 constexpr uint32_t kStreamPackets = 256, kManySmall = 10240, kSmallPacket = 512;
 constexpr uint64_t kStreamFrom = 512u << 10, kStreamSmallFrom = 896u << 10, kStreamOpenFrom = 4u << 20, kStreamLarge = 24u << 20;
-constexpr uint32_t kStreamCopy = 1000, kStreamOpenCopy = 1520, kStreamSmallCopy = 180; // bytes
+constexpr uint32_t kStreamCopy = 1000, kStreamOpenCopy = 1520, kStreamSmallCopy = 290; // bytes
+constexpr uint32_t kStreamOrderedCopy = 120, kStreamOrderedPer = 400;                  // and a byte more for each so many packets
 inline bool in_stream(const Layout &l, uint32_t n, bool open) {
     const bool small = l.bytes <= (uint64_t)kSmallPacket * n;
     if (!l.dense || n <= kStreamPackets || l.bytes < (open == small ? kStreamFrom : open ? kStreamOpenFrom : kStreamSmallFrom)) return false;
     const uint64_t copies = n - l.joined; // (or a few more)
-    if (small) return 8ull * l.joined >= 5ull * n || (n >= kManySmall && l.bytes >= kStreamSmallCopy * copies);
+    if (small) {
+        const uint64_t least = l.in_order ? kStreamOrderedCopy + n / kStreamOrderedPer : kStreamSmallCopy;
+        return 8ull * l.joined >= 5ull * n || (n >= kManySmall && l.bytes >= least * copies);
+    }
     return l.end >= kStreamLarge || l.bytes >= (open ? kStreamOpenCopy : kStreamCopy) * copies;
 }
 

@@ -90,6 +90,10 @@ def test_batches_whose_packets_join_go_by_neighbours(look, opened):
         got = look(*_lies(n, size + extra, step, order), opened)
         assert not got["stream"], name
         assert got["dense"] == (name in ("falling", "any order", "slots", "few")), name
+    # very many small ones that do not join: as many bytes a copy as there is little to gain in pieces; in no order more
+    for n, size, step, order, goes in ((20_000, 64, 128, None, False), (20_000, 150, 224, None, True), (80_000, 150, 224, None, False), (80_000, 300, 384, None, True),
+                                       (16_000, 200, 240, rng.permutation(16_000), False), (16_000, 300, 352, rng.permutation(16_000), True)):
+        assert look(*_lies(n, size + extra, step, order), opened)["stream"] == goes, (n, size)
     # large packets that do not join are sealed that way, and opened only where they would otherwise go in pieces
     got = look(*_lies(4096, 1300 + extra, 1472), opened)
     assert got["dense"] and got["stream"] == (not opened)
